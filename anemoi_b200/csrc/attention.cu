@@ -4,27 +4,36 @@
 // shape) and walks that tile's ragged list of 64-key stages in the order
 // NVFP4 -> INT8 -> FP16 with one online-softmax state.
 //
-// Warp roles (256 threads = two warpgroups; the second one gives most of its registers to the
-// first with setmaxnreg, so a softmax thread may use 192 registers at two CTAs per SM):
-//   warps 0-3  softmax: warp w owns TMEM lanes 32*w.. (query rows); one thread per row holds
-//              the row's 64 scores of a stage in registers (few threads with long unrolled
-//              instruction streams: the per-stage fixed cost is paid once per row)
-//   warp 4     loader: one lane issues 1-D bulk copies (TMA engine) of the Q record of
-//              each phase and of one K|V record per stage into a ring of shared-memory
-//              slots, completion counted on mbarriers
-//   warp 5     MMA: allocates TMEM; one lane issues tcgen05.mma
-//                S[128x64]  = Q K^T   kind::mxf4nvf4 / kind::i8 / kind::f16
-//                O[128xD]  += P V     kind::mxf4nvf4 / kind::f8f6f4 / kind::f16
-//              and tcgen05.commit to mbarriers
-//   warps 6-7  idle (they complete the second warpgroup)
-// TMEM columns: S0 [0,64), O [64,64+D), and [192,256) holds the NVFP4 scale factors in the
-// NVFP4 phase and a second score buffer S1 in the INT8 / FP16 phases (QK of stage g+1 runs
-// while the softmax threads still read the scores of stage g).
-// O stays in TMEM across all stages; it is rescaled (read-modify-write by the
-// softmax threads) only when some row's running maximum moved, and at a phase
-// change, where it is also converted between the phases' value domains.  P is
-// double-buffered in shared memory for the 4- and 8-bit cells, so the softmax
-// threads only wait for the previous PV when they have to rescale O.
+// Roles (512 threads = four warpgroups, two CTAs per SM; registers move between them with setmaxnreg):
+//   warps 0-3, 4-7  softmax of the even and of the odd stages: warp w owns TMEM lanes 32*(w%4)..
+//                   (query rows), one thread per row with the row's 64 scores in registers
+//   warps 8-11      rescale of O: when a stage moved some row's maximum, or at a phase change
+//                   (where O also moves between the phases' value domains)
+//   warp 12         loader: one lane issues 1-D bulk copies (TMA engine) of the Q record of each
+//                   phase and of one K|V record per stage into a ring of shared-memory slots
+//   warp 13         S[128x64]  = Q K^T   kind::mxf4nvf4 / kind::i8 / kind::f16
+//   warp 14         O[128xD]  += P V     kind::mxf4nvf4 / kind::f8f6f4 / kind::f16
+//   warp 15         idle
+// TMEM columns: S0 [0,64), O [64,64+D), a second score buffer S1 and the NVFP4 scale factors
+// (which share [192,256) at D = 128: the NVFP4 phase then has one score buffer).
+//
+// Why this split.  A stage needs 8,192 exponentials = 512 cycles of the special-function unit and
+// 130-580 cycles of the tensor core per SM, but one warp's chain through a stage (wait for S, load
+// it, maximum, exponentials, conversion, store, fence, arrive) is over 2,000 cycles long, and with
+// one softmax warp per row quadrant and CTA (8 per SM, all that tensor memory and two query tiles
+// allow) latency set the pace: 1,250-1,400 cycles per stage and SM.  So two warpgroups share a tile
+// and run alternate stages.  P is quantised against the running maximum of a strictly sequential
+// walk, so the maximum is handed from stage to stage through shared memory as soon as it is known,
+// and the exponentials of two stages overlap.  O's rescale, which waits for the previous PV, is
+// off the softmax warps' path; QK and PV are issued by different warps so that QK of a stage waits
+// for nothing but its key tile and its score buffer.
+// Measured per stage and SM at D = 128, cycles, before -> now: NVFP4 1,282 -> 811, INT8 1,394 -> 853,
+// FP16 1,332 -> 1,170, the mixed layer of S = 85,184 (8 heads) 1,250 -> 943 (6.55 -> 4.94 ms).
+// Now bound by instruction issue (about 600 warp instructions per stage and scheduler) and the
+// special-function unit; FP16 by its 32 KB per stage, of which two stages and a half fit in a ring.
+//
+// P is stored over the stage's K tile, which the tensor core has finished reading when the scores
+// arrive; that leaves the ring all of the shared memory that Q does not take.
 //
 // Numerics follow the reference's phases
 // (csrc/attention/cuda/sm120/q64_attention_phase_composer.inl:1-146, 506-932,
@@ -38,10 +47,7 @@
 //   FP16 : P -> f16
 // Accumulation is fp32 in TMEM (the reference accumulates a stage in fp16 for the
 // INT8 and FP16 cells).
-#include <climits>
 #include <cuda_fp16.h>
-#include <cuda_fp4.h>
-#include <cuda_fp8.h>
 
 #include "bounded_wait.cuh"
 #include "records.cuh"
@@ -51,24 +57,37 @@ namespace {
 
 using namespace sm100;
 
-constexpr int kThreads = 256;         // two warpgroups: softmax | loader, MMA and two idle warps
-constexpr int kSoftmaxRegs = 192;     // 128 * 192 + 128 * 64 == 256 * 128 (two CTAs per SM)
-constexpr int kOtherRegs = 64;
-constexpr int kSoftmaxThreads = 128;
-constexpr int kLoaderWarp = 4;
-constexpr int kMmaWarp = 5;
+// Four warpgroups: softmax of the even stages, softmax of the odd stages, rescale of O, and
+// loader / QK / PV (one warp each, the fourth idle).
+constexpr int kThreads = 512;
+constexpr int kSoftmaxRegs = 88;  // 128 * (2 * 88 + 48 + 32) == 512 * 64 (two CTAs per SM)
+constexpr int kCorrRegs = 48;
+constexpr int kOtherRegs = 32;
+constexpr int kCorrWarp = 8;
+constexpr int kLoaderWarp = 12;
+constexpr int kQkWarp = 13;
+constexpr int kPvWarp = 14;
+enum WaitRole : int { kSoftmaxRole = 0, kRescaleRole = 1, kMmaRole = 2 };
 constexpr int kTmemCols = 256;
 constexpr int kColS = 0;
-constexpr int kColS1 = 192;  // second score buffer; aliases the scale-factor columns
 constexpr int kColO = 64;
 constexpr int kColSfaQ = 192;  // 2 k-steps x 4 columns
 constexpr int kColSfbK = 200;  // 2 k-steps x 4 columns
 constexpr int kColSfaP = 208;
 constexpr int kColSfbV = 212;
-constexpr int kMaxSlots = 8;
+constexpr int kRing = 8;       // entries of the per-stage rings, and the most key/value slots
 constexpr float kFp8Offset = 8.807f;
+constexpr uint64_t kDrainNs = 100000000;  // limit of the waits for copies and MMAs in flight after a give-up
 
 enum Cell : int { kNv = 0, kI8 = 1, kF16 = 2 };
+// Which cells a kernel is built for: one, or any mix.
+enum Cells : int { kAny = 3 };
+
+// Second score buffer: D = 128 aliases the scale-factor columns, D = 64 has room behind O.
+template <int D>
+struct Cols {
+  static constexpr int kS1 = D == 128 ? 192 : 128;
+};
 
 struct AttnParams {
   anemoi_sm100_shape s;
@@ -92,21 +111,30 @@ struct AttnParams {
   int out_rows;      // rows per head in `out`
   int ring_bytes;    // key/value ring; re-partitioned into equal slots at every phase
   int q_region;      // bytes
-  int p_region;      // bytes
 };
 
-struct Barriers {
-  uint64_t kv_full[kMaxSlots];
-  uint64_t kv_free[kMaxSlots];
+// Entry g % kRing of a ring belongs to stage g, in phase g / kRing of the barrier.  Stage
+// g + kRing cannot begin before PV of stage g is complete (it needs a key/value slot and there are
+// at most kRing), so no entry is reused while a role still needs it, and no waiter can miss a phase.
+struct Shared {
+  uint64_t kv_full[kRing];    // key/value record landed
+  uint64_t pv_done[kRing];    // PV complete: slot free, O may be touched
+  uint64_t p_full[kRing];     // per quadrant: P stored (softmax warp), O in the right scale (rescale warp)
+  uint64_t m_full[4][kRing];  // running maxima of the quadrant's rows up to this stage published
+  uint64_t v_full;            // value tile landed (phases whose key and value tiles have rings of their own)
   uint64_t q_full, q_free;
-  uint64_t s_full[2];  // scores ready, per score buffer
-  uint64_t s_free;     // scores read by the softmax warps (NVFP4 phase: single buffer)
-  uint64_t all_done;  // every MMA of the tile complete (epilogue)
-  // Two P barriers used alternately: a warp that skips the wait for the previous PV may run one stage
-  // ahead, and its arrival must not be counted into the previous stage's phase.
-  uint64_t p_full[2];
+  uint64_t s_full[2];  // scores ready, per softmax warpgroup (a waiter has to see every phase)
+  uint64_t s_free[2];  // scores read, per score buffer
+  uint64_t nv_done;    // every PV of the NVFP4 phase complete
+  uint64_t all_done;   // every PV of the tile complete
+  uint64_t qk_done;    // unwinding only
   WaitContext wc;
+  int cnt[3], first_of[3];  // the tile's stages per phase, where each phase starts inside the list
   uint32_t tmem_base;
+  // per stage and query block of the tile: score scale, real keys (negative: not a stage of this block)
+  float2 meta[kRing][2];
+  // per stage and row: running maximum m(g), denominator d(g - 2)
+  float2 rec[kRing][128];
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -137,7 +165,6 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
-
 __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
   float2 d;
   asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
@@ -146,197 +173,214 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
+// Four fp32 -> four e4m3, eight fp32 -> eight e2m1, in element order (one register, no byte shuffles).
+__device__ __forceinline__ uint32_t e4m3x4(float a, float b, float c, float d) {
+  uint32_t v;
+  asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n\tmov.b32 %0, {lo, hi};\n\t}"
+      : "=r"(v)
+      : "f"(a), "f"(b), "f"(c), "f"(d));
+  return v;
+}
+__device__ __forceinline__ uint32_t e2m1x8(const float* e) {
+  uint32_t v;
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\tcvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\tcvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\tmov.b32 %0, {b0, b1, b2, b3};\n\t}"
+      : "=r"(v)
+      : "f"(e[0]), "f"(e[1]), "f"(e[2]), "f"(e[3]), "f"(e[4]), "f"(e[5]), "f"(e[6]), "f"(e[7]));
+  return v;
+}
+__device__ __forceinline__ uint32_t f16x2(float a, float b) {
+  uint32_t v;
+  asm("cvt.rn.f16x2.f32 %0, %2, %1;" : "=r"(v) : "f"(a), "f"(b));
+  return v;
+}
 
 __device__ __forceinline__ void tmem_st4(uint32_t taddr, uint32_t v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(v),
                "r"(v), "r"(v), "r"(v)
                : "memory");
 }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(r));
+  return r != 0;
+}
+// `issue` == 0 turns the arrival into a no-op (predicated, no branch).
+__device__ __forceinline__ void mbar_arrive_if(uint64_t* bar, uint32_t issue) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(
+          smem_u32(bar)),
+      "r"(issue)
+      : "memory");
+}
 
+// ------------------------------------------------------------------------------------------
+// geometry of a key/value slot
+// ------------------------------------------------------------------------------------------
+// The P tile of a stage (128 rows x 64 keys) takes the place of the stage's K tile, which the
+// tensor core has finished reading when the scores arrive; what follows K in the record (V, scale
+// blocks) starts behind the larger of the two.
+__host__ __device__ constexpr int k_bytes(int d, int cell) { return 32 * d * (cell == kF16 ? 4 : cell == kI8 ? 2 : 1); }
+__host__ __device__ constexpr int p_bytes(int cell) { return 4096 * (cell == kF16 ? 4 : cell == kI8 ? 2 : 1); }
+__host__ __device__ constexpr int record_bytes(int d, int cell) {
+  return cell == kNv ? 64 * d + (d / 64) * 512 + 512 : (cell == kI8 ? 128 * d : 256 * d);
+}
+__host__ __device__ constexpr int rest_offset(int d, int cell) {
+  return k_bytes(d, cell) > p_bytes(cell) ? k_bytes(d, cell) : p_bytes(cell);
+}
+__host__ __device__ constexpr int slot_bytes(int d, int cell) {
+  return (rest_offset(d, cell) + record_bytes(d, cell) - k_bytes(d, cell) + 127) & ~127;
+}
+// FP16 at D = 128: two whole slots of 32 KB would fit, but a slot is held from the start of its
+// copy to the end of its PV.  Key tiles (which P replaces) get three buffers and values one: the
+// value copy of stage g + 1 runs while stage g + 1's probabilities are computed.
+__host__ __device__ constexpr bool split_kv(int d, int cell) { return d == 128 && cell == kF16; }
+__host__ __device__ constexpr int stage_bytes(int d, int cell) {  // distance of two slots
+  return split_kv(d, cell) ? rest_offset(d, cell) : slot_bytes(d, cell);
+}
+__host__ __device__ constexpr int slot_count(int ring, int d, int cell) {
+  const int n = split_kv(d, cell) ? ring / rest_offset(d, cell) - 1 : ring / slot_bytes(d, cell);
+  return n < kRing ? n : kRing;
+}
+// Score buffer of stage g: the NVFP4 phase of D = 128 has a single one (the other's columns
+// hold its scale factors).
 template <int D>
-struct CellInfo {
-  // bytes per stage record and per Q record, chunk counts (16-byte chunks per row)
-  __device__ static int kv_bytes(int cell) {
-    return cell == kNv ? (int)rec::kv_nvfp4_bytes(D)
-                       : (cell == kI8 ? (int)rec::kv_int8_bytes(D) : (int)rec::kv_fp16_bytes(D));
-  }
-  __device__ static int q_bytes(int cell, int qb) {
-    return cell == kNv ? (int)rec::q_nvfp4_bytes(qb, D)
-                       : (cell == kI8 ? (int)rec::q_int8_bytes(qb, D) : (int)rec::q_fp16_bytes(qb, D));
-  }
-};
+__device__ __forceinline__ int s_buffer(int cell, int g) {
+  return D == 128 && cell == kNv ? 0 : (g & 1);
+}
 
-// ------------------------------------------------------------------------------------------
-// softmax side
-// ------------------------------------------------------------------------------------------
-struct RowState {
-  float m, d;
-};
-
-// O[row][c] *= alpha (* colf[c] when kColf) for all D columns of the thread's row, 64 columns
-// (two TMEM loads in flight) per step.
-template <int D, bool kColf>
+// O[row][c] *= alpha (* colf[c] when given) for all D columns of the thread's row.
+template <int D>
 __device__ __forceinline__ void rescale_o(uint32_t tmem_row, float alpha, const float* colf) {
   const float2 alpha2 = make_float2(alpha, alpha);
 #pragma unroll 1
-  for (int c0 = 0; c0 < D; c0 += 64) {
-    uint32_t r[64];
-    tmem_ld32(tmem_row + kColO + c0, *reinterpret_cast<uint32_t(*)[32]>(r));
-    tmem_ld32(tmem_row + kColO + c0 + 32, *reinterpret_cast<uint32_t(*)[32]>(r + 32));
+  for (int c0 = 0; c0 < D; c0 += 32) {
+    uint32_t r[32];
+    tmem_ld32(tmem_row + kColO + c0, r);
     tmem_wait_ld();
 #pragma unroll
-    for (int j = 0; j < 64; j += 2) {
-      float2 v = fmul2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), alpha2);
-      if (kColf) v = fmul2(v, *reinterpret_cast<const float2*>(colf + c0 + j));
+    for (int j = 0; j < 32; j += 2) {
+      const float2 v = fmul2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), alpha2);
       r[j] = __float_as_uint(v.x);
       r[j + 1] = __float_as_uint(v.y);
     }
-    tmem_st32(tmem_row + kColO + c0, *reinterpret_cast<uint32_t(*)[32]>(r));
-    tmem_st32(tmem_row + kColO + c0 + 32, *reinterpret_cast<uint32_t(*)[32]>(r + 32));
+    if (colf != nullptr) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) {
+        const float2 v = fmul2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])),
+                               *reinterpret_cast<const float2*>(colf + c0 + j));
+        r[j] = __float_as_uint(v.x);
+        r[j + 1] = __float_as_uint(v.y);
+      }
+    }
+    tmem_st32(tmem_row + kColO + c0, r);
   }
   tmem_wait_st();
 }
 
-// Writes the thread's 64 probabilities (one query row of the stage) into the K-major P tile
-// in shared memory.
+// ------------------------------------------------------------------------------------------
+// softmax side
+// ------------------------------------------------------------------------------------------
+// Probabilities of the thread's 64 scores, P = 2^(s * scale + bias), rounded to the cell's operand
+// format and stored into its row of the K-major P tile 16 bytes at a time (the conversions and
+// stores of one piece run under the exponentials of the next); returns their unrounded sum.
 template <int CELL>
-__device__ __forceinline__ void write_p(uint8_t* p_tile, int row, const float (&p)[64]) {
-  if (CELL == kF16) {
+__device__ __forceinline__ float exp_store(const float (&s)[64], float scale, float bias,
+                                           uint8_t* p_row) {
+  const float2 scale2 = make_float2(scale, scale);
+  const float2 bias2 = make_float2(bias, bias);
+  float2 acc0 = make_float2(0.0f, 0.0f), acc1 = make_float2(0.0f, 0.0f);
+  constexpr int kPer = CELL == kNv ? 32 : (CELL == kI8 ? 16 : 8);  // keys per 16 bytes
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      uint4 v;
-      __half2* h = reinterpret_cast<__half2*>(&v);
+  for (int c = 0; c < 64 / kPer; ++c) {
+    float e[kPer];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(p[j * 8 + 2 * i], p[j * 8 + 2 * i + 1]);
-      *reinterpret_cast<uint4*>(p_tile + rec::tile_offset(row, j, 8)) = v;
+    for (int j = 0; j < kPer; j += 4) {
+      const float2 a0 = ffma2(make_float2(s[c * kPer + j], s[c * kPer + j + 1]), scale2, bias2);
+      const float2 a1 = ffma2(make_float2(s[c * kPer + j + 2], s[c * kPer + j + 3]), scale2, bias2);
+      e[j] = ex2(a0.x);
+      e[j + 1] = ex2(a0.y);
+      e[j + 2] = ex2(a1.x);
+      e[j + 3] = ex2(a1.y);
+      acc0 = fadd2(acc0, make_float2(e[j], e[j + 1]));
+      acc1 = fadd2(acc1, make_float2(e[j + 2], e[j + 3]));
     }
-  } else if (CELL == kI8) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint4 v;
-      uint16_t* h = reinterpret_cast<uint16_t*>(&v);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        h[i] = __nv_cvt_float2_to_fp8x2(make_float2(p[j * 16 + 2 * i], p[j * 16 + 2 * i + 1]),
-                                        __NV_SATFINITE, __NV_E4M3);
-      *reinterpret_cast<uint4*>(p_tile + rec::tile_offset(row, j, 4)) = v;
+    uint4 v;
+    if (CELL == kF16) {
+      v = make_uint4(f16x2(e[0], e[1]), f16x2(e[2], e[3]), f16x2(e[4], e[5]), f16x2(e[6], e[7]));
+    } else if (CELL == kI8) {
+      v = make_uint4(e4m3x4(e[0], e[1], e[2], e[3]), e4m3x4(e[4 % kPer], e[5 % kPer], e[6 % kPer], e[7 % kPer]),
+                     e4m3x4(e[8 % kPer], e[9 % kPer], e[10 % kPer], e[11 % kPer]),
+                     e4m3x4(e[12 % kPer], e[13 % kPer], e[14 % kPer], e[15 % kPer]));
+    } else {
+      v = make_uint4(e2m1x8(e), e2m1x8(e + 8 % kPer), e2m1x8(e + 16 % kPer), e2m1x8(e + 24 % kPer));  // e holds 6 P
     }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      uint4 v;
-      uint8_t* h = reinterpret_cast<uint8_t*>(&v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        h[i] = __nv_cvt_float2_to_fp4x2(make_float2(p[j * 32 + 2 * i], p[j * 32 + 2 * i + 1]),
-                                        __NV_E2M1, cudaRoundNearest);  // p already holds 6 P
-      *reinterpret_cast<uint4*>(p_tile + rec::tile_offset(row, j, 2)) = v;
-    }
+    *reinterpret_cast<uint4*>(p_row + c * 128) = v;
   }
+  return (acc0.x + acc0.y) + (acc1.x + acc1.y);
 }
 
-// A row of zeros in the P tile (a stage that does not belong to this row's query block).
-__device__ __forceinline__ void write_zero_p(uint8_t* p_tile, int row, int cell) {
-  const int chunks = cell == kF16 ? 8 : (cell == kI8 ? 4 : 2);
-  for (int j = 0; j < chunks; ++j)
-    *reinterpret_cast<uint4*>(p_tile + rec::tile_offset(row, j, chunks)) = make_uint4(0, 0, 0, 0);
-}
+// State of a softmax row.  The two softmax warpgroups alternate stages; the running maximum and
+// the denominator travel between them through Shared::rec.  The denominator is carried two stages
+// late, so that a group waits for nothing but the other's maximum: entry g holds m(g) and d(g - 2),
+// and d(g) = d(g - 1) * alpha(g) + sum(g) is formed by the group that ran stage g when it publishes
+// stage g + 2 - the order (and rounding) of a strictly sequential walk.
+struct SoftmaxWalk {
+  uint32_t s_par;     // parity of this group's next scores
+  float d;            // denominator before the last two stages of this group's last stage
+  float alpha, sum;   // of this group's last stage
+};
 
-// Bytes of one P tile (128 rows x 64 keys) per cell, and which of the two buffers stage g uses.
-__device__ __forceinline__ int p_tile_bytes(int cell) {
-  return cell == kNv ? 128 * 32 : (cell == kI8 ? 128 * 64 : 128 * 128);
-}
-__device__ __forceinline__ int p_buffer(int cell, int g) { return cell == kF16 ? 0 : (g & 1); }
-// Score buffer of stage g: the NVFP4 phase has a single one (the other holds its scale factors).
-__device__ __forceinline__ int s_buffer(int cell, int g) { return cell == kNv ? 0 : (g & 1); }
-__device__ __forceinline__ uint32_t s_column(int sb) { return sb ? kColS1 : kColS; }
-
-// One stage of one phase for the thread's row.  A single copy of this code serves the three
-// cells (the cell is a run-time value): the kernel's hot code has to stay well inside the
-// instruction cache, and three unrolled copies did not.
-template <int D>
-__device__ __forceinline__ void softmax_stage(Barriers* b, const AttnParams& p, uint8_t* p_smem,
-                                              const float* colf, uint32_t tmem_row, int row,
-                                              int cell, int g, bool phase_first,
-                                              float score_scale, int valid, bool live_warp,
-                                              bool member, int sb, uint32_t s_parity,
-                                              uint64_t* prev_pv_bar, uint32_t prev_pv_parity,
-                                              RowState& st) {
-  wait(&b->wc, &b->s_full[sb], s_parity, 10 + cell);
+// One stage.
+template <int D, bool kPairs>
+__device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_t tmem_row, int row, int g, int cell,
+                                              bool live_warp, int my_block, SoftmaxWalk& w) {
+  const int at = g & (kRing - 1), before_at = (g - 1) & (kRing - 1);
+  uint64_t* m_full = b->m_full[row >> 5];
+  const uint32_t lead = (row & 31) == 0;
+  const int sb = s_buffer<D>(cell, g);
+  wait(&b->wc, &b->s_full[g & 1], w.s_par, 10);
+  w.s_par ^= 1u;
   tc_fence_after_sync();
-  // Barrier arrivals are one per warp (lane 0 after a warp sync).
-  const bool lead = (row & 31) == 0;
-  if (!live_warp) {
-    // padding rows of a 64-row tile: keep the barrier protocol, skip the math
-    if (lead) {
-      if (cell == kNv) mbar_arrive(&b->s_free);
-      mbar_arrive(&b->p_full[g & 1]);
-    }
-    return;
-  }
-  if (!member) {
-    // A stage of the other query block of the pair (warp-uniform: a warp's rows belong to one
-    // block).  These rows contribute nothing: P = 0, running maximum and denominator untouched.
-    // O still has to change its value domain at the first stage of a phase.
-    if (cell == kNv) {
-      __syncwarp();
-      if (lead) mbar_arrive(&b->s_free);
-    }
-    if (g > 0 && (phase_first || cell == kF16)) {
-      wait(&b->wc, prev_pv_bar, prev_pv_parity, 20 + cell);
-      tc_fence_after_sync();
-      if (phase_first) rescale_o<D, true>(tmem_row, 1.0f, colf);
-    }
-    write_zero_p(p_smem + p_buffer(cell, g) * p_tile_bytes(cell), row, cell);
-    fence_proxy_async_smem();
-    tc_fence_before_sync();
-    __syncwarp();
-    if (lead) mbar_arrive(&b->p_full[g & 1]);
-    return;
-  }
+  const uint32_t tmem_s = tmem_row + (sb ? Cols<D>::kS1 : kColS);
   float s[64];
   {
     uint32_t r[64];
-    tmem_ld32(tmem_row + s_column(sb), *reinterpret_cast<uint32_t(*)[32]>(r));
-    tmem_ld32(tmem_row + s_column(sb) + 32, *reinterpret_cast<uint32_t(*)[32]>(r + 32));
+    tmem_ld32(tmem_s, *reinterpret_cast<uint32_t(*)[32]>(r));
+    tmem_ld32(tmem_s + 32, *reinterpret_cast<uint32_t(*)[32]>(r + 32));
     tmem_wait_ld();
-    if (cell == kNv) {
-      // Only the NVFP4 phase has a single score buffer, whose release the MMA warp must see
-      // before the next QK.  With two buffers, QK of stage g+2 is issued after the MMA warp has
-      // waited for P of stage g, which every softmax thread writes after this load.
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lead) mbar_arrive(&b->s_free);
-    }
-    if (cell == kI8) {
-      // Scores are s32; as_float(i + 0x4B400000) == 12582912 + i exactly for |i| < 2^22, so
-      // the conversion is an integer add and a float subtract (no conversion instruction).
-      const float2 magic2 = make_float2(-12582912.0f, -12582912.0f);
 #pragma unroll
-      for (int j = 0; j < 64; j += 2) {
-        const float2 v = fadd2(make_float2(__int_as_float((int)r[j] + 0x4B400000),
-                                           __int_as_float((int)r[j + 1] + 0x4B400000)),
-                               magic2);
-        s[j] = v.x;
-        s[j + 1] = v.y;
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 64; ++j) s[j] = __uint_as_float(r[j]);
-    }
+    for (int j = 0; j < 64; ++j) s[j] = __uint_as_float(r[j]);
   }
-  if (valid < 64) {
-    // ragged blocks usually lose only a few keys: the common case touches the last 8 columns
-    if (valid >= 56) {
+  // (the loader wrote the stage's metadata before it started the copy of the stage's key tile)
+  const float2 meta = b->meta[at][kPairs ? my_block : 0];
+  const float scale = meta.x;
+  const int valid = __float_as_int(meta.y);
+  tc_fence_before_sync();
+  __syncwarp();
+  mbar_arrive_if(&b->s_free[sb], lead);
+  // Padding rows of a 64-row tile, and stages of the other query block of the pair (warp-uniform: a
+  // warp's rows belong to one block), contribute nothing: P = 0, running maximum and denominator
+  // untouched.
+  const bool active = !kPairs || (live_warp && valid >= 0);
+  float mx = -INFINITY;
+  if (active) {
+    if (cell == kI8) {
+#pragma unroll
+      for (int j = 0; j < 64; ++j) s[j] = __int2float_rn(__float_as_int(s[j]));  // |score| < 2^22: exact
+    }
+    if (valid < 64) {
+      // ragged blocks usually lose only a few keys: the common case touches the last 8 columns
 #pragma unroll
       for (int j = 56; j < 64; ++j) s[j] = j < valid ? s[j] : -INFINITY;
-    } else {
+      if (valid < 56) {
 #pragma unroll
-      for (int j = 0; j < 64; ++j) s[j] = j < valid ? s[j] : -INFINITY;
+        for (int j = 0; j < 56; ++j) s[j] = j < valid ? s[j] : -INFINITY;
+      }
     }
-  }
-  float mx;
-  {
     float m0 = max3(s[0], s[1], s[2]), m1 = max3(s[3], s[4], s[5]);
     float m2 = max3(s[6], s[7], s[8]), m3 = max3(s[9], s[10], s[11]);
 #pragma unroll
@@ -350,141 +394,114 @@ __device__ __forceinline__ void softmax_stage(Barriers* b, const AttnParams& p, 
     m1 = max3(m1, s[62], s[63]);
     mx = fmaxf(max3(m0, m1, m2), m3);
   }
-
-  const float m_new = fmaxf(st.m, mx * score_scale);
-  const float alpha = ex2(st.m - m_new);
-  // exponent = s * scale + bias; the NVFP4 cell produces 6 P directly (e2m1 input range),
-  // the INT8 cell P * 2^8.807 (e4m3 input range); the sums are scaled back.
-  const float bias = cell == kI8 ? kFp8Offset - m_new
-                                 : (cell == kNv ? 2.5849625007f - m_new : -m_new);
-  const float sum_scale = cell == kI8 ? 0.0022326917f : (cell == kNv ? 0.16666667f : 1.0f);
-  const float2 scale2 = make_float2(score_scale, score_scale);
-  const float2 bias2 = make_float2(bias, bias);
-  float2 acc0 = make_float2(0.0f, 0.0f), acc1 = make_float2(0.0f, 0.0f);
-#pragma unroll
-  for (int j = 0; j < 64; j += 4) {
-    const float2 a0 = ffma2(make_float2(s[j], s[j + 1]), scale2, bias2);
-    const float2 a1 = ffma2(make_float2(s[j + 2], s[j + 3]), scale2, bias2);
-    const float e0 = ex2(a0.x), e1 = ex2(a0.y), e2 = ex2(a1.x), e3 = ex2(a1.y);
-    s[j] = e0;
-    s[j + 1] = e1;
-    s[j + 2] = e2;
-    s[j + 3] = e3;
-    acc0 = fadd2(acc0, make_float2(e0, e1));
-    acc1 = fadd2(acc1, make_float2(e2, e3));
-  }
-  const float sum = ((acc0.x + acc0.y) + (acc1.x + acc1.y)) * sum_scale;
-  st.d = st.d * alpha + sum;
-  st.m = m_new;
-
-  if (g > 0) {
-    const bool need = phase_first || __any_sync(0xffffffffu, alpha != 1.0f);
-    // O may only be touched once the previous PV is complete.  The single FP16 P
-    // buffer also needs that; the double-buffered 4/8-bit P tiles are free as soon as
-    // this stage's scores arrived (QK of stage g is issued after PV of stage g-2).
-    if (need || cell == kF16) {
-      // the previous stage's PV signals the release of its key/value slot
-      wait(&b->wc, prev_pv_bar, prev_pv_parity, 20 + cell);
-      tc_fence_after_sync();
+  // (entry -1 was filled before the roles started, and the phase before a barrier's first counts as over)
+  wait(&b->wc, &m_full[before_at], ((g - 1) >> 3) & 1, 9);
+  const float2 before = b->rec[before_at][row];
+  const float m_new = fmaxf(before.x, mx * scale);
+  w.d = before.y * w.alpha + w.sum;
+  b->rec[at][row] = make_float2(m_new, w.d);
+  __syncwarp();
+  mbar_arrive_if(&m_full[at], lead);
+  w.alpha = ex2(before.x - m_new);
+  if (kPairs) w.sum = 0.0f;
+  if (active) {
+    // exponent = s * scale + bias; the NVFP4 cell produces 6 P directly (e2m1 input range),
+    // the INT8 cell P * 2^8.807 (e4m3 input range); the sums are scaled back.
+    const float bias = (cell == kI8 ? kFp8Offset : (cell == kNv ? 2.5849625007f : 0.0f)) - m_new;
+    const float sum_scale = cell == kI8 ? 0.0022326917f : (cell == kNv ? 0.16666667f : 1.0f);
+    float sum;
+    if (cell == kI8) {
+      sum = exp_store<kI8>(s, scale, bias, p_row);
+    } else if (cell == kNv) {
+      sum = exp_store<kNv>(s, scale, bias, p_row);
+    } else {
+      sum = exp_store<kF16>(s, scale, bias, p_row);
     }
-    if (need) {
-      if (phase_first) {
-        rescale_o<D, true>(tmem_row, alpha, colf);
-      } else {
-        rescale_o<D, false>(tmem_row, alpha, nullptr);
-      }
-    }
-  }
-  uint8_t* p_tile = p_smem + p_buffer(cell, g) * p_tile_bytes(cell);
-  if (cell == kNv) {
-    write_p<kNv>(p_tile, row, s);
-  } else if (cell == kI8) {
-    write_p<kI8>(p_tile, row, s);
-  } else {
-    write_p<kF16>(p_tile, row, s);
+    w.sum = sum * sum_scale;
+  } else if (live_warp) {
+    const int chunks = p_bytes(cell) / 2048;
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) *reinterpret_cast<uint4*>(p_row + c * 128) = make_uint4(0, 0, 0, 0);
   }
   fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncwarp();
-  if (lead) mbar_arrive(&b->p_full[g & 1]);
+  mbar_arrive_if(&b->p_full[at], lead);
 }
 
 // ------------------------------------------------------------------------------------------
 // MMA side
 // ------------------------------------------------------------------------------------------
-template <int D>
-__device__ __forceinline__ void issue_qk(int cell, uint32_t tmem_s, uint32_t tmem, uint32_t q_addr,
-                                         uint32_t k_addr, uint32_t kv_slot_addr, uint32_t issue) {
-  if (cell == kF16) {
+template <int D, int CELL>
+__device__ __forceinline__ void issue_qk(uint32_t tmem_s, uint32_t tmem, uint32_t q_addr,
+                                         uint32_t slot_addr) {
+  if (CELL == kF16) {
     constexpr uint32_t chunks = D / 8;
-    const uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, 64, 0, 0);
+    constexpr uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, 64, 0, 0);
+    const uint64_t qd = smem_desc(q_addr, 128, chunks * 128), kd = smem_desc(slot_addr, 128, chunks * 128);
 #pragma unroll
-    for (int k = 0; k < D / 16; ++k)
-      mma_f16_ss(tmem_s, smem_desc(q_addr + k * 256, 128, chunks * 128),
-                 smem_desc(k_addr + k * 256, 128, chunks * 128), idesc, k > 0, issue);
-  } else if (cell == kI8) {
+    for (int k = 0; k < D / 16; ++k) mma_f16_ss(tmem_s, qd + k * 16, kd + k * 16, idesc, k > 0);
+  } else if (CELL == kI8) {
     constexpr uint32_t chunks = D / 16;
-    const uint32_t idesc = instr_desc(kFmtS8, kFmtS8, kAccS32, 128, 64, 0, 0);
+    constexpr uint32_t idesc = instr_desc(kFmtS8, kFmtS8, kAccS32, 128, 64, 0, 0);
+    const uint64_t qd = smem_desc(q_addr, 128, chunks * 128), kd = smem_desc(slot_addr, 128, chunks * 128);
 #pragma unroll
-    for (int k = 0; k < D / 32; ++k)
-      mma_i8_ss(tmem_s, smem_desc(q_addr + k * 256, 128, chunks * 128),
-                smem_desc(k_addr + k * 256, 128, chunks * 128), idesc, k > 0, issue);
+    for (int k = 0; k < D / 32; ++k) mma_i8_ss(tmem_s, qd + k * 16, kd + k * 16, idesc, k > 0);
   } else {
     constexpr uint32_t chunks = D / 32;
-    const uint32_t idesc = instr_desc_nvf4(128, 64);
-    const uint32_t ksf = kv_slot_addr + rec::kv_nvfp4_ksf_offset(D);
+    constexpr uint32_t idesc = instr_desc_nvf4(128, 64);
+    const uint64_t qd = smem_desc(q_addr, 128, chunks * 128), kd = smem_desc(slot_addr, 128, chunks * 128);
+    const uint64_t sd = smem_desc(slot_addr + rest_offset(D, CELL) + 32 * D, 128, 128);
+#pragma unroll
+    for (int k = 0; k < D / 64; ++k) tmem_cp_32x128b_warpx4(tmem + kColSfbK + 4 * k, sd + k * 32);
 #pragma unroll
     for (int k = 0; k < D / 64; ++k)
-      tmem_cp_32x128b_warpx4(tmem + kColSfbK + 4 * k, smem_desc(ksf + 512 * k, 128, 128), issue);
-#pragma unroll
-    for (int k = 0; k < D / 64; ++k)
-      mma_nvf4_ss(tmem_s, smem_desc(q_addr + k * 256, 128, chunks * 128),
-                  smem_desc(k_addr + k * 256, 128, chunks * 128), idesc, k > 0,
-                  tmem + kColSfaQ + 4 * k, tmem + kColSfbK + 4 * k, issue);
+      mma_nvf4_ss(tmem_s, qd + k * 16, kd + k * 16, idesc, k > 0, tmem + kColSfaQ + 4 * k,
+                  tmem + kColSfbK + 4 * k);
   }
 }
 
-template <int D>
-__device__ __forceinline__ void issue_pv(int cell, uint32_t tmem, uint32_t p_addr,
-                                         uint32_t kv_slot_addr, uint32_t accumulate,
-                                         uint32_t issue) {
-  if (cell == kF16) {
-    const uint32_t v_addr = kv_slot_addr + 64 * D * 2;
-    const uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, D, 0, 1);
+template <int D, int CELL>
+__device__ __forceinline__ void issue_pv(uint32_t tmem, uint32_t slot_addr, uint32_t v_addr, uint32_t accumulate) {
+  if (CELL == kF16) {
+    constexpr uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, D, 0, 1);
     constexpr uint32_t v_lbo = (D / 8) * 128;  // between 8-key groups
+    const uint64_t pd = smem_desc(slot_addr, 128, 8 * 128), vd = smem_desc(v_addr, v_lbo, 128);
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      mma_f16_ss(tmem + kColO, smem_desc(p_addr + k * 256, 128, 8 * 128),
-                 smem_desc(v_addr + k * 2 * v_lbo, v_lbo, 128), idesc, accumulate | (k > 0), issue);
-  } else if (cell == kI8) {
-    const uint32_t v_addr = kv_slot_addr + 64 * D;
-    const uint32_t idesc = instr_desc(kFmtE4M3, kFmtE4M3, kAccF32, 128, D, 0, 0);
+      mma_f16_ss(tmem + kColO, pd + k * 16, vd + k * (2 * v_lbo / 16), idesc, k > 0 ? 1u : accumulate);
+  } else if (CELL == kI8) {
+    constexpr uint32_t idesc = instr_desc(kFmtE4M3, kFmtE4M3, kAccF32, 128, D, 0, 0);
+    const uint64_t pd = smem_desc(slot_addr, 128, 4 * 128), vd = smem_desc(v_addr, 128, 4 * 128);
 #pragma unroll
     for (int k = 0; k < 2; ++k)
-      mma_f8_ss(tmem + kColO, smem_desc(p_addr + k * 256, 128, 4 * 128),
-                smem_desc(v_addr + k * 256, 128, 4 * 128), idesc, accumulate | (k > 0), issue);
+      mma_f8_ss(tmem + kColO, pd + k * 16, vd + k * 16, idesc, k > 0 ? 1u : accumulate);
   } else {
-    const uint32_t v_addr = kv_slot_addr + rec::kv_nvfp4_v_offset(D);
-    const uint32_t vsf = kv_slot_addr + rec::kv_nvfp4_vsf_offset(D);
-    const uint32_t idesc = instr_desc_nvf4(128, D);
-    tmem_cp_32x128b_warpx4(tmem + kColSfbV, smem_desc(vsf, 128, 128), issue);
-    mma_nvf4_ss(tmem + kColO, smem_desc(p_addr, 128, 2 * 128), smem_desc(v_addr, 128, 2 * 128),
-                idesc, accumulate, tmem + kColSfaP, tmem + kColSfbV, issue);
+    constexpr uint32_t idesc = instr_desc_nvf4(128, D);
+    tmem_cp_32x128b_warpx4(tmem + kColSfbV, smem_desc(v_addr + 32 * D + (D / 64) * 512, 128, 128));
+    mma_nvf4_ss(tmem + kColO, smem_desc(slot_addr, 128, 2 * 128), smem_desc(v_addr, 128, 2 * 128), idesc,
+                accumulate, tmem + kColSfaP, tmem + kColSfbV);
   }
 }
 
 // ------------------------------------------------------------------------------------------
 // kernel
 // ------------------------------------------------------------------------------------------
-template <int D>
+// CELLS: the one cell of every stage, or kAny.  A kernel of one cell has that cell's code only and
+// its sizes as constants; in the mixed kernel the cell is a run-time value and one copy of the
+// stage code serves all: the CTAs of an SM are in different phases, and hot code that outgrows the
+// instruction cache costs more than the constants give (three whole copies of the softmax stage,
+// 100 KB of code: 1.48 us per 64-key stage and SM at D = 64 instead of 1.11).
+template <int D, int CELLS, bool kQ64>
 __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
-  const int QB = p.s.query_block;
+  constexpr int kFirst = CELLS == kAny ? 0 : CELLS, kLast = CELLS == kAny ? 2 : CELLS;
+  constexpr int QB = kQ64 ? 64 : 128;
   const int head = blockIdx.y;
   // launch order of the head's query blocks (longest list first) as written by the routing
   // stage; 0 = no order given
   int tile = blockIdx.x;
-  const bool pairs = p.pair_counts != nullptr;
+  const bool pairs = kQ64 && p.pair_counts != nullptr;
   const int pair_tiles = (p.s.video_blocks + 1) / 2;
   if (!p.dense_prefix) {
     const int ordered =
@@ -498,72 +515,63 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   const int block0 = pairs ? 2 * tile : tile;
 
   // ---- this tile's work list ----
-  int cnt[3];
-  int first_of[3] = {0, 0, 0};  // where each phase starts inside the list
-  const int32_t* list;
-  if (p.dense_prefix) {
-    cnt[0] = 0;
-    cnt[1] = p.stages;
-    cnt[2] = 0;
-    list = nullptr;
-  } else if (pairs) {
-    const int32_t* pc = p.pair_counts + ((int64_t)head * pair_tiles + tile) * 4;
-    cnt[0] = pc[0];
-    cnt[1] = pc[1];
-    cnt[2] = pc[2];
-    // phase c of the union sits where the two blocks' phases before it would end
+  int cnt[3] = {0, p.stages, 0};
+  const int32_t* list = nullptr;
+  if (!p.dense_prefix) {
     const int32_t* ra = p.row_counts + ((int64_t)head * p.s.video_blocks + block0) * 4;
-    int before = 0;
-    for (int c = 0; c < 3; ++c) {
-      first_of[c] = before;
-      before += ra[c] + (tile_blocks == 2 ? ra[4 + c] : 0);
-    }
-    list = p.pair_ids + (int64_t)head * p.capacity +
+    const int32_t* counts = pairs ? p.pair_counts + ((int64_t)head * pair_tiles + tile) * 4 : ra;
+    for (int c = 0; c < 3; ++c) cnt[c] = counts[c];
+    list = (pairs ? p.pair_ids : p.stage_ids) + (int64_t)head * p.capacity +
            p.row_offset[(int64_t)head * p.s.video_blocks + block0];
-  } else {
-    const int32_t* rc = p.row_counts + ((int64_t)head * p.s.video_blocks + tile) * 4;
-    cnt[0] = rc[0];
-    cnt[1] = rc[1];
-    cnt[2] = rc[2];
-    list = p.stage_ids + (int64_t)head * p.capacity +
-           p.row_offset[(int64_t)head * p.s.video_blocks + tile];
-    first_of[1] = cnt[0];
-    first_of[2] = cnt[0] + cnt[1];
   }
-  const int total = cnt[0] + cnt[1] + cnt[2];
-  if (total == 0) return;
+  if (cnt[0] + cnt[1] + cnt[2] == 0) return;
   // After a give-up anywhere on this device the status word stays set: later CTAs (of this and
   // of later launches, until the host clears the word) return at once instead of each running
   // into its own wait limit.
   if (*reinterpret_cast<volatile int32_t*>(p.status) != 0) return;
 
   uint8_t* q_smem = smem;
-  uint8_t* p_smem = smem + p.q_region;
-  uint8_t* slots = p_smem + p.p_region;
-  float* colf = reinterpret_cast<float*>(slots + (size_t)p.ring_bytes);
-  Barriers* b = reinterpret_cast<Barriers*>(colf + D);
+  uint8_t* ring = smem + p.q_region;
+  float* colf = reinterpret_cast<float*>(ring + (size_t)p.ring_bytes);
+  Shared* b = reinterpret_cast<Shared*>(colf + D);
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kMaxSlots; ++i) {
-      mbar_init(&b->kv_full[i], 1);
-      mbar_init(&b->kv_free[i], 1);
+  if (warp == 0) {
+    if (lane < kRing) {
+      mbar_init(&b->kv_full[lane], 1);
+      mbar_init(&b->pv_done[lane], 1);
+      mbar_init(&b->p_full[lane], 8);
     }
-    mbar_init(&b->q_full, 1);
-    mbar_init(&b->q_free, 1);
-    mbar_init(&b->s_full[0], 1);
-    mbar_init(&b->s_full[1], 1);
-    mbar_init(&b->s_free, kSoftmaxThreads / 32);
-    mbar_init(&b->p_full[0], kSoftmaxThreads / 32);
-    mbar_init(&b->p_full[1], kSoftmaxThreads / 32);
-    mbar_init(&b->all_done, 1);
-    b->wc.abort = 0;
-    b->wc.status = p.status;
-    b->wc.limit_ns = p.wait_ns;
+    mbar_init(&b->m_full[0][lane], 1);  // all four quadrants' rings
+    if (lane == 0) {
+      mbar_init(&b->v_full, 1);
+      mbar_init(&b->q_full, 1);
+      mbar_init(&b->q_free, 1);
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&b->s_full[i], 1);
+        mbar_init(&b->s_free[i], 4);
+      }
+      mbar_init(&b->nv_done, 1);
+      mbar_init(&b->all_done, 1);
+      mbar_init(&b->qk_done, 1);
+      b->wc.abort = 0;
+      b->wc.status = p.status;
+      b->wc.limit_ns = p.wait_ns;
+      // phase c of a pair's union sits where the two blocks' phases before it would end
+      const int32_t* ra = pairs ? p.row_counts + ((int64_t)head * p.s.video_blocks + block0) * 4 : nullptr;
+      int before = 0;
+      for (int c = 0; c < 3; ++c) {
+        b->cnt[c] = cnt[c];
+        b->first_of[c] = before;
+        before += pairs ? ra[c] + (tile_blocks == 2 ? ra[4 + c] : 0) : cnt[c];
+      }
+    }
     mbar_init_fence();
+  } else if (warp < 5) {
+    b->rec[kRing - 1][threadIdx.x - 32] = make_float2(-5.0e6f, 0.0f);  // before the first stage
   }
   // Query rows beyond QB (64-row tiles padded to the 128-row MMA shape) are never
   // initialised: rows are independent, their results stay in TMEM lanes nobody reads.
-  if (warp == kMmaWarp) {
+  if (warp == kPvWarp) {
     tmem_alloc(&b->tmem_base, kTmemCols);
     tmem_relinquish();
   }
@@ -572,260 +580,365 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   tc_fence_after_sync();
   const uint32_t tmem = b->tmem_base;
 
-  const int q_index_fp = head * p.s.video_blocks + block0;  // q_fp16 / q_nvfp4 record
-  const int64_t q_index_i8 =
-      (int64_t)head * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks + tile : block0);
-  const float sigma = (D == 64 ? 0.125f : 0.08838834764831845f) * 1.4426950408889634f;
+  const float* vscale = p.o.v_e4m3_scale ? p.o.v_e4m3_scale + (int64_t)head * D : nullptr;
+  const float nv_dom = p.s.v_global_scale * (1.0f / (6.0f * 448.0f));
 
-  // The second warpgroup (loader, MMA and two idle warps) hands most of its registers to the
-  // softmax warpgroup.  All four warps of a warpgroup execute the same setmaxnreg instruction,
-  // and each sits at the top of the branch whose code runs under the new register count.
+  // Register counts move between the warpgroups; all four warps of a warpgroup execute the same
+  // setmaxnreg instruction, and each sits at the top of the branch that runs under the new count.
   if (warp >= kLoaderWarp) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
-  if (warp == kLoaderWarp) {
-    // =============================== loader ===============================
-    // The whole warp walks the list with uniform control flow; one lane issues.
-    const uint32_t lead = lane == 0;
-    int phase_ord = 0;
-    uint32_t filled = 0, fillpar = 0;  // per slot: ever filled / parity of the fill count
-    for (int cell = 0; cell < 3; ++cell) {
-      if (cnt[cell] == 0) continue;
-      if (phase_ord > 0) wait<kPark>(&b->wc, &b->q_free, (phase_ord - 1) & 1, 1);
-      const int qbytes = CellInfo<D>::q_bytes(cell, QB);
-      const uint8_t* qsrc =
-          cell == kNv ? static_cast<const uint8_t*>(p.o.q_nvfp4) + (int64_t)q_index_fp * qbytes
-          : cell == kI8 ? static_cast<const uint8_t*>(p.o.q_int8) + q_index_i8 * qbytes
-                        : static_cast<const uint8_t*>(p.o.q_fp16) + (int64_t)q_index_fp * qbytes;
-      mbar_arrive_expect_tx(&b->q_full, qbytes * tile_blocks, lead);
-      if (cell == kNv && QB == 64) {
-        // codes fill the first half of the 128-row tile; scale blocks follow the full tile.
-        // A pair's second record: codes into the second half of the tile, scale blocks behind
-        // the first record's (the MMA warp folds them into one block before it copies them).
-        const int codes = QB * D / 2;
-        bulk_g2s(q_smem, qsrc, codes, &b->q_full, lead);
-        bulk_g2s(q_smem + 128 * D / 2, qsrc + codes, qbytes - codes, &b->q_full, lead);
-        if (tile_blocks == 2) {
-          bulk_g2s(q_smem + codes, qsrc + qbytes, codes, &b->q_full, lead);
-          bulk_g2s(q_smem + 128 * D / 2 + (qbytes - codes), qsrc + qbytes + codes, qbytes - codes,
-                   &b->q_full, lead);
-        }
-      } else {
-        // records of consecutive query blocks follow one another: two make a 128-row tile
-        bulk_g2s(q_smem, qsrc, qbytes * tile_blocks, &b->q_full, lead);
-      }
-      const int kvbytes = CellInfo<D>::kv_bytes(cell);
-      const uint8_t* kvbase =
-          (cell == kNv ? static_cast<const uint8_t*>(p.o.kv_nvfp4)
-           : cell == kI8 ? static_cast<const uint8_t*>(p.o.kv_int8)
-                         : static_cast<const uint8_t*>(p.o.kv_fp16)) +
-          (int64_t)head * p.stages * kvbytes;
-      const int first = first_of[cell];
-      // The ring is cut into equal slots of this phase's record size; slots of the
-      // previous phase must all be released before the new geometry is written.
-      const int slot_bytes = (kvbytes + 127) & ~127;
-      const int nslot = min(kMaxSlots, p.ring_bytes / slot_bytes);
-      for (int sl = 0; sl < kMaxSlots; ++sl)
-        if ((filled >> sl) & 1u)
-          wait<kPark>(&b->wc, &b->kv_free[sl], ((fillpar >> sl) & 1u) ^ 1u, 2);
-      int stage_l = 0;  // list entries, 32 at a time, one per lane
-      int slot = -1;
-      for (int i = 0; i < cnt[cell]; ++i) {
-        if ((i & 31) == 0 && list != nullptr && i + lane < cnt[cell])
-          stage_l = list[first + i + lane];
-        const int stage = list ? (__shfl_sync(0xffffffffu, stage_l, i & 31) & 0x3fffffff) : i;
-        slot = slot + 1 == nslot ? 0 : slot + 1;
-        if ((filled >> slot) & 1u)
-          wait<kPark>(&b->wc, &b->kv_free[slot], ((fillpar >> slot) & 1u) ^ 1u, 2);
-        mbar_arrive_expect_tx(&b->kv_full[slot], kvbytes, lead);
-        bulk_g2s(slots + (size_t)slot * slot_bytes, kvbase + (int64_t)stage * kvbytes, kvbytes,
-                 &b->kv_full[slot], lead);
-        filled |= 1u << slot;
-        fillpar ^= 1u << slot;
-      }
-      ++phase_ord;
-    }
-  } else if (warp == kMmaWarp) {
-    // =============================== MMA issue ===============================
-    // Uniform control flow for the whole warp (descriptors stay warp-uniform values);
-    // only the tcgen05 instructions themselves are predicated on one lane.
-    const uint32_t lead = lane == 0;
-    int g = 0, phase_ord = 0;
-    uint32_t usepar = 0;  // per slot: parity of the number of fills consumed
-    const uint32_t q_addr = smem_u32(q_smem), p_addr = smem_u32(p_smem);
-    for (int cell = 0; cell < 3; ++cell) {
-      if (cnt[cell] == 0) continue;
-      wait<kPark>(&b->wc, &b->q_full, phase_ord & 1, 3);
-      tc_fence_after_sync();
-      if (cell == kNv) {
-        if (tile_blocks == 2) {
-          // Scale bytes of rows 0-63 sit in the low eight bytes of every 16-byte chunk, those of
-          // rows 64-127 in the high eight.  Both records hold their 64 rows in the low halves:
-          // the second record's move up into the first record's empty high halves.
-          uint8_t* sfa = q_smem + 128 * D / 2;
-          const uint8_t* sfb = sfa + (D / 64) * 512;
-          for (int c = lane; c < (D / 64) * 32; c += 32) {
-            const uint2 lo = *reinterpret_cast<const uint2*>(sfb + c * 16);
-            *reinterpret_cast<uint2*>(sfa + c * 16 + 8) = lo;
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+    if (warp == kLoaderWarp) {
+      // =============================== loader ===============================
+      // The whole warp walks the list with uniform control flow; one lane issues.
+      const uint32_t lead = lane == 0;
+      const int q_index_fp = head * p.s.video_blocks + block0;  // q_fp16 / q_nvfp4 record
+      const int64_t q_index_i8 =
+          (int64_t)head * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks + tile : block0);
+      const float sigma = (D == 64 ? 0.125f : 0.08838834764831845f) * 1.4426950408889634f;
+      int phase_ord = 0, g = 0, v_fills = 0;
+#pragma unroll 1
+      for (int cell = kFirst; cell <= kLast; ++cell) {
+        const int n = b->cnt[cell];
+        if (n == 0) continue;
+        if (phase_ord > 0) wait<kMmaRole>(&b->wc, &b->q_free, (phase_ord - 1) & 1, 1);
+        const int qbytes = cell == kNv ? (int)rec::q_nvfp4_bytes(QB, D)
+                                       : (cell == kI8 ? (int)rec::q_int8_bytes(QB, D) : (int)rec::q_fp16_bytes(QB, D));
+        const uint8_t* qsrc =
+            cell == kNv ? static_cast<const uint8_t*>(p.o.q_nvfp4) + (int64_t)q_index_fp * qbytes
+            : cell == kI8 ? static_cast<const uint8_t*>(p.o.q_int8) + q_index_i8 * qbytes
+                          : static_cast<const uint8_t*>(p.o.q_fp16) + (int64_t)q_index_fp * qbytes;
+        mbar_arrive_expect_tx(&b->q_full, qbytes * tile_blocks, lead);
+        if (cell == kNv && kQ64) {
+          // codes fill the first half of the 128-row tile; scale blocks follow the full tile.
+          // A pair's second record: codes into the second half of the tile, scale blocks behind
+          // the first record's (the QK warp folds them into one block before it copies them).
+          const int codes = QB * D / 2;
+          bulk_g2s(q_smem, qsrc, codes, &b->q_full, lead);
+          bulk_g2s(q_smem + 128 * D / 2, qsrc + codes, qbytes - codes, &b->q_full, lead);
+          if (tile_blocks == 2) {
+            bulk_g2s(q_smem + codes, qsrc + qbytes, codes, &b->q_full, lead);
+            bulk_g2s(q_smem + 128 * D / 2 + (qbytes - codes), qsrc + qbytes + codes, qbytes - codes,
+                     &b->q_full, lead);
           }
-          fence_proxy_async_smem();
+        } else {
+          // records of consecutive query blocks follow one another: two make a 128-row tile
+          bulk_g2s(q_smem, qsrc, qbytes * tile_blocks, &b->q_full, lead);
+        }
+        const int kvbytes = record_bytes(D, cell), kbytes = k_bytes(D, cell), rest = rest_offset(D, cell);
+        const uint8_t* kvbase =
+            (cell == kNv ? static_cast<const uint8_t*>(p.o.kv_nvfp4)
+             : cell == kI8 ? static_cast<const uint8_t*>(p.o.kv_int8)
+                           : static_cast<const uint8_t*>(p.o.kv_fp16)) +
+            (int64_t)head * p.stages * kvbytes;
+        const int first = b->first_of[cell];
+        // The ring is cut into equal slots of this phase's size; the slots of the previous phase
+        // must all be released before the new geometry is written (PVs complete in stage order).
+        const int slot_size = stage_bytes(D, cell);
+        const int nslot = slot_count(p.ring_bytes, D, cell);
+        if (g > 0) wait<kMmaRole>(&b->wc, &b->pv_done[(g - 1) & (kRing - 1)], ((g - 1) >> 3) & 1, 2);
+        float q_scale[2] = {1.0f, 1.0f};
+        const float* kscale = nullptr;
+        if (cell == kI8) {
+          q_scale[0] = p.o.q_int8_scale[q_index_i8];
+          if (tile_blocks == 2) q_scale[1] = p.o.q_int8_scale[q_index_i8 + 1];
+          kscale = p.o.k_int8_scale + (int64_t)head * p.stages;
+        }
+        const float base = cell == kNv ? sigma * p.s.q_global_scale * p.s.k_global_scale : sigma;
+        const bool split = split_kv(D, cell);
+        // list entries, 32 at a time, one per lane, with their metadata
+        int stage_l = 0, v_stage = 0;
+        float2 meta_l[2] = {make_float2(base, 0.0f), make_float2(base, 0.0f)};
+        int slot = 0;
+        // Split phases: with one value buffer, the values of stage i - nslot + 1 may follow when PV of
+        // stage i - nslot is complete, which is also what the key tile of stage i waits for.
+        const int end = split ? n + nslot - 1 : n;
+#pragma unroll 1
+        for (int i = 0; i < end; ++i) {
+          if ((i & 31) == 0 && i < n) {
+            const int at = i + lane;
+            int entry = 0;
+            if (at < n) entry = list != nullptr ? list[first + at] : at;
+            stage_l = entry & 0x3fffffff;
+            const int valid = p.valid_k[stage_l];
+            meta_l[0].y = __int_as_float(!pairs || ((entry >> 30) & 1) ? valid : -1);
+            if (kQ64) meta_l[1].y = __int_as_float(entry < 0 ? valid : -1);
+            if (cell == kI8) {
+              const float ks = kscale[stage_l];
+              meta_l[0].x = sigma * (q_scale[0] * ks);
+              if (kQ64) meta_l[1].x = sigma * (q_scale[1] * ks);
+            }
+          }
+          const int stage = __shfl_sync(0xffffffffu, stage_l, i & 31);
+          const int gi = g + i;
+          if (i >= nslot)
+            wait<kMmaRole>(&b->wc, &b->pv_done[(gi - nslot) & (kRing - 1)], ((gi - nslot) >> 3) & 1, 2);
+          if (split) {
+            const int vi = i - nslot + 1;
+            if (vi >= 0) {
+              mbar_arrive_expect_tx(&b->v_full, kvbytes - kbytes, lead);
+              bulk_g2s(ring + nslot * slot_size, kvbase + (int64_t)v_stage * kvbytes + kbytes, kvbytes - kbytes,
+                       &b->v_full, lead);
+              ++v_fills;
+            }
+            // the stage whose values come next
+            if (vi + 1 >= 0 && vi + 1 < n) v_stage = list != nullptr ? list[first + vi + 1] & 0x3fffffff : vi + 1;
+          }
+          if (i < n) {
+            const int at = gi & (kRing - 1);
+            if (lane == (i & 31)) {
+              b->meta[at][0] = meta_l[0];
+              if (kQ64) b->meta[at][1] = meta_l[1];
+            }
+            __syncwarp();
+            const int bytes = split ? kbytes : kvbytes;
+            const uint8_t* src = kvbase + (int64_t)stage * kvbytes;
+            uint8_t* dst = ring + (size_t)slot * slot_size;
+            mbar_arrive_expect_tx(&b->kv_full[at], bytes, lead);
+            if (split || rest == kbytes) {
+              bulk_g2s(dst, src, bytes, &b->kv_full[at], lead);
+            } else {
+              bulk_g2s(dst, src, kbytes, &b->kv_full[at], lead);
+              bulk_g2s(dst + rest, src + kbytes, kvbytes - kbytes, &b->kv_full[at], lead);
+            }
+            slot = slot + 1 == nslot ? 0 : slot + 1;
+          }
+        }
+        g += n;
+        ++phase_ord;
+      }
+      if (b->wc.abort) {
+        // unwinding: the copies in flight must land before the CTA gives its shared memory back
+        for (int k = max(0, g - kRing); k < g; ++k)
+          drain_wait(&b->kv_full[k & (kRing - 1)], (k >> 3) & 1, kDrainNs);
+        if (v_fills > 0) drain_wait(&b->v_full, (v_fills - 1) & 1, kDrainNs);
+        if (phase_ord > 0) drain_wait(&b->q_full, (phase_ord - 1) & 1, kDrainNs);
+      }
+    } else if (warp == kQkWarp) {
+      // =============================== S = Q K^T ===============================
+      // Uniform control flow for the whole warp; the tcgen05 instructions sit in elect.sync blocks.
+      int g = 0, phase_ord = 0;
+      uint32_t used = 0, free_par = 0;
+      const uint32_t q_addr = smem_u32(q_smem), ring_addr = smem_u32(ring);
+#pragma unroll 1
+      for (int cell = kFirst; cell <= kLast; ++cell) {
+        const int n = b->cnt[cell];
+        if (n == 0) continue;
+        wait<kMmaRole>(&b->wc, &b->q_full, phase_ord & 1, 3);
+        // the second score buffer takes the place of the NVFP4 phase's scale factors
+        if (CELLS == kAny && cell != kNv && b->cnt[kNv] > 0) wait<kMmaRole>(&b->wc, &b->nv_done, 0, 3);
+        tc_fence_after_sync();
+        const int nslot = slot_count(p.ring_bytes, D, cell);
+        const uint32_t stride = stage_bytes(D, cell);
+        if (cell == kNv) {
+          if (tile_blocks == 2) {
+            // Scale bytes of rows 0-63 sit in the low eight bytes of every 16-byte chunk, those of
+            // rows 64-127 in the high eight.  Both records hold their 64 rows in the low halves:
+            // the second record's move up into the first record's empty high halves.
+            uint8_t* sfa = q_smem + 128 * D / 2;
+            const uint8_t* sfb = sfa + (D / 64) * 512;
+            for (int c = lane; c < (D / 64) * 32; c += 32) {
+              const uint2 lo = *reinterpret_cast<const uint2*>(sfb + c * 16);
+              *reinterpret_cast<uint2*>(sfa + c * 16 + 8) = lo;
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+          }
+          const uint32_t qsf = q_addr + 128 * D / 2;
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < D / 64; ++k)
+              tmem_cp_32x128b_warpx4(tmem + kColSfaQ + 4 * k, smem_desc(qsf + 512 * k, 128, 128));
+          }
           __syncwarp();
         }
-        const uint32_t qsf = q_addr + 128 * D / 2;
-#pragma unroll
-        for (int k = 0; k < D / 64; ++k)
-          tmem_cp_32x128b_warpx4(tmem + kColSfaQ + 4 * k, smem_desc(qsf + 512 * k, 128, 128),
-                                 lead);
-      }
-      const int n = cnt[cell];
-      const int slot_bytes = (CellInfo<D>::kv_bytes(cell) + 127) & ~127;
-      const int nslot = min(kMaxSlots, p.ring_bytes / slot_bytes);
-      const uint32_t ring_addr = smem_u32(slots);
-      // software pipeline: QK of stage i+1 is issued before PV of stage i
-      int qk_slot = 0, pv_slot = 0;
-      for (int i = 0; i <= n; ++i) {
-        if (i < n) {
-          const int gi = g + i;
-          const int slot = qk_slot;
-          qk_slot = qk_slot + 1 == nslot ? 0 : qk_slot + 1;
-          wait<kPark>(&b->wc, &b->kv_full[slot], (usepar >> slot) & 1u, 4);
-          usepar ^= 1u << slot;
-          const int sb = s_buffer(cell, gi);
-          // single score buffer of the NVFP4 phase (always the first phase: gi == i)
-          if (cell == kNv && i > 0) wait<kPark>(&b->wc, &b->s_free, (uint32_t)(i - 1) & 1u, 5);
+        // a stage's scores are computed as soon as its key tile has landed and its score buffer
+        // has been read
+        int slot = 0;
+#pragma unroll 1
+        for (int i = 0; i < n; ++i, ++g) {
+          const int sb = s_buffer<D>(cell, g);
+          wait<kMmaRole>(&b->wc, &b->kv_full[g & (kRing - 1)], (g >> 3) & 1, 4);
+          if ((used >> sb) & 1u) {
+            wait<kMmaRole>(&b->wc, &b->s_free[sb], (free_par >> sb) & 1u, 5);
+            free_par ^= 1u << sb;
+          }
+          used |= 1u << sb;
           tc_fence_after_sync();
-          const uint32_t slot_addr = ring_addr + slot * slot_bytes;
-          issue_qk<D>(cell, tmem + s_column(sb), tmem, q_addr, slot_addr, slot_addr, lead);
-          mma_commit(&b->s_full[sb], lead);
-          if (i == n - 1) mma_commit(&b->q_free, lead);
+          if (elect_one()) {
+            const uint32_t tmem_s = tmem + (sb ? Cols<D>::kS1 : kColS), slot_addr = ring_addr + slot * stride;
+            if (cell == kI8) {
+              issue_qk<D, kI8>(tmem_s, tmem, q_addr, slot_addr);
+            } else if (cell == kNv) {
+              issue_qk<D, kNv>(tmem_s, tmem, q_addr, slot_addr);
+            } else {
+              issue_qk<D, kF16>(tmem_s, tmem, q_addr, slot_addr);
+            }
+            mma_commit(&b->s_full[g & 1]);
+            if (i == n - 1) mma_commit(&b->q_free);
+          }
+          __syncwarp();
+          slot = slot + 1 == nslot ? 0 : slot + 1;
         }
-        if (i > 0) {
-          const int gj = g + i - 1;
-          const int slot = pv_slot;
-          pv_slot = pv_slot + 1 == nslot ? 0 : pv_slot + 1;
-          wait<kPark>(&b->wc, &b->p_full[gj & 1], (gj >> 1) & 1, 6);
+        ++phase_ord;
+      }
+      if (b->wc.abort) {
+        if (elect_one()) mma_commit(&b->qk_done);
+        __syncwarp();
+        drain_wait(&b->qk_done, 0, kDrainNs);
+      }
+    } else if (warp == kPvWarp) {
+      // =============================== O += P V ===============================
+      int g = 0;
+      const uint32_t ring_addr = smem_u32(ring);
+#pragma unroll 1
+      for (int cell = kFirst; cell <= kLast; ++cell) {
+        const int n = b->cnt[cell];
+        if (n == 0) continue;
+        const int nslot = slot_count(p.ring_bytes, D, cell);
+        const uint32_t stride = stage_bytes(D, cell);
+        const bool split = split_kv(D, cell);
+        int slot = 0;
+#pragma unroll 1
+        for (int i = 0; i < n; ++i, ++g) {
+          if (split) wait<kMmaRole>(&b->wc, &b->v_full, i & 1, 6);  // (a tile has at most one such phase)
+          wait<kMmaRole>(&b->wc, &b->p_full[g & (kRing - 1)], (g >> 3) & 1, 6);
           tc_fence_after_sync();
-          const uint32_t slot_addr = ring_addr + slot * slot_bytes;
-          issue_pv<D>(cell, tmem, p_addr + p_buffer(cell, gj) * p_tile_bytes(cell), slot_addr,
-                      gj > 0, lead);
-          mma_commit(&b->kv_free[slot], lead);  // also tells the softmax warps this PV is done
+          if (elect_one()) {
+            const uint32_t slot_addr = ring_addr + slot * stride;
+            const uint32_t v_addr = split ? ring_addr + nslot * stride : slot_addr + rest_offset(D, cell);
+            if (cell == kI8) {
+              issue_pv<D, kI8>(tmem, slot_addr, v_addr, g > 0);
+            } else if (cell == kNv) {
+              issue_pv<D, kNv>(tmem, slot_addr, v_addr, g > 0);
+            } else {
+              issue_pv<D, kF16>(tmem, slot_addr, v_addr, g > 0);
+            }
+            mma_commit(&b->pv_done[g & (kRing - 1)]);
+            if (CELLS == kAny && cell == kNv && i == n - 1) mma_commit(&b->nv_done);
+          }
+          __syncwarp();
+          slot = slot + 1 == nslot ? 0 : slot + 1;
         }
       }
-      g += n;
-      ++phase_ord;
+      if (elect_one()) mma_commit(&b->all_done);
+      __syncwarp();
+      // unwinding: the MMAs in flight must be over before tensor memory is given back
+      if (b->wc.abort) drain_wait(&b->all_done, 0, kDrainNs);
     }
-    // The end of the tile is signalled on a barrier of its own.
-    mma_commit(&b->all_done, lead);
-  }
-  } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
-    // =============================== softmax rows ===============================
-    const int row = warp * 32 + lane;            // query row == TMEM lane
-    const uint32_t tmem_row = tmem + ((uint32_t)(warp * 32) << 16);
-    RowState st{-5.0e6f, 0.0f};
-    int s_use0 = 0, s_use1 = 0;  // stages consumed from each score buffer so far
-    uint32_t pvpar = 0;         // per slot: parity of the number of PVs that used it
-    int prev_slot = 0;
-    uint32_t prev_slot_parity = 0;
-    int g = 0;
-    int prev_cell = -1;
-    const float nv_dom = p.s.v_global_scale * (1.0f / (6.0f * 448.0f));
-    const float* vscale = p.o.v_e4m3_scale ? p.o.v_e4m3_scale + (int64_t)head * D : nullptr;
-    const bool live_warp = warp * 32 < QB * tile_blocks;
-    const int my_block = warp * 32 >= QB && tile_blocks == 2 ? 1 : 0;  // which block of a pair
-    if (cnt[kNv] > 0) {
-      tmem_st4(tmem_row + kColSfaP, 0x7e7e7e7eu);  // constant 448 block scale of P
-      tmem_wait_st();
-    }
-    for (int cell = 0; cell < 3; ++cell) {
-      if (cnt[cell] == 0) continue;
-      if (prev_cell >= 0) {
+  } else if (warp >= kCorrWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kCorrRegs));
+    // =============================== O rescale ===============================
+    const int row = (warp - kCorrWarp) * 32 + lane;
+    uint64_t* m_full = b->m_full[warp - kCorrWarp];
+    const uint32_t tmem_row = tmem + ((uint32_t)((warp - kCorrWarp) * 32) << 16);
+    const uint32_t lead = lane == 0;
+    float m = -5.0e6f;
+    int g = 0, prev_cell = -1;
+#pragma unroll 1
+    for (int cell = kFirst; cell <= kLast; ++cell) {
+      const int n = b->cnt[cell];
+      if (n == 0) continue;
+      const bool change = CELLS == kAny && prev_cell >= 0;
+      if (change) {
         // per-channel factor that moves O from the previous phase's domain into this one's
         asm volatile("bar.sync 5, 128;" ::: "memory");
-        for (int c = threadIdx.x; c < D; c += kSoftmaxThreads) {
+        if (row < D) {
           const float from = prev_cell == kNv ? nv_dom
-                                              : (prev_cell == kI8 ? vscale[c] * 0.0022326917f : 1.0f);
-          const float to = cell == kI8 ? vscale[c] * 0.0022326917f : 1.0f;
-          colf[c] = to == 0.0f ? 0.0f : from / to;
+                                              : (prev_cell == kI8 ? vscale[row] * 0.0022326917f : 1.0f);
+          const float to = cell == kI8 ? vscale[row] * 0.0022326917f : 1.0f;
+          colf[row] = to == 0.0f ? 0.0f : from / to;
         }
         asm volatile("bar.sync 5, 128;" ::: "memory");
       }
-      const int first = first_of[cell];
-      const float q_scale =
-          cell == kI8 ? p.o.q_int8_scale[q_index_i8 + my_block] : 1.0f;
-      const float base_scale =
-          cell == kNv ? sigma * p.s.q_global_scale * p.s.k_global_scale : sigma;
-      // Per-stage metadata (stage id -> real keys, key scale) is fetched 32 stages at a
-      // time, one stage per lane, and handed out with shuffles: no dependent global
-      // loads sit on the per-stage critical path.
-      int meta_valid = 64;
-      int meta_member = 1;
-      float meta_scale = 1.0f;
-      const int nslot = min(kMaxSlots, p.ring_bytes / ((CellInfo<D>::kv_bytes(cell) + 127) & ~127));
-      const float* kscale = cell == kI8 ? p.o.k_int8_scale + (int64_t)head * p.stages : nullptr;
-      int slot = 0;
-      for (int i = 0; i < cnt[cell]; ++i, ++g) {
-        if ((i & 31) == 0) {
-          const int mine = i + lane;
-          if (mine < cnt[cell]) {
-            const int entry = list ? list[first + mine] : mine;
-            const int stage = entry & 0x3fffffff;
-            if (pairs) meta_member = (entry >> (30 + my_block)) & 1;
-            meta_valid = p.valid_k[stage];
-            if (cell == kI8) meta_scale = sigma * (q_scale * kscale[stage]);
-          }
+#pragma unroll 1
+      for (int i = 0; i < n; ++i, ++g) {
+        const int at = g & (kRing - 1);
+        wait<kRescaleRole>(&b->wc, &m_full[at], (g >> 3) & 1, 30);
+        const float m_new = b->rec[at][row].x;
+        const bool first = change && i == 0;
+        if (g > 0 && (first || __any_sync(0xffffffffu, m_new != m))) {
+          const float alpha = ex2(m - m_new);
+          // O may only be touched once the previous PV is complete
+          wait<kRescaleRole>(&b->wc, &b->pv_done[(g - 1) & (kRing - 1)], ((g - 1) >> 3) & 1, 20);
+          tc_fence_after_sync();
+          rescale_o<D>(tmem_row, alpha, first ? colf : nullptr);
+          tc_fence_before_sync();
         }
-        const int valid = __shfl_sync(0xffffffffu, meta_valid, i & 31);
-        const bool member = !pairs || __shfl_sync(0xffffffffu, meta_member, i & 31) != 0;
-        const bool phase_first = i == 0 && prev_cell >= 0;
-        const int sb = s_buffer(cell, g);
-        const uint32_t s_parity = (sb ? s_use1 : s_use0) & 1;
-        s_use0 += sb ? 0 : 1;
-        s_use1 += sb ? 1 : 0;
-        // barrier that the PV of the previous stage completes (its key/value slot release)
-        uint64_t* pv_bar = &b->kv_free[prev_slot];
-        const uint32_t pv_parity = prev_slot_parity;
-        prev_slot = slot;
-        prev_slot_parity = (pvpar >> slot) & 1u;
-        pvpar ^= 1u << slot;
-        slot = slot + 1 == nslot ? 0 : slot + 1;
-        const float sc =
-            cell == kI8 ? __shfl_sync(0xffffffffu, meta_scale, i & 31) : base_scale;
-        softmax_stage<D>(b, p, p_smem, colf, tmem_row, row, cell, g, phase_first, sc, valid,
-                         live_warp, member, sb, s_parity, pv_bar, pv_parity, st);
+        m = m_new;
+        __syncwarp();
+        mbar_arrive_if(&b->p_full[at], lead);
       }
       prev_cell = cell;
     }
-    // ---- epilogue: O_true / d -> fp16, packed row order ----
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+    // =============================== softmax rows ===============================
+    const int row = (warp & 3) * 32 + lane;  // query row == TMEM lane
+    const int parity = warp >> 2;            // which stages this warpgroup runs
+    const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    SoftmaxWalk w{0u, 0.0f, 1.0f, 0.0f};
+    int g = 0, last_cell = kFirst;
+    const bool live_warp = !kQ64 || (warp & 3) * 32 < QB * tile_blocks;
+    const int my_block = kQ64 && (warp & 3) * 32 >= QB && tile_blocks == 2 ? 1 : 0;  // which block of a pair
+    if (kFirst == kNv && b->cnt[kNv] > 0 && parity == 0) {
+      tmem_st4(tmem_row + kColSfaP, 0x7e7e7e7eu);  // constant 448 block scale of P
+      tmem_wait_st();
+    }
+#pragma unroll 1
+    for (int cell = kFirst; cell <= kLast; ++cell) {
+      const int n = b->cnt[cell];
+      if (n == 0) continue;
+      const int nslot = slot_count(p.ring_bytes, D, cell);
+      const int stride = stage_bytes(D, cell);
+      uint8_t* p_row = ring + rec::tile_offset(row, 0, p_bytes(cell) / 2048);
+      int slot = (g & 1) == parity ? 0 : 1;
+#pragma unroll 1
+      for (int i = slot; i < n; i += 2) {
+        softmax_stage<D, kQ64>(b, p_row + slot * stride, tmem_row, row, g + i, cell, live_warp, my_block, w);
+        slot += 2;
+        if (slot >= nslot) slot -= nslot;
+      }
+      g += n;
+      last_cell = cell;
+    }
+    // ---- epilogue: O_true / d -> fp16, packed row order; each warpgroup writes half the channels ----
     wait(&b->wc, &b->all_done, 0, 7);
+    // d(G-1) from d(G-3) and the last two stages' (alpha, sum), which the two groups hold; every
+    // other use of rec is over
+    const bool last_mine = ((g - 1) & 1) == parity;
+    if (!last_mine) b->rec[0][row] = make_float2(w.alpha, w.sum);
+    asm volatile("bar.sync 6, 256;" ::: "memory");
+    if (last_mine) {
+      const float2 other = b->rec[0][row];
+      const float d = (w.d * other.x + other.y) * w.alpha + w.sum;
+      b->rec[1][row] = make_float2(d, 0.0f);
+    }
+    asm volatile("bar.sync 6, 256;" ::: "memory");
     if (live_warp) {
       tc_fence_after_sync();
+      const float d = b->rec[1][row].x;
       // a block of a pair may have an empty list of its own: its rows are never read
-      const float inv = st.d > 0.0f ? 1.0f / st.d : 0.0f;
+      const float inv = d > 0.0f ? 1.0f / d : 0.0f;
       const bool live = row < QB * tile_blocks;
       __half* dst = p.out + ((int64_t)head * p.out_rows + (int64_t)block0 * QB + row) * D;
 #pragma unroll 1
-      for (int c0 = 0; c0 < D; c0 += 32) {
+      for (int c0 = parity * (D / 2); c0 < (parity + 1) * (D / 2); c0 += 32) {
         uint32_t r[32];
         tmem_ld32(tmem_row + kColO + c0, r);
         tmem_wait_ld();
         if (live) {
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
-            uint4 v;
-            __half2* h = reinterpret_cast<__half2*>(&v);
+            float f[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              float a = __uint_as_float(r[j + 2 * i]), c = __uint_as_float(r[j + 2 * i + 1]);
-              if (prev_cell == kNv) {
-                a *= nv_dom;
-                c *= nv_dom;
-              } else if (prev_cell == kI8) {
-                a *= vscale[c0 + j + 2 * i] * 0.0022326917f;
-                c *= vscale[c0 + j + 2 * i + 1] * 0.0022326917f;
-              }
-              h[i] = __floats2half2_rn(a * inv, c * inv);
+            for (int i = 0; i < 8; ++i) {
+              f[i] = __uint_as_float(r[j + i]);
+              if (last_cell == kNv) f[i] *= nv_dom;
+              if (last_cell == kI8) f[i] *= vscale[c0 + j + i] * 0.0022326917f;
+              f[i] *= inv;
             }
-            *reinterpret_cast<uint4*>(dst + c0 + j) = v;
+            *reinterpret_cast<uint4*>(dst + c0 + j) =
+                make_uint4(f16x2(f[0], f[1]), f16x2(f[2], f[3]), f16x2(f[4], f[5]), f16x2(f[6], f[7]));
           }
         }
       }
@@ -834,48 +947,53 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == kMmaWarp) tmem_dealloc(tmem, kTmemCols);
+  if (warp == kPvWarp) tmem_dealloc(tmem, kTmemCols);
 }
 
-template <int D>
-int launch(AttnParams& p, int tiles, cudaStream_t st) {
-  const int QB = p.s.query_block;
-  int q_region = 0, p_region = 0, slot = 0;
-  const bool nv = p.s.has_nvfp4 && !p.dense_prefix, f16 = p.s.has_fp16 && !p.dense_prefix;
-  if (nv) {
-    // a pair of Q64 blocks brings a second set of scale blocks
-    q_region = max(q_region, 128 * D / 2 + (D / 64) * 512 * (p.pair_counts ? 2 : 1));
-    p_region = max(p_region, 2 * 128 * 32);
-    slot = max(slot, (int)rec::kv_nvfp4_bytes(D));
-  }
-  if (p.s.has_int8) {
-    q_region = max(q_region, 128 * D);
-    p_region = max(p_region, 2 * 128 * 64);
-    slot = max(slot, (int)rec::kv_int8_bytes(D));
-  }
-  if (f16) {
-    q_region = max(q_region, 128 * D * 2);
-    p_region = max(p_region, 128 * 128);
-    slot = max(slot, (int)rec::kv_fp16_bytes(D));
-  }
-  (void)QB;
-  q_region = (q_region + 1023) & ~1023;
-  const int fixed = q_region + p_region + D * 4 + (int)sizeof(Barriers);
-  // two CTAs per SM: measured limit is 115,528 bytes of dynamic shared memory per CTA
-  const int budget = 115528;
-  int ring = ((budget - fixed) / 128) * 128;
-  ring = max(ring, 2 * ((slot + 127) & ~127));
-  ring = min(ring, kMaxSlots * ((slot + 127) & ~127));
-  p.ring_bytes = ring;
-  p.q_region = q_region;
-  p.p_region = p_region;
-  const size_t smem = (size_t)fixed + (size_t)ring;
-  auto kernel = attention_kernel<D>;
+template <int D, int CELLS, bool kQ64>
+int launch_kernel(const AttnParams& p, int tiles, size_t smem, cudaStream_t st) {
+  auto kernel = attention_kernel<D, CELLS, kQ64>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
   kernel<<<dim3(tiles, p.s.heads), kThreads, smem, st>>>(p);
   return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
+}
+
+template <int D, bool kQ64>
+int launch(AttnParams& p, int tiles, cudaStream_t st) {
+  int q_region = 0, slot = 0, cells = 0, one = kAny;
+  const bool use[3] = {p.s.has_nvfp4 && !p.dense_prefix, p.s.has_int8 != 0, p.s.has_fp16 && !p.dense_prefix};
+  for (int cell = 0; cell < 3; ++cell) {
+    if (!use[cell]) continue;
+    one = cells++ == 0 ? cell : kAny;
+    // a pair of Q64 blocks brings a second set of scale blocks
+    q_region = max(q_region, cell == kNv ? 128 * D / 2 + (D / 64) * 512 * (p.pair_counts ? 2 : 1)
+                                         : (cell == kI8 ? 128 * D : 256 * D));
+    slot = max(slot, slot_bytes(D, cell));
+  }
+  q_region = (q_region + 127) & ~127;
+  const int fixed = q_region + D * 4 + (int)sizeof(Shared);
+  // two CTAs per SM: measured limit is 115,528 bytes of dynamic shared memory per CTA
+  const int budget = 115528;
+  int ring = ((budget - fixed) / 128) * 128;
+  ring = max(ring, 2 * slot);
+  ring = min(ring, kRing * slot);
+  p.ring_bytes = ring;
+  p.q_region = q_region;
+  const size_t smem = (size_t)fixed + (size_t)ring;
+  switch (one) {
+    case kNv: return launch_kernel<D, kNv, kQ64>(p, tiles, smem, st);
+    case kI8: return launch_kernel<D, kI8, kQ64>(p, tiles, smem, st);
+    case kF16: return launch_kernel<D, kF16, kQ64>(p, tiles, smem, st);
+    default: return launch_kernel<D, kAny, kQ64>(p, tiles, smem, st);
+  }
+}
+
+int launch_for(AttnParams& p, int tiles, cudaStream_t st) {
+  if (p.s.query_block == 64)
+    return p.s.head_dim == 64 ? launch<64, true>(p, tiles, st) : launch<128, true>(p, tiles, st);
+  return p.s.head_dim == 64 ? launch<64, false>(p, tiles, st) : launch<128, false>(p, tiles, st);
 }
 
 int check_ops(const anemoi_sm100_shape& s, const anemoi_sm100_operands& o, bool dense_prefix) {
@@ -950,7 +1068,7 @@ int video_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operands
   p.out_rows = shape->video_blocks * shape->query_block;
   const int tiles = pair_counts ? (shape->video_blocks + 1) / 2 : shape->video_blocks;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return shape->head_dim == 64 ? launch<64>(p, tiles, st) : launch<128>(p, tiles, st);
+  return launch_for(p, tiles, st);
 }
 }  // namespace
 
@@ -996,5 +1114,5 @@ extern "C" int anemoi_sm100_prefix_attention(const anemoi_sm100_shape* shape,
   p.q_tiles_int8 = shape->video_blocks + tiles;
   p.out_rows = tiles * shape->query_block;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return shape->head_dim == 64 ? launch<64>(p, tiles, st) : launch<128>(p, tiles, st);
+  return launch_for(p, tiles, st);
 }

@@ -27,47 +27,38 @@ struct WaitContext {
   uint64_t limit_ns;
 };
 
-// Two flavours.  kSpin: tight polls (the softmax rows, whose hand-offs are on the critical path
-// and arrive within tens of cycles).  kPark: mbarrier.try_wait with a suspend-time hint parks the
-// thread in hardware until the phase completes or the hint runs out, so a role that mostly waits
-// (loader, MMA issue) takes no issue slots from the arithmetic warps of its scheduler.  Between
-// batches of polls, or parked tries, the waiter looks at the abort flag and the clock.
-enum WaitMode : int { kSpin = 0, kPark = 1 };
-constexpr uint32_t kParkNs = 2000;
-
-template <int kMode>
+// mbarrier.try_wait parks the thread in hardware until the phase completes, or for a few
+// microseconds at most (about 8,000 cycles on this GPU; a waiter wakes about 50 cycles after the
+// arrival), so a waiting warp takes no issue slots.  The suspend-time form of the instruction is
+// slower: 77-100 cycles to wake, and instructions around it.  Between parked tries the waiter looks
+// at the abort flag and the clock.
+// `kRole` only makes copies of the out-of-line part: warpgroups that run with different register
+// counts (setmaxnreg) cannot share a function.
+template <int kRole>
 __device__ __noinline__ void wait_slow(WaitContext* w, uint64_t* bar, uint32_t parity, int where) {
-  uint64_t t0 = 0;
+  const uint64_t t0 = globaltimer_ns();
   for (;;) {
-    if (kMode == kPark) {
-      if (mbar_try_wait_hint(bar, parity, kParkNs)) return;
-    } else {
-#pragma unroll 1
-      for (int k = 0; k < 256; ++k)
-        if (mbar_try_wait(bar, parity)) return;
-    }
+    if (mbar_try_wait(bar, parity)) return;
     if (w->abort) return;
-    const uint64_t now = globaltimer_ns();
-    if (t0 == 0) t0 = now;
-    if (now - t0 > w->limit_ns) break;
+    if (globaltimer_ns() - t0 > w->limit_ns) break;
   }
   w->abort = 1;
   atomicCAS(w->status, 0, where);
 }
 
-// One inline poll; the bounded loop is a shared out-of-line function (code size).
-template <int kMode = kSpin>
+// One inline try; the bounded loop is a shared out-of-line function (code size).
+template <int kRole = 0>
 __device__ __forceinline__ void wait(WaitContext* w, uint64_t* bar, uint32_t parity, int where) {
   if (mbar_try_wait(bar, parity)) return;
-  wait_slow<kMode>(w, bar, parity, where);
+  wait_slow<kRole>(w, bar, parity, where);
 }
 
 // Wait that ignores the abort flag (used while unwinding: copies and MMAs already in flight
 // must land before shared or tensor memory is given back), with a limit of its own.
-__device__ __noinline__ bool drain_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
+__device__ __forceinline__ bool drain_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
   const uint64_t t0 = globaltimer_ns();
   for (;;) {
-    if (mbar_try_wait_hint(bar, parity, kParkNs)) return true;
+    if (mbar_try_wait(bar, parity)) return true;
     if (globaltimer_ns() - t0 > limit_ns) return false;
   }
 }

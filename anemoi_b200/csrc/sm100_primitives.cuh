@@ -57,52 +57,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 
-// Non-blocking test of the phase (never parks the thread).
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-// Same test, but lets the hardware park the thread for up to `hint_ns` before it reports
-// "not yet": fewer issue slots spent by threads that only wait (loader and MMA lanes).
-__device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parity,
-                                                   uint32_t hint_ns) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(hint_ns)
-      : "memory");
-  return done != 0;
-}
-
-// Every wait in this library is bounded: after `kSpinLimit` failed polls the
-// waiter records where it gave up in `*error_flag` (global memory) and returns
-// false, and the caller unwinds (frees TMEM, returns). The host reads the flag.
-constexpr uint32_t kSpinLimit = 1u << 24;
-
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* error_flag,
-                                          int where) {
-  for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
-    if (mbar_try_wait(bar, parity)) return true;
-  }
-  if (error_flag != nullptr) atomicCAS(error_flag, 0, where);
-  return false;
-}
-
 // ----------------------------------------------------------------------------
 // proxies and bulk copies
 // ----------------------------------------------------------------------------
