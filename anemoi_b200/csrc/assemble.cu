@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "layer.cuh"
 #include "records.cuh"
 
 namespace {
@@ -73,6 +74,21 @@ int launch(const anemoi_sm100_shape& s, const void* prefix_out, int64_t prefix_r
       static_cast<OutT*>(out), s.seq_tokens, s.heads, s.prefix_tokens, s.query_block,
       s.video_blocks);
   return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
+}
+
+// Prefix rows only (the attention kernel writes video rows to their tokens itself).
+template <typename OutT, int D>
+__global__ void __launch_bounds__(256) assemble_prefix_kernel(const void* prefix_out, int64_t prefix_rows,
+                                                              int prefix_is_caller_dtype, OutT* out, int H,
+                                                              int prefix) {
+  constexpr int kVec = D / 8;
+  const int total = prefix * H * kVec;
+  for (int idx = blockIdx.x * 256 + threadIdx.x; idx < total; idx += gridDim.x * 256) {
+    const int c8 = idx % kVec, h = idx / kVec % H, s = idx / kVec / H;
+    const int64_t off = ((int64_t)h * prefix_rows + s) * D + c8 * 8;
+    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(prefix_out) + off));
+    *reinterpret_cast<uint4*>(out + (int64_t)idx * 8) = prefix_is_caller_dtype ? raw : convert8<OutT>(raw);
+  }
 }
 
 // ---- Ulysses relayouts: pure 16-byte copies --------------------------------------------
@@ -211,4 +227,22 @@ extern "C" int anemoi_sm100_copy_rows(void* dst, int64_t dst_pitch, const void* 
       dst, (size_t)dst_pitch, src, (size_t)src_pitch, (size_t)width, (size_t)height,
       to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
   return err == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
+}
+
+int layer::assemble_prefix(const anemoi_sm100_shape& s, const void* prefix_out, int64_t prefix_rows,
+                           int prefix_is_caller, void* out, cudaStream_t st) {
+  const int64_t total = (int64_t)s.prefix_tokens * s.heads * (s.head_dim / 8);
+  if (total > INT32_MAX / 2) return ANEMOI_SM100_ELIMIT;
+  const int blocks = (int)min((total + 255) / 256, (int64_t)(148 * 8));
+  auto go = [&](auto kernel, auto* o) {
+    kernel<<<blocks, 256, 0, st>>>(prefix_out, prefix_rows, prefix_is_caller, o, s.heads, s.prefix_tokens);
+  };
+  if (s.input_is_bf16) {
+    auto* o = static_cast<__nv_bfloat16*>(out);
+    s.head_dim == 64 ? go(assemble_prefix_kernel<__nv_bfloat16, 64>, o) : go(assemble_prefix_kernel<__nv_bfloat16, 128>, o);
+  } else {
+    auto* o = static_cast<__half*>(out);
+    s.head_dim == 64 ? go(assemble_prefix_kernel<__half, 64>, o) : go(assemble_prefix_kernel<__half, 128>, o);
+  }
+  return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
 }

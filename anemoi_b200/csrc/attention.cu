@@ -50,12 +50,14 @@
 #include <cuda_fp16.h>
 
 #include "bounded_wait.cuh"
+#include "layer.cuh"
 #include "records.cuh"
 #include "sm100_primitives.cuh"
 
 namespace {
 
 using namespace sm100;
+using layer::TokenRows;
 
 // Four warpgroups: softmax of the even stages, softmax of the odd stages, rescale of O, and
 // loader / QK / PV (one warp each, the fourth idle).
@@ -102,7 +104,11 @@ struct AttnParams {
   // of the two blocks the stage belongs to.  Null: one query block per CTA.
   const int32_t* pair_counts;  // [H][ceil(R/2)][4]
   const int32_t* pair_ids;     // [H][capacity], a pair's list starts at row_offset of block 2t
-  __half* out;       // [H][tiles*QB][D]
+  __half* out;       // [H][tiles*QB][D], or null:
+  void* tokens;      // [S][H][D] in the caller's type: rows go straight to their tokens
+  int tokens_bf16;
+  const int32_t* indices;  // raster token of a packed slot
+  const int32_t* counts;   // real tokens of a block
   int32_t* status;
   uint64_t wait_ns;  // limit of every mbarrier wait
   int dense_prefix;  // 1: prefix query tiles, INT8 cell over every stage
@@ -194,6 +200,14 @@ __device__ __forceinline__ uint32_t e2m1x8(const float* e) {
 __device__ __forceinline__ uint32_t f16x2(float a, float b) {
   uint32_t v;
   asm("cvt.rn.f16x2.f32 %0, %2, %1;" : "=r"(v) : "f"(a), "f"(b));
+  return v;
+}
+
+// Two fp32 -> fp16 (the result's precision) -> bf16, as the assembly of packed rows rounds.
+__device__ __forceinline__ uint32_t bf16x2_of_f16x2(uint32_t h) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+  uint32_t v;
+  asm("cvt.rn.bf16x2.f32 %0, %2, %1;" : "=r"(v) : "f"(f.x), "f"(f.y));
   return v;
 }
 
@@ -492,12 +506,28 @@ __device__ __forceinline__ void issue_pv(uint32_t tmem, uint32_t slot_addr, uint
 // stage code serves all: the CTAs of an SM are in different phases, and hot code that outgrows the
 // instruction cache costs more than the constants give (three whole copies of the softmax stage,
 // 100 KB of code: 1.48 us per 64-key stage and SM at D = 64 instead of 1.11).
+// Where a row of the tile goes in `tokens` (element offset of its first channel), -1: a padding row.
+template <int D>
+__device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, int tile, int block0, int QB, int row) {
+  int token;
+  if (p.dense_prefix) {
+    token = tile * QB + row;
+    if (row >= QB || token >= p.s.prefix_tokens) return -1;
+  } else {
+    const int block = block0 + row / QB;
+    if (row % QB >= p.counts[block]) return -1;
+    token = p.s.prefix_tokens + p.indices[block0 * QB + row];
+  }
+  return ((int64_t)token * p.s.heads + head) * D;
+}
+
 template <int D, int CELLS, bool kQ64>
 __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int kFirst = CELLS == kAny ? 0 : CELLS, kLast = CELLS == kAny ? 2 : CELLS;
   constexpr int QB = kQ64 ? 64 : 128;
   const int head = blockIdx.y;
+  layer::grid_dependency_wait();
   // launch order of the head's query blocks (longest list first) as written by the routing
   // stage; 0 = no order given
   int tile = blockIdx.x;
@@ -524,7 +554,16 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     list = (pairs ? p.pair_ids : p.stage_ids) + (int64_t)head * p.capacity +
            p.row_offset[(int64_t)head * p.s.video_blocks + block0];
   }
-  if (cnt[0] + cnt[1] + cnt[2] == 0) return;
+  if (cnt[0] + cnt[1] + cnt[2] == 0) {
+    // nothing to attend to: +0 rows (packed rows are left alone, the assembly knows)
+    if (p.tokens != nullptr)
+      for (int i = threadIdx.x; i < QB * tile_blocks * (D / 8); i += kThreads) {
+        const int64_t at = token_offset<D>(p, head, tile, block0, QB, i / (D / 8));
+        if (at >= 0)
+          *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.tokens) + at + i % (D / 8) * 8) = make_uint4(0, 0, 0, 0);
+      }
+    return;
+  }
   // After a give-up anywhere on this device the status word stays set: later CTAs (of this and
   // of later launches, until the host clears the word) return at once instead of each running
   // into its own wait limit.
@@ -917,16 +956,23 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     if (live_warp) {
       tc_fence_after_sync();
       const float d = b->rec[1][row].x;
-      // a block of a pair may have an empty list of its own: its rows are never read
       const float inv = d > 0.0f ? 1.0f / d : 0.0f;
-      const bool live = row < QB * tile_blocks;
-      __half* dst = p.out + ((int64_t)head * p.out_rows + (int64_t)block0 * QB + row) * D;
+      // packed rows: this tile's place; token rows: the row's token, in the caller's type
+      uint16_t* dst = nullptr;
+      if (p.tokens == nullptr) {
+        if (row < QB * tile_blocks)
+          dst = reinterpret_cast<uint16_t*>(p.out) + ((int64_t)head * p.out_rows + (int64_t)block0 * QB + row) * D;
+      } else if (row < QB * tile_blocks) {
+        const int64_t at = token_offset<D>(p, head, tile, block0, QB, row);
+        if (at >= 0) dst = static_cast<uint16_t*>(p.tokens) + at;
+      }
+      const bool bf16 = p.tokens != nullptr && p.tokens_bf16;
 #pragma unroll 1
       for (int c0 = parity * (D / 2); c0 < (parity + 1) * (D / 2); c0 += 32) {
         uint32_t r[32];
         tmem_ld32(tmem_row + kColO + c0, r);
         tmem_wait_ld();
-        if (live) {
+        if (dst != nullptr) {
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
             float f[8];
@@ -937,8 +983,12 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
               if (last_cell == kI8) f[i] *= vscale[c0 + j + i] * 0.0022326917f;
               f[i] *= inv;
             }
-            *reinterpret_cast<uint4*>(dst + c0 + j) =
-                make_uint4(f16x2(f[0], f[1]), f16x2(f[2], f[3]), f16x2(f[4], f[5]), f16x2(f[6], f[7]));
+            uint4 v = make_uint4(f16x2(f[0], f[1]), f16x2(f[2], f[3]), f16x2(f[4], f[5]), f16x2(f[6], f[7]));
+            if (bf16)
+              v = make_uint4(bf16x2_of_f16x2(v.x), bf16x2_of_f16x2(v.y), bf16x2_of_f16x2(v.z), bf16x2_of_f16x2(v.w));
+            // a block of a pair may have an empty list of its own: +0 rows
+            if (d == 0.0f) v = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(dst + c0 + j) = v;
           }
         }
       }
@@ -956,8 +1006,9 @@ int launch_kernel(const AttnParams& p, int tiles, size_t smem, cudaStream_t st) 
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
-  kernel<<<dim3(tiles, p.s.heads), kThreads, smem, st>>>(p);
-  return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
+  return layer::launch(kernel, dim3(tiles, p.s.heads), dim3(kThreads), smem, st, p) == cudaSuccess
+             ? ANEMOI_SM100_OK
+             : ANEMOI_SM100_ELAUNCH;
 }
 
 template <int D, bool kQ64>
@@ -972,6 +1023,9 @@ int launch(AttnParams& p, int tiles, cudaStream_t st) {
                                          : (cell == kI8 ? 128 * D : 256 * D));
     slot = max(slot, slot_bytes(D, cell));
   }
+  // Prefix tiles run beside video tiles: of a mixed call in the same kernel, so that an SM's CTAs share
+  // their code in the instruction cache.
+  if (p.dense_prefix && p.s.has_nvfp4 + p.s.has_fp16 > 0) one = kAny;
   q_region = (q_region + 127) & ~127;
   const int fixed = q_region + D * 4 + (int)sizeof(Shared);
   // two CTAs per SM: measured limit is 115,528 bytes of dynamic shared memory per CTA
@@ -1041,12 +1095,21 @@ extern "C" int anemoi_sm100_wait_selftest(uint64_t limit_ns, int32_t* status, vo
 }
 
 namespace {
+void set_rows(AttnParams& p, const TokenRows* rows) {
+  if (rows == nullptr) return;
+  p.tokens = rows->out;
+  p.tokens_bf16 = p.s.input_is_bf16;
+  p.indices = rows->indices;
+  p.counts = rows->counts;
+}
+
 int video_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operands* ops,
                     const int32_t* row_offset, const int32_t* row_counts, const int32_t* stage_ids,
                     const int32_t* pair_counts, const int32_t* pair_ids, int64_t list_capacity,
-                    const int32_t* valid_k, void* out_packed, int32_t* status, void* stream) {
+                    const int32_t* valid_k, void* out_packed, const TokenRows* rows, int32_t* status,
+                    void* stream) {
   if (rec::validate_shape(shape) != ANEMOI_SM100_OK || !ops || !row_offset || !row_counts ||
-      !valid_k || !out_packed || !status || list_capacity <= 0)
+      !valid_k || (!out_packed && !rows) || !status || list_capacity <= 0)
     return ANEMOI_SM100_EINVAL;
   if (check_ops(*shape, *ops, false) != ANEMOI_SM100_OK) return ANEMOI_SM100_EINVAL;
   AttnParams p{};
@@ -1066,6 +1129,7 @@ int video_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operands
   p.stages = rec::stages(*shape);
   p.q_tiles_int8 = shape->video_blocks + rec::prefix_query_tiles(*shape);
   p.out_rows = shape->video_blocks * shape->query_block;
+  set_rows(p, rows);
   const int tiles = pair_counts ? (shape->video_blocks + 1) / 2 : shape->video_blocks;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return launch_for(p, tiles, st);
@@ -1079,7 +1143,7 @@ extern "C" int anemoi_sm100_attention(const anemoi_sm100_shape* shape,
                                       void* out_packed, int32_t* status, void* stream) {
   if (!stage_ids) return ANEMOI_SM100_EINVAL;
   return video_attention(shape, ops, row_offset, row_counts, stage_ids, nullptr, nullptr,
-                         list_capacity, valid_k, out_packed, status, stream);
+                         list_capacity, valid_k, out_packed, nullptr, status, stream);
 }
 
 extern "C" int anemoi_sm100_attention_pairs(const anemoi_sm100_shape* shape,
@@ -1090,14 +1154,13 @@ extern "C" int anemoi_sm100_attention_pairs(const anemoi_sm100_shape* shape,
                                             void* out_packed, int32_t* status, void* stream) {
   if (!pair_counts || !pair_ids || !shape || shape->query_block != 64) return ANEMOI_SM100_EINVAL;
   return video_attention(shape, ops, row_offset, row_counts, nullptr, pair_counts, pair_ids,
-                         list_capacity, valid_k, out_packed, status, stream);
+                         list_capacity, valid_k, out_packed, nullptr, status, stream);
 }
 
-extern "C" int anemoi_sm100_prefix_attention(const anemoi_sm100_shape* shape,
-                                             const anemoi_sm100_operands* ops,
-                                             const int32_t* valid_k, void* out_prefix,
-                                             int32_t* status, void* stream) {
-  if (rec::validate_shape(shape) != ANEMOI_SM100_OK || !ops || !valid_k || !out_prefix || !status)
+namespace {
+int prefix_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operands* ops, const int32_t* valid_k,
+                     void* out_prefix, const TokenRows* rows, int32_t* status, void* stream) {
+  if (rec::validate_shape(shape) != ANEMOI_SM100_OK || !ops || !valid_k || (!out_prefix && !rows) || !status)
     return ANEMOI_SM100_EINVAL;
   if (!shape->has_prefix_query_int8 || shape->prefix_tokens == 0) return ANEMOI_SM100_EINVAL;
   if (check_ops(*shape, *ops, true) != ANEMOI_SM100_OK) return ANEMOI_SM100_EINVAL;
@@ -1113,6 +1176,32 @@ extern "C" int anemoi_sm100_prefix_attention(const anemoi_sm100_shape* shape,
   const int tiles = rec::prefix_query_tiles(*shape);
   p.q_tiles_int8 = shape->video_blocks + tiles;
   p.out_rows = tiles * shape->query_block;
+  set_rows(p, rows);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return launch_for(p, tiles, st);
 }
+}  // namespace
+
+extern "C" int anemoi_sm100_prefix_attention(const anemoi_sm100_shape* shape,
+                                             const anemoi_sm100_operands* ops,
+                                             const int32_t* valid_k, void* out_prefix,
+                                             int32_t* status, void* stream) {
+  return prefix_attention(shape, ops, valid_k, out_prefix, nullptr, status, stream);
+}
+
+namespace layer {
+
+int video_rows(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, const int32_t* row_offset,
+               const int32_t* row_counts, const int32_t* stage_ids, const int32_t* pair_counts,
+               const int32_t* pair_ids, int64_t capacity, const int32_t* valid_k, const TokenRows& rows,
+               int32_t* status, cudaStream_t st) {
+  return video_attention(&s, &ops, row_offset, row_counts, stage_ids, pair_counts, pair_ids, capacity, valid_k,
+                         nullptr, &rows, status, st);
+}
+
+int prefix_rows(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, const int32_t* valid_k,
+                const TokenRows& rows, int32_t* status, cudaStream_t st) {
+  return prefix_attention(&s, &ops, valid_k, nullptr, &rows, status, st);
+}
+
+}  // namespace layer

@@ -17,6 +17,7 @@
 // A CPU restatement with the same sequence reproduces the map bit for bit.
 #include <cuda_fp16.h>
 
+#include "layer.cuh"
 #include "records.cuh"
 
 namespace {
@@ -261,6 +262,8 @@ __global__ void __launch_bounds__(kWarps * 32) draft_kernel(const __half* q_pool
   const int head = blockIdx.y, row0 = blockIdx.x * kRows;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  layer::grid_dependency_wait();
+  layer::grid_dependency_trigger();
   row_logits<D, RPW>(q_pool, k_pool, head, R, row0, kc, qs, lg, lg_stride);
   if (kBlend) {
     __syncthreads();
@@ -307,8 +310,9 @@ int launch_rows(const __half* qp, const __half* kp, const __half* qx, const __ha
     return ANEMOI_SM100_ELAUNCH;
   constexpr int kRows = kWarps * RPW;
   dim3 grid((R + kRows - 1) / kRows, H);
-  kernel<<<grid, kWarps * 32, smem, st>>>(qp, kp, qx, kx, w, R, prob);
-  return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
+  return layer::launch(kernel, grid, dim3(kWarps * 32), smem, st, qp, kp, qx, kx, w, R, prob) == cudaSuccess
+             ? ANEMOI_SM100_OK
+             : ANEMOI_SM100_ELAUNCH;
 }
 
 // Four rows per warp while two CTAs still fit an SM's shared memory, else two rows per warp.

@@ -1,0 +1,171 @@
+// One anemoi_attention call in one entry point: operands, draft map, routing, video attention and
+// prefix attention, with the results written straight to their tokens.
+//
+// A small call is bound by its launches, not by its kernels: with one Python wrapper, allocation and
+// marshaling per stage the 1,024-token call spent 200 us on the host for 70 us of kernels.  Here the
+// host work is one function: one workspace cut up by offsets, fourteen launches less three (routing
+// is one kernel, the output needs no assembly pass), programmatic dependent launches between them.
+//
+// Order of the launches.  The prefix rows' tiles walk every stage of the head: few CTAs, each as
+// long as the whole video launch of a small call, so they start on the side stream as soon as the
+// operands are there and run beside draft and routing.  When they alone fill the GPU
+// they would only keep draft and routing waiting for a free SM (each CTA holds half of one for up to
+// milliseconds): then they start after routing, in front of the video tiles.
+#include <cuda_runtime.h>
+
+#include "layer.cuh"
+#include "records.cuh"
+
+namespace {
+
+constexpr int64_t kAlign = 256;
+constexpr int kPrefixFillsGpu = 148;  // prefix CTAs from which they start after routing
+
+int64_t up(int64_t n) { return (n + kAlign - 1) / kAlign * kAlign; }
+
+struct Workspace {
+  anemoi_sm100_operands ops;
+  uint8_t* prob;
+  int32_t *row_offset, *row_counts, *stage_ids, *pair_counts, *pair_ids;
+  uint8_t* scratch;
+  int64_t scratch_bytes, bytes;
+};
+
+// Cuts `base` (null: only the size is wanted) into the call's buffers.
+Workspace cut(const anemoi_sm100_layer_plan& p, uint8_t* base) {
+  const anemoi_sm100_shape& s = p.shape;
+  const int64_t H = s.heads, R = s.video_blocks;
+  Workspace w = {};
+  int64_t at = 0;
+  auto take = [&](int64_t n) -> uint8_t* {
+    uint8_t* ptr = n > 0 && base != nullptr ? base + at : nullptr;
+    at += up(n);
+    return ptr;
+  };
+  auto operand = [&](int which) { return take(anemoi_sm100_operand_bytes(&s, which)); };
+  w.ops.v_amax = reinterpret_cast<float*>(operand(ANEMOI_SM100_BUF_V_AMAX));
+  w.ops.q_fp16 = operand(ANEMOI_SM100_BUF_Q_FP16);
+  w.ops.kv_fp16 = operand(ANEMOI_SM100_BUF_KV_FP16);
+  w.ops.q_int8 = operand(ANEMOI_SM100_BUF_Q_INT8);
+  w.ops.kv_int8 = operand(ANEMOI_SM100_BUF_KV_INT8);
+  w.ops.q_nvfp4 = operand(ANEMOI_SM100_BUF_Q_NVFP4);
+  w.ops.kv_nvfp4 = operand(ANEMOI_SM100_BUF_KV_NVFP4);
+  w.ops.q_int8_scale = reinterpret_cast<float*>(operand(ANEMOI_SM100_BUF_Q_INT8_SCALE));
+  w.ops.k_int8_scale = reinterpret_cast<float*>(operand(ANEMOI_SM100_BUF_K_INT8_SCALE));
+  w.ops.v_e4m3_scale = reinterpret_cast<float*>(operand(ANEMOI_SM100_BUF_V_E4M3_SCALE));
+  w.ops.q_pool = operand(ANEMOI_SM100_BUF_POOL);
+  w.ops.k_pool = operand(ANEMOI_SM100_BUF_POOL);
+  if (s.has_maxpool) {
+    w.ops.q_max_pool = operand(ANEMOI_SM100_BUF_POOL);
+    w.ops.k_max_pool = operand(ANEMOI_SM100_BUF_POOL);
+  }
+  w.prob = take(H * R * R * 2);
+  w.row_offset = reinterpret_cast<int32_t*>(take(H * R * 4));
+  w.row_counts = reinterpret_cast<int32_t*>(take(H * R * 16));
+  const bool pairs = p.pair_q64 && s.query_block == 64, fused = pairs && layer::routes_pairs(s);
+  const int64_t list = H * p.list_capacity * 4;
+  // (routed in one kernel, the pairs need neither the blocks' own lists nor scratch)
+  if (!fused) w.stage_ids = reinterpret_cast<int32_t*>(take(list));
+  if (pairs) {
+    w.pair_counts = reinterpret_cast<int32_t*>(take(H * ((R + 1) / 2) * 16));
+    w.pair_ids = reinterpret_cast<int32_t*>(take(list));
+  }
+  w.scratch_bytes = fused ? 0 : anemoi_sm100_route_scratch_bytes(&s);
+  w.scratch = take(w.scratch_bytes);
+  w.bytes = at;
+  return w;
+}
+
+bool valid(const anemoi_sm100_layer_plan* p) {
+  return p != nullptr && rec::validate_shape(&p->shape) == ANEMOI_SM100_OK && p->indices && p->counts &&
+         p->valid_k && p->status && p->shape.has_maxpool != 2 && p->list_capacity > 0;
+}
+
+}  // namespace
+
+extern "C" int anemoi_sm100_routes_in_one_kernel(const anemoi_sm100_shape* shape) {
+  return rec::validate_shape(shape) == ANEMOI_SM100_OK && layer::routes_pairs(*shape);
+}
+
+extern "C" int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan) {
+  return valid(plan) ? cut(*plan, nullptr).bytes : ANEMOI_SM100_EINVAL;
+}
+
+extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const void* q, const void* k, const void* v,
+                                  const int64_t* strides, const float* nvfp4_scales, const void* prefix_out,
+                                  int64_t prefix_rows, int prefix_is_caller_dtype, void* out, void* workspace,
+                                  int64_t workspace_bytes, void* stream, void* side_stream) {
+  if (!valid(plan) || !q || !k || !v || !out || !workspace) return ANEMOI_SM100_EINVAL;
+  anemoi_sm100_layer_plan p = *plan;
+  anemoi_sm100_shape& s = p.shape;
+  if (nvfp4_scales != nullptr) {
+    s.q_global_scale = nvfp4_scales[0];
+    s.k_global_scale = nvfp4_scales[1];
+    s.v_global_scale = nvfp4_scales[2];
+    if (rec::validate_shape(&s) != ANEMOI_SM100_OK) return ANEMOI_SM100_EINVAL;
+  }
+  const bool native_prefix = s.has_prefix_query_int8 && s.prefix_tokens > 0;
+  if (s.prefix_tokens > 0 && !native_prefix && prefix_out == nullptr) return ANEMOI_SM100_EINVAL;
+  if (s.prefix_tokens > 0 && side_stream == nullptr) return ANEMOI_SM100_EINVAL;
+  const Workspace w = cut(p, static_cast<uint8_t*>(workspace));
+  if (workspace_bytes < w.bytes) return ANEMOI_SM100_EINVAL;
+  cudaStream_t st = static_cast<cudaStream_t>(stream), side = static_cast<cudaStream_t>(side_stream);
+  const layer::TokenRows rows{out, p.indices, p.counts};
+
+  int code = anemoi_sm100_prepare(&s, q, k, v, strides, p.indices, p.counts, &w.ops, stream);
+  if (code != ANEMOI_SM100_OK) return code;
+
+  // fork and join of the side stream: an event each, destroyed when its use is over
+  cudaEvent_t fork = nullptr, join = nullptr;
+  auto done = [&](int c) {
+    if (c != ANEMOI_SM100_OK && fork != nullptr && join == nullptr &&
+        cudaEventCreateWithFlags(&join, cudaEventDisableTiming) == cudaSuccess &&
+        cudaEventRecord(join, side) == cudaSuccess)
+      cudaStreamWaitEvent(st, join, 0);  // the workspace is not free before the side stream is done with it
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    return c;
+  };
+  auto prefix = [&]() -> int {
+    if (cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventRecord(fork, st) != cudaSuccess || cudaStreamWaitEvent(side, fork, 0) != cudaSuccess)
+      return ANEMOI_SM100_ELAUNCH;
+    return layer::prefix_rows(s, w.ops, p.valid_k, rows, p.status, side);
+  };
+  const bool late = native_prefix && rec::prefix_query_tiles(s) * s.heads >= kPrefixFillsGpu;
+  if (native_prefix && !late && (code = prefix()) != ANEMOI_SM100_OK) return done(code);
+
+  code = anemoi_sm100_draft_probability(&s, w.ops.q_pool, w.ops.k_pool, w.ops.q_max_pool, w.ops.k_max_pool,
+                                        p.maxpool_weight, w.prob, stream);
+  if (code != ANEMOI_SM100_OK) return done(code);
+  const int32_t* pair_counts = nullptr;
+  if (p.pair_q64 && s.query_block == 64) {
+    if (layer::routes_pairs(s)) {
+      code = anemoi_sm100_route_pairs(&s, w.prob, p.n16, p.n8, p.n4, p.prefix_phase, w.row_offset, w.row_counts,
+                                      w.pair_counts, w.pair_ids, p.list_capacity, stream);
+    } else {
+      code = anemoi_sm100_route(&s, w.prob, p.n16, p.n8, p.n4, p.prefix_phase, w.scratch, w.scratch_bytes,
+                                w.row_offset, w.row_counts, w.stage_ids, p.list_capacity, stream);
+      if (code == ANEMOI_SM100_OK)
+        code = anemoi_sm100_pair_lists(&s, w.row_offset, w.row_counts, w.stage_ids, p.list_capacity, w.pair_counts,
+                                       w.pair_ids, stream);
+    }
+    pair_counts = w.pair_counts;
+  } else {
+    code = anemoi_sm100_route(&s, w.prob, p.n16, p.n8, p.n4, p.prefix_phase, w.scratch, w.scratch_bytes,
+                              w.row_offset, w.row_counts, w.stage_ids, p.list_capacity, stream);
+  }
+  if (code != ANEMOI_SM100_OK) return done(code);
+  if (late && (code = prefix()) != ANEMOI_SM100_OK) return done(code);
+  code = layer::video_rows(s, w.ops, w.row_offset, w.row_counts, w.stage_ids, pair_counts, w.pair_ids,
+                           p.list_capacity, p.valid_k, rows, p.status, st);
+  if (code != ANEMOI_SM100_OK) return done(code);
+  if (s.prefix_tokens > 0) {
+    if (cudaEventCreateWithFlags(&join, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventRecord(join, side) != cudaSuccess || cudaStreamWaitEvent(st, join, 0) != cudaSuccess)
+      return done(ANEMOI_SM100_ELAUNCH);
+    if (!native_prefix)
+      code = layer::assemble_prefix(s, prefix_out, prefix_rows, prefix_is_caller_dtype, out, st);
+  }
+  return done(code);
+}

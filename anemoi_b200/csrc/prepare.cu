@@ -19,6 +19,7 @@
 #include <cuda_fp4.h>
 #include <cuda_fp8.h>
 
+#include "layer.cuh"
 #include "records.cuh"
 
 namespace {
@@ -38,8 +39,6 @@ struct PrepParams {
   int64_t stride[6];  // token and head stride (elements) of q, k, v
 };
 
-template <typename InT>
-__device__ __forceinline__ uint4 load_narrow8(const InT* p);
 // 8 raw 16-bit elements -> 8 fp16 (bf16 through fp32, round to nearest even; fp16 unchanged)
 template <typename InT>
 __device__ __forceinline__ uint4 narrow8(uint4 raw);
@@ -49,24 +48,6 @@ __device__ __forceinline__ uint4 narrow8<__half>(uint4 raw) {
 }
 template <>
 __device__ __forceinline__ uint4 narrow8<__nv_bfloat16>(uint4 raw) {
-  const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&raw);
-  uint4 out;
-  __half2* h = reinterpret_cast<__half2*>(&out);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float2 f = __bfloat1622float2(b[i]);
-    h[i] = __floats2half2_rn(f.x, f.y);
-  }
-  return out;
-}
-
-template <>
-__device__ __forceinline__ uint4 load_narrow8<__half>(const __half* p) {
-  return __ldg(reinterpret_cast<const uint4*>(p));
-}
-template <>
-__device__ __forceinline__ uint4 load_narrow8<__nv_bfloat16>(const __nv_bfloat16* p) {
-  uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
   const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&raw);
   uint4 out;
   __half2* h = reinterpret_cast<__half2*>(&out);
@@ -318,6 +299,8 @@ __global__ void __launch_bounds__(kThreads) prepare_kernel(PrepParams p) {
   __shared__ float red[kThreads / 32];
   __shared__ float recip[D];
 
+  layer::grid_dependency_wait();
+  layer::grid_dependency_trigger();
   const int R = p.s.video_blocks;
   // heads vary fastest across concurrently running CTAs: neighbours read adjacent 2*D-byte
   // pieces of the same token rows
@@ -438,26 +421,74 @@ __global__ void __launch_bounds__(kThreads) prepare_kernel(PrepParams p) {
   }
 }
 
-// max |v| per (head, channel) over every token, as the bit pattern of a
-// non-negative float (integer max == float max).  `out` must be zeroed first.
+// Two 16-bit magnitudes at a time; a NaN never wins (as fmaxf).
 template <typename InT>
-__global__ void __launch_bounds__(256) v_amax_kernel(const InT* v, int* out, int64_t tokens,
-                                                     int heads, int d8, int64_t token_stride,
-                                                     int64_t head_stride, int tokens_per_block) {
-  const int col8 = blockIdx.x * 256 + threadIdx.x;
-  if (col8 >= heads * d8) return;
-  const int head = col8 / d8, c8 = col8 % d8;
-  const int64_t t0 = (int64_t)blockIdx.y * tokens_per_block;
-  const int64_t t1 = min(tokens, t0 + tokens_per_block);
-  float m[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int64_t t = t0; t < t1; ++t) {
-    uint4 raw = load_narrow8<InT>(v + t * token_stride + head * head_stride + c8 * 8);
-    const __half* h = reinterpret_cast<const __half*>(&raw);
+struct Abs2;
+template <>
+struct Abs2<__half> {
+  using T = __half2;
+};
+template <>
+struct Abs2<__nv_bfloat16> {
+  using T = __nv_bfloat162;
+};
+
+// max |v| per (head, channel) over every token, as the bit pattern of a non-negative float
+// (integer max == float max).  `out` must be zeroed first.  A pure read of V, so HBM bound; the
+// maximum is taken in the input's own type (rounding to fp16 is monotonic and happens once at
+// the end).  One CTA = 32 vectors of 8 channels x 8 token lanes, four 16-byte loads in flight per
+// thread, and about eight CTAs per SM whatever the number of heads: with one thread per vector
+// walking 128 tokens alone, V of 7 heads x 33,272 tokens (60 MB) took 60 us, now 15.
+constexpr int kAmaxLanes = 8;
+template <typename InT>
+__global__ void __launch_bounds__(32 * kAmaxLanes) v_amax_kernel(const InT* v, int* out, int64_t tokens,
+                                                                 int heads, int d8, int64_t token_stride,
+                                                                 int64_t head_stride, int tokens_per_block) {
+  using T2 = typename Abs2<InT>::T;
+  __shared__ T2 part[kAmaxLanes][32][4 + 1];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int col8 = blockIdx.x * 32 + x;
+  const bool live = col8 < heads * d8;
+  layer::grid_dependency_wait();
+  layer::grid_dependency_trigger();
+  T2 m[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) m[i] = fmaxf(m[i], fabsf(__half2float(h[i])));
+  for (int i = 0; i < 4; ++i) m[i] = T2(InT(0.0f), InT(0.0f));
+  if (live) {
+    const InT* src = v + (int64_t)(col8 / d8) * head_stride + (col8 % d8) * 8;
+    const int64_t t0 = (int64_t)blockIdx.y * tokens_per_block;
+    const int64_t t1 = min(tokens, t0 + tokens_per_block);
+    int64_t t = t0 + y;
+    for (; t + 3 * kAmaxLanes < t1; t += 4 * kAmaxLanes) {
+      uint4 raw[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        raw[k] = __ldg(reinterpret_cast<const uint4*>(src + (t + k * kAmaxLanes) * token_stride));
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const T2* h = reinterpret_cast<const T2*>(&raw[k]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m[i] = __hmax2(m[i], __habs2(h[i]));
+      }
+    }
+    for (; t < t1; t += kAmaxLanes) {
+      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src + t * token_stride));
+      const T2* h = reinterpret_cast<const T2*>(&raw);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m[i] = __hmax2(m[i], __habs2(h[i]));
+    }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) atomicMax(out + col8 * 8 + i, __float_as_int(m[i]));
+  for (int i = 0; i < 4; ++i) part[y][x][i] = m[i];
+  __syncthreads();
+  // thread (x, y) finishes channel y of vector x
+  T2 r = part[0][x][y >> 1];
+#pragma unroll
+  for (int k = 1; k < kAmaxLanes; ++k) r = __hmax2(r, part[k][x][y >> 1]);
+  if (live) {
+    const float f = static_cast<float>(y & 1 ? r.y : r.x);
+    atomicMax(out + col8 * 8 + y, __float_as_int(__half2float(__float2half_rn(f))));
+  }
 }
 
 template <typename InT, int QB, int D>
@@ -470,18 +501,21 @@ int launch(const PrepParams& p, cudaStream_t stream) {
   if (p.s.has_int8) {
     if (cudaMemsetAsync(p.o.v_amax, 0, sizeof(float) * p.s.heads * D, stream) != cudaSuccess)
       return ANEMOI_SM100_ELAUNCH;
-    const int cols = p.s.heads * D / 8;
-    const int tokens_per_block = 128;
-    dim3 grid((cols + 255) / 256, (p.s.seq_tokens + tokens_per_block - 1) / tokens_per_block);
-    v_amax_kernel<InT><<<grid, 256, 0, stream>>>(
-        static_cast<const InT*>(p.v), reinterpret_cast<int*>(p.o.v_amax), p.s.seq_tokens,
-        p.s.heads, D / 8, p.stride[4], p.stride[5], tokens_per_block);
+    const int chunks = (p.s.heads * D / 8 + 31) / 32;
+    // about eight CTAs per SM, each with at least two loads per thread
+    const int rows = max(1, 8 * 148 / chunks);
+    const int tokens_per_block = max(2 * kAmaxLanes, (p.s.seq_tokens + rows - 1) / rows);
+    dim3 grid(chunks, (p.s.seq_tokens + tokens_per_block - 1) / tokens_per_block);
+    if (layer::launch(v_amax_kernel<InT>, grid, dim3(32 * kAmaxLanes), 0, stream, static_cast<const InT*>(p.v),
+                      reinterpret_cast<int*>(p.o.v_amax), p.s.seq_tokens, p.s.heads, D / 8, p.stride[4],
+                      p.stride[5], tokens_per_block) != cudaSuccess)
+      return ANEMOI_SM100_ELAUNCH;
   }
   const int tasks = 2 * p.s.video_blocks + p.prefix_stages + p.prefix_q_tiles;
   if (tasks > 65535) return ANEMOI_SM100_ELIMIT;
   dim3 grid(p.s.heads, tasks);
-  kernel<<<grid, kThreads, smem, stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
+  return layer::launch(kernel, grid, dim3(kThreads), smem, stream, p) == cudaSuccess ? ANEMOI_SM100_OK
+                                                                                    : ANEMOI_SM100_ELAUNCH;
 }
 
 }  // namespace

@@ -21,8 +21,10 @@
 // the map again; a last pass per row writes the lists.  The per-row passes use one
 // warp per row: ranks inside a row come from ballots, no block-wide barrier.
 #include <climits>
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
+#include "layer.cuh"
 #include "records.cuh"
 
 namespace {
@@ -529,6 +531,429 @@ __global__ void __launch_bounds__(kRowWarps * 32) anchor_emit_kernel(
   }
 }
 
+// ---- the whole routing of a head in one kernel ------------------------------------------------
+// One cluster of 1-8 CTAs per head, each with a contiguous range of the head's rows: histogram
+// (32,768 bins in shared memory), boundaries, per-row counts, scans over the rows, lists, launch
+// order; with kPairs the union lists of the Q64 query-block pairs instead of the rows' own lists.
+// The CTAs of a cluster add up histograms and row totals through distributed shared memory.  The
+// map is read three times from L2; what bounds the kernel is the shared-memory atomics of the
+// histogram and, for short maps, its dozen barriers.  As five launches (and two more for the
+// pairs, whose merge was one lane per phase) the same work took, alone, 8 heads x 64 blocks: 22 us
+// in kernels and 20 in gaps; 56 heads x 672 blocks: 250 us; 56 heads x 592 pairs: 720 us.
+constexpr int kFusedThreads = 1024;
+constexpr int kFusedWarps = kFusedThreads / 32;
+
+struct FusedShared {
+  int block_sum[1024];   // items per 32 bins, this CTA's rows
+  int warp_sum[kFusedWarps];
+  int part[8];           // this CTA's totals, read by the CTAs behind it
+  int hit_block[3], hit_off[3];
+  int key[3], quota[3];
+};
+
+__host__ __device__ inline size_t fused_smem() { return (size_t)kBins * 4 + sizeof(FusedShared); }
+
+// CTAs per head: as many as keep every head on an SM of its own at once, each with at least 16K
+// pairs; `rows_per` rows each (even, so that no pair of blocks is split).
+inline int fused_ctas(int H, int R) {
+  int c = 1;
+  while (c < 8 && (int64_t)R * R / c > 32768 && H * c * 2 <= 148) c *= 2;
+  return c;
+}
+inline int fused_rows(int R, int ctas) { return ((R + ctas - 1) / ctas + 1) & ~1; }
+// The rows' counts take the histogram's place, which bounds the rows of a CTA; and few heads with long
+// maps leave most SMs without work, where the launches over all rows are quicker (2 heads x 1,501
+// blocks: 163 us against 219; 7 heads x 672: 77 against 71).
+inline bool fused_fits(int H, int R) {
+  const int ctas = fused_ctas(H, R);
+  if (R > 4096 || 9 * fused_rows(R, ctas) + R > kBins) return false;
+  return H * ctas >= 74 || (int64_t)R * R / ctas <= 65536;
+}
+
+// Exclusive prefix of v over the CTA's threads; `total` gets the sum.
+__device__ __forceinline__ int fused_exclusive(int v, int* warp_sum, int& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += n;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  const int w = warp_sum[lane];
+  int winc = w;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, winc, off);
+    if (lane >= off) winc += n;
+  }
+  total = __shfl_sync(0xffffffffu, winc, 31);
+  const int base = __shfl_sync(0xffffffffu, winc - w, warp);
+  __syncthreads();
+  return base + incl - v;
+}
+
+constexpr int kAhead = 8;  // 32-column pieces of a row whose keys are loaded before the first is looked at
+
+// The keys of columns [j0, j0 + 32 * kAhead) of a row, -2 past its end.
+__device__ __forceinline__ void fused_keys(const unsigned short* src, int j0, int R, int (&key)[kAhead]) {
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+    const int j = j0 + u * 32 + (threadIdx.x & 31);
+    key[u] = j < R ? (__ldg(src + j) & 0x7fff) : -2;
+  }
+}
+
+// Precision code (3 FP16, 2 INT8, 1 NVFP4, 0 dropped) of the lane's column; advances the row's
+// counters of straddling keys met so far.  Straddling keys are rare: one vote skips their ranks.
+__device__ __forceinline__ int fused_code(int key, const int (&key_b)[3], const int (&quota_b)[3], int (&run)[3],
+                                          unsigned lower) {
+  int c = (key > key_b[0]) + (key > key_b[1]) + (key > key_b[2]);
+  if (__any_sync(0xffffffffu, key == key_b[0] || key == key_b[1] || key == key_b[2])) {
+    c = 0;
+#pragma unroll
+    for (int b = 2; b >= 0; --b) {
+      const unsigned ties = __ballot_sync(0xffffffffu, key == key_b[b]);
+      const bool below = key > key_b[b] || (key == key_b[b] && run[b] + __popc(ties & lower) < quota_b[b]);
+      run[b] += __popc(ties);
+      c = below ? 3 - b : c;
+    }
+  }
+  return c;
+}
+
+template <bool kPairs>
+__global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
+    const unsigned short* prob, int R, int rows_per, int b0, int b1, int b2, int factor, int prefix_stages,
+    int prefix_phase, int64_t capacity, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids,
+    int32_t* pair_counts, int32_t* pair_ids) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) int hist[];
+  FusedShared& sh = *reinterpret_cast<FusedShared*>(hist + kBins);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ctas = cluster.num_blocks(), me = cluster.block_rank();
+  const int head = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lower = (1u << lane) - 1u;
+  const int r0 = min(R, me * rows_per), r1 = min(R, r0 + rows_per), mine = r1 - r0;
+  const unsigned short* map = prob + (int64_t)head * R * R;
+
+  // ---- histogram of this CTA's rows ----
+  for (int i = threadIdx.x; i < kBins / 4; i += kFusedThreads) reinterpret_cast<int4*>(hist)[i] = make_int4(0, 0, 0, 0);
+  __syncthreads();
+  layer::grid_dependency_wait();
+  layer::grid_dependency_trigger();
+  {
+    const unsigned short* src = map + (int64_t)r0 * R;
+    const int items = mine * R;
+    const int head_items = min(items, (int)((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 2);
+    const int vecs = (items - head_items) / 8;
+    const uint4* v = reinterpret_cast<const uint4*>(src + head_items);
+    if ((int)threadIdx.x < head_items) atomicAdd(&hist[__ldg(src + threadIdx.x) & 0x7fff], 1);
+    const int tail = head_items + vecs * 8;
+    if (tail + (int)threadIdx.x < items && threadIdx.x < 8) atomicAdd(&hist[__ldg(src + tail + threadIdx.x) & 0x7fff], 1);
+#pragma unroll 2
+    for (int i = threadIdx.x; i < vecs; i += kFusedThreads) {
+      const uint4 q = __ldg(v + i);
+      const unsigned w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        atomicAdd(&hist[w[k] & 0x7fff], 1);
+        atomicAdd(&hist[(w[k] >> 16) & 0x7fff], 1);
+      }
+    }
+  }
+  __syncthreads();
+  // ---- the key that straddles each boundary (keys ranked from the largest down) ----
+#pragma unroll 4
+  for (int i = 0; i < 32; ++i) {
+    const int sum = __reduce_add_sync(0xffffffffu, hist[(warp * 32 + i) * 32 + lane]);
+    if (lane == 0) sh.block_sum[warp * 32 + i] = sum;
+  }
+  if (threadIdx.x < 3) sh.hit_block[threadIdx.x] = -1;
+  cluster.sync();
+  {
+    const int blk = 1023 - threadIdx.x;  // blocks in descending key order
+    int total = 0;
+    for (int c = 0; c < ctas; ++c) total += cluster.map_shared_rank(sh.block_sum, c)[blk];
+    int all;
+    const int above = fused_exclusive(total, sh.warp_sum, all);
+    const int bound[3] = {b0, b1, b2};
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      if (total > 0 && above <= bound[b] && bound[b] < above + total) {
+        sh.hit_block[b] = blk;
+        sh.hit_off[b] = bound[b] - above;
+      }
+  }
+  __syncthreads();
+  if (warp < 3) {
+    int key = -1, quota = 0;  // boundary at or past the last item: every key lies above it
+    const int hb = sh.hit_block[warp];
+    if (hb >= 0) {
+      const int bin = hb * 32 + 31 - lane;  // descending inside the block
+      int n = 0;
+      for (int c = 0; c < ctas; ++c) n += cluster.map_shared_rank(hist, c)[bin];
+      int incl = n;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int m = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += m;
+      }
+      const int off = sh.hit_off[warp];
+      const int src = __ffs(__ballot_sync(0xffffffffu, n > 0 && incl - n <= off && off < incl)) - 1;
+      key = __shfl_sync(0xffffffffu, bin, src);
+      quota = __shfl_sync(0xffffffffu, off - (incl - n), src);
+    }
+    if (lane == 0) {
+      sh.key[warp] = key;
+      sh.quota[warp] = quota;
+    }
+  }
+  cluster.sync();  // the histograms are read; their space holds the rows' counts from here on
+  const int key_b[3] = {sh.key[0], sh.key[1], sh.key[2]};
+  const int quota_b[3] = {sh.quota[0], sh.quota[1], sh.quota[2]};
+  int* stat = hist;                    // [mine][6]: keys above boundary 0-2, equal to its key 0-2
+  int* totals = stat + 6 * rows_per;   // [mine] stages of a row
+  int* offset = totals + rows_per;     // [mine] where its list starts
+  int* unions = offset + rows_per;     // [pairs of mine] stages of a pair's union
+  int* every = unions + rows_per;      // [R] the totals (unions) of the whole head
+
+  // ---- per row: keys above and equal to each straddling key ----
+  for (int i = warp; i < mine; i += kFusedWarps) {
+    const unsigned short* src = map + (int64_t)(r0 + i) * R;
+    int g[3] = {0, 0, 0}, e[3] = {0, 0, 0};
+    for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
+      int key[kAhead];
+      fused_keys(src, j0, R, key);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+          g[b] += key[u] > key_b[b];
+          e[b] += key[u] == key_b[b];
+        }
+    }
+    int v = 0;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const int gs = __reduce_add_sync(0xffffffffu, g[b]), es = __reduce_add_sync(0xffffffffu, e[b]);
+      v = lane == b ? gs : (lane == 3 + b ? es : v);
+    }
+    if (lane < 6) stat[i * 6 + lane] = v;
+  }
+  __syncthreads();
+  // ---- scans over the rows: position inside the straddling bins, stages per phase, list offset ----
+  const int p = prefix_phase >= 0 ? prefix_stages : 0;
+  int carry[4] = {0, 0, 0, 0};
+  {
+    int own[3] = {0, 0, 0};
+    for (int i = threadIdx.x; i < mine; i += kFusedThreads)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) own[b] += stat[i * 6 + 3 + b];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      int all;
+      fused_exclusive(own[b], sh.warp_sum, all);
+      if (threadIdx.x == 0) sh.part[b] = all;
+    }
+    cluster.sync();
+    for (int c = 0; c < me; ++c)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) carry[b] += cluster.map_shared_rank(sh.part, c)[b];
+  }
+  int sum_mine = 0;
+  for (int i0 = 0; i0 < mine; i0 += kFusedThreads) {
+    const int i = i0 + threadIdx.x;
+    const bool in = i < mine;
+    int below[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const int eq = in ? stat[i * 6 + 3 + b] : 0;
+      int all;
+      const int pre = carry[b] + fused_exclusive(eq, sh.warp_sum, all);
+      carry[b] += all;
+      // items of the straddling key in this row that still fall above the boundary
+      below[b] = in ? stat[i * 6 + b] + max(0, min(eq, quota_b[b] - pre)) : 0;
+      if (in) stat[i * 6 + 3 + b] = pre;
+    }
+    const int n0 = (below[2] - below[1]) * factor + (prefix_phase == 0 ? p : 0);  // NVFP4
+    const int n1 = (below[1] - below[0]) * factor + (prefix_phase == 1 ? p : 0);  // INT8
+    const int n2 = below[0] * factor + (prefix_phase == 2 ? p : 0);               // FP16
+    if (in) {
+      stat[i * 6] = n0;
+      stat[i * 6 + 1] = n1;
+      stat[i * 6 + 2] = n2;
+      totals[i] = n0 + n1 + n2;
+      sum_mine += n0 + n1 + n2;
+    }
+  }
+  {
+    int all;
+    fused_exclusive(sum_mine, sh.warp_sum, all);
+    if (threadIdx.x == 0) sh.part[3] = all;
+    cluster.sync();
+    for (int c = 0; c < me; ++c) carry[3] += cluster.map_shared_rank(sh.part, c)[3];
+  }
+  for (int i0 = 0; i0 < mine; i0 += kFusedThreads) {
+    const int i = i0 + threadIdx.x;
+    const bool in = i < mine;
+    int all;
+    const int off = carry[3] + fused_exclusive(in ? totals[i] : 0, sh.warp_sum, all);
+    carry[3] += all;
+    if (in) {
+      offset[i] = off;
+      row_offset[(int64_t)head * R + r0 + i] = off;
+      int32_t* rc = row_counts + ((int64_t)head * R + r0 + i) * 4;
+      rc[0] = stat[i * 6];
+      rc[1] = stat[i * 6 + 1];
+      rc[2] = stat[i * 6 + 2];
+      if (kPairs) rc[3] = 0;  // no launch order of single blocks
+    }
+  }
+  __syncthreads();
+  // ---- lists ----
+  const bool active[3] = {b2 > b1, b1 > b0, b0 > 0};  // phases with a budget
+  if (!kPairs) {
+    for (int i = warp; i < mine; i += kFusedWarps) {
+      const int n0 = stat[i * 6], n1 = stat[i * 6 + 1], total = totals[i];
+      const int64_t base = offset[i];
+      if (total == 0 || base + total > capacity) continue;  // (the latter cannot happen with exact budgets)
+      int32_t* list = stage_ids + (int64_t)head * capacity + base;
+      // where the video stages of each phase start
+      int at[3] = {prefix_phase == 0 ? p : 0, n0 + (prefix_phase == 1 ? p : 0),
+                   n0 + n1 + (prefix_phase == 2 ? p : 0)};
+      if (prefix_phase >= 0) {
+        const int seg = prefix_phase == 0 ? 0 : (prefix_phase == 1 ? n0 : n0 + n1);
+        for (int s = lane; s < p; s += 32) list[seg + s] = s;
+      }
+      int run[3] = {stat[i * 6 + 3], stat[i * 6 + 4], stat[i * 6 + 5]};
+      const unsigned short* src = map + (int64_t)(r0 + i) * R;
+      for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
+        int key[kAhead];
+        fused_keys(src, j0, R, key);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const int stage = prefix_stages + (j0 + u * 32 + lane) * factor;
+          const int c = fused_code(key[u], key_b, quota_b, run, lower);
+#pragma unroll
+          for (int k = 1; k <= 3; ++k) {
+            if (!active[k - 1]) continue;
+            const unsigned members = __ballot_sync(0xffffffffu, c == k);
+            if (c == k) {
+              int32_t* dst = list + at[k - 1] + __popc(members & lower) * factor;
+              dst[0] = stage;
+              if (factor == 2) dst[1] = stage + 1;
+            }
+            at[k - 1] += __popc(members) * factor;
+          }
+        }
+      }
+    }
+  } else {
+    // One warp per pair (blocks 2t and 2t+1; rows_per is even): a stage of either block's list
+    // enters the union of its phase once, with a bit per block.  The union of phase c starts where
+    // the two blocks' phases before it would end, so no offsets are scanned.
+    const int pairs_all = (R + 1) / 2;
+    for (int i = 2 * warp; i < mine; i += 2 * kFusedWarps) {
+      const bool has_b = i + 1 < mine;
+      const int a = i, bb = has_b ? i + 1 : i;
+      const int n0 = stat[a * 6] + (has_b ? stat[bb * 6] : 0), n1 = stat[a * 6 + 1] + (has_b ? stat[bb * 6 + 1] : 0);
+      const int total = totals[a] + (has_b ? totals[bb] : 0);
+      const int64_t base = offset[a];
+      const bool fits = base + total <= capacity;
+      int32_t* list = pair_ids + (int64_t)head * capacity + base;
+      const int start[3] = {0, n0, n0 + n1};
+      int at[3] = {start[0], start[1], start[2]};
+      const int both = has_b ? (int)0xc0000000u : 1 << 30;
+      if (prefix_phase >= 0 && fits) {
+        for (int s = lane; s < p; s += 32) list[start[prefix_phase] + s] = s | both;
+        at[prefix_phase] += p;
+      }
+      int run_a[3] = {stat[a * 6 + 3], stat[a * 6 + 4], stat[a * 6 + 5]};
+      int run_b[3] = {stat[bb * 6 + 3], stat[bb * 6 + 4], stat[bb * 6 + 5]};
+      const unsigned short* src_a = map + (int64_t)(r0 + a) * R;
+      const unsigned short* src_b = map + (int64_t)(r0 + bb) * R;
+      for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
+        int ka[kAhead], kb[kAhead];
+        fused_keys(src_a, j0, R, ka);
+        fused_keys(src_b, j0, has_b ? R : 0, kb);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const int stage = prefix_stages + j0 + u * 32 + lane;
+          const int ca = fused_code(ka[u], key_b, quota_b, run_a, lower);
+          const int cb = fused_code(kb[u], key_b, quota_b, run_b, lower);
+#pragma unroll
+          for (int k = 1; k <= 3; ++k) {
+            if (!active[k - 1]) continue;
+            const bool in = ca == k || cb == k;
+            const unsigned members = __ballot_sync(0xffffffffu, in);
+            if (in && fits)
+              list[at[k - 1] + __popc(members & lower)] =
+                  stage | (ca == k ? 1 << 30 : 0) | (cb == k ? (int)(1u << 31) : 0);
+            at[k - 1] += __popc(members);
+          }
+        }
+      }
+      const int u[3] = {at[0] - start[0], at[1] - start[1], at[2] - start[2]};
+      if (lane < 3) pair_counts[((int64_t)head * pairs_all + (r0 + i) / 2) * 4 + lane] = lane == 0 ? u[0] : lane == 1 ? u[1] : u[2];
+      if (lane == 0) unions[i / 2] = u[0] + u[1] + u[2];
+    }
+  }
+  // ---- launch order: longest list first, ties by block index, as block + 1 in the fourth entry of
+  // the position's counts ----
+  const int unit = kPairs ? 2 : 1;
+  const int count = (R + unit - 1) / unit, per = rows_per / unit, first = r0 / unit;
+  const int own = (mine + unit - 1) / unit;
+  cluster.sync();
+  for (int j = threadIdx.x; j < count; j += kFusedThreads)
+    every[j] = cluster.map_shared_rank(kPairs ? unions : totals, j / per)[j % per];
+  __syncthreads();
+  int32_t* order = (kPairs ? pair_counts + (int64_t)head * count * 4 : row_counts + (int64_t)head * count * 4) + 3;
+  for (int i = threadIdx.x; i < own; i += kFusedThreads) {
+    const int me_i = first + i, len = every[me_i];
+    int rank = 0;
+#pragma unroll 8
+    for (int j = 0; j < count; ++j) rank += every[j] > len || (every[j] == len && j < me_i);
+    order[rank * 4] = me_i + 1;
+  }
+  cluster.sync();  // no CTA leaves while another may still read its totals
+}
+
+template <bool kPairs>
+int launch_fused(const anemoi_sm100_shape& s, const void* probability, int64_t n16, int64_t n8, int64_t n4,
+                 int prefix_phase, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids, int64_t capacity,
+                 int32_t* pair_counts, int32_t* pair_ids, cudaStream_t st) {
+  const int H = s.heads, R = s.video_blocks, ctas = fused_ctas(H, R);
+  auto kernel = route_fused_kernel<kPairs>;
+  // Function attributes belong to a device: the opt-in is made at every call (a cheap host-side
+  // driver call), so a process that routes on several GPUs, or from several host threads,
+  // never launches the kernel without the opt-in for its dynamic shared memory.
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem()) != cudaSuccess)
+    return ANEMOI_SM100_ELAUNCH;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas, H);
+  cfg.blockDim = dim3(kFusedThreads);
+  cfg.dynamicSmemBytes = fused_smem();
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<const unsigned short*>(probability), R, fused_rows(R, ctas),
+                            (int)n16, (int)(n16 + n8), (int)(n16 + n8 + n4), s.query_block / 64,
+                            rec::prefix_stages(s), prefix_phase, capacity, row_offset, row_counts, stage_ids,
+                            pair_counts, pair_ids) == cudaSuccess
+             ? ANEMOI_SM100_OK
+             : ANEMOI_SM100_ELAUNCH;
+}
+
 // Q64 query blocks 2t and 2t+1 of a head run as one CTA of the attention kernel (rows 0-63 and
 // 64-127 of the 128-row MMA shape).  That CTA walks, phase by phase, the union of the two
 // blocks' lists; bits 30 and 31 of an entry say which of the two blocks the stage belongs to.
@@ -591,6 +1016,10 @@ __global__ void __launch_bounds__(1024) pair_order_kernel(int pairs, int32_t* pa
 }
 
 }  // namespace
+
+bool layer::routes_pairs(const anemoi_sm100_shape& s) {
+  return fused_fits(s.heads, s.video_blocks) && rec::stages(s) < (1 << 30);
+}
 
 extern "C" int64_t anemoi_sm100_route_anchored_scratch_bytes(const anemoi_sm100_shape* shape) {
   if (rec::validate_shape(shape) != ANEMOI_SM100_OK) return ANEMOI_SM100_EINVAL;
@@ -698,6 +1127,9 @@ extern "C" int anemoi_sm100_route(const anemoi_sm100_shape* shape, const void* p
     return ANEMOI_SM100_EINVAL;
   if (R > 65535 || items * H >= (1ll << 40)) return ANEMOI_SM100_ELIMIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (fused_fits(H, R))
+    return launch_fused<false>(*shape, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids,
+                               list_capacity, nullptr, nullptr, st);
   RouteScratch sc;
   sc.hist = static_cast<int*>(scratch);
   sc.thr = sc.hist + (int64_t)H * kBins;
@@ -724,6 +1156,25 @@ extern "C" int anemoi_sm100_route(const anemoi_sm100_shape* shape, const void* p
                                                prefix_phase, list_capacity, row_offset, row_counts,
                                                stage_ids);
   return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
+}
+
+extern "C" int anemoi_sm100_route_pairs(const anemoi_sm100_shape* shape, const void* probability, int64_t n16,
+                                        int64_t n8, int64_t n4, int prefix_phase, int32_t* row_offset,
+                                        int32_t* row_counts, int32_t* pair_counts, int32_t* pair_ids,
+                                        int64_t list_capacity, void* stream) {
+  if (rec::validate_shape(shape) != ANEMOI_SM100_OK || !probability || !row_offset || !row_counts ||
+      !pair_counts || !pair_ids || shape->query_block != 64)
+    return ANEMOI_SM100_EINVAL;
+  const int64_t items = (int64_t)shape->video_blocks * shape->video_blocks;
+  if (n16 < 0 || n8 < 0 || n4 < 0 || n16 + n8 + n4 > items || n16 + n8 + n4 <= 0)
+    return ANEMOI_SM100_EINVAL;
+  if (prefix_phase < -1 || prefix_phase > 2) return ANEMOI_SM100_EINVAL;
+  if (prefix_phase >= 0 && shape->prefix_tokens == 0) prefix_phase = -1;
+  if (list_capacity < anemoi_sm100_route_list_capacity(shape, n16, n8, n4, prefix_phase))
+    return ANEMOI_SM100_EINVAL;
+  if (!fused_fits(shape->heads, shape->video_blocks) || rec::stages(*shape) >= (1 << 30)) return ANEMOI_SM100_ELIMIT;
+  return launch_fused<true>(*shape, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, nullptr,
+                            list_capacity, pair_counts, pair_ids, static_cast<cudaStream_t>(stream));
 }
 
 // ------------------------------------------------------------------------------------------

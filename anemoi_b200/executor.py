@@ -12,6 +12,7 @@ draft map, no diag-Jensen term, no anchors, no MXFP8 cell.
 
 from __future__ import annotations
 
+import ctypes as C
 import math
 from functools import lru_cache
 
@@ -98,7 +99,10 @@ class _Stage:
 
 @lru_cache(maxsize=8)
 def _prefix_stream(device: torch.device) -> torch.cuda.Stream:
-    return torch.cuda.Stream(device=device)
+    # High priority: the prefix rows' CTAs walk every stage and are the longest of a call, so they go
+    # first wherever an SM has room (launched with the video CTAs of a 9 ms call they would else start
+    # behind them; 1 % of the call).
+    return torch.cuda.Stream(device=device, priority=-1)
 
 
 @lru_cache(maxsize=64)
@@ -211,6 +215,10 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
     ):
         raise ValueError("video_shape must match the post-prefix token count")
 
+    if not (return_parts or nvtx or diag_jensen or enable_anchors or _STAGE_EVENTS is not None):
+        return _one_call(q_bshd, k_bshd, v_bshd, prefix_tokens, float(sparsity_ratio), float(retained_nvfp4_ratio),
+                         float(retained_int8_ratio), float(retained_fp16_ratio), video_shape, query_block_size,
+                         prefix_kv_precision, prefix_query_precision, float(maxpool_weight), nvfp4_scales)
     device = q_bshd.device
     video = video_phases(retained_nvfp4_ratio, retained_int8_ratio, retained_fp16_ratio)
     if prefix_query_precision not in ("int8", "fp16"):
@@ -285,6 +293,88 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
         return out, dict(shape=shape, store=store, prob=prob, lists=lists, packed=packed,
                          prefix_out=prefix_out, valid_k=valid_k, budgets=(n16, n8, n4),
                          layout=layout, status=status)
+    return out
+
+
+class _Plan:
+    """The native plan of one configuration with the tensors it points to."""
+
+    def __init__(self, device, tokens, heads, dim, dtype, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape,
+                 query_block, prefix_kv, prefix_query, maxpool_weight, pair_q64):
+        video = video_phases(nvfp4, int8, fp16)
+        if prefix_query not in ("int8", "fp16"):
+            raise ValueError("prefix_query_precision must be int8 or fp16")
+        self.native_prefix = prefix_tokens > 0 and prefix_query == "int8" and "int8" in video
+        active, prefix_phase = resolve_phases(video, prefix_tokens, prefix_kv)
+        frames, height, width = video_shape
+        self.layout = materialize_ragged_2d_layout(device, frames=frames, height=height, width=width,
+                                                   logical_block=query_block)
+        blocks = self.layout.video_blocks
+        self.valid_k = _valid_k(device, prefix_tokens, query_block, _counts_key(self.layout))
+        self.status = _status_word(device)
+        n16, n8, n4 = route_counts(blocks * blocks, sparsity_ratio=sparsity, nvfp4_ratio=nvfp4, int8_ratio=int8,
+                                   fp16_ratio=fp16)
+        shape = native.Shape(
+            heads=heads, head_dim=dim, query_block=query_block, seq_tokens=tokens, prefix_tokens=prefix_tokens,
+            video_blocks=blocks, has_nvfp4=int("nvfp4" in active), has_int8=int("int8" in active),
+            has_fp16=int("fp16" in active), has_prefix_query_int8=int(self.native_prefix),
+            has_maxpool=int(maxpool_weight != 0.0), input_is_bf16=int(dtype == torch.bfloat16),
+            q_global_scale=1.0, k_global_scale=1.0, v_global_scale=1.0)
+        lib = native.library()
+        phase = -1 if prefix_phase is None else PHASE_ORDER.index(prefix_phase)
+        capacity = max(1, int(lib.anemoi_sm100_route_list_capacity(C.byref(shape), n16, n8, n4, phase)))
+        self.struct = native.LayerPlan(
+            shape=shape, indices=self.layout.indices.data_ptr(), counts=self.layout.counts.data_ptr(),
+            valid_k=self.valid_k.data_ptr(), status=self.status.data_ptr(), n16=n16, n8=n8, n4=n4,
+            list_capacity=capacity, prefix_phase=phase, pair_q64=int(pair_q64), maxpool_weight=maxpool_weight)
+        self.ref = C.byref(self.struct)
+        self.bytes = int(lib.anemoi_sm100_layer_workspace_bytes(self.ref))
+        if self.bytes < 0:
+            raise RuntimeError("invalid attention shape")
+        self.side = _prefix_stream(device) if prefix_tokens else None
+        self.side_handle = self.side.cuda_stream if prefix_tokens else None
+        self.uses_scales = "nvfp4" in active
+        # kernels per call: V amax, preparation, draft, routing (and pair lists), attention, prefix rows
+        self.launches = 4 + int("int8" in active) + int(prefix_tokens > 0)
+        if not lib.anemoi_sm100_routes_in_one_kernel(C.byref(shape)):
+            self.launches += 4 + 2 * int(pair_q64 and query_block == 64)
+        self.call = lib.anemoi_sm100_layer
+
+
+# One entry per configuration a process uses (a few hundred bytes each; the tables are the layout's).
+_plan = lru_cache(maxsize=256)(_Plan)
+_Strides, _Scales = C.c_int64 * 6, C.c_float * 3
+
+
+def _one_call(q, k, v, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape, query_block, prefix_kv, prefix_query,
+              maxpool_weight, nvfp4_scales):
+    """The whole call through ``anemoi_sm100_layer``: one workspace, one native function."""
+    device, dtype = q.device, q.dtype
+    _, tokens, heads, dim = q.shape
+    plan = _plan(device, tokens, heads, dim, dtype, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape, query_block,
+                 prefix_kv, prefix_query, maxpool_weight, _PAIR_Q64)
+    current = torch.cuda.current_stream(device)
+    prefix_out, prefix_ptr, prefix_rows = None, None, 0
+    if prefix_tokens and not plan.native_prefix:
+        # dense attention of the prefix rows on the caller's tensors, as the reference does
+        plan.side.wait_stream(current)
+        with torch.cuda.stream(plan.side):
+            prefix_out = F.scaled_dot_product_attention(
+                q[:, :prefix_tokens].permute(0, 2, 1, 3), k.permute(0, 2, 1, 3), v.permute(0, 2, 1, 3),
+                dropout_p=0.0, is_causal=False)[0].contiguous()
+        prefix_ptr, prefix_rows = prefix_out.data_ptr(), prefix_tokens
+    workspace = torch.empty(plan.bytes, dtype=torch.uint8, device=device)
+    out = torch.empty((1, tokens, heads, dim), dtype=dtype, device=device)
+    code = plan.call(
+        plan.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(),
+        _Strides(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2)),
+        _Scales(*nvfp4_scales) if plan.uses_scales else None, prefix_ptr, prefix_rows, 1, out.data_ptr(),
+        workspace.data_ptr(), plan.bytes, current.cuda_stream, plan.side_handle)
+    if code != 0:
+        native._check(code, "anemoi_sm100_layer")
+    native._count("layer", plan.launches)
+    if prefix_out is not None:
+        prefix_out.record_stream(current)
     return out
 
 

@@ -69,6 +69,15 @@ class Operands(C.Structure):
         "k_int8_scale", "v_e4m3_scale", "v_amax", "q_pool", "k_pool", "q_max_pool", "k_max_pool")]
 
 
+class LayerPlan(C.Structure):
+    """What calls of one configuration share (``anemoi_sm100_layer_plan``)."""
+
+    _fields_ = [("shape", Shape), ("indices", C.c_void_p), ("counts", C.c_void_p), ("valid_k", C.c_void_p),
+                ("status", C.c_void_p), ("n16", C.c_int64), ("n8", C.c_int64), ("n4", C.c_int64),
+                ("list_capacity", C.c_int64), ("prefix_phase", C.c_int32), ("pair_q64", C.c_int32),
+                ("maxpool_weight", C.c_float)]
+
+
 @lru_cache(maxsize=1)
 def library() -> C.CDLL:
     """Load the in-tree shared library; raise if it has not been built."""
@@ -98,6 +107,11 @@ def library() -> C.CDLL:
         "anemoi_sm100_attention_pairs": (C.c_int, [SP, OP, P, P, P, P, I64, P, P, P, P]),
         "anemoi_sm100_pair_lists": (C.c_int, [SP, P, P, P, I64, P, P, P]),
         "anemoi_sm100_prefix_attention": (C.c_int, [SP, OP, P, P, P, P]),
+        "anemoi_sm100_route_pairs": (C.c_int, [SP, P, I64, I64, I64, C.c_int, P, P, P, P, I64, P]),
+        "anemoi_sm100_routes_in_one_kernel": (C.c_int, [SP]),
+        "anemoi_sm100_layer_workspace_bytes": (I64, [C.POINTER(LayerPlan)]),
+        "anemoi_sm100_layer": (C.c_int, [C.POINTER(LayerPlan), P, P, P, C.POINTER(I64), C.POINTER(F), P, I64, C.c_int,
+                                         P, P, I64, P, P]),
         "anemoi_sm100_copy_rows": (C.c_int, [P, I64, P, I64, I64, I64, I32, P]),
         "anemoi_sm100_peer_alloc": (C.c_int, [I64, C.POINTER(P), P]),
         "anemoi_sm100_peer_open": (C.c_int, [P, C.POINTER(P)]),
@@ -137,7 +151,8 @@ EXPORTED = (
     "anemoi_sm100_draft_probability", "anemoi_sm100_draft_probability_jensen", "anemoi_sm100_route_scratch_bytes",
     "anemoi_sm100_route_list_capacity", "anemoi_sm100_route", "anemoi_sm100_route_static",
     "anemoi_sm100_route_static_max_bytes", "anemoi_sm100_attention",
-    "anemoi_sm100_attention_pairs", "anemoi_sm100_pair_lists",
+    "anemoi_sm100_attention_pairs", "anemoi_sm100_pair_lists", "anemoi_sm100_route_pairs",
+    "anemoi_sm100_layer", "anemoi_sm100_layer_workspace_bytes", "anemoi_sm100_routes_in_one_kernel",
     "anemoi_sm100_route_anchored", "anemoi_sm100_route_anchored_scratch_bytes",
     "anemoi_sm100_prefix_attention", "anemoi_sm100_assemble", "anemoi_sm100_pack_qkv",
     "anemoi_sm100_merge_heads", "anemoi_sm100_pack_qkv_heads", "anemoi_sm100_merge_heads_into",
@@ -273,7 +288,8 @@ def route(shape: Shape, prob: torch.Tensor, n16: int, n8: int, n4: int, prefix_p
         stage_ids=torch.empty((h, max(cap, 1)), dtype=torch.int32, device=dev),
         capacity=max(cap, 1),
     )
-    _count("route", 5)                                  # hist, threshold, rowstat, headscan, emit
+    # one kernel, or hist, threshold, rowstat, headscan, emit
+    _count("route", 1 if lib.anemoi_sm100_routes_in_one_kernel(C.byref(shape)) else 5)
     _check(lib.anemoi_sm100_route(C.byref(shape), _ptr(prob), n16, n8, n4, prefix_phase,
                                   _ptr(scratch), scratch.numel(), _ptr(lists.row_offset),
                                   _ptr(lists.row_counts), _ptr(lists.stage_ids), lists.capacity,

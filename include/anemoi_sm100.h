@@ -219,6 +219,15 @@ int anemoi_sm100_pair_lists(const anemoi_sm100_shape* shape, const int32_t* row_
                             const int32_t* row_counts, const int32_t* stage_ids,
                             int64_t list_capacity, int32_t* pair_counts, int32_t* pair_ids,
                             void* stream);
+/* 1 if anemoi_sm100_route runs as one kernel for this shape (five otherwise), 0 if not. */
+int anemoi_sm100_routes_in_one_kernel(const anemoi_sm100_shape* shape);
+/* Routing and pair lists in one kernel (no lists of single blocks): row_offset and row_counts as from
+ * anemoi_sm100_route (launch order 0), pair_counts and pair_ids as from pair_lists.
+ * ANEMOI_SM100_ELIMIT where the one-kernel routing does not apply: use the two functions. */
+int anemoi_sm100_route_pairs(const anemoi_sm100_shape* shape, const void* probability, int64_t n16,
+                             int64_t n8, int64_t n4, int prefix_phase, int32_t* row_offset,
+                             int32_t* row_counts, int32_t* pair_counts, int32_t* pair_ids,
+                             int64_t list_capacity, void* stream);
 int anemoi_sm100_attention_pairs(const anemoi_sm100_shape* shape, const anemoi_sm100_operands* ops,
                                  const int32_t* row_offset, const int32_t* row_counts,
                                  const int32_t* pair_counts, const int32_t* pair_ids,
@@ -232,6 +241,42 @@ int anemoi_sm100_attention_pairs(const anemoi_sm100_shape* shape, const anemoi_s
 int anemoi_sm100_prefix_attention(const anemoi_sm100_shape* shape,
                                   const anemoi_sm100_operands* ops, const int32_t* valid_k,
                                   void* out_prefix, int32_t* status, void* stream);
+
+/* One whole call, from raw Q/K/V to the output in token order: prepare, draft_probability, route (and
+ * pair_lists), attention and the prefix rows, with the attention's results written straight to their
+ * tokens.  A plan holds what calls of one configuration share; the tables stay the caller's.
+ *   indices, counts  slot tables of the layout (as for anemoi_sm100_prepare)
+ *   valid_k          real keys per stage; status: the device's sticky status word
+ *   n16, n8, n4      budgets per head; prefix_phase -1 / 0 / 1 / 2 as for anemoi_sm100_route
+ *   list_capacity    anemoi_sm100_route_list_capacity() of the plan
+ *   pair_q64         Q64: two query blocks per CTA */
+typedef struct anemoi_sm100_layer_plan {
+  anemoi_sm100_shape shape;
+  const int32_t* indices;
+  const int32_t* counts;
+  const int32_t* valid_k;
+  int32_t* status;
+  int64_t n16, n8, n4;
+  int64_t list_capacity;
+  int32_t prefix_phase;
+  int32_t pair_q64;
+  float maxpool_weight;
+} anemoi_sm100_layer_plan;
+
+int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan);
+/*   strides          as for anemoi_sm100_prepare
+ *   nvfp4_scales     q, k, v tensor-level scales of this call, or null for the plan's
+ *   prefix_out       prefix rows computed elsewhere on `side_stream` ([H][prefix_rows][D], the caller's
+ *                    dtype if prefix_is_caller_dtype); null with has_prefix_query_int8 or without a prefix
+ *   out              [S][H][D] contiguous, the input's dtype
+ *   workspace        anemoi_sm100_layer_workspace_bytes() bytes, 256-byte aligned, free for reuse on
+ *                    `stream` when the call returns
+ *   side_stream      runs beside `stream` and is joined before the call's work ends (with a prefix)
+ * Counterpart of sm120_ragged_h3_attention (anemoi/layers/attention/mpa/executor.py:876-1224). */
+int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const void* q, const void* k, const void* v,
+                       const int64_t* strides, const float* nvfp4_scales, const void* prefix_out,
+                       int64_t prefix_rows, int prefix_is_caller_dtype, void* out, void* workspace,
+                       int64_t workspace_bytes, void* stream, void* side_stream);
 
 /* Inverse scatter into [1,S,H,D] of the caller's dtype: prefix rows from
  * `prefix_out` ([H][rows][D], fp16 if prefix_is_caller_dtype == 0 else the
