@@ -22,43 +22,71 @@
 
 namespace {
 
-// One row (token, head) per group of D/8 consecutive lanes; 8 channels per thread.
-template <typename T, int D>
-__global__ void __launch_bounds__(256) qknorm_rope_kernel(T* x, const T* weight, const float* cos_table,
-                                                          const float* sin_table, int64_t rows,
-                                                          int heads, int rotary_dim, float eps,
-                                                          int64_t token_stride, int64_t head_stride) {
+// A group of D/8 consecutive lanes takes kRows heads of one token, 8 channels per thread.  HBM bound
+// (read + write of x), which takes loads in flight: with one row per group (a 16-byte load per
+// thread, then the whole arithmetic) 33,272 tokens x 56 heads x 128 took 289 us = 3.3 TB/s.  Four rows
+// give four loads in flight, one read of the token's cos / sin entries and of the weights for all four,
+// and the square root and division of a row, which every lane of the group used to repeat, are
+// done once, by lane i for row i: 180 us = 5.3 TB/s, at 64 registers (80 registers, three CTAs per SM:
+// 218 us; two rows: 206; eight: 321).  One row per group where a token has no more than two heads.
+template <typename T, int D, int kRows>
+__global__ void __launch_bounds__(256, 4) qknorm_rope_kernel(T* x, const T* weight, const float* cos_table,
+                                                             const float* sin_table, uint32_t units, int quads,
+                                                             int heads, int rotary_dim, float eps,
+                                                             int64_t token_stride, int64_t head_stride) {
   constexpr int kLanes = D / 8;
-  const int64_t row = ((int64_t)blockIdx.x * 256 + threadIdx.x) / kLanes;
+  const uint32_t unit = (blockIdx.x * 256u + threadIdx.x) / kLanes;
   const int lane = threadIdx.x % kLanes;
-  const bool live = row < rows;
-  // rows < 2^31 (checked by the launcher): 32-bit division
-  const uint32_t r32 = live ? (uint32_t)row : 0u;
-  const int64_t token = r32 / (uint32_t)heads;
-  const int head = (int)(r32 - (uint32_t)token * (uint32_t)heads);
-  T* p = x + token * token_stride + (int64_t)head * head_stride + lane * 8;
-  uint4 raw = make_uint4(0, 0, 0, 0);
-  if (live) raw = *reinterpret_cast<const uint4*>(p);
-  const uint4 out = nr::norm_rope8<T, D>(raw, weight, cos_table + token * rotary_dim,
-                                         sin_table + token * rotary_dim, rotary_dim, eps, lane, live);
-  if (live) *reinterpret_cast<uint4*>(p) = out;
+  const bool in = unit < units;
+  const uint32_t token = in ? unit / (uint32_t)quads : 0u;
+  const int head0 = in ? (int)(unit - token * (uint32_t)quads) * kRows : 0;
+  T* p = x + (int64_t)token * token_stride + (int64_t)head0 * head_stride + lane * 8;
+  uint4 raw[kRows];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    raw[i] = make_uint4(0, 0, 0, 0);
+    if (in && head0 + i < heads) raw[i] = *reinterpret_cast<const uint4*>(p + i * head_stride);
+  }
+  const nr::Rotary rot(lane, rotary_dim);
+  float cs[8], sn[8];
+  if (rot.in && in)
+    nr::load_tables(cos_table + (int64_t)token * rotary_dim, sin_table + (int64_t)token * rotary_dim, lane, cs, sn);
+  const uint4 wraw = __ldg(reinterpret_cast<const uint4*>(weight + lane * 8));
+  float mine = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const float sum = nr::square_sum<T, D>(raw[i]);
+    if ((lane & (kRows - 1)) == i) mine = sum;
+  }
+  const float r_mine = nr::inverse_rms<D>(mine, eps);
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const float r = __shfl_sync(0xffffffffu, r_mine, i, kLanes);
+    const uint4 out = nr::norm_rope_row<T, D>(raw[i], wraw, r, rot, cs, sn);
+    if (in && head0 + i < heads) *reinterpret_cast<uint4*>(p + i * head_stride) = out;
+  }
+}
+
+template <typename T, int D, int kRows>
+int launch_rows(void* x, const void* weight, const float* c, const float* s, int64_t tokens, int heads, int rotary,
+                float eps, const int64_t* strides, cudaStream_t st) {
+  const int64_t quads = (heads + kRows - 1) / kRows, units = tokens * quads;
+  constexpr int64_t kUnits = 256 / (D / 8);
+  if (tokens * heads > 0x7fffffffLL) return ANEMOI_SM100_ELIMIT;
+  qknorm_rope_kernel<T, D, kRows><<<(unsigned)((units + kUnits - 1) / kUnits), 256, 0, st>>>(
+      static_cast<T*>(x), static_cast<const T*>(weight), c, s, (uint32_t)units, (int)quads, heads, rotary, eps,
+      strides[0], strides[1]);
+  return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
 }
 
 template <typename T>
 int launch(void* x, const void* weight, const float* c, const float* s, int64_t tokens, int heads, int d,
            int rotary, float eps, const int64_t* strides, cudaStream_t st) {
-  const int64_t rows = tokens * heads;
-  const int64_t rows_per_block = 256 / (d / 8);
-  const int64_t blocks = (rows + rows_per_block - 1) / rows_per_block;
-  if (blocks > 0x7fffffffLL || rows > 0x7fffffffLL) return ANEMOI_SM100_ELIMIT;
-  if (d == 64) {
-    qknorm_rope_kernel<T, 64><<<(unsigned)blocks, 256, 0, st>>>(static_cast<T*>(x), static_cast<const T*>(weight),
-                                                                c, s, rows, heads, rotary, eps, strides[0], strides[1]);
-  } else {
-    qknorm_rope_kernel<T, 128><<<(unsigned)blocks, 256, 0, st>>>(static_cast<T*>(x), static_cast<const T*>(weight),
-                                                                 c, s, rows, heads, rotary, eps, strides[0], strides[1]);
-  }
-  return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
+  if (d == 64)
+    return heads > 2 ? launch_rows<T, 64, 4>(x, weight, c, s, tokens, heads, rotary, eps, strides, st)
+                     : launch_rows<T, 64, 1>(x, weight, c, s, tokens, heads, rotary, eps, strides, st);
+  return heads > 2 ? launch_rows<T, 128, 4>(x, weight, c, s, tokens, heads, rotary, eps, strides, st)
+                   : launch_rows<T, 128, 1>(x, weight, c, s, tokens, heads, rotary, eps, strides, st);
 }
 
 }  // namespace

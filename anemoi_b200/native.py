@@ -628,11 +628,13 @@ def qknorm_rope_(x: torch.Tensor, weight: torch.Tensor, cos: torch.Tensor, sin: 
         raise ValueError("weight must be a contiguous [D] tensor of x's dtype")
     if cos.shape != sin.shape or cos.ndim != 2 or cos.size(0) != tokens:
         raise ValueError("cos and sin must be [tokens, rotary_dim]")
-    cos = cos.to(device=x.device, dtype=torch.float32).contiguous()
-    sin = sin.to(device=x.device, dtype=torch.float32).contiguous()
-    strides = (C.c_int64 * 2)(x.stride(0), x.stride(1))
-    _check(library().anemoi_sm100_qknorm_rope(_ptr(x), _ptr(weight), _ptr(cos), _ptr(sin), tokens, heads, d,
-                                              cos.size(1), float(eps), int(x.dtype == torch.bfloat16),
-                                              strides, _stream(x.device)),
+    if cos.dtype != torch.float32 or cos.device != x.device or not cos.is_contiguous():
+        cos = cos.to(device=x.device, dtype=torch.float32).contiguous()
+    if sin.dtype != torch.float32 or sin.device != x.device or not sin.is_contiguous():
+        sin = sin.to(device=x.device, dtype=torch.float32).contiguous()
+    _check(library().anemoi_sm100_qknorm_rope(
+        x.data_ptr(), weight.data_ptr(), cos.data_ptr(), sin.data_ptr(), tokens, heads, d, cos.size(1), float(eps),
+        int(x.dtype == torch.bfloat16), (C.c_int64 * 2)(x.stride(0), x.stride(1)),
+        torch.cuda.current_stream(x.device).cuda_stream),
            "anemoi_sm100_qknorm_rope")
     return x

@@ -33,7 +33,9 @@ def fused_qknorm_rope(x: torch.Tensor, weight: torch.Tensor, cos: torch.Tensor, 
     for b in range(batch):
         c = cos[b] if cos.ndim == 3 else cos
         s = sin[b] if sin.ndim == 3 else sin
-        native.qknorm_rope_(x[b], weight, c.reshape(seq, rotary_dim), s.reshape(seq, rotary_dim), eps)
+        if c.ndim != 2 or s.ndim != 2 or s.shape != c.shape:
+            c, s = c.reshape(seq, rotary_dim), s.reshape(seq, rotary_dim)
+        native.qknorm_rope_(x[b], weight, c, s, eps)
     return x
 
 
