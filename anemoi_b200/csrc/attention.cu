@@ -8,14 +8,15 @@
 //   warps 0-3, 4-7  softmax of the even and of the odd stages: warp w owns TMEM lanes 32*(w%4)..
 //                   (query rows), one thread per row with the row's 64 scores in registers
 //   warps 8-11      rescale of O: when a stage moved some row's maximum, or at a phase change
-//                   (where O also moves between the phases' value domains)
+//                   (where O also moves between the phases' value domains); they also move the
+//                   FP16 phase's Q into tensor memory
 //   warp 12         loader: one lane issues 1-D bulk copies (TMA engine) of the Q record of each
 //                   phase and of one K|V record per stage into a ring of shared-memory slots
 //   warp 13         S[128x64]  = Q K^T   kind::mxf4nvf4 / kind::i8 / kind::f16
 //   warp 14         O[128xD]  += P V     kind::mxf4nvf4 / kind::f8f6f4 / kind::f16
 //   warp 15         idle
-// TMEM columns: S0 [0,64), O [64,64+D), a second score buffer S1 and the NVFP4 scale factors
-// (which share [192,256) at D = 128: the NVFP4 phase then has one score buffer).
+// TMEM columns: S0 [0,64), O [64,64+D), and at [192,256) the NVFP4 scale factors, the FP16 phase's Q
+// or (INT8 at D = 128) a second score buffer S1; D = 64 has S1 behind O in every phase.
 //
 // Why this split.  A stage needs 8,192 exponentials = 512 cycles of the special-function unit and
 // 130-580 cycles of the tensor core per SM, but one warp's chain through a stage (wait for S, load
@@ -27,10 +28,10 @@
 // and the exponentials of two stages overlap.  O's rescale, which waits for the previous PV, is
 // off the softmax warps' path; QK and PV are issued by different warps so that QK of a stage waits
 // for nothing but its key tile and its score buffer.
-// Measured per stage and SM at D = 128, cycles, before -> now: NVFP4 1,282 -> 811, INT8 1,394 -> 853,
-// FP16 1,332 -> 1,170, the mixed layer of S = 85,184 (8 heads) 1,250 -> 943 (6.55 -> 4.94 ms).
-// Now bound by instruction issue (about 600 warp instructions per stage and scheduler) and the
-// special-function unit; FP16 by its 32 KB per stage, of which two stages and a half fit in a ring.
+// Measured per stage and SM at D = 128, cycles, with one softmax warpgroup -> now: NVFP4 1,282 -> 791,
+// INT8 1,394 -> 857, FP16 1,332 -> 1,050, the mixed layer of S = 85,184 (8 heads) 1,250 -> 900.  Now bound
+// by the special-function unit (66 % busy: 520 of INT8's cycles) and the waits around it; FP16 by
+// shared memory, which moves 96 KB = 768 cycles' worth per stage, and, in long runs, by the power limit.
 //
 // P is stored over the stage's K tile, which the tensor core has finished reading when the scores
 // arrive; that leaves the ring all of the shared memory that Q does not take.
@@ -62,9 +63,17 @@ using layer::TokenRows;
 // Four warpgroups: softmax of the even stages, softmax of the odd stages, rescale of O, and
 // loader / QK / PV (one warp each, the fourth idle).
 constexpr int kThreads = 512;
-constexpr int kSoftmaxRegs = 88;  // 128 * (2 * 88 + 48 + 32) == 512 * 64 (two CTAs per SM)
-constexpr int kCorrRegs = 48;
+// Registers per thread: 128 * (2 * softmax + rescale + other) == 512 * 64 (two CTAs per SM).  With 96 a
+// softmax thread spills nothing, but rescales then go 16 columns at a time.  That is the better
+// trade at D = 64 (where O is half as wide: the mixed Q64 kernel 834 -> 778 cycles per stage, FP16
+// 930 -> 846) and for NVFP4 (821 -> 796); at D = 128 FP16 and mixed lose (1,005 -> 1,071, 863 -> 899).
 constexpr int kOtherRegs = 32;
+template <int D, int CELLS>
+struct Regs {
+  static constexpr bool kWide = D == 64 || CELLS == 0;
+  static constexpr int kSoftmax = kWide ? 96 : 88, kRescale = kWide ? 32 : 48;
+  static constexpr int kRescaleColumns = kWide ? 16 : 32;
+};
 constexpr int kCorrWarp = 8;
 constexpr int kLoaderWarp = 12;
 constexpr int kQkWarp = 13;
@@ -73,11 +82,13 @@ enum WaitRole : int { kSoftmaxRole = 0, kRescaleRole = 1, kMmaRole = 2 };
 constexpr int kTmemCols = 256;
 constexpr int kColS = 0;
 constexpr int kColO = 64;
+constexpr int kColQ = 192;     // FP16: D / 2 columns
 constexpr int kColSfaQ = 192;  // 2 k-steps x 4 columns
 constexpr int kColSfbK = 200;  // 2 k-steps x 4 columns
 constexpr int kColSfaP = 208;
 constexpr int kColSfbV = 212;
 constexpr int kRing = 8;       // entries of the per-stage rings, and the most key/value slots
+constexpr int kSplitKeys = 4, kSplitValues = 2;  // key and value buffers of phases that keep them apart
 constexpr float kFp8Offset = 8.807f;
 constexpr uint64_t kDrainNs = 100000000;  // limit of the waits for copies and MMAs in flight after a give-up
 
@@ -127,7 +138,8 @@ struct Shared {
   uint64_t pv_done[kRing];    // PV complete: slot free, O may be touched
   uint64_t p_full[kRing];     // per quadrant: P stored (softmax warp), O in the right scale (rescale warp)
   uint64_t m_full[4][kRing];  // running maxima of the quadrant's rows up to this stage published
-  uint64_t v_full;            // value tile landed (phases whose key and value tiles have rings of their own)
+  uint64_t v_full[kSplitValues];  // value tile landed (phases with buffers of their own for keys and values)
+  uint64_t q_moved;               // FP16: Q in tensor memory
   uint64_t q_full, q_free;
   uint64_t s_full[2];  // scores ready, per softmax warpgroup (a waiter has to see every phase)
   uint64_t s_free[2];  // scores read, per score buffer
@@ -216,6 +228,11 @@ __device__ __forceinline__ void tmem_st4(uint32_t taddr, uint32_t v) {
                "r"(v), "r"(v), "r"(v)
                : "memory");
 }
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -248,49 +265,72 @@ __host__ __device__ constexpr int rest_offset(int d, int cell) {
 __host__ __device__ constexpr int slot_bytes(int d, int cell) {
   return (rest_offset(d, cell) + record_bytes(d, cell) - k_bytes(d, cell) + 127) & ~127;
 }
-// FP16 at D = 128: two whole slots of 32 KB would fit, but a slot is held from the start of its
-// copy to the end of its PV.  Key tiles (which P replaces) get three buffers and values one: the
-// value copy of stage g + 1 runs while stage g + 1's probabilities are computed.
+// FP16: Q is an operand in tensor memory, moved there from its region at the start of the phase.  As
+// a shared-memory operand a stage of D = 128 read 48 KB for QK alone (48 cycles of shared-memory
+// bandwidth per instruction of 36) and moved 128 KB = 1,024 cycles in all, which was the bound.
+// At D = 128 Q's 32 KB then serve keys and values, in buffers of their own: four for key tiles, held until
+// PV (P replaces them), and two for value tiles, which are not needed before the probabilities are there.
 __host__ __device__ constexpr bool split_kv(int d, int cell) { return d == 128 && cell == kF16; }
 __host__ __device__ constexpr int stage_bytes(int d, int cell) {  // distance of two slots
-  return split_kv(d, cell) ? rest_offset(d, cell) : slot_bytes(d, cell);
+  return split_kv(d, cell) ? k_bytes(d, cell) : slot_bytes(d, cell);
 }
+// The first two key buffers lie in Q's region and are filled last, once Q has moved.
+__host__ __device__ constexpr int first_slot(int d, int cell) { return split_kv(d, cell) ? 2 : 0; }
 __host__ __device__ constexpr int slot_count(int ring, int d, int cell) {
-  const int n = split_kv(d, cell) ? ring / rest_offset(d, cell) - 1 : ring / slot_bytes(d, cell);
+  const int n = split_kv(d, cell) ? kSplitKeys : ring / slot_bytes(d, cell);
   return n < kRing ? n : kRing;
 }
-// Score buffer of stage g: the NVFP4 phase of D = 128 has a single one (the other's columns
-// hold its scale factors).
+// Score buffer of stage g: the NVFP4 and FP16 phases of D = 128 have a single one (the other's
+// columns hold the scale factors or Q).
 template <int D>
 __device__ __forceinline__ int s_buffer(int cell, int g) {
-  return D == 128 && cell == kNv ? 0 : (g & 1);
+  return D == 128 && cell != kI8 ? 0 : (g & 1);
 }
 
-// O[row][c] *= alpha (* colf[c] when given) for all D columns of the thread's row.
-template <int D>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[32]) { tmem_st32(taddr, r); }
+__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
+          taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
+// O[row][c] *= alpha (* colf[c] when given) for all D columns of the thread's row, kCols at a time.
+template <int D, int kCols>
 __device__ __forceinline__ void rescale_o(uint32_t tmem_row, float alpha, const float* colf) {
   const float2 alpha2 = make_float2(alpha, alpha);
 #pragma unroll 1
-  for (int c0 = 0; c0 < D; c0 += 32) {
-    uint32_t r[32];
-    tmem_ld32(tmem_row + kColO + c0, r);
+  for (int c0 = 0; c0 < D; c0 += kCols) {
+    uint32_t r[kCols];
+    tmem_ld(tmem_row + kColO + c0, r);
     tmem_wait_ld();
 #pragma unroll
-    for (int j = 0; j < 32; j += 2) {
+    for (int j = 0; j < kCols; j += 2) {
       const float2 v = fmul2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), alpha2);
       r[j] = __float_as_uint(v.x);
       r[j + 1] = __float_as_uint(v.y);
     }
     if (colf != nullptr) {
 #pragma unroll
-      for (int j = 0; j < 32; j += 2) {
+      for (int j = 0; j < kCols; j += 2) {
         const float2 v = fmul2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])),
                                *reinterpret_cast<const float2*>(colf + c0 + j));
         r[j] = __float_as_uint(v.x);
         r[j + 1] = __float_as_uint(v.y);
       }
     }
-    tmem_st32(tmem_row + kColO + c0, r);
+    tmem_st(tmem_row + kColO + c0, r);
   }
   tmem_wait_st();
 }
@@ -338,8 +378,8 @@ __device__ __forceinline__ float exp_store(const float (&s)[64], float scale, fl
 }
 
 // State of a softmax row.  The two softmax warpgroups alternate stages; the running maximum and
-// the denominator travel between them through Shared::rec.  The denominator is carried two stages
-// late, so that a group waits for nothing but the other's maximum: entry g holds m(g) and d(g - 2),
+// the denominator travel between them through shared memory.  The denominator is carried two stages
+// late, so that a group waits for nothing but the other's maximum: stage g publishes m(g) and d(g - 2),
 // and d(g) = d(g - 1) * alpha(g) + sum(g) is formed by the group that ran stage g when it publishes
 // stage g + 2 - the order (and rounding) of a strictly sequential walk.
 struct SoftmaxWalk {
@@ -452,9 +492,9 @@ __device__ __forceinline__ void issue_qk(uint32_t tmem_s, uint32_t tmem, uint32_
   if (CELL == kF16) {
     constexpr uint32_t chunks = D / 8;
     constexpr uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, 64, 0, 0);
-    const uint64_t qd = smem_desc(q_addr, 128, chunks * 128), kd = smem_desc(slot_addr, 128, chunks * 128);
+    const uint64_t kd = smem_desc(slot_addr, 128, chunks * 128);
 #pragma unroll
-    for (int k = 0; k < D / 16; ++k) mma_f16_ss(tmem_s, qd + k * 16, kd + k * 16, idesc, k > 0);
+    for (int k = 0; k < D / 16; ++k) mma_f16_ts(tmem_s, tmem + kColQ + k * 8, kd + k * 16, idesc, k > 0);
   } else if (CELL == kI8) {
     constexpr uint32_t chunks = D / 16;
     constexpr uint32_t idesc = instr_desc(kFmtS8, kFmtS8, kAccS32, 128, 64, 0, 0);
@@ -508,15 +548,13 @@ __device__ __forceinline__ void issue_pv(uint32_t tmem, uint32_t slot_addr, uint
 // 100 KB of code: 1.48 us per 64-key stage and SM at D = 64 instead of 1.11).
 // Where a row of the tile goes in `tokens` (element offset of its first channel), -1: a padding row.
 template <int D>
-__device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, int tile, int block0, int QB, int row) {
-  int token;
+__device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, int block0, int QB, int row) {
+  int token = block0 * QB + row;
   if (p.dense_prefix) {
-    token = tile * QB + row;
-    if (row >= QB || token >= p.s.prefix_tokens) return -1;
+    if (token >= p.s.prefix_tokens) return -1;
   } else {
-    const int block = block0 + row / QB;
-    if (row % QB >= p.counts[block]) return -1;
-    token = p.s.prefix_tokens + p.indices[block0 * QB + row];
+    if (row % QB >= p.counts[block0 + row / QB]) return -1;
+    token = p.s.prefix_tokens + p.indices[token];
   }
   return ((int64_t)token * p.s.heads + head) * D;
 }
@@ -541,8 +579,11 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // query blocks of this CTA (two for a complete pair) and the first one's index
-  const int tile_blocks = pairs && 2 * tile + 1 < p.s.video_blocks ? 2 : 1;
-  const int block0 = pairs ? 2 * tile : tile;
+  // (prefix tiles of 64 rows also go in twos: both walk every stage)
+  const bool twos = pairs || (kQ64 && p.dense_prefix);
+  const int tile_blocks =
+      twos && 2 * tile + 1 < (p.dense_prefix ? p.q_tiles_int8 - p.s.video_blocks : p.s.video_blocks) ? 2 : 1;
+  const int block0 = twos ? 2 * tile : tile;
 
   // ---- this tile's work list ----
   int cnt[3] = {0, p.stages, 0};
@@ -558,7 +599,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     // nothing to attend to: +0 rows (packed rows are left alone, the assembly knows)
     if (p.tokens != nullptr)
       for (int i = threadIdx.x; i < QB * tile_blocks * (D / 8); i += kThreads) {
-        const int64_t at = token_offset<D>(p, head, tile, block0, QB, i / (D / 8));
+        const int64_t at = token_offset<D>(p, head, block0, QB, i / (D / 8));
         if (at >= 0)
           *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.tokens) + at + i % (D / 8) * 8) = make_uint4(0, 0, 0, 0);
       }
@@ -582,7 +623,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     }
     mbar_init(&b->m_full[0][lane], 1);  // all four quadrants' rings
     if (lane == 0) {
-      mbar_init(&b->v_full, 1);
+      for (int i = 0; i < kSplitValues; ++i) mbar_init(&b->v_full[i], 1);
+      mbar_init(&b->q_moved, 4);
       mbar_init(&b->q_full, 1);
       mbar_init(&b->q_free, 1);
       for (int i = 0; i < 2; ++i) {
@@ -632,7 +674,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       const uint32_t lead = lane == 0;
       const int q_index_fp = head * p.s.video_blocks + block0;  // q_fp16 / q_nvfp4 record
       const int64_t q_index_i8 =
-          (int64_t)head * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks + tile : block0);
+          (int64_t)head * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks : 0) + block0;
       const float sigma = (D == 64 ? 0.125f : 0.08838834764831845f) * 1.4426950408889634f;
       int phase_ord = 0, g = 0, v_fills = 0;
 #pragma unroll 1
@@ -683,14 +725,14 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           kscale = p.o.k_int8_scale + (int64_t)head * p.stages;
         }
         const float base = cell == kNv ? sigma * p.s.q_global_scale * p.s.k_global_scale : sigma;
-        const bool split = split_kv(D, cell);
         // list entries, 32 at a time, one per lane, with their metadata
-        int stage_l = 0, v_stage = 0;
+        int stage_l = 0;
         float2 meta_l[2] = {make_float2(base, 0.0f), make_float2(base, 0.0f)};
-        int slot = 0;
-        // Split phases: with one value buffer, the values of stage i - nslot + 1 may follow when PV of
-        // stage i - nslot is complete, which is also what the key tile of stage i waits for.
-        const int end = split ? n + nslot - 1 : n;
+        int slot = first_slot(D, cell);
+        const bool split = split_kv(D, cell);
+        int prev_stage = 0;
+        // (split phases: a stage's values follow the next stage's keys)
+        const int end = n + (split ? 1 : 0);
 #pragma unroll 1
         for (int i = 0; i < end; ++i) {
           if ((i & 31) == 0 && i < n) {
@@ -700,7 +742,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             stage_l = entry & 0x3fffffff;
             const int valid = p.valid_k[stage_l];
             meta_l[0].y = __int_as_float(!pairs || ((entry >> 30) & 1) ? valid : -1);
-            if (kQ64) meta_l[1].y = __int_as_float(entry < 0 ? valid : -1);
+            if (kQ64) meta_l[1].y = __int_as_float(entry < 0 || p.dense_prefix ? valid : -1);
             if (cell == kI8) {
               const float ks = kscale[stage_l];
               meta_l[0].x = sigma * (q_scale[0] * ks);
@@ -709,20 +751,10 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           }
           const int stage = __shfl_sync(0xffffffffu, stage_l, i & 31);
           const int gi = g + i;
-          if (i >= nslot)
-            wait<kMmaRole>(&b->wc, &b->pv_done[(gi - nslot) & (kRing - 1)], ((gi - nslot) >> 3) & 1, 2);
-          if (split) {
-            const int vi = i - nslot + 1;
-            if (vi >= 0) {
-              mbar_arrive_expect_tx(&b->v_full, kvbytes - kbytes, lead);
-              bulk_g2s(ring + nslot * slot_size, kvbase + (int64_t)v_stage * kvbytes + kbytes, kvbytes - kbytes,
-                       &b->v_full, lead);
-              ++v_fills;
-            }
-            // the stage whose values come next
-            if (vi + 1 >= 0 && vi + 1 < n) v_stage = list != nullptr ? list[first + vi + 1] & 0x3fffffff : vi + 1;
-          }
           if (i < n) {
+            if (i >= nslot)
+              wait<kMmaRole>(&b->wc, &b->pv_done[(gi - nslot) & (kRing - 1)], ((gi - nslot) >> 3) & 1, 2);
+            if (split && i == 2) wait<kMmaRole>(&b->wc, &b->q_moved, 0, 2);
             const int at = gi & (kRing - 1);
             if (lane == (i & 31)) {
               b->meta[at][0] = meta_l[0];
@@ -731,7 +763,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             __syncwarp();
             const int bytes = split ? kbytes : kvbytes;
             const uint8_t* src = kvbase + (int64_t)stage * kvbytes;
-            uint8_t* dst = ring + (size_t)slot * slot_size;
+            uint8_t* dst = (split ? smem : ring) + (size_t)slot * slot_size;
             mbar_arrive_expect_tx(&b->kv_full[at], bytes, lead);
             if (split || rest == kbytes) {
               bulk_g2s(dst, src, bytes, &b->kv_full[at], lead);
@@ -741,6 +773,16 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             }
             slot = slot + 1 == nslot ? 0 : slot + 1;
           }
+          if (split && i > 0) {
+            const int before = gi - 1 - kSplitValues;  // the stage that had the value buffer
+            if (i > kSplitValues) wait<kMmaRole>(&b->wc, &b->pv_done[before & (kRing - 1)], (before >> 3) & 1, 2);
+            uint64_t* full = &b->v_full[(i - 1) & 1];
+            mbar_arrive_expect_tx(full, kvbytes - kbytes, lead);
+            bulk_g2s(smem + (kSplitKeys + ((i - 1) & 1)) * slot_size, kvbase + (int64_t)prev_stage * kvbytes + kbytes,
+                     kvbytes - kbytes, full, lead);
+            ++v_fills;
+          }
+          prev_stage = stage;
         }
         g += n;
         ++phase_ord;
@@ -749,7 +791,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         // unwinding: the copies in flight must land before the CTA gives its shared memory back
         for (int k = max(0, g - kRing); k < g; ++k)
           drain_wait(&b->kv_full[k & (kRing - 1)], (k >> 3) & 1, kDrainNs);
-        if (v_fills > 0) drain_wait(&b->v_full, (v_fills - 1) & 1, kDrainNs);
+        for (int j = max(0, v_fills - kSplitValues); j < v_fills; ++j)
+          drain_wait(&b->v_full[j & 1], (j >> 1) & 1, kDrainNs);
         if (phase_ord > 0) drain_wait(&b->q_full, (phase_ord - 1) & 1, kDrainNs);
       }
     } else if (warp == kQkWarp) {
@@ -762,12 +805,17 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       for (int cell = kFirst; cell <= kLast; ++cell) {
         const int n = b->cnt[cell];
         if (n == 0) continue;
-        wait<kMmaRole>(&b->wc, &b->q_full, phase_ord & 1, 3);
+        if (cell == kF16) {
+          wait<kMmaRole>(&b->wc, &b->q_moved, 0, 3);
+        } else {
+          wait<kMmaRole>(&b->wc, &b->q_full, phase_ord & 1, 3);
+        }
         // the second score buffer takes the place of the NVFP4 phase's scale factors
         if (CELLS == kAny && cell != kNv && b->cnt[kNv] > 0) wait<kMmaRole>(&b->wc, &b->nv_done, 0, 3);
         tc_fence_after_sync();
         const int nslot = slot_count(p.ring_bytes, D, cell);
         const uint32_t stride = stage_bytes(D, cell);
+        const uint32_t base_addr = split_kv(D, cell) ? smem_u32(smem) : ring_addr;
         if (cell == kNv) {
           if (tile_blocks == 2) {
             // Scale bytes of rows 0-63 sit in the low eight bytes of every 16-byte chunk, those of
@@ -792,7 +840,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         }
         // a stage's scores are computed as soon as its key tile has landed and its score buffer
         // has been read
-        int slot = 0;
+        int slot = first_slot(D, cell);
 #pragma unroll 1
         for (int i = 0; i < n; ++i, ++g) {
           const int sb = s_buffer<D>(cell, g);
@@ -804,7 +852,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           used |= 1u << sb;
           tc_fence_after_sync();
           if (elect_one()) {
-            const uint32_t tmem_s = tmem + (sb ? Cols<D>::kS1 : kColS), slot_addr = ring_addr + slot * stride;
+            const uint32_t tmem_s = tmem + (sb ? Cols<D>::kS1 : kColS), slot_addr = base_addr + slot * stride;
             if (cell == kI8) {
               issue_qk<D, kI8>(tmem_s, tmem, q_addr, slot_addr);
             } else if (cell == kNv) {
@@ -835,16 +883,18 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         if (n == 0) continue;
         const int nslot = slot_count(p.ring_bytes, D, cell);
         const uint32_t stride = stage_bytes(D, cell);
-        const bool split = split_kv(D, cell);
-        int slot = 0;
+        const uint32_t base_addr = split_kv(D, cell) ? smem_u32(smem) : ring_addr;
+        int slot = first_slot(D, cell);
 #pragma unroll 1
         for (int i = 0; i < n; ++i, ++g) {
-          if (split) wait<kMmaRole>(&b->wc, &b->v_full, i & 1, 6);  // (a tile has at most one such phase)
+          // (a tile has at most one phase with value buffers)
+          if (split_kv(D, cell)) wait<kMmaRole>(&b->wc, &b->v_full[i & 1], (i >> 1) & 1, 6);
           wait<kMmaRole>(&b->wc, &b->p_full[g & (kRing - 1)], (g >> 3) & 1, 6);
           tc_fence_after_sync();
           if (elect_one()) {
-            const uint32_t slot_addr = ring_addr + slot * stride;
-            const uint32_t v_addr = split ? ring_addr + nslot * stride : slot_addr + rest_offset(D, cell);
+            const uint32_t slot_addr = base_addr + slot * stride;
+            const uint32_t v_addr = split_kv(D, cell) ? base_addr + (kSplitKeys + (i & 1)) * stride
+                                                      : slot_addr + rest_offset(D, cell);
             if (cell == kI8) {
               issue_pv<D, kI8>(tmem, slot_addr, v_addr, g > 0);
             } else if (cell == kNv) {
@@ -865,14 +915,14 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       if (b->wc.abort) drain_wait(&b->all_done, 0, kDrainNs);
     }
   } else if (warp >= kCorrWarp) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kCorrRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS>::kRescale));
     // =============================== O rescale ===============================
     const int row = (warp - kCorrWarp) * 32 + lane;
     uint64_t* m_full = b->m_full[warp - kCorrWarp];
     const uint32_t tmem_row = tmem + ((uint32_t)((warp - kCorrWarp) * 32) << 16);
     const uint32_t lead = lane == 0;
     float m = -5.0e6f;
-    int g = 0, prev_cell = -1;
+    int g = 0, prev_cell = -1, phase_ord = 0;
 #pragma unroll 1
     for (int cell = kFirst; cell <= kLast; ++cell) {
       const int n = b->cnt[cell];
@@ -889,6 +939,26 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         }
         asm volatile("bar.sync 5, 128;" ::: "memory");
       }
+      if (cell == kF16) {
+        // Q into tensor memory.  Its columns are free: this quadrant's rows of every earlier score
+        // tile have been read (their maxima were published after that), and so have, after the NVFP4
+        // phase, its scale factors.
+        if (CELLS == kAny && b->cnt[kNv] > 0) wait<kRescaleRole>(&b->wc, &b->nv_done, 0, 31);
+        wait<kRescaleRole>(&b->wc, &b->q_full, phase_ord & 1, 32);
+#pragma unroll 1
+        for (int c = 0; c < D / 8; c += 2) {
+          uint32_t r[8];
+          *reinterpret_cast<uint4*>(r) = *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c, D / 8));
+          *reinterpret_cast<uint4*>(r + 4) =
+              *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c + 1, D / 8));
+          tmem_st8(tmem_row + kColQ + c * 4, r);
+        }
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        mbar_arrive_if(&b->q_moved, lead);
+      }
+      ++phase_ord;
 #pragma unroll 1
       for (int i = 0; i < n; ++i, ++g) {
         const int at = g & (kRing - 1);
@@ -900,7 +970,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           // O may only be touched once the previous PV is complete
           wait<kRescaleRole>(&b->wc, &b->pv_done[(g - 1) & (kRing - 1)], ((g - 1) >> 3) & 1, 20);
           tc_fence_after_sync();
-          rescale_o<D>(tmem_row, alpha, first ? colf : nullptr);
+          rescale_o<D, Regs<D, CELLS>::kRescaleColumns>(tmem_row, alpha, first ? colf : nullptr);
           tc_fence_before_sync();
         }
         m = m_new;
@@ -910,7 +980,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       prev_cell = cell;
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS>::kSoftmax));
     // =============================== softmax rows ===============================
     const int row = (warp & 3) * 32 + lane;  // query row == TMEM lane
     const int parity = warp >> 2;            // which stages this warpgroup runs
@@ -929,10 +999,11 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       if (n == 0) continue;
       const int nslot = slot_count(p.ring_bytes, D, cell);
       const int stride = stage_bytes(D, cell);
-      uint8_t* p_row = ring + rec::tile_offset(row, 0, p_bytes(cell) / 2048);
-      int slot = (g & 1) == parity ? 0 : 1;
+      uint8_t* p_row = (split_kv(D, cell) ? smem : ring) + rec::tile_offset(row, 0, p_bytes(cell) / 2048);
+      const int first = (g & 1) == parity ? 0 : 1;
+      int slot = first_slot(D, cell) + first;
 #pragma unroll 1
-      for (int i = slot; i < n; i += 2) {
+      for (int i = first; i < n; i += 2) {
         softmax_stage<D, kQ64>(b, p_row + slot * stride, tmem_row, row, g + i, cell, live_warp, my_block, w);
         slot += 2;
         if (slot >= nslot) slot -= nslot;
@@ -949,8 +1020,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     asm volatile("bar.sync 6, 256;" ::: "memory");
     if (last_mine) {
       const float2 other = b->rec[0][row];
-      const float d = (w.d * other.x + other.y) * w.alpha + w.sum;
-      b->rec[1][row] = make_float2(d, 0.0f);
+      b->rec[1][row] = make_float2((w.d * other.x + other.y) * w.alpha + w.sum, 0.0f);
     }
     asm volatile("bar.sync 6, 256;" ::: "memory");
     if (live_warp) {
@@ -963,7 +1033,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         if (row < QB * tile_blocks)
           dst = reinterpret_cast<uint16_t*>(p.out) + ((int64_t)head * p.out_rows + (int64_t)block0 * QB + row) * D;
       } else if (row < QB * tile_blocks) {
-        const int64_t at = token_offset<D>(p, head, tile, block0, QB, row);
+        const int64_t at = token_offset<D>(p, head, block0, QB, row);
         if (at >= 0) dst = static_cast<uint16_t*>(p.tokens) + at;
       }
       const bool bf16 = p.tokens != nullptr && p.tokens_bf16;
@@ -1173,9 +1243,10 @@ int prefix_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operand
   p.wait_ns = g_wait_limit_ns;
   p.dense_prefix = 1;
   p.stages = rec::stages(*shape);
-  const int tiles = rec::prefix_query_tiles(*shape);
-  p.q_tiles_int8 = shape->video_blocks + tiles;
-  p.out_rows = tiles * shape->query_block;
+  const int blocks = rec::prefix_query_tiles(*shape);
+  const int tiles = shape->query_block == 64 ? (blocks + 1) / 2 : blocks;
+  p.q_tiles_int8 = shape->video_blocks + blocks;
+  p.out_rows = blocks * shape->query_block;
   set_rows(p, rows);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return launch_for(p, tiles, st);

@@ -38,7 +38,11 @@ template <int kRole>
 __device__ __noinline__ void wait_slow(WaitContext* w, uint64_t* bar, uint32_t parity, int where) {
   const uint64_t t0 = globaltimer_ns();
   for (;;) {
-    if (mbar_try_wait(bar, parity)) return;
+    // a try also returns when the barrier changes without completing its phase: several tries for
+    // each look at the clock
+#pragma unroll 1
+    for (int k = 0; k < 8; ++k)
+      if (mbar_try_wait(bar, parity)) return;
     if (w->abort) return;
     if (globaltimer_ns() - t0 > w->limit_ns) break;
   }

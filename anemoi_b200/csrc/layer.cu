@@ -132,7 +132,8 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
       return ANEMOI_SM100_ELAUNCH;
     return layer::prefix_rows(s, w.ops, p.valid_k, rows, p.status, side);
   };
-  const bool late = native_prefix && rec::prefix_query_tiles(s) * s.heads >= kPrefixFillsGpu;
+  const int prefix_ctas = (rec::prefix_query_tiles(s) * s.query_block + 127) / 128 * s.heads;
+  const bool late = native_prefix && prefix_ctas >= kPrefixFillsGpu;
   if (native_prefix && !late && (code = prefix()) != ANEMOI_SM100_OK) return done(code);
 
   code = anemoi_sm100_draft_probability(&s, w.ops.q_pool, w.ops.k_pool, w.ops.q_max_pool, w.ops.k_max_pool,
