@@ -410,14 +410,17 @@ def copy_head_group(dst: torch.Tensor, src: torch.Tensor, stream: torch.cuda.Str
             raise ValueError("copy_head_group needs views contiguous over (heads, D)")
         if t.device.type == "cpu" and not t.is_pinned():
             raise ValueError("the host side of copy_head_group must be pinned memory")
-    to_device = dst.device.type == "cuda"
-    if to_device == (src.device.type == "cuda"):
+    if (dst.device.type == "cuda") == (src.device.type == "cuda"):
         raise ValueError("copy_head_group copies between the host and the device")
+    copy_rows(dst, src, stream)
+
+
+def copy_rows(dst: torch.Tensor, src: torch.Tensor, stream: torch.cuda.Stream) -> None:
+    """``copy_head_group`` without its checks, for callers that made them for whole tensors."""
     size = dst.element_size()
     _check(library().anemoi_sm100_copy_rows(
-        _ptr(dst), dst.stride(1) * size, _ptr(src), src.stride(1) * size,
-        dst.size(2) * dst.size(3) * size, dst.size(1), int(to_device),
-        C.c_void_p(stream.cuda_stream)), "anemoi_sm100_copy_rows")
+        dst.data_ptr(), dst.stride(1) * size, src.data_ptr(), src.stride(1) * size,
+        dst.size(2) * dst.size(3) * size, dst.size(1), int(dst.is_cuda), stream.cuda_stream), "anemoi_sm100_copy_rows")
 
 
 def set_wait_limit_ns(limit_ns: int) -> None:
