@@ -44,7 +44,7 @@ __device__ __forceinline__ float exp_canonical(float t) {
 }
 
 // fp16 logits of kWarps * RPW query blocks against every key block of the head.  Each warp owns
-// RPW (2 or 4) rows, each lane four key columns of the 128-column pass: per channel one 16-byte
+// RPW (1, 2 or 4) rows, each lane four key columns of the 128-column pass: per channel one 16-byte
 // load of keys (four shared-memory wavefronts per warp) and one broadcast load of the warp's
 // query values feed 4 * RPW FMAs, so with four rows the FMA pipe rather than shared memory
 // sets the pace.  Every logit is still the plain channel-ordered FMA chain (the canonical
@@ -63,51 +63,61 @@ __device__ __forceinline__ void row_logits(const __half* q_pool, const __half* k
     qs[((r / RPW) * D + c) * RPW + (r % RPW)] =
         row < R ? __half2float(q_pool[((int64_t)head * R + row) * D + c]) : 0.0f;
   }
-  for (int c0 = 0; c0 < R; c0 += kChunk) {
-    float acc[RPW][4];
+  // Key pools of columns [c0, c0 + kChunk), kSlab channels at a time, as [channel][column] floats (the
+  // chain still runs over c = 0..D-1).  The next piece is loaded while this one is multiplied.
+  constexpr int kSlabs = D / kSlab, kLoads = kChunk * (kSlab / 8) / (kWarps * 32);
+  const int pieces = (R + kChunk - 1) / kChunk * kSlabs;
+  uint4 raw[kLoads];
+  auto fetch = [&](int piece) {
+    const int c0 = piece / kSlabs * kChunk, s0 = piece % kSlabs * kSlab;
 #pragma unroll
-    for (int r = 0; r < RPW; ++r)
+    for (int i = 0; i < kLoads; ++i) {
+      const int idx = threadIdx.x + i * kWarps * 32, col = c0 + idx % kChunk, c8 = idx / kChunk;
+      raw[i] = make_uint4(0, 0, 0, 0);
+      if (col < R) raw[i] = __ldg(reinterpret_cast<const uint4*>(k_pool + ((int64_t)head * R + col) * D + s0) + c8);
+    }
+  };
+  fetch(0);
+  const float* qw = qs + warp * D * RPW;
+  float acc[RPW][4];
+  for (int piece = 0; piece < pieces; ++piece) {
+    const int c0 = piece / kSlabs * kChunk, s0 = piece % kSlabs * kSlab;
+    __syncthreads();
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[r][j] = 0.0f;
-    const float* qw = qs + warp * D * RPW;
-    // the key tile is staged kSlab channels at a time; the chain still runs over c = 0..D-1
-    for (int s0 = 0; s0 < D; s0 += kSlab) {
-      __syncthreads();
-      // key pools of columns [c0, c0 + kChunk), channels [s0, s0 + kSlab), as [channel][column] floats
-      for (int idx = threadIdx.x; idx < kChunk * (kSlab / 8); idx += kWarps * 32) {
-        const int col = idx % kChunk, c8 = idx / kChunk;
-        uint4 raw = make_uint4(0, 0, 0, 0);
-        if (c0 + col < R)
-          raw = __ldg(reinterpret_cast<const uint4*>(k_pool + ((int64_t)head * R + c0 + col) * D + s0) + c8);
-        const __half* h = reinterpret_cast<const __half*>(&raw);
+    for (int i = 0; i < kLoads; ++i) {
+      const int idx = threadIdx.x + i * kWarps * 32;
+      const __half* h = reinterpret_cast<const __half*>(&raw[i]);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) kc[(c8 * 8 + i) * kPitch + col] = __half2float(h[i]);
+      for (int j = 0; j < 8; ++j) kc[(idx / kChunk * 8 + j) * kPitch + idx % kChunk] = __half2float(h[j]);
+    }
+    __syncthreads();
+    if (piece + 1 < pieces) fetch(piece + 1);
+    if (s0 == 0) {
+#pragma unroll
+      for (int r = 0; r < RPW; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[r][j] = 0.0f;
+    }
+#pragma unroll 8
+    for (int c = 0; c < kSlab; ++c) {
+      float qv[RPW];
+      if (RPW == 4) {
+        *reinterpret_cast<float4*>(qv) = *reinterpret_cast<const float4*>(qw + (s0 + c) * 4);
+      } else if (RPW == 2) {
+        *reinterpret_cast<float2*>(qv) = *reinterpret_cast<const float2*>(qw + (s0 + c) * 2);
+      } else {
+        qv[0] = qw[s0 + c];
       }
-      __syncthreads();
-#pragma unroll 4
-      for (int c = 0; c < kSlab; ++c) {
-        float qv[RPW];
-        if (RPW == 4) {
-          const float4 t = *reinterpret_cast<const float4*>(qw + (s0 + c) * 4);
-          qv[0] = t.x;
-          qv[1] = t.y;
-          qv[RPW - 2] = t.z;
-          qv[RPW - 1] = t.w;
-        } else {
-          const float2 t = *reinterpret_cast<const float2*>(qw + (s0 + c) * 2);
-          qv[0] = t.x;
-          qv[1] = t.y;
-        }
-        const float4 kv = *reinterpret_cast<const float4*>(kc + c * kPitch + lane * 4);
+      const float4 kv = *reinterpret_cast<const float4*>(kc + c * kPitch + lane * 4);
 #pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-          acc[r][0] = __fmaf_rn(qv[r], kv.x, acc[r][0]);
-          acc[r][1] = __fmaf_rn(qv[r], kv.y, acc[r][1]);
-          acc[r][2] = __fmaf_rn(qv[r], kv.z, acc[r][2]);
-          acc[r][3] = __fmaf_rn(qv[r], kv.w, acc[r][3]);
-        }
+      for (int r = 0; r < RPW; ++r) {
+        acc[r][0] = __fmaf_rn(qv[r], kv.x, acc[r][0]);
+        acc[r][1] = __fmaf_rn(qv[r], kv.y, acc[r][1]);
+        acc[r][2] = __fmaf_rn(qv[r], kv.z, acc[r][2]);
+        acc[r][3] = __fmaf_rn(qv[r], kv.w, acc[r][3]);
       }
     }
+    if (s0 + kSlab < D) continue;
 #pragma unroll
     for (int r = 0; r < RPW; ++r)
 #pragma unroll
@@ -256,7 +266,7 @@ __global__ void __launch_bounds__(kWarps * 32) draft_kernel(const __half* q_pool
   constexpr int kRows = kWarps * RPW;
   const int lg_stride = (R + 7) & ~7;
   float* kc = reinterpret_cast<float*>(smem_raw);                   // [kSlab][kPitch]
-  float* qs = kc + kSlab * kPitch;                                      // [kWarps][D][2]
+  float* qs = kc + kSlab * kPitch;                                  // [kWarps][D][RPW]
   __half* lg = reinterpret_cast<__half*>(qs + kRows * D);           // [kRows][lg_stride]
   __half* lgx = lg + kRows * lg_stride;                             // blend only
   const int head = blockIdx.y, row0 = blockIdx.x * kRows;
@@ -315,13 +325,19 @@ int launch_rows(const __half* qp, const __half* kp, const __half* qx, const __ha
              : ANEMOI_SM100_ELAUNCH;
 }
 
-// Four rows per warp while two CTAs still fit an SM's shared memory, else two rows per warp.
+// Rows per warp.  Four while two CTAs still fit an SM's shared memory, else two: a key tile read serves
+// more rows.  But while a grid of fewer rows has no more CTAs than there are SMs, every CTA has one to
+// itself and the shorter one wins: one row per warp for 8 heads x 33 blocks (31 -> 16 us with the
+// loads ahead), two for 7 x 273 (64 -> 41); at 7 x 672 (294 CTAs of two) four are quicker, 57 against 65.
+constexpr int kSms = 148;
 template <int D, bool kBlend>
 int launch(const __half* qp, const __half* kp, const __half* qx, const __half* kx, float w, int R,
            int H, __half* prob, cudaStream_t st) {
-  if (smem_bytes<D, kBlend, 4>(R) <= 113 * 1024)
-    return launch_rows<D, kBlend, 4>(qp, kp, qx, kx, w, R, H, prob, st);
-  return launch_rows<D, kBlend, 2>(qp, kp, qx, kx, w, R, H, prob, st);
+  auto ctas = [&](int rpw) { return (int64_t)((R + kWarps * rpw - 1) / (kWarps * rpw)) * H; };
+  if (ctas(1) <= kSms) return launch_rows<D, kBlend, 1>(qp, kp, qx, kx, w, R, H, prob, st);
+  if (ctas(2) <= kSms || smem_bytes<D, kBlend, 4>(R) > 113 * 1024)
+    return launch_rows<D, kBlend, 2>(qp, kp, qx, kx, w, R, H, prob, st);
+  return launch_rows<D, kBlend, 4>(qp, kp, qx, kx, w, R, H, prob, st);
 }
 
 }  // namespace

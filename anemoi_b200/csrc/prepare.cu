@@ -7,6 +7,11 @@
 // (narrowed to fp16), derives pools / amax / scales from shared memory, and
 // streams the tile records out with 16-byte coalesced stores.
 //
+// Between HBM and issue bound: maxima are taken two halves at a time, V is read two channels
+// at a time (lanes side by side; single halves 16 rows apart met in four banks), codes are
+// packed by the converting instructions.  56 heads, prefix 512: S = 85,184 (11.5 GB) 2,544 -> 2,130 us =
+// 4.9 TB/s, S = 33,272 845 -> 730; Q64 INT8, S = 38,247 794 -> 600; 8 heads x 4,109 tokens 48 -> 24.
+//
 // Numeric contract (reference: csrc/attention/cuda/sm120/q128_microscaling_preparation.cu):
 //   narrow  bf16 -> f32 -> f16 rn (:227-232); invalid slots and prefix padding are +0 (:369-374)
 //   mean    f16( sum_slots f32 in slot order / count ), IEEE division (:375-377,511-517)
@@ -25,6 +30,9 @@
 namespace {
 
 constexpr int kThreads = 256;
+// CTAs per SM: 51 registers per thread for 128-row blocks, 32 for 64-row ones; fewer CTAs
+// with more registers are slower (56 heads x 33,272 tokens: 759 us at four, 728 at five, 821 at six).
+__host__ __device__ constexpr int min_ctas(int qb) { return qb == 128 ? 5 : 8; }
 constexpr int kPad = 8;  // halves of padding per shared-memory row
 
 struct PrepParams {
@@ -91,11 +99,22 @@ __device__ __forceinline__ uint8_t e2m1_pair(float lo, float hi, float dq, float
   return __nv_cvt_float2_to_fp4x2(make_float2(div_rn(lo, dq, inv_dq), div_rn(hi, dq, inv_dq)),
                                   __NV_E2M1, cudaRoundNearest);
 }
-__device__ __forceinline__ int8_t int8_code(float x, float scale, float inv_scale) {
-  float t = div_rn(x, scale, inv_scale);
-  t = __fadd_rn(t, t >= 0.0f ? 0.5f : -0.5f);
-  return static_cast<int8_t>(__float2int_rz(t));
+// trunc(x / scale +- 0.5); |result| <= 127
+__device__ __forceinline__ int int8_code(float x, float scale, float inv_scale) {
+  const float t = div_rn(x, scale, inv_scale);
+  const float half = __int_as_float((__float_as_int(t) & 0x80000000) | 0x3f000000);
+  return __float2int_rz(__fadd_rn(t, half));
 }
+// Four codes as bytes, the first one lowest.
+__device__ __forceinline__ uint32_t pack_s8(int a, int b, int c, int d) {
+  uint32_t r;
+  asm("{\n\t.reg .b32 t;\n\tcvt.pack.sat.s8.s32.b32 t, %4, %3, 0;\n\tcvt.pack.sat.s8.s32.b32 %0, %2, %1, t;\n\t}"
+      : "=r"(r)
+      : "r"(a), "r"(b), "r"(c), "r"(d));
+  return r;
+}
+// The larger of two magnitudes, both halves at once.
+__device__ __forceinline__ __half2 max_abs2(__half2 m, __half2 x) { return __hmax2(m, __habs2(x)); }
 
 // Gathers ROWS rows into `tile` ([ROWS][D + kPad] halves), zero for invalid slots.  The trip
 // count is a compile-time constant and the loop is split into a load pass and a store pass, so
@@ -150,17 +169,15 @@ __device__ __forceinline__ void write_fp16_tile(uint8_t* dst, const __half* tile
 template <int D>
 __device__ __forceinline__ float tile_amax(const __half* tile, int row0, int rows, float* red) {
   constexpr int kVec = D / 8;
-  float m = 0.0f;
+  __half2 m2 = __half2(__half(0.0f), __half(0.0f));
   for (int idx = threadIdx.x; idx < rows * kVec; idx += kThreads) {
     const int r = idx / kVec, c8 = idx % kVec;
-    uint4 raw = *reinterpret_cast<const uint4*>(tile + (row0 + r) * (D + kPad) + c8 * 8);
+    const uint4 raw = *reinterpret_cast<const uint4*>(tile + (row0 + r) * (D + kPad) + c8 * 8);
     const __half2* h = reinterpret_cast<const __half2*>(&raw);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float2 f = __half22float2(h[i]);
-      m = fmaxf(m, fmaxf(fabsf(f.x), fabsf(f.y)));
-    }
+    for (int i = 0; i < 4; ++i) m2 = max_abs2(m2, h[i]);
   }
+  const float m = __half2float(__hmax(m2.x, m2.y));
   return block_max(m, red);
 }
 
@@ -175,13 +192,11 @@ __device__ __forceinline__ void write_int8_tile(uint8_t* dst, const __half* tile
     uint4 a = *reinterpret_cast<const uint4*>(src), b = *reinterpret_cast<const uint4*>(src + 8);
     const __half* ha = reinterpret_cast<const __half*>(&a);
     const __half* hb = reinterpret_cast<const __half*>(&b);
-    uint4 out;
-    int8_t* c = reinterpret_cast<int8_t*>(&out);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      c[i] = int8_code(__half2float(ha[i]), scale, inv_scale);
-      c[8 + i] = int8_code(__half2float(hb[i]), scale, inv_scale);
-    }
+    auto code = [&](__half h) { return int8_code(__half2float(h), scale, inv_scale); };
+    const uint4 out = make_uint4(pack_s8(code(ha[0]), code(ha[1]), code(ha[2]), code(ha[3])),
+                                 pack_s8(code(ha[4]), code(ha[5]), code(ha[6]), code(ha[7])),
+                                 pack_s8(code(hb[0]), code(hb[1]), code(hb[2]), code(hb[3])),
+                                 pack_s8(code(hb[4]), code(hb[5]), code(hb[6]), code(hb[7])));
     *reinterpret_cast<uint4*>(dst + (size_t)idx * 16) = out;
   }
 }
@@ -202,16 +217,16 @@ __device__ __forceinline__ void write_nvfp4_rows(uint8_t* codes, uint8_t* sf, co
       uint4 a = *reinterpret_cast<const uint4*>(src + g * 16);
       uint4 b = *reinterpret_cast<const uint4*>(src + g * 16 + 8);
       float x[16];
-      const __half* ha = reinterpret_cast<const __half*>(&a);
-      const __half* hb = reinterpret_cast<const __half*>(&b);
-      float amax = 0.0f;
+      const __half2* ha = reinterpret_cast<const __half2*>(&a);
+      const __half2* hb = reinterpret_cast<const __half2*>(&b);
+      __half2 m2 = __hmax2(__habs2(ha[0]), __habs2(hb[0]));
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        x[i] = __half2float(ha[i]);
-        x[8 + i] = __half2float(hb[i]);
+      for (int i = 0; i < 4; ++i) {
+        *reinterpret_cast<float2*>(x + 2 * i) = __half22float2(ha[i]);
+        *reinterpret_cast<float2*>(x + 8 + 2 * i) = __half22float2(hb[i]);
+        if (i > 0) m2 = max_abs2(max_abs2(m2, ha[i]), hb[i]);
       }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(x[i]));
+      const float amax = __half2float(__hmax(m2.x, m2.y));
       sb[g] = nv_scale_byte(amax, gs);
       const float dq = __fmul_rn(e4m3_to_float(sb[g]), gs);
       const float inv_dq = __frcp_rn(dq);
@@ -224,51 +239,63 @@ __device__ __forceinline__ void write_nvfp4_rows(uint8_t* codes, uint8_t* sf, co
   }
 }
 
-// V^T tiles of one 64-key stage: channels x keys, keys contiguous.
+// V^T tiles of one 64-key stage: channels x keys, keys contiguous.  A thread takes two neighbouring
+// channels of 16 keys: 4-byte reads, lanes side by side along the channels.
 template <int D>
 __device__ __forceinline__ void write_v_e4m3(uint8_t* dst, const __half* tile, int row0,
                                              const float* recip) {
-  for (int idx = threadIdx.x; idx < D * 4; idx += kThreads) {
-    const int c = (idx >> 5) * 8 + (idx & 7), jj = (idx >> 3) & 3;
-    const float rc = recip[c];
-    uint4 out;
-    uint8_t* o = reinterpret_cast<uint8_t*>(&out);
+  for (int idx = threadIdx.x; idx < D * 2; idx += kThreads) {
+    const int c = idx % (D / 2) * 2, jj = idx / (D / 2);
+    const float2 rc = *reinterpret_cast<const float2*>(recip + c);
+    const __half* src = tile + (row0 + jj * 16) * (D + kPad) + c;
+    uint4 out[2];
+    uint16_t* o0 = reinterpret_cast<uint16_t*>(&out[0]);
+    uint16_t* o1 = reinterpret_cast<uint16_t*>(&out[1]);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float v = __half2float(tile[(row0 + jj * 16 + i) * (D + kPad) + c]);
-      o[i] = rc == 0.0f ? (uint8_t)0
-                        : (uint8_t)__nv_cvt_float_to_fp8(__fmul_rn(v, rc), __NV_SATFINITE, __NV_E4M3);
+    for (int i = 0; i < 8; ++i) {
+      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(src + 2 * i * (D + kPad)));
+      const float2 b = __half22float2(*reinterpret_cast<const __half2*>(src + (2 * i + 1) * (D + kPad)));
+      // (a channel whose factor is zero holds zeros only)
+      o0[i] = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a.x, rc.x), __fmul_rn(b.x, rc.x)), __NV_SATFINITE, __NV_E4M3);
+      o1[i] = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a.y, rc.y), __fmul_rn(b.y, rc.y)), __NV_SATFINITE, __NV_E4M3);
     }
-    *reinterpret_cast<uint4*>(dst + (size_t)idx * 16) = out;
+    if (rc.x == 0.0f) out[0] = make_uint4(0, 0, 0, 0);
+    if (rc.y == 0.0f) out[1] = make_uint4(0, 0, 0, 0);
+    uint4* to = reinterpret_cast<uint4*>(dst + rec::tile_offset(c, jj, 4));
+    to[0] = out[0];
+    to[1] = out[1];
   }
 }
 
 template <int D>
 __device__ __forceinline__ void write_v_nvfp4(uint8_t* codes, uint8_t* sf, const __half* tile,
                                               int row0, float gs) {
+  // a thread: two neighbouring channels, 16 of the 64 keys
   for (int idx = threadIdx.x; idx < D * 2; idx += kThreads) {
-    const int c = (idx >> 4) * 8 + (idx & 7), jj = (idx >> 3) & 1;
-    uint4 out;
-    uint8_t* o = reinterpret_cast<uint8_t*>(&out);
-    uint8_t sb[2];
+    const int c = idx % (D / 2) * 2, jg = idx / (D / 2);
+    const __half* src = tile + (row0 + jg * 16) * (D + kPad) + c;
+    float2 x[16];
+    __half2 m2 = __half2(__half(0.0f), __half(0.0f));
 #pragma unroll
-    for (int g = 0; g < 2; ++g) {
-      float x[16];
-      float amax = 0.0f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        x[i] = __half2float(tile[(row0 + jj * 32 + g * 16 + i) * (D + kPad) + c]);
-        amax = fmaxf(amax, fabsf(x[i]));
-      }
-      sb[g] = nv_scale_byte(amax, gs);
-      const float dq = __fmul_rn(e4m3_to_float(sb[g]), gs);
-      const float inv_dq = __frcp_rn(dq);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[g * 8 + i] = e2m1_pair(x[2 * i], x[2 * i + 1], dq, inv_dq);
+    for (int i = 0; i < 16; ++i) {
+      const __half2 h = *reinterpret_cast<const __half2*>(src + i * (D + kPad));
+      m2 = max_abs2(m2, h);
+      x[i] = __half22float2(h);
     }
-    *reinterpret_cast<uint4*>(codes + (size_t)idx * 16) = out;
-    uint8_t* s = sf + rec::sf_offset(c, jj * 2);
-    *reinterpret_cast<uint16_t*>(s) = (uint16_t)sb[0] | ((uint16_t)sb[1] << 8);
+    const float2 amax = __half22float2(m2);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const uint8_t sb = nv_scale_byte(k ? amax.y : amax.x, gs);
+      const float dq = __fmul_rn(e4m3_to_float(sb), gs);
+      const float inv_dq = __frcp_rn(dq);
+      uint2 out;
+      uint8_t* o = reinterpret_cast<uint8_t*>(&out);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        o[i] = k ? e2m1_pair(x[2 * i].y, x[2 * i + 1].y, dq, inv_dq) : e2m1_pair(x[2 * i].x, x[2 * i + 1].x, dq, inv_dq);
+      *reinterpret_cast<uint2*>(codes + rec::tile_offset(c + k, jg >> 1, 2) + (jg & 1) * 8) = out;
+      sf[rec::sf_offset(c + k, jg)] = sb;
+    }
   }
 }
 
@@ -277,47 +304,68 @@ template <int D>
 // row order; padding rows are zero) instead of the maxima - the diag-Jensen draft map's input.
 __device__ __forceinline__ void write_pools(const __half* tile, int rows, int count, __half* mean,
                                             __half* maxp, bool second) {
-  if (threadIdx.x < D) {
-    const int c = threadIdx.x;
-    float sum = 0.0f, mx = -INFINITY, sq = 0.0f;
+  // a thread: two neighbouring channels, all rows in order
+  if (threadIdx.x < D / 2) {
+    const int c = threadIdx.x * 2;
+    const __half* src = tile + c;
+    float2 sum = make_float2(0.0f, 0.0f);
+    if (maxp == nullptr) {
+#pragma unroll 16
+      for (int r = 0; r < rows; ++r) {
+        const float2 x = __half22float2(*reinterpret_cast<const __half2*>(src + r * (D + kPad)));
+        sum.x = __fadd_rn(sum.x, x.x);
+        sum.y = __fadd_rn(sum.y, x.y);
+      }
+    } else {
+      float2 sq = make_float2(0.0f, 0.0f), mx = make_float2(-INFINITY, -INFINITY);
 #pragma unroll 8
-    for (int r = 0; r < rows; ++r) {
-      const float x = __half2float(tile[r * (D + kPad) + c]);
-      sum = __fadd_rn(sum, x);
-      sq = __fmaf_rn(x, x, sq);
-      if (r < count) mx = fmaxf(mx, x);
+      for (int r = 0; r < rows; ++r) {
+        const float2 x = __half22float2(*reinterpret_cast<const __half2*>(src + r * (D + kPad)));
+        sum.x = __fadd_rn(sum.x, x.x);
+        sum.y = __fadd_rn(sum.y, x.y);
+        if (second) {
+          sq.x = __fmaf_rn(x.x, x.x, sq.x);
+          sq.y = __fmaf_rn(x.y, x.y, sq.y);
+        } else if (r < count) {
+          mx.x = fmaxf(mx.x, x.x);
+          mx.y = fmaxf(mx.y, x.y);
+        }
+      }
+      if (second) mx = make_float2(__fdiv_rn(sq.x, (float)count), __fdiv_rn(sq.y, (float)count));
+      *reinterpret_cast<__half2*>(maxp + c) = __floats2half2_rn(mx.x, mx.y);
     }
-    mean[c] = __float2half_rn(__fdiv_rn(sum, (float)count));
-    if (maxp != nullptr) maxp[c] = __float2half_rn(second ? __fdiv_rn(sq, (float)count) : mx);
+    *reinterpret_cast<__half2*>(mean + c) =
+        __floats2half2_rn(__fdiv_rn(sum.x, (float)count), __fdiv_rn(sum.y, (float)count));
   }
 }
 
-template <typename InT, int QB, int D>
-__global__ void __launch_bounds__(kThreads) prepare_kernel(PrepParams p) {
+// Tasks of a head, in grid order: query tiles (video, prefix), then key/value blocks (R video blocks
+// of QB rows = QB/64 stages each, then the 64-row prefix stages).  With kSplit keys and values of a
+// block are separate CTAs (all keys first).
+template <typename InT, int QB, int D, bool kSplit>
+__global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __half* tile = reinterpret_cast<__half*>(smem_raw);
   __shared__ float red[kThreads / 32];
   __shared__ float recip[D];
 
-  layer::grid_dependency_wait();
   layer::grid_dependency_trigger();
   const int R = p.s.video_blocks;
   // heads vary fastest across concurrently running CTAs: neighbours read adjacent 2*D-byte
   // pieces of the same token rows
-  const int head = blockIdx.x;
-  const int task = blockIdx.y;
+  const int task = blockIdx.x / p.s.heads, head = blockIdx.x - task * p.s.heads;
   constexpr int kF = QB / 64;
-  const InT* q = static_cast<const InT*>(p.q);
-  const InT* k = static_cast<const InT*>(p.k);
-  const InT* v = static_cast<const InT*>(p.v);
   const int64_t qtiles_i8 = R + p.prefix_q_tiles;
 
-  if (task < R || task >= 2 * R + p.prefix_stages) {
+  if (task < qtiles_i8) {
     // ---------------- query tile (video or prefix) ----------------
+    // (after the maxima's kernel, whose CTAs all began when what was before it in the stream was
+    // complete; without INT8 there is no such kernel)
+    if (!p.s.has_int8) layer::grid_dependency_wait();
     const bool video = task < R;
-    const int t = video ? task : task - (2 * R + p.prefix_stages);
+    const int t = video ? task : task - R;
     const int valid = video ? p.counts[t] : min(QB, p.s.prefix_tokens - t * QB);
-    gather_tile<InT, D, QB>(tile, q, p, head, video, t * QB, t * QB, valid, p.stride[0],
+    gather_tile<InT, D, QB>(tile, static_cast<const InT*>(p.q), p, head, video, t * QB, t * QB, valid, p.stride[0],
                             p.stride[1]);
     __syncthreads();
     if (video) {
@@ -338,7 +386,7 @@ __global__ void __launch_bounds__(kThreads) prepare_kernel(PrepParams p) {
       }
     }
     if (p.s.has_int8) {
-      const int64_t slot = (int64_t)head * qtiles_i8 + (video ? t : R + t);
+      const int64_t slot = (int64_t)head * qtiles_i8 + task;
       const float amax = tile_amax<D>(tile, 0, QB, red);
       const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1.0e-7f);
       if (threadIdx.x == 0) p.o.q_int8_scale[slot] = scale;
@@ -348,58 +396,68 @@ __global__ void __launch_bounds__(kThreads) prepare_kernel(PrepParams p) {
     return;
   }
 
-  // ---------------- key/value block (video) or stage (prefix) ----------------
-  const bool video = task < 2 * R;
-  const int b = video ? task - R : task - 2 * R;
+  // ---------------- key or value block (video) or stage (prefix) ----------------
+  const int blocks = R + p.prefix_stages;
+  const bool second_half = kSplit && task >= qtiles_i8 + blocks;
+  const int block = task - (int)qtiles_i8 - (second_half ? blocks : 0);
+  const bool video = block < R;
+  const int b = video ? block : block - R;
   const int nst = video ? kF : 1;
   const int stage0 = video ? p.prefix_stages + b * kF : b;
   const int valid = video ? p.counts[b] : min(64, p.s.prefix_tokens - b * 64);
   const int64_t rec0 = (int64_t)head * p.stages + stage0;
-
-  if (video) {
-    gather_tile<InT, D, QB>(tile, k, p, head, true, b * QB, 0, valid, p.stride[2], p.stride[3]);
-  } else {
-    gather_tile<InT, D, 64>(tile, k, p, head, false, 0, b * 64, valid, p.stride[2], p.stride[3]);
-  }
-  __syncthreads();
-  if (video) {
-    __half* mean = static_cast<__half*>(p.o.k_pool) + ((int64_t)head * R + b) * D;
-    __half* mx = p.s.has_maxpool
-                     ? static_cast<__half*>(p.o.k_max_pool) + ((int64_t)head * R + b) * D
-                     : nullptr;
-    write_pools<D>(tile, QB, valid, mean, mx, p.s.has_maxpool == 2);
-  }
-  for (int g = 0; g < nst; ++g) {
-    if (p.s.has_fp16) {
-      write_fp16_tile<D>(static_cast<uint8_t*>(p.o.kv_fp16) + (rec0 + g) * rec::kv_fp16_bytes(D),
-                         tile, g * 64, 64);
+  if (!p.s.has_int8) layer::grid_dependency_wait();
+  auto gather = [&](const void* src, int64_t token_stride, int64_t head_stride) {
+    if (video) {
+      gather_tile<InT, D, QB>(tile, static_cast<const InT*>(src), p, head, true, b * QB, 0, valid, token_stride,
+                              head_stride);
+    } else {
+      gather_tile<InT, D, 64>(tile, static_cast<const InT*>(src), p, head, false, 0, b * 64, valid, token_stride,
+                              head_stride);
     }
-    if (p.s.has_int8) {
-      const float amax = tile_amax<D>(tile, g * 64, 64, red);
-      const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1.0e-7f);
-      if (threadIdx.x == 0) p.o.k_int8_scale[rec0 + g] = scale;
-      write_int8_tile<D>(static_cast<uint8_t*>(p.o.kv_int8) + (rec0 + g) * rec::kv_int8_bytes(D),
-                         tile, g * 64, 64, scale);
+  };
+  if (!second_half) {
+    gather(p.k, p.stride[2], p.stride[3]);
+    __syncthreads();
+    if (video) {
+      __half* mean = static_cast<__half*>(p.o.k_pool) + ((int64_t)head * R + b) * D;
+      __half* mx = p.s.has_maxpool
+                       ? static_cast<__half*>(p.o.k_max_pool) + ((int64_t)head * R + b) * D
+                       : nullptr;
+      write_pools<D>(tile, QB, valid, mean, mx, p.s.has_maxpool == 2);
     }
-    if (p.s.has_nvfp4) {
-      uint8_t* r4 = static_cast<uint8_t*>(p.o.kv_nvfp4) + (rec0 + g) * rec::kv_nvfp4_bytes(D);
-      write_nvfp4_rows<D>(r4, r4 + rec::kv_nvfp4_ksf_offset(D), tile, g * 64, 64,
-                          p.s.k_global_scale);
+    for (int g = 0; g < nst; ++g) {
+      if (p.s.has_fp16) {
+        write_fp16_tile<D>(static_cast<uint8_t*>(p.o.kv_fp16) + (rec0 + g) * rec::kv_fp16_bytes(D),
+                           tile, g * 64, 64);
+      }
+      if (p.s.has_nvfp4) {
+        uint8_t* r4 = static_cast<uint8_t*>(p.o.kv_nvfp4) + (rec0 + g) * rec::kv_nvfp4_bytes(D);
+        write_nvfp4_rows<D>(r4, r4 + rec::kv_nvfp4_ksf_offset(D), tile, g * 64, 64,
+                            p.s.k_global_scale);
+      }
+      if (p.s.has_int8) {
+        const float amax = tile_amax<D>(tile, g * 64, 64, red);
+        const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1.0e-7f);
+        if (threadIdx.x == 0) p.o.k_int8_scale[rec0 + g] = scale;
+        write_int8_tile<D>(static_cast<uint8_t*>(p.o.kv_int8) + (rec0 + g) * rec::kv_int8_bytes(D),
+                           tile, g * 64, 64, scale);
+      }
     }
+    if (kSplit) return;
+    __syncthreads();
   }
-  __syncthreads();
 
   // ---- values of the same rows ----
-  if (video) {
-    gather_tile<InT, D, QB>(tile, v, p, head, true, b * QB, 0, valid, p.stride[4], p.stride[5]);
-  } else {
-    gather_tile<InT, D, 64>(tile, v, p, head, false, 0, b * 64, valid, p.stride[4], p.stride[5]);
-  }
-  if (p.s.has_int8 && threadIdx.x < D) {
-    const float amax =
-        __half2float(__float2half_rn(p.o.v_amax[(int64_t)head * D + threadIdx.x]));
-    recip[threadIdx.x] = amax == 0.0f ? 0.0f : __fdiv_rn(2.25f, amax);
-    if (task == R) p.o.v_e4m3_scale[(int64_t)head * D + threadIdx.x] = __fdiv_rn(amax, 2.25f);
+  gather(p.v, p.stride[4], p.stride[5]);
+  if (p.s.has_int8) {
+    layer::grid_dependency_wait();
+    if (threadIdx.x < D) {
+      const float amax =
+          __half2float(__float2half_rn(p.o.v_amax[(int64_t)head * D + threadIdx.x]));
+      recip[threadIdx.x] = amax == 0.0f ? 0.0f : __fdiv_rn(2.25f, amax);
+      if (block == 0) p.o.v_e4m3_scale[(int64_t)head * D + threadIdx.x] = __fdiv_rn(amax, 2.25f);
+    }
   }
   __syncthreads();
   for (int g = 0; g < nst; ++g) {
@@ -437,7 +495,7 @@ struct Abs2<__nv_bfloat16> {
 // (integer max == float max).  `out` must be zeroed first.  A pure read of V, so HBM bound; the
 // maximum is taken in the input's own type (rounding to fp16 is monotonic and happens once at
 // the end).  One CTA = 32 vectors of 8 channels x 8 token lanes, four 16-byte loads in flight per
-// thread, and about eight CTAs per SM whatever the number of heads: with one thread per vector
+// thread, and about three CTAs per SM whatever the number of heads: with one thread per vector
 // walking 128 tokens alone, V of 7 heads x 33,272 tokens (60 MB) took 60 us, now 15.
 constexpr int kAmaxLanes = 8;
 template <typename InT>
@@ -491,10 +549,10 @@ __global__ void __launch_bounds__(32 * kAmaxLanes) v_amax_kernel(const InT* v, i
   }
 }
 
-template <typename InT, int QB, int D>
+template <typename InT, int QB, int D, bool kSplit>
 int launch(const PrepParams& p, cudaStream_t stream) {
   const size_t smem = (size_t)QB * (D + kPad) * sizeof(__half);
-  auto kernel = prepare_kernel<InT, QB, D>;
+  auto kernel = prepare_kernel<InT, QB, D, kSplit>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
@@ -502,18 +560,20 @@ int launch(const PrepParams& p, cudaStream_t stream) {
     if (cudaMemsetAsync(p.o.v_amax, 0, sizeof(float) * p.s.heads * D, stream) != cudaSuccess)
       return ANEMOI_SM100_ELAUNCH;
     const int chunks = (p.s.heads * D / 8 + 31) / 32;
-    // about eight CTAs per SM, each with at least two loads per thread
-    const int rows = max(1, 8 * 148 / chunks);
-    const int tokens_per_block = max(2 * kAmaxLanes, (p.s.seq_tokens + rows - 1) / rows);
+    // about three CTAs per SM, each with at least sixteen loads per thread: every CTA ends in 256 atomics
+    // (8 heads x 4,109 tokens with eight per SM and two loads: the preparation took 40 us, now 24)
+    const int rows = max(1, 3 * 148 / chunks);
+    const int tokens_per_block = max(16 * kAmaxLanes, (p.s.seq_tokens + rows - 1) / rows);
     dim3 grid(chunks, (p.s.seq_tokens + tokens_per_block - 1) / tokens_per_block);
     if (layer::launch(v_amax_kernel<InT>, grid, dim3(32 * kAmaxLanes), 0, stream, static_cast<const InT*>(p.v),
                       reinterpret_cast<int*>(p.o.v_amax), p.s.seq_tokens, p.s.heads, D / 8, p.stride[4],
                       p.stride[5], tokens_per_block) != cudaSuccess)
       return ANEMOI_SM100_ELAUNCH;
   }
-  const int tasks = 2 * p.s.video_blocks + p.prefix_stages + p.prefix_q_tiles;
-  if (tasks > 65535) return ANEMOI_SM100_ELIMIT;
-  dim3 grid(p.s.heads, tasks);
+  const int64_t blocks = (int64_t)p.s.video_blocks + p.prefix_stages;
+  const int64_t tasks = p.s.video_blocks + p.prefix_q_tiles + (kSplit ? 2 : 1) * blocks;
+  if (tasks * p.s.heads > INT32_MAX) return ANEMOI_SM100_ELIMIT;
+  const dim3 grid((unsigned)(tasks * p.s.heads));
   return layer::launch(kernel, grid, dim3(kThreads), smem, stream, p) == cudaSuccess ? ANEMOI_SM100_OK
                                                                                     : ANEMOI_SM100_ELAUNCH;
 }
@@ -572,9 +632,14 @@ extern "C" int anemoi_sm100_prepare(const anemoi_sm100_shape* shape, const void*
   p.stages = rec::stages(s);
   p.prefix_q_tiles = rec::prefix_query_tiles(s);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define ANEMOI_DISPATCH(T)                                                        \
-  (s.query_block == 64 ? (s.head_dim == 64 ? launch<T, 64, 64>(p, st) : launch<T, 64, 128>(p, st)) \
-                       : (s.head_dim == 64 ? launch<T, 128, 64>(p, st) : launch<T, 128, 128>(p, st)))
+  // Keys and values of a block in CTAs of their own: half the serial chain, which is quicker for
+  // 128-row blocks (sweep's 4 heads 71 -> 64 us, 56 heads x 85,184 tokens 2,178 -> 2,128) and for small grids; for
+  // many 64-row blocks a CTA's fixed cost weighs more (620 -> 687).
+  const bool split = s.query_block == 128 || ((int64_t)2 * s.video_blocks + p.prefix_stages) * s.heads <= 4 * 148;
+#define ANEMOI_DISPATCH(T)                                                                              \
+  (s.query_block == 128 ? (s.head_dim == 64 ? launch<T, 128, 64, true>(p, st) : launch<T, 128, 128, true>(p, st)) \
+   : split              ? (s.head_dim == 64 ? launch<T, 64, 64, true>(p, st) : launch<T, 64, 128, true>(p, st))   \
+                        : (s.head_dim == 64 ? launch<T, 64, 64, false>(p, st) : launch<T, 64, 128, false>(p, st)))
   return s.input_is_bf16 ? ANEMOI_DISPATCH(__nv_bfloat16) : ANEMOI_DISPATCH(__half);
 #undef ANEMOI_DISPATCH
 }
