@@ -540,13 +540,16 @@ __global__ void __launch_bounds__(kRowWarps * 32) anchor_emit_kernel(
 // histogram and, for short maps, its dozen barriers.  As five launches (and two more for the
 // pairs, whose merge was one lane per phase) the same work took, alone, 8 heads x 64 blocks: 22 us
 // in kernels and 20 in gaps; 56 heads x 672 blocks: 250 us; 56 heads x 592 pairs: 720 us.
+// Small maps are bound by the chain of barriers, so the scans of the three boundaries share theirs, the
+// CTAs of a cluster exchange their sums once, and a cluster of one uses the CTA's barrier: with its call
+// 4 heads x 64 pairs went from 22.5 to 19.3 us, 5 x 133 from 38.9 to 32.8, 8 x 33 from 22.5 to 18.4.
 constexpr int kFusedThreads = 1024;
 constexpr int kFusedWarps = kFusedThreads / 32;
 
 struct FusedShared {
   int block_sum[1024];   // items per 32 bins, this CTA's rows
-  int warp_sum[kFusedWarps];
-  int part[8];           // this CTA's totals, read by the CTAs behind it
+  int4 warp_sum[kFusedWarps];
+  int part[4];           // this CTA's sums over its rows, read by the CTAs behind it
   int hit_block[3], hit_off[3];
   int key[3], quota[3];
 };
@@ -570,28 +573,42 @@ inline bool fused_fits(int H, int R) {
   return H * ctas >= 74 || (int64_t)R * R / ctas <= 65536;
 }
 
-// Exclusive prefix of v over the CTA's threads; `total` gets the sum.
-__device__ __forceinline__ int fused_exclusive(int v, int* warp_sum, int& total) {
+// Exclusive prefixes of the N values over the CTA's threads (two barriers for all of them); `total`
+// gets the sums.
+template <int N>
+__device__ __forceinline__ void fused_exclusive(int (&v)[N], int4* warp_sum, int (&total)[N]) {
+  static_assert(N <= 4, "one int4 per warp");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = v;
+  int incl[N];
 #pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int n = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += n;
-  }
-  if (lane == 31) warp_sum[warp] = incl;
-  __syncthreads();
-  const int w = warp_sum[lane];
-  int winc = w;
+  for (int k = 0; k < N; ++k) incl[k] = v[k];
 #pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int n = __shfl_up_sync(0xffffffffu, winc, off);
-    if (lane >= off) winc += n;
-  }
-  total = __shfl_sync(0xffffffffu, winc, 31);
-  const int base = __shfl_sync(0xffffffffu, winc - w, warp);
+  for (int off = 1; off < 32; off <<= 1)
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int n = __shfl_up_sync(0xffffffffu, incl[k], off);
+      if (lane >= off) incl[k] += n;
+    }
+  if (lane == 31)
+#pragma unroll
+    for (int k = 0; k < N; ++k) reinterpret_cast<int*>(&warp_sum[warp])[k] = incl[k];
   __syncthreads();
-  return base + incl - v;
+  int w[N], winc[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) winc[k] = w[k] = reinterpret_cast<int*>(&warp_sum[lane])[k];
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1)
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int n = __shfl_up_sync(0xffffffffu, winc[k], off);
+      if (lane >= off) winc[k] += n;
+    }
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    total[k] = __shfl_sync(0xffffffffu, winc[k], 31);
+    v[k] = __shfl_sync(0xffffffffu, winc[k] - w[k], warp) + incl[k] - v[k];
+  }
+  __syncthreads();
 }
 
 constexpr int kAhead = 8;  // 32-column pieces of a row whose keys are loaded before the first is looked at
@@ -633,6 +650,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   FusedShared& sh = *reinterpret_cast<FusedShared*>(hist + kBins);
   cg::cluster_group cluster = cg::this_cluster();
   const int ctas = cluster.num_blocks(), me = cluster.block_rank();
+  auto sync_all = [&]() {
+    if (ctas > 1) {
+      cluster.sync();
+    } else {
+      __syncthreads();
+    }
+  };
   const int head = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lower = (1u << lane) - 1u;
@@ -672,13 +696,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
     if (lane == 0) sh.block_sum[warp * 32 + i] = sum;
   }
   if (threadIdx.x < 3) sh.hit_block[threadIdx.x] = -1;
-  cluster.sync();
+  if (threadIdx.x < 4) sh.part[threadIdx.x] = 0;
+  sync_all();
   {
     const int blk = 1023 - threadIdx.x;  // blocks in descending key order
     int total = 0;
     for (int c = 0; c < ctas; ++c) total += cluster.map_shared_rank(sh.block_sum, c)[blk];
-    int all;
-    const int above = fused_exclusive(total, sh.warp_sum, all);
+    int before[1] = {total}, all[1];
+    fused_exclusive(before, sh.warp_sum, all);
+    const int above = before[0];
     const int bound[3] = {b0, b1, b2};
 #pragma unroll
     for (int b = 0; b < 3; ++b)
@@ -711,7 +737,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       sh.quota[warp] = quota;
     }
   }
-  cluster.sync();  // the histograms are read; their space holds the rows' counts from here on
+  sync_all();  // the histograms are read; their space holds the rows' counts from here on
   const int key_b[3] = {sh.key[0], sh.key[1], sh.key[2]};
   const int quota_b[3] = {sh.quota[0], sh.quota[1], sh.quota[2]};
   int* stat = hist;                    // [mine][6]: keys above boundary 0-2, equal to its key 0-2
@@ -742,74 +768,52 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       v = lane == b ? gs : (lane == 3 + b ? es : v);
     }
     if (lane < 6) stat[i * 6 + lane] = v;
+    // the CTA's sums: keys equal to each boundary's key, keys above the last boundary
+    if (ctas > 1 && lane >= 2 && lane < 6) atomicAdd(&sh.part[lane - 2], v);
   }
-  __syncthreads();
+  sync_all();
   // ---- scans over the rows: position inside the straddling bins, stages per phase, list offset ----
   const int p = prefix_phase >= 0 ? prefix_stages : 0;
-  int carry[4] = {0, 0, 0, 0};
-  {
-    int own[3] = {0, 0, 0};
-    for (int i = threadIdx.x; i < mine; i += kFusedThreads)
+  int carry[4] = {0, 0, 0, 0};  // of the rows before: keys equal to each boundary's key, stages
+  for (int c = 0; c < me; ++c) {
+    const int* part = cluster.map_shared_rank(sh.part, c);
+    const int rows = min(R, (c + 1) * rows_per) - min(R, c * rows_per);
+    carry[3] += (part[0] + max(0, min(part[3], quota_b[2] - carry[2]))) * factor + rows * p;
 #pragma unroll
-      for (int b = 0; b < 3; ++b) own[b] += stat[i * 6 + 3 + b];
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      int all;
-      fused_exclusive(own[b], sh.warp_sum, all);
-      if (threadIdx.x == 0) sh.part[b] = all;
-    }
-    cluster.sync();
-    for (int c = 0; c < me; ++c)
-#pragma unroll
-      for (int b = 0; b < 3; ++b) carry[b] += cluster.map_shared_rank(sh.part, c)[b];
+    for (int b = 0; b < 3; ++b) carry[b] += part[1 + b];
   }
-  int sum_mine = 0;
   for (int i0 = 0; i0 < mine; i0 += kFusedThreads) {
     const int i = i0 + threadIdx.x;
     const bool in = i < mine;
-    int below[3];
+    int pre[3], all[3], below[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) pre[b] = in ? stat[i * 6 + 3 + b] : 0;
+    fused_exclusive(pre, sh.warp_sum, all);
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const int eq = in ? stat[i * 6 + 3 + b] : 0;
-      int all;
-      const int pre = carry[b] + fused_exclusive(eq, sh.warp_sum, all);
-      carry[b] += all;
+      pre[b] += carry[b];
+      carry[b] += all[b];
       // items of the straddling key in this row that still fall above the boundary
-      below[b] = in ? stat[i * 6 + b] + max(0, min(eq, quota_b[b] - pre)) : 0;
-      if (in) stat[i * 6 + 3 + b] = pre;
+      below[b] = in ? stat[i * 6 + b] + max(0, min(stat[i * 6 + 3 + b], quota_b[b] - pre[b])) : 0;
     }
     const int n0 = (below[2] - below[1]) * factor + (prefix_phase == 0 ? p : 0);  // NVFP4
     const int n1 = (below[1] - below[0]) * factor + (prefix_phase == 1 ? p : 0);  // INT8
     const int n2 = below[0] * factor + (prefix_phase == 2 ? p : 0);               // FP16
+    int off[1] = {in ? n0 + n1 + n2 : 0}, sum[1];
+    fused_exclusive(off, sh.warp_sum, sum);
+    off[0] += carry[3];
+    carry[3] += sum[0];
     if (in) {
+#pragma unroll
+      for (int b = 0; b < 3; ++b) stat[i * 6 + 3 + b] = pre[b];
       stat[i * 6] = n0;
       stat[i * 6 + 1] = n1;
       stat[i * 6 + 2] = n2;
       totals[i] = n0 + n1 + n2;
-      sum_mine += n0 + n1 + n2;
-    }
-  }
-  {
-    int all;
-    fused_exclusive(sum_mine, sh.warp_sum, all);
-    if (threadIdx.x == 0) sh.part[3] = all;
-    cluster.sync();
-    for (int c = 0; c < me; ++c) carry[3] += cluster.map_shared_rank(sh.part, c)[3];
-  }
-  for (int i0 = 0; i0 < mine; i0 += kFusedThreads) {
-    const int i = i0 + threadIdx.x;
-    const bool in = i < mine;
-    int all;
-    const int off = carry[3] + fused_exclusive(in ? totals[i] : 0, sh.warp_sum, all);
-    carry[3] += all;
-    if (in) {
-      offset[i] = off;
-      row_offset[(int64_t)head * R + r0 + i] = off;
-      int32_t* rc = row_counts + ((int64_t)head * R + r0 + i) * 4;
-      rc[0] = stat[i * 6];
-      rc[1] = stat[i * 6 + 1];
-      rc[2] = stat[i * 6 + 2];
-      if (kPairs) rc[3] = 0;  // no launch order of single blocks
+      offset[i] = off[0];
+      row_offset[(int64_t)head * R + r0 + i] = off[0];
+      // (with pairs there is no launch order of single blocks; the other kernel fills it in)
+      *reinterpret_cast<int4*>(row_counts + ((int64_t)head * R + r0 + i) * 4) = make_int4(n0, n1, n2, 0);
     }
   }
   __syncthreads();
@@ -906,7 +910,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   const int unit = kPairs ? 2 : 1;
   const int count = (R + unit - 1) / unit, per = rows_per / unit, first = r0 / unit;
   const int own = (mine + unit - 1) / unit;
-  cluster.sync();
+  sync_all();
   for (int j = threadIdx.x; j < count; j += kFusedThreads)
     every[j] = cluster.map_shared_rank(kPairs ? unions : totals, j / per)[j % per];
   __syncthreads();
@@ -918,7 +922,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
     for (int j = 0; j < count; ++j) rank += every[j] > len || (every[j] == len && j < me_i);
     order[rank * 4] = me_i + 1;
   }
-  cluster.sync();  // no CTA leaves while another may still read its totals
+  if (ctas > 1) cluster.sync();  // no CTA leaves while another may still read its totals
 }
 
 template <bool kPairs>
