@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import math
 from dataclasses import dataclass
+from functools import lru_cache
 
 import torch
 
@@ -169,31 +170,22 @@ def anemoi_attention(
         raise ValueError("Q sequence length must match layout.sequence_tokens")
     if scale is not None and not math.isclose(scale, 1.0 / math.sqrt(query.size(-1))):
         raise ValueError("scale must be None or 1/sqrt(head_dim)")
-    sparse = sparse_config if sparse_config else SparseConfig()
-    quant = quant_config if quant_config else QuantConfig()
-    calib = NVFP4Calibration() if calibration is None else calibration
+    sparse = sparse_config if sparse_config else _DEFAULT_SPARSE
+    quant = quant_config if quant_config else _DEFAULT_QUANT
+    calib = _DEFAULT_CALIBRATION if calibration is None else calibration
     if not isinstance(calib, NVFP4Calibration):
         raise TypeError("calibration must be NVFP4Calibration")
+    return _executor().attention_call(query, key, value, layout, layer, sparse, quant, calib)
 
-    from .executor import execute_ragged_attention
 
-    return execute_ragged_attention(
-        query,
-        key,
-        value,
-        prefix_tokens=layout.prefix_tokens,
-        video_shape=layout.video_shape,
-        layer=layer,
-        query_block_size=sparse.query_block_size,
-        sparsity_ratio=sparse.sparsity_for_layer(layer),
-        nvfp4_ratio=quant.nvfp4_ratio,
-        int8_ratio=quant.int8_ratio,
-        fp16_ratio=quant.fp16_ratio,
-        prefix_kv_precision=quant.prefix_kv_precision,
-        prefix_query_precision=quant.prefix_query_precision,
-        maxpool_weight=float(sparse.maxpool_weight),
-        nvfp4_scales=calib.scales,
-    )
+_DEFAULT_SPARSE, _DEFAULT_QUANT, _DEFAULT_CALIBRATION = SparseConfig(), QuantConfig(), NVFP4Calibration()
+
+
+@lru_cache(maxsize=1)
+def _executor():
+    from . import executor
+
+    return executor
 
 
 __all__ = [

@@ -14,12 +14,14 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 from functools import lru_cache
 
 import torch
 import torch.nn.functional as F
 
 from . import native
+from .api import NVFP4Calibration, QuantConfig, SparseConfig, VisualLayout
 from .layout import materialize_ragged_2d_layout
 from .routing import PHASE_ORDER, resolve_phases, route_counts, video_phases
 
@@ -346,35 +348,112 @@ _plan = lru_cache(maxsize=256)(_Plan)
 _Strides, _Scales = C.c_int64 * 6, C.c_float * 3
 
 
+@lru_cache(maxsize=256)
+def _scale_array(nvfp4_scales):
+    return _Scales(*nvfp4_scales)
+
+
+@lru_cache(maxsize=256)
+def _stride_array(*strides):
+    return _Strides(*strides)
+
+
 def _one_call(q, k, v, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape, query_block, prefix_kv, prefix_query,
               maxpool_weight, nvfp4_scales):
     """The whole call through ``anemoi_sm100_layer``: one workspace, one native function."""
-    device, dtype = q.device, q.dtype
     _, tokens, heads, dim = q.shape
-    plan = _plan(device, tokens, heads, dim, dtype, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape, query_block,
-                 prefix_kv, prefix_query, maxpool_weight, _PAIR_Q64)
-    current = torch.cuda.current_stream(device)
+    plan = _plan(q.device, tokens, heads, dim, q.dtype, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape,
+                 query_block, prefix_kv, prefix_query, maxpool_weight, _PAIR_Q64)
+    (_, q1, q2, _), (_, k1, k2, _), (_, v1, v2, _) = q.stride(), k.stride(), v.stride()
+    return _launch(plan, q, k, v, q.device, prefix_tokens, _stride_array(q1, q2, k1, k2, v1, v2),
+                   _scale_array(nvfp4_scales) if plan.uses_scales else None)
+
+
+def _launch(plan, q, k, v, device, prefix_tokens, strides, scales):
     prefix_out, prefix_ptr, prefix_rows = None, None, 0
     if prefix_tokens and not plan.native_prefix:
         # dense attention of the prefix rows on the caller's tensors, as the reference does
+        current = torch.cuda.current_stream(device)
         plan.side.wait_stream(current)
         with torch.cuda.stream(plan.side):
             prefix_out = F.scaled_dot_product_attention(
                 q[:, :prefix_tokens].permute(0, 2, 1, 3), k.permute(0, 2, 1, 3), v.permute(0, 2, 1, 3),
                 dropout_p=0.0, is_causal=False)[0].contiguous()
+        prefix_out.record_stream(current)
         prefix_ptr, prefix_rows = prefix_out.data_ptr(), prefix_tokens
     workspace = torch.empty(plan.bytes, dtype=torch.uint8, device=device)
-    out = torch.empty((1, tokens, heads, dim), dtype=dtype, device=device)
+    out = torch.empty(q.shape, dtype=q.dtype, device=device)
     code = plan.call(
-        plan.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(),
-        _Strides(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2)),
-        _Scales(*nvfp4_scales) if plan.uses_scales else None, prefix_ptr, prefix_rows, 1, out.data_ptr(),
-        workspace.data_ptr(), plan.bytes, current.cuda_stream, plan.side_handle)
+        plan.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, scales, prefix_ptr, prefix_rows, 1, out.data_ptr(),
+        workspace.data_ptr(), plan.bytes, torch._C._cuda_getCurrentRawStream(device.index), plan.side_handle)
     if code != 0:
         native._check(code, "anemoi_sm100_layer")
     native._count("layer", plan.launches)
-    if prefix_out is not None:
-        prefix_out.record_stream(current)
+    return out
+
+
+class _Checked:
+    """Configuration objects of the public call that a call has already gone through with, and the
+    arguments they come to.  The objects are frozen and checked themselves when they are made, so the
+    same ones (by identity: they are held here) need no second check; on a small call the checks cost
+    as much as the launches."""
+
+    __slots__ = ("layout", "sparse", "quant", "calib", "tokens", "plans", "pair")
+
+    def __init__(self, layout, sparse, quant, calib):
+        self.layout, self.sparse, self.quant, self.calib = layout, sparse, quant, calib
+        self.tokens = layout.sequence_tokens
+        self.plans = {}        # (device, heads, dim, dtype, sparsity) -> (plan, device, NVFP4 scales)
+        self.pair = _PAIR_Q64
+
+
+_FROZEN = (VisualLayout, SparseConfig, QuantConfig, NVFP4Calibration)
+_CHECKED: dict = {}
+_CHECKED_MOST, _CHECKED_LOCK = 64, threading.Lock()
+
+
+def attention_call(query, key, value, layout, layer, sparse, quant, calib):
+    """One public call: ``execute_ragged_attention``, less the checks that a call with the same
+    configuration objects has passed before."""
+    entry = _CHECKED.get((id(layout), id(sparse), id(quant), id(calib)))
+    index = query.get_device()
+    if entry is not None and index >= 0 and entry.pair is _PAIR_Q64 and not _PROFILE_NVTX and _STAGE_EVENTS is None:
+        shape, dtype = query.shape, query.dtype
+        sparsity = sparse.sparsity_for_layer(layer) if sparse.layer_sparsity_bands else sparse.sparsity_ratio
+        known = entry.plans.get((index, shape[2], shape[3], dtype, sparsity))
+        if (known is not None and shape[1] == entry.tokens and shape[0] == 1 and key.shape == shape
+                and value.shape == shape and key.dtype is dtype and value.dtype is dtype
+                and key.get_device() == index and value.get_device() == index):
+            plan, device, scales = known
+            (_, q1, q2, q3), (_, k1, k2, k3), (_, v1, v2, v3) = query.stride(), key.stride(), value.stride()
+            if (q3 == k3 == v3 == 1 and not (q1 | q2 | k1 | k2 | v1 | v2) % 8
+                    and not (query.data_ptr() | key.data_ptr() | value.data_ptr()) % 16):
+                return _launch(plan, query, key, value, device, layout.prefix_tokens,
+                               _stride_array(q1, q2, k1, k2, v1, v2), scales)
+    sparsity = sparse.sparsity_for_layer(layer)
+    maxpool_weight = float(sparse.maxpool_weight)
+    out = execute_ragged_attention(
+        query, key, value, prefix_tokens=layout.prefix_tokens, video_shape=layout.video_shape, layer=layer,
+        query_block_size=sparse.query_block_size, sparsity_ratio=sparsity, nvfp4_ratio=quant.nvfp4_ratio,
+        int8_ratio=quant.int8_ratio, fp16_ratio=quant.fp16_ratio, prefix_kv_precision=quant.prefix_kv_precision,
+        prefix_query_precision=quant.prefix_query_precision, maxpool_weight=maxpool_weight,
+        nvfp4_scales=calib.scales)
+    if (type(layout), type(sparse), type(quant), type(calib)) != _FROZEN:
+        return out                 # look-alikes may change between calls
+    if entry is None or entry.pair is not _PAIR_Q64:
+        entry = _Checked(layout, sparse, quant, calib)
+        with _CHECKED_LOCK:
+            while len(_CHECKED) >= _CHECKED_MOST:
+                del _CHECKED[next(iter(_CHECKED))]
+            _CHECKED[(id(layout), id(sparse), id(quant), id(calib))] = entry
+    device = query.device
+    if len(entry.plans) < 64:
+        plan = _plan(device, entry.tokens, query.size(2), query.size(3), query.dtype, layout.prefix_tokens,
+                     float(sparsity), float(quant.nvfp4_ratio), float(quant.int8_ratio), float(quant.fp16_ratio),
+                     layout.video_shape, sparse.query_block_size, quant.prefix_kv_precision,
+                     quant.prefix_query_precision, maxpool_weight, _PAIR_Q64)
+        entry.plans[(index, query.size(2), query.size(3), query.dtype, sparsity)] = (
+            plan, device, _scale_array(calib.scales) if plan.uses_scales else None)
     return out
 
 
