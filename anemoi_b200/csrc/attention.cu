@@ -15,8 +15,8 @@
 //   warp 13         S[128x64]  = Q K^T   kind::mxf4nvf4 / kind::i8 / kind::f16
 //   warp 14         O[128xD]  += P V     kind::mxf4nvf4 / kind::f8f6f4 / kind::f16
 //   warp 15         idle
-// TMEM columns: S0 [0,64), O [64,64+D), and at [192,256) the NVFP4 scale factors, the FP16 phase's Q
-// or (INT8 at D = 128) a second score buffer S1; D = 64 has S1 behind O in every phase.
+// TMEM columns: S0 [0,64), O [64,64+D), from 192 on the NVFP4 scale factors or the INT8 and FP16 phases'
+// Q; D = 64 has a second score buffer S1 behind O.
 //
 // Why this split.  A stage needs 8,192 exponentials = 512 cycles of the special-function unit and
 // 130-580 cycles of the tensor core per SM, but one warp's chain through a stage (wait for S, load
@@ -29,8 +29,9 @@
 // off the softmax warps' path; QK and PV are issued by different warps so that QK of a stage waits
 // for nothing but its key tile and its score buffer.
 // Measured per stage and SM at D = 128, cycles, with one softmax warpgroup -> now: NVFP4 1,282 -> 791,
-// INT8 1,394 -> 857, FP16 1,332 -> 1,050, the mixed layer of S = 85,184 (8 heads) 1,250 -> 900.  Now bound
-// by the special-function unit (66 % busy: 520 of INT8's cycles) and the waits around it; FP16 by
+// INT8 1,394 -> 835, FP16 1,332 -> 1,050, the mixed layer of S = 85,184 (8 heads) 1,250 -> 900.  Now bound
+// by issue slots and the special-function unit (each 66 % busy: 520 of INT8's 790 cycles at the clock it
+// ran at) and the waits around them - moving exponentials to the FMA pipe only adds issue slots -; FP16 by
 // shared memory, which moves 96 KB = 768 cycles' worth per stage, and, in long runs, by the power limit.
 //
 // P is stored over the stage's K tile, which the tensor core has finished reading when the scores
@@ -82,7 +83,7 @@ enum WaitRole : int { kSoftmaxRole = 0, kRescaleRole = 1, kMmaRole = 2 };
 constexpr int kTmemCols = 256;
 constexpr int kColS = 0;
 constexpr int kColO = 64;
-constexpr int kColQ = 192;     // FP16: D / 2 columns
+constexpr int kColQ = 192;     // INT8: D / 4 columns, FP16: D / 2
 constexpr int kColSfaQ = 192;  // 2 k-steps x 4 columns
 constexpr int kColSfbK = 200;  // 2 k-steps x 4 columns
 constexpr int kColSfaP = 208;
@@ -96,11 +97,7 @@ enum Cell : int { kNv = 0, kI8 = 1, kF16 = 2 };
 // Which cells a kernel is built for: one, or any mix.
 enum Cells : int { kAny = 3 };
 
-// Second score buffer: D = 128 aliases the scale-factor columns, D = 64 has room behind O.
-template <int D>
-struct Cols {
-  static constexpr int kS1 = D == 128 ? 192 : 128;
-};
+constexpr int kColS1 = 128;    // D = 64: second score buffer
 
 struct AttnParams {
   anemoi_sm100_shape s;
@@ -139,7 +136,7 @@ struct Shared {
   uint64_t p_full[kRing];     // per quadrant: P stored (softmax warp), O in the right scale (rescale warp)
   uint64_t m_full[4][kRing];  // running maxima of the quadrant's rows up to this stage published
   uint64_t v_full[kSplitValues];  // value tile landed (phases with buffers of their own for keys and values)
-  uint64_t q_moved;               // FP16: Q in tensor memory
+  uint64_t q_moved;               // INT8, FP16: Q in tensor memory
   uint64_t q_full, q_free;
   uint64_t s_full[2];  // scores ready, per softmax warpgroup (a waiter has to see every phase)
   uint64_t s_free[2];  // scores read, per score buffer
@@ -265,10 +262,11 @@ __host__ __device__ constexpr int rest_offset(int d, int cell) {
 __host__ __device__ constexpr int slot_bytes(int d, int cell) {
   return (rest_offset(d, cell) + record_bytes(d, cell) - k_bytes(d, cell) + 127) & ~127;
 }
-// FP16: Q is an operand in tensor memory, moved there from its region at the start of the phase.  As
-// a shared-memory operand a stage of D = 128 read 48 KB for QK alone (48 cycles of shared-memory
-// bandwidth per instruction of 36) and moved 128 KB = 1,024 cycles in all, which was the bound.
-// At D = 128 Q's 32 KB then serve keys and values, in buffers of their own: four for key tiles, held until
+// INT8 and FP16: Q is an operand in tensor memory, moved there from its region at the start of the
+// phase.  As a shared-memory operand an FP16 stage of D = 128 read 48 KB for QK alone (48 cycles of
+// shared-memory bandwidth per instruction of 36) and moved 128 KB = 1,024 cycles in all, which was the bound; INT8 gained
+// 2-4 % (16 heads of S = 33,272: 1.59 -> 1.55 ms; Q64, 8 heads of S = 38,247: 1.47 -> 1.41 ms).
+// At D = 128 the FP16 Q's 32 KB then serve keys and values, in buffers of their own: four for key tiles, held until
 // PV (P replaces them), and two for value tiles, which are not needed before the probabilities are there.
 __host__ __device__ constexpr bool split_kv(int d, int cell) { return d == 128 && cell == kF16; }
 __host__ __device__ constexpr int stage_bytes(int d, int cell) {  // distance of two slots
@@ -280,11 +278,11 @@ __host__ __device__ constexpr int slot_count(int ring, int d, int cell) {
   const int n = split_kv(d, cell) ? kSplitKeys : ring / slot_bytes(d, cell);
   return n < kRing ? n : kRing;
 }
-// Score buffer of stage g: the NVFP4 and FP16 phases of D = 128 have a single one (the other's
-// columns hold the scale factors or Q).
+// Score buffer of stage g: D = 128 has a single one, which the softmax warps have read, soon after the
+// scores arrived, long before the next stage's are needed.
 template <int D>
-__device__ __forceinline__ int s_buffer(int cell, int g) {
-  return D == 128 && cell != kI8 ? 0 : (g & 1);
+__device__ __forceinline__ int s_buffer(int g) {
+  return D == 128 ? 0 : (g & 1);
 }
 
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
@@ -395,11 +393,11 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
   const int at = g & (kRing - 1), before_at = (g - 1) & (kRing - 1);
   uint64_t* m_full = b->m_full[row >> 5];
   const uint32_t lead = (row & 31) == 0;
-  const int sb = s_buffer<D>(cell, g);
+  const int sb = s_buffer<D>(g);
   wait(&b->wc, &b->s_full[g & 1], w.s_par, 10);
   w.s_par ^= 1u;
   tc_fence_after_sync();
-  const uint32_t tmem_s = tmem_row + (sb ? Cols<D>::kS1 : kColS);
+  const uint32_t tmem_s = tmem_row + (sb ? kColS1 : kColS);
   float s[64];
   {
     uint32_t r[64];
@@ -488,7 +486,7 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
 // ------------------------------------------------------------------------------------------
 template <int D, int CELL>
 __device__ __forceinline__ void issue_qk(uint32_t tmem_s, uint32_t tmem, uint32_t q_addr,
-                                         uint32_t slot_addr) {
+                                         uint32_t slot_addr) {  // q_addr: NVFP4 only
   if (CELL == kF16) {
     constexpr uint32_t chunks = D / 8;
     constexpr uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, 64, 0, 0);
@@ -498,9 +496,9 @@ __device__ __forceinline__ void issue_qk(uint32_t tmem_s, uint32_t tmem, uint32_
   } else if (CELL == kI8) {
     constexpr uint32_t chunks = D / 16;
     constexpr uint32_t idesc = instr_desc(kFmtS8, kFmtS8, kAccS32, 128, 64, 0, 0);
-    const uint64_t qd = smem_desc(q_addr, 128, chunks * 128), kd = smem_desc(slot_addr, 128, chunks * 128);
+    const uint64_t kd = smem_desc(slot_addr, 128, chunks * 128);
 #pragma unroll
-    for (int k = 0; k < D / 32; ++k) mma_i8_ss(tmem_s, qd + k * 16, kd + k * 16, idesc, k > 0);
+    for (int k = 0; k < D / 32; ++k) mma_i8_ts(tmem_s, tmem + kColQ + k * 8, kd + k * 16, idesc, k > 0);
   } else {
     constexpr uint32_t chunks = D / 32;
     constexpr uint32_t idesc = instr_desc_nvf4(128, 64);
@@ -676,7 +674,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       const int64_t q_index_i8 =
           (int64_t)head * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks : 0) + block0;
       const float sigma = (D == 64 ? 0.125f : 0.08838834764831845f) * 1.4426950408889634f;
-      int phase_ord = 0, g = 0, v_fills = 0;
+      int phase_ord = 0, g = 0, v_fills = 0, moves = 0;
 #pragma unroll 1
       for (int cell = kFirst; cell <= kLast; ++cell) {
         const int n = b->cnt[cell];
@@ -754,7 +752,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           if (i < n) {
             if (i >= nslot)
               wait<kMmaRole>(&b->wc, &b->pv_done[(gi - nslot) & (kRing - 1)], ((gi - nslot) >> 3) & 1, 2);
-            if (split && i == 2) wait<kMmaRole>(&b->wc, &b->q_moved, 0, 2);
+            if (split && i == 2) wait<kMmaRole>(&b->wc, &b->q_moved, moves & 1, 2);
             const int at = gi & (kRing - 1);
             if (lane == (i & 31)) {
               b->meta[at][0] = meta_l[0];
@@ -786,6 +784,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         }
         g += n;
         ++phase_ord;
+        moves += cell != kNv;
       }
       if (b->wc.abort) {
         // unwinding: the copies in flight must land before the CTA gives its shared memory back
@@ -799,19 +798,19 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       // =============================== S = Q K^T ===============================
       // Uniform control flow for the whole warp; the tcgen05 instructions sit in elect.sync blocks.
       int g = 0, phase_ord = 0;
+      int moves = 0;
       uint32_t used = 0, free_par = 0;
       const uint32_t q_addr = smem_u32(q_smem), ring_addr = smem_u32(ring);
 #pragma unroll 1
       for (int cell = kFirst; cell <= kLast; ++cell) {
         const int n = b->cnt[cell];
         if (n == 0) continue;
-        if (cell == kF16) {
-          wait<kMmaRole>(&b->wc, &b->q_moved, 0, 3);
+        if (cell != kNv) {
+          wait<kMmaRole>(&b->wc, &b->q_moved, moves & 1, 3);
+          ++moves;
         } else {
           wait<kMmaRole>(&b->wc, &b->q_full, phase_ord & 1, 3);
         }
-        // the second score buffer takes the place of the NVFP4 phase's scale factors
-        if (CELLS == kAny && cell != kNv && b->cnt[kNv] > 0) wait<kMmaRole>(&b->wc, &b->nv_done, 0, 3);
         tc_fence_after_sync();
         const int nslot = slot_count(p.ring_bytes, D, cell);
         const uint32_t stride = stage_bytes(D, cell);
@@ -843,7 +842,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         int slot = first_slot(D, cell);
 #pragma unroll 1
         for (int i = 0; i < n; ++i, ++g) {
-          const int sb = s_buffer<D>(cell, g);
+          const int sb = s_buffer<D>(g);
           wait<kMmaRole>(&b->wc, &b->kv_full[g & (kRing - 1)], (g >> 3) & 1, 4);
           if ((used >> sb) & 1u) {
             wait<kMmaRole>(&b->wc, &b->s_free[sb], (free_par >> sb) & 1u, 5);
@@ -852,7 +851,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           used |= 1u << sb;
           tc_fence_after_sync();
           if (elect_one()) {
-            const uint32_t tmem_s = tmem + (sb ? Cols<D>::kS1 : kColS), slot_addr = base_addr + slot * stride;
+            const uint32_t tmem_s = tmem + (sb ? kColS1 : kColS), slot_addr = base_addr + slot * stride;
             if (cell == kI8) {
               issue_qk<D, kI8>(tmem_s, tmem, q_addr, slot_addr);
             } else if (cell == kNv) {
@@ -939,18 +938,18 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         }
         asm volatile("bar.sync 5, 128;" ::: "memory");
       }
-      if (cell == kF16) {
-        // Q into tensor memory.  Its columns are free: this quadrant's rows of every earlier score
-        // tile have been read (their maxima were published after that), and so have, after the NVFP4
-        // phase, its scale factors.
+      if (cell != kNv) {
+        // Q into tensor memory.  Its columns are free: the INT8 phase's Q has been read when the record
+        // that takes its place in shared memory arrives, the NVFP4 phase's scale factors below.
         if (CELLS == kAny && b->cnt[kNv] > 0) wait<kRescaleRole>(&b->wc, &b->nv_done, 0, 31);
         wait<kRescaleRole>(&b->wc, &b->q_full, phase_ord & 1, 32);
+        const int chunks = cell == kI8 ? D / 16 : D / 8;
 #pragma unroll 1
-        for (int c = 0; c < D / 8; c += 2) {
+        for (int c = 0; c < chunks; c += 2) {
           uint32_t r[8];
-          *reinterpret_cast<uint4*>(r) = *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c, D / 8));
+          *reinterpret_cast<uint4*>(r) = *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c, chunks));
           *reinterpret_cast<uint4*>(r + 4) =
-              *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c + 1, D / 8));
+              *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c + 1, chunks));
           tmem_st8(tmem_row + kColQ + c * 4, r);
         }
         tmem_wait_st();
