@@ -264,8 +264,8 @@ __host__ __device__ constexpr int slot_bytes(int d, int cell) {
 }
 // INT8 and FP16: Q is an operand in tensor memory, moved there from its region at the start of the
 // phase.  As a shared-memory operand an FP16 stage of D = 128 read 48 KB for QK alone (48 cycles of
-// shared-memory bandwidth per instruction of 36) and moved 128 KB = 1,024 cycles in all, which was the bound; INT8 gained
-// 2-4 % (16 heads of S = 33,272: 1.59 -> 1.55 ms; Q64, 8 heads of S = 38,247: 1.47 -> 1.41 ms).
+// shared-memory bandwidth per instruction of 36) and moved 128 KB = 1,024 cycles in all, which was the
+// bound; INT8 gained 2-4 % (16 heads of S = 33,272: 1.59 -> 1.55 ms; Q64, 8 heads of S = 38,247: 1.47 -> 1.41 ms).
 // At D = 128 the FP16 Q's 32 KB then serve keys and values, in buffers of their own: four for key tiles, held until
 // PV (P replaces them), and two for value tiles, which are not needed before the probabilities are there.
 __host__ __device__ constexpr bool split_kv(int d, int cell) { return d == 128 && cell == kF16; }
@@ -386,8 +386,12 @@ struct SoftmaxWalk {
   float alpha, sum;   // of this group's last stage
 };
 
-// One stage.
-template <int D, bool kPairs>
+// One stage.  Padding rows of a 64-row tile, and stages of the other query block of a pair (warp-uniform:
+// a warp's rows belong to one block), contribute nothing: P = 0, running maximum and denominator
+// untouched.  `kPass`: such a stage has a path of its own, without the scores.  A third of a pair's stages
+// are passed over so: Q64 kernels of one cell gain 1-3 % (INT8, 8 heads of S = 38,247: 1.42 -> 1.38 ms); the
+// mixed one, whose instruction cache is full, would lose 10 %.
+template <int D, bool kPairs, bool kPass>
 __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_t tmem_row, int row, int g, int cell,
                                               bool live_warp, int my_block, SoftmaxWalk& w) {
   const int at = g & (kRing - 1), before_at = (g - 1) & (kRing - 1);
@@ -398,6 +402,28 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
   w.s_par ^= 1u;
   tc_fence_after_sync();
   const uint32_t tmem_s = tmem_row + (sb ? kColS1 : kColS);
+  const auto store_zeros = [&]() {
+    const int chunks = p_bytes(cell) / 2048;
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) *reinterpret_cast<uint4*>(p_row + c * 128) = make_uint4(0, 0, 0, 0);
+  };
+  if (kPass && (!live_warp || __float_as_int(b->meta[at][my_block].y) < 0)) {
+    tc_fence_before_sync();
+    mbar_arrive_if(&b->s_free[sb], lead);
+    wait(&b->wc, &m_full[before_at], ((g - 1) >> 3) & 1, 9);
+    const float2 before = b->rec[before_at][row];
+    w.d = before.y * w.alpha + w.sum;
+    b->rec[at][row] = make_float2(before.x, w.d);
+    __syncwarp();
+    mbar_arrive_if(&m_full[at], lead);
+    w.alpha = 1.0f;
+    w.sum = 0.0f;
+    if (live_warp) store_zeros();
+    fence_proxy_async_smem();
+    __syncwarp();
+    mbar_arrive_if(&b->p_full[at], lead);
+    return;
+  }
   float s[64];
   {
     uint32_t r[64];
@@ -414,10 +440,7 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
   tc_fence_before_sync();
   __syncwarp();
   mbar_arrive_if(&b->s_free[sb], lead);
-  // Padding rows of a 64-row tile, and stages of the other query block of the pair (warp-uniform: a
-  // warp's rows belong to one block), contribute nothing: P = 0, running maximum and denominator
-  // untouched.
-  const bool active = !kPairs || (live_warp && valid >= 0);
+  const bool active = !kPairs || kPass || (live_warp && valid >= 0);
   float mx = -INFINITY;
   if (active) {
     if (cell == kI8) {
@@ -471,9 +494,7 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
     }
     w.sum = sum * sum_scale;
   } else if (live_warp) {
-    const int chunks = p_bytes(cell) / 2048;
-#pragma unroll 1
-    for (int c = 0; c < chunks; ++c) *reinterpret_cast<uint4*>(p_row + c * 128) = make_uint4(0, 0, 0, 0);
+    store_zeros();
   }
   fence_proxy_async_smem();
   tc_fence_before_sync();
@@ -1003,7 +1024,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       int slot = first_slot(D, cell) + first;
 #pragma unroll 1
       for (int i = first; i < n; i += 2) {
-        softmax_stage<D, kQ64>(b, p_row + slot * stride, tmem_row, row, g + i, cell, live_warp, my_block, w);
+        softmax_stage<D, kQ64, kQ64 && CELLS != kAny>(b, p_row + slot * stride, tmem_row, row, g + i, cell, live_warp,
+                                                        my_block, w);
         slot += 2;
         if (slot >= nslot) slot -= nslot;
       }
