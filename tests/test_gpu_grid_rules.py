@@ -1,0 +1,103 @@
+"""Kernels whose split of the work follows the size of the grid: each branch of the rule."""
+
+import numpy as np
+import pytest
+import torch
+
+from tests.helpers import Records, smooth_fields
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads, blocks, dim, weight", [
+    (1, 1, 64, 0.0),       # one query block per warp: a grid of at most 148 CTAs
+    (29, 40, 128, 0.5),
+    (60, 17, 64, 0.25),    # two: 180 CTAs of one, 120 of two
+    (2, 1185, 128, 0.5),   # two: four would not leave room for two CTAs on an SM
+    (80, 20, 128, 0.0),    # four
+    (75, 33, 64, 1.0),     # four, the last CTA with one block
+])
+def test_draft_rows_per_warp(native_library, heads, blocks, dim, weight):
+    """The draft map of pooled blocks, bit for bit the oracle's, first and last head."""
+    from anemoi_b200 import native
+    from oracle import route as R
+
+    shape = native.Shape(heads=heads, head_dim=dim, query_block=128, seq_tokens=blocks * 128, prefix_tokens=0,
+                         video_blocks=blocks, has_nvfp4=0, has_int8=1, has_fp16=0, has_prefix_query_int8=0,
+                         has_maxpool=int(weight != 0.0), input_is_bf16=1, q_global_scale=1.0, k_global_scale=1.0,
+                         v_global_scale=1.0)
+    g = torch.Generator().manual_seed(5)
+    pools = [torch.randn(heads, blocks, dim, generator=g).half() for _ in range(4)]
+    q, k, qx, kx = (t.cuda() for t in pools)
+    prob = torch.empty(heads, blocks, blocks, dtype=torch.float16, device="cuda")
+    p = native._ptr
+    assert native.library().anemoi_sm100_draft_probability(
+        shape, p(q), p(k), p(qx), p(kx), weight, p(prob), native._stream(prob.device)) == 0
+    for h in sorted({0, heads - 1}):
+        want = R.draft_probability(*(t[h].numpy() for t in pools), weight)
+        assert np.array_equal(prob[h].cpu().numpy().view(np.uint16), want.view(np.uint16))
+
+
+@pytest.mark.parametrize("dim, dtype", [(64, torch.float16), (128, torch.bfloat16)])
+def test_preparation_of_many_q64_heads(native_library, dim, dtype):
+    """32 heads of 9 Q64 blocks and a prefix (640 key and value tasks: one CTA per block for both)
+    against each head alone (20 tasks: a CTA each): the same records, scales and pools."""
+    from anemoi_b200 import executor
+
+    vs, heads, prefix = (3, 9, 21), 32, 70
+    q, k, v = (t.cuda() for t in smooth_fields(*vs, heads, dim, prefix, seed=2, outliers=(5, 41), dtype=dtype))
+    kw = dict(prefix_tokens=prefix, sparsity_ratio=0.5, retained_nvfp4_ratio=0.4, retained_int8_ratio=0.4,
+              retained_fp16_ratio=0.2, video_shape=vs, layer=0, query_block_size=64, maxpool_weight=0.5,
+              nvfp4_scales=(0.01, 0.01, 0.002), return_parts=True)
+
+    def prepared(*tensors):
+        _, parts = executor.sm100_ragged_attention(*tensors, **kw)
+        torch.cuda.synchronize()
+        return parts["store"], parts["shape"]
+
+    many = prepared(q, k, v)
+    assert (2 * many[1].video_blocks + 2) * heads == 640
+    for h in (0, heads - 1):
+        a = Records(*many, h)
+        b = Records(*prepared(*(t[:, :, h:h + 1].contiguous() for t in (q, k, v))), 0)
+        views = [(r.q_fp16(), *r.kv_fp16(), *r.q_int8(), *r.kv_int8(), *r.q_int8(prefix=True), *r.q_nvfp4(),
+                  *r.kv_nvfp4(), *(r.b[n][r.h] for n in ("q_pool", "k_pool", "q_max_pool", "k_max_pool")))
+                 for r in (a, b)]
+        for x, y in zip(*views):
+            assert x.dtype == y.dtype and x.tobytes() == y.tobytes()
+
+
+def test_repeated_public_calls(native_library):
+    """A call with configuration objects seen before skips their checks, not the tensors': other
+    strides, heads and types give what the staged path gives, and bad tensors still raise."""
+    from anemoi_b200 import QuantConfig, SparseConfig, VisualLayout, anemoi_attention, executor
+
+    vs, prefix = (2, 10, 14), 30
+    layout, sparse = VisualLayout(vs, prefix), SparseConfig(64, 0.5, ((0, 1, 0.5), (1, 2, 0.8)))
+    quant = QuantConfig(0.0, 0.5, 0.5)
+    tokens = layout.sequence_tokens
+
+    def call(q, k, v, layer=0):
+        return anemoi_attention(q, k, v, layout=layout, layer=layer, sparse_config=sparse, quant_config=quant)
+
+    def staged(q, k, v, layer=0):
+        return executor.sm100_ragged_attention(
+            q, k, v, prefix_tokens=prefix, sparsity_ratio=sparse.sparsity_for_layer(layer),
+            retained_nvfp4_ratio=0.0, retained_int8_ratio=0.5, retained_fp16_ratio=0.5, video_shape=vs, layer=layer,
+            query_block_size=64, return_parts=True)[0]
+
+    packed = torch.randn(1, tokens, 3, 3, 128, device="cuda", dtype=torch.bfloat16)
+    sets = [tuple(packed[:, :, i] for i in range(3)),
+            tuple(packed[:, :, i].contiguous() for i in range(3)),
+            tuple(packed[:, :, i, :2].half() for i in range(3))]
+    for _ in range(2):
+        for t in sets:
+            for layer in (0, 1):
+                assert torch.equal(call(*t, layer), staged(*t, layer))
+    q, k, v = sets[1]
+    shifted = torch.zeros(q.numel() + 1, dtype=q.dtype, device="cuda")[1:].view(q.shape)
+    for bad in ((q[:, :-1], k, v), (q, k[:, :-1], v), (q, k, v.half()), (q, k, v.cpu()), (q[..., :64], k, v),
+                (q, k, shifted)):
+        with pytest.raises(ValueError):
+            call(*bad)
+    assert torch.equal(call(q, k, v), staged(q, k, v))
