@@ -19,15 +19,18 @@ template <>
 __device__ __forceinline__ float to_float<__nv_bfloat16>(__nv_bfloat16 v) {
   return __bfloat162float(v);
 }
+// Two results rounded to T, in one register.
 template <typename T>
-__device__ __forceinline__ T from_float(float v);
+__device__ __forceinline__ uint32_t pack2(float a, float b);
 template <>
-__device__ __forceinline__ __half from_float<__half>(float v) {
-  return __float2half_rn(v);
+__device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
 template <>
-__device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) {
-  return __float2bfloat16_rn(v);
+__device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 // The steps of one row.  Every lane of the warp must call them (they shuffle inside groups of D/8
@@ -67,15 +70,19 @@ struct Rotary {
   }
 };
 
-// 8 consecutive table entries of a token's row: two 16-byte loads each.
-__device__ __forceinline__ void load_tables(const float* cos_row, const float* sin_row, int lane, float (&cs)[8],
-                                            float (&sn)[8]) {
+// 8 consecutive table entries of a token's row: two 16-byte loads each.  The first half's sines change
+// sign here: -pn * sn and pn * -sn are the same number.
+__device__ __forceinline__ void load_tables(const float* cos_row, const float* sin_row, int lane, bool first,
+                                            float (&cs)[8], float (&sn)[8]) {
   const float4* ct = reinterpret_cast<const float4*>(cos_row + lane * 8);
   const float4* st = reinterpret_cast<const float4*>(sin_row + lane * 8);
   *reinterpret_cast<float4*>(cs) = __ldg(ct);
   *reinterpret_cast<float4*>(cs + 4) = __ldg(ct + 1);
   *reinterpret_cast<float4*>(sn) = __ldg(st);
   *reinterpret_cast<float4*>(sn + 4) = __ldg(st + 1);
+  if (first)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sn[i] = -sn[i];
 }
 
 // Norm, weight and rotation; cs / sn: the table entries of the thread's channels, only read inside
@@ -85,16 +92,15 @@ __device__ __forceinline__ uint4 norm_rope_row(uint4 raw, uint4 wraw, float r, c
                                                const float (&cs)[8], const float (&sn)[8]) {
   const T* e = reinterpret_cast<const T*>(&raw);
   const T* w = reinterpret_cast<const T*>(&wraw);
-  uint4 packed;
-  T* o = reinterpret_cast<T*>(&packed);
+  float o[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float n = __fmul_rn(__fmul_rn(to_float<T>(e[i]), r), to_float<T>(w[i]));
     // every lane takes part in the shuffle; lanes outside the span read themselves
     const float pn = __shfl_sync(0xffffffffu, n, rot.partner, D / 8);
-    o[i] = from_float<T>(rot.in ? __fmaf_rn(rot.first ? -pn : pn, sn[i], __fmul_rn(n, cs[i])) : n);
+    o[i] = rot.in ? __fmaf_rn(pn, sn[i], __fmul_rn(n, cs[i])) : n;
   }
-  return packed;
+  return make_uint4(pack2<T>(o[0], o[1]), pack2<T>(o[2], o[3]), pack2<T>(o[4], o[5]), pack2<T>(o[6], o[7]));
 }
 
 // One row at once.  `cos_row` / `sin_row` point at the row's token in the fp32 tables ([rotary_dim]
@@ -104,8 +110,8 @@ __device__ __forceinline__ uint4 norm_rope8(uint4 raw, const T* weight, const fl
                                             const float* sin_row, int rotary_dim, float eps, int lane,
                                             bool live) {
   const Rotary rot(lane, rotary_dim);
-  float cs[8] = {0, 0, 0, 0, 0, 0, 0, 0}, sn[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (rot.in && live) load_tables(cos_row, sin_row, lane, cs, sn);
+  float cs[8] = {}, sn[8] = {};
+  if (rot.in && live) load_tables(cos_row, sin_row, lane, rot.first, cs, sn);
   const float r = inverse_rms<D>(square_sum<T, D>(raw), eps);
   return norm_rope_row<T, D>(raw, *reinterpret_cast<const uint4*>(weight + lane * 8), r, rot, cs, sn);
 }

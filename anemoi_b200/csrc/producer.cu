@@ -27,15 +27,18 @@ namespace {
 // thread, then the whole arithmetic) 33,272 tokens x 56 heads x 128 took 289 us = 3.3 TB/s.  Four rows
 // give four loads in flight, one read of the token's cos / sin entries and of the weights for all four,
 // and the square root and division of a row, which every lane of the group used to repeat, are
-// done once, by lane i for row i: 180 us = 5.3 TB/s, at 64 registers (80 registers, three CTAs per SM:
-// 218 us; two rows: 206; eight: 321).  One row per group where a token has no more than two heads.
+// done once, by lane i for row i: 180 us = 5.3 TB/s (two rows: 206; eight: 321).  With two results per
+// conversion and the sines' sign turned once, and 80 registers, so that nothing spills, in CTAs of two
+// warps: 166 us = 5.7 TB/s (of 128 threads 169, of 256 175; at 64 registers 205; with packed multiplications
+// 188).  One row per group where a token has no more than two heads.
+constexpr int kThreads = 64;
 template <typename T, int D, int kRows>
-__global__ void __launch_bounds__(256, 4) qknorm_rope_kernel(T* x, const T* weight, const float* cos_table,
+__global__ void __launch_bounds__(kThreads, 12) qknorm_rope_kernel(T* x, const T* weight, const float* cos_table,
                                                              const float* sin_table, uint32_t units, int quads,
                                                              int heads, int rotary_dim, float eps,
                                                              int64_t token_stride, int64_t head_stride) {
   constexpr int kLanes = D / 8;
-  const uint32_t unit = (blockIdx.x * 256u + threadIdx.x) / kLanes;
+  const uint32_t unit = (blockIdx.x * (uint32_t)kThreads + threadIdx.x) / kLanes;
   const int lane = threadIdx.x % kLanes;
   const bool in = unit < units;
   const uint32_t token = in ? unit / (uint32_t)quads : 0u;
@@ -50,7 +53,8 @@ __global__ void __launch_bounds__(256, 4) qknorm_rope_kernel(T* x, const T* weig
   const nr::Rotary rot(lane, rotary_dim);
   float cs[8], sn[8];
   if (rot.in && in)
-    nr::load_tables(cos_table + (int64_t)token * rotary_dim, sin_table + (int64_t)token * rotary_dim, lane, cs, sn);
+    nr::load_tables(cos_table + (int64_t)token * rotary_dim, sin_table + (int64_t)token * rotary_dim, lane, rot.first,
+                    cs, sn);
   const uint4 wraw = __ldg(reinterpret_cast<const uint4*>(weight + lane * 8));
   float mine = 0.0f;
 #pragma unroll
@@ -71,9 +75,9 @@ template <typename T, int D, int kRows>
 int launch_rows(void* x, const void* weight, const float* c, const float* s, int64_t tokens, int heads, int rotary,
                 float eps, const int64_t* strides, cudaStream_t st) {
   const int64_t quads = (heads + kRows - 1) / kRows, units = tokens * quads;
-  constexpr int64_t kUnits = 256 / (D / 8);
+  constexpr int64_t kUnits = kThreads / (D / 8);
   if (tokens * heads > 0x7fffffffLL) return ANEMOI_SM100_ELIMIT;
-  qknorm_rope_kernel<T, D, kRows><<<(unsigned)((units + kUnits - 1) / kUnits), 256, 0, st>>>(
+  qknorm_rope_kernel<T, D, kRows><<<(unsigned)((units + kUnits - 1) / kUnits), kThreads, 0, st>>>(
       static_cast<T*>(x), static_cast<const T*>(weight), c, s, (uint32_t)units, (int)quads, heads, rotary, eps,
       strides[0], strides[1]);
   return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
