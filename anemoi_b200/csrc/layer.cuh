@@ -37,18 +37,27 @@ int assemble_prefix(const anemoi_sm100_shape& s, const void* prefix_out, int64_t
 // their writes visible.  Between the short kernels of a small call that takes the 2-4 us gap of an
 // ordinary launch to about 1.
 template <typename... P, typename... A>
-cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+cudaError_t launch_cluster(void (*kernel)(P...), dim3 grid, dim3 cluster, dim3 block, size_t smem, cudaStream_t st,
+                           A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster.x;
+  attr[1].val.clusterDim.y = cluster.y;
+  attr[1].val.clusterDim.z = cluster.z;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster.x * cluster.y * cluster.z > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<A>(args))...);
+}
+template <typename... P, typename... A>
+cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  return launch_cluster(kernel, grid, dim3(1), block, smem, st, std::forward<A>(args)...);
 }
 
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

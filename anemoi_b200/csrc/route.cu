@@ -936,24 +936,11 @@ int launch_fused(const anemoi_sm100_shape& s, const void* probability, int64_t n
   // never launches the kernel without the opt-in for its dynamic shared memory.
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem()) != cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas, H);
-  cfg.blockDim = dim3(kFusedThreads);
-  cfg.dynamicSmemBytes = fused_smem();
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = ctas;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<const unsigned short*>(probability), R, fused_rows(R, ctas),
-                            (int)n16, (int)(n16 + n8), (int)(n16 + n8 + n4), s.query_block / 64,
-                            rec::prefix_stages(s), prefix_phase, capacity, row_offset, row_counts, stage_ids,
-                            pair_counts, pair_ids) == cudaSuccess
+  return layer::launch_cluster(kernel, dim3(ctas, H), dim3(ctas), dim3(kFusedThreads), fused_smem(), st,
+                               static_cast<const unsigned short*>(probability), R, fused_rows(R, ctas), (int)n16,
+                               (int)(n16 + n8), (int)(n16 + n8 + n4), s.query_block / 64, rec::prefix_stages(s),
+                               prefix_phase, capacity, row_offset, row_counts, stage_ids, pair_counts,
+                               pair_ids) == cudaSuccess
              ? ANEMOI_SM100_OK
              : ANEMOI_SM100_ELAUNCH;
 }

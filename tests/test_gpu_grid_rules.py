@@ -101,3 +101,25 @@ def test_repeated_public_calls(native_library):
         with pytest.raises(ValueError):
             call(*bad)
     assert torch.equal(call(q, k, v), staged(q, k, v))
+
+
+@pytest.mark.parametrize("video, heads, dim, dtype", [
+    ((1, 8, 16), 1, 64, torch.float16),        # one range of tokens
+    ((3, 12, 9), 5, 128, torch.bfloat16),      # three ranges and a half-empty group of channels
+    ((4, 16, 16), 3, 64, torch.bfloat16),      # eight: the largest cluster
+    ((3, 19, 18), 3, 64, torch.float16),       # nine: atomics
+    ((2, 8, 16), 130, 128, torch.float16),     # many heads
+])
+def test_value_maxima(native_library, video, heads, dim, dtype):
+    """max |v| per head and channel, with the largest value at either end of the sequence, twice."""
+    from anemoi_b200 import executor
+
+    tokens = int(np.prod(video))
+    q, k, v = (torch.randn(1, tokens, heads, dim, device="cuda").to(dtype) for _ in range(3))
+    for at in (0, tokens - 1):
+        v[0, at, :, 3:40:7] *= -8.0
+        _, parts = executor.sm100_ragged_attention(
+            q, k, v, prefix_tokens=0, sparsity_ratio=0.5, retained_nvfp4_ratio=0.0, retained_int8_ratio=1.0,
+            retained_fp16_ratio=0.0, video_shape=video, layer=0, query_block_size=64, return_parts=True)
+        got = parts["store"].buffers["v_amax"].view(heads, dim)
+        assert torch.equal(got, v[0].abs().amax(0).half().float())
