@@ -543,6 +543,8 @@ __global__ void __launch_bounds__(kRowWarps * 32) anchor_emit_kernel(
 // Small maps are bound by the chain of barriers, so the scans of the three boundaries share theirs, the
 // CTAs of a cluster exchange their sums once, and a cluster of one uses the CTA's barrier: with its call
 // 4 heads x 64 pairs went from 22.5 to 19.3 us, 5 x 133 from 38.9 to 32.8, 8 x 33 from 22.5 to 18.4.
+// Block sums by exchanges of halves instead of a reduction per block, scans only in warps that have rows,
+// and no look at columns past the row's end: 4 x 16 pairs 11.7 -> 7.7 us, 8 x 33 15.0 -> 10.2, 56 x 273 55 -> 46.
 constexpr int kFusedThreads = 1024;
 constexpr int kFusedWarps = kFusedThreads / 32;
 
@@ -574,11 +576,17 @@ inline bool fused_fits(int H, int R) {
 }
 
 // Exclusive prefixes of the N values over the CTA's threads (two barriers for all of them); `total`
-// gets the sums.
+// gets the sums.  Warps that are not `live` have zeros, take part in the barriers only and get nothing.
 template <int N>
-__device__ __forceinline__ void fused_exclusive(int (&v)[N], int4* warp_sum, int (&total)[N]) {
+__device__ __forceinline__ void fused_exclusive(int (&v)[N], int4* warp_sum, int (&total)[N], bool live = true) {
   static_assert(N <= 4, "one int4 per warp");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (!live) {
+    if (lane == 0) warp_sum[warp] = make_int4(0, 0, 0, 0);
+    __syncthreads();
+    __syncthreads();
+    return;
+  }
   int incl[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) incl[k] = v[k];
@@ -690,10 +698,25 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   }
   __syncthreads();
   // ---- the key that straddles each boundary (keys ranked from the largest down) ----
-#pragma unroll 4
-  for (int i = 0; i < 32; ++i) {
-    const int sum = __reduce_add_sync(0xffffffffu, hist[(warp * 32 + i) * 32 + lane]);
-    if (lane == 0) sh.block_sum[warp * 32 + i] = sum;
+  {
+    // eight lanes hold four bins each of a block, of eight blocks; every exchange halves the blocks a
+    // lane still sums, so that each ends with one
+    int sum[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int4 bins = *reinterpret_cast<const int4*>(hist + warp * 1024 + k * 128 + lane * 4);
+      sum[k] = (bins.x + bins.y) + (bins.z + bins.w);
+    }
+#pragma unroll
+    for (int half = 4; half > 0; half >>= 1) {
+      const bool upper = lane & half;
+#pragma unroll
+      for (int k = 0; k < half; ++k) {
+        const int got = __shfl_xor_sync(0xffffffffu, upper ? sum[k] : sum[k + half], half);
+        sum[k] = (upper ? sum[k + half] : sum[k]) + got;
+      }
+    }
+    sh.block_sum[warp * 32 + 4 * (lane & 7) + (lane >> 3)] = sum[0];
   }
   if (threadIdx.x < 3) sh.hit_block[threadIdx.x] = -1;
   if (threadIdx.x < 4) sh.part[threadIdx.x] = 0;
@@ -754,12 +777,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       int key[kAhead];
       fused_keys(src, j0, R, key);
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u)
+      for (int u = 0; u < kAhead; ++u) {
+        if (j0 + u * 32 >= R) break;
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
           g[b] += key[u] > key_b[b];
           e[b] += key[u] == key_b[b];
         }
+      }
     }
     int v = 0;
 #pragma unroll
@@ -785,10 +810,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   for (int i0 = 0; i0 < mine; i0 += kFusedThreads) {
     const int i = i0 + threadIdx.x;
     const bool in = i < mine;
-    int pre[3], all[3], below[3];
+    int pre[3], all[3] = {0, 0, 0}, below[3];
 #pragma unroll
     for (int b = 0; b < 3; ++b) pre[b] = in ? stat[i * 6 + 3 + b] : 0;
-    fused_exclusive(pre, sh.warp_sum, all);
+    const bool live = i0 + warp * 32 < mine;
+    fused_exclusive(pre, sh.warp_sum, all, live);
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       pre[b] += carry[b];
@@ -799,8 +825,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
     const int n0 = (below[2] - below[1]) * factor + (prefix_phase == 0 ? p : 0);  // NVFP4
     const int n1 = (below[1] - below[0]) * factor + (prefix_phase == 1 ? p : 0);  // INT8
     const int n2 = below[0] * factor + (prefix_phase == 2 ? p : 0);               // FP16
-    int off[1] = {in ? n0 + n1 + n2 : 0}, sum[1];
-    fused_exclusive(off, sh.warp_sum, sum);
+    int off[1] = {in ? n0 + n1 + n2 : 0}, sum[1] = {0};
+    fused_exclusive(off, sh.warp_sum, sum, live);
     off[0] += carry[3];
     carry[3] += sum[0];
     if (in) {
@@ -839,6 +865,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
         fused_keys(src, j0, R, key);
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
+          if (j0 + u * 32 >= R) break;
           const int stage = prefix_stages + (j0 + u * 32 + lane) * factor;
           const int c = fused_code(key[u], key_b, quota_b, run, lower);
 #pragma unroll
@@ -885,6 +912,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
         fused_keys(src_b, j0, has_b ? R : 0, kb);
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
+          if (j0 + u * 32 >= R) break;
           const int stage = prefix_stages + j0 + u * 32 + lane;
           const int ca = fused_code(ka[u], key_b, quota_b, run_a, lower);
           const int cb = fused_code(kb[u], key_b, quota_b, run_b, lower);
