@@ -544,7 +544,8 @@ __global__ void __launch_bounds__(kRowWarps * 32) anchor_emit_kernel(
 // CTAs of a cluster exchange their sums once, and a cluster of one uses the CTA's barrier: with its call
 // 4 heads x 64 pairs went from 22.5 to 19.3 us, 5 x 133 from 38.9 to 32.8, 8 x 33 from 22.5 to 18.4.
 // Block sums by exchanges of halves instead of a reduction per block, scans only in warps that have rows,
-// and no look at columns past the row's end: 4 x 16 pairs 11.7 -> 7.7 us, 8 x 33 15.0 -> 10.2, 56 x 273 55 -> 46.
+// and no look at columns past the row's end: 4 x 16 pairs 11.7 -> 7.7 us, 8 x 33 15.0 -> 10.2, 56 x 273 55 -> 46;
+// one sum for a boundary's two counts and eight lanes per launch rank: 56 x 273 -> 44, 4 x 672 52 -> 49.
 constexpr int kFusedThreads = 1024;
 constexpr int kFusedWarps = kFusedThreads / 32;
 
@@ -772,7 +773,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   // ---- per row: keys above and equal to each straddling key ----
   for (int i = warp; i < mine; i += kFusedWarps) {
     const unsigned short* src = map + (int64_t)(r0 + i) * R;
-    int g[3] = {0, 0, 0}, e[3] = {0, 0, 0};
+    int n[3] = {0, 0, 0};  // keys above | equal << 16 (a row has 4,096 at most)
     for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
       int key[kAhead];
       fused_keys(src, j0, R, key);
@@ -780,17 +781,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       for (int u = 0; u < kAhead; ++u) {
         if (j0 + u * 32 >= R) break;
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
-          g[b] += key[u] > key_b[b];
-          e[b] += key[u] == key_b[b];
-        }
+        for (int b = 0; b < 3; ++b) n[b] += key[u] > key_b[b] ? 1 : (key[u] == key_b[b] ? 1 << 16 : 0);
       }
     }
     int v = 0;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const int gs = __reduce_add_sync(0xffffffffu, g[b]), es = __reduce_add_sync(0xffffffffu, e[b]);
-      v = lane == b ? gs : (lane == 3 + b ? es : v);
+      const int both = __reduce_add_sync(0xffffffffu, n[b]);
+      v = lane == b ? both & 0xffff : (lane == 3 + b ? both >> 16 : v);
     }
     if (lane < 6) stat[i * 6 + lane] = v;
     // the CTA's sums: keys equal to each boundary's key, keys above the last boundary
@@ -943,12 +941,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
     every[j] = cluster.map_shared_rank(kPairs ? unions : totals, j / per)[j % per];
   __syncthreads();
   int32_t* order = (kPairs ? pair_counts + (int64_t)head * count * 4 : row_counts + (int64_t)head * count * 4) + 3;
-  for (int i = threadIdx.x; i < own; i += kFusedThreads) {
-    const int me_i = first + i, len = every[me_i];
+  // (eight lanes per position: a thread each was 273 steps for 273 blocks)
+  for (int i0 = 0; i0 < own; i0 += kFusedThreads / 8) {
+    const int i = i0 + threadIdx.x / 8, me_i = first + min(i, own - 1), len = every[me_i];
     int rank = 0;
-#pragma unroll 8
-    for (int j = 0; j < count; ++j) rank += every[j] > len || (every[j] == len && j < me_i);
-    order[rank * 4] = me_i + 1;
+#pragma unroll 4
+    for (int j = threadIdx.x & 7; j < count; j += 8) rank += every[j] > len || (every[j] == len && j < me_i);
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, off);
+    if (i < own && (threadIdx.x & 7) == 0) order[rank * 4] = me_i + 1;
   }
   if (ctas > 1) cluster.sync();  // no CTA leaves while another may still read its totals
 }
