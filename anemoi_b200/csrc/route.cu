@@ -559,21 +559,24 @@ struct FusedShared {
 
 __host__ __device__ inline size_t fused_smem() { return (size_t)kBins * 4 + sizeof(FusedShared); }
 
-// CTAs per head: as many as keep every head on an SM of its own at once, each with at least 16K
-// pairs; `rows_per` rows each (even, so that no pair of blocks is split).
+// CTAs per head: as many as keep every head on an SM of its own at once (clusters do not cross GPCs: 33 of
+// four fit, 37 are 33 us against 27; 15 of eight, 16 are 46 against 29), down to 64 rows each: two per warp.
+// With at least 16K pairs each, 5 heads x 133 blocks had one CTA per head, 27.6 us against 17.7, 16 x 234
+// two (29.9, 21.2), 7 x 273 four (29.2, 23.8); with 32 rows, 8 x 33 would be slower (11.3 against 10.1).
 inline int fused_ctas(int H, int R) {
   int c = 1;
-  while (c < 8 && (int64_t)R * R / c > 32768 && H * c * 2 <= 148) c *= 2;
+  while (c < 8 && R > 64 * c && H * c * 2 <= (c == 4 ? 120 : c == 2 ? 132 : 148)) c *= 2;
   return c;
 }
 inline int fused_rows(int R, int ctas) { return ((R + ctas - 1) / ctas + 1) & ~1; }
 // The rows' counts take the histogram's place, which bounds the rows of a CTA; and few heads with long
 // maps leave most SMs without work, where the launches over all rows are quicker (2 heads x 1,501
-// blocks: 163 us against 219; 7 heads x 672: 77 against 71).
+// blocks: 163 us against 219; 7 heads x 672: 77 against 71).  Heads in clusters of four are 16 at least:
+// 16 heads x 592 blocks 70 us against 82.
 inline bool fused_fits(int H, int R) {
   const int ctas = fused_ctas(H, R);
   if (R > 4096 || 9 * fused_rows(R, ctas) + R > kBins) return false;
-  return H * ctas >= 74 || (int64_t)R * R / ctas <= 65536;
+  return H * ctas >= (ctas == 4 ? 60 : 74) || (int64_t)R * R / ctas <= 65536;
 }
 
 // Exclusive prefixes of the N values over the CTA's threads (two barriers for all of them); `total`
