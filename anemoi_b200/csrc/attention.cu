@@ -626,8 +626,10 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   }
   // After a give-up anywhere on this device the status word stays set: later CTAs (of this and
   // of later launches, until the host clears the word) return at once instead of each running
-  // into its own wait limit.
-  if (*reinterpret_cast<volatile int32_t*>(p.status) != 0) return;
+  // into its own wait limit.  One thread reads the word for the whole CTA: another CTA may set it at any
+  // time, and if only some warps of this one left, the others would go on without tensor memory, without
+  // barriers or with a warpgroup short of the warps its setmaxnreg waits for.
+  if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t*>(p.status) != 0)) return;
 
   uint8_t* q_smem = smem;
   uint8_t* ring = smem + p.q_region;
