@@ -38,7 +38,8 @@ __global__ void __launch_bounds__(kThreads, 12) qknorm_rope_kernel(T* x, const T
                                                              int heads, int rotary_dim, float eps,
                                                              int64_t token_stride, int64_t head_stride) {
   constexpr int kLanes = D / 8;
-  const uint32_t unit = (blockIdx.x * (uint32_t)kThreads + threadIdx.x) / kLanes;
+  // (in units, not threads: 32 bits hold every unit that the launcher admits, threads are 8 or 16 times as many)
+  const uint32_t unit = blockIdx.x * (uint32_t)(kThreads / kLanes) + threadIdx.x / kLanes;
   const int lane = threadIdx.x % kLanes;
   const bool in = unit < units;
   const uint32_t token = in ? unit / (uint32_t)quads : 0u;
