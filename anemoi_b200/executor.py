@@ -348,9 +348,9 @@ _plan = lru_cache(maxsize=256)(_Plan)
 _Strides, _Scales = C.c_int64 * 6, C.c_float * 3
 
 
-@lru_cache(maxsize=256)
 def _scale_array(nvfp4_scales):
-    return _Scales(*nvfp4_scales)
+    # converted at every call: the caller's numbers may be a list's, or tensors whose values change
+    return _Scales(nvfp4_scales[0], nvfp4_scales[1], nvfp4_scales[2])
 
 
 @lru_cache(maxsize=256)
@@ -366,7 +366,7 @@ def _one_call(q, k, v, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape, 
                  query_block, prefix_kv, prefix_query, maxpool_weight, _PAIR_Q64)
     (_, q1, q2, _), (_, k1, k2, _), (_, v1, v2, _) = q.stride(), k.stride(), v.stride()
     return _launch(plan, q, k, v, q.device, prefix_tokens, _stride_array(q1, q2, k1, k2, v1, v2),
-                   _scale_array(nvfp4_scales) if plan.uses_scales else None)
+                   _scale_array(nvfp4_scales))
 
 
 def _launch(plan, q, k, v, device, prefix_tokens, strides, scales):
