@@ -14,7 +14,6 @@ from __future__ import annotations
 
 import ctypes as C
 import math
-import threading
 from functools import lru_cache
 
 import torch
@@ -303,6 +302,7 @@ class _Plan:
 
     def __init__(self, device, tokens, heads, dim, dtype, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape,
                  query_block, prefix_kv, prefix_query, maxpool_weight, pair_q64):
+        self.device = device
         video = video_phases(nvfp4, int8, fp16)
         if prefix_query not in ("int8", "fp16"):
             raise ValueError("prefix_query_precision must be int8 or fp16")
@@ -392,69 +392,50 @@ def _launch(plan, q, k, v, device, prefix_tokens, strides, scales):
     return out
 
 
-class _Checked:
-    """Configuration objects of the public call that a call has already gone through with, and the
-    arguments they come to.  The objects are frozen and checked themselves when they are made, so the
-    same ones (by identity: they are held here) need no second check; on a small call the checks cost
-    as much as the launches."""
-
-    __slots__ = ("layout", "sparse", "quant", "calib", "tokens", "plans", "pair")
-
-    def __init__(self, layout, sparse, quant, calib):
-        self.layout, self.sparse, self.quant, self.calib = layout, sparse, quant, calib
-        self.tokens = layout.sequence_tokens
-        self.plans = {}        # (device, heads, dim, dtype, sparsity) -> (plan, device, NVFP4 scales)
-        self.pair = _PAIR_Q64
+@lru_cache(maxsize=256)
+def _public_plan(index, heads, dim, dtype, video_shape, prefix_tokens, query_block, sparsity, maxpool_weight, nvfp4,
+                 int8, fp16, prefix_kv, prefix_query, pair_q64):
+    """The plan of a public call's configuration, after the checks that ``execute_ragged_attention`` makes
+    of it (those of the tensors are made at every call)."""
+    device = torch.device("cuda", index)
+    _check_backend(device, prefix_tokens, prefix_query, nvfp4, int8, fp16)
+    return _plan(device, prefix_tokens + math.prod(video_shape), heads, dim, dtype, prefix_tokens, float(sparsity),
+                 float(nvfp4), float(int8), float(fp16), video_shape, query_block, prefix_kv, prefix_query,
+                 float(maxpool_weight), pair_q64)
 
 
 _FROZEN = (VisualLayout, SparseConfig, QuantConfig, NVFP4Calibration)
-_CHECKED: dict = {}
-_CHECKED_MOST, _CHECKED_LOCK = 64, threading.Lock()
 
 
 def attention_call(query, key, value, layout, layer, sparse, quant, calib):
-    """One public call: ``execute_ragged_attention``, less the checks that a call with the same
-    configuration objects has passed before."""
-    entry = _CHECKED.get((id(layout), id(sparse), id(quant), id(calib)))
-    index = query.get_device()
-    if entry is not None and index >= 0 and entry.pair is _PAIR_Q64 and not _PROFILE_NVTX and _STAGE_EVENTS is None:
-        shape, dtype = query.shape, query.dtype
-        sparsity = sparse.sparsity_for_layer(layer) if sparse.layer_sparsity_bands else sparse.sparsity_ratio
-        known = entry.plans.get((index, shape[2], shape[3], dtype, sparsity))
-        if (known is not None and shape[1] == entry.tokens and shape[0] == 1 and key.shape == shape
-                and value.shape == shape and key.dtype is dtype and value.dtype is dtype
-                and key.get_device() == index and value.get_device() == index):
-            plan, device, scales = known
-            (_, q1, q2, q3), (_, k1, k2, k3), (_, v1, v2, v3) = query.stride(), key.stride(), value.stride()
-            if (q3 == k3 == v3 == 1 and not (q1 | q2 | k1 | k2 | v1 | v2) % 8
-                    and not (query.data_ptr() | key.data_ptr() | value.data_ptr()) % 16):
-                return _launch(plan, query, key, value, device, layout.prefix_tokens,
-                               _stride_array(q1, q2, k1, k2, v1, v2), scales)
+    """One public call: what ``execute_ragged_attention`` does, with the plan looked up by the values of the
+    configuration.  The four objects check themselves when they are made and are frozen, so only what none
+    of them sees alone is left (``_public_plan``); on a small call the whole chain of checks costs as much as the
+    launches.  Anything unusual - look-alike objects, tensors that do not fit, profiling - goes through
+    ``execute_ragged_attention``, which says what is wrong."""
     sparsity = sparse.sparsity_for_layer(layer)
-    maxpool_weight = float(sparse.maxpool_weight)
-    out = execute_ragged_attention(
+    shape, dtype, index = query.shape, query.dtype, query.get_device()
+    if (index >= 0 and (type(layout), type(sparse), type(quant), type(calib)) == _FROZEN
+            and dtype in (torch.float16, torch.bfloat16) and shape[0] == 1 and shape[3] in (64, 128)
+            and key.shape == shape and value.shape == shape and key.dtype is dtype and value.dtype is dtype
+            and query.is_cuda and key.get_device() == index and value.get_device() == index
+            and not _PROFILE_NVTX and _STAGE_EVENTS is None):
+        (_, q1, q2, q3), (_, k1, k2, k3), (_, v1, v2, v3) = query.stride(), key.stride(), value.stride()
+        if (q3 == k3 == v3 == 1 and not (q1 | q2 | k1 | k2 | v1 | v2) % 8
+                and not (query.data_ptr() | key.data_ptr() | value.data_ptr()) % 16):
+            plan = _public_plan(index, shape[2], shape[3], dtype, layout.video_shape, layout.prefix_tokens,
+                                sparse.query_block_size, sparsity, sparse.maxpool_weight, quant.nvfp4_ratio,
+                                quant.int8_ratio, quant.fp16_ratio, quant.prefix_kv_precision,
+                                quant.prefix_query_precision, _PAIR_Q64)
+            return _launch(plan, query, key, value, plan.device, layout.prefix_tokens,
+                           _stride_array(q1, q2, k1, k2, v1, v2),
+                           _Scales(calib.q_scale, calib.k_scale, calib.v_scale) if plan.uses_scales else None)
+    return execute_ragged_attention(
         query, key, value, prefix_tokens=layout.prefix_tokens, video_shape=layout.video_shape, layer=layer,
         query_block_size=sparse.query_block_size, sparsity_ratio=sparsity, nvfp4_ratio=quant.nvfp4_ratio,
         int8_ratio=quant.int8_ratio, fp16_ratio=quant.fp16_ratio, prefix_kv_precision=quant.prefix_kv_precision,
-        prefix_query_precision=quant.prefix_query_precision, maxpool_weight=maxpool_weight,
+        prefix_query_precision=quant.prefix_query_precision, maxpool_weight=float(sparse.maxpool_weight),
         nvfp4_scales=calib.scales)
-    if (type(layout), type(sparse), type(quant), type(calib)) != _FROZEN:
-        return out                 # look-alikes may change between calls
-    if entry is None or entry.pair is not _PAIR_Q64:
-        entry = _Checked(layout, sparse, quant, calib)
-        with _CHECKED_LOCK:
-            while len(_CHECKED) >= _CHECKED_MOST:
-                del _CHECKED[next(iter(_CHECKED))]
-            _CHECKED[(id(layout), id(sparse), id(quant), id(calib))] = entry
-    device = query.device
-    if len(entry.plans) < 64:
-        plan = _plan(device, entry.tokens, query.size(2), query.size(3), query.dtype, layout.prefix_tokens,
-                     float(sparsity), float(quant.nvfp4_ratio), float(quant.int8_ratio), float(quant.fp16_ratio),
-                     layout.video_shape, sparse.query_block_size, quant.prefix_kv_precision,
-                     quant.prefix_query_precision, maxpool_weight, _PAIR_Q64)
-        entry.plans[(index, query.size(2), query.size(3), query.dtype, sparsity)] = (
-            plan, device, _scale_array(calib.scales) if plan.uses_scales else None)
-    return out
 
 
 def _counts_key(layout) -> tuple:
@@ -497,6 +478,17 @@ def reset_status(device=None) -> None:
         word.zero_()
 
 
+def _check_backend(device, prefix_tokens, prefix_query, nvfp4, int8, fp16) -> None:
+    if device.type != "cuda":
+        raise RuntimeError("Anemoi attention requires an SM100 (B200) CUDA device")
+    capability = tuple(torch.cuda.get_device_capability(device))
+    if capability != (10, 0):
+        raise RuntimeError("Anemoi attention requires SM100 (B200)")
+    phases = video_phases(nvfp4, int8, fp16)
+    if prefix_tokens and prefix_query == "int8" and "int8" not in phases:
+        raise RuntimeError("prefix-query INT8 requires an active INT8 phase")
+
+
 def execute_ragged_attention(
     query: torch.Tensor,
     key: torch.Tensor,
@@ -516,14 +508,7 @@ def execute_ragged_attention(
     nvfp4_scales: tuple[float, float, float] = (1.0, 1.0, 1.0),
 ) -> torch.Tensor:
     """Dispatch the stable routing configuration to the sm_100a backend."""
-    if query.device.type != "cuda":
-        raise RuntimeError("Anemoi attention requires an SM100 (B200) CUDA device")
-    capability = tuple(torch.cuda.get_device_capability(query.device))
-    if capability != (10, 0):
-        raise RuntimeError("Anemoi attention requires SM100 (B200)")
-    phases = video_phases(nvfp4_ratio, int8_ratio, fp16_ratio)
-    if prefix_tokens and prefix_query_precision == "int8" and "int8" not in phases:
-        raise RuntimeError("prefix-query INT8 requires an active INT8 phase")
+    _check_backend(query.device, prefix_tokens, prefix_query_precision, nvfp4_ratio, int8_ratio, fp16_ratio)
     return sm100_ragged_attention(
         query,
         key,
