@@ -343,8 +343,9 @@ class _Plan:
         self.call = lib.anemoi_sm100_layer
 
 
-# One entry per configuration a process uses (a few hundred bytes each; the tables are the layout's).
-_plan = lru_cache(maxsize=256)(_Plan)
+# One entry per configuration a process uses (a few hundred bytes each; the tables are the layout's).  By type
+# too: 64.0 is refused as a block size whether or not 64 has been used.
+_plan = lru_cache(maxsize=256, typed=True)(_Plan)
 _Strides, _Scales = C.c_int64 * 6, C.c_float * 3
 
 

@@ -68,3 +68,21 @@ def test_refusals_do_not_depend_on_earlier_calls(native_library):
         twin.maxpool_weight = 2.0
         with pytest.raises(ValueError):
             call(q, k, v, sparse=twin)
+
+
+def test_block_size_of_another_type(native_library):
+    """Refused before and after the same call with an integer."""
+    from anemoi_b200 import executor
+
+    q, k, v = (torch.randn(1, 280, 2, 64, device="cuda", dtype=torch.float16) for _ in range(3))
+
+    def call(block):
+        return executor.sm100_ragged_attention(
+            q, k, v, prefix_tokens=0, sparsity_ratio=0.5, retained_nvfp4_ratio=0.0, retained_int8_ratio=1.0,
+            retained_fp16_ratio=0.0, video_shape=(2, 10, 14), layer=0, query_block_size=block)
+
+    executor._plan.cache_clear()
+    for _ in range(2):
+        with pytest.raises(TypeError):
+            call(64.0)
+        call(64)
