@@ -126,6 +126,11 @@ class HostAttention:
             if i + 1 < len(groups):
                 load(i + 1)
             dq, dk, dv = self._slot(i & 1, tokens, h1 - h0, dim, query.dtype, most)
+            if i < 2 or self.world > 1:
+                # this call's stream reads them, whichever stream's memory they are: a runner that is dropped
+                # while the call runs must not give them back before it is done
+                for t in (dq, dk, dv):
+                    t.record_stream(compute)
             compute.wait_event(ready[i])
             if self.world == 1:
                 result = anemoi_attention(dq, dk, dv, layout=layout, layer=layer, sparse_config=sparse_config,
