@@ -111,6 +111,8 @@ class HostAttention:
             raise ValueError("every head group must divide evenly over the ranks")
         ready, done, copied = {}, {}, {}
         self.copy_in.wait_stream(compute)
+        # an earlier call from another stream may still be reading the slots: its copies out follow its layers
+        self.copy_in.wait_stream(self.copy_out)
 
         def load(i):
             h0, h1 = groups[i]

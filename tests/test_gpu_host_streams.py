@@ -55,3 +55,24 @@ def test_runner_dropped_while_another_stream_computes(native_library, monkeypatc
         taken = [torch.full(s, float("nan"), dtype=torch.bfloat16, device="cuda") for s in sizes]
     torch.cuda.synchronize()
     assert len(taken) == 6 and torch.equal(out, want)
+
+
+def test_calls_from_two_streams_take_turns(native_library, monkeypatch):
+    """A call from a second stream while the first one's layers wait: its copies in must not overwrite the
+    slots that those layers still have to read."""
+    from anemoi_b200 import HostAttention
+
+    (q, k, v), out, how, want = _setup(1)
+    (q2, k2, v2), out2, _, want2 = _setup(2)
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    runner = HostAttention("cuda", group_heads=4)
+    runner(q, k, v, out, **how)
+    torch.cuda.synchronize()
+    out.zero_()
+    _slowly(monkeypatch, 50_000_000)
+    with torch.cuda.stream(first):
+        runner(q, k, v, out, **how)
+    with torch.cuda.stream(second):
+        runner(q2, k2, v2, out2, **how)
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and torch.equal(out2, want2)
