@@ -227,7 +227,8 @@ __device__ __forceinline__ void write_nvfp4_rows(uint8_t* codes, uint8_t* sf, co
         *reinterpret_cast<float2*>(x + 8 + 2 * i) = __half22float2(hb[i]);
         if (i > 0) m2 = max_abs2(max_abs2(m2, ha[i]), hb[i]);
       }
-      const float amax = __half2float(__hmax(m2.x, m2.y));
+      // (a group of NaNs alone has maximum zero, like one with no values: its scale byte and codes are zero)
+      const float amax = fmaxf(__half2float(__hmax(m2.x, m2.y)), 0.0f);
       sb[g] = nv_scale_byte(amax, gs);
       const float dq = __fmul_rn(e4m3_to_float(sb[g]), gs);
       const float inv_dq = __frcp_rn(dq);
