@@ -106,6 +106,10 @@ extern "C" int anemoi_sm100_qknorm_rope(void* x, const void* weight, const float
   // the pairing j <-> j + rotary_dim/2 must move whole 8-channel vectors
   if (rotary_dim < 0 || rotary_dim > head_dim || rotary_dim % 16) return ANEMOI_SM100_EINVAL;
   if (strides[0] % 8 || strides[1] % 8 || !(eps >= 0.0f)) return ANEMOI_SM100_EINVAL;
+  // every load and store takes 16 bytes
+  for (const void* p : {static_cast<const void*>(x), weight, static_cast<const void*>(cos_table),
+                        static_cast<const void*>(sin_table)})
+    if (reinterpret_cast<uintptr_t>(p) % 16) return ANEMOI_SM100_EINVAL;
   if (tokens == 0) return ANEMOI_SM100_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return is_bf16 ? launch<__nv_bfloat16>(x, weight, cos_table, sin_table, tokens, heads, head_dim, rotary_dim,

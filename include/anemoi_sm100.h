@@ -381,6 +381,7 @@ int anemoi_sm100_copy_rows(void* dst, int64_t dst_pitch, const void* src, int64_
  * rotary embedding, in place on Q or K.  x [tokens][heads][head_dim] 16-bit (strides[2] = token and
  * head stride in elements, multiples of 8; head_dim contiguous), weight [head_dim] in x's type,
  * cos/sin fp32 [tokens][rotary_dim]; rotary_dim a multiple of 16, at most head_dim (0: norm only).
+ * All pointers 16-byte aligned (ANEMOI_SM100_EINVAL otherwise).
  * Replaces the Triton kernel _qknorm_partial_rope_kernel / fused_qknorm_rope of
  * anemoi/models/minimax_h3/solengine/models/minimax_h3/optimized/fusions.py:208-274. */
 int anemoi_sm100_qknorm_rope(void* x, const void* weight, const float* cos_table,
