@@ -1,0 +1,48 @@
+"""Routing and the order of the launches where their rules change."""
+
+import ctypes as C
+
+import pytest
+import torch
+
+from tests.test_gpu_one_call import test_routing_lists_equal_the_oracle as lists_equal_the_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads, blocks, one_kernel", [
+    (75, 1100, 1),      # one CTA per head with more rows than threads: a second round of the scans
+    (16, 592, 1),       # clusters of four
+    (33, 400, 1),
+    (34, 400, 0),       # 68 CTAs in clusters of two, long maps: five kernels
+    (36, 672, 0),
+    (37, 400, 1),       # 74 CTAs
+    (2, 500, 1),        # few heads, clusters of eight: up to 65,536 pairs per CTA
+    (2, 800, 0),
+])
+def test_each_side_of_the_one_kernel_rule(native_library, heads, blocks, one_kernel):
+    from anemoi_b200 import native
+
+    shape = native.Shape(heads=heads, head_dim=128, query_block=64, seq_tokens=70 + blocks * 64, prefix_tokens=70,
+                         video_blocks=blocks, has_nvfp4=1, has_int8=1, has_fp16=1, has_prefix_query_int8=0,
+                         has_maxpool=0, input_is_bf16=1, q_global_scale=1.0, k_global_scale=1.0, v_global_scale=1.0)
+    assert native.library().anemoi_sm100_routes_in_one_kernel(C.byref(shape)) == one_kernel
+    lists_equal_the_oracle(native_library, heads, blocks, (0.4, 0.4, 0.2), 70, 1)
+
+
+@pytest.mark.parametrize("heads, query_block", [(18, 128), (19, 128), (18, 64), (19, 64)])
+def test_prefix_tiles_beside_and_after_routing(native_library, heads, query_block):
+    """A prefix of 1,000 tokens is eight tiles per head: 144 of them start before routing, whose clusters need SMs
+    of their own, 152 after it.  Bit for bit the stages."""
+    from anemoi_b200 import executor
+
+    vs, prefix = (5, 30, 52), 1000
+    gen = torch.Generator(device="cuda").manual_seed(heads)
+    q, k, v = (torch.randn(1, prefix + 7800, heads, 128, generator=gen, device="cuda").to(torch.bfloat16)
+               for _ in range(3))
+    kw = dict(prefix_tokens=prefix, sparsity_ratio=0.8, retained_nvfp4_ratio=0.0, retained_int8_ratio=0.5,
+              retained_fp16_ratio=0.5, video_shape=vs, layer=0, query_block_size=query_block)
+    staged, _ = executor.sm100_ragged_attention(q, k, v, return_parts=True, **kw)
+    for _ in range(3):
+        assert torch.equal(executor.sm100_ragged_attention(q, k, v, **kw), staged)
+    assert executor.last_status() == 0
