@@ -397,15 +397,14 @@ def _launch(plan, q, k, v, device, prefix_tokens, strides, scales):
 def _public_plan(index, heads, dim, dtype, video_shape, prefix_tokens, query_block, sparsity, maxpool_weight, nvfp4,
                  int8, fp16, prefix_kv, prefix_query, pair_q64):
     """The plan of a public call's configuration, after the checks that ``execute_ragged_attention`` makes
-    of it (those of the tensors are made at every call)."""
+    of it and of the tensors' type and head dimension (their other checks are made at every call)."""
     device = torch.device("cuda", index)
     _check_backend(device, prefix_tokens, prefix_query, nvfp4, int8, fp16)
+    if dim not in (64, 128) or dtype not in (torch.float16, torch.bfloat16):
+        raise ValueError("Q/K/V must be same-dtype CUDA [1,S,H,D], D in {64,128}")
     return _plan(device, prefix_tokens + math.prod(video_shape), heads, dim, dtype, prefix_tokens, float(sparsity),
                  float(nvfp4), float(int8), float(fp16), video_shape, query_block, prefix_kv, prefix_query,
                  float(maxpool_weight), pair_q64)
-
-
-_FROZEN = (VisualLayout, SparseConfig, QuantConfig, NVFP4Calibration)
 
 
 def attention_call(query, key, value, layout, layer, sparse, quant, calib):
@@ -414,29 +413,28 @@ def attention_call(query, key, value, layout, layer, sparse, quant, calib):
     of them sees alone is left (``_public_plan``); on a small call the whole chain of checks costs as much as the
     launches.  Anything unusual - look-alike objects, tensors that do not fit, profiling - goes through
     ``execute_ragged_attention``, which says what is wrong."""
-    sparsity = sparse.sparsity_for_layer(layer)
-    shape, dtype, index = query.shape, query.dtype, query.get_device()
-    if (index >= 0 and (type(layout), type(sparse), type(quant), type(calib)) == _FROZEN
-            and dtype in (torch.float16, torch.bfloat16) and shape[0] == 1 and shape[3] in (64, 128)
-            and key.shape == shape and value.shape == shape and key.dtype is dtype and value.dtype is dtype
-            and query.is_cuda and key.get_device() == index and value.get_device() == index
-            and not _PROFILE_NVTX and _STAGE_EVENTS is None):
+    index, shape, dtype = query.get_device(), query.shape, query.dtype
+    if (index >= 0 and type(layout) is VisualLayout and type(sparse) is SparseConfig and type(quant) is QuantConfig
+            and type(calib) is NVFP4Calibration and not _PROFILE_NVTX and _STAGE_EVENTS is None
+            and key.shape == shape and value.shape == shape and shape[0] == 1 and key.dtype is dtype
+            and value.dtype is dtype and key.get_device() == index and value.get_device() == index):
         (_, q1, q2, q3), (_, k1, k2, k3), (_, v1, v2, v3) = query.stride(), key.stride(), value.stride()
         if (q3 == k3 == v3 == 1 and not (q1 | q2 | k1 | k2 | v1 | v2) % 8
                 and not (query.data_ptr() | key.data_ptr() | value.data_ptr()) % 16):
-            plan = _public_plan(index, shape[2], shape[3], dtype, layout.video_shape, layout.prefix_tokens,
-                                sparse.query_block_size, sparsity, sparse.maxpool_weight, quant.nvfp4_ratio,
-                                quant.int8_ratio, quant.fp16_ratio, quant.prefix_kv_precision,
-                                quant.prefix_query_precision, _PAIR_Q64)
-            return _launch(plan, query, key, value, plan.device, layout.prefix_tokens,
-                           _stride_array(q1, q2, k1, k2, v1, v2),
+            prefix = layout.prefix_tokens
+            plan = _public_plan(
+                index, shape[2], shape[3], dtype, layout.video_shape, prefix, sparse.query_block_size,
+                sparse.sparsity_for_layer(layer) if sparse.layer_sparsity_bands else sparse.sparsity_ratio,
+                sparse.maxpool_weight, quant.nvfp4_ratio, quant.int8_ratio, quant.fp16_ratio,
+                quant.prefix_kv_precision, quant.prefix_query_precision, _PAIR_Q64)
+            return _launch(plan, query, key, value, plan.device, prefix, _stride_array(q1, q2, k1, k2, v1, v2),
                            _Scales(calib.q_scale, calib.k_scale, calib.v_scale) if plan.uses_scales else None)
     return execute_ragged_attention(
         query, key, value, prefix_tokens=layout.prefix_tokens, video_shape=layout.video_shape, layer=layer,
-        query_block_size=sparse.query_block_size, sparsity_ratio=sparsity, nvfp4_ratio=quant.nvfp4_ratio,
-        int8_ratio=quant.int8_ratio, fp16_ratio=quant.fp16_ratio, prefix_kv_precision=quant.prefix_kv_precision,
-        prefix_query_precision=quant.prefix_query_precision, maxpool_weight=float(sparse.maxpool_weight),
-        nvfp4_scales=calib.scales)
+        query_block_size=sparse.query_block_size, sparsity_ratio=sparse.sparsity_for_layer(layer),
+        nvfp4_ratio=quant.nvfp4_ratio, int8_ratio=quant.int8_ratio, fp16_ratio=quant.fp16_ratio,
+        prefix_kv_precision=quant.prefix_kv_precision, prefix_query_precision=quant.prefix_query_precision,
+        maxpool_weight=float(sparse.maxpool_weight), nvfp4_scales=calib.scales)
 
 
 def _counts_key(layout) -> tuple:

@@ -620,16 +620,6 @@ def tensor_peak(kind: str, device=None, iterations: int = 4096, repeats: int = 3
     return best
 
 
-def _table(t: torch.Tensor, device) -> torch.Tensor:
-    if t.dtype == torch.float32 and t.device == device and t.is_contiguous():
-        return t
-    return t.to(device=device, dtype=torch.float32).contiguous()
-
-
-def _aligned(t: torch.Tensor) -> torch.Tensor:
-    return t.clone() if t.data_ptr() % 16 else t
-
-
 def qknorm_rope_(x: torch.Tensor, weight: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
                  eps: float) -> torch.Tensor:
     """In place: per-head RMS norm with ``weight`` then partial rotary on ``x`` ``[tokens, heads, D]``
@@ -641,13 +631,20 @@ def qknorm_rope_(x: torch.Tensor, weight: torch.Tensor, cos: torch.Tensor, sin: 
         raise ValueError("weight must be a contiguous [D] tensor of x's dtype")
     if cos.shape != sin.shape or cos.ndim != 2 or cos.size(0) != tokens:
         raise ValueError("cos and sin must be [tokens, rotary_dim]")
-    if not x.is_cuda or weight.device != x.device:
+    device = x.device
+    if not x.is_cuda or weight.device != device:
         raise ValueError("x and weight must be on one CUDA device")
-    # the kernel reads weights and tables 16 bytes at a time: slices that start elsewhere are copied
-    weight, cos, sin = _aligned(weight), _aligned(_table(cos, x.device)), _aligned(_table(sin, x.device))
+    if cos.dtype != torch.float32 or cos.device != device or not cos.is_contiguous():
+        cos = cos.to(device=device, dtype=torch.float32).contiguous()
+    if sin.dtype != torch.float32 or sin.device != device or not sin.is_contiguous():
+        sin = sin.to(device=device, dtype=torch.float32).contiguous()
+    w_at, cos_at, sin_at = weight.data_ptr(), cos.data_ptr(), sin.data_ptr()
+    if (w_at | cos_at | sin_at) % 16:
+        # the kernel reads them 16 bytes at a time: slices that start elsewhere are copied
+        weight, cos, sin = (t.clone() if t.data_ptr() % 16 else t for t in (weight, cos, sin))
+        w_at, cos_at, sin_at = weight.data_ptr(), cos.data_ptr(), sin.data_ptr()
     _check(library().anemoi_sm100_qknorm_rope(
-        x.data_ptr(), weight.data_ptr(), cos.data_ptr(), sin.data_ptr(), tokens, heads, d, cos.size(1), float(eps),
-        int(x.dtype == torch.bfloat16), (C.c_int64 * 2)(x.stride(0), x.stride(1)),
-        torch.cuda.current_stream(x.device).cuda_stream),
+        x.data_ptr(), w_at, cos_at, sin_at, tokens, heads, d, cos.size(1), float(eps), int(x.dtype == torch.bfloat16),
+        (C.c_int64 * 2)(x.stride(0), x.stride(1)), torch.cuda.current_stream(device).cuda_stream),
            "anemoi_sm100_qknorm_rope")
     return x

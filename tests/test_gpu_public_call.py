@@ -60,6 +60,8 @@ def test_refusals_do_not_depend_on_earlier_calls(native_library):
             call(q.float(), k.float(), v.float())
         with pytest.raises(ValueError):
             call(*(t.expand(2, -1, -1, -1) for t in (q, k, v)))
+        with pytest.raises(ValueError, match="share"):
+            call(q, k[0], v)
         with pytest.raises(RuntimeError):
             call(q.cpu(), k.cpu(), v.cpu())
         twin = SimpleNamespace(query_block_size=64, sparsity_ratio=0.8, layer_sparsity_bands=(), maxpool_weight=0.0,
