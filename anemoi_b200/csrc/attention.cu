@@ -28,8 +28,8 @@
 // and the exponentials of two stages overlap.  O's rescale, which waits for the previous PV, is
 // off the softmax warps' path; QK and PV are issued by different warps so that QK of a stage waits
 // for nothing but its key tile and its score buffer.
-// Measured per stage and SM at D = 128, cycles, with one softmax warpgroup -> now: NVFP4 1,282 -> 791,
-// INT8 1,394 -> 835, FP16 1,332 -> 1,050, the mixed layer of S = 85,184 (8 heads) 1,250 -> 900.  Now bound
+// Measured per stage and SM at D = 128, cycles, one softmax warpgroup / two: NVFP4 1,282 / 791,
+// INT8 1,394 / 835, FP16 1,332 / 1,050, the mixed layer of S = 85,184 (8 heads) 1,250 / 900.  Bound
 // by issue slots and the special-function unit (each 66 % busy: 520 of INT8's 790 cycles at the clock it
 // ran at) and the waits around them - moving exponentials to the FMA pipe only adds issue slots -; FP16 by
 // shared memory, which moves 96 KB = 768 cycles' worth per stage, and, in long runs, by the power limit.

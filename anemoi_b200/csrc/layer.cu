@@ -2,15 +2,19 @@
 // prefix attention, with the results written straight to their tokens.
 //
 // A small call is bound by its launches, not by its kernels: with one Python wrapper, allocation and
-// marshaling per stage the 1,024-token call spent 200 us on the host for 70 us of kernels.  Here the
-// host work is one function: one workspace cut up by offsets, fourteen launches less three (routing
-// is one kernel, the output needs no assembly pass), programmatic dependent launches between them.
+// marshaling per stage the 1,024-token call takes 210 us, here 31 (25 of them host time).  The host work
+// is one function: one workspace cut up by offsets, four to six kernels (routing is one for most shapes,
+// the output needs no assembly pass), programmatic dependent launches between them.
 //
 // Order of the launches.  The prefix rows' tiles walk every stage of the head: few CTAs, each as
 // long as the whole video launch of a small call, so they start on the side stream as soon as the
-// operands are there and run beside draft and routing.  When they alone fill the GPU
-// they would only keep draft and routing waiting for a free SM (each CTA holds half of one for up to
-// milliseconds): then they start after routing, in front of the video tiles.
+// operands are there and run beside draft and routing.  When there is one for every SM they start after
+// routing, in front of the video tiles: a CTA holds half of an SM for up to milliseconds, and the routing
+// kernel needs a whole one's shared memory.  Where they leave routing few SMs the two orders are close; early /
+// late, D = 128, a 1,000-token prefix (eight tiles per head): 18 heads (144 tiles) with 7,800 video tokens 400 /
+// 419 us, 32,760 tokens 3.09 / 3.11 ms, 84,672 tokens 15.11 / 14.99 ms; 12 heads of the latter 10.05 / 10.01; past
+// the line, 24 heads (192 tiles), 526 / 550 us and 20.02 / 19.94 ms.  With few tiles early is the quicker one (8
+// heads, 16 tiles, 7,800 tokens: 183 / 221 us).
 #include <cuda_runtime.h>
 
 #include "layer.cuh"
@@ -19,7 +23,7 @@
 namespace {
 
 constexpr int64_t kAlign = 256;
-constexpr int kPrefixFillsGpu = 148;  // prefix CTAs from which they start after routing
+constexpr int kPrefixFillsGpu = 148;  // prefix CTAs from which they start after routing: one per SM
 
 int64_t up(int64_t n) { return (n + kAlign - 1) / kAlign * kAlign; }
 

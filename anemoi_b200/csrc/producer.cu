@@ -24,13 +24,14 @@ namespace {
 
 // A group of D/8 consecutive lanes takes kRows heads of one token, 8 channels per thread.  HBM bound
 // (read + write of x), which takes loads in flight: with one row per group (a 16-byte load per
-// thread, then the whole arithmetic) 33,272 tokens x 56 heads x 128 took 289 us = 3.3 TB/s.  Four rows
+// thread, then the whole arithmetic) 33,272 tokens x 56 heads x 128 take 289 us = 3.3 TB/s.  Four rows
 // give four loads in flight, one read of the token's cos / sin entries and of the weights for all four,
-// and the square root and division of a row, which every lane of the group used to repeat, are
-// done once, by lane i for row i: 180 us = 5.3 TB/s (two rows: 206; eight: 321).  With two results per
-// conversion and the sines' sign turned once, and 80 registers, so that nothing spills, in CTAs of two
-// warps: 166 us = 5.7 TB/s (of 128 threads 169, of 256 175; at 64 registers 205; with packed multiplications
-// 188).  One row per group where a token has no more than two heads.
+// and the square root and division of a row, which every lane of the group would repeat, are
+// done once, by lane i for row i: 180 us (two rows: 206; eight: 321).  With two results per conversion and
+// the sines' sign turned once, and 80 registers, so that nothing spills, in CTAs of two warps: 166-170 us = 5.7 TB/s
+// over one tensor again and again (of 128 threads 169, of 256 175; at 64 registers 205; with packed multiplications
+// 188); Q and K of a model in turn, 333-360 us, 82-88 % of a plain copy's rate.  One row per group where a token
+// has no more than two heads.
 constexpr int kThreads = 64;
 template <typename T, int D, int kRows>
 __global__ void __launch_bounds__(kThreads, 12) qknorm_rope_kernel(T* x, const T* weight, const float* cos_table,

@@ -537,15 +537,11 @@ __global__ void __launch_bounds__(kRowWarps * 32) anchor_emit_kernel(
 // order; with kPairs the union lists of the Q64 query-block pairs instead of the rows' own lists.
 // The CTAs of a cluster add up histograms and row totals through distributed shared memory.  The
 // map is read three times from L2; what bounds the kernel is the shared-memory atomics of the
-// histogram and, for short maps, its dozen barriers.  As five launches (and two more for the
-// pairs, whose merge was one lane per phase) the same work took, alone, 8 heads x 64 blocks: 22 us
-// in kernels and 20 in gaps; 56 heads x 672 blocks: 250 us; 56 heads x 592 pairs: 720 us.
-// Small maps are bound by the chain of barriers, so the scans of the three boundaries share theirs, the
-// CTAs of a cluster exchange their sums once, and a cluster of one uses the CTA's barrier: with its call
-// 4 heads x 64 pairs went from 22.5 to 19.3 us, 5 x 133 from 38.9 to 32.8, 8 x 33 from 22.5 to 18.4.
-// Block sums by exchanges of halves instead of a reduction per block, scans only in warps that have rows,
-// and no look at columns past the row's end: 4 x 16 pairs 11.7 -> 7.7 us, 8 x 33 15.0 -> 10.2, 56 x 273 55 -> 46;
-// one sum for a boundary's two counts and eight lanes per launch rank: 56 x 273 -> 44, 4 x 672 52 -> 49.
+// histogram and, for short maps, its dozen barriers.  Those are why the scans of the three boundaries share
+// theirs, the CTAs of a cluster exchange their sums once, a cluster of one uses the CTA's barrier, block sums
+// go by exchanges of halves and only warps that have rows scan.  Alone, in several launches (five, seven with
+// pairs) / in this one, us: 8 heads x 33 blocks 34 / 9.0, 8 x 64 34 / 10.5, 56 x 273 75 / 46, 56 x 672 235 / 190; with pairs
+// 4 x 16 40 / 6.8, 56 x 592 277 / 122.
 constexpr int kFusedThreads = 1024;
 constexpr int kFusedWarps = kFusedThreads / 32;
 
@@ -559,20 +555,23 @@ struct FusedShared {
 
 __host__ __device__ inline size_t fused_smem() { return (size_t)kBins * 4 + sizeof(FusedShared); }
 
-// CTAs per head: as many as keep every head on an SM of its own at once (clusters do not cross GPCs: 33 of
-// four fit, 37 are 33 us against 27; 15 of eight, 16 are 46 against 29), down to 64 rows each: two per warp.
-// With at least 16K pairs each, 5 heads x 133 blocks had one CTA per head, 27.6 us against 17.7, 16 x 234
-// two (29.9, 21.2), 7 x 273 four (29.2, 23.8); with 32 rows, 8 x 33 would be slower (11.3 against 10.1).
+// CTAs per head: as many as keep every head on an SM of its own at once, down to 64 rows each (two per
+// warp; 8 heads x 33 blocks take 9.0 us in one CTA each, 10.1 in two).  Clusters do not cross GPCs, so 15 of eight fit
+// at a time and 33 of four.  672 blocks, us: 15 heads in clusters of eight 59, of four 105; 16 heads 115, 105; 33 heads
+// in clusters of four 105, of two 188; 37 heads 208, 188; 66 heads in clusters of two 191, of one 359.
 inline int fused_ctas(int H, int R) {
   int c = 1;
   while (c < 8 && R > 64 * c && H * c * 2 <= (c == 4 ? 120 : c == 2 ? 132 : 148)) c *= 2;
   return c;
 }
 inline int fused_rows(int R, int ctas) { return ((R + ctas - 1) / ctas + 1) & ~1; }
-// The rows' counts take the histogram's place, which bounds the rows of a CTA; and few heads with long
-// maps leave most SMs without work, where the launches over all rows are quicker (2 heads x 1,501
-// blocks: 163 us against 219; 7 heads x 672: 77 against 71).  Heads in clusters of four are 16 at least:
-// 16 heads x 592 blocks 70 us against 82.
+// The rows' counts take the histogram's place, which bounds the rows of a CTA.  Otherwise one kernel where at
+// least half the SMs have a CTA (of clusters of four, 60), or a CTA has no more than 65,536 pairs: few heads with
+// long maps leave most SMs without work, and launches over all rows are quicker.  Lists, us in several kernels / in
+// one: 2 heads x 500 blocks 52 / 37, 7 x 672 75 / 58, 16 x 592 90 / 84, 66 x 672 277 / 191; refused 2 x 1,501 163 / 228,
+// 4 x 1,000 104 / 108, 36 x 672 160 / 188; on the wrong side of the line 34 x 400 86 / 79 and 37 x 672 166 / 188.  The line is
+// that of the lists; pair lists, which cost two kernels more, would gain beyond it (2 x 1,501 225 / 174, 36 x 672
+// 246 / 150).
 inline bool fused_fits(int H, int R) {
   const int ctas = fused_ctas(H, R);
   if (R > 4096 || 9 * fused_rows(R, ctas) + R > kBins) return false;

@@ -63,8 +63,9 @@ class HostAttention:
 
     def _groups(self, heads: int, bytes_per_head: int) -> list[tuple[int, int]]:
         """Head ranges, in order.  What nothing overlaps is the last group's layer and its copy out,
-        so the last groups shrink (4, 4, 4, 2, 1, 1 for 16 heads: 9.2 -> 8.4 ms at 33,272 tokens), as
-        long as a head's three copies in (55 GB/s) take longer than a call costs on the host."""
+        so the last groups shrink (4, 4, 4, 2, 1, 1 for 16 heads: 8.6 ms at 33,272 tokens, 9.2 with four
+        groups of 4), as long as a head's three copies in (55 GB/s) take longer than a call costs on
+        the host."""
         groups = [(h, min(h + self.group_heads, heads)) for h in range(0, heads, self.group_heads)]
         while self.world == 1 and bytes_per_head >= _TAPER_BYTES and groups[-1][1] - groups[-1][0] > 1:
             first, last = groups.pop()

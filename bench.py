@@ -650,6 +650,9 @@ def run_ours(args) -> None:
             # attention, assemble; with N > 1 also pack and merge)
             "gpu_launches": launches,
             "stage_ms": stages,
+            "stage_note": "calls taken apart by events outside the timed region: stage by stage with an assembly pass, "
+                          "draft and routing beside the prefix rows; the layer time is of the one-call path, whose "
+                          "attention launch writes the tokens itself and overlaps its neighbours",
             "roofline": {"bound": "tensor", "kernel": "attention_kernel<128> (video query blocks)",
                          "achieved": achieved, "peak": mixed_peak, "unit": "TFLOP/s",
                          "frac": (achieved / mixed_peak) if achieved else None, "traffic": traffic,
