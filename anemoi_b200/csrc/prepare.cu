@@ -10,7 +10,7 @@
 // Between HBM and issue bound: maxima are taken two halves at a time, V is read two channels
 // at a time (lanes side by side; single halves 16 rows apart met in four banks), codes are
 // packed by the converting instructions.  With the maxima of V, 56 heads, prefix 512: S = 85,184 (11.5 GB)
-// 2,180 us = 5.3 TB/s, S = 33,272 730; Q64 INT8, S = 38,247 600; 8 heads x 4,109 tokens 24 (a half at a time,
+// 2,180-2,280 us = 5.1-5.3 TB/s, S = 33,272 730; Q64 INT8, S = 38,247 600; 8 heads x 4,109 tokens 24 (a half at a time,
 // codes packed by shifts: 2,544, 845, 794 and 48).
 //
 // Numeric contract (reference: csrc/attention/cuda/sm120/q128_microscaling_preparation.cu):
