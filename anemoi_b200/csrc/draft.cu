@@ -15,6 +15,13 @@
 //           xor butterfly 16, 8, 4, 2, 1
 //   prob    f16_rn(e * (1/sum)), IEEE reciprocal; blend f16_rn((1-w)*pm + w*px)
 // A CPU restatement with the same sequence reproduces the map bit for bit.
+//
+// Bound by the FMA pipe (56 heads x 672 blocks x 128 channels: 90 us of FMAs) and, as it is read here, as much again
+// of shared memory and conversions; the softmax takes some 60 us.  Before / now, us: that map 312 / 262, 56 x 592
+// 266 / 217, 7 x 672 51 / 38, 4 x 672 x 64 31 / 24, 7 x 273 with two maps 35 / 27, 8 x 33 with two 11.3 / 7.7.  What
+// changed: all channels of a key tile at a time instead of 64 (half the barriers), keys in shared memory as fp16
+// (half the bytes), both maps in one walk; the exponentials packed and without conversion
+// instructions, and kept between the sum and the quotients.
 #include <cuda_fp16.h>
 
 #include "layer.cuh"
@@ -24,7 +31,6 @@ namespace {
 
 constexpr int kWarps = 8;
 constexpr int kChunk = 128;                   // key blocks per pass: 4 per lane
-constexpr int kPitch = kChunk + 4;            // floats per channel row of the key tile
 constexpr int kSlab = 64;                     // channels of the key tile held at a time
 constexpr int kMaxBlocks = 4096;              // rows per head the shared-memory buffers allow
 
@@ -43,106 +49,235 @@ __device__ __forceinline__ float exp_canonical(float t) {
   return __fmul_rn(p, __int_as_float((static_cast<int>(n) + 127) << 23));
 }
 
-// fp16 logits of kWarps * RPW query blocks against every key block of the head.  Each warp owns
-// RPW (1, 2 or 4) rows, each lane four key columns of the 128-column pass: per channel one 16-byte
-// load of keys (four shared-memory wavefronts per warp) and one broadcast load of the warp's
-// query values feed 4 * RPW FMAs, so with four rows the FMA pipe rather than shared memory
-// sets the pace.  Every logit is still the plain channel-ordered FMA chain (the canonical
-// order).
-template <int D, int RPW>
-__device__ __forceinline__ void row_logits(const __half* q_pool, const __half* k_pool, int head,
-                                           int R, int row0, float* kc, float* qs, __half* lg,
-                                           int lg_stride) {
-  constexpr int kRows = kWarps * RPW;
+__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "mov.b64 rc, {%6, %7};\n\tfma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
+// fp16 logits of kWarps * RPW query blocks against every key block of the head, for one pair of pools or two.
+// Each warp owns RPW (1, 2 or 4) rows, each lane four key columns of the 128-column pass.  The key tile holds
+// all channels, as it comes (fp16, two channels of a column in a word, so that one 16-byte load
+// serves two channels of four columns); query values are floats, read by broadcasts.  Every logit is still
+// the plain channel-ordered FMA chain (the canonical order).
+template <int D, int RPW, int kMaps>
+__device__ __forceinline__ void row_logits(const __half* const (&q_pool)[2], const __half* const (&k_pool)[2], int head,
+                                           int R, int row0, uint32_t* kc, float* qs, __half* lg, int groups) {
+  constexpr int kRows = kWarps * RPW, kThreads = kWarps * 32;
+  constexpr int kLoads = kChunk * (D / 8) / kThreads;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float scale = D == 64 ? 0.125f : __int_as_float(0x3db504f3);
-  // query pools as floats, the rows of a warp interleaved: qs[warp][channel][RPW]
-  for (int idx = threadIdx.x; idx < kRows * D; idx += kWarps * 32) {
-    const int r = idx / D, c = idx % D;
-    const int row = row0 + r;
-    qs[((r / RPW) * D + c) * RPW + (r % RPW)] =
-        row < R ? __half2float(q_pool[((int64_t)head * R + row) * D + c]) : 0.0f;
-  }
-  // Key pools of columns [c0, c0 + kChunk), kSlab channels at a time, as [channel][column] floats (the
-  // chain still runs over c = 0..D-1).  The next piece is loaded while this one is multiplied.
-  constexpr int kSlabs = D / kSlab, kLoads = kChunk * (kSlab / 8) / (kWarps * 32);
-  const int pieces = (R + kChunk - 1) / kChunk * kSlabs;
+  const int chunks = (R + kChunk - 1) / kChunk;
+  // the next tile is on its way while this one is multiplied
   uint4 raw[kLoads];
-  auto fetch = [&](int piece) {
-    const int c0 = piece / kSlabs * kChunk, s0 = piece % kSlabs * kSlab;
+  const auto fetch = [&](int piece) {
+    const __half* src = (kMaps == 2 && piece >= chunks ? k_pool[1] : k_pool[0]) + (int64_t)head * R * D;
+    const int c0 = (kMaps == 2 && piece >= chunks ? piece - chunks : piece) * kChunk;
 #pragma unroll
     for (int i = 0; i < kLoads; ++i) {
-      const int idx = threadIdx.x + i * kWarps * 32, col = c0 + idx % kChunk, c8 = idx / kChunk;
+      const int idx = threadIdx.x + i * kThreads, col = c0 + idx % kChunk;
       raw[i] = make_uint4(0, 0, 0, 0);
-      if (col < R) raw[i] = __ldg(reinterpret_cast<const uint4*>(k_pool + ((int64_t)head * R + col) * D + s0) + c8);
+      if (col < R) raw[i] = __ldg(reinterpret_cast<const uint4*>(src + (int64_t)col * D) + idx / kChunk);
     }
   };
   fetch(0);
   const float* qw = qs + warp * D * RPW;
-  float acc[RPW][4];
-  for (int piece = 0; piece < pieces; ++piece) {
-    const int c0 = piece / kSlabs * kChunk, s0 = piece % kSlabs * kSlab;
-    __syncthreads();
+  for (int piece = 0; piece < kMaps * chunks; ++piece) {
+    const int map = kMaps == 2 && piece >= chunks, c0 = (piece - map * chunks) * kChunk;
+    if (piece > 0) __syncthreads();
+    if (c0 == 0) {
+      // the rows of a warp interleaved: qs[warp][channel][RPW]
+      for (int idx = threadIdx.x; idx < kRows * (D / 8); idx += kThreads) {
+        const int r = idx % kRows, c8 = idx / kRows, row = row0 + r;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (row < R) v = __ldg(reinterpret_cast<const uint4*>(q_pool[map] + ((int64_t)head * R + row) * D) + c8);
+        const __half* h = reinterpret_cast<const __half*>(&v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) qs[((r / RPW) * D + c8 * 8 + j) * RPW + r % RPW] = __half2float(h[j]);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < kLoads; ++i) {
-      const int idx = threadIdx.x + i * kWarps * 32;
-      const __half* h = reinterpret_cast<const __half*>(&raw[i]);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) kc[(idx / kChunk * 8 + j) * kPitch + idx % kChunk] = __half2float(h[j]);
+      const int idx = threadIdx.x + i * kThreads;
+      uint32_t* dst = kc + idx / kChunk * 4 * kChunk + idx % kChunk;
+      dst[0] = raw[i].x;
+      dst[kChunk] = raw[i].y;
+      dst[2 * kChunk] = raw[i].z;
+      dst[3 * kChunk] = raw[i].w;
     }
     __syncthreads();
-    if (piece + 1 < pieces) fetch(piece + 1);
-    if (s0 == 0) {
-#pragma unroll
-      for (int r = 0; r < RPW; ++r)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[r][j] = 0.0f;
-    }
-#pragma unroll 8
-    for (int c = 0; c < kSlab; ++c) {
-      float qv[RPW];
-      if (RPW == 4) {
-        *reinterpret_cast<float4*>(qv) = *reinterpret_cast<const float4*>(qw + (s0 + c) * 4);
-      } else if (RPW == 2) {
-        *reinterpret_cast<float2*>(qv) = *reinterpret_cast<const float2*>(qw + (s0 + c) * 2);
-      } else {
-        qv[0] = qw[s0 + c];
-      }
-      const float4 kv = *reinterpret_cast<const float4*>(kc + c * kPitch + lane * 4);
-#pragma unroll
-      for (int r = 0; r < RPW; ++r) {
-        acc[r][0] = __fmaf_rn(qv[r], kv.x, acc[r][0]);
-        acc[r][1] = __fmaf_rn(qv[r], kv.y, acc[r][1]);
-        acc[r][2] = __fmaf_rn(qv[r], kv.z, acc[r][2]);
-        acc[r][3] = __fmaf_rn(qv[r], kv.w, acc[r][3]);
-      }
-    }
-    if (s0 + kSlab < D) continue;
+    if (piece + 1 < kMaps * chunks) fetch(piece + 1);
+    float acc[RPW][4];
 #pragma unroll
     for (int r = 0; r < RPW; ++r)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = c0 + lane * 4 + j;
-        if (col < R)
-          lg[(warp * RPW + r) * lg_stride + col] = __float2half_rn(__fmul_rn(acc[r][j], scale));
+      for (int j = 0; j < 4; ++j) acc[r][j] = 0.0f;
+#pragma unroll 4
+    for (int c2 = 0; c2 < D / 2; ++c2) {
+      const uint4 kv = *reinterpret_cast<const uint4*>(kc + c2 * kChunk + lane * 4);
+      float2 k[4];
+      k[0] = __half22float2(*reinterpret_cast<const __half2*>(&kv.x));
+      k[1] = __half22float2(*reinterpret_cast<const __half2*>(&kv.y));
+      k[2] = __half22float2(*reinterpret_cast<const __half2*>(&kv.z));
+      k[3] = __half22float2(*reinterpret_cast<const __half2*>(&kv.w));
+      float qv[2 * RPW];
+      if (RPW == 1) {
+        *reinterpret_cast<float2*>(qv) = *reinterpret_cast<const float2*>(qw + c2 * 2);
+      } else {
+#pragma unroll
+        for (int r = 0; r < 2 * RPW; r += 4)
+          *reinterpret_cast<float4*>(qv + r) = *reinterpret_cast<const float4*>(qw + c2 * 2 * RPW + r);
       }
+#pragma unroll
+      for (int r = 0; r < RPW; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[r][j] = __fmaf_rn(qv[r], k[j].x, acc[r][j]);
+#pragma unroll
+      for (int r = 0; r < RPW; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[r][j] = __fmaf_rn(qv[RPW + r], k[j].y, acc[r][j]);
+    }
+    // (columns from R on are written, too, and left out by the reader)
+    __half* dst = lg + (map * kRows + warp * RPW) * 32 * groups + (lane & 7) * 4 * groups + (c0 >> 5) + (lane >> 3);
+#pragma unroll
+    for (int r = 0; r < RPW; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dst[(r * 32 + j) * groups] = __float2half_rn(__fmul_rn(acc[r][j], scale));
   }
   __syncwarp();
 }
 
-// max and 1/sum of one row held in shared memory (warp-collective).
-__device__ __forceinline__ void row_stats(const __half* lg, int R, float& mx, float& inv) {
+// Columns l, l + 32, ... of a row, lane l's share of the canonical sum, follow one another in shared memory:
+// `groups` values per lane, a multiple of four but not of sixteen (8-byte loads; two at most meet in a bank).
+__host__ __device__ inline int column_groups(int R) {
+  const int n = (R + 31) / 32, fours = (n + 3) / 4;
+  return 4 * (fours % 4 == 0 ? fours + 1 : fours);
+}
+
+// Four values of exp_canonical(x - m), packed arithmetic of the same roundings.  round(y) is a pair of
+// additions (|y| <= 125, half to even as rintf), 2^n an addition to the exponent: the product is normal.  The
+// conversion instructions of the plain form run at 1/8 of the rate of an addition.
+// A product is a * b + zero with zero = -0, a value that the compiler does not know (an argument of the kernel): a
+// packed mul, or one with a constant zero, comes back fused with the addition after it, .rn or not.
+__device__ __forceinline__ void exp_four(const uint2& raw, float m, float zero, float (&e)[4]) {
+  const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
+  const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+  const auto both = [](float v) { return make_float2(v, v); };
+  const auto bits = [&](int v) { return both(__int_as_float(v)); };
+  const auto fmul2 = [&](float2 a, float2 b) { return ffma2(a, b, both(zero)); };
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float2 y = fmul2(fadd2(h ? hi : lo, both(-m)), bits(0x3fb8aa3b));
+    y = make_float2(fmaxf(y.x, -125.0f), fmaxf(y.y, -125.0f));
+    const float2 t = fadd2(y, both(12582912.0f));
+    const float2 f = fadd2(y, ffma2(t, both(-1.0f), both(12582912.0f)));
+    float2 p = bits(0x377fe5fe);
+    p = fadd2(fmul2(p, f), bits(0x39218489));
+    p = fadd2(fmul2(p, f), bits(0x3aaec3ff));
+    p = fadd2(fmul2(p, f), bits(0x3c1d955b));
+    p = fadd2(fmul2(p, f), bits(0x3d635847));
+    p = fadd2(fmul2(p, f), bits(0x3e75fdf0));
+    p = fadd2(fmul2(p, f), bits(0x3f317218));
+    p = fadd2(fmul2(p, f), both(1.0f));
+    e[2 * h] = __int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23));
+    e[2 * h + 1] = __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23));
+  }
+}
+
+// One row of the map.  Up to kKept * 128 columns its exponentials stay in registers between the sum and
+// the quotients; a longer row forms them twice.
+constexpr int kKept = 6;
+struct RowMap {
+  float m, inv;
+  float e[kKept][4];
+};
+template <bool kKeep>
+__device__ __forceinline__ void row_map(const __half* lg, int R, int fours, float zero, RowMap& row) {
   const int lane = threadIdx.x & 31;
+  const auto load = [&](int k) { return reinterpret_cast<const uint2*>(lg)[k]; };
+  const int mine = (R - lane + 31) >> 5;  // the lane's values before the padding
   float m = -INFINITY;
-  for (int j = lane; j < R; j += 32) m = fmaxf(m, __half2float(lg[j]));
+  const auto fold = [&](int k) {
+    const uint2 raw = load(k);
+    const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
+    const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+    const float v[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (4 * k + j < mine) m = fmaxf(m, v[j]);
+  };
+  float s = 0.0f;
+  const auto add = [&](int k, float (&e)[4]) {
+    exp_four(load(k), m, zero, e);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (4 * k + j < mine) s = __fadd_rn(s, e[j]);
+  };
+  if (kKeep) {
+#pragma unroll
+    for (int k = 0; k < kKept; ++k)
+      if (k < fours) fold(k);
+  } else {
+    for (int k = 0; k < fours; ++k) fold(k);
+  }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-  float s = 0.0f;
-  for (int j = lane; j < R; j += 32) s = __fadd_rn(s, exp_canonical(__fsub_rn(__half2float(lg[j]), m)));
+  if (kKeep) {
+#pragma unroll
+    for (int k = 0; k < kKept; ++k)
+      if (k < fours) add(k, row.e[k]);
+  } else {
+    float e[4];
+    for (int k = 0; k < fours; ++k) add(k, e);
+  }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, off));
-  mx = m;
-  inv = __fdiv_rn(1.0f, s);
+  row.m = m;
+  row.inv = __fdiv_rn(1.0f, s);
+}
+template <bool kBlend, bool kKeep>
+__device__ __forceinline__ void write_row(const __half* lg, const __half* lgx, float w, int R, int groups, float zero,
+                                          __half* out) {
+  const int lane = threadIdx.x & 31, fours = (R + 127) / 128;
+  const float wm = __fsub_rn(1.0f, w);
+  lg += lane * groups;
+  lgx += lane * groups;
+  RowMap mean, most;
+  row_map<kKeep>(lg, R, fours, zero, mean);
+  if (kBlend) row_map<kKeep>(lgx, R, fours, zero, most);
+  const auto put = [&](int k, const float (&e)[4], const float (&ex)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int col = lane + 32 * (4 * k + j);
+      const float p = __fmul_rn(e[j], mean.inv);
+      if (col < R)
+        out[col] =
+            __float2half_rn(kBlend ? __fadd_rn(__fmul_rn(wm, p), __fmul_rn(w, __fmul_rn(ex[j], most.inv))) : p);
+    }
+  };
+  if (kKeep) {
+#pragma unroll
+    for (int k = 0; k < kKept; ++k)
+      if (k < fours) put(k, mean.e[k], kBlend ? most.e[k] : mean.e[k]);
+  } else {
+    for (int k = 0; k < fours; ++k) {
+      float e[4], ex[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      exp_four(reinterpret_cast<const uint2*>(lg)[k], mean.m, zero, e);
+      if (kBlend) exp_four(reinterpret_cast<const uint2*>(lgx)[k], most.m, zero, ex);
+      put(k, e, ex);
+    }
+  }
 }
 
 // ---- diag-Jensen variant (an experimental routing proxy of the reference,
@@ -182,14 +317,14 @@ __device__ __forceinline__ void jensen_pass(const __half* q_src, const __half* k
         for (int i = 0; i < 8; ++i) {
           float x = __half2float(h[i]);
           if (kStep == 2) x = __fmul_rn(x, x);
-          kc[(c8 * 8 + i) * kPitch + col] = x;
+          kc[(c8 * 8 + i) * kChunk + col] = x;
         }
       }
       __syncthreads();
 #pragma unroll 4
       for (int c = 0; c < kSlab; ++c) {
         const float2 qv = *reinterpret_cast<const float2*>(qw + (s0 + c) * 2);
-        const float4 kv = *reinterpret_cast<const float4*>(kc + c * kPitch + lane * 4);
+        const float4 kv = *reinterpret_cast<const float4*>(kc + c * kChunk + lane * 4);
         acc[0][0] = __fmaf_rn(qv.x, kv.x, acc[0][0]);
         acc[0][1] = __fmaf_rn(qv.x, kv.y, acc[0][1]);
         acc[0][2] = __fmaf_rn(qv.x, kv.z, acc[0][2]);
@@ -229,8 +364,8 @@ __global__ void __launch_bounds__(kWarps * 32) draft_jensen_kernel(const __half*
   extern __shared__ __align__(16) uint8_t smem_raw[];
   constexpr int kRows = kWarps * 2;
   const int stride = (R + 3) & ~3;
-  float* kc = reinterpret_cast<float*>(smem_raw);  // [kSlab][kPitch]
-  float* qs = kc + kSlab * kPitch;                 // [kWarps][D][2]
+  float* kc = reinterpret_cast<float*>(smem_raw);  // [kSlab][kChunk]
+  float* qs = kc + kSlab * kChunk;                 // [kWarps][D][2]
   float* lg = qs + kRows * D;                      // [kRows][stride] fp32 logits
   float* var = lg + kRows * stride;                // [kRows][stride]
   const int head = blockIdx.y, row0 = blockIdx.x * kRows;
@@ -258,56 +393,39 @@ __global__ void __launch_bounds__(kWarps * 32) draft_jensen_kernel(const __half*
 }
 
 template <int D, bool kBlend, int RPW>
-__global__ void __launch_bounds__(kWarps * 32) draft_kernel(const __half* q_pool,
-                                                            const __half* k_pool,
-                                                            const __half* q_max, const __half* k_max,
-                                                            float w, int R, __half* prob) {
+__global__ void __launch_bounds__(kWarps * 32, 2)
+    draft_kernel(const __half* q_pool, const __half* k_pool, const __half* q_max, const __half* k_max, float w, int R,
+                 float zero, __half* prob) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   constexpr int kRows = kWarps * RPW;
-  const int lg_stride = (R + 7) & ~7;
-  float* kc = reinterpret_cast<float*>(smem_raw);                   // [kSlab][kPitch]
-  float* qs = kc + kSlab * kPitch;                                  // [kWarps][D][RPW]
-  __half* lg = reinterpret_cast<__half*>(qs + kRows * D);           // [kRows][lg_stride]
-  __half* lgx = lg + kRows * lg_stride;                             // blend only
+  const int groups = column_groups(R);
+  uint32_t* kc = reinterpret_cast<uint32_t*>(smem_raw);         // [D / 2][kChunk], two channels a word
+  float* qs = reinterpret_cast<float*>(kc + D / 2 * kChunk);    // [kWarps][D][RPW]
+  __half* lg = reinterpret_cast<__half*>(qs + kRows * D);       // [kRows][32][groups], twice when blending
   const int head = blockIdx.y, row0 = blockIdx.x * kRows;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
 
   layer::grid_dependency_wait();
   layer::grid_dependency_trigger();
-  row_logits<D, RPW>(q_pool, k_pool, head, R, row0, kc, qs, lg, lg_stride);
-  if (kBlend) {
-    __syncthreads();
-    row_logits<D, RPW>(q_max, k_max, head, R, row0, kc, qs, lgx, lg_stride);
-  }
-  for (int r = 0; r < RPW; ++r) {
-    const int row = row0 + warp * RPW + r;
-    if (row >= R) break;
-    const __half* mine = lg + (warp * RPW + r) * lg_stride;
-    float m, inv;
-    row_stats(mine, R, m, inv);
-    __half* out = prob + ((int64_t)head * R + row) * R;
-    if (!kBlend) {
-      for (int j = lane; j < R; j += 32)
-        out[j] = __float2half_rn(__fmul_rn(exp_canonical(__fsub_rn(__half2float(mine[j]), m)), inv));
-    } else {
-      const __half* minex = lgx + (warp * RPW + r) * lg_stride;
-      float mxx, invx;
-      row_stats(minex, R, mxx, invx);
-      const float wm = __fsub_rn(1.0f, w);
-      for (int j = lane; j < R; j += 32) {
-        const float pm = __fmul_rn(exp_canonical(__fsub_rn(__half2float(mine[j]), m)), inv);
-        const float px = __fmul_rn(exp_canonical(__fsub_rn(__half2float(minex[j]), mxx)), invx);
-        out[j] = __float2half_rn(__fadd_rn(__fmul_rn(wm, pm), __fmul_rn(w, px)));
-      }
-    }
+  const __half* const q[2] = {q_pool, q_max};
+  const __half* const k[2] = {k_pool, k_max};
+  row_logits<D, RPW, kBlend ? 2 : 1>(q, k, head, R, row0, kc, qs, lg, groups);
+  for (int r = warp * RPW; r < warp * RPW + RPW; ++r) {
+    if (row0 + r >= R) break;
+    __half* out = prob + ((int64_t)head * R + row0 + r) * R;
+    const __half *mean = lg + r * 32 * groups, *most = mean + kRows * 32 * groups;  // most: blend only
+    if (R <= kKept * 128)
+      write_row<kBlend, true>(mean, most, w, R, groups, zero, out);
+    else
+      write_row<kBlend, false>(mean, most, w, R, groups, zero, out);
   }
 }
 
 // Shared memory of one CTA: key tile, query rows, the logits of its rows (twice when blending).
 template <int D, bool kBlend, int RPW>
-constexpr size_t smem_bytes(int R) {
-  return (size_t)kSlab * kPitch * 4 + (size_t)kWarps * RPW * D * 4 +
-         (size_t)kWarps * RPW * ((R + 7) & ~7) * 2 * (kBlend ? 2 : 1);
+size_t smem_bytes(int R) {
+  constexpr size_t kRows = kWarps * RPW;
+  return (size_t)D / 2 * kChunk * 4 + kRows * D * 4 + kRows * 32 * column_groups(R) * 2 * (kBlend ? 2 : 1);
 }
 
 template <int D, bool kBlend, int RPW>
@@ -320,15 +438,17 @@ int launch_rows(const __half* qp, const __half* kp, const __half* qx, const __ha
     return ANEMOI_SM100_ELAUNCH;
   constexpr int kRows = kWarps * RPW;
   dim3 grid((R + kRows - 1) / kRows, H);
-  return layer::launch(kernel, grid, dim3(kWarps * 32), smem, st, qp, kp, qx, kx, w, R, prob) == cudaSuccess
+  return layer::launch(kernel, grid, dim3(kWarps * 32), smem, st, qp, kp, qx, kx, w, R, -0.0f, prob) == cudaSuccess
              ? ANEMOI_SM100_OK
              : ANEMOI_SM100_ELAUNCH;
 }
 
 // Rows per warp.  Four while two CTAs still fit an SM's shared memory, else two: a key tile read serves
 // more rows.  But while a grid of fewer rows has no more CTAs than there are SMs, every CTA has one to
-// itself and the shorter one wins: one row per warp for 8 heads x 33 blocks (31 -> 16 us with the
-// loads ahead), two for 7 x 273 (64 -> 41); at 7 x 672 (294 CTAs of two) four are quicker, 57 against 65.
+// itself and the shorter one wins.  One / two / four rows, us: 8 heads x 33 blocks, two maps (40 CTAs of one row)
+// 7.7 / 10.6 / 16.4, 5 x 247 (80 of two) 8.5 / 7.0 / 10.5, 7 x 273, two maps (126 of two) 35.8 / 26.9 / 39.1, 4 x 672
+// (168 of two) 29.8 / 27.0 / 24.2, 16 x 225 (240) 25.8 / 18.6 / 15.7, 56 x 672 541 / 354 / 262 (eight rows, in CTAs of
+// four warps, 250).
 constexpr int kSms = 148;
 template <int D, bool kBlend>
 int launch(const __half* qp, const __half* kp, const __half* qx, const __half* kx, float w, int R,
@@ -380,7 +500,7 @@ extern "C" int anemoi_sm100_draft_probability_jensen(const anemoi_sm100_shape* s
       !probability)
     return ANEMOI_SM100_EINVAL;
   const int R = shape->video_blocks, H = shape->heads, D = shape->head_dim;
-  const size_t smem = (size_t)kSlab * kPitch * 4 + (size_t)kWarps * 2 * D * 4 +
+  const size_t smem = (size_t)kSlab * kChunk * 4 + (size_t)kWarps * 2 * D * 4 +
                       (size_t)kWarps * 2 * ((R + 3) & ~3) * 4 * 2;
   if (smem > 227 * 1024) return ANEMOI_SM100_ELIMIT;  // two fp32 row buffers: R up to about 1,400
   cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -38,6 +38,33 @@ def test_draft_rows_per_warp(native_library, heads, blocks, dim, weight):
         assert np.array_equal(prob[h].cpu().numpy().view(np.uint16), want.view(np.uint16))
 
 
+@pytest.mark.parametrize("blocks, weight", [
+    (128, 0.0), (129, 0.5),                # one and two loads of four values per lane
+    (385, 0.0), (512, 0.5),                # sixteen values per lane: the padded rows
+    (768, 0.5), (769, 0.5),                # exponentials kept, and formed twice
+])
+def test_draft_row_lengths(native_library, blocks, weight):
+    """Rows around the steps of the softmax's layout, with logits far below the maximum among them, bit for bit."""
+    from anemoi_b200 import native
+    from oracle import route as R
+
+    shape = native.Shape(heads=1, head_dim=64, query_block=64, seq_tokens=blocks * 64, prefix_tokens=0,
+                         video_blocks=blocks, has_nvfp4=0, has_int8=1, has_fp16=0, has_prefix_query_int8=0,
+                         has_maxpool=int(weight != 0.0), input_is_bf16=1, q_global_scale=1.0, k_global_scale=1.0,
+                         v_global_scale=1.0)
+    g = torch.Generator().manual_seed(blocks)
+    pools = [torch.randn(1, blocks, 64, generator=g).half() for _ in range(4)]
+    pools[0][:, ::7] *= 40.0
+    pools[1][:, ::5] *= 3.0
+    q, k, qx, kx = (t.cuda() for t in pools)
+    prob = torch.empty(1, blocks, blocks, dtype=torch.float16, device="cuda")
+    p = native._ptr
+    assert native.library().anemoi_sm100_draft_probability(
+        shape, p(q), p(k), p(qx), p(kx), weight, p(prob), native._stream(prob.device)) == 0
+    want = R.draft_probability(*(t[0].numpy() for t in pools), weight)
+    assert np.array_equal(prob[0].cpu().numpy().view(np.uint16), want.view(np.uint16))
+
+
 @pytest.mark.parametrize("dim, dtype", [(64, torch.float16), (128, torch.bfloat16)])
 def test_preparation_of_many_q64_heads(native_library, dim, dtype):
     """32 heads of 9 Q64 blocks and a prefix (640 key and value tasks: one CTA per block for both)
