@@ -505,56 +505,72 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
 // ------------------------------------------------------------------------------------------
 // MMA side
 // ------------------------------------------------------------------------------------------
+// The operands' descriptors are made once per phase and move with the slot: `step` is the slot's distance from
+// the first one in 16-byte units (NVFP4 D = 128 16 heads of S = 32,760 1.52 -> 1.50 ms, Q64 INT8 8 heads of 38,247
+// 1.72 -> 1.70: 10 of a stage's 2,050 warp instructions).
+__device__ __forceinline__ uint64_t moved(uint64_t desc, uint32_t step) {
+  // (the address field does not overflow: shared memory ends below 2^18)
+  uint32_t lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(desc));
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo + step), "r"(hi));
+  return d;
+}
 template <int D, int CELL>
-__device__ __forceinline__ void issue_qk(uint32_t tmem_s, uint32_t tmem, uint32_t q_addr,
-                                         uint32_t slot_addr) {  // q_addr: NVFP4 only
+__device__ __forceinline__ void issue_qk(uint32_t tmem_s, uint32_t tmem, uint64_t q_desc, uint64_t base,
+                                         uint32_t step) {  // q_desc: NVFP4 only
+  const uint64_t kd = moved(base, step);
   if (CELL == kF16) {
-    constexpr uint32_t chunks = D / 8;
     constexpr uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, 64, 0, 0);
-    const uint64_t kd = smem_desc(slot_addr, 128, chunks * 128);
 #pragma unroll
     for (int k = 0; k < D / 16; ++k) mma_f16_ts(tmem_s, tmem + kColQ + k * 8, kd + k * 16, idesc, k > 0);
   } else if (CELL == kI8) {
-    constexpr uint32_t chunks = D / 16;
     constexpr uint32_t idesc = instr_desc(kFmtS8, kFmtS8, kAccS32, 128, 64, 0, 0);
-    const uint64_t kd = smem_desc(slot_addr, 128, chunks * 128);
 #pragma unroll
     for (int k = 0; k < D / 32; ++k) mma_i8_ts(tmem_s, tmem + kColQ + k * 8, kd + k * 16, idesc, k > 0);
   } else {
-    constexpr uint32_t chunks = D / 32;
     constexpr uint32_t idesc = instr_desc_nvf4(128, 64);
-    const uint64_t qd = smem_desc(q_addr, 128, chunks * 128), kd = smem_desc(slot_addr, 128, chunks * 128);
-    const uint64_t sd = smem_desc(slot_addr + rest_offset(D, CELL) + 32 * D, 128, 128);
+    // the scale blocks follow the codes of V
+    const uint64_t sd = smem_desc(0, 128, 128) + ((uint32_t)kd & 0x3fffu) + (rest_offset(D, CELL) + 32 * D) / 16;
 #pragma unroll
     for (int k = 0; k < D / 64; ++k) tmem_cp_32x128b_warpx4(tmem + kColSfbK + 4 * k, sd + k * 32);
 #pragma unroll
     for (int k = 0; k < D / 64; ++k)
-      mma_nvf4_ss(tmem_s, qd + k * 16, kd + k * 16, idesc, k > 0, tmem + kColSfaQ + 4 * k,
+      mma_nvf4_ss(tmem_s, q_desc + k * 16, kd + k * 16, idesc, k > 0, tmem + kColSfaQ + 4 * k,
                   tmem + kColSfbK + 4 * k);
   }
 }
+// Descriptor of the keys at `addr` (NVFP4: of the query codes, too).
+__device__ __forceinline__ uint64_t k_desc(int d, int cell, uint32_t addr) {
+  return smem_desc(addr, 128, (uint32_t)d * (cell == kF16 ? 16 : cell == kI8 ? 8 : 4));
+}
 
 template <int D, int CELL>
-__device__ __forceinline__ void issue_pv(uint32_t tmem, uint32_t slot_addr, uint32_t v_addr, uint32_t accumulate) {
+__device__ __forceinline__ void issue_pv(uint32_t tmem, uint64_t pd, uint64_t vd, uint32_t accumulate) {
   if (CELL == kF16) {
     constexpr uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, D, 0, 1);
     constexpr uint32_t v_lbo = (D / 8) * 128;  // between 8-key groups
-    const uint64_t pd = smem_desc(slot_addr, 128, 8 * 128), vd = smem_desc(v_addr, v_lbo, 128);
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       mma_f16_ss(tmem + kColO, pd + k * 16, vd + k * (2 * v_lbo / 16), idesc, k > 0 ? 1u : accumulate);
   } else if (CELL == kI8) {
     constexpr uint32_t idesc = instr_desc(kFmtE4M3, kFmtE4M3, kAccF32, 128, D, 0, 0);
-    const uint64_t pd = smem_desc(slot_addr, 128, 4 * 128), vd = smem_desc(v_addr, 128, 4 * 128);
 #pragma unroll
     for (int k = 0; k < 2; ++k)
       mma_f8_ss(tmem + kColO, pd + k * 16, vd + k * 16, idesc, k > 0 ? 1u : accumulate);
   } else {
     constexpr uint32_t idesc = instr_desc_nvf4(128, D);
-    tmem_cp_32x128b_warpx4(tmem + kColSfbV, smem_desc(v_addr + 32 * D + (D / 64) * 512, 128, 128));
-    mma_nvf4_ss(tmem + kColO, smem_desc(slot_addr, 128, 2 * 128), smem_desc(v_addr, 128, 2 * 128), idesc,
-                accumulate, tmem + kColSfaP, tmem + kColSfbV);
+    tmem_cp_32x128b_warpx4(tmem + kColSfbV,
+                           smem_desc(0, 128, 128) + ((uint32_t)vd & 0x3fffu) + (32 * D + (D / 64) * 512) / 16);
+    mma_nvf4_ss(tmem + kColO, pd, vd, idesc, accumulate, tmem + kColSfaP, tmem + kColSfbV);
   }
+}
+// Descriptors of the probabilities and the values at `addr`.
+__device__ __forceinline__ uint64_t p_desc(int cell, uint32_t addr) {
+  return smem_desc(addr, 128, (uint32_t)p_bytes(cell) / 16);
+}
+__device__ __forceinline__ uint64_t v_desc(int d, int cell, uint32_t addr) {
+  return cell == kF16 ? smem_desc(addr, (uint32_t)d * 16, 128) : smem_desc(addr, 128, (uint32_t)p_bytes(cell) / 16);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -819,10 +835,11 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       }
     } else if (warp == kQkWarp) {
       // =============================== S = Q K^T ===============================
-      // Uniform control flow for the whole warp; the tcgen05 instructions sit in elect.sync blocks.
+      // Uniform control flow for the whole warp; the tcgen05 instructions are one elected lane's.
       int g = 0, phase_ord = 0;
       int moves = 0;
       uint32_t used = 0, free_par = 0;
+      const bool leader = elect_one();
       const uint32_t q_addr = smem_u32(q_smem), ring_addr = smem_u32(ring);
 #pragma unroll 1
       for (int cell = kFirst; cell <= kLast; ++cell) {
@@ -837,7 +854,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         tc_fence_after_sync();
         const int nslot = slot_count(p.ring_bytes, D, cell);
         const uint32_t stride = stage_bytes(D, cell);
-        const uint32_t base_addr = split_kv(D, cell) ? smem_u32(smem) : ring_addr;
+        const uint64_t base = k_desc(D, cell, split_kv(D, cell) ? smem_u32(smem) : ring_addr);
+        const uint64_t q_desc = k_desc(D, kNv, q_addr);
         if (cell == kNv) {
           if (tile_blocks == 2) {
             // Scale bytes of rows 0-63 sit in the low eight bytes of every 16-byte chunk, those of
@@ -853,7 +871,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             __syncwarp();
           }
           const uint32_t qsf = q_addr + 128 * D / 2;
-          if (elect_one()) {
+          if (leader) {
 #pragma unroll
             for (int k = 0; k < D / 64; ++k)
               tmem_cp_32x128b_warpx4(tmem + kColSfaQ + 4 * k, smem_desc(qsf + 512 * k, 128, 128));
@@ -873,14 +891,14 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           }
           used |= 1u << sb;
           tc_fence_after_sync();
-          if (elect_one()) {
-            const uint32_t tmem_s = tmem + (sb ? kColS1 : kColS), slot_addr = base_addr + slot * stride;
+          if (leader) {
+            const uint32_t tmem_s = tmem + (sb ? kColS1 : kColS), step = slot * (stride / 16);
             if (cell == kI8) {
-              issue_qk<D, kI8>(tmem_s, tmem, q_addr, slot_addr);
+              issue_qk<D, kI8>(tmem_s, tmem, q_desc, base, step);
             } else if (cell == kNv) {
-              issue_qk<D, kNv>(tmem_s, tmem, q_addr, slot_addr);
+              issue_qk<D, kNv>(tmem_s, tmem, q_desc, base, step);
             } else {
-              issue_qk<D, kF16>(tmem_s, tmem, q_addr, slot_addr);
+              issue_qk<D, kF16>(tmem_s, tmem, q_desc, base, step);
             }
             mma_commit(&b->s_full[g & 1]);
             if (i == n - 1) mma_commit(&b->q_free);
@@ -891,7 +909,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         ++phase_ord;
       }
       if (b->wc.abort) {
-        if (elect_one()) mma_commit(&b->qk_done);
+        if (leader) mma_commit(&b->qk_done);
         __syncwarp();
         drain_wait(&b->qk_done, 0, kDrainNs);
       }
@@ -899,6 +917,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       // =============================== O += P V ===============================
       int g = 0;
       const uint32_t ring_addr = smem_u32(ring);
+      const bool leader = elect_one();
 #pragma unroll 1
       for (int cell = kFirst; cell <= kLast; ++cell) {
         const int n = b->cnt[cell];
@@ -906,6 +925,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         const int nslot = slot_count(p.ring_bytes, D, cell);
         const uint32_t stride = stage_bytes(D, cell);
         const uint32_t base_addr = split_kv(D, cell) ? smem_u32(smem) : ring_addr;
+        const uint64_t p_base = p_desc(cell, base_addr);
+        const uint64_t v_base =
+            v_desc(D, cell, base_addr + (split_kv(D, cell) ? kSplitKeys * stride : rest_offset(D, cell)));
         int slot = first_slot(D, cell);
 #pragma unroll 1
         for (int i = 0; i < n; ++i, ++g) {
@@ -913,16 +935,15 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           if (split_kv(D, cell)) wait<kMmaRole>(&b->wc, &b->v_full[i & 1], (i >> 1) & 1, 6);
           wait<kMmaRole>(&b->wc, &b->p_full[g & (kRing - 1)], (g >> 3) & 1, 6);
           tc_fence_after_sync();
-          if (elect_one()) {
-            const uint32_t slot_addr = base_addr + slot * stride;
-            const uint32_t v_addr = split_kv(D, cell) ? base_addr + (kSplitKeys + (i & 1)) * stride
-                                                      : slot_addr + rest_offset(D, cell);
+          if (leader) {
+            const uint64_t pd = moved(p_base, slot * (stride / 16));
+            const uint64_t vd = moved(v_base, (split_kv(D, cell) ? i & 1 : slot) * (stride / 16));
             if (cell == kI8) {
-              issue_pv<D, kI8>(tmem, slot_addr, v_addr, g > 0);
+              issue_pv<D, kI8>(tmem, pd, vd, g > 0);
             } else if (cell == kNv) {
-              issue_pv<D, kNv>(tmem, slot_addr, v_addr, g > 0);
+              issue_pv<D, kNv>(tmem, pd, vd, g > 0);
             } else {
-              issue_pv<D, kF16>(tmem, slot_addr, v_addr, g > 0);
+              issue_pv<D, kF16>(tmem, pd, vd, g > 0);
             }
             mma_commit(&b->pv_done[g & (kRing - 1)]);
             if (CELLS == kAny && cell == kNv && i == n - 1) mma_commit(&b->nv_done);
@@ -931,7 +952,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           slot = slot + 1 == nslot ? 0 : slot + 1;
         }
       }
-      if (elect_one()) mma_commit(&b->all_done);
+      if (leader) mma_commit(&b->all_done);
       __syncwarp();
       // unwinding: the MMAs in flight must be over before tensor memory is given back
       if (b->wc.abort) drain_wait(&b->all_done, 0, kDrainNs);
