@@ -25,9 +25,13 @@
 #include <cuda_fp16.h>
 
 #include "layer.cuh"
+#include "packed.cuh"
 #include "records.cuh"
 
 namespace {
+
+using sm100::fadd2;
+using sm100::ffma2;
 
 constexpr int kWarps = 8;
 constexpr int kChunk = 128;                   // key blocks per pass: 4 per lane
@@ -47,23 +51,6 @@ __device__ __forceinline__ float exp_canonical(float t) {
   p = __fadd_rn(__fmul_rn(p, f), __int_as_float(0x3f317218));
   p = __fadd_rn(__fmul_rn(p, f), 1.0f);
   return __fmul_rn(p, __int_as_float((static_cast<int>(n) + 127) << 23));
-}
-
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-      "mov.b64 rc, {%6, %7};\n\tfma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
 }
 
 // fp16 logits of kWarps * RPW query blocks against every key block of the head, for one pair of pools or two.

@@ -27,9 +27,14 @@
 #include <cuda_fp8.h>
 
 #include "layer.cuh"
+#include "packed.cuh"
 #include "records.cuh"
 
 namespace {
+
+using sm100::fadd2;
+using sm100::ffma2;
+using sm100::fmul2;
 
 constexpr int kThreads = 256;
 // CTAs per SM: 51 registers per thread for 128-row blocks, 32 for 64-row ones; fewer CTAs
@@ -88,31 +93,32 @@ __device__ __forceinline__ float e4m3_to_float(uint8_t bits) {
   __half_raw h = __nv_cvt_fp8_to_halfraw(bits, __NV_E4M3);
   return __half2float(*reinterpret_cast<__half*>(&h));
 }
-// Correctly rounded x / y from the correctly rounded reciprocal `inv` = 1/y shared by a
+// Correctly rounded x / y, two at a time, from the correctly rounded reciprocal `inv` = 1/y shared by a
 // whole group: q0 = x*inv, residual r = x - q0*y (exact in an FMA), q = q0 + r*inv.  For the
 // normal-range operands here this equals IEEE division bit for bit at a third of its cost.
-__device__ __forceinline__ float div_rn(float x, float y, float inv) {
-  const float q0 = __fmul_rn(x, inv);
-  const float r = __fmaf_rn(-q0, y, x);
-  return __fmaf_rn(r, inv, q0);
+__device__ __forceinline__ float2 div_rn(float2 x, float y, float inv) {
+  const float2 inv2 = make_float2(inv, inv);
+  const float2 q0 = fmul2(x, inv2);
+  const float2 r = ffma2(q0, make_float2(-y, -y), x);
+  return ffma2(r, inv2, q0);
 }
-__device__ __forceinline__ uint8_t e2m1_pair(float lo, float hi, float dq, float inv_dq) {
+__device__ __forceinline__ uint8_t e2m1_pair(float2 x, float dq, float inv_dq) {
   if (dq == 0.0f) return 0;
-  return __nv_cvt_float2_to_fp4x2(make_float2(div_rn(lo, dq, inv_dq), div_rn(hi, dq, inv_dq)),
-                                  __NV_E2M1, cudaRoundNearest);
+  return __nv_cvt_float2_to_fp4x2(div_rn(x, dq, inv_dq), __NV_E2M1, cudaRoundNearest);
 }
 // trunc(x / scale +- 0.5); |result| <= 127
-__device__ __forceinline__ int int8_code(float x, float scale, float inv_scale) {
-  const float t = div_rn(x, scale, inv_scale);
-  const float half = __int_as_float((__float_as_int(t) & 0x80000000) | 0x3f000000);
-  return __float2int_rz(__fadd_rn(t, half));
+__device__ __forceinline__ int2 int8_codes(__half2 h, float scale, float inv_scale) {
+  const float2 t = div_rn(__half22float2(h), scale, inv_scale);
+  const auto half = [](float v) { return __int_as_float((__float_as_int(v) & 0x80000000) | 0x3f000000); };
+  const float2 u = fadd2(t, make_float2(half(t.x), half(t.y)));
+  return make_int2(__float2int_rz(u.x), __float2int_rz(u.y));
 }
 // Four codes as bytes, the first one lowest.
-__device__ __forceinline__ uint32_t pack_s8(int a, int b, int c, int d) {
+__device__ __forceinline__ uint32_t pack_s8(int2 lo, int2 hi) {
   uint32_t r;
   asm("{\n\t.reg .b32 t;\n\tcvt.pack.sat.s8.s32.b32 t, %4, %3, 0;\n\tcvt.pack.sat.s8.s32.b32 %0, %2, %1, t;\n\t}"
       : "=r"(r)
-      : "r"(a), "r"(b), "r"(c), "r"(d));
+      : "r"(lo.x), "r"(lo.y), "r"(hi.x), "r"(hi.y));
   return r;
 }
 // The larger of two magnitudes, both halves at once.
@@ -192,13 +198,12 @@ __device__ __forceinline__ void write_int8_tile(uint8_t* dst, const __half* tile
     const int r = (idx / (8 * kChunks)) * 8 + (idx & 7), j = (idx >> 3) % kChunks;
     const __half* src = tile + (row0 + r) * (D + kPad) + j * 16;
     uint4 a = *reinterpret_cast<const uint4*>(src), b = *reinterpret_cast<const uint4*>(src + 8);
-    const __half* ha = reinterpret_cast<const __half*>(&a);
-    const __half* hb = reinterpret_cast<const __half*>(&b);
-    auto code = [&](__half h) { return int8_code(__half2float(h), scale, inv_scale); };
-    const uint4 out = make_uint4(pack_s8(code(ha[0]), code(ha[1]), code(ha[2]), code(ha[3])),
-                                 pack_s8(code(ha[4]), code(ha[5]), code(ha[6]), code(ha[7])),
-                                 pack_s8(code(hb[0]), code(hb[1]), code(hb[2]), code(hb[3])),
-                                 pack_s8(code(hb[4]), code(hb[5]), code(hb[6]), code(hb[7])));
+    const __half2* ha = reinterpret_cast<const __half2*>(&a);
+    const __half2* hb = reinterpret_cast<const __half2*>(&b);
+    const auto four = [&](__half2 lo, __half2 hi) {
+      return pack_s8(int8_codes(lo, scale, inv_scale), int8_codes(hi, scale, inv_scale));
+    };
+    const uint4 out = make_uint4(four(ha[0], ha[1]), four(ha[2], ha[3]), four(hb[0], hb[1]), four(hb[2], hb[3]));
     *reinterpret_cast<uint4*>(dst + (size_t)idx * 16) = out;
   }
 }
@@ -218,14 +223,14 @@ __device__ __forceinline__ void write_nvfp4_rows(uint8_t* codes, uint8_t* sf, co
     for (int g = 0; g < 2; ++g) {
       uint4 a = *reinterpret_cast<const uint4*>(src + g * 16);
       uint4 b = *reinterpret_cast<const uint4*>(src + g * 16 + 8);
-      float x[16];
+      float2 x[8];
       const __half2* ha = reinterpret_cast<const __half2*>(&a);
       const __half2* hb = reinterpret_cast<const __half2*>(&b);
       __half2 m2 = __hmax2(__habs2(ha[0]), __habs2(hb[0]));
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        *reinterpret_cast<float2*>(x + 2 * i) = __half22float2(ha[i]);
-        *reinterpret_cast<float2*>(x + 8 + 2 * i) = __half22float2(hb[i]);
+        x[i] = __half22float2(ha[i]);
+        x[4 + i] = __half22float2(hb[i]);
         if (i > 0) m2 = max_abs2(max_abs2(m2, ha[i]), hb[i]);
       }
       // (a group of NaNs alone has maximum zero, like one with no values: its scale byte and codes are zero)
@@ -234,7 +239,7 @@ __device__ __forceinline__ void write_nvfp4_rows(uint8_t* codes, uint8_t* sf, co
       const float dq = __fmul_rn(e4m3_to_float(sb[g]), gs);
       const float inv_dq = __frcp_rn(dq);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) c[g * 8 + i] = e2m1_pair(x[2 * i], x[2 * i + 1], dq, inv_dq);
+      for (int i = 0; i < 8; ++i) c[g * 8 + i] = e2m1_pair(x[i], dq, inv_dq);
     }
     *reinterpret_cast<uint4*>(codes + (size_t)idx * 16) = out;
     uint8_t* s = sf + (j >> 1) * 512 + rec::sf_offset(r, (j & 1) * 2);
@@ -259,8 +264,9 @@ __device__ __forceinline__ void write_v_e4m3(uint8_t* dst, const __half* tile, i
       const float2 a = __half22float2(*reinterpret_cast<const __half2*>(src + 2 * i * (D + kPad)));
       const float2 b = __half22float2(*reinterpret_cast<const __half2*>(src + (2 * i + 1) * (D + kPad)));
       // (a channel whose factor is zero holds zeros only)
-      o0[i] = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a.x, rc.x), __fmul_rn(b.x, rc.x)), __NV_SATFINITE, __NV_E4M3);
-      o1[i] = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a.y, rc.y), __fmul_rn(b.y, rc.y)), __NV_SATFINITE, __NV_E4M3);
+      const float2 sa = fmul2(a, rc), sb = fmul2(b, rc);
+      o0[i] = __nv_cvt_float2_to_fp8x2(make_float2(sa.x, sb.x), __NV_SATFINITE, __NV_E4M3);
+      o1[i] = __nv_cvt_float2_to_fp8x2(make_float2(sa.y, sb.y), __NV_SATFINITE, __NV_E4M3);
     }
     if (rc.x == 0.0f) out[0] = make_uint4(0, 0, 0, 0);
     if (rc.y == 0.0f) out[1] = make_uint4(0, 0, 0, 0);
@@ -295,7 +301,7 @@ __device__ __forceinline__ void write_v_nvfp4(uint8_t* codes, uint8_t* sf, const
       uint8_t* o = reinterpret_cast<uint8_t*>(&out);
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        o[i] = k ? e2m1_pair(x[2 * i].y, x[2 * i + 1].y, dq, inv_dq) : e2m1_pair(x[2 * i].x, x[2 * i + 1].x, dq, inv_dq);
+        o[i] = e2m1_pair(k ? make_float2(x[2 * i].y, x[2 * i + 1].y) : make_float2(x[2 * i].x, x[2 * i + 1].x), dq, inv_dq);
       *reinterpret_cast<uint2*>(codes + rec::tile_offset(c + k, jg >> 1, 2) + (jg & 1) * 8) = out;
       sf[rec::sf_offset(c + k, jg)] = sb;
     }
@@ -316,19 +322,16 @@ __device__ __forceinline__ void write_pools(const __half* tile, int rows, int co
 #pragma unroll 16
       for (int r = 0; r < rows; ++r) {
         const float2 x = __half22float2(*reinterpret_cast<const __half2*>(src + r * (D + kPad)));
-        sum.x = __fadd_rn(sum.x, x.x);
-        sum.y = __fadd_rn(sum.y, x.y);
+        sum = fadd2(sum, x);
       }
     } else {
       float2 sq = make_float2(0.0f, 0.0f), mx = make_float2(-INFINITY, -INFINITY);
 #pragma unroll 8
       for (int r = 0; r < rows; ++r) {
         const float2 x = __half22float2(*reinterpret_cast<const __half2*>(src + r * (D + kPad)));
-        sum.x = __fadd_rn(sum.x, x.x);
-        sum.y = __fadd_rn(sum.y, x.y);
+        sum = fadd2(sum, x);
         if (second) {
-          sq.x = __fmaf_rn(x.x, x.x, sq.x);
-          sq.y = __fmaf_rn(x.y, x.y, sq.y);
+          sq = ffma2(x, x, sq);
         } else if (r < count) {
           mx.x = fmaxf(mx.x, x.x);
           mx.y = fmaxf(mx.y, x.y);
