@@ -1032,6 +1032,15 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       last_cell = cell;
     }
     // ---- epilogue: O_true / d -> fp16, packed row order; each warpgroup writes half the channels ----
+    // packed rows: this tile's place; token rows: the row's token, in the caller's type (looked up under the last PV)
+    uint16_t* dst = nullptr;
+    if (p.tokens == nullptr) {
+      if (row < QB * tile_blocks)
+        dst = reinterpret_cast<uint16_t*>(p.out) + ((int64_t)head * p.out_rows + (int64_t)block0 * QB + row) * D;
+    } else if (row < QB * tile_blocks) {
+      const int64_t at = token_offset<D>(p, head, block0, QB, row);
+      if (at >= 0) dst = static_cast<uint16_t*>(p.tokens) + at;
+    }
     wait(&b->wc, &b->all_done, 0, 7);
     // d(G-1) from d(G-3) and the last two stages' (alpha, sum), which the two groups hold; every
     // other use of rec is over
@@ -1047,15 +1056,6 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       tc_fence_after_sync();
       const float d = b->rec[1][row].x;
       const float inv = d > 0.0f ? 1.0f / d : 0.0f;
-      // packed rows: this tile's place; token rows: the row's token, in the caller's type
-      uint16_t* dst = nullptr;
-      if (p.tokens == nullptr) {
-        if (row < QB * tile_blocks)
-          dst = reinterpret_cast<uint16_t*>(p.out) + ((int64_t)head * p.out_rows + (int64_t)block0 * QB + row) * D;
-      } else if (row < QB * tile_blocks) {
-        const int64_t at = token_offset<D>(p, head, block0, QB, row);
-        if (at >= 0) dst = static_cast<uint16_t*>(p.tokens) + at;
-      }
       const bool bf16 = p.tokens != nullptr && p.tokens_bf16;
 #pragma unroll 1
       for (int c0 = parity * (D / 2); c0 < (parity + 1) * (D / 2); c0 += 32) {
