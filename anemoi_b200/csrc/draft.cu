@@ -24,12 +24,14 @@
 // instructions, and kept between the sum and the quotients.
 #include <cuda_fp16.h>
 
+#include "canonical.cuh"
 #include "layer.cuh"
 #include "packed.cuh"
 #include "records.cuh"
 
 namespace {
 
+using canonical::exp_canonical;
 using sm100::fadd2;
 using sm100::ffma2;
 
@@ -37,21 +39,6 @@ constexpr int kWarps = 8;
 constexpr int kChunk = 128;                   // key blocks per pass: 4 per lane
 constexpr int kSlab = 64;                     // channels of the key tile held at a time
 constexpr int kMaxBlocks = 4096;              // rows per head the shared-memory buffers allow
-
-__device__ __forceinline__ float exp_canonical(float t) {
-  const float y = fmaxf(__fmul_rn(t, __int_as_float(0x3fb8aa3b)), -125.0f);
-  const float n = rintf(y);
-  const float f = __fsub_rn(y, n);
-  float p = __int_as_float(0x377fe5fe);
-  p = __fadd_rn(__fmul_rn(p, f), __int_as_float(0x39218489));
-  p = __fadd_rn(__fmul_rn(p, f), __int_as_float(0x3aaec3ff));
-  p = __fadd_rn(__fmul_rn(p, f), __int_as_float(0x3c1d955b));
-  p = __fadd_rn(__fmul_rn(p, f), __int_as_float(0x3d635847));
-  p = __fadd_rn(__fmul_rn(p, f), __int_as_float(0x3e75fdf0));
-  p = __fadd_rn(__fmul_rn(p, f), __int_as_float(0x3f317218));
-  p = __fadd_rn(__fmul_rn(p, f), 1.0f);
-  return __fmul_rn(p, __int_as_float((static_cast<int>(n) + 127) << 23));
-}
 
 // fp16 logits of kWarps * RPW query blocks against every key block of the head, for one pair of pools or two.
 // Each warp owns RPW (1, 2 or 4) rows, each lane four key columns of the 128-column pass.  The key tile holds

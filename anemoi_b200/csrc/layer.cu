@@ -91,6 +91,10 @@ extern "C" int anemoi_sm100_routes_in_one_kernel(const anemoi_sm100_shape* shape
   return rec::validate_shape(shape) == ANEMOI_SM100_OK && layer::routes_pairs(*shape);
 }
 
+extern "C" int anemoi_sm100_drafts_in_routing(const anemoi_sm100_shape* shape) {
+  return rec::validate_shape(shape) == ANEMOI_SM100_OK && layer::drafts_in_routing(*shape);
+}
+
 extern "C" int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan) {
   return valid(plan) ? cut(*plan, nullptr).bytes : ANEMOI_SM100_EINVAL;
 }
@@ -140,25 +144,24 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
   const bool late = native_prefix && prefix_ctas >= kPrefixFillsGpu;
   if (native_prefix && !late && (code = prefix()) != ANEMOI_SM100_OK) return done(code);
 
-  code = anemoi_sm100_draft_probability(&s, w.ops.q_pool, w.ops.k_pool, w.ops.q_max_pool, w.ops.k_max_pool,
-                                        p.maxpool_weight, w.prob, stream);
-  if (code != ANEMOI_SM100_OK) return done(code);
-  const int32_t* pair_counts = nullptr;
-  if (p.pair_q64 && s.query_block == 64) {
-    if (layer::routes_pairs(s)) {
+  const int32_t* pair_counts = w.pair_counts;
+  if (layer::drafts_in_routing(s)) {
+    code = layer::draft_and_route(s, w.ops, p.maxpool_weight, w.prob, p.n16, p.n8, p.n4, p.prefix_phase, w.row_offset,
+                                  w.row_counts, w.stage_ids, w.pair_counts, w.pair_ids, p.list_capacity, st);
+  } else {
+    code = anemoi_sm100_draft_probability(&s, w.ops.q_pool, w.ops.k_pool, w.ops.q_max_pool, w.ops.k_max_pool,
+                                          p.maxpool_weight, w.prob, stream);
+    if (code != ANEMOI_SM100_OK) return done(code);
+    if (pair_counts != nullptr && layer::routes_pairs(s)) {
       code = anemoi_sm100_route_pairs(&s, w.prob, p.n16, p.n8, p.n4, p.prefix_phase, w.row_offset, w.row_counts,
                                       w.pair_counts, w.pair_ids, p.list_capacity, stream);
     } else {
       code = anemoi_sm100_route(&s, w.prob, p.n16, p.n8, p.n4, p.prefix_phase, w.scratch, w.scratch_bytes,
                                 w.row_offset, w.row_counts, w.stage_ids, p.list_capacity, stream);
-      if (code == ANEMOI_SM100_OK)
+      if (code == ANEMOI_SM100_OK && pair_counts != nullptr)
         code = anemoi_sm100_pair_lists(&s, w.row_offset, w.row_counts, w.stage_ids, p.list_capacity, w.pair_counts,
                                        w.pair_ids, stream);
     }
-    pair_counts = w.pair_counts;
-  } else {
-    code = anemoi_sm100_route(&s, w.prob, p.n16, p.n8, p.n4, p.prefix_phase, w.scratch, w.scratch_bytes,
-                              w.row_offset, w.row_counts, w.stage_ids, p.list_capacity, stream);
   }
   if (code != ANEMOI_SM100_OK) return done(code);
   if (late && (code = prefix()) != ANEMOI_SM100_OK) return done(code);

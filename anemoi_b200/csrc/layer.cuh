@@ -25,6 +25,12 @@ int video_rows(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, co
                int32_t* status, cudaStream_t st);
 int prefix_rows(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, const int32_t* valid_k,
                 const TokenRows& rows, int32_t* status, cudaStream_t st);
+// Whether the draft map is formed by the routing kernel, and both in one launch (pair_counts: for pairs).
+bool drafts_in_routing(const anemoi_sm100_shape& s);
+int draft_and_route(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, float maxpool_weight,
+                    void* probability, int64_t n16, int64_t n8, int64_t n4, int prefix_phase, int32_t* row_offset,
+                    int32_t* row_counts, int32_t* stage_ids, int32_t* pair_counts, int32_t* pair_ids, int64_t capacity,
+                    cudaStream_t st);
 // Whether a Q64 call's pair lists come out of the routing kernel itself.
 bool routes_pairs(const anemoi_sm100_shape& s);
 // The prefix rows alone, from [H][rows][D] (fp16, or already in the caller's type).

@@ -24,6 +24,7 @@
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
+#include "canonical.cuh"
 #include "layer.cuh"
 #include "records.cuh"
 
@@ -624,12 +625,19 @@ __device__ __forceinline__ void fused_exclusive(int (&v)[N], int4* warp_sum, int
 
 constexpr int kAhead = 8;  // 32-column pieces of a row whose keys are loaded before the first is looked at
 
+// A map entry; `kOwn`: of a map that this CTA has written itself (not through the read-only path).
+template <bool kOwn, typename T>
+__device__ __forceinline__ T map_entry(const T* at) {
+  return kOwn ? *at : __ldg(at);
+}
+
 // The keys of columns [j0, j0 + 32 * kAhead) of a row, -2 past its end.
+template <bool kOwn>
 __device__ __forceinline__ void fused_keys(const unsigned short* src, int j0, int R, int (&key)[kAhead]) {
 #pragma unroll
   for (int u = 0; u < kAhead; ++u) {
     const int j = j0 + u * 32 + (threadIdx.x & 31);
-    key[u] = j < R ? (__ldg(src + j) & 0x7fff) : -2;
+    key[u] = j < R ? (map_entry<kOwn>(src + j) & 0x7fff) : -2;
   }
 }
 
@@ -651,9 +659,86 @@ __device__ __forceinline__ int fused_code(int key, const int (&key_b)[3], const 
   return c;
 }
 
-template <bool kPairs>
+// ---- the draft map in the same kernel: up to 32 blocks per head, one CTA -------------------------
+// The arithmetic of draft.cu with a row per warp and a column per lane, the pools in the histogram's space.
+// Up to there a head's map is 1-2 us of work, and a launch of its own costs 2.5 us on the host and as much on the
+// device.  Calls without a prefix, us, in two launches / in one: 1,024 tokens x 4 heads (16 blocks) 35.5 / 31.7, 1,872 x 3
+// (15) 43.9 / 41.2, 2,016 x 8, two maps (16) 52.0 / 47.6, 4,032 x 8 (32) 69.6 / 69.4, 3,024 x 40 (24) 157.4 / 155.3.  With
+// prefix tiles on the side stream the one kernel loses (4,032 x 8 and 77: 77.5 / 86.7), and so it does with two
+// rows per warp and two columns per lane (51 blocks 32.4 / 36.2).
+constexpr int kDraftBlocks = 32;
+struct DraftPools {
+  const __half* q[2];  // mean, max
+  const __half* k[2];
+  int maps;      // 1 or 2
+  float weight;  // of the max pools' map
+  unsigned short* map;
+};
+
+template <int D>
+__device__ __forceinline__ void draft_rows(const DraftPools& d, int head, int R, uint32_t* smem) {
+  uint32_t* kc = smem;                                                   // [2][D / 2][32], two channels a word
+  float* qs = reinterpret_cast<float*>(smem + 2 * D / 2 * kDraftBlocks);  // [2][32][D]
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    if (m >= d.maps) break;
+    for (int idx = threadIdx.x; idx < kDraftBlocks * (D / 8); idx += kFusedThreads) {
+      const int col = idx % kDraftBlocks, c8 = idx / kDraftBlocks;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (col < R) v = __ldg(reinterpret_cast<const uint4*>(d.k[m] + ((int64_t)head * R + col) * D) + c8);
+      uint32_t* dst = kc + (m * (D / 2) + c8 * 4) * kDraftBlocks + col;
+      dst[0] = v.x;
+      dst[kDraftBlocks] = v.y;
+      dst[2 * kDraftBlocks] = v.z;
+      dst[3 * kDraftBlocks] = v.w;
+    }
+    for (int idx = threadIdx.x; idx < R * (D / 2); idx += kFusedThreads)
+      reinterpret_cast<float2*>(qs + m * kDraftBlocks * D)[idx] =
+          __half22float2(__ldg(reinterpret_cast<const __half2*>(d.q[m] + (int64_t)head * R * D) + idx));
+  }
+  __syncthreads();
+  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool in = lane < R;
+  if (r < R) {
+    float p[2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      if (m >= d.maps) break;
+      const float4* q = reinterpret_cast<const float4*>(qs + (m * kDraftBlocks + r) * D);
+      const uint32_t* k = kc + m * (D / 2) * kDraftBlocks + lane;
+      float acc = 0.0f;
+#pragma unroll 8
+      for (int c4 = 0; c4 < D / 4; ++c4) {
+        const float4 qv = q[c4];
+        const uint32_t w0 = k[2 * c4 * kDraftBlocks], w1 = k[(2 * c4 + 1) * kDraftBlocks];
+        const float2 k0 = __half22float2(*reinterpret_cast<const __half2*>(&w0));
+        const float2 k1 = __half22float2(*reinterpret_cast<const __half2*>(&w1));
+        acc = __fmaf_rn(qv.y, k0.y, __fmaf_rn(qv.x, k0.x, acc));
+        acc = __fmaf_rn(qv.w, k1.y, __fmaf_rn(qv.z, k1.x, acc));
+      }
+      const float logit =
+          __half2float(__float2half_rn(__fmul_rn(acc, D == 64 ? 0.125f : __int_as_float(0x3db504f3))));
+      float mx = in ? fmaxf(-INFINITY, logit) : -INFINITY;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      const float e = canonical::exp_canonical(__fsub_rn(logit, mx));
+      float sum = in ? e : 0.0f;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, off));
+      p[m] = __fmul_rn(e, __fdiv_rn(1.0f, sum));
+    }
+    const float v = d.maps == 1
+                        ? p[0]
+                        : __fadd_rn(__fmul_rn(__fsub_rn(1.0f, d.weight), p[0]), __fmul_rn(d.weight, p[1]));
+    if (in) d.map[((int64_t)head * R + r) * R + lane] = __half_as_ushort(__float2half_rn(v));
+  }
+  __syncthreads();
+}
+
+// kDraft: 0, or the head dimension of the pools that the map is formed from first.
+template <bool kPairs, int kDraft>
 __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
-    const unsigned short* prob, int R, int rows_per, int b0, int b1, int b2, int factor, int prefix_stages,
+    const DraftPools draft, const unsigned short* prob, int R, int rows_per, int b0, int b1, int b2, int factor, int prefix_stages,
     int prefix_phase, int64_t capacity, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids,
     int32_t* pair_counts, int32_t* pair_ids) {
   namespace cg = cooperative_groups;
@@ -675,22 +760,31 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   const unsigned short* map = prob + (int64_t)head * R * R;
 
   // ---- histogram of this CTA's rows ----
+  constexpr bool kOwn = kDraft != 0;
+  if constexpr (kOwn) {
+    layer::grid_dependency_wait();
+    layer::grid_dependency_trigger();
+    draft_rows<kDraft>(draft, head, R, reinterpret_cast<uint32_t*>(hist));
+  }
   for (int i = threadIdx.x; i < kBins / 4; i += kFusedThreads) reinterpret_cast<int4*>(hist)[i] = make_int4(0, 0, 0, 0);
   __syncthreads();
-  layer::grid_dependency_wait();
-  layer::grid_dependency_trigger();
+  if constexpr (!kOwn) {
+    layer::grid_dependency_wait();
+    layer::grid_dependency_trigger();
+  }
   {
     const unsigned short* src = map + (int64_t)r0 * R;
     const int items = mine * R;
     const int head_items = min(items, (int)((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 2);
     const int vecs = (items - head_items) / 8;
     const uint4* v = reinterpret_cast<const uint4*>(src + head_items);
-    if ((int)threadIdx.x < head_items) atomicAdd(&hist[__ldg(src + threadIdx.x) & 0x7fff], 1);
+    if ((int)threadIdx.x < head_items) atomicAdd(&hist[map_entry<kOwn>(src + threadIdx.x) & 0x7fff], 1);
     const int tail = head_items + vecs * 8;
-    if (tail + (int)threadIdx.x < items && threadIdx.x < 8) atomicAdd(&hist[__ldg(src + tail + threadIdx.x) & 0x7fff], 1);
+    if (tail + (int)threadIdx.x < items && threadIdx.x < 8) 
+      atomicAdd(&hist[map_entry<kOwn>(src + tail + threadIdx.x) & 0x7fff], 1);
 #pragma unroll 2
     for (int i = threadIdx.x; i < vecs; i += kFusedThreads) {
-      const uint4 q = __ldg(v + i);
+      const uint4 q = map_entry<kOwn>(v + i);
       const unsigned w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -778,7 +872,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
     int n[3] = {0, 0, 0};  // keys above | equal << 16 (a row has 4,096 at most)
     for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
       int key[kAhead];
-      fused_keys(src, j0, R, key);
+      fused_keys<kOwn>(src, j0, R, key);
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
         if (j0 + u * 32 >= R) break;
@@ -862,7 +956,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       const unsigned short* src = map + (int64_t)(r0 + i) * R;
       for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
         int key[kAhead];
-        fused_keys(src, j0, R, key);
+        fused_keys<kOwn>(src, j0, R, key);
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
           if (j0 + u * 32 >= R) break;
@@ -908,8 +1002,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       const unsigned short* src_b = map + (int64_t)(r0 + bb) * R;
       for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
         int ka[kAhead], kb[kAhead];
-        fused_keys(src_a, j0, R, ka);
-        fused_keys(src_b, j0, has_b ? R : 0, kb);
+        fused_keys<kOwn>(src_a, j0, R, ka);
+        fused_keys<kOwn>(src_b, j0, has_b ? R : 0, kb);
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
           if (j0 + u * 32 >= R) break;
@@ -956,19 +1050,19 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   if (ctas > 1) cluster.sync();  // no CTA leaves while another may still read its totals
 }
 
-template <bool kPairs>
-int launch_fused(const anemoi_sm100_shape& s, const void* probability, int64_t n16, int64_t n8, int64_t n4,
+template <bool kPairs, int kDraft>
+int launch_fused(const anemoi_sm100_shape& s, const DraftPools& draft, const void* probability, int64_t n16, int64_t n8, int64_t n4,
                  int prefix_phase, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids, int64_t capacity,
                  int32_t* pair_counts, int32_t* pair_ids, cudaStream_t st) {
   const int H = s.heads, R = s.video_blocks, ctas = fused_ctas(H, R);
-  auto kernel = route_fused_kernel<kPairs>;
+  auto kernel = route_fused_kernel<kPairs, kDraft>;
   // Function attributes belong to a device: the opt-in is made at every call (a cheap host-side
   // driver call), so a process that routes on several GPUs, or from several host threads,
   // never launches the kernel without the opt-in for its dynamic shared memory.
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem()) != cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
   return layer::launch_cluster(kernel, dim3(ctas, H), dim3(ctas), dim3(kFusedThreads), fused_smem(), st,
-                               static_cast<const unsigned short*>(probability), R, fused_rows(R, ctas), (int)n16,
+                               draft, static_cast<const unsigned short*>(probability), R, fused_rows(R, ctas), (int)n16,
                                (int)(n16 + n8), (int)(n16 + n8 + n4), s.query_block / 64, rec::prefix_stages(s),
                                prefix_phase, capacity, row_offset, row_counts, stage_ids, pair_counts,
                                pair_ids) == cudaSuccess
@@ -1150,7 +1244,7 @@ extern "C" int anemoi_sm100_route(const anemoi_sm100_shape* shape, const void* p
   if (R > 65535 || items * H >= (1ll << 40)) return ANEMOI_SM100_ELIMIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (fused_fits(H, R))
-    return launch_fused<false>(*shape, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids,
+    return launch_fused<false, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids,
                                list_capacity, nullptr, nullptr, st);
   RouteScratch sc;
   sc.hist = static_cast<int*>(scratch);
@@ -1195,8 +1289,45 @@ extern "C" int anemoi_sm100_route_pairs(const anemoi_sm100_shape* shape, const v
   if (list_capacity < anemoi_sm100_route_list_capacity(shape, n16, n8, n4, prefix_phase))
     return ANEMOI_SM100_EINVAL;
   if (!fused_fits(shape->heads, shape->video_blocks) || rec::stages(*shape) >= (1 << 30)) return ANEMOI_SM100_ELIMIT;
-  return launch_fused<true>(*shape, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, nullptr,
+  return launch_fused<true, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, nullptr,
                             list_capacity, pair_counts, pair_ids, static_cast<cudaStream_t>(stream));
+}
+
+bool layer::drafts_in_routing(const anemoi_sm100_shape& s) {
+  return s.prefix_tokens == 0 && s.video_blocks <= kDraftBlocks && fused_ctas(s.heads, s.video_blocks) == 1 &&
+         routes_pairs(s);
+}
+
+int layer::draft_and_route(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, float maxpool_weight,
+                           void* probability, int64_t n16, int64_t n8, int64_t n4, int prefix_phase,
+                           int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids, int32_t* pair_counts,
+                           int32_t* pair_ids, int64_t capacity, cudaStream_t st) {
+  // (the conditions of draft_probability, route and route_pairs)
+  const int64_t items = (int64_t)s.video_blocks * s.video_blocks;
+  const bool pairs = pair_counts != nullptr;
+  if (!ops.q_pool || !ops.k_pool || !probability || !row_offset || !row_counts || !(pairs ? pair_ids : stage_ids))
+    return ANEMOI_SM100_EINVAL;
+  if (!(maxpool_weight >= 0.0f && maxpool_weight <= 1.0f)) return ANEMOI_SM100_EINVAL;
+  if (maxpool_weight != 0.0f && (!ops.q_max_pool || !ops.k_max_pool)) return ANEMOI_SM100_EINVAL;
+  if (n16 < 0 || n8 < 0 || n4 < 0 || n16 + n8 + n4 > items || n16 + n8 + n4 <= 0) return ANEMOI_SM100_EINVAL;
+  if (prefix_phase < -1 || prefix_phase > 2) return ANEMOI_SM100_EINVAL;
+  if (prefix_phase >= 0 && s.prefix_tokens == 0) prefix_phase = -1;
+  if (capacity < anemoi_sm100_route_list_capacity(&s, n16, n8, n4, prefix_phase)) return ANEMOI_SM100_EINVAL;
+  DraftPools d = {};
+  const bool most = maxpool_weight == 1.0f;  // max pools only
+  d.q[0] = static_cast<const __half*>(most ? ops.q_max_pool : ops.q_pool);
+  d.k[0] = static_cast<const __half*>(most ? ops.k_max_pool : ops.k_pool);
+  d.q[1] = static_cast<const __half*>(ops.q_max_pool);
+  d.k[1] = static_cast<const __half*>(ops.k_max_pool);
+  d.maps = maxpool_weight != 0.0f && !most ? 2 : 1;
+  d.weight = maxpool_weight;
+  d.map = static_cast<unsigned short*>(probability);
+#define ANEMOI_LAUNCH(PAIRS, D)                                                                                       \
+  launch_fused<PAIRS, D>(s, d, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids, capacity, \
+                         pair_counts, pair_ids, st)
+  if (pairs) return s.head_dim == 64 ? ANEMOI_LAUNCH(true, 64) : ANEMOI_LAUNCH(true, 128);
+  return s.head_dim == 64 ? ANEMOI_LAUNCH(false, 64) : ANEMOI_LAUNCH(false, 128);
+#undef ANEMOI_LAUNCH
 }
 
 // ------------------------------------------------------------------------------------------

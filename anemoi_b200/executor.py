@@ -338,6 +338,7 @@ class _Plan:
         self.uses_scales = "nvfp4" in active
         # kernels per call: V amax, preparation, draft, routing (and pair lists), attention, prefix rows
         self.launches = 4 + int("int8" in active) + int(prefix_tokens > 0)
+        self.launches -= lib.anemoi_sm100_drafts_in_routing(C.byref(shape))
         if not lib.anemoi_sm100_routes_in_one_kernel(C.byref(shape)):
             self.launches += 4 + 2 * int(pair_q64 and query_block == 64)
         self.call = lib.anemoi_sm100_layer

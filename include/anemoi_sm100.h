@@ -221,6 +221,8 @@ int anemoi_sm100_pair_lists(const anemoi_sm100_shape* shape, const int32_t* row_
                             void* stream);
 /* 1 if anemoi_sm100_route runs as one kernel for this shape (five otherwise), 0 if not. */
 int anemoi_sm100_routes_in_one_kernel(const anemoi_sm100_shape* shape);
+/* 1 if anemoi_sm100_layer() forms the draft map in that kernel, too (a launch less). */
+int anemoi_sm100_drafts_in_routing(const anemoi_sm100_shape* shape);
 /* Routing and pair lists in one kernel (no lists of single blocks): row_offset and row_counts as from
  * anemoi_sm100_route (launch order 0), pair_counts and pair_ids as from pair_lists.
  * ANEMOI_SM100_ELIMIT where the one-kernel routing does not apply: use the two functions. */

@@ -46,3 +46,32 @@ def test_prefix_tiles_beside_and_after_routing(native_library, heads, query_bloc
     for _ in range(3):
         assert torch.equal(executor.sm100_ragged_attention(q, k, v, **kw), staged)
     assert executor.last_status() == 0
+
+
+@pytest.mark.parametrize("video, query_block, dim, weight, prefix, one_launch", [
+    ((1, 8, 16), 64, 64, 0.0, 0, 1),       # two blocks
+    ((31, 8, 8), 64, 128, 0.5, 0, 1),      # 31 blocks, both maps, pairs with a single block at the end
+    ((32, 8, 16), 128, 64, 1.0, 0, 1),     # 32 blocks, the max pools' map alone
+    ((32, 8, 16), 128, 128, 0.5, 0, 1),
+    ((32, 8, 16), 128, 128, 0.5, 20, 0),   # a draft launch of its own: beside prefix tiles
+    ((33, 8, 8), 64, 64, 0.5, 0, 0),       # and for more blocks
+])
+def test_map_and_routing_in_one_launch(native_library, video, query_block, dim, weight, prefix, one_launch):
+    """Calls whose routing kernel forms the draft map, up to 32 blocks per head and no prefix: bit for bit the stages."""
+    from anemoi_b200 import executor, native
+
+    frames, height, width = video
+    tokens = prefix + frames * height * width
+    shape = native.Shape(heads=3, head_dim=dim, query_block=query_block, seq_tokens=tokens, prefix_tokens=prefix,
+                         video_blocks=frames * height * width // query_block, has_nvfp4=0, has_int8=1, has_fp16=1,
+                         has_prefix_query_int8=0, has_maxpool=int(weight != 0.0), input_is_bf16=0, q_global_scale=1.0,
+                         k_global_scale=1.0, v_global_scale=1.0)
+    assert native.library().anemoi_sm100_drafts_in_routing(C.byref(shape)) == one_launch
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    q, k, v = (torch.randn(1, tokens, 3, dim, generator=gen, device="cuda").half() for _ in range(3))
+    kw = dict(prefix_tokens=prefix, sparsity_ratio=0.7, retained_nvfp4_ratio=0.0, retained_int8_ratio=0.6,
+              retained_fp16_ratio=0.4, video_shape=video, layer=0, query_block_size=query_block, maxpool_weight=weight)
+    staged, _ = executor.sm100_ragged_attention(q, k, v, return_parts=True, **kw)
+    for _ in range(3):
+        assert torch.equal(executor.sm100_ragged_attention(q, k, v, **kw), staged)
+    assert executor.last_status() == 0
