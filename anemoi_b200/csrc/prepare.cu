@@ -51,6 +51,7 @@ struct PrepParams {
   const int32_t* indices;
   const int32_t* counts;
   int prefix_stages, stages, prefix_q_tiles;
+  int own_maxima;  // of a short sequence's V, by every CTA of values: no kernel before this one
   int64_t stride[6];  // token and head stride (elements) of q, k, v
 };
 
@@ -345,6 +346,51 @@ __device__ __forceinline__ void write_pools(const __half* tile, int rows, int co
   }
 }
 
+// Two 16-bit magnitudes at a time; a NaN never wins (as fmaxf).
+template <typename InT>
+struct Abs2;
+template <>
+struct Abs2<__half> {
+  using T = __half2;
+};
+template <>
+struct Abs2<__nv_bfloat16> {
+  using T = __nv_bfloat162;
+};
+
+// max |v| of channel threadIdx.x over every token of a short sequence (as v_amax_kernel finds it); `part`: 4 KB.
+template <typename InT, int D>
+__device__ __forceinline__ float channel_maximum(const InT* v, const PrepParams& p, int head, void* part) {
+  using T2 = typename Abs2<InT>::T;
+  constexpr int kVec = D / 8, kLanes = kThreads / kVec;
+  const int x = threadIdx.x % kVec, y = threadIdx.x / kVec;
+  const InT* src = v + (int64_t)head * p.stride[5] + x * 8;
+  T2 m[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) m[i] = T2(InT(0.0f), InT(0.0f));
+#pragma unroll 8
+  for (int t = y; t < p.s.seq_tokens; t += kLanes) {
+    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src + (int64_t)t * p.stride[4]));
+    const T2* h = reinterpret_cast<const T2*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = __hmax2(m[i], __habs2(h[i]));
+  }
+  T2* own = static_cast<T2*>(part) + threadIdx.x * 4;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) own[i] = m[i];
+  __syncthreads();
+  float found = 0.0f;
+  if (threadIdx.x < D) {
+    const int c = threadIdx.x;
+    const T2* all = static_cast<const T2*>(part) + (c / 8) * 4 + c % 8 / 2;
+    T2 r = all[0];
+    for (int k = 1; k < kLanes; ++k) r = __hmax2(r, all[k * kVec * 4]);
+    found = __half2float(__float2half_rn(static_cast<float>(c & 1 ? r.y : r.x)));
+  }
+  __syncthreads();
+  return found;
+}
+
 // Tasks of a head, in grid order: query tiles (video, prefix), then key/value blocks (R video blocks
 // of QB rows = QB/64 stages each, then the 64-row prefix stages).  With kSplit keys and values of a
 // block are separate CTAs (all keys first).
@@ -367,7 +413,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
     // ---------------- query tile (video or prefix) ----------------
     // (after the maxima's kernel, whose CTAs all began when what was before it in the stream was
     // complete; without INT8 there is no such kernel)
-    if (!p.s.has_int8) layer::grid_dependency_wait();
+    if (!p.s.has_int8 || p.own_maxima) layer::grid_dependency_wait();
     const bool video = task < R;
     const int t = video ? task : task - R;
     const int valid = video ? p.counts[t] : min(QB, p.s.prefix_tokens - t * QB);
@@ -412,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
   const int stage0 = video ? p.prefix_stages + b * kF : b;
   const int valid = video ? p.counts[b] : min(64, p.s.prefix_tokens - b * 64);
   const int64_t rec0 = (int64_t)head * p.stages + stage0;
-  if (!p.s.has_int8) layer::grid_dependency_wait();
+  if (!p.s.has_int8 || p.own_maxima) layer::grid_dependency_wait();
   auto gather = [&](const void* src, int64_t token_stride, int64_t head_stride) {
     if (video) {
       gather_tile<InT, D, QB>(tile, static_cast<const InT*>(src), p, head, true, b * QB, 0, valid, token_stride,
@@ -455,12 +501,17 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
   }
 
   // ---- values of the same rows ----
+  float maximum = 0.0f;
+  if (p.own_maxima) {
+    maximum = channel_maximum<InT, D>(static_cast<const InT*>(p.v), p, head, tile);
+    if (block == 0 && threadIdx.x < D) p.o.v_amax[(int64_t)head * D + threadIdx.x] = maximum;
+  }
   gather(p.v, p.stride[4], p.stride[5]);
   if (p.s.has_int8) {
-    layer::grid_dependency_wait();
+    if (!p.own_maxima) layer::grid_dependency_wait();
     if (threadIdx.x < D) {
       const float amax =
-          __half2float(__float2half_rn(p.o.v_amax[(int64_t)head * D + threadIdx.x]));
+          p.own_maxima ? maximum : __half2float(__float2half_rn(p.o.v_amax[(int64_t)head * D + threadIdx.x]));
       recip[threadIdx.x] = amax == 0.0f ? 0.0f : __fdiv_rn(2.25f, amax);
       if (block == 0) p.o.v_e4m3_scale[(int64_t)head * D + threadIdx.x] = __fdiv_rn(amax, 2.25f);
     }
@@ -484,18 +535,6 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
     }
   }
 }
-
-// Two 16-bit magnitudes at a time; a NaN never wins (as fmaxf).
-template <typename InT>
-struct Abs2;
-template <>
-struct Abs2<__half> {
-  using T = __half2;
-};
-template <>
-struct Abs2<__nv_bfloat16> {
-  using T = __nv_bfloat162;
-};
 
 // max |v| per (head, channel) over every token, as the bit pattern of a non-negative float
 // (integer max == float max).  The token ranges' maxima meet in global atomics (`out` must be zeroed
@@ -568,14 +607,25 @@ __global__ void __launch_bounds__(32 * kAmaxLanes) v_amax_kernel(const InT* v, i
   }
 }
 
+// Values of a head up to which every CTA of values finds the maxima of V itself, while each of them has an SM of its
+// own: reading 192 KB from L2 takes 1-2 us, a kernel for them 4 and its launch 2.5 on the host.  Calls, us, with the
+// kernel / without: 1,024 tokens x 4 heads x 64 31.5 / 29.3, 1,200 x 8 x 64 29.8 / 27.1; not taken: 2,040 x 3 x 64
+// 33.4 / 33.1, 2,040 x 30 x 64 (960 CTAs) 61 / 68, 2,040 x 40 x 128 93 / 119.
+constexpr int64_t kOwnMaxima = 96 * 1024;
+inline bool own_maxima(const anemoi_sm100_shape& s) {
+  return s.has_int8 && (int64_t)s.seq_tokens * s.head_dim <= kOwnMaxima &&
+         ((int64_t)s.video_blocks + rec::prefix_stages(s)) * s.heads <= 148;
+}
+
 template <typename InT, int QB, int D, bool kSplit>
-int launch(const PrepParams& p, cudaStream_t stream) {
+int launch(PrepParams p, cudaStream_t stream) {
   const size_t smem = (size_t)QB * (D + kPad) * sizeof(__half);
   auto kernel = prepare_kernel<InT, QB, D, kSplit>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
-  if (p.s.has_int8) {
+  p.own_maxima = own_maxima(p.s);
+  if (p.s.has_int8 && !p.own_maxima) {
     const int chunks = (p.s.heads * D / 8 + 31) / 32;
     // about three CTAs per SM, each with at least sixteen loads per thread: every CTA ends in 256 atomics
     // (8 heads x 4,109 tokens with eight per SM and two loads: the preparation took 40 us, now 24)
@@ -609,6 +659,10 @@ int launch(const PrepParams& p, cudaStream_t stream) {
 }  // namespace
 
 extern "C" int anemoi_sm100_arch(void) { return 100; }
+
+extern "C" int anemoi_sm100_prepare_kernels(const anemoi_sm100_shape* shape) {
+  return rec::validate_shape(shape) == ANEMOI_SM100_OK ? 1 + (shape->has_int8 && !own_maxima(*shape)) : 0;
+}
 
 extern "C" int64_t anemoi_sm100_operand_bytes(const anemoi_sm100_shape* s, int which) {
   if (rec::validate_shape(s) != ANEMOI_SM100_OK) return ANEMOI_SM100_EINVAL;

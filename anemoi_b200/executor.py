@@ -336,8 +336,8 @@ class _Plan:
         self.side = _prefix_stream(device) if prefix_tokens else None
         self.side_handle = self.side.cuda_stream if prefix_tokens else None
         self.uses_scales = "nvfp4" in active
-        # kernels per call: V amax, preparation, draft, routing (and pair lists), attention, prefix rows
-        self.launches = 4 + int("int8" in active) + int(prefix_tokens > 0)
+        # kernels per call: preparation (with V's maxima), draft, routing (and pair lists), attention, prefix rows
+        self.launches = 3 + lib.anemoi_sm100_prepare_kernels(C.byref(shape)) + int(prefix_tokens > 0)
         self.launches -= lib.anemoi_sm100_drafts_in_routing(C.byref(shape))
         if not lib.anemoi_sm100_routes_in_one_kernel(C.byref(shape)):
             self.launches += 4 + 2 * int(pair_q64 and query_block == 64)

@@ -136,6 +136,11 @@ def test_repeated_public_calls(native_library):
     ((4, 16, 16), 3, 64, torch.bfloat16),      # eight: the largest cluster
     ((3, 19, 18), 3, 64, torch.float16),       # nine: atomics
     ((2, 8, 16), 130, 128, torch.float16),     # many heads
+    ((3, 16, 16), 12, 128, torch.bfloat16),    # found by the CTAs of values: 144 CTAs, the longest heads
+    ((3, 16, 16), 13, 128, torch.bfloat16),    # 156: the kernel of six ranges
+    ((1, 16, 96), 3, 64, torch.float16),       # 96 K values of a head: the last such length
+    ((1, 16, 97), 3, 64, torch.float16),       # past it
+    ((4, 16, 16), 3, 128, torch.bfloat16),     # the kernel's eight ranges
 ])
 def test_value_maxima(native_library, video, heads, dim, dtype):
     """max |v| per head and channel, with the largest value at either end of the sequence, twice."""
