@@ -9,9 +9,10 @@
 //
 // Between HBM and issue bound: maxima are taken two halves at a time, V is read two channels
 // at a time (lanes side by side; single halves 16 rows apart met in four banks), codes are
-// packed by the converting instructions.  With the maxima of V, 56 heads, prefix 512: S = 85,184 (11.5 GB)
-// 2,180-2,280 us = 5.1-5.3 TB/s, S = 33,272 730; Q64 INT8, S = 38,247 600; 8 heads x 4,109 tokens 24 (a half at a time,
-// codes packed by shifts: 2,544, 845, 794 and 48).
+// packed by the converting instructions, and the quotients, sums and products are packed fp32 instructions.  56 heads,
+// prefix 512, the maxima of V apart (184, 81, 93 and 4.4 us): S = 85,184 (11.5 GB) 2,023 us, S = 33,272 663; Q64 INT8, S =
+// 38,247 504; 8 heads x 4,109 tokens 13 (one value per instruction 2,075, 659, 526 and 14; NVFP4 D = 64, 4 heads of
+// 84,672 62, now 58).
 //
 // Numeric contract (reference: csrc/attention/cuda/sm120/q128_microscaling_preparation.cu):
 //   narrow  bf16 -> f32 -> f16 rn (:227-232); invalid slots and prefix padding are +0 (:369-374)
