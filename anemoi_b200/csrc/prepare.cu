@@ -52,7 +52,6 @@ struct PrepParams {
   const int32_t* indices;
   const int32_t* counts;
   int prefix_stages, stages, prefix_q_tiles;
-  int own_maxima;  // of a short sequence's V, by every CTA of values: no kernel before this one
   int64_t stride[6];  // token and head stride (elements) of q, k, v
 };
 
@@ -394,13 +393,23 @@ __device__ __forceinline__ float channel_maximum(const InT* v, const PrepParams&
 
 // Tasks of a head, in grid order: query tiles (video, prefix), then key/value blocks (R video blocks
 // of QB rows = QB/64 stages each, then the 64-row prefix stages).  With kSplit keys and values of a
-// block are separate CTAs (all keys first).
-template <typename InT, int QB, int D, bool kSplit>
+// block are separate CTAs (all keys first).  kOwnMaxima: of a short sequence's V, by every CTA of values, with no
+// kernel before this one.
+// kCells: a kernel holds the quantisers of the cells that its call may have.  They need the most registers, and what
+// is live around them is spilled for every call of the kernel (at 32 and 48 registers).  Of all cells / of the
+// call's, 16 heads x 33,272 tokens of D = 64, fp16, us: FP16 alone Q64 80.0 / 77.3, with max pools 100.5 / 79.8,
+// Q128 87.1 / 84.7; INT8 Q64 102 / 98.5, with max pools 132.5 / 102.
+enum Cells { kFp16Alone, kNoNvfp4, kAllCells };
+template <typename InT, int QB, int D, bool kSplit, bool kOwnMaxima, Cells kCells>
 __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __half* tile = reinterpret_cast<__half*>(smem_raw);
   __shared__ float red[kThreads / 32];
   __shared__ float recip[D];
+
+  // (read anew where they are asked for: kept, they take the registers that this is about)
+  const auto has_int8 = [&] { return kCells != kFp16Alone && p.s.has_int8; };
+  const auto has_nvfp4 = [&] { return kCells == kAllCells && p.s.has_nvfp4; };
 
   layer::grid_dependency_trigger();
   const int R = p.s.video_blocks;
@@ -414,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
     // ---------------- query tile (video or prefix) ----------------
     // (after the maxima's kernel, whose CTAs all began when what was before it in the stream was
     // complete; without INT8 there is no such kernel)
-    if (!p.s.has_int8 || p.own_maxima) layer::grid_dependency_wait();
+    if (kOwnMaxima || !has_int8()) layer::grid_dependency_wait();
     const bool video = task < R;
     const int t = video ? task : task - R;
     const int valid = video ? p.counts[t] : min(QB, p.s.prefix_tokens - t * QB);
@@ -432,13 +441,13 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
                                ((int64_t)head * R + t) * rec::q_fp16_bytes(QB, D),
                            tile, 0, QB);
       }
-      if (p.s.has_nvfp4) {
+      if (has_nvfp4()) {
         uint8_t* r4 = static_cast<uint8_t*>(p.o.q_nvfp4) +
                       ((int64_t)head * R + t) * rec::q_nvfp4_bytes(QB, D);
         write_nvfp4_rows<D>(r4, r4 + QB * D / 2, tile, 0, QB, p.s.q_global_scale);
       }
     }
-    if (p.s.has_int8) {
+    if (has_int8()) {
       const int64_t slot = (int64_t)head * qtiles_i8 + task;
       const float amax = tile_amax<D>(tile, 0, QB, red);
       const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1.0e-7f);
@@ -459,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
   const int stage0 = video ? p.prefix_stages + b * kF : b;
   const int valid = video ? p.counts[b] : min(64, p.s.prefix_tokens - b * 64);
   const int64_t rec0 = (int64_t)head * p.stages + stage0;
-  if (!p.s.has_int8 || p.own_maxima) layer::grid_dependency_wait();
+  if (kOwnMaxima || !has_int8()) layer::grid_dependency_wait();
   auto gather = [&](const void* src, int64_t token_stride, int64_t head_stride) {
     if (video) {
       gather_tile<InT, D, QB>(tile, static_cast<const InT*>(src), p, head, true, b * QB, 0, valid, token_stride,
@@ -484,12 +493,12 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
         write_fp16_tile<D>(static_cast<uint8_t*>(p.o.kv_fp16) + (rec0 + g) * rec::kv_fp16_bytes(D),
                            tile, g * 64, 64);
       }
-      if (p.s.has_nvfp4) {
+      if (has_nvfp4()) {
         uint8_t* r4 = static_cast<uint8_t*>(p.o.kv_nvfp4) + (rec0 + g) * rec::kv_nvfp4_bytes(D);
         write_nvfp4_rows<D>(r4, r4 + rec::kv_nvfp4_ksf_offset(D), tile, g * 64, 64,
                             p.s.k_global_scale);
       }
-      if (p.s.has_int8) {
+      if (has_int8()) {
         const float amax = tile_amax<D>(tile, g * 64, 64, red);
         const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1.0e-7f);
         if (threadIdx.x == 0) p.o.k_int8_scale[rec0 + g] = scale;
@@ -503,16 +512,16 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
 
   // ---- values of the same rows ----
   float maximum = 0.0f;
-  if (p.own_maxima) {
+  if constexpr (kOwnMaxima) {
     maximum = channel_maximum<InT, D>(static_cast<const InT*>(p.v), p, head, tile);
     if (block == 0 && threadIdx.x < D) p.o.v_amax[(int64_t)head * D + threadIdx.x] = maximum;
   }
   gather(p.v, p.stride[4], p.stride[5]);
-  if (p.s.has_int8) {
-    if (!p.own_maxima) layer::grid_dependency_wait();
+  if (has_int8()) {
+    if (!kOwnMaxima) layer::grid_dependency_wait();
     if (threadIdx.x < D) {
       const float amax =
-          p.own_maxima ? maximum : __half2float(__float2half_rn(p.o.v_amax[(int64_t)head * D + threadIdx.x]));
+          kOwnMaxima ? maximum : __half2float(__float2half_rn(p.o.v_amax[(int64_t)head * D + threadIdx.x]));
       recip[threadIdx.x] = amax == 0.0f ? 0.0f : __fdiv_rn(2.25f, amax);
       if (block == 0) p.o.v_e4m3_scale[(int64_t)head * D + threadIdx.x] = __fdiv_rn(amax, 2.25f);
     }
@@ -524,12 +533,12 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
                              64 * D * 2,
                          tile, g * 64, 64);
     }
-    if (p.s.has_int8) {
+    if (has_int8()) {
       write_v_e4m3<D>(static_cast<uint8_t*>(p.o.kv_int8) + (rec0 + g) * rec::kv_int8_bytes(D) +
                           64 * D,
                       tile, g * 64, recip);
     }
-    if (p.s.has_nvfp4) {
+    if (has_nvfp4()) {
       uint8_t* r4 = static_cast<uint8_t*>(p.o.kv_nvfp4) + (rec0 + g) * rec::kv_nvfp4_bytes(D);
       write_v_nvfp4<D>(r4 + rec::kv_nvfp4_v_offset(D), r4 + rec::kv_nvfp4_vsf_offset(D), tile,
                        g * 64, p.s.v_global_scale);
@@ -612,21 +621,20 @@ __global__ void __launch_bounds__(32 * kAmaxLanes) v_amax_kernel(const InT* v, i
 // own: reading 192 KB from L2 takes 1-2 us, a kernel for them 4 and its launch 2.5 on the host.  Calls, us, with the
 // kernel / without: 1,024 tokens x 4 heads x 64 31.5 / 29.3, 1,200 x 8 x 64 29.8 / 27.1; not taken: 2,040 x 3 x 64
 // 33.4 / 33.1, 2,040 x 30 x 64 (960 CTAs) 61 / 68, 2,040 x 40 x 128 93 / 119.
-constexpr int64_t kOwnMaxima = 96 * 1024;
+constexpr int64_t kOwnMaximaValues = 96 * 1024;
 inline bool own_maxima(const anemoi_sm100_shape& s) {
-  return s.has_int8 && (int64_t)s.seq_tokens * s.head_dim <= kOwnMaxima &&
+  return s.has_int8 && (int64_t)s.seq_tokens * s.head_dim <= kOwnMaximaValues &&
          ((int64_t)s.video_blocks + rec::prefix_stages(s)) * s.heads <= 148;
 }
 
-template <typename InT, int QB, int D, bool kSplit>
-int launch(PrepParams p, cudaStream_t stream) {
+template <typename InT, int QB, int D, bool kSplit, bool kOwnMaxima, Cells kCells>
+int launch(const PrepParams& p, cudaStream_t stream) {
   const size_t smem = (size_t)QB * (D + kPad) * sizeof(__half);
-  auto kernel = prepare_kernel<InT, QB, D, kSplit>;
+  auto kernel = prepare_kernel<InT, QB, D, kSplit, kOwnMaxima, kCells>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
-  p.own_maxima = own_maxima(p.s);
-  if (p.s.has_int8 && !p.own_maxima) {
+  if (p.s.has_int8 && !kOwnMaxima) {
     const int chunks = (p.s.heads * D / 8 + 31) / 32;
     // about three CTAs per SM, each with at least sixteen loads per thread: every CTA ends in 256 atomics
     // (8 heads x 4,109 tokens with eight per SM and two loads: the preparation took 40 us, now 24)
@@ -718,11 +726,18 @@ extern "C" int anemoi_sm100_prepare(const anemoi_sm100_shape* shape, const void*
   // Keys and values of a block in CTAs of their own: half the serial chain, which is quicker for
   // 128-row blocks (sweep's 4 heads 71 -> 64 us, 56 heads x 85,184 tokens 2,178 -> 2,128) and for small grids; for
   // many 64-row blocks a CTA's fixed cost weighs more (620 -> 687).
+  const bool own = own_maxima(s);  // (a grid that small is split)
   const bool split = s.query_block == 128 || ((int64_t)2 * s.video_blocks + p.prefix_stages) * s.heads <= 4 * 148;
-#define ANEMOI_DISPATCH(T)                                                                              \
-  (s.query_block == 128 ? (s.head_dim == 64 ? launch<T, 128, 64, true>(p, st) : launch<T, 128, 128, true>(p, st)) \
-   : split              ? (s.head_dim == 64 ? launch<T, 64, 64, true>(p, st) : launch<T, 64, 128, true>(p, st))   \
-                        : (s.head_dim == 64 ? launch<T, 64, 64, false>(p, st) : launch<T, 64, 128, false>(p, st)))
+#define ANEMOI_DIM(T, QB, SPLIT, OWN, CELLS) \
+  (s.head_dim == 64 ? launch<T, QB, 64, SPLIT, OWN, CELLS>(p, st) : launch<T, QB, 128, SPLIT, OWN, CELLS>(p, st))
+#define ANEMOI_CELLS(T, QB, SPLIT)                                                                        \
+  (s.has_nvfp4  ? (own ? ANEMOI_DIM(T, QB, true, true, kAllCells) : ANEMOI_DIM(T, QB, SPLIT, false, kAllCells)) \
+   : s.has_int8 ? (own ? ANEMOI_DIM(T, QB, true, true, kNoNvfp4) : ANEMOI_DIM(T, QB, SPLIT, false, kNoNvfp4))   \
+                : ANEMOI_DIM(T, QB, SPLIT, false, kFp16Alone))
+#define ANEMOI_DISPATCH(T) \
+  (s.query_block == 128 ? ANEMOI_CELLS(T, 128, true) : split ? ANEMOI_CELLS(T, 64, true) : ANEMOI_CELLS(T, 64, false))
   return s.input_is_bf16 ? ANEMOI_DISPATCH(__nv_bfloat16) : ANEMOI_DISPATCH(__half);
 #undef ANEMOI_DISPATCH
+#undef ANEMOI_CELLS
+#undef ANEMOI_DIM
 }

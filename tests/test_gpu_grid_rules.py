@@ -94,6 +94,45 @@ def test_preparation_of_many_q64_heads(native_library, dim, dtype):
             assert x.dtype == y.dtype and x.tobytes() == y.tobytes()
 
 
+@pytest.mark.parametrize("dim, query_block, heads, video, dtype", [
+    (64, 64, 2, (3, 9, 21), torch.float16),       # keys and values in CTAs of their own; maxima found by those of values
+    (128, 64, 2, (3, 30, 40), torch.bfloat16),    # the same after a kernel for the maxima
+    (64, 64, 32, (3, 9, 21), torch.bfloat16),     # one CTA per block for both
+    (128, 64, 32, (3, 9, 21), torch.float16),
+    (64, 128, 2, (3, 9, 21), torch.bfloat16),     # 128-row blocks, either way to the maxima
+    (64, 128, 32, (3, 9, 21), torch.float16),
+    (128, 128, 2, (2, 9, 21), torch.float16),
+    (128, 128, 32, (3, 9, 21), torch.bfloat16),
+])
+def test_records_do_not_depend_on_the_other_cells(native_library, dim, query_block, heads, video, dtype):
+    """A preparation kernel holds the cells that its call may have (FP16 alone, no NVFP4, all): each cell's records,
+    scales and the pools are those of every other kernel that writes them."""
+    from anemoi_b200 import native
+    from anemoi_b200.executor import make_shape
+    from anemoi_b200.layout import materialize_ragged_2d_layout
+
+    prefix = 70
+    q, k, v = (t.cuda() for t in smooth_fields(*video, heads, dim, prefix, seed=3, outliers=(5, 41), dtype=dtype))
+    layout = materialize_ragged_2d_layout(q.device, frames=video[0], height=video[1], width=video[2],
+                                          logical_block=query_block)
+    seen = {}
+    for maxpool in (False, True):
+        for cells in (("fp16",), ("int8",), ("int8", "fp16"), ("nvfp4",), ("nvfp4", "fp16"), ("nvfp4", "int8", "fp16")):
+            shape = make_shape(q, prefix_tokens=prefix, video_blocks=layout.video_blocks, query_block_size=query_block,
+                               active=cells, native_prefix=False, has_maxpool=maxpool, nvfp4_scales=(0.01, 0.01, 0.002))
+            store = native.allocate_operands(shape, q.device)
+            for t in store.buffers.values():
+                if t is not None:
+                    t.zero_()        # the bytes between the rows of a scale block are nobody's
+            native.prepare(shape, q, k, v, layout.indices, layout.counts, store)
+            torch.cuda.synchronize()
+            for name, t in store.buffers.items():
+                if t is not None:
+                    bits = t.view(torch.uint8) if t.dtype != torch.uint8 else t
+                    assert torch.equal(seen.setdefault(name, bits), bits), (name, cells, maxpool)
+    assert len(seen) == len(native.Operands._fields_)
+
+
 def test_repeated_public_calls(native_library):
     """A call with configuration objects seen before skips their checks, not the tensors': other
     strides, heads and types give what the staged path gives, and bad tensors still raise."""
