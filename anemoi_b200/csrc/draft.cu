@@ -72,13 +72,22 @@ __device__ __forceinline__ void row_logits(const __half* const (&q_pool)[2], con
     if (piece > 0) __syncthreads();
     if (c0 == 0) {
       // the rows of a warp interleaved: qs[warp][channel][RPW]
-      for (int idx = threadIdx.x; idx < kRows * (D / 8); idx += kThreads) {
-        const int r = idx % kRows, c8 = idx / kRows, row = row0 + r;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (row < R) v = __ldg(reinterpret_cast<const uint4*>(q_pool[map] + ((int64_t)head * R + row) * D) + c8);
-        const __half* h = reinterpret_cast<const __half*>(&v);
+      const __half* pools = (kMaps == 2 && map ? q_pool[1] : q_pool[0]) + (int64_t)head * R * D;
+      if ((reinterpret_cast<uintptr_t>(pools) & 15) == 0) {
+        for (int idx = threadIdx.x; idx < kRows * (D / 8); idx += kThreads) {
+          const int r = idx % kRows, c8 = idx / kRows, row = row0 + r;
+          uint4 v = make_uint4(0, 0, 0, 0);
+          if (row < R) v = __ldg(reinterpret_cast<const uint4*>(pools + (int64_t)row * D) + c8);
+          const __half* h = reinterpret_cast<const __half*>(&v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) qs[((r / RPW) * D + c8 * 8 + j) * RPW + r % RPW] = __half2float(h[j]);
+          for (int j = 0; j < 8; ++j) qs[((r / RPW) * D + c8 * 8 + j) * RPW + r % RPW] = __half2float(h[j]);
+        }
+      } else {  // query pools may start at any half
+#pragma unroll 1
+        for (int idx = threadIdx.x; idx < kRows * D; idx += kThreads) {
+          const int r = idx / D, c = idx % D, row = row0 + r;
+          qs[((r / RPW) * D + c) * RPW + r % RPW] = row < R ? __half2float(pools[(int64_t)row * D + c]) : 0.0f;
+        }
       }
     }
 #pragma unroll
@@ -434,6 +443,9 @@ int launch(const __half* qp, const __half* kp, const __half* qx, const __half* k
   return launch_rows<D, kBlend, 4>(qp, kp, qx, kx, w, R, H, prob, st);
 }
 
+// Key pools are read 16 bytes at a time, query pools and the map by halves where they are not aligned.
+bool aligned(const void* ptr, int bytes) { return reinterpret_cast<uintptr_t>(ptr) % bytes == 0; }
+
 }  // namespace
 
 extern "C" int anemoi_sm100_draft_probability(const anemoi_sm100_shape* shape, const void* q_pool,
@@ -459,6 +471,8 @@ extern "C" int anemoi_sm100_draft_probability(const anemoi_sm100_shape* shape, c
     maxpool_weight = 0.0f;
   }
   const bool blend = maxpool_weight != 0.0f;
+  if (!aligned(kp, 16) || !aligned(qp, 2) || !aligned(prob, 2) || (blend && (!aligned(kx, 16) || !aligned(qx, 2))))
+    return ANEMOI_SM100_EINVAL;
   if (D == 64)
     return blend ? launch<64, true>(qp, kp, qx, kx, maxpool_weight, R, H, prob, st)
                  : launch<64, false>(qp, kp, qx, kx, maxpool_weight, R, H, prob, st);
@@ -472,6 +486,9 @@ extern "C" int anemoi_sm100_draft_probability_jensen(const anemoi_sm100_shape* s
                                                      void* probability, void* stream) {
   if (rec::validate_shape(shape) != ANEMOI_SM100_OK || !q_pool || !k_pool || !q_second || !k_second ||
       !probability)
+    return ANEMOI_SM100_EINVAL;
+  if (!aligned(k_pool, 16) || !aligned(k_second, 16) || !aligned(q_pool, 2) || !aligned(q_second, 2) ||
+      !aligned(probability, 2))
     return ANEMOI_SM100_EINVAL;
   const int R = shape->video_blocks, H = shape->heads, D = shape->head_dim;
   const size_t smem = (size_t)kSlab * kChunk * 4 + (size_t)kWarps * 2 * D * 4 +

@@ -101,7 +101,8 @@ int anemoi_sm100_prepare(const anemoi_sm100_shape* shape, const void* q, const v
 int anemoi_sm100_prepare_kernels(const anemoi_sm100_shape* shape);
 
 /* Pooled-QK row softmax -> fp16 probability [H][R][R]; with 0 < w < 1 the mean
- * and max maps are blended, w == 1 uses the max pools only.
+ * and max maps are blended, w == 1 uses the max pools only.  Key pools are 16-byte
+ * aligned (ANEMOI_SM100_EINVAL otherwise), query pools and the map may start at any half.
  * Replaces sm120_h3_draft_probability (sm120/h3_draft_probability.cu:531-670). */
 int anemoi_sm100_draft_probability(const anemoi_sm100_shape* shape, const void* q_pool,
                                    const void* k_pool, const void* q_max_pool,
@@ -113,7 +114,8 @@ int anemoi_sm100_draft_probability(const anemoi_sm100_shape* shape, const void* 
  * with the max-pool blend): logits q.k/sqrt(D) + 0.5 * max((q2.k2 - (q*q).(k*k)) / D, 0) in fp32,
  * row softmax, fp16 [H][R][R].  `q_second`, `k_second` [H][R][D] fp16 are the per-channel second
  * moments of the blocks; anemoi_sm100_prepare writes them into the max-pool slots of the operands
- * when shape.has_maxpool == 2.  The reference computes this map with torch matmuls. */
+ * when shape.has_maxpool == 2.  Alignment as above.  The reference computes this map with torch
+ * matmuls. */
 int anemoi_sm100_draft_probability_jensen(const anemoi_sm100_shape* shape, const void* q_pool,
                                           const void* k_pool, const void* q_second,
                                           const void* k_second, void* probability, void* stream);
