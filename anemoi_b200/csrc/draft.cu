@@ -40,14 +40,27 @@ constexpr int kChunk = 128;                   // key blocks per pass: 4 per lane
 constexpr int kSlab = 64;                     // channels of the key tile held at a time
 constexpr int kMaxBlocks = 4096;              // rows per head the shared-memory buffers allow
 
+// Columns l, l + 32, ... of a row, lane l's share of the canonical sum, follow one another in shared memory as `fours`
+// 8-byte words.  Where four or more divide their number, as many lanes of sixteen would meet in a bank: there word k
+// lies at k ^ column_swizzle (no conflicts).  Elsewhere two meet at most, and the exclusive-or costs more (56 heads x 592
+// blocks x 128 213 us plain, 220 with it).  Padding instead of it takes the shared memory of four rows per warp: 56 x 448
+// with two maps 273 us, 327 padded, 56 x 1,024 618 and 791.
+__host__ __device__ constexpr int column_fours(int R) { return (R + 127) / 128; }
+template <bool kSwizzle>
+__device__ __forceinline__ int column_swizzle(int lane, int fours) {
+  if (!kSwizzle) return 0;
+  const int n = min(fours & -fours, 16);
+  return (lane >> (__clz(n) - 27)) & (n - 1);
+}
+
 // fp16 logits of kWarps * RPW query blocks against every key block of the head, for one pair of pools or two.
 // Each warp owns RPW (1, 2 or 4) rows, each lane four key columns of the 128-column pass.  The key tile holds
 // all channels, as it comes (fp16, two channels of a column in a word, so that one 16-byte load
 // serves two channels of four columns); query values are floats, read by broadcasts.  Every logit is still
 // the plain channel-ordered FMA chain (the canonical order).
-template <int D, int RPW, int kMaps>
+template <int D, int RPW, int kMaps, bool kSwizzle>
 __device__ __forceinline__ void row_logits(const __half* const (&q_pool)[2], const __half* const (&k_pool)[2], int head,
-                                           int R, int row0, uint32_t* kc, float* qs, __half* lg, int groups) {
+                                           int R, int row0, uint32_t* kc, float* qs, __half* lg, int fours) {
   constexpr int kRows = kWarps * RPW, kThreads = kWarps * 32;
   constexpr int kLoads = kChunk * (D / 8) / kThreads;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -132,20 +145,17 @@ __device__ __forceinline__ void row_logits(const __half* const (&q_pool)[2], con
         for (int j = 0; j < 4; ++j) acc[r][j] = __fmaf_rn(qv[RPW + r], k[j].y, acc[r][j]);
     }
     // (columns from R on are written, too, and left out by the reader)
-    __half* dst = lg + (map * kRows + warp * RPW) * 32 * groups + (lane & 7) * 4 * groups + (c0 >> 5) + (lane >> 3);
+    __half* dst = lg + ((map * kRows + warp * RPW) * 32 + (lane & 7) * 4) * 4 * fours + (lane >> 3);
+    if (!kSwizzle) dst += c0 >> 5;
 #pragma unroll
     for (int r = 0; r < RPW; ++r)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dst[(r * 32 + j) * groups] = __float2half_rn(__fmul_rn(acc[r][j], scale));
+      for (int j = 0; j < 4; ++j) {
+        const int word = kSwizzle ? (c0 >> 7) ^ column_swizzle<true>((lane & 7) * 4 + j, fours) : 0;
+        dst[((r * 32 + j) * fours + word) * 4] = __float2half_rn(__fmul_rn(acc[r][j], scale));
+      }
   }
   __syncwarp();
-}
-
-// Columns l, l + 32, ... of a row, lane l's share of the canonical sum, follow one another in shared memory:
-// `groups` values per lane, a multiple of four but not of sixteen (8-byte loads; two at most meet in a bank).
-__host__ __device__ inline int column_groups(int R) {
-  const int n = (R + 31) / 32, fours = (n + 3) / 4;
-  return 4 * (fours % 4 == 0 ? fours + 1 : fours);
 }
 
 // Four values of exp_canonical(x - m), packed arithmetic of the same roundings.  round(y) is a pair of
@@ -185,10 +195,11 @@ struct RowMap {
   float m, inv;
   float e[kKept][4];
 };
-template <bool kKeep>
+template <bool kKeep, bool kSwizzle>
 __device__ __forceinline__ void row_map(const __half* lg, int R, int fours, float zero, RowMap& row) {
   const int lane = threadIdx.x & 31;
-  const auto load = [&](int k) { return reinterpret_cast<const uint2*>(lg)[k]; };
+  const int swizzle = column_swizzle<kSwizzle>(lane, fours);
+  const auto load = [&](int k) { return reinterpret_cast<const uint2*>(lg)[k ^ swizzle]; };
   const int mine = (R - lane + 31) >> 5;  // the lane's values before the padding
   float m = -INFINITY;
   const auto fold = [&](int k) {
@@ -229,16 +240,16 @@ __device__ __forceinline__ void row_map(const __half* lg, int R, int fours, floa
   row.m = m;
   row.inv = __fdiv_rn(1.0f, s);
 }
-template <bool kBlend, bool kKeep>
-__device__ __forceinline__ void write_row(const __half* lg, const __half* lgx, float w, int R, int groups, float zero,
+template <bool kBlend, bool kKeep, bool kSwizzle>
+__device__ __forceinline__ void write_row(const __half* lg, const __half* lgx, float w, int R, float zero,
                                           __half* out) {
-  const int lane = threadIdx.x & 31, fours = (R + 127) / 128;
+  const int lane = threadIdx.x & 31, fours = column_fours(R);
   const float wm = __fsub_rn(1.0f, w);
-  lg += lane * groups;
-  lgx += lane * groups;
+  lg += lane * 4 * fours;
+  lgx += lane * 4 * fours;
   RowMap mean, most;
-  row_map<kKeep>(lg, R, fours, zero, mean);
-  if (kBlend) row_map<kKeep>(lgx, R, fours, zero, most);
+  row_map<kKeep, kSwizzle>(lg, R, fours, zero, mean);
+  if (kBlend) row_map<kKeep, kSwizzle>(lgx, R, fours, zero, most);
   const auto put = [&](int k, const float (&e)[4], const float (&ex)[4]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -254,10 +265,11 @@ __device__ __forceinline__ void write_row(const __half* lg, const __half* lgx, f
     for (int k = 0; k < kKept; ++k)
       if (k < fours) put(k, mean.e[k], kBlend ? most.e[k] : mean.e[k]);
   } else {
+    const int swizzle = column_swizzle<kSwizzle>(lane, fours);
     for (int k = 0; k < fours; ++k) {
       float e[4], ex[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      exp_four(reinterpret_cast<const uint2*>(lg)[k], mean.m, zero, e);
-      if (kBlend) exp_four(reinterpret_cast<const uint2*>(lgx)[k], most.m, zero, ex);
+      exp_four(reinterpret_cast<const uint2*>(lg)[k ^ swizzle], mean.m, zero, e);
+      if (kBlend) exp_four(reinterpret_cast<const uint2*>(lgx)[k ^ swizzle], most.m, zero, ex);
       put(k, e, ex);
     }
   }
@@ -375,16 +387,16 @@ __global__ void __launch_bounds__(kWarps * 32) draft_jensen_kernel(const __half*
   }
 }
 
-template <int D, bool kBlend, int RPW>
+template <int D, bool kBlend, int RPW, bool kSwizzle>
 __global__ void __launch_bounds__(kWarps * 32, 2)
     draft_kernel(const __half* q_pool, const __half* k_pool, const __half* q_max, const __half* k_max, float w, int R,
                  float zero, __half* prob) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   constexpr int kRows = kWarps * RPW;
-  const int groups = column_groups(R);
+  const int fours = column_fours(R);
   uint32_t* kc = reinterpret_cast<uint32_t*>(smem_raw);         // [D / 2][kChunk], two channels a word
   float* qs = reinterpret_cast<float*>(kc + D / 2 * kChunk);    // [kWarps][D][RPW]
-  __half* lg = reinterpret_cast<__half*>(qs + kRows * D);       // [kRows][32][groups], twice when blending
+  __half* lg = reinterpret_cast<__half*>(qs + kRows * D);       // [kRows][32][4 * fours], twice when blending
   const int head = blockIdx.y, row0 = blockIdx.x * kRows;
   const int warp = threadIdx.x >> 5;
 
@@ -392,15 +404,15 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
   layer::grid_dependency_trigger();
   const __half* const q[2] = {q_pool, q_max};
   const __half* const k[2] = {k_pool, k_max};
-  row_logits<D, RPW, kBlend ? 2 : 1>(q, k, head, R, row0, kc, qs, lg, groups);
+  row_logits<D, RPW, kBlend ? 2 : 1, kSwizzle>(q, k, head, R, row0, kc, qs, lg, fours);
   for (int r = warp * RPW; r < warp * RPW + RPW; ++r) {
     if (row0 + r >= R) break;
     __half* out = prob + ((int64_t)head * R + row0 + r) * R;
-    const __half *mean = lg + r * 32 * groups, *most = mean + kRows * 32 * groups;  // most: blend only
+    const __half *mean = lg + r * 128 * fours, *most = mean + kRows * 128 * fours;  // most: blend only
     if (R <= kKept * 128)
-      write_row<kBlend, true>(mean, most, w, R, groups, zero, out);
+      write_row<kBlend, true, kSwizzle>(mean, most, w, R, zero, out);
     else
-      write_row<kBlend, false>(mean, most, w, R, groups, zero, out);
+      write_row<kBlend, false, kSwizzle>(mean, most, w, R, zero, out);
   }
 }
 
@@ -408,14 +420,14 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 template <int D, bool kBlend, int RPW>
 size_t smem_bytes(int R) {
   constexpr size_t kRows = kWarps * RPW;
-  return (size_t)D / 2 * kChunk * 4 + kRows * D * 4 + kRows * 32 * column_groups(R) * 2 * (kBlend ? 2 : 1);
+  return (size_t)D / 2 * kChunk * 4 + kRows * D * 4 + kRows * 128 * column_fours(R) * 2 * (kBlend ? 2 : 1);
 }
 
 template <int D, bool kBlend, int RPW>
 int launch_rows(const __half* qp, const __half* kp, const __half* qx, const __half* kx, float w, int R,
                 int H, __half* prob, cudaStream_t st) {
   const size_t smem = smem_bytes<D, kBlend, RPW>(R);
-  auto kernel = draft_kernel<D, kBlend, RPW>;
+  auto kernel = column_fours(R) % 4 == 0 ? draft_kernel<D, kBlend, RPW, true> : draft_kernel<D, kBlend, RPW, false>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;

@@ -14,8 +14,15 @@ pytestmark = pytest.mark.gpu
     (29, 40, 128, 0.5),
     (60, 17, 64, 0.25),    # two: 180 CTAs of one, 120 of two
     (2, 1185, 128, 0.5),   # two: four would not leave room for two CTAs on an SM
+    (7, 273, 128, 0.5),    # two, three key tiles
     (80, 20, 128, 0.0),    # four
     (75, 33, 64, 1.0),     # four, the last CTA with one block
+    (20, 300, 128, 0.5),   # four, three key tiles: the query rows change with the map
+    (16, 672, 128, 0.0),   # four, six key tiles, exponentials kept
+    (20, 385, 64, 0.5),    # four key tiles: the row's words are swizzled
+    (18, 512, 128, 0.5),   # the last size of four rows with two maps
+    (10, 1024, 128, 0.0),  # and with one, eight key tiles
+    (10, 1025, 128, 0.0),  # past it
 ])
 def test_draft_rows_per_warp(native_library, heads, blocks, dim, weight):
     """The draft map of pooled blocks, bit for bit the oracle's, first and last head."""
@@ -40,8 +47,9 @@ def test_draft_rows_per_warp(native_library, heads, blocks, dim, weight):
 
 @pytest.mark.parametrize("blocks, weight", [
     (128, 0.0), (129, 0.5),                # one and two loads of four values per lane
-    (385, 0.0), (512, 0.5),                # sixteen values per lane: the padded rows
+    (384, 0.5), (385, 0.0), (512, 0.5),    # words in order, and swizzled
     (768, 0.5), (769, 0.5),                # exponentials kept, and formed twice
+    (1000, 0.5), (2048, 0.0),              # eight and sixteen words swizzled
 ])
 def test_draft_row_lengths(native_library, blocks, weight):
     """Rows around the steps of the softmax's layout, with logits far below the maximum among them, bit for bit."""
