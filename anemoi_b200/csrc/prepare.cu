@@ -466,9 +466,9 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepPar
   const int b = video ? block : block - R;
   const int nst = video ? kF : 1;
   const int stage0 = video ? p.prefix_stages + b * kF : b;
+  if (kOwnMaxima || !has_int8()) layer::grid_dependency_wait();  // (the layout's tables, too, may be new)
   const int valid = video ? p.counts[b] : min(64, p.s.prefix_tokens - b * 64);
   const int64_t rec0 = (int64_t)head * p.stages + stage0;
-  if (kOwnMaxima || !has_int8()) layer::grid_dependency_wait();
   auto gather = [&](const void* src, int64_t token_stride, int64_t head_stride) {
     if (video) {
       gather_tile<InT, D, QB>(tile, static_cast<const InT*>(src), p, head, true, b * QB, 0, valid, token_stride,

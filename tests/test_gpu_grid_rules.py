@@ -1,5 +1,7 @@
 """Kernels whose split of the work follows the size of the grid: each branch of the rule."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -139,6 +141,32 @@ def test_records_do_not_depend_on_the_other_cells(native_library, dim, query_blo
                     bits = t.view(torch.uint8) if t.dtype != torch.uint8 else t
                     assert torch.equal(seen.setdefault(name, bits), bits), (name, cells, maxpool)
     assert len(seen) == len(native.Operands._fields_)
+
+
+@pytest.mark.parametrize("cells", [("int8",), ("nvfp4",), ("fp16",)])
+def test_layout_written_just_before(native_library, cells):
+    """Slot tables that a kernel in front of the preparation writes (no kernel for the maxima between the two)."""
+    from anemoi_b200 import native
+    from anemoi_b200.executor import make_shape
+    from anemoi_b200.layout import materialize_ragged_2d_layout
+
+    video = (3, 9, 21)
+    q, k, v = (t.cuda() for t in smooth_fields(*video, 4, 64, 0, seed=4))
+    layout = materialize_ragged_2d_layout(q.device, frames=video[0], height=video[1], width=video[2], logical_block=64)
+    shape = make_shape(q, prefix_tokens=0, video_blocks=layout.video_blocks, query_block_size=64, active=cells,
+                       native_prefix=False, has_maxpool=False, nvfp4_scales=(0.01, 0.01, 0.002))
+    assert native.library().anemoi_sm100_prepare_kernels(C.byref(shape)) == 1
+    store = native.allocate_operands(shape, q.device)
+    native.prepare(shape, q, k, v, layout.indices, layout.counts, store)
+    want = {n: t.clone() for n, t in store.buffers.items() if n in ("q_pool", "k_pool", "k_int8_scale") and t is not None}
+    for _ in range(20):
+        counts, indices = torch.ones_like(layout.counts), torch.zeros_like(layout.indices)
+        torch.cuda.synchronize()
+        counts.copy_(layout.counts)
+        indices.add_(layout.indices)
+        native.prepare(shape, q, k, v, indices, counts, store)
+        for n, t in want.items():
+            assert torch.equal(store.buffers[n], t)
 
 
 def test_repeated_public_calls(native_library):
