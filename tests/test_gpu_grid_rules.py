@@ -230,3 +230,108 @@ def test_value_maxima(native_library, video, heads, dim, dtype):
             retained_fp16_ratio=0.0, video_shape=video, layer=0, query_block_size=64, return_parts=True)
         got = parts["store"].buffers["v_amax"].view(heads, dim)
         assert torch.equal(got, v[0].abs().amax(0).half().float())
+
+
+@pytest.mark.parametrize("video, prefix, heads, dim, query_block, dtype, kernels", [
+    ((4, 16, 16), 0, 4, 64, 64, torch.bfloat16, 1),
+    ((3, 16, 16), 0, 12, 128, 64, torch.float16, 1),      # 144 CTAs of values, 96 K values of a head
+    ((3, 16, 16), 0, 13, 128, 64, torch.float16, 2),
+    ((1, 16, 97), 0, 1, 64, 128, torch.bfloat16, 2),      # a row more than 96 K values
+    ((5, 15, 17), 200, 5, 64, 128, torch.bfloat16, 1),    # prefix stages count, and their values
+    ((2, 9, 21), 70, 16, 128, 128, torch.float16, 1),
+    ((2, 9, 21), 70, 25, 128, 128, torch.float16, 2),
+])
+def test_value_maxima_of_short_sequences(native_library, video, prefix, heads, dim, query_block, dtype, kernels):
+    """Where CTAs of values find the maxima themselves and where a kernel does: q|k|v views of one buffer, NaNs among
+    the values (they win no maximum), the largest in the prefix or the last token.  The same records as the same
+    heads among enough others for the kernel."""
+    from anemoi_b200 import native
+    from anemoi_b200.executor import make_shape
+    from anemoi_b200.layout import materialize_ragged_2d_layout
+
+    tokens, many = prefix + int(np.prod(video)), max(heads, 160)
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    base = torch.randn(1, tokens, heads, 3 * dim, generator=gen, device="cuda").to(dtype)
+    base[0, 0, :, 2 * dim + 3] = 9.0
+    base[0, tokens - 1, :, 2 * dim + 5] = -11.0
+    base[0, 7::50, :, 2 * dim + 8] = float("nan")
+    layout = materialize_ragged_2d_layout(base.device, frames=video[0], height=video[1], width=video[2],
+                                          logical_block=query_block)
+
+    def prepared(buffer):
+        q, k, v = buffer.split(dim, dim=3)
+        shape = make_shape(q, prefix_tokens=prefix, video_blocks=layout.video_blocks, query_block_size=query_block,
+                           active=("int8",), native_prefix=prefix > 0, has_maxpool=False)
+        store = native.allocate_operands(shape, q.device)
+        native.prepare(shape, q, k, v, layout.indices, layout.counts, store)
+        return native.library().anemoi_sm100_prepare_kernels(C.byref(shape)), store.buffers
+
+    launched, own = prepared(base)
+    assert launched == kernels
+    v = base[0, :, :, 2 * dim:].float()
+    want = torch.nan_to_num(v, nan=0.0).abs().amax(0)
+    assert torch.equal(own["v_amax"].view(heads, dim), want) and want[0, 3] == 9.0 and want[0, 5] == 11.0
+    launched, other = prepared(base.repeat(1, 1, -(-many // heads), 1))
+    assert launched == 2
+    for name in ("v_amax", "v_e4m3_scale", "kv_int8", "k_int8_scale", "q_int8", "q_int8_scale"):
+        bits = own[name].view(torch.uint8)
+        assert torch.equal(bits, other[name].view(torch.uint8)[:bits.numel()]), name
+
+
+def _scalar_map(q, k, q_max, k_max, weight):
+    """The map of one head with the kernel's maxima, which a NaN does not win (the oracle's does)."""
+    from oracle import route as R
+
+    def softmax(logit16):
+        x = logit16.astype(np.float32)
+        m = np.fmax.reduce(x, axis=1, keepdims=True, initial=-np.inf)
+        y = np.fmax(((x - m) * R.LOG2E).astype(np.float32), np.float32(-125.0))
+        n = np.rint(y).astype(np.float32)
+        f = (y - n).astype(np.float32)
+        p = np.full_like(f, R.EXP2_COEFFS[7])
+        for c in R.EXP2_COEFFS[6::-1]:
+            p = ((p * f).astype(np.float32) + c).astype(np.float32)
+        e = np.ldexp(p, n.astype(np.int32)).astype(np.float32)
+        return (e * (np.float32(1.0) / R._row_sum32(e)).astype(np.float32)[:, None]).astype(np.float32)
+
+    with np.errstate(all="ignore"):
+        if weight in (0.0, 1.0):
+            return softmax(R._logits16(*((q, k) if weight == 0.0 else (q_max, k_max)))).astype(np.float16)
+        w = np.float32(weight)
+        a = ((np.float32(1.0) - w) * softmax(R._logits16(q, k))).astype(np.float32)
+        return (a + (w * softmax(R._logits16(q_max, k_max))).astype(np.float32)).astype(np.float32).astype(np.float16)
+
+
+@pytest.mark.parametrize("heads, blocks, dim, weight", [
+    (2, 45, 64, 0.0), (3, 130, 128, 0.5),      # one row per warp
+    (7, 273, 128, 0.5),                        # two
+    (20, 300, 64, 1.0), (12, 800, 64, 0.0),    # four, exponentials kept and formed twice
+])
+def test_draft_map_of_infinities_and_nans(native_library, heads, blocks, dim, weight):
+    """Pools with infinities and NaNs, and logits that overflow: bit for bit the scalar arithmetic."""
+    from anemoi_b200 import native
+
+    shape = native.Shape(heads=heads, head_dim=dim, query_block=64, seq_tokens=blocks * 64, prefix_tokens=0,
+                         video_blocks=blocks, has_nvfp4=0, has_int8=1, has_fp16=0, has_prefix_query_int8=0,
+                         has_maxpool=int(weight != 0.0), input_is_bf16=1, q_global_scale=1.0, k_global_scale=1.0,
+                         v_global_scale=1.0)
+    g = torch.Generator().manual_seed(blocks)
+    pools = [torch.randn(heads, blocks, dim, generator=g).half() for _ in range(4)]
+    for t in pools[::2]:
+        t[:, 1] = float("nan")                    # a row of NaNs
+        t[:, 2, 5] = float("inf")
+        t[:, 3] *= 3000.0                         # logits past 65,504 once the keys are as large
+        t[:, 4] = 0.0                             # a row of ties
+    for t in pools[1::2]:
+        t[:, 7, 3] = float("nan")                 # a column of NaNs
+        t[:, 9, 5] = float("-inf")
+        t[:, 11::13] *= 3000.0
+    q, k, qx, kx = (t.cuda() for t in pools)
+    prob = torch.empty(heads, blocks, blocks, dtype=torch.float16, device="cuda")
+    p = native._ptr
+    assert native.library().anemoi_sm100_draft_probability(
+        shape, p(q), p(k), p(qx), p(kx), weight, p(prob), native._stream(prob.device)) == 0
+    for h in (0, heads - 1):
+        want = _scalar_map(*(t[h].numpy() for t in pools), weight)
+        assert np.isfinite(want).all()
+        assert np.array_equal(prob[h].cpu().numpy().view(np.uint16), want.view(np.uint16))

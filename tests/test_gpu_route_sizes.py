@@ -75,3 +75,65 @@ def test_map_and_routing_in_one_launch(native_library, video, query_block, dim, 
     for _ in range(3):
         assert torch.equal(executor.sm100_ragged_attention(q, k, v, **kw), staged)
     assert executor.last_status() == 0
+
+
+@pytest.mark.parametrize("video, query_block, dim, weight", [
+    ((1, 8, 16), 64, 64, 0.0), ((17, 8, 8), 64, 128, 0.5), ((31, 8, 8), 64, 64, 1.0), ((32, 8, 16), 128, 128, 0.5),
+])
+@pytest.mark.parametrize("values", ["plain", "ties", "overflow"])
+def test_map_of_the_one_launch(native_library, video, query_block, dim, weight, values):
+    """The map that the routing kernel forms (it lies in the layer's workspace), bit for bit the draft kernel's and
+    the oracle's on the same pools: rows of ties, logits far below the maximum, and ones that overflow to infinity."""
+    import numpy as np
+
+    from anemoi_b200 import executor, native
+    from oracle import route as R
+
+    heads, tokens = 3, video[0] * video[1] * video[2]
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    q, k, v = (torch.randn(1, tokens, heads, dim, generator=gen, device="cuda") for _ in range(3))
+    if values == "ties":
+        q[:, ::2] = 0.0
+        q[:, 1::2] *= 40.0
+        k[:, tokens // 2:] = k[:, :tokens - tokens // 2].clone()
+    elif values == "overflow":
+        q, k = q.abs() * 900.0, k * 900.0        # mean pools too have entries of some hundreds
+    q, k, v = (t.half() for t in (q, k, v))
+    plan = executor._Plan(q.device, tokens, heads, dim, q.dtype, 0, 0.7, 0.0, 0.6, 0.4, video, query_block, "int8",
+                          "int8", weight, True)
+    lib, shape = native.library(), plan.struct.shape
+    assert lib.anemoi_sm100_drafts_in_routing(C.byref(shape)) == 1
+    workspace = torch.empty(plan.bytes, dtype=torch.uint8, device="cuda")
+    out = torch.empty_like(q)
+    strides = executor._stride_array(*(heads * dim, dim) * 3)
+    assert plan.call(plan.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, executor._scale_array((1.0, 1.0, 1.0)),
+                     None, 0, 1, out.data_ptr(), workspace.data_ptr(), plan.bytes,
+                     torch.cuda.current_stream().cuda_stream, None) == 0
+    # the workspace is cut in this order, each piece a multiple of 256 bytes
+    at = 0
+    for which in (native.BUF_V_AMAX, native.BUF_Q_FP16, native.BUF_KV_FP16, native.BUF_Q_INT8, native.BUF_KV_INT8,
+                  native.BUF_Q_NVFP4, native.BUF_KV_NVFP4, native.BUF_Q_INT8_SCALE, native.BUF_K_INT8_SCALE,
+                  native.BUF_V_E4M3_SCALE):
+        at += -(-lib.anemoi_sm100_operand_bytes(C.byref(shape), which) // 256) * 256
+    blocks, pools = shape.video_blocks, {}
+
+    def take(*size):
+        nonlocal at
+        n = 2 * int(np.prod(size))
+        piece = workspace[at:at + n].view(torch.float16).view(size)
+        at += -(-n // 256) * 256
+        return piece
+
+    for name in ("q_pool", "k_pool", "q_max_pool", "k_max_pool")[:4 if weight else 2]:
+        pools[name] = take(heads, blocks, dim)
+    got = take(heads, blocks, blocks)
+    pools = {n: pools.get(n) for n in ("q_pool", "k_pool", "q_max_pool", "k_max_pool")}
+    store = native.OperandStore(shape=shape, struct=native.Operands(), buffers=pools)
+    assert torch.equal(got.view(torch.int16), native.draft_probability(shape, store, weight).view(torch.int16))
+    if values != "overflow":
+        for h in range(heads):
+            want = R.draft_probability(*(None if t is None else t[h].cpu().numpy() for t in pools.values()), weight)
+            assert np.array_equal(got[h].cpu().numpy().view(np.uint16), want.view(np.uint16))
+    else:
+        assert torch.isfinite(got).all()
+    assert executor.last_status() == 0
