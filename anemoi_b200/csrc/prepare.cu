@@ -40,7 +40,10 @@ using sm100::fmul2;
 constexpr int kThreads = 256;
 // CTAs per SM: 51 registers per thread for 128-row blocks, 32 for 64-row ones; fewer CTAs
 // with more registers are slower (56 heads x 33,272 tokens: 759 us at four, 728 at five, 821 at six).
-__host__ __device__ constexpr int min_ctas(int qb) { return qb == 128 ? 5 : 8; }
+// Four where the CTAs of values find the maxima themselves: such grids are small, and the maxima's loads in flight need
+// registers (with a query block's own limit 12 heads x 768 tokens of D = 128, Q64, 29.3 us a call, now 27.7; 2 x 1,040 of
+// D = 64 25.4 and 23.7).
+__host__ __device__ constexpr int min_ctas(int qb, bool own_maxima) { return own_maxima ? 4 : qb == 128 ? 5 : 8; }
 constexpr int kPad = 8;  // halves of padding per shared-memory row
 
 struct PrepParams {
@@ -401,7 +404,7 @@ __device__ __forceinline__ float channel_maximum(const InT* v, const PrepParams&
 // Q128 87.1 / 84.7; INT8 Q64 102 / 98.5, with max pools 132.5 / 102.
 enum Cells { kFp16Alone, kNoNvfp4, kAllCells };
 template <typename InT, int QB, int D, bool kSplit, bool kOwnMaxima, Cells kCells>
-__global__ void __launch_bounds__(kThreads, min_ctas(QB)) prepare_kernel(PrepParams p) {
+__global__ void __launch_bounds__(kThreads, min_ctas(QB, kOwnMaxima)) prepare_kernel(PrepParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __half* tile = reinterpret_cast<__half*>(smem_raw);
   __shared__ float red[kThreads / 32];
@@ -617,10 +620,13 @@ __global__ void __launch_bounds__(32 * kAmaxLanes) v_amax_kernel(const InT* v, i
   }
 }
 
-// Values of a head up to which every CTA of values finds the maxima of V itself, while each of them has an SM of its
-// own: reading 192 KB from L2 takes 1-2 us, a kernel for them 4 and its launch 2.5 on the host.  Calls, us, with the
-// kernel / without: 1,024 tokens x 4 heads x 64 31.5 / 29.3, 1,200 x 8 x 64 29.8 / 27.1; not taken: 2,040 x 3 x 64
-// 33.4 / 33.1, 2,040 x 30 x 64 (960 CTAs) 61 / 68, 2,040 x 40 x 128 93 / 119.
+// Values of a head up to which every CTA of values finds the maxima of V itself: reading 192 KB from L2 takes 1-2 us, a
+// kernel for them 4 and its launch 2.5 on the host.  Every such CTA reads all of its head's V, so their number is
+// bounded, too.  Calls of INT8, us, with the kernel / without, one after another: D = 64 Q64 4 heads x 1,024 tokens 25.1 /
+// 23.5, 6 x 1,536 (144 CTAs) 30.2 / 27.7, Q128 12 x 1,536 30.8 / 27.9; D = 128 Q64 12 x 768 28.0 / 27.7, Q128 24 x 768 30.8 / 28.7;
+// with 256 prefix tokens Q64 6 x 1,536 of D = 64 37.3 / 37.1, Q128 18 x 768 of D = 128 35.8 / 35.1.  Alone each gains 1-4; the
+// worst is 5 x 1,480 with 200 prefix tokens, Q64 D = 64: 35.9 / 36.9 one after another, 57.2 / 54.9 alone.  Past the lines, in an
+// earlier form: 3 x 2,040 of D = 64 33.4 / 33.1, 30 x 2,040 (960 CTAs) 61 / 68, 40 x 2,040 of D = 128 93 / 119.
 constexpr int64_t kOwnMaximaValues = 96 * 1024;
 inline bool own_maxima(const anemoi_sm100_shape& s) {
   return s.has_int8 && (int64_t)s.seq_tokens * s.head_dim <= kOwnMaximaValues &&
