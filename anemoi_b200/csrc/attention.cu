@@ -482,8 +482,9 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
 // MMA side
 // ------------------------------------------------------------------------------------------
 // The operands' descriptors are made once per phase and move with the slot: `step` is the slot's distance from
-// the first one in 16-byte units (NVFP4 D = 128 16 heads of S = 32,760 1.52 -> 1.50 ms, Q64 INT8 8 heads of 38,247
-// 1.72 -> 1.70: 10 of a stage's 2,050 warp instructions).
+// the first one in 16-byte units (NVFP4 D = 128 16 heads of S = 32,760 1.50 ms, 1.52 with descriptors made per stage, Q64
+// INT8 8 heads of 38,247 1.70 and 1.72; with the early token lookup some 25 of a stage's 2,050 warp instructions: 5.71e8 ->
+// 5.64e8 for 8 mixed heads of 33,272).
 __device__ __forceinline__ uint64_t moved(uint64_t desc, uint32_t step) {
   // (the address field does not overflow: shared memory ends below 2^18)
   uint32_t lo, hi;

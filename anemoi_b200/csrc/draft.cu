@@ -17,11 +17,11 @@
 // A CPU restatement with the same sequence reproduces the map bit for bit.
 //
 // Bound by the FMA pipe (56 heads x 672 blocks x 128 channels: 90 us of FMAs) and, as it is read here, as much again
-// of shared memory and conversions; the softmax takes some 60 us.  Before / now, us: that map 312 / 262, 56 x 592
-// 266 / 217, 7 x 672 51 / 38, 4 x 672 x 64 31 / 24, 7 x 273 with two maps 35 / 27, 8 x 33 with two 11.3 / 7.7.  What
-// changed: all channels of a key tile at a time instead of 64 (half the barriers), keys in shared memory as fp16
-// (half the bytes), both maps in one walk; the exponentials packed and without conversion
-// instructions, and kept between the sum and the quotients.
+// of shared memory and conversions; the softmax takes some 60 us.  So a key tile holds all channels (half the barriers
+// of 64 at a time), as fp16 (half the bytes of floats), both maps go in one walk, and the exponentials are packed, without
+// conversion instructions, and kept between the sum and the quotients.  us, 64 channels of floats and scalar
+// exponentials / so: that map 312 / 260, 56 x 592 266 / 213, 7 x 672 51 / 38.5, 4 x 672 x 64 31.4 / 24.1, 7 x 273 with two maps
+// 35.0 / 26.4, 8 x 33 with two 11.3 / 7.8.
 #include <cuda_fp16.h>
 
 #include "canonical.cuh"
@@ -442,8 +442,8 @@ int launch_rows(const __half* qp, const __half* kp, const __half* qx, const __ha
 // more rows.  But while a grid of fewer rows has no more CTAs than there are SMs, every CTA has one to
 // itself and the shorter one wins.  One / two / four rows, us: 8 heads x 33 blocks, two maps (40 CTAs of one row)
 // 7.7 / 10.6 / 16.4, 5 x 247 (80 of two) 8.5 / 7.0 / 10.5, 7 x 273, two maps (126 of two) 35.8 / 26.9 / 39.1, 4 x 672
-// (168 of two) 29.8 / 27.0 / 24.2, 16 x 225 (240) 25.8 / 18.6 / 15.7, 56 x 672 541 / 354 / 262 (eight rows, in CTAs of
-// four warps, 250).
+// (168 of two) 29.8 / 27.0 / 24.2, 16 x 225 (240) 25.8 / 18.6 / 15.7, 56 x 672 541 / 354 / 260; two / four, two maps, 56 x 512
+// (the last size of four) 396 / 324, 12 x 512 96.5 / 98.4.
 constexpr int kSms = 148;
 template <int D, bool kBlend>
 int launch(const __half* qp, const __half* kp, const __half* qx, const __half* kx, float w, int R,

@@ -9,10 +9,10 @@
 //
 // Between HBM and issue bound: maxima are taken two halves at a time, V is read two channels
 // at a time (lanes side by side; single halves 16 rows apart met in four banks), codes are
-// packed by the converting instructions, and the quotients, sums and products are packed fp32 instructions.  56 heads,
-// prefix 512, the maxima of V apart (184, 81, 93 and 4.4 us): S = 85,184 (11.5 GB) 2,023 us, S = 33,272 663; Q64 INT8, S =
-// 38,247 504; 8 heads x 4,109 tokens 13 (one value per instruction 2,075, 659, 526 and 14; NVFP4 D = 64, 4 heads of
-// 84,672 62, now 58).
+// packed by the converting instructions, and the quotients, sums and products are packed fp32 instructions (one value
+// per instruction / two, with the maxima of V, us: 56 heads of D = 128 and S = 85,184, all cells, 11.5 GB, 2,281 / 2,230; S =
+// 33,272 914 / 907, INT8 + FP16 with max pools 730 / 731; Q64 INT8, S = 38,247 601 / 588; NVFP4 D = 64, 4 heads of 84,672
+// 58.1 / 55.0; 8 heads of 4,109 19.0 / 18.9).
 //
 // Numeric contract (reference: csrc/attention/cuda/sm120/q128_microscaling_preparation.cu):
 //   narrow  bf16 -> f32 -> f16 rn (:227-232); invalid slots and prefix padding are +0 (:369-374)

@@ -662,10 +662,10 @@ __device__ __forceinline__ int fused_code(int key, const int (&key_b)[3], const 
 // ---- the draft map in the same kernel: up to 32 blocks per head, one CTA -------------------------
 // The arithmetic of draft.cu with a row per warp and a column per lane, the pools in the histogram's space.
 // Up to there a head's map is 1-2 us of work, and a launch of its own costs 2.5 us on the host and as much on the
-// device.  Calls without a prefix, us, in two launches / in one: 1,024 tokens x 4 heads (16 blocks) 35.5 / 31.7, 1,872 x 3
-// (15) 43.9 / 41.2, 2,016 x 8, two maps (16) 52.0 / 47.6, 4,032 x 8 (32) 69.6 / 69.4, 3,024 x 40 (24) 157.4 / 155.3.  With
-// prefix tiles on the side stream the one kernel loses (4,032 x 8 and 77: 77.5 / 86.7), and so it does with two
-// rows per warp and two columns per lane (51 blocks 32.4 / 36.2).
+// device.  Calls of INT8 without a prefix, us, in two launches / in one: D = 64 1 head x 8 blocks 22.3 / 20.4, 8 x 32 48.1 /
+// 47.1, 24 x 24, two maps 43.3 / 40.5; D = 128 1 x 32 34.2 / 34.3, 8 x 16, two maps 34.6 / 28.9, 56 x 32, two maps, Q128 222.3 /
+// 218.4.  In an earlier form, with prefix tiles on the side stream the one kernel lost (32 blocks x 8 heads and 77 tokens
+// 77.5 / 86.7), and so it did with two rows per warp and two columns per lane (51 blocks 32.4 / 36.2).
 constexpr int kDraftBlocks = 32;
 struct DraftPools {
   const __half* q[2];  // mean, max
@@ -1294,8 +1294,9 @@ extern "C" int anemoi_sm100_route_pairs(const anemoi_sm100_shape* shape, const v
 }
 
 bool layer::drafts_in_routing(const anemoi_sm100_shape& s) {
-  return s.prefix_tokens == 0 && s.video_blocks <= kDraftBlocks && fused_ctas(s.heads, s.video_blocks) == 1 &&
-         routes_pairs(s);
+  // (one CTA per head, and one kernel for lists and pairs, whatever the number of heads)
+  static_assert(kDraftBlocks <= 64 && kDraftBlocks * kDraftBlocks <= 65536 && kDraftBlocks <= kFusedWarps);
+  return s.prefix_tokens == 0 && s.video_blocks <= kDraftBlocks;
 }
 
 int layer::draft_and_route(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, float maxpool_weight,
