@@ -75,3 +75,24 @@ def test_kernels_match_the_oracle(native_library, vs, dim, qb, prefix):
         got = parts["prob"][head].cpu().numpy()
         assert np.array_equal(got.view(np.uint16), want.view(np.uint16)), head
     assert not torch.equal(parts["prob"], plain["prob"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads, blocks, dim", [(2, 129, 64), (1, 300, 64), (1, 260, 128)])
+def test_map_over_several_key_tiles(native_library, heads, blocks, dim):
+    """The map kernel alone, rows of more than one key tile and of a part of one, bit for bit."""
+    from anemoi_b200 import native
+    from oracle import route as R
+
+    shape = native.Shape(heads=heads, head_dim=dim, query_block=64, seq_tokens=blocks * 64, prefix_tokens=0,
+                         video_blocks=blocks, has_nvfp4=0, has_int8=1, has_fp16=0, has_prefix_query_int8=0,
+                         has_maxpool=2, input_is_bf16=1, q_global_scale=1.0, k_global_scale=1.0, v_global_scale=1.0)
+    gen = torch.Generator().manual_seed(blocks)
+    q, k = (torch.randn(heads, blocks, dim, generator=gen).half() for _ in range(2))
+    q2, k2 = ((t.float() ** 2 + torch.rand(t.shape, generator=gen)).half() for t in (q, k))
+    store = native.OperandStore(shape=shape, struct=native.Operands(), buffers={
+        "q_pool": q.cuda(), "k_pool": k.cuda(), "q_max_pool": q2.cuda(), "k_max_pool": k2.cuda()})
+    got = native.draft_probability_jensen(shape, store)
+    for h in range(heads):
+        want = R.draft_probability_jensen(*(t[h].numpy() for t in (q, k, q2, k2)))
+        assert np.array_equal(got[h].cpu().numpy().view(np.uint16), want.view(np.uint16))
