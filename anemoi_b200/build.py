@@ -11,7 +11,7 @@ PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libanemoi_sm100.so"
 SOURCES = ("prepare.cu", "draft.cu", "route.cu", "attention.cu", "assemble.cu", "peaks.cu", "producer.cu", "exchange.cu",
-           "layer.cu")
+           "match.cu", "layer.cu")
 FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC",

@@ -113,6 +113,9 @@ struct AttnParams {
   // of the two blocks the stage belongs to.  Null: one query block per CTA.
   const int32_t* pair_counts;  // [H][ceil(R/2)][4]
   const int32_t* pair_ids;     // [H][capacity], a pair's list starts at row_offset of block 2t
+  // Pairs of any two blocks, in launch order: [H][ceil(R/2)][8] first block, second or -1, start of the list in
+  // pair_ids, its stages, those of each phase.  Null: the pairs above.
+  const int4* pair_table;
   __half* out;       // [H][tiles*QB][D], or null:
   void* tokens;      // [S][H][D] in the caller's type: rows go straight to their tokens
   int tokens_bf16;
@@ -280,7 +283,8 @@ __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[16])
       : "memory");
 }
 
-// O[row][c] *= alpha (* colf[c] when given) for all D columns of the thread's row, kCols at a time.
+// O[row][c] *= (colf[c] when given, then) alpha, for all D columns of the thread's row, kCols at a time.  In that
+// order: a row whose first stage in a phase comes after its pair's has the two factors at two stages.
 template <int D, int kCols>
 __device__ __forceinline__ void rescale_o(uint32_t tmem_row, float alpha, const float* colf) {
   const float2 alpha2 = make_float2(alpha, alpha);
@@ -289,12 +293,6 @@ __device__ __forceinline__ void rescale_o(uint32_t tmem_row, float alpha, const 
     uint32_t r[kCols];
     tmem_ld(tmem_row + kColO + c0, r);
     tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < kCols; j += 2) {
-      const float2 v = fmul2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), alpha2);
-      r[j] = __float_as_uint(v.x);
-      r[j + 1] = __float_as_uint(v.y);
-    }
     if (colf != nullptr) {
 #pragma unroll
       for (int j = 0; j < kCols; j += 2) {
@@ -303,6 +301,12 @@ __device__ __forceinline__ void rescale_o(uint32_t tmem_row, float alpha, const 
         r[j] = __float_as_uint(v.x);
         r[j + 1] = __float_as_uint(v.y);
       }
+    }
+#pragma unroll
+    for (int j = 0; j < kCols; j += 2) {
+      const float2 v = fmul2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), alpha2);
+      r[j] = __float_as_uint(v.x);
+      r[j + 1] = __float_as_uint(v.y);
     }
     tmem_st(tmem_row + kColO + c0, r);
   }
@@ -559,13 +563,16 @@ __device__ __forceinline__ uint64_t v_desc(int d, int cell, uint32_t addr) {
 // instruction cache costs more than the constants give (three whole copies of the softmax stage,
 // 100 KB of code: 1.48 us per 64-key stage and SM at D = 64 instead of 1.11).
 // Where a row of the tile goes in `tokens` (element offset of its first channel), -1: a padding row.
-template <int D>
-__device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, int block0, int QB, int row) {
-  int token = block0 * QB + row;
+template <int D, bool kQ64>
+__device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, int block0, int block1, int row) {
+  constexpr int QB = kQ64 ? 64 : 128;
+  const bool second = kQ64 && row >= QB;
+  const int block = second ? block1 : block0, in = second ? row - QB : row;
+  int token = block * QB + in;
   if (p.dense_prefix) {
     if (token >= p.s.prefix_tokens) return -1;
   } else {
-    if (row % QB >= p.counts[block0 + row / QB]) return -1;
+    if (in >= p.counts[block]) return -1;
     token = p.s.prefix_tokens + p.indices[token];
   }
   return ((int64_t)token * p.s.heads + head) * D;
@@ -581,9 +588,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   // launch order of the head's query blocks (longest list first) as written by the routing
   // stage; 0 = no order given
   int tile = blockIdx.x;
-  const bool pairs = kQ64 && p.pair_counts != nullptr;
+  const bool table = kQ64 && p.pair_table != nullptr, pairs = table || (kQ64 && p.pair_counts != nullptr);
   const int pair_tiles = (p.s.video_blocks + 1) / 2;
-  if (!p.dense_prefix) {
+  if (!p.dense_prefix && !table) {
     const int ordered =
         pairs ? p.pair_counts[((int64_t)head * pair_tiles + blockIdx.x) * 4 + 3]
               : p.row_counts[((int64_t)head * p.s.video_blocks + blockIdx.x) * 4 + 3];
@@ -593,14 +600,24 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   // query blocks of this CTA (two for a complete pair) and the first one's index
   // (prefix tiles of 64 rows also go in twos: both walk every stage)
   const bool twos = pairs || (kQ64 && p.dense_prefix);
-  const int tile_blocks =
+  int tile_blocks =
       twos && 2 * tile + 1 < (p.dense_prefix ? p.q_tiles_int8 - p.s.video_blocks : p.s.video_blocks) ? 2 : 1;
-  const int block0 = twos ? 2 * tile : tile;
+  int block0 = twos ? 2 * tile : tile, block1 = block0 + 1;
 
   // ---- this tile's work list ----
   int cnt[3] = {0, p.stages, 0};
   const int32_t* list = nullptr;
-  if (!p.dense_prefix) {
+  if (table) {
+    const int4* entry = p.pair_table + ((int64_t)head * pair_tiles + tile) * 2;
+    const int4 e = entry[0], n = entry[1];
+    block0 = e.x;
+    block1 = e.y;
+    tile_blocks = e.y >= 0 ? 2 : 1;
+    list = p.pair_ids + (int64_t)head * p.capacity + e.z;
+    cnt[0] = n.x;
+    cnt[1] = n.y;
+    cnt[2] = n.z;
+  } else if (!p.dense_prefix) {
     const int32_t* ra = p.row_counts + ((int64_t)head * p.s.video_blocks + block0) * 4;
     const int32_t* counts = pairs ? p.pair_counts + ((int64_t)head * pair_tiles + tile) * 4 : ra;
     for (int c = 0; c < 3; ++c) cnt[c] = counts[c];
@@ -611,7 +628,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     // nothing to attend to: +0 rows (packed rows are left alone, the assembly knows)
     if (p.tokens != nullptr)
       for (int i = threadIdx.x; i < QB * tile_blocks * (D / 8); i += kThreads) {
-        const int64_t at = token_offset<D>(p, head, block0, QB, i / (D / 8));
+        const int64_t at = token_offset<D, kQ64>(p, head, block0, block1, i / (D / 8));
         if (at >= 0)
           *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.tokens) + at + i % (D / 8) * 8) = make_uint4(0, 0, 0, 0);
       }
@@ -651,13 +668,14 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       b->wc.abort = 0;
       b->wc.status = p.status;
       b->wc.limit_ns = p.wait_ns;
-      // phase c of a pair's union sits where the two blocks' phases before it would end
-      const int32_t* ra = pairs ? p.row_counts + ((int64_t)head * p.s.video_blocks + block0) * 4 : nullptr;
+      // phase c of a union of neighbours sits where the two blocks' phases before it would end
+      const bool apart = pairs && !table;
+      const int32_t* ra = apart ? p.row_counts + ((int64_t)head * p.s.video_blocks + block0) * 4 : nullptr;
       int before = 0;
       for (int c = 0; c < 3; ++c) {
         b->cnt[c] = cnt[c];
         b->first_of[c] = before;
-        before += pairs ? ra[c] + (tile_blocks == 2 ? ra[4 + c] : 0) : cnt[c];
+        before += apart ? ra[c] + (tile_blocks == 2 ? ra[4 + c] : 0) : cnt[c];
       }
     }
     mbar_init_fence();
@@ -689,6 +707,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       const int q_index_fp = head * p.s.video_blocks + block0;  // q_fp16 / q_nvfp4 record
       const int64_t q_index_i8 =
           (int64_t)head * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks : 0) + block0;
+      const int step = block1 - block0;  // from a pair's first record to its second
       const float sigma = (D == 64 ? 0.125f : 0.08838834764831845f) * 1.4426950408889634f;
       int phase_ord = 0, g = 0, v_fills = 0, moves = 0;
 #pragma unroll 1
@@ -711,13 +730,14 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           bulk_g2s(q_smem, qsrc, codes, &b->q_full, lead);
           bulk_g2s(q_smem + 128 * D / 2, qsrc + codes, qbytes - codes, &b->q_full, lead);
           if (tile_blocks == 2) {
-            bulk_g2s(q_smem + codes, qsrc + qbytes, codes, &b->q_full, lead);
-            bulk_g2s(q_smem + 128 * D / 2 + (qbytes - codes), qsrc + qbytes + codes, qbytes - codes,
-                     &b->q_full, lead);
+            const uint8_t* second = qsrc + (int64_t)step * qbytes;
+            bulk_g2s(q_smem + codes, second, codes, &b->q_full, lead);
+            bulk_g2s(q_smem + 128 * D / 2 + (qbytes - codes), second + codes, qbytes - codes, &b->q_full, lead);
           }
         } else {
-          // records of consecutive query blocks follow one another: two make a 128-row tile
-          bulk_g2s(q_smem, qsrc, qbytes * tile_blocks, &b->q_full, lead);
+          // two records of 64 rows make a 128-row tile
+          bulk_g2s(q_smem, qsrc, qbytes, &b->q_full, lead);
+          if (kQ64 && tile_blocks == 2) bulk_g2s(q_smem + qbytes, qsrc + (int64_t)step * qbytes, qbytes, &b->q_full, lead);
         }
         const int kvbytes = record_bytes(D, cell), kbytes = k_bytes(D, cell), rest = rest_offset(D, cell);
         const uint8_t* kvbase =
@@ -735,7 +755,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         const float* kscale = nullptr;
         if (cell == kI8) {
           q_scale[0] = p.o.q_int8_scale[q_index_i8];
-          if (tile_blocks == 2) q_scale[1] = p.o.q_int8_scale[q_index_i8 + 1];
+          if (tile_blocks == 2) q_scale[1] = p.o.q_int8_scale[q_index_i8 + step];
           kscale = p.o.k_int8_scale + (int64_t)head * p.stages;
         }
         const float base = cell == kNv ? sigma * p.s.q_global_scale * p.s.k_global_scale : sigma;
@@ -1037,9 +1057,10 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     uint16_t* dst = nullptr;
     if (p.tokens == nullptr) {
       if (row < QB * tile_blocks)
-        dst = reinterpret_cast<uint16_t*>(p.out) + ((int64_t)head * p.out_rows + (int64_t)block0 * QB + row) * D;
+        dst = reinterpret_cast<uint16_t*>(p.out) +
+              ((int64_t)head * p.out_rows + (kQ64 && row >= QB ? block1 * QB + row - QB : block0 * QB + row)) * D;
     } else if (row < QB * tile_blocks) {
-      const int64_t at = token_offset<D>(p, head, block0, QB, row);
+      const int64_t at = token_offset<D, kQ64>(p, head, block0, block1, row);
       if (at >= 0) dst = static_cast<uint16_t*>(p.tokens) + at;
     }
     wait(&b->wc, &b->all_done, 0, 7);
@@ -1110,7 +1131,7 @@ int launch(AttnParams& p, int tiles, cudaStream_t st) {
     if (!use[cell]) continue;
     one = cells++ == 0 ? cell : kAny;
     // a pair of Q64 blocks brings a second set of scale blocks
-    q_region = max(q_region, cell == kNv ? 128 * D / 2 + (D / 64) * 512 * (p.pair_counts ? 2 : 1)
+    q_region = max(q_region, cell == kNv ? 128 * D / 2 + (D / 64) * 512 * (p.pair_counts || p.pair_table ? 2 : 1)
                                          : (cell == kI8 ? 128 * D : 256 * D));
     slot = max(slot, slot_bytes(D, cell));
   }
@@ -1198,7 +1219,7 @@ int video_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operands
                     const int32_t* row_offset, const int32_t* row_counts, const int32_t* stage_ids,
                     const int32_t* pair_counts, const int32_t* pair_ids, int64_t list_capacity,
                     const int32_t* valid_k, void* out_packed, const TokenRows* rows, int32_t* status,
-                    void* stream) {
+                    void* stream, const int32_t* pair_table = nullptr) {
   if (rec::validate_shape(shape) != ANEMOI_SM100_OK || !ops || !row_offset || !row_counts ||
       !valid_k || (!out_packed && !rows) || !status || list_capacity <= 0)
     return ANEMOI_SM100_EINVAL;
@@ -1211,6 +1232,7 @@ int video_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operands
   p.stage_ids = stage_ids;
   p.pair_counts = pair_counts;
   p.pair_ids = pair_ids;
+  p.pair_table = reinterpret_cast<const int4*>(pair_table);
   p.capacity = list_capacity;
   p.valid_k = valid_k;
   p.out = static_cast<__half*>(out_packed);
@@ -1221,7 +1243,7 @@ int video_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operands
   p.q_tiles_int8 = shape->video_blocks + rec::prefix_query_tiles(*shape);
   p.out_rows = shape->video_blocks * shape->query_block;
   set_rows(p, rows);
-  const int tiles = pair_counts ? (shape->video_blocks + 1) / 2 : shape->video_blocks;
+  const int tiles = pair_counts || pair_table ? (shape->video_blocks + 1) / 2 : shape->video_blocks;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return launch_for(p, tiles, st);
 }
@@ -1286,10 +1308,12 @@ namespace layer {
 int video_rows(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, const int32_t* row_offset,
                const int32_t* row_counts, const int32_t* stage_ids, const int32_t* pair_counts,
                const int32_t* pair_ids, int64_t capacity, const int32_t* valid_k, const TokenRows& rows,
-               int32_t* status, cudaStream_t st) {
+               int32_t* status, cudaStream_t st, const int32_t* pair_table) {
   return video_attention(&s, &ops, row_offset, row_counts, stage_ids, pair_counts, pair_ids, capacity, valid_k,
-                         nullptr, &rows, status, st);
+                         nullptr, &rows, status, st, pair_table);
 }
+
+uint64_t wait_limit_ns() { return g_wait_limit_ns; }
 
 int prefix_rows(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, const int32_t* valid_k,
                 const TokenRows& rows, int32_t* status, cudaStream_t st) {

@@ -23,6 +23,7 @@
 namespace {
 
 constexpr int64_t kAlign = 256;
+constexpr int kMatchMaxBlocks = 4096;
 constexpr int kPrefixFillsGpu = 148;  // prefix CTAs from which they start after routing: one per SM
 
 int64_t up(int64_t n) { return (n + kAlign - 1) / kAlign * kAlign; }
@@ -31,9 +32,27 @@ struct Workspace {
   anemoi_sm100_operands ops;
   uint8_t* prob;
   int32_t *row_offset, *row_counts, *stage_ids, *pair_counts, *pair_ids;
+  int32_t* pair_table;  // pairs chosen by what their lists share; null: neighbours
+  layer::PairBits pair_bits;
   uint8_t* scratch;
   int64_t scratch_bytes, bytes;
 };
+
+// Whether the Q64 pairs are chosen by what their lists share (match.cu) rather than by index: where that many
+// stages, the blocks' lists summed, are walked that the choice, some 10 us between routing and attention, pays even for
+// inputs in which no blocks attend alike.  Index / chosen, us, 80 % dropped and 200 tokens of prefix, such inputs and ones with
+// two loud channels:  INT8, D = 128, 4 heads x 225 blocks (44,100 stages) 187 / 196, 211 / 195; 8 x 225 (88,200) 304 / 304,
+// 324 / 286; 8 x 525 (457,800) 1,181 / 1,171, 1,218 / 1,005.  NVFP4, D = 64, 5 x 247 (61,010) 186 / 190, 191 / 171;
+// 8 x 225 236 / 235, 242 / 212.  Several cells, whose lists share less (a column in the same cell), D = 64:  8 x 225 362 /
+// 369, 370 / 340; 16 x 225 (176,400) 644 / 647, 663 / 587; 8 x 525 1,351 / 1,348, 1,376 / 1,175.
+constexpr int64_t kMatchStages = 80000, kMatchStagesMixed = 160000;
+bool matches(const anemoi_sm100_layer_plan& p) {
+  const int R = p.shape.video_blocks;
+  const int64_t stages = p.shape.heads * (p.n16 + p.n8 + p.n4 + (int64_t)R * rec::prefix_stages(p.shape));
+  const int cells = (p.n16 > 0) + (p.n8 > 0) + (p.n4 > 0);
+  return R > 32 && R <= kMatchMaxBlocks && rec::stages(p.shape) < (1 << 30) &&
+         stages >= (cells > 1 ? kMatchStagesMixed : kMatchStages);
+}
 
 // Cuts `base` (null: only the size is wanted) into the call's buffers.
 Workspace cut(const anemoi_sm100_layer_plan& p, uint8_t* base) {
@@ -63,15 +82,23 @@ Workspace cut(const anemoi_sm100_layer_plan& p, uint8_t* base) {
     w.ops.q_max_pool = operand(ANEMOI_SM100_BUF_POOL);
     w.ops.k_max_pool = operand(ANEMOI_SM100_BUF_POOL);
   }
+  const bool pairs = p.pair_q64 && s.query_block == 64, matched = pairs && matches(p);
   w.prob = take(H * R * R * 2);
   w.row_offset = reinterpret_cast<int32_t*>(take(H * R * 4));
   w.row_counts = reinterpret_cast<int32_t*>(take(H * R * 16));
-  const bool pairs = p.pair_q64 && s.query_block == 64, fused = pairs && layer::routes_pairs(s);
+  const bool fused = pairs && layer::routes_pairs(s);
   const int64_t list = H * p.list_capacity * 4;
   // (routed in one kernel, the pairs need neither the blocks' own lists nor scratch)
-  if (!fused) w.stage_ids = reinterpret_cast<int32_t*>(take(list));
-  if (pairs) {
+  if (!fused && !matched) w.stage_ids = reinterpret_cast<int32_t*>(take(list));
+  if (matched) {
+    const int64_t budget[3] = {p.n4, p.n8, p.n16};
+    for (int c = 0; c < 3; ++c) w.pair_bits.slot[c] = budget[c] > 0 ? w.pair_bits.phases++ : -1;
+    w.pair_bits.words = reinterpret_cast<uint32_t*>(take(H * w.pair_bits.phases * R * layer::pair_bit_words(R) * 4));
+    w.pair_table = reinterpret_cast<int32_t*>(take(H * ((R + 1) / 2) * 32));
+  } else if (pairs) {
     w.pair_counts = reinterpret_cast<int32_t*>(take(H * ((R + 1) / 2) * 16));
+  }
+  if (pairs) {
     w.pair_ids = reinterpret_cast<int32_t*>(take(list));
   }
   w.scratch_bytes = fused ? 0 : anemoi_sm100_route_scratch_bytes(&s);
@@ -93,6 +120,10 @@ extern "C" int anemoi_sm100_routes_in_one_kernel(const anemoi_sm100_shape* shape
 
 extern "C" int anemoi_sm100_drafts_in_routing(const anemoi_sm100_shape* shape) {
   return rec::validate_shape(shape) == ANEMOI_SM100_OK && layer::drafts_in_routing(*shape);
+}
+
+extern "C" int anemoi_sm100_matches_pairs(const anemoi_sm100_layer_plan* plan) {
+  return valid(plan) && plan->pair_q64 && plan->shape.query_block == 64 && matches(*plan);
 }
 
 extern "C" int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan) {
@@ -152,7 +183,14 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
     code = anemoi_sm100_draft_probability(&s, w.ops.q_pool, w.ops.k_pool, w.ops.q_max_pool, w.ops.k_max_pool,
                                           p.maxpool_weight, w.prob, stream);
     if (code != ANEMOI_SM100_OK) return done(code);
-    if (pair_counts != nullptr && layer::routes_pairs(s)) {
+    if (w.pair_table != nullptr) {
+      const int phase = s.prefix_tokens > 0 || p.prefix_phase < 0 || p.prefix_phase > 2 ? p.prefix_phase : -1;
+      code = layer::route_bits(s, w.prob, p.n16, p.n8, p.n4, phase, w.scratch, w.row_offset, w.row_counts,
+                               w.pair_bits, p.list_capacity, st);
+      if (code == ANEMOI_SM100_OK)
+        code = layer::match_pairs(s, w.pair_bits, phase, w.row_offset, w.row_counts, w.pair_table, w.pair_ids,
+                                  p.list_capacity, p.status, st);
+    } else if (pair_counts != nullptr && layer::routes_pairs(s)) {
       code = anemoi_sm100_route_pairs(&s, w.prob, p.n16, p.n8, p.n4, p.prefix_phase, w.row_offset, w.row_counts,
                                       w.pair_counts, w.pair_ids, p.list_capacity, stream);
     } else {
@@ -166,7 +204,7 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
   if (code != ANEMOI_SM100_OK) return done(code);
   if (late && (code = prefix()) != ANEMOI_SM100_OK) return done(code);
   code = layer::video_rows(s, w.ops, w.row_offset, w.row_counts, w.stage_ids, pair_counts, w.pair_ids,
-                           p.list_capacity, p.valid_k, rows, p.status, st);
+                           p.list_capacity, p.valid_k, rows, p.status, st, w.pair_table);
   if (code != ANEMOI_SM100_OK) return done(code);
   if (s.prefix_tokens > 0) {
     if (cudaEventCreateWithFlags(&join, cudaEventDisableTiming) != cudaSuccess ||

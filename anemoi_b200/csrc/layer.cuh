@@ -22,7 +22,7 @@ struct TokenRows {
 int video_rows(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, const int32_t* row_offset,
                const int32_t* row_counts, const int32_t* stage_ids, const int32_t* pair_counts,
                const int32_t* pair_ids, int64_t capacity, const int32_t* valid_k, const TokenRows& rows,
-               int32_t* status, cudaStream_t st);
+               int32_t* status, cudaStream_t st, const int32_t* pair_table);
 int prefix_rows(const anemoi_sm100_shape& s, const anemoi_sm100_operands& ops, const int32_t* valid_k,
                 const TokenRows& rows, int32_t* status, cudaStream_t st);
 // Whether the draft map is formed by the routing kernel, and both in one launch (pair_counts: for pairs).
@@ -31,6 +31,24 @@ int draft_and_route(const anemoi_sm100_shape& s, const anemoi_sm100_operands& op
                     void* probability, int64_t n16, int64_t n8, int64_t n4, int prefix_phase, int32_t* row_offset,
                     int32_t* row_counts, int32_t* stage_ids, int32_t* pair_counts, int32_t* pair_ids, int64_t capacity,
                     cudaStream_t st);
+// What the routing leaves for the choice of the Q64 pairs: bit j of a row = column j is in its list, per phase with a
+// budget, [H][phases][R][pair_bit_words(R)] words; `slot`: place of the NVFP4, INT8, FP16 phase among them, or -1.
+struct PairBits {
+  uint32_t* words;
+  int phases, slot[3];
+};
+// (rows are whole 16-byte pieces: 128 columns)
+__host__ __device__ inline int pair_bit_words(int R) { return (R + 127) / 128 * 4; }
+int route_bits(const anemoi_sm100_shape& s, const void* probability, int64_t n16, int64_t n8, int64_t n4,
+               int prefix_phase, void* scratch, int32_t* row_offset, int32_t* row_counts, const PairBits& bits,
+               int64_t capacity, cudaStream_t st);
+// The pairs and their lists.  `table` [H][ceil(R/2)][8] in launch order: first block, second (-1: none), where the
+// list starts, its stages, and those of each phase.
+int match_pairs(const anemoi_sm100_shape& s, const PairBits& bits, int prefix_phase, const int32_t* row_offset,
+                const int32_t* row_counts, int32_t* table, int32_t* pair_ids, int64_t capacity, int32_t* status,
+                cudaStream_t st);
+// Limit of the bounded waits of kernels launched now.
+uint64_t wait_limit_ns();
 // Whether a Q64 call's pair lists come out of the routing kernel itself.
 bool routes_pairs(const anemoi_sm100_shape& s);
 // The prefix rows alone, from [H][rows][D] (fp16, or already in the caller's type).

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) rowstat_kernel(const unsigned 
 // order (the fourth entries stay 0).
 constexpr int kOrderMaxBlocks = 4096;
 __global__ void __launch_bounds__(1024) headscan_kernel(int R, const int* thr, int* stat, int factor,
-                                                        int prefix_stages, int prefix_phase,
+                                                        int prefix_stages, int prefix_phase, bool ordered,
                                                         int32_t* row_offset, int32_t* row_counts) {
   __shared__ long long warp_sum[32];
   __shared__ int total_s[kOrderMaxBlocks];
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(1024) headscan_kernel(int R, const int* thr, i
       if (row < kOrderMaxBlocks) total_s[row] = total;
     }
   }
-  if (R > kOrderMaxBlocks) return;
+  if (!ordered || R > kOrderMaxBlocks) return;
   __syncthreads();
   int32_t* rc = row_counts + (int64_t)head * R * 4;
   for (int i = threadIdx.x; i < R; i += 1024) {
@@ -735,12 +735,43 @@ __device__ __forceinline__ void draft_rows(const DraftPools& d, int head, int R,
   __syncthreads();
 }
 
+// What the kernel leaves: the rows' lists, the union lists of neighbouring Q64 blocks, or a bit per (row, phase,
+// column) for the choice of the pairs (match.cu).
+enum Leaves : int { kLists = 0, kNeighbours = 1, kBits = 2 };
+
+// A row's bits, 32 columns (a word) at a time: lane w keeps word w of each phase until 32 are there.
+struct RowBits {
+  uint32_t* out[3];  // by precision code - 1; null: no budget
+  uint32_t keep[3];
+  __device__ __forceinline__ void put(int k, int word, uint32_t members) {
+    if ((word & 31) == (int)(threadIdx.x & 31)) keep[k] = members;
+  }
+  // After word `word` (the row's last of `words` in use, or the last of a group of 32); rows are `stride` words.
+  __device__ __forceinline__ void flush(int word, int words, int stride) {
+    if ((word & 31) != 31 && word != words - 1) return;
+    const int lane = threadIdx.x & 31, at = (word & ~31) + lane;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (out[k] != nullptr && at < stride) out[k][at] = keep[k];
+      keep[k] = 0;
+    }
+  }
+};
+__device__ __forceinline__ RowBits row_bits(const layer::PairBits& bits, int head, int R, int row, int stride) {
+  RowBits b = {};
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (bits.slot[k] >= 0) b.out[k] = bits.words + (((int64_t)head * bits.phases + bits.slot[k]) * R + row) * stride;
+  return b;
+}
+
 // kDraft: 0, or the head dimension of the pools that the map is formed from first.
-template <bool kPairs, int kDraft>
+template <int kLeaves, int kDraft>
 __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
     const DraftPools draft, const unsigned short* prob, int R, int rows_per, int b0, int b1, int b2, int factor, int prefix_stages,
     int prefix_phase, int64_t capacity, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids,
-    int32_t* pair_counts, int32_t* pair_ids) {
+    int32_t* pair_counts, int32_t* pair_ids, const layer::PairBits bits) {
+  constexpr bool kPairs = kLeaves == kNeighbours;
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) int hist[];
   FusedShared& sh = *reinterpret_cast<FusedShared*>(hist + kBins);
@@ -939,7 +970,29 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   __syncthreads();
   // ---- lists ----
   const bool active[3] = {b2 > b1, b1 > b0, b0 > 0};  // phases with a budget
-  if (!kPairs) {
+  if constexpr (kLeaves == kBits) {
+    const int words = (R + 31) / 32, stride = layer::pair_bit_words(R);
+    for (int i = warp; i < mine; i += kFusedWarps) {
+      RowBits row = row_bits(bits, head, R, r0 + i, stride);
+      int run[3] = {stat[i * 6 + 3], stat[i * 6 + 4], stat[i * 6 + 5]};
+      const unsigned short* src = map + (int64_t)(r0 + i) * R;
+      for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
+        int key[kAhead];
+        fused_keys<kOwn>(src, j0, R, key);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          if (j0 + u * 32 >= R) break;
+          const int c = fused_code(key[u], key_b, quota_b, run, lower);
+#pragma unroll
+          for (int k = 1; k <= 3; ++k)
+            if (active[k - 1]) row.put(k - 1, j0 / 32 + u, __ballot_sync(0xffffffffu, c == k));
+          row.flush(j0 / 32 + u, words, stride);
+        }
+      }
+    }
+    if (ctas > 1) cluster.sync();  // no CTA leaves while another may still read its sums
+    return;
+  } else if constexpr (!kPairs) {
     for (int i = warp; i < mine; i += kFusedWarps) {
       const int n0 = stat[i * 6], n1 = stat[i * 6 + 1], total = totals[i];
       const int64_t base = offset[i];
@@ -1050,12 +1103,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   if (ctas > 1) cluster.sync();  // no CTA leaves while another may still read its totals
 }
 
-template <bool kPairs, int kDraft>
+template <int kLeaves, int kDraft>
 int launch_fused(const anemoi_sm100_shape& s, const DraftPools& draft, const void* probability, int64_t n16, int64_t n8, int64_t n4,
                  int prefix_phase, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids, int64_t capacity,
-                 int32_t* pair_counts, int32_t* pair_ids, cudaStream_t st) {
+                 int32_t* pair_counts, int32_t* pair_ids, cudaStream_t st, const layer::PairBits& bits = {}) {
   const int H = s.heads, R = s.video_blocks, ctas = fused_ctas(H, R);
-  auto kernel = route_fused_kernel<kPairs, kDraft>;
+  auto kernel = route_fused_kernel<kLeaves, kDraft>;
   // Function attributes belong to a device: the opt-in is made at every call (a cheap host-side
   // driver call), so a process that routes on several GPUs, or from several host threads,
   // never launches the kernel without the opt-in for its dynamic shared memory.
@@ -1064,10 +1117,36 @@ int launch_fused(const anemoi_sm100_shape& s, const DraftPools& draft, const voi
   return layer::launch_cluster(kernel, dim3(ctas, H), dim3(ctas), dim3(kFusedThreads), fused_smem(), st,
                                draft, static_cast<const unsigned short*>(probability), R, fused_rows(R, ctas), (int)n16,
                                (int)(n16 + n8), (int)(n16 + n8 + n4), s.query_block / 64, rec::prefix_stages(s),
-                               prefix_phase, capacity, row_offset, row_counts, stage_ids, pair_counts,
-                               pair_ids) == cudaSuccess
+                               prefix_phase, capacity, row_offset, row_counts, stage_ids, pair_counts, pair_ids,
+                               bits) == cudaSuccess
              ? ANEMOI_SM100_OK
              : ANEMOI_SM100_ELAUNCH;
+}
+
+// One warp per row writes the row's bits instead, for the choice of the Q64 pairs (match.cu).
+__global__ void __launch_bounds__(kRowWarps * 32) emit_bits_kernel(const unsigned short* prob, int R, const int* thr,
+                                                                   const int* stat, const layer::PairBits bits) {
+  const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5), head = blockIdx.y;
+  if (row >= R) return;
+  const int lane = threadIdx.x & 31;
+  const unsigned lower = (1u << lane) - 1u;
+  int key_b[3], quota_b[3], run[3];
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    key_b[b] = thr[head * 8 + 2 * b];
+    quota_b[b] = thr[head * 8 + 2 * b + 1];
+    run[b] = stat[((int64_t)head * R + row) * kStat + 3 + b];
+  }
+  const int words = (R + 31) / 32, stride = layer::pair_bit_words(R);
+  RowBits out = row_bits(bits, head, R, row, stride);
+  const unsigned short* src = prob + ((int64_t)head * R + row) * R;
+  for (int w = 0; w < words; ++w) {
+    const int j = w * 32 + lane;
+    const int c = fused_code(j < R ? (__ldg(src + j) & 0x7fff) : -2, key_b, quota_b, run, lower);
+#pragma unroll
+    for (int k = 1; k <= 3; ++k) out.put(k - 1, w, __ballot_sync(0xffffffffu, c == k));
+    out.flush(w, words, stride);
+  }
 }
 
 // Q64 query blocks 2t and 2t+1 of a head run as one CTA of the attention kernel (rows 0-63 and
@@ -1129,6 +1208,37 @@ __global__ void __launch_bounds__(1024) pair_order_kernel(int pairs, int32_t* pa
     for (int j = 0; j < pairs; ++j) rank += (total_s[j] > mine) || (total_s[j] == mine && j < i);
     pc[rank * 4 + 3] = i + 1;
   }
+}
+
+// The launches in front of the lists where routing takes several kernels: histogram, boundaries, per-row counts, and
+// the scans over the rows with the lists' offsets and (`ordered`) the launch order.
+int rank_rows(const anemoi_sm100_shape& s, const void* probability, int64_t n16, int64_t n8, int64_t n4,
+              int prefix_phase, bool ordered, void* scratch, int32_t* row_offset, int32_t* row_counts, RouteScratch& sc,
+              cudaStream_t st) {
+  const int H = s.heads, R = s.video_blocks;
+  const int64_t items = (int64_t)R * R;
+  sc.hist = static_cast<int*>(scratch);
+  sc.thr = sc.hist + (int64_t)H * kBins;
+  sc.stat = sc.thr + (int64_t)H * 8;
+  if (cudaMemsetAsync(sc.hist, 0, (size_t)H * kBins * 4, st) != cudaSuccess)
+    return ANEMOI_SM100_ELAUNCH;
+  const unsigned short* prob = static_cast<const unsigned short*>(probability);
+  // Function attributes belong to a device: the opt-in is made at every call (a cheap host-side
+  // driver call), so a process that routes on several GPUs, or from several host threads,
+  // never launches the kernel without the opt-in for its dynamic shared memory.
+  if (cudaFuncSetAttribute(hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHalfBins * 4) !=
+      cudaSuccess)
+    return ANEMOI_SM100_ELAUNCH;
+  // about two waves of histogram CTAs per key-range half, each with at least 8192 items
+  const int chunks = (int)max((int64_t)1, min(min((int64_t)16, items / 8192), (int64_t)((296 + H / 2) / H)));
+  const int factor = s.query_block / 64, prefix_stages = rec::prefix_stages(s);
+  const dim3 rows((R + kRowWarps - 1) / kRowWarps, H);
+  hist_kernel<<<dim3(chunks, H, 2), kHistThreads, kHalfBins * 4, st>>>(prob, items, chunks, sc.hist);
+  threshold_kernel<<<H, 1024, 0, st>>>(sc.hist, nullptr, sc.thr, 8, 0, n16, n16 + n8, n16 + n8 + n4);
+  rowstat_kernel<<<rows, kRowWarps * 32, 0, st>>>(prob, R, sc.thr, sc.stat);
+  headscan_kernel<<<H, 1024, 0, st>>>(R, sc.thr, sc.stat, factor, prefix_stages, prefix_phase, ordered,
+                                      row_offset, row_counts);
+  return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
 }
 
 }  // namespace
@@ -1244,33 +1354,14 @@ extern "C" int anemoi_sm100_route(const anemoi_sm100_shape* shape, const void* p
   if (R > 65535 || items * H >= (1ll << 40)) return ANEMOI_SM100_ELIMIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (fused_fits(H, R))
-    return launch_fused<false, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids,
+    return launch_fused<kLists, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids,
                                list_capacity, nullptr, nullptr, st);
   RouteScratch sc;
-  sc.hist = static_cast<int*>(scratch);
-  sc.thr = sc.hist + (int64_t)H * kBins;
-  sc.stat = sc.thr + (int64_t)H * 8;
-  if (cudaMemsetAsync(sc.hist, 0, (size_t)H * kBins * 4, st) != cudaSuccess)
-    return ANEMOI_SM100_ELAUNCH;
-  const unsigned short* prob = static_cast<const unsigned short*>(probability);
-  // Function attributes belong to a device: the opt-in is made at every call (a cheap host-side
-  // driver call), so a process that routes on several GPUs, or from several host threads,
-  // never launches the kernel without the opt-in for its dynamic shared memory.
-  if (cudaFuncSetAttribute(hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHalfBins * 4) !=
-      cudaSuccess)
-    return ANEMOI_SM100_ELAUNCH;
-  // about two waves of histogram CTAs per key-range half, each with at least 8192 items
-  const int chunks = (int)max((int64_t)1, min(min((int64_t)16, items / 8192), (int64_t)((296 + H / 2) / H)));
-  const int factor = shape->query_block / 64, prefix_stages = rec::prefix_stages(*shape);
-  const dim3 rows((R + kRowWarps - 1) / kRowWarps, H);
-  hist_kernel<<<dim3(chunks, H, 2), kHistThreads, kHalfBins * 4, st>>>(prob, items, chunks, sc.hist);
-  threshold_kernel<<<H, 1024, 0, st>>>(sc.hist, nullptr, sc.thr, 8, 0, n16, n16 + n8, n16 + n8 + n4);
-  rowstat_kernel<<<rows, kRowWarps * 32, 0, st>>>(prob, R, sc.thr, sc.stat);
-  headscan_kernel<<<H, 1024, 0, st>>>(R, sc.thr, sc.stat, factor, prefix_stages, prefix_phase,
-                                      row_offset, row_counts);
-  emit_kernel<<<rows, kRowWarps * 32, 0, st>>>(prob, R, sc.thr, sc.stat, factor, prefix_stages,
-                                               prefix_phase, list_capacity, row_offset, row_counts,
-                                               stage_ids);
+  const int code = rank_rows(*shape, probability, n16, n8, n4, prefix_phase, true, scratch, row_offset, row_counts, sc, st);
+  if (code != ANEMOI_SM100_OK) return code;
+  emit_kernel<<<dim3((R + kRowWarps - 1) / kRowWarps, H), kRowWarps * 32, 0, st>>>(
+      static_cast<const unsigned short*>(probability), R, sc.thr, sc.stat, shape->query_block / 64,
+      rec::prefix_stages(*shape), prefix_phase, list_capacity, row_offset, row_counts, stage_ids);
   return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
 }
 
@@ -1289,8 +1380,28 @@ extern "C" int anemoi_sm100_route_pairs(const anemoi_sm100_shape* shape, const v
   if (list_capacity < anemoi_sm100_route_list_capacity(shape, n16, n8, n4, prefix_phase))
     return ANEMOI_SM100_EINVAL;
   if (!fused_fits(shape->heads, shape->video_blocks) || rec::stages(*shape) >= (1 << 30)) return ANEMOI_SM100_ELIMIT;
-  return launch_fused<true, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, nullptr,
+  return launch_fused<kNeighbours, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, nullptr,
                             list_capacity, pair_counts, pair_ids, static_cast<cudaStream_t>(stream));
+}
+
+int layer::route_bits(const anemoi_sm100_shape& s, const void* probability, int64_t n16, int64_t n8, int64_t n4,
+                      int prefix_phase, void* scratch, int32_t* row_offset, int32_t* row_counts, const PairBits& bits,
+                      int64_t capacity, cudaStream_t st) {
+  // (the conditions of draft_probability's map, route and pair_lists)
+  const int H = s.heads, R = s.video_blocks;
+  const int64_t items = (int64_t)R * R;
+  if (n16 < 0 || n8 < 0 || n4 < 0 || n16 + n8 + n4 > items || n16 + n8 + n4 <= 0) return ANEMOI_SM100_EINVAL;
+  if (prefix_phase < -1 || prefix_phase > 2) return ANEMOI_SM100_EINVAL;
+  if (capacity < anemoi_sm100_route_list_capacity(&s, n16, n8, n4, prefix_phase)) return ANEMOI_SM100_EINVAL;
+  if (fused_fits(H, R))
+    return launch_fused<kBits, 0>(s, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts,
+                                  nullptr, 0, nullptr, nullptr, st, bits);
+  RouteScratch sc;
+  const int code = rank_rows(s, probability, n16, n8, n4, prefix_phase, false, scratch, row_offset, row_counts, sc, st);
+  if (code != ANEMOI_SM100_OK) return code;
+  emit_bits_kernel<<<dim3((R + kRowWarps - 1) / kRowWarps, H), kRowWarps * 32, 0, st>>>(
+      static_cast<const unsigned short*>(probability), R, sc.thr, sc.stat, bits);
+  return cudaGetLastError() == cudaSuccess ? ANEMOI_SM100_OK : ANEMOI_SM100_ELAUNCH;
 }
 
 bool layer::drafts_in_routing(const anemoi_sm100_shape& s) {
@@ -1323,11 +1434,11 @@ int layer::draft_and_route(const anemoi_sm100_shape& s, const anemoi_sm100_opera
   d.maps = maxpool_weight != 0.0f && !most ? 2 : 1;
   d.weight = maxpool_weight;
   d.map = static_cast<unsigned short*>(probability);
-#define ANEMOI_LAUNCH(PAIRS, D)                                                                                       \
-  launch_fused<PAIRS, D>(s, d, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids, capacity, \
+#define ANEMOI_LAUNCH(LEAVES, D)                                                                                      \
+  launch_fused<LEAVES, D>(s, d, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids, capacity, \
                          pair_counts, pair_ids, st)
-  if (pairs) return s.head_dim == 64 ? ANEMOI_LAUNCH(true, 64) : ANEMOI_LAUNCH(true, 128);
-  return s.head_dim == 64 ? ANEMOI_LAUNCH(false, 64) : ANEMOI_LAUNCH(false, 128);
+  if (pairs) return s.head_dim == 64 ? ANEMOI_LAUNCH(kNeighbours, 64) : ANEMOI_LAUNCH(kNeighbours, 128);
+  return s.head_dim == 64 ? ANEMOI_LAUNCH(kLists, 64) : ANEMOI_LAUNCH(kLists, 128);
 #undef ANEMOI_LAUNCH
 }
 

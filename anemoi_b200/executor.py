@@ -339,8 +339,10 @@ class _Plan:
         # kernels per call: preparation (with V's maxima), draft, routing (and pair lists), attention, prefix rows
         self.launches = 3 + lib.anemoi_sm100_prepare_kernels(C.byref(shape)) + int(prefix_tokens > 0)
         self.launches -= lib.anemoi_sm100_drafts_in_routing(C.byref(shape))
+        matched = lib.anemoi_sm100_matches_pairs(self.ref)
+        self.launches += matched
         if not lib.anemoi_sm100_routes_in_one_kernel(C.byref(shape)):
-            self.launches += 4 + 2 * int(pair_q64 and query_block == 64)
+            self.launches += 4 + 2 * int(pair_q64 and query_block == 64 and not matched)
         self.call = lib.anemoi_sm100_layer
 
 

@@ -112,6 +112,7 @@ def library() -> C.CDLL:
         "anemoi_sm100_drafts_in_routing": (C.c_int, [SP]),
         "anemoi_sm100_prepare_kernels": (C.c_int, [SP]),
         "anemoi_sm100_layer_workspace_bytes": (I64, [C.POINTER(LayerPlan)]),
+        "anemoi_sm100_matches_pairs": (C.c_int, [C.POINTER(LayerPlan)]),
         "anemoi_sm100_layer": (C.c_int, [C.POINTER(LayerPlan), P, P, P, C.POINTER(I64), C.POINTER(F), P, I64, C.c_int,
                                          P, P, I64, P, P]),
         "anemoi_sm100_copy_rows": (C.c_int, [P, I64, P, I64, I64, I64, I32, P]),
@@ -155,7 +156,7 @@ EXPORTED = (
     "anemoi_sm100_route_static_max_bytes", "anemoi_sm100_attention",
     "anemoi_sm100_attention_pairs", "anemoi_sm100_pair_lists", "anemoi_sm100_route_pairs",
     "anemoi_sm100_layer", "anemoi_sm100_layer_workspace_bytes", "anemoi_sm100_routes_in_one_kernel",
-    "anemoi_sm100_drafts_in_routing", "anemoi_sm100_prepare_kernels",
+    "anemoi_sm100_drafts_in_routing", "anemoi_sm100_matches_pairs", "anemoi_sm100_prepare_kernels",
     "anemoi_sm100_route_anchored", "anemoi_sm100_route_anchored_scratch_bytes",
     "anemoi_sm100_prefix_attention", "anemoi_sm100_assemble", "anemoi_sm100_pack_qkv",
     "anemoi_sm100_merge_heads", "anemoi_sm100_pack_qkv_heads", "anemoi_sm100_merge_heads_into",

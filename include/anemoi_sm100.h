@@ -269,6 +269,9 @@ typedef struct anemoi_sm100_layer_plan {
   float maxpool_weight;
 } anemoi_sm100_layer_plan;
 
+/* 1 if the plan's Q64 blocks are paired by what their lists share (a launch for the choice) rather than by
+ * index, 0 if not. */
+int anemoi_sm100_matches_pairs(const anemoi_sm100_layer_plan* plan);
 int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan);
 /*   strides          as for anemoi_sm100_prepare
  *   nvfp4_scales     q, k, v tensor-level scales of this call, or null for the plan's
