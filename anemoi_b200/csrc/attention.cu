@@ -129,6 +129,7 @@ struct AttnParams {
   int out_rows;      // rows per head in `out`
   int ring_bytes;    // key/value ring; re-partitioned into equal slots at every phase
   int q_region;      // bytes
+  int turn;          // a head's lists before this place in the order start shortest first
 };
 
 // Entry g % kRing of a ring belongs to stage g, in phase g / kRing of the barrier.  Stage
@@ -149,6 +150,9 @@ struct Shared {
   uint64_t qk_done;    // unwinding only
   WaitContext wc;
   int cnt[3], first_of[3];  // the tile's stages per phase, where each phase starts inside the list
+  // which tile it is: read by the roles where they need it, or kept in registers from the start (kReread)
+  volatile int head, block[2], tile_blocks;
+  const int32_t* volatile list;
   uint32_t tmem_base;
   // per stage and query block of the tile: score scale, real keys (negative: not a stage of this block)
   float2 meta[kRing][2];
@@ -583,17 +587,23 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int kFirst = CELLS == kAny ? 0 : CELLS, kLast = CELLS == kAny ? 2 : CELLS;
   constexpr int QB = kQ64 ? 64 : 128;
-  const int head = blockIdx.y;
+  // Kernels of one cell spill less (and are 1-5 % quicker) if the roles read again from shared memory which tile they
+  // work on; those of any mix, and the ones with registers to spare, do not (4-12 % slower).
+  constexpr bool kReread = CELLS != kAny && (kQ64 || Regs<D, CELLS>::kWide);
+  // CTAs start in the order x, y, z: the longest lists of a few heads, the second ones, ..., then the next few heads
+  const int head = blockIdx.z * gridDim.x + blockIdx.x;
+  if (head >= p.s.heads) return;
+  const int place = (int)blockIdx.y < p.turn ? p.turn - 1 - (int)blockIdx.y : (int)blockIdx.y;
   layer::grid_dependency_wait();
   // launch order of the head's query blocks (longest list first) as written by the routing
   // stage; 0 = no order given
-  int tile = blockIdx.x;
+  int tile = place;
   const bool table = kQ64 && p.pair_table != nullptr, pairs = table || (kQ64 && p.pair_counts != nullptr);
   const int pair_tiles = (p.s.video_blocks + 1) / 2;
   if (!p.dense_prefix && !table) {
     const int ordered =
-        pairs ? p.pair_counts[((int64_t)head * pair_tiles + blockIdx.x) * 4 + 3]
-              : p.row_counts[((int64_t)head * p.s.video_blocks + blockIdx.x) * 4 + 3];
+        pairs ? p.pair_counts[((int64_t)head * pair_tiles + place) * 4 + 3]
+              : p.row_counts[((int64_t)head * p.s.video_blocks + place) * 4 + 3];
     if (ordered > 0) tile = ordered - 1;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -668,6 +678,11 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       b->wc.abort = 0;
       b->wc.status = p.status;
       b->wc.limit_ns = p.wait_ns;
+      b->head = head;
+      b->block[0] = block0;
+      b->block[1] = block1;
+      b->tile_blocks = tile_blocks;
+      b->list = list;
       // phase c of a union of neighbours sits where the two blocks' phases before it would end
       const bool apart = pairs && !table;
       const int32_t* ra = apart ? p.row_counts + ((int64_t)head * p.s.video_blocks + block0) * 4 : nullptr;
@@ -693,7 +708,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   tc_fence_after_sync();
   const uint32_t tmem = b->tmem_base;
 
-  const float* vscale = p.o.v_e4m3_scale ? p.o.v_e4m3_scale + (int64_t)head * D : nullptr;
+  const float* vscale_kept = p.o.v_e4m3_scale ? p.o.v_e4m3_scale + (int64_t)head * D : nullptr;
   const float nv_dom = p.s.v_global_scale * (1.0f / (6.0f * 448.0f));
 
   // Register counts move between the warpgroups; all four warps of a warpgroup execute the same
@@ -704,10 +719,13 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       // =============================== loader ===============================
       // The whole warp walks the list with uniform control flow; one lane issues.
       const uint32_t lead = lane == 0;
-      const int q_index_fp = head * p.s.video_blocks + block0;  // q_fp16 / q_nvfp4 record
+      const int head_at = kReread ? b->head : head, first_block = kReread ? b->block[0] : block0;
+      const int blocks = kReread ? b->tile_blocks : tile_blocks;
+      const int32_t* list_at = kReread ? b->list : list;
+      const int q_index_fp = head_at * p.s.video_blocks + first_block;  // q_fp16 / q_nvfp4 record
       const int64_t q_index_i8 =
-          (int64_t)head * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks : 0) + block0;
-      const int step = block1 - block0;  // from a pair's first record to its second
+          (int64_t)head_at * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks : 0) + first_block;
+      const int step = (kReread ? b->block[1] : block1) - first_block;  // from a pair's first record to its second
       const float sigma = (D == 64 ? 0.125f : 0.08838834764831845f) * 1.4426950408889634f;
       int phase_ord = 0, g = 0, v_fills = 0, moves = 0;
 #pragma unroll 1
@@ -721,7 +739,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             cell == kNv ? static_cast<const uint8_t*>(p.o.q_nvfp4) + (int64_t)q_index_fp * qbytes
             : cell == kI8 ? static_cast<const uint8_t*>(p.o.q_int8) + q_index_i8 * qbytes
                           : static_cast<const uint8_t*>(p.o.q_fp16) + (int64_t)q_index_fp * qbytes;
-        mbar_arrive_expect_tx(&b->q_full, qbytes * tile_blocks, lead);
+        mbar_arrive_expect_tx(&b->q_full, qbytes * blocks, lead);
         if (cell == kNv && kQ64) {
           // codes fill the first half of the 128-row tile; scale blocks follow the full tile.
           // A pair's second record: codes into the second half of the tile, scale blocks behind
@@ -729,7 +747,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           const int codes = QB * D / 2;
           bulk_g2s(q_smem, qsrc, codes, &b->q_full, lead);
           bulk_g2s(q_smem + 128 * D / 2, qsrc + codes, qbytes - codes, &b->q_full, lead);
-          if (tile_blocks == 2) {
+          if (blocks == 2) {
             const uint8_t* second = qsrc + (int64_t)step * qbytes;
             bulk_g2s(q_smem + codes, second, codes, &b->q_full, lead);
             bulk_g2s(q_smem + 128 * D / 2 + (qbytes - codes), second + codes, qbytes - codes, &b->q_full, lead);
@@ -737,14 +755,14 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         } else {
           // two records of 64 rows make a 128-row tile
           bulk_g2s(q_smem, qsrc, qbytes, &b->q_full, lead);
-          if (kQ64 && tile_blocks == 2) bulk_g2s(q_smem + qbytes, qsrc + (int64_t)step * qbytes, qbytes, &b->q_full, lead);
+          if (kQ64 && blocks == 2) bulk_g2s(q_smem + qbytes, qsrc + (int64_t)step * qbytes, qbytes, &b->q_full, lead);
         }
         const int kvbytes = record_bytes(D, cell), kbytes = k_bytes(D, cell), rest = rest_offset(D, cell);
         const uint8_t* kvbase =
             (cell == kNv ? static_cast<const uint8_t*>(p.o.kv_nvfp4)
              : cell == kI8 ? static_cast<const uint8_t*>(p.o.kv_int8)
                            : static_cast<const uint8_t*>(p.o.kv_fp16)) +
-            (int64_t)head * p.stages * kvbytes;
+            (int64_t)head_at * p.stages * kvbytes;
         const int first = b->first_of[cell];
         // The ring is cut into equal slots of this phase's size; the slots of the previous phase
         // must all be released before the new geometry is written (PVs complete in stage order).
@@ -755,8 +773,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         const float* kscale = nullptr;
         if (cell == kI8) {
           q_scale[0] = p.o.q_int8_scale[q_index_i8];
-          if (tile_blocks == 2) q_scale[1] = p.o.q_int8_scale[q_index_i8 + step];
-          kscale = p.o.k_int8_scale + (int64_t)head * p.stages;
+          if (blocks == 2) q_scale[1] = p.o.q_int8_scale[q_index_i8 + step];
+          kscale = p.o.k_int8_scale + (int64_t)head_at * p.stages;
         }
         const float base = cell == kNv ? sigma * p.s.q_global_scale * p.s.k_global_scale : sigma;
         // list entries, 32 at a time, one per lane, with their metadata
@@ -772,7 +790,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           if ((i & 31) == 0 && i < n) {
             const int at = i + lane;
             int entry = 0;
-            if (at < n) entry = list != nullptr ? list[first + at] : at;
+            if (at < n) entry = list_at != nullptr ? list_at[first + at] : at;
             stage_l = entry & 0x3fffffff;
             const int valid = p.valid_k[stage_l];
             meta_l[0].y = __int_as_float(!pairs || ((entry >> 30) & 1) ? valid : -1);
@@ -854,7 +872,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         const uint64_t base = k_desc(D, cell, split_kv(D, cell) ? smem_u32(smem) : ring_addr);
         const uint64_t q_desc = k_desc(D, kNv, q_addr);
         if (cell == kNv) {
-          if (tile_blocks == 2) {
+          if ((kReread ? b->tile_blocks : tile_blocks) == 2) {
             // Scale bytes of rows 0-63 sit in the low eight bytes of every 16-byte chunk, those of
             // rows 64-127 in the high eight.  Both records hold their 64 rows in the low halves:
             // the second record's move up into the first record's empty high halves.
@@ -971,6 +989,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       if (change) {
         // per-channel factor that moves O from the previous phase's domain into this one's
         asm volatile("bar.sync 5, 128;" ::: "memory");
+        const float* vscale = kReread ? p.o.v_e4m3_scale + (int64_t)b->head * D : vscale_kept;
         if (row < D) {
           const float from = prev_cell == kNv ? nv_dom
                                               : (prev_cell == kI8 ? vscale[row] * 0.0022326917f : 1.0f);
@@ -1027,8 +1046,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     SoftmaxWalk w{0u, 0.0f, 1.0f, 0.0f};
     int g = 0, last_cell = kFirst;
-    const bool live_warp = !kQ64 || (warp & 3) * 32 < QB * tile_blocks;
-    const int my_block = kQ64 && (warp & 3) * 32 >= QB && tile_blocks == 2 ? 1 : 0;  // which block of a pair
+    const int blocks = kReread ? b->tile_blocks : tile_blocks;
+    const bool live_warp = !kQ64 || (warp & 3) * 32 < QB * blocks;
+    const int my_block = kQ64 && (warp & 3) * 32 >= QB && blocks == 2 ? 1 : 0;  // which block of a pair
     if (kFirst == kNv && b->cnt[kNv] > 0 && parity == 0) {
       tmem_st4(tmem_row + kColSfaP, 0x7e7e7e7eu);  // constant 448 block scale of P
       tmem_wait_st();
@@ -1055,14 +1075,18 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     // ---- epilogue: O_true / d -> fp16, packed row order; each warpgroup writes half the channels ----
     // packed rows: this tile's place; token rows: the row's token, in the caller's type (looked up under the last PV)
     uint16_t* dst = nullptr;
-    if (p.tokens == nullptr) {
-      if (row < QB * tile_blocks)
+    const int head_at = kReread ? b->head : head;
+    const int first_block = kReread ? b->block[0] : block0, second_block = kReread ? b->block[1] : block1;
+    if (row < QB * (kReread ? b->tile_blocks : tile_blocks)) {
+      if (p.tokens == nullptr) {
         dst = reinterpret_cast<uint16_t*>(p.out) +
-              ((int64_t)head * p.out_rows + (kQ64 && row >= QB ? block1 * QB + row - QB : block0 * QB + row)) * D;
-    } else if (row < QB * tile_blocks) {
-      const int64_t at = token_offset<D, kQ64>(p, head, block0, block1, row);
-      if (at >= 0) dst = static_cast<uint16_t*>(p.tokens) + at;
+              ((int64_t)head_at * p.out_rows + (kQ64 && row >= QB ? second_block * QB + row - QB : first_block * QB + row)) * D;
+      } else {
+        const int64_t at = token_offset<D, kQ64>(p, head_at, first_block, second_block, row);
+        if (at >= 0) dst = static_cast<uint16_t*>(p.tokens) + at;
+      }
     }
+    const float* vscale = kReread ? p.o.v_e4m3_scale + (int64_t)head_at * D : vscale_kept;
     wait(&b->wc, &b->all_done, 0, 7);
     // d(G-1) from d(G-3) and the last two stages' (alpha, sum), which the two groups hold; every
     // other use of rec is over
@@ -1112,13 +1136,37 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   if (warp == kPvWarp) tmem_dealloc(tmem, kTmemCols);
 }
 
+// Heads whose query tiles start in turns, longest lists first: as many as keep keys and values of up to 48 MB in use (they
+// stay in L2).  With heads one after the other a call of a few waves of CTAs ends with the last head's lists, whichever they
+// are; lists of different lengths gain up to 13 %, equal ones nothing.  One after the other / in turns, us: NVFP4 D = 64,
+// Q64, 9 heads x 14,161 tokens 201.5 / 177.6, Q128, 8 x 9,360 106.6 / 97.1; INT8 + NVFP4 D = 128, 11 x 9,464 450 / 407; INT8
+// Q128, 33 x 2,790 95.9 / 91.8.  24 MB gain less (11 x 9,464 424), past L2 it turns (10 MB per head, 56 x 38,247 tokens INT8,
+// with 2, 4, 6, 16 and 56 heads at a time 9.66, 9.82, 9.92, 10.32 and 10.69 ms).  Calls of less than a CTA per SM lose: 70 / 71.
+// Calls of one to two CTAs per SM: the lists of the first 148 CTAs start shortest first, so that the SM of the shortest gets
+// the longest of the others (4 x 6,664 tokens NVFP4 D = 64, 208 CTAs, 60.4 / 54.9, without the turn 55.3; 1 x 4,032 + 77, 264
+// CTAs 78.0 / 77.5 and 79.5).
+constexpr int kSms = 148;
+constexpr int64_t kHeadsBytes = 48 << 20;
+int heads_at_a_time(const AttnParams& p) {
+  if (p.dense_prefix) return 1;
+  const int64_t bytes = (p.s.has_nvfp4 ? rec::kv_nvfp4_bytes(p.s.head_dim) : 0) +
+                        (p.s.has_int8 ? rec::kv_int8_bytes(p.s.head_dim) : 0) +
+                        (p.s.has_fp16 ? rec::kv_fp16_bytes(p.s.head_dim) : 0);
+  return (int)max((int64_t)1, min((int64_t)p.s.heads, kHeadsBytes / (bytes * p.stages)));
+}
+
 template <int D, int CELLS, bool kQ64>
-int launch_kernel(const AttnParams& p, int tiles, size_t smem, cudaStream_t st) {
+int launch_kernel(AttnParams& p, int tiles, size_t smem, cudaStream_t st) {
   auto kernel = attention_kernel<D, CELLS, kQ64>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
-  return layer::launch(kernel, dim3(tiles, p.s.heads), dim3(kThreads), smem, st, p) == cudaSuccess
+  if (tiles > 65535) return ANEMOI_SM100_ELIMIT;
+  const int64_t ctas = (int64_t)tiles * p.s.heads;
+  const int most = p.dense_prefix || ctas <= kSms ? 1 : heads_at_a_time(p), groups = (p.s.heads + most - 1) / most;
+  const dim3 grid((p.s.heads + groups - 1) / groups, tiles, groups);
+  p.turn = !p.dense_prefix && groups == 1 && ctas > kSms && ctas <= 2 * kSms ? kSms / p.s.heads : 0;
+  return layer::launch(kernel, grid, dim3(kThreads), smem, st, p) == cudaSuccess
              ? ANEMOI_SM100_OK
              : ANEMOI_SM100_ELAUNCH;
 }
