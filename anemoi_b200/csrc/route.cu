@@ -541,8 +541,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) anchor_emit_kernel(
 // histogram and, for short maps, its dozen barriers.  Those are why the scans of the three boundaries share
 // theirs, the CTAs of a cluster exchange their sums once, a cluster of one uses the CTA's barrier, block sums
 // go by exchanges of halves and only warps that have rows scan.  Alone, in several launches (five, seven with
-// pairs) / in this one, us: 8 heads x 33 blocks 34 / 9.0, 8 x 64 34 / 10.5, 56 x 273 75 / 46, 56 x 672 235 / 190; with pairs
-// 4 x 16 40 / 6.8, 56 x 592 277 / 122.
+// pairs) / in this one, us: 56 x 273 75 / 46, 56 x 672 235 / 190; with pairs 56 x 592 277 / 122.
 constexpr int kFusedThreads = 1024;
 constexpr int kFusedWarps = kFusedThreads / 32;
 
@@ -557,7 +556,7 @@ struct FusedShared {
 __host__ __device__ inline size_t fused_smem() { return (size_t)kBins * 4 + sizeof(FusedShared); }
 
 // CTAs per head: as many as keep every head on an SM of its own at once, down to 64 rows each (two per
-// warp; 8 heads x 33 blocks take 9.0 us in one CTA each, 10.1 in two).  Clusters do not cross GPCs, so 15 of eight fit
+// warp).  Clusters do not cross GPCs, so 15 of eight fit
 // at a time and 33 of four.  672 blocks, us: 15 heads in clusters of eight 59, of four 105; 16 heads 115, 105; 33 heads
 // in clusters of four 105, of two 188; 37 heads 208, 188; 66 heads in clusters of two 191, of one 359.
 inline int fused_ctas(int H, int R) {
@@ -625,19 +624,12 @@ __device__ __forceinline__ void fused_exclusive(int (&v)[N], int4* warp_sum, int
 
 constexpr int kAhead = 8;  // 32-column pieces of a row whose keys are loaded before the first is looked at
 
-// A map entry; `kOwn`: of a map that this CTA has written itself (not through the read-only path).
-template <bool kOwn, typename T>
-__device__ __forceinline__ T map_entry(const T* at) {
-  return kOwn ? *at : __ldg(at);
-}
-
 // The keys of columns [j0, j0 + 32 * kAhead) of a row, -2 past its end.
-template <bool kOwn>
 __device__ __forceinline__ void fused_keys(const unsigned short* src, int j0, int R, int (&key)[kAhead]) {
 #pragma unroll
   for (int u = 0; u < kAhead; ++u) {
     const int j = j0 + u * 32 + (threadIdx.x & 31);
-    key[u] = j < R ? (map_entry<kOwn>(src + j) & 0x7fff) : -2;
+    key[u] = j < R ? (__ldg(src + j) & 0x7fff) : -2;
   }
 }
 
@@ -659,13 +651,10 @@ __device__ __forceinline__ int fused_code(int key, const int (&key_b)[3], const 
   return c;
 }
 
-// ---- the draft map in the same kernel: up to 32 blocks per head, one CTA -------------------------
-// The arithmetic of draft.cu with a row per warp and a column per lane, the pools in the histogram's space.
-// Up to there a head's map is 1-2 us of work, and a launch of its own costs 2.5 us on the host and as much on the
-// device.  Calls of INT8 without a prefix, us, in two launches / in one: D = 64 1 head x 8 blocks 22.3 / 20.4, 8 x 32 48.1 /
-// 47.1, 24 x 24, two maps 43.3 / 40.5; D = 128 1 x 32 34.2 / 34.3, 8 x 16, two maps 34.6 / 28.9, 56 x 32, two maps, Q128 222.3 /
-// 218.4.  In an earlier form, with prefix tiles on the side stream the one kernel lost (32 blocks x 8 heads and 77 tokens
-// 77.5 / 86.7), and so it did with two rows per warp and two columns per lane (51 blocks 32.4 / 36.2).
+// ---- the draft map in the routing kernel: up to 32 blocks per head ---------------------------------
+// The arithmetic of draft.cu with a column per lane.  Up to there a head's map is 1-2 us of work, and a launch of its own costs
+// 2.5 us on the host and as much on the device (INT8 without a prefix, in two launches / in one, D = 64, 1 head x 8 blocks
+// 22.3 / 20.4, 24 x 24, two maps 43.3 / 40.5, D = 128, 8 x 16, two maps 34.6 / 28.9).
 constexpr int kDraftBlocks = 32;
 struct DraftPools {
   const __half* q[2];  // mean, max
@@ -675,14 +664,15 @@ struct DraftPools {
   unsigned short* map;
 };
 
-template <int D>
-__device__ __forceinline__ void draft_rows(const DraftPools& d, int head, int R, uint32_t* smem) {
-  uint32_t* kc = smem;                                                   // [2][D / 2][32], two channels a word
-  float* qs = reinterpret_cast<float*>(smem + 2 * D / 2 * kDraftBlocks);  // [2][32][D]
+// The map's entries of kRows neighbouring rows per warp, a column per lane.
+template <int D, int kRows, int kThreads>
+__device__ __forceinline__ void draft_rows(const DraftPools& d, int head, int R, uint32_t* smem, float (&out)[kRows]) {
+  uint32_t* kc = smem;                                                         // [maps][D / 2][32], two channels a word
+  float* qs = reinterpret_cast<float*>(smem + d.maps * D / 2 * kDraftBlocks);  // [maps][32][D]
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
     if (m >= d.maps) break;
-    for (int idx = threadIdx.x; idx < kDraftBlocks * (D / 8); idx += kFusedThreads) {
+    for (int idx = threadIdx.x; idx < kDraftBlocks * (D / 8); idx += kThreads) {
       const int col = idx % kDraftBlocks, c8 = idx / kDraftBlocks;
       uint4 v = make_uint4(0, 0, 0, 0);
       if (col < R) v = __ldg(reinterpret_cast<const uint4*>(d.k[m] + ((int64_t)head * R + col) * D) + c8);
@@ -692,32 +682,42 @@ __device__ __forceinline__ void draft_rows(const DraftPools& d, int head, int R,
       dst[2 * kDraftBlocks] = v.z;
       dst[3 * kDraftBlocks] = v.w;
     }
-    for (int idx = threadIdx.x; idx < R * (D / 2); idx += kFusedThreads)
+    for (int idx = threadIdx.x; idx < R * (D / 2); idx += kThreads)
       reinterpret_cast<float2*>(qs + m * kDraftBlocks * D)[idx] =
           __half22float2(__ldg(reinterpret_cast<const __half2*>(d.q[m] + (int64_t)head * R * D) + idx));
   }
   __syncthreads();
-  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r0 = (threadIdx.x >> 5) * kRows, lane = threadIdx.x & 31;
   const bool in = lane < R;
-  if (r < R) {
-    float p[2];
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      if (m >= d.maps) break;
-      const float4* q = reinterpret_cast<const float4*>(qs + (m * kDraftBlocks + r) * D);
-      const uint32_t* k = kc + m * (D / 2) * kDraftBlocks + lane;
-      float acc = 0.0f;
+  for (int r = 0; r < kRows; ++r) out[r] = 0.0f;
+  if (r0 >= R) return;
+  float p[2][kRows];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    if (m >= d.maps) break;
+    // (rows past the map are read from rows of it)
+    const float4* q[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) q[r] = reinterpret_cast<const float4*>(qs + (m * kDraftBlocks + min(r0 + r, R - 1)) * D);
+    const uint32_t* k = kc + m * (D / 2) * kDraftBlocks + lane;
+    float acc[kRows] = {};
 #pragma unroll 8
-      for (int c4 = 0; c4 < D / 4; ++c4) {
-        const float4 qv = q[c4];
-        const uint32_t w0 = k[2 * c4 * kDraftBlocks], w1 = k[(2 * c4 + 1) * kDraftBlocks];
-        const float2 k0 = __half22float2(*reinterpret_cast<const __half2*>(&w0));
-        const float2 k1 = __half22float2(*reinterpret_cast<const __half2*>(&w1));
-        acc = __fmaf_rn(qv.y, k0.y, __fmaf_rn(qv.x, k0.x, acc));
-        acc = __fmaf_rn(qv.w, k1.y, __fmaf_rn(qv.z, k1.x, acc));
+    for (int c4 = 0; c4 < D / 4; ++c4) {
+      const uint32_t w0 = k[2 * c4 * kDraftBlocks], w1 = k[(2 * c4 + 1) * kDraftBlocks];
+      const float2 k0 = __half22float2(*reinterpret_cast<const __half2*>(&w0));
+      const float2 k1 = __half22float2(*reinterpret_cast<const __half2*>(&w1));
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        const float4 qv = q[r][c4];
+        acc[r] = __fmaf_rn(qv.y, k0.y, __fmaf_rn(qv.x, k0.x, acc[r]));
+        acc[r] = __fmaf_rn(qv.w, k1.y, __fmaf_rn(qv.z, k1.x, acc[r]));
       }
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
       const float logit =
-          __half2float(__float2half_rn(__fmul_rn(acc, D == 64 ? 0.125f : __int_as_float(0x3db504f3))));
+          __half2float(__float2half_rn(__fmul_rn(acc[r], D == 64 ? 0.125f : __int_as_float(0x3db504f3))));
       float mx = in ? fmaxf(-INFINITY, logit) : -INFINITY;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
@@ -725,14 +725,13 @@ __device__ __forceinline__ void draft_rows(const DraftPools& d, int head, int R,
       float sum = in ? e : 0.0f;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, off));
-      p[m] = __fmul_rn(e, __fdiv_rn(1.0f, sum));
+      p[m][r] = __fmul_rn(e, __fdiv_rn(1.0f, sum));
     }
-    const float v = d.maps == 1
-                        ? p[0]
-                        : __fadd_rn(__fmul_rn(__fsub_rn(1.0f, d.weight), p[0]), __fmul_rn(d.weight, p[1]));
-    if (in) d.map[((int64_t)head * R + r) * R + lane] = __half_as_ushort(__float2half_rn(v));
   }
-  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kRows; ++r)
+    out[r] = d.maps == 1 ? p[0][r]
+                         : __fadd_rn(__fmul_rn(__fsub_rn(1.0f, d.weight), p[0][r]), __fmul_rn(d.weight, p[1][r]));
 }
 
 // What the kernel leaves: the rows' lists, the union lists of neighbouring Q64 blocks, or a bit per (row, phase,
@@ -765,10 +764,9 @@ __device__ __forceinline__ RowBits row_bits(const layer::PairBits& bits, int hea
   return b;
 }
 
-// kDraft: 0, or the head dimension of the pools that the map is formed from first.
-template <int kLeaves, int kDraft>
+template <int kLeaves>
 __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
-    const DraftPools draft, const unsigned short* prob, int R, int rows_per, int b0, int b1, int b2, int factor, int prefix_stages,
+    const unsigned short* prob, int R, int rows_per, int b0, int b1, int b2, int factor, int prefix_stages,
     int prefix_phase, int64_t capacity, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids,
     int32_t* pair_counts, int32_t* pair_ids, const layer::PairBits bits) {
   constexpr bool kPairs = kLeaves == kNeighbours;
@@ -791,31 +789,23 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   const unsigned short* map = prob + (int64_t)head * R * R;
 
   // ---- histogram of this CTA's rows ----
-  constexpr bool kOwn = kDraft != 0;
-  if constexpr (kOwn) {
-    layer::grid_dependency_wait();
-    layer::grid_dependency_trigger();
-    draft_rows<kDraft>(draft, head, R, reinterpret_cast<uint32_t*>(hist));
-  }
   for (int i = threadIdx.x; i < kBins / 4; i += kFusedThreads) reinterpret_cast<int4*>(hist)[i] = make_int4(0, 0, 0, 0);
   __syncthreads();
-  if constexpr (!kOwn) {
-    layer::grid_dependency_wait();
-    layer::grid_dependency_trigger();
-  }
+  layer::grid_dependency_wait();
+  layer::grid_dependency_trigger();
   {
     const unsigned short* src = map + (int64_t)r0 * R;
     const int items = mine * R;
     const int head_items = min(items, (int)((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 2);
     const int vecs = (items - head_items) / 8;
     const uint4* v = reinterpret_cast<const uint4*>(src + head_items);
-    if ((int)threadIdx.x < head_items) atomicAdd(&hist[map_entry<kOwn>(src + threadIdx.x) & 0x7fff], 1);
+    if ((int)threadIdx.x < head_items) atomicAdd(&hist[__ldg(src + threadIdx.x) & 0x7fff], 1);
     const int tail = head_items + vecs * 8;
     if (tail + (int)threadIdx.x < items && threadIdx.x < 8) 
-      atomicAdd(&hist[map_entry<kOwn>(src + tail + threadIdx.x) & 0x7fff], 1);
+      atomicAdd(&hist[__ldg(src + tail + threadIdx.x) & 0x7fff], 1);
 #pragma unroll 2
     for (int i = threadIdx.x; i < vecs; i += kFusedThreads) {
-      const uint4 q = map_entry<kOwn>(v + i);
+      const uint4 q = __ldg(v + i);
       const unsigned w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -903,7 +893,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
     int n[3] = {0, 0, 0};  // keys above | equal << 16 (a row has 4,096 at most)
     for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
       int key[kAhead];
-      fused_keys<kOwn>(src, j0, R, key);
+      fused_keys(src, j0, R, key);
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
         if (j0 + u * 32 >= R) break;
@@ -978,7 +968,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       const unsigned short* src = map + (int64_t)(r0 + i) * R;
       for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
         int key[kAhead];
-        fused_keys<kOwn>(src, j0, R, key);
+        fused_keys(src, j0, R, key);
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
           if (j0 + u * 32 >= R) break;
@@ -1009,7 +999,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       const unsigned short* src = map + (int64_t)(r0 + i) * R;
       for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
         int key[kAhead];
-        fused_keys<kOwn>(src, j0, R, key);
+        fused_keys(src, j0, R, key);
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
           if (j0 + u * 32 >= R) break;
@@ -1055,8 +1045,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       const unsigned short* src_b = map + (int64_t)(r0 + bb) * R;
       for (int j0 = 0; j0 < R; j0 += 32 * kAhead) {
         int ka[kAhead], kb[kAhead];
-        fused_keys<kOwn>(src_a, j0, R, ka);
-        fused_keys<kOwn>(src_b, j0, has_b ? R : 0, kb);
+        fused_keys(src_a, j0, R, ka);
+        fused_keys(src_b, j0, has_b ? R : 0, kb);
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
           if (j0 + u * 32 >= R) break;
@@ -1103,22 +1093,339 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
   if (ctas > 1) cluster.sync();  // no CTA leaves while another may still read its totals
 }
 
-template <int kLeaves, int kDraft>
-int launch_fused(const anemoi_sm100_shape& s, const DraftPools& draft, const void* probability, int64_t n16, int64_t n8, int64_t n4,
+template <int kLeaves>
+int launch_fused(const anemoi_sm100_shape& s, const void* probability, int64_t n16, int64_t n8, int64_t n4,
                  int prefix_phase, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids, int64_t capacity,
                  int32_t* pair_counts, int32_t* pair_ids, cudaStream_t st, const layer::PairBits& bits = {}) {
   const int H = s.heads, R = s.video_blocks, ctas = fused_ctas(H, R);
-  auto kernel = route_fused_kernel<kLeaves, kDraft>;
+  auto kernel = route_fused_kernel<kLeaves>;
   // Function attributes belong to a device: the opt-in is made at every call (a cheap host-side
   // driver call), so a process that routes on several GPUs, or from several host threads,
   // never launches the kernel without the opt-in for its dynamic shared memory.
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem()) != cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
   return layer::launch_cluster(kernel, dim3(ctas, H), dim3(ctas), dim3(kFusedThreads), fused_smem(), st,
-                               draft, static_cast<const unsigned short*>(probability), R, fused_rows(R, ctas), (int)n16,
+                               static_cast<const unsigned short*>(probability), R, fused_rows(R, ctas), (int)n16,
                                (int)(n16 + n8), (int)(n16 + n8 + n4), s.query_block / 64, rec::prefix_stages(s),
                                prefix_phase, capacity, row_offset, row_counts, stage_ids, pair_counts, pair_ids,
                                bits) == cudaSuccess
+             ? ANEMOI_SM100_OK
+             : ANEMOI_SM100_ELAUNCH;
+}
+
+// ---- short maps: up to 64 blocks per head -------------------------------------------------------
+// One CTA per head with the map's keys in registers: a lane has columns lane and lane + 32, a warp kCols * 2
+// neighbouring rows.  The kernel is a chain of latencies (and int operations run at half rate), so the
+// histogram is of 1,024 bins of 32 keys, resolved by a second one of the bins that hold the boundaries, rows
+// are counted by ballots, and every warp scans all rows for itself instead of waiting for one that does.  A CTA
+// leaves room for one of the prefix rows beside it, which the kernel above does not.
+// Whole calls, with the kernel above / with this one, us: 4 heads x 16 blocks INT8 D = 64 (with the map) 23.9 / 19.5,
+// 24 x 18 NVFP4 33.6 / 30.6, 2 x 12 and 288 tokens of prefix 37.0 / 32.9, 21 x 17 pairs 51.3 / 47.2, 1 x 42 three cells
+// 47.2 / 42.6, 11 x 44 FP16 35.4 / 31.5; 50 x 64 INT8 366 / 365.
+constexpr int kShortThreads = 512;
+constexpr int kShortWarps = kShortThreads / 32;
+constexpr int kShortBlocks = 64;
+
+struct ShortShared {
+  alignas(16) int bins[1024];
+  int fine[3][32];
+  int warp_sum[kShortWarps];
+  int hit[3], off[3];
+  int equal[3][kShortBlocks], above[3][kShortBlocks];
+  int unions[kShortBlocks / 2];
+};
+__host__ __device__ constexpr int draft_words(int D, int maps) {  // both pools of the map: halves, and floats
+  return maps * (D / 2 * kDraftBlocks + kDraftBlocks * D);
+}
+
+template <int kCols, bool kPairs, int kDraft>
+__global__ void __launch_bounds__(kShortThreads) route_short_kernel(
+    const DraftPools draft, const unsigned short* prob, int R, int b0, int b1, int b2, int factor, int prefix_stages,
+    int prefix_phase, int64_t capacity, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids,
+    int32_t* pair_counts, int32_t* pair_ids) {
+  static_assert(kDraft == 0 || kCols == 1, "the map is formed up to 32 blocks");
+  constexpr int kRows = 2 * kCols;  // of a warp
+  extern __shared__ __align__(16) uint32_t pools[];
+  __shared__ ShortShared sh;
+  const int head = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row0 = warp * kRows;
+  const unsigned lower = (1u << lane) - 1u;
+  for (int i = threadIdx.x; i < 1024; i += kShortThreads) sh.bins[i] = 0;
+  if (threadIdx.x < 96) sh.fine[threadIdx.x / 32][lane] = 0;
+  if (threadIdx.x < 3) sh.hit[threadIdx.x] = -1;
+  layer::grid_dependency_wait();
+  layer::grid_dependency_trigger();
+
+  // ---- keys, -2 past the map ----
+  int key[kRows][kCols];
+  if constexpr (kDraft != 0) {
+    float p[kRows];
+    draft_rows<kDraft, kRows, kShortThreads>(draft, head, R, pools, p);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const bool in = row0 + r < R && lane < R;
+      const unsigned short entry = __half_as_ushort(__float2half_rn(p[r]));
+      if (in) draft.map[((int64_t)head * R + row0 + r) * R + lane] = entry;
+      key[r][0] = in ? entry & 0x7fff : -2;
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        const int j = c * 32 + lane;
+        key[r][c] = row0 + r < R && j < R ? __ldg(prob + ((int64_t)head * R + row0 + r) * R + j) & 0x7fff : -2;
+      }
+    __syncthreads();  // the bins are empty
+  }
+  // ---- bins of 32 keys that hold the boundaries, then the keys ----
+#pragma unroll
+  for (int r = 0; r < kRows; ++r)
+#pragma unroll
+    for (int c = 0; c < kCols; ++c)
+      if (key[r][c] >= 0) atomicAdd(&sh.bins[key[r][c] >> 5], 1);
+  __syncthreads();
+  {
+    // thread t has bins 1023 - 2t and 1022 - 2t: keys in descending order
+    const int2 two = *reinterpret_cast<const int2*>(&sh.bins[1022 - 2 * threadIdx.x]);
+    int incl = two.x + two.y;
+    const int mine = incl;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += v;
+    }
+    if (lane == 31) sh.warp_sum[warp] = incl;
+    __syncthreads();
+    const int before = __reduce_add_sync(0xffffffffu, lane < warp ? sh.warp_sum[lane & (kShortWarps - 1)] : 0);
+    const int start[2] = {before + incl - mine, before + incl - mine + two.y}, count[2] = {two.y, two.x};
+    const int bound[3] = {b0, b1, b2};
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (start[h] <= bound[b] && bound[b] < start[h] + count[h]) {
+          sh.hit[b] = 1023 - 2 * (int)threadIdx.x - h;
+          sh.off[b] = bound[b] - start[h];
+        }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    const int bin = sh.hit[b];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int c = 0; c < kCols; ++c)
+        if (key[r][c] >= 0 && key[r][c] >> 5 == bin) atomicAdd(&sh.fine[b][key[r][c] & 31], 1);
+  }
+  __syncthreads();
+  int key_b[3], quota_b[3];
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    const int n = sh.fine[b][31 - lane], off = sh.off[b], bin = sh.hit[b];  // descending
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const int src = __ffs(__ballot_sync(0xffffffffu, n > 0 && incl - n <= off && off < incl)) - 1;
+    // (a boundary at or past the last item: every key lies above it)
+    key_b[b] = bin < 0 ? -1 : bin * 32 + 31 - src;
+    quota_b[b] = bin < 0 ? 0 : off - __shfl_sync(0xffffffffu, incl - n, src & 31);
+  }
+  // ---- per row: keys above and equal to each straddling key ----
+#pragma unroll
+  for (int r = 0; r < kRows; ++r)
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      int above = 0, equal = 0;
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        above += __popc(__ballot_sync(0xffffffffu, key[r][c] > key_b[b]));
+        equal += __popc(__ballot_sync(0xffffffffu, key[r][c] == key_b[b]));
+      }
+      if (lane == 0) {
+        sh.above[b][row0 + r] = above;
+        sh.equal[b][row0 + r] = equal;
+      }
+    }
+  __syncthreads();
+  // ---- scans over the rows, a lane per row of 32: position inside the straddling bins, stages, list offsets ----
+  const int p = prefix_phase >= 0 ? prefix_stages : 0;
+  int pre[kCols][3], n[kCols][3], total[kCols], offset[kCols];
+  int carry[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int h = 0; h < kCols; ++h) {
+    const int row = h * 32 + lane;
+    int below[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const int equal = row < R ? sh.equal[b][row] : 0;
+      int incl = equal;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      pre[h][b] = carry[b] + incl - equal;
+      carry[b] += __shfl_sync(0xffffffffu, incl, 31);
+      // items of the straddling key in this row that still fall above the boundary
+      below[b] = row < R ? sh.above[b][row] + max(0, min(equal, quota_b[b] - pre[h][b])) : 0;
+    }
+    n[h][0] = (below[2] - below[1]) * factor + (prefix_phase == 0 ? p : 0);  // NVFP4
+    n[h][1] = (below[1] - below[0]) * factor + (prefix_phase == 1 ? p : 0);  // INT8
+    n[h][2] = below[0] * factor + (prefix_phase == 2 ? p : 0);               // FP16
+    total[h] = row < R ? n[h][0] + n[h][1] + n[h][2] : -1;
+    int incl = max(total[h], 0);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    offset[h] = carry[3] + incl - max(total[h], 0);
+    carry[3] += __shfl_sync(0xffffffffu, incl, 31);
+    if (warp == h && row < R) {
+      row_offset[(int64_t)head * R + row] = offset[h];
+      int32_t* rc = row_counts + ((int64_t)head * R + row) * 4;
+      *reinterpret_cast<int2*>(rc) = make_int2(n[h][0], n[h][1]);
+      rc[2] = n[h][2];
+      if (kPairs) rc[3] = 0;
+    }
+  }
+  // A row's own numbers (row0 is even: the rows of a warp lie in one half)
+  const int half = kCols == 2 && row0 >= 32 ? 1 : 0;
+  const auto of_row = [&](const int (&v)[kCols], int row) {
+    return __shfl_sync(0xffffffffu, kCols == 2 && half ? v[kCols - 1] : v[0], row & 31);
+  };
+  int mine[kRows][3], run[kRows][3], len[kRows], at0[kRows];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      int v[kCols], w[kCols];
+#pragma unroll
+      for (int h = 0; h < kCols; ++h) {
+        v[h] = n[h][b];
+        w[h] = pre[h][b];
+      }
+      mine[r][b] = of_row(v, row0 + r);
+      run[r][b] = of_row(w, row0 + r);
+    }
+    len[r] = of_row(total, row0 + r);
+    at0[r] = of_row(offset, row0 + r);
+  }
+  if constexpr (!kPairs) {
+    // ---- launch order: longest list first, ties by block index, as block + 1 in the fourth entry of the
+    // position's counts ----
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      int rank = 0;
+#pragma unroll
+      for (int h = 0; h < kCols; ++h)
+        rank += __popc(__ballot_sync(0xffffffffu, total[h] > len[r] || (total[h] == len[r] && h * 32 + lane < row0 + r)));
+      if (lane == 0 && row0 + r < R) row_counts[((int64_t)head * R + rank) * 4 + 3] = row0 + r + 1;
+    }
+  }
+  const bool active[3] = {b2 > b1, b1 > b0, b0 > 0};  // phases with a budget
+  // ---- lists ----
+  if constexpr (!kPairs) {
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      if (len[r] <= 0 || (int64_t)at0[r] + len[r] > capacity) continue;  // (the latter cannot happen with exact budgets)
+      int32_t* list = stage_ids + (int64_t)head * capacity + at0[r];
+      const int n0 = mine[r][0], n1 = mine[r][1];
+      int at[3] = {prefix_phase == 0 ? p : 0, n0 + (prefix_phase == 1 ? p : 0), n0 + n1 + (prefix_phase == 2 ? p : 0)};
+      if (prefix_phase >= 0) {
+        const int seg = prefix_phase == 0 ? 0 : (prefix_phase == 1 ? n0 : n0 + n1);
+        for (int k = lane; k < p; k += 32) list[seg + k] = k;
+      }
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        const int stage = prefix_stages + (c * 32 + lane) * factor;
+        const int code = fused_code(key[r][c], key_b, quota_b, run[r], lower);
+#pragma unroll
+        for (int k = 1; k <= 3; ++k) {
+          if (!active[k - 1]) continue;
+          const unsigned members = __ballot_sync(0xffffffffu, code == k);
+          if (code == k) {
+            int32_t* dst = list + at[k - 1] + __popc(members & lower) * factor;
+            dst[0] = stage;
+            if (factor == 2) dst[1] = stage + 1;
+          }
+          at[k - 1] += __popc(members) * factor;
+        }
+      }
+    }
+  } else {
+    // One pair after the other (blocks 2t and 2t + 1): as in the kernel above
+    const int pairs_all = (R + 1) / 2;
+#pragma unroll
+    for (int r = 0; r < kRows; r += 2) {
+      const int a = row0 + r;
+      if (a >= R) continue;
+      const bool has_b = a + 1 < R;
+      const int n0 = mine[r][0] + (has_b ? mine[r + 1][0] : 0), n1 = mine[r][1] + (has_b ? mine[r + 1][1] : 0);
+      const bool fits = (int64_t)at0[r] + len[r] + (has_b ? len[r + 1] : 0) <= capacity;
+      int32_t* list = pair_ids + (int64_t)head * capacity + at0[r];
+      const int start[3] = {0, n0, n0 + n1};
+      int at[3] = {start[0], start[1], start[2]};
+      const int both = has_b ? (int)0xc0000000u : 1 << 30;
+      if (prefix_phase >= 0) {
+        if (fits)
+          for (int k = lane; k < p; k += 32) list[start[prefix_phase] + k] = k | both;
+        at[0] += prefix_phase == 0 ? p : 0;
+        at[1] += prefix_phase == 1 ? p : 0;
+        at[2] += prefix_phase == 2 ? p : 0;
+      }
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        const int stage = prefix_stages + c * 32 + lane;
+        const int ca = fused_code(key[r][c], key_b, quota_b, run[r], lower);
+        const int cb = fused_code(key[r + 1][c], key_b, quota_b, run[r + 1], lower);
+#pragma unroll
+        for (int k = 1; k <= 3; ++k) {
+          if (!active[k - 1]) continue;
+          const bool in = ca == k || cb == k;
+          const unsigned members = __ballot_sync(0xffffffffu, in);
+          if (in && fits)
+            list[at[k - 1] + __popc(members & lower)] = stage | (ca == k ? 1 << 30 : 0) | (cb == k ? (int)(1u << 31) : 0);
+          at[k - 1] += __popc(members);
+        }
+      }
+      if (lane == 0) {
+        int32_t* pc = pair_counts + ((int64_t)head * pairs_all + a / 2) * 4;
+        *reinterpret_cast<int2*>(pc) = make_int2(at[0] - start[0], at[1] - start[1]);
+        pc[2] = at[2] - start[2];
+        sh.unions[a / 2] = at[0] + at[1] + at[2] - start[1] - start[2];
+      }
+    }
+    __syncthreads();
+    const int mine_union = lane < pairs_all ? sh.unions[lane] : -1;
+#pragma unroll
+    for (int r = 0; r < kRows; r += 2) {
+      const int t = (row0 + r) / 2, length = t < pairs_all ? sh.unions[t] : 0;
+      const int rank = __popc(__ballot_sync(0xffffffffu, mine_union > length || (mine_union == length && lane < t)));
+      if (lane == 0 && t < pairs_all) pair_counts[((int64_t)head * pairs_all + rank) * 4 + 3] = t + 1;
+    }
+  }
+}
+
+template <bool kPairs, int kDraft>
+int launch_short(const anemoi_sm100_shape& s, const DraftPools& draft, const void* probability, int64_t n16, int64_t n8,
+                 int64_t n4, int prefix_phase, int32_t* row_offset, int32_t* row_counts, int32_t* stage_ids,
+                 int64_t capacity, int32_t* pair_counts, int32_t* pair_ids, cudaStream_t st) {
+  const int R = s.video_blocks;
+  const size_t smem = (size_t)draft_words(kDraft, kDraft ? draft.maps : 0) * 4;
+  auto kernel = route_short_kernel<1, kPairs, kDraft>;
+  if constexpr (kDraft == 0)
+    if (R > 32) kernel = route_short_kernel<2, kPairs, 0>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return ANEMOI_SM100_ELAUNCH;
+  return layer::launch(kernel, dim3(s.heads), dim3(kShortThreads), smem, st, draft,
+                       static_cast<const unsigned short*>(probability), R, (int)n16, (int)(n16 + n8),
+                       (int)(n16 + n8 + n4), s.query_block / 64, rec::prefix_stages(s), prefix_phase, capacity,
+                       row_offset, row_counts, stage_ids, pair_counts, pair_ids) == cudaSuccess
              ? ANEMOI_SM100_OK
              : ANEMOI_SM100_ELAUNCH;
 }
@@ -1353,8 +1660,11 @@ extern "C" int anemoi_sm100_route(const anemoi_sm100_shape* shape, const void* p
     return ANEMOI_SM100_EINVAL;
   if (R > 65535 || items * H >= (1ll << 40)) return ANEMOI_SM100_ELIMIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (R <= kShortBlocks)
+    return launch_short<false, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts,
+                                  stage_ids, list_capacity, nullptr, nullptr, st);
   if (fused_fits(H, R))
-    return launch_fused<kLists, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids,
+    return launch_fused<kLists>(*shape, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids,
                                list_capacity, nullptr, nullptr, st);
   RouteScratch sc;
   const int code = rank_rows(*shape, probability, n16, n8, n4, prefix_phase, true, scratch, row_offset, row_counts, sc, st);
@@ -1380,7 +1690,10 @@ extern "C" int anemoi_sm100_route_pairs(const anemoi_sm100_shape* shape, const v
   if (list_capacity < anemoi_sm100_route_list_capacity(shape, n16, n8, n4, prefix_phase))
     return ANEMOI_SM100_EINVAL;
   if (!fused_fits(shape->heads, shape->video_blocks) || rec::stages(*shape) >= (1 << 30)) return ANEMOI_SM100_ELIMIT;
-  return launch_fused<kNeighbours, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, nullptr,
+  if (shape->video_blocks <= kShortBlocks)
+    return launch_short<true, 0>(*shape, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts,
+                                 nullptr, list_capacity, pair_counts, pair_ids, static_cast<cudaStream_t>(stream));
+  return launch_fused<kNeighbours>(*shape, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, nullptr,
                             list_capacity, pair_counts, pair_ids, static_cast<cudaStream_t>(stream));
 }
 
@@ -1394,7 +1707,7 @@ int layer::route_bits(const anemoi_sm100_shape& s, const void* probability, int6
   if (prefix_phase < -1 || prefix_phase > 2) return ANEMOI_SM100_EINVAL;
   if (capacity < anemoi_sm100_route_list_capacity(&s, n16, n8, n4, prefix_phase)) return ANEMOI_SM100_EINVAL;
   if (fused_fits(H, R))
-    return launch_fused<kBits, 0>(s, DraftPools{}, probability, n16, n8, n4, prefix_phase, row_offset, row_counts,
+    return launch_fused<kBits>(s, probability, n16, n8, n4, prefix_phase, row_offset, row_counts,
                                   nullptr, 0, nullptr, nullptr, st, bits);
   RouteScratch sc;
   const int code = rank_rows(s, probability, n16, n8, n4, prefix_phase, false, scratch, row_offset, row_counts, sc, st);
@@ -1434,11 +1747,11 @@ int layer::draft_and_route(const anemoi_sm100_shape& s, const anemoi_sm100_opera
   d.maps = maxpool_weight != 0.0f && !most ? 2 : 1;
   d.weight = maxpool_weight;
   d.map = static_cast<unsigned short*>(probability);
-#define ANEMOI_LAUNCH(LEAVES, D)                                                                                      \
-  launch_fused<LEAVES, D>(s, d, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids, capacity, \
+#define ANEMOI_LAUNCH(PAIRS, D)                                                                                      \
+  launch_short<PAIRS, D>(s, d, probability, n16, n8, n4, prefix_phase, row_offset, row_counts, stage_ids, capacity, \
                          pair_counts, pair_ids, st)
-  if (pairs) return s.head_dim == 64 ? ANEMOI_LAUNCH(kNeighbours, 64) : ANEMOI_LAUNCH(kNeighbours, 128);
-  return s.head_dim == 64 ? ANEMOI_LAUNCH(kLists, 64) : ANEMOI_LAUNCH(kLists, 128);
+  if (pairs) return s.head_dim == 64 ? ANEMOI_LAUNCH(true, 64) : ANEMOI_LAUNCH(true, 128);
+  return s.head_dim == 64 ? ANEMOI_LAUNCH(false, 64) : ANEMOI_LAUNCH(false, 128);
 #undef ANEMOI_LAUNCH
 }
 

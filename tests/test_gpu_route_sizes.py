@@ -137,3 +137,10 @@ def test_map_of_the_one_launch(native_library, video, query_block, dim, weight, 
     else:
         assert torch.isfinite(got).all()
     assert executor.last_status() == 0
+
+
+@pytest.mark.parametrize("heads, blocks", [(3, 1), (3, 2), (2, 31), (2, 32), (2, 33), (5, 63), (150, 64), (2, 65)])
+@pytest.mark.parametrize("cells, prefix, phase", [((0.4, 0.4, 0.2), 0, -1), ((0.0, 1.0, 0.0), 200, 1), ((0.5, 0.0, 0.5), 70, 2)])
+def test_short_maps(native_library, heads, blocks, cells, prefix, phase):
+    """Up to 64 blocks a head's map is held in registers: one and two columns per lane, and the kernel past it."""
+    lists_equal_the_oracle(native_library, heads, blocks, cells, prefix, phase)
