@@ -1142,9 +1142,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
 // Q64, 9 heads x 14,161 tokens 201.5 / 177.6, Q128, 8 x 9,360 106.6 / 97.1; INT8 + NVFP4 D = 128, 11 x 9,464 450 / 407; INT8
 // Q128, 33 x 2,790 95.9 / 91.8.  24 MB gain less (11 x 9,464 424), past L2 it turns (10 MB per head, 56 x 38,247 tokens INT8,
 // with 2, 4, 6, 16 and 56 heads at a time 9.66, 9.82, 9.92, 10.32 and 10.69 ms).  Calls of less than a CTA per SM lose: 70 / 71.
-// Calls of one to two CTAs per SM: the lists of the first 148 CTAs start shortest first, so that the SM of the shortest gets
-// the longest of the others (4 x 6,664 tokens NVFP4 D = 64, 208 CTAs, 60.4 / 54.9, without the turn 55.3; 1 x 4,032 + 77, 264
-// CTAs 78.0 / 77.5 and 79.5).
+// Calls of one to four CTAs per SM: the lists of the first 148 CTAs start shortest first, so that the SM of the shortest gets
+// the longest of the others (4 x 6,664 tokens NVFP4 D = 64, 208 CTAs, 60.4 / 54.9, without the turn 55.3; 8 x 4,485 INT8,
+// 360 CTAs, 91.0 and 94.9 without; 1 x 43,680, 342 CTAs, 424 and 445; past four CTAs nothing).
 constexpr int kSms = 148;
 constexpr int64_t kHeadsBytes = 48 << 20;
 int heads_at_a_time(const AttnParams& p) {
@@ -1165,7 +1165,7 @@ int launch_kernel(AttnParams& p, int tiles, size_t smem, cudaStream_t st) {
   const int64_t ctas = (int64_t)tiles * p.s.heads;
   const int most = p.dense_prefix || ctas <= kSms ? 1 : heads_at_a_time(p), groups = (p.s.heads + most - 1) / most;
   const dim3 grid((p.s.heads + groups - 1) / groups, tiles, groups);
-  p.turn = !p.dense_prefix && groups == 1 && ctas > kSms && ctas <= 2 * kSms ? kSms / p.s.heads : 0;
+  p.turn = !p.dense_prefix && groups == 1 && ctas > kSms && ctas <= 4 * kSms ? kSms / p.s.heads : 0;
   return layer::launch(kernel, grid, dim3(kThreads), smem, st, p) == cudaSuccess
              ? ANEMOI_SM100_OK
              : ANEMOI_SM100_ELAUNCH;
