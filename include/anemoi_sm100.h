@@ -97,7 +97,8 @@ int64_t anemoi_sm100_operand_bytes(const anemoi_sm100_shape* shape, int which);
 int anemoi_sm100_prepare(const anemoi_sm100_shape* shape, const void* q, const void* k,
                          const void* v, const int64_t* strides, const int32_t* indices,
                          const int32_t* counts, const anemoi_sm100_operands* out, void* stream);
-/* Kernels of one such call: two, or one where there is no INT8 or the sequence is short. */
+/* Kernels of one such call, but for the one that zeroes memory: two, or one where there is no INT8 or the sequence is
+ * short. */
 int anemoi_sm100_prepare_kernels(const anemoi_sm100_shape* shape);
 
 /* Pooled-QK row softmax -> fp16 probability [H][R][R]; with 0 < w < 1 the mean
