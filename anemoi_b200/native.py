@@ -46,6 +46,7 @@ class Shape(C.Structure):
         ("has_prefix_query_int8", C.c_int32), ("has_maxpool", C.c_int32),
         ("input_is_bf16", C.c_int32),
         ("q_global_scale", C.c_float), ("k_global_scale", C.c_float), ("v_global_scale", C.c_float),
+        ("has_prefix_query_fp16", C.c_int32),
     ]
 
     @property
@@ -61,6 +62,10 @@ class Shape(C.Structure):
         if not self.has_prefix_query_int8:
             return 0
         return math.ceil(self.prefix_tokens / self.query_block)
+
+    @property
+    def prefix_fp16_tiles(self) -> int:
+        return math.ceil(self.prefix_tokens / self.query_block) if self.has_prefix_query_fp16 else 0
 
 
 class Operands(C.Structure):
@@ -393,7 +398,7 @@ def attention(shape: Shape, store: OperandStore, lists: RouteLists, valid_k: tor
 def prefix_attention(shape: Shape, store: OperandStore, valid_k: torch.Tensor,
                      status: torch.Tensor) -> torch.Tensor:
     dev = valid_k.device
-    rows = shape.prefix_query_tiles * shape.query_block
+    rows = (shape.prefix_query_tiles + shape.prefix_fp16_tiles) * shape.query_block
     out = torch.empty((shape.heads, rows, shape.head_dim), dtype=torch.float16, device=dev)
     _count("prefix_attention", 1)
     _check(library().anemoi_sm100_prefix_attention(
