@@ -133,6 +133,7 @@ struct AttnParams {
   int ring_bytes;    // key/value ring; re-partitioned into equal slots at every phase
   int q_region;      // bytes
   int turn;          // a head's lists before this place in the order start shortest first
+  int first_place;   // of a launch's tiles
 };
 
 // Entry g % kRing of a ring belongs to stage g, in phase g / kRing of the barrier.  Stage
@@ -596,7 +597,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   // CTAs start in the order x, y, z: the longest lists of a few heads, the second ones, ..., then the next few heads
   const int head = blockIdx.z * gridDim.x + blockIdx.x;
   if (head >= p.s.heads) return;
-  const int place = (int)blockIdx.y < p.turn ? p.turn - 1 - (int)blockIdx.y : (int)blockIdx.y;
+  const int place = p.first_place + ((int)blockIdx.y < p.turn ? p.turn - 1 - (int)blockIdx.y : (int)blockIdx.y);
   layer::grid_dependency_wait();
   // launch order of the head's query blocks (longest list first) as written by the routing
   // stage; 0 = no order given
@@ -1164,14 +1165,15 @@ int launch_kernel(AttnParams& p, int tiles, size_t smem, cudaStream_t st) {
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
-  if (tiles > 65535) return ANEMOI_SM100_ELIMIT;
   const int64_t ctas = (int64_t)tiles * p.s.heads;
   const int most = p.dense_prefix || ctas <= kSms ? 1 : heads_at_a_time(p), groups = (p.s.heads + most - 1) / most;
-  const dim3 grid((p.s.heads + groups - 1) / groups, tiles, groups);
   p.turn = !p.dense_prefix && groups == 1 && ctas > kSms && ctas <= 4 * kSms ? kSms / p.s.heads : 0;
-  return layer::launch(kernel, grid, dim3(kThreads), smem, st, p) == cudaSuccess
-             ? ANEMOI_SM100_OK
-             : ANEMOI_SM100_ELAUNCH;
+  // (the tiles of a head are the grid's y: a prefix of millions of rows takes several launches)
+  for (p.first_place = 0; p.first_place < tiles; p.first_place += 65535) {
+    const dim3 grid((p.s.heads + groups - 1) / groups, min(65535, tiles - p.first_place), groups);
+    if (layer::launch(kernel, grid, dim3(kThreads), smem, st, p) != cudaSuccess) return ANEMOI_SM100_ELAUNCH;
+  }
+  return ANEMOI_SM100_OK;
 }
 
 template <int D, bool kQ64>
