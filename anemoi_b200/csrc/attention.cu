@@ -1190,7 +1190,7 @@ int launch(AttnParams& p, int tiles, cudaStream_t st) {
   }
   // Prefix tiles run beside video tiles: of a mixed call in the same kernel, so that an SM's CTAs share
   // their code in the instruction cache.
-  if (p.dense_prefix && p.s.has_nvfp4 + p.s.has_int8 + p.s.has_fp16 > 1) one = kAny;
+  if (p.dense_prefix && (p.s.has_nvfp4 != 0) + (p.s.has_int8 != 0) + (p.s.has_fp16 != 0) > 1) one = kAny;
   q_region = (q_region + 127) & ~127;
   const int fixed = q_region + D * 4 + (int)sizeof(Shared);
   // two CTAs per SM: measured limit is 115,528 bytes of dynamic shared memory per CTA
@@ -1218,8 +1218,8 @@ int launch_for(AttnParams& p, int tiles, cudaStream_t st) {
 int check_ops(const anemoi_sm100_shape& s, const anemoi_sm100_operands& o, bool dense_prefix) {
   if (s.has_int8 && (!o.q_int8 || !o.kv_int8 || !o.q_int8_scale || !o.k_int8_scale || !o.v_e4m3_scale))
     return ANEMOI_SM100_EINVAL;
-  if (s.has_fp16 && (!dense_prefix || s.has_prefix_query_fp16) && (!o.q_fp16 || !o.kv_fp16)) return ANEMOI_SM100_EINVAL;
-  if (dense_prefix) return s.has_int8 || s.has_prefix_query_fp16 ? ANEMOI_SM100_OK : ANEMOI_SM100_EINVAL;
+  if (s.has_fp16 && (!dense_prefix || rec::prefix_fp16(s)) && (!o.q_fp16 || !o.kv_fp16)) return ANEMOI_SM100_EINVAL;
+  if (dense_prefix) return s.has_int8 || rec::prefix_fp16(s) ? ANEMOI_SM100_OK : ANEMOI_SM100_EINVAL;
   if (s.has_nvfp4 && (!o.q_nvfp4 || !o.kv_nvfp4)) return ANEMOI_SM100_EINVAL;
   return ANEMOI_SM100_OK;
 }
@@ -1329,7 +1329,7 @@ int prefix_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operand
                      void* out_prefix, const TokenRows* rows, int32_t* status, void* stream) {
   if (rec::validate_shape(shape) != ANEMOI_SM100_OK || !ops || !valid_k || (!out_prefix && !rows) || !status)
     return ANEMOI_SM100_EINVAL;
-  const bool fp16 = shape->has_prefix_query_fp16 != 0;
+  const bool fp16 = rec::prefix_fp16(*shape);
   if (!(shape->has_prefix_query_int8 || fp16) || shape->prefix_tokens == 0) return ANEMOI_SM100_EINVAL;
   if (check_ops(*shape, *ops, true) != ANEMOI_SM100_OK) return ANEMOI_SM100_EINVAL;
   AttnParams p{};

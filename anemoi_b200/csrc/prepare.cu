@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB, kOwnMaxima)) prepare_ke
         write_nvfp4_rows<D>(r4, r4 + QB * D / 2, tile, 0, QB, p.s.q_global_scale);
       }
     }
-    if (!video && p.s.has_prefix_query_fp16) {
+    if (!video && rec::prefix_fp16(p.s)) {
       write_fp16_tile<D>(static_cast<uint8_t*>(p.o.q_fp16) +
                              ((int64_t)p.s.heads * R + (int64_t)head * p.prefix_q_tiles + t) * rec::q_fp16_bytes(QB, D),
                          tile, 0, QB);
@@ -674,7 +674,7 @@ int launch(const PrepParams& p, cudaStream_t stream) {
       const int n = p.s.heads * D;
       // (beside prefix rows that the library computes on another stream, the memset: its wait lets their few long CTAs in
       // first, each on an SM of its own; 5 heads x 19,425 tokens with 62 of prefix 494 us, with the kernel 628)
-      if (p.s.prefix_tokens > 0 && !p.s.has_prefix_query_int8 && !p.s.has_prefix_query_fp16)
+      if (p.s.prefix_tokens > 0 && !p.s.has_prefix_query_int8 && !rec::prefix_fp16(p.s))
         err = cudaMemsetAsync(p.o.v_amax, 0, sizeof(float) * n, stream);
       else
         err = layer::launch(zero_kernel, dim3(min(148, (n + kZeroThreads - 1) / kZeroThreads)), dim3(kZeroThreads), 0, stream,

@@ -126,10 +126,10 @@ def make_shape(q: torch.Tensor, *, prefix_tokens: int, video_blocks: int, query_
         heads=q.size(2), head_dim=q.size(3), query_block=query_block_size, seq_tokens=q.size(1),
         prefix_tokens=prefix_tokens, video_blocks=video_blocks,
         has_nvfp4=int("nvfp4" in active), has_int8=int("int8" in active),
-        has_fp16=int("fp16" in active), has_prefix_query_int8=int(native_prefix),
+        has_fp16=2 if fp16_prefix else int("fp16" in active), has_prefix_query_int8=int(native_prefix),
         has_maxpool=int(has_maxpool), input_is_bf16=int(q.dtype == torch.bfloat16),
         q_global_scale=nvfp4_scales[0], k_global_scale=nvfp4_scales[1],
-        v_global_scale=nvfp4_scales[2], has_prefix_query_fp16=int(fp16_prefix),
+        v_global_scale=nvfp4_scales[2],
     )
 
 
@@ -340,9 +340,9 @@ class _Plan:
         shape = native.Shape(
             heads=heads, head_dim=dim, query_block=query_block, seq_tokens=tokens, prefix_tokens=prefix_tokens,
             video_blocks=blocks, has_nvfp4=int("nvfp4" in active), has_int8=int("int8" in active),
-            has_fp16=int("fp16" in active), has_prefix_query_int8=int(int8_prefix),
+            has_fp16=2 if fp16_prefix else int("fp16" in active), has_prefix_query_int8=int(int8_prefix),
             has_maxpool=int(maxpool_weight != 0.0), input_is_bf16=int(dtype == torch.bfloat16),
-            q_global_scale=1.0, k_global_scale=1.0, v_global_scale=1.0, has_prefix_query_fp16=int(fp16_prefix))
+            q_global_scale=1.0, k_global_scale=1.0, v_global_scale=1.0)
         lib = native.library()
         phase = -1 if prefix_phase is None else PHASE_ORDER.index(prefix_phase)
         capacity = max(1, int(lib.anemoi_sm100_route_list_capacity(C.byref(shape), n16, n8, n4, phase)))

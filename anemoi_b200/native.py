@@ -46,7 +46,6 @@ class Shape(C.Structure):
         ("has_prefix_query_int8", C.c_int32), ("has_maxpool", C.c_int32),
         ("input_is_bf16", C.c_int32),
         ("q_global_scale", C.c_float), ("k_global_scale", C.c_float), ("v_global_scale", C.c_float),
-        ("has_prefix_query_fp16", C.c_int32),
     ]
 
     @property
@@ -65,7 +64,7 @@ class Shape(C.Structure):
 
     @property
     def prefix_fp16_tiles(self) -> int:
-        return math.ceil(self.prefix_tokens / self.query_block) if self.has_prefix_query_fp16 else 0
+        return math.ceil(self.prefix_tokens / self.query_block) if self.has_fp16 == 2 else 0
 
 
 class Operands(C.Structure):
