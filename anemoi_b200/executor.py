@@ -230,7 +230,7 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
                                           logical_block=query_block_size, enable_anchors=enable_anchors)
     blocks = layout.video_blocks
     fp16_prefix = not int8_prefix and _fp16_prefix(prefix_tokens, q_bshd.size(2), q_bshd.size(3), query_block_size,
-                                                   blocks, active)
+                                                   blocks, active, float(sparsity_ratio))
     native_prefix = int8_prefix or fp16_prefix
 
     current = torch.cuda.current_stream(device)
@@ -299,7 +299,7 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
     return out
 
 
-def _fp16_prefix(prefix_tokens, heads, dim, query_block, blocks, active):
+def _fp16_prefix(prefix_tokens, heads, dim, query_block, blocks, active, sparsity):
     """Whether FP16 prefix queries take the FP16 cell's kernel rather than the library's dense attention.
 
     They can where that cell's keys and values are there anyway.  The library's kernel is the better one for many
@@ -308,11 +308,20 @@ def _fp16_prefix(prefix_tokens, heads, dim, query_block, blocks, active):
     and while the tiles start beside draft and routing (fewer than one per SM).  Library / kernel, us, 80 % dropped:
     FP16 and INT8, D = 128, 12 heads x 7,800 tokens + 500 (6,200 steps) 237 / 216, 20 heads (10,400) 352 / 341, 20 x 20,280 + 250
     (13,000) 1,224 / 1,267; FP16 alone, D = 128, 16 x 3,120 + 250 (1,700) 100 / 82, 12 x 7,800 + 500 182 / 187; D = 64, 8 x 3,120 + 250
-    (840) 124 / 49, 12 x 20,280 + 500 (15,600) 577 / 556 and, with INT8, 689 / 678, 8 x 84,672 + 500 (42,000) 4,496 / 4,520."""
+    (840) 124 / 49, 12 x 20,280 + 500 (15,600) 577 / 556 and, with INT8, 689 / 678, 8 x 84,672 + 500 (42,000) 4,496 / 4,520.
+
+    The kernel's tiles start behind the preparation, the library's with it.  Where a tile's walk (0.8 us a stage) is long and
+    twice as long as the video's lists take (0.45 us a stage and SM), that counts, and D = 128 stays with the library:
+    5 heads x 19,680 tokens + 427 in host groups, 90 % dropped, 1,945 / 2,000."""
     if not prefix_tokens or "fp16" not in active:
         return False
     tiles = math.ceil(prefix_tokens / 128) * heads
-    steps = tiles * (math.ceil(prefix_tokens / 64) + blocks * (query_block // 64))
+    prefix_stages = math.ceil(prefix_tokens / 64)
+    stages = prefix_stages + blocks * (query_block // 64)
+    steps = tiles * stages
+    lists = heads * blocks * ((1.0 - sparsity) * blocks * (query_block // 64) + prefix_stages)
+    if dim == 128 and stages > 190 and lists < 131 * stages:
+        return False
     return tiles < 148 and steps <= (20000 if dim == 64 else 10000 if len(active) > 1 else 5000)
 
 
@@ -331,7 +340,7 @@ class _Plan:
         self.layout = materialize_ragged_2d_layout(device, frames=frames, height=height, width=width,
                                                    logical_block=query_block)
         blocks = self.layout.video_blocks
-        fp16_prefix = not int8_prefix and _fp16_prefix(prefix_tokens, heads, dim, query_block, blocks, active)
+        fp16_prefix = not int8_prefix and _fp16_prefix(prefix_tokens, heads, dim, query_block, blocks, active, sparsity)
         self.native_prefix = int8_prefix or fp16_prefix
         self.valid_k = _valid_k(device, prefix_tokens, query_block, _counts_key(self.layout))
         self.status = _status_word(device)
