@@ -1151,8 +1151,11 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
 // 360 CTAs, 91.0 and 94.9 without; 1 x 43,680, 342 CTAs, 424 and 445; past four CTAs nothing).
 constexpr int kSms = 148;
 constexpr int64_t kHeadsBytes = 48 << 20;
-int heads_at_a_time(const AttnParams& p) {
-  if (p.dense_prefix) return 1;
+// FP16 alone at D = 128, whose stages are the largest, loses once a call has many waves (45 heads x 11,600 tokens, 15 waves,
+// 625 / 641; 16 x 14,040 with pairs, 6 waves, 563 / 553).
+int heads_at_a_time(const AttnParams& p, int64_t ctas) {
+  if (p.dense_prefix || ctas <= kSms) return 1;
+  if (p.s.head_dim == 128 && !p.s.has_int8 && !p.s.has_nvfp4 && ctas > 16 * kSms) return 1;
   const int64_t bytes = (p.s.has_nvfp4 ? rec::kv_nvfp4_bytes(p.s.head_dim) : 0) +
                         (p.s.has_int8 ? rec::kv_int8_bytes(p.s.head_dim) : 0) +
                         (p.s.has_fp16 ? rec::kv_fp16_bytes(p.s.head_dim) : 0);
@@ -1166,7 +1169,7 @@ int launch_kernel(AttnParams& p, int tiles, size_t smem, cudaStream_t st) {
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
   const int64_t ctas = (int64_t)tiles * p.s.heads;
-  const int most = p.dense_prefix || ctas <= kSms ? 1 : heads_at_a_time(p), groups = (p.s.heads + most - 1) / most;
+  const int most = heads_at_a_time(p, ctas), groups = (p.s.heads + most - 1) / most;
   p.turn = !p.dense_prefix && groups == 1 && ctas > kSms && ctas <= 4 * kSms ? kSms / p.s.heads : 0;
   // (the tiles of a head are the grid's y: a prefix of millions of rows takes several launches)
   for (p.first_place = 0; p.first_place < tiles; p.first_place += 65535) {
