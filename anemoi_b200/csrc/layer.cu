@@ -2,8 +2,8 @@
 // prefix attention, with the results written straight to their tokens.
 //
 // A small call is bound by its launches, not by its kernels: with one Python wrapper, allocation and
-// marshaling per stage the 1,024-token call takes 210 us, here 24 (20 of them host time).  The host work
-// is one function: one workspace cut up by offsets, three to six kernels (routing is one for most shapes, and forms
+// marshaling per stage the 1,024-token call takes 210 us, here 19.5 (all of them host time).  The host work
+// is one function: one workspace cut up by offsets, three to eight kernels (routing is one for most shapes, and forms
 // the draft map of short calls; the output needs no assembly pass), programmatic dependent launches between them.
 //
 // Order of the launches.  The prefix rows' tiles walk every stage of the head: few CTAs, each as
