@@ -123,10 +123,7 @@ struct AttnParams {
   const int32_t* counts;   // real tokens of a block
   int32_t* status;
   uint64_t wait_ns;  // limit of every mbarrier wait
-  int dense_prefix;  // prefix query tiles over every stage: 1 in the INT8 cell, 2 in the FP16 cell
-  int prefix_tiles;  // prefix query tiles of such a launch
-  int q_fp_first;    // first record of the launch in q_fp16 (q_nvfp4), records per head
-  int q_fp_tiles;
+  int dense_prefix;  // 1: prefix query tiles, INT8 cell over every stage
   int stages;        // 64-key stages per head
   int q_tiles_int8;  // records per head in q_int8 (R + prefix query tiles)
   int out_rows;      // rows per head in `out`
@@ -615,11 +612,11 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   // (prefix tiles of 64 rows also go in twos: both walk every stage)
   const bool twos = pairs || (kQ64 && p.dense_prefix);
   int tile_blocks =
-      twos && 2 * tile + 1 < (p.dense_prefix ? p.prefix_tiles : p.s.video_blocks) ? 2 : 1;
+      twos && 2 * tile + 1 < (p.dense_prefix ? p.q_tiles_int8 - p.s.video_blocks : p.s.video_blocks) ? 2 : 1;
   int block0 = twos ? 2 * tile : tile, block1 = block0 + 1;
 
   // ---- this tile's work list ----
-  int cnt[3] = {0, p.dense_prefix == 1 ? p.stages : 0, p.dense_prefix == 2 ? p.stages : 0};
+  int cnt[3] = {0, p.stages, 0};
   const int32_t* list = nullptr;
   if (table) {
     const int4* entry = p.pair_table + ((int64_t)head * pair_tiles + tile) * 2;
@@ -726,7 +723,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       const int head_at = kReread ? b->head : head, first_block = kReread ? b->block[0] : block0;
       const int blocks = kReread ? b->tile_blocks : tile_blocks;
       const int32_t* list_at = kReread ? b->list : list;
-      const int q_index_fp = p.q_fp_first + head_at * p.q_fp_tiles + first_block;  // q_fp16 / q_nvfp4 record
+      const int q_index_fp = head_at * p.s.video_blocks + first_block;  // q_fp16 / q_nvfp4 record
       const int64_t q_index_i8 =
           (int64_t)head_at * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks : 0) + first_block;
       const int step = (kReread ? b->block[1] : block1) - first_block;  // from a pair's first record to its second
@@ -1182,7 +1179,7 @@ int launch_kernel(AttnParams& p, int tiles, size_t smem, cudaStream_t st) {
 template <int D, bool kQ64>
 int launch(AttnParams& p, int tiles, cudaStream_t st) {
   int q_region = 0, slot = 0, cells = 0, one = kAny;
-  const bool use[3] = {p.s.has_nvfp4 && !p.dense_prefix, p.s.has_int8 && p.dense_prefix != 2, p.s.has_fp16 && p.dense_prefix != 1};
+  const bool use[3] = {p.s.has_nvfp4 && !p.dense_prefix, p.s.has_int8 != 0, p.s.has_fp16 && !p.dense_prefix};
   for (int cell = 0; cell < 3; ++cell) {
     if (!use[cell]) continue;
     one = cells++ == 0 ? cell : kAny;
@@ -1193,7 +1190,7 @@ int launch(AttnParams& p, int tiles, cudaStream_t st) {
   }
   // Prefix tiles run beside video tiles: of a mixed call in the same kernel, so that an SM's CTAs share
   // their code in the instruction cache.
-  if (p.dense_prefix && (p.s.has_nvfp4 != 0) + (p.s.has_int8 != 0) + (p.s.has_fp16 != 0) > 1) one = kAny;
+  if (p.dense_prefix && (p.s.has_nvfp4 || p.s.has_fp16)) one = kAny;
   q_region = (q_region + 127) & ~127;
   const int fixed = q_region + D * 4 + (int)sizeof(Shared);
   // two CTAs per SM: measured limit is 115,528 bytes of dynamic shared memory per CTA
@@ -1221,8 +1218,8 @@ int launch_for(AttnParams& p, int tiles, cudaStream_t st) {
 int check_ops(const anemoi_sm100_shape& s, const anemoi_sm100_operands& o, bool dense_prefix) {
   if (s.has_int8 && (!o.q_int8 || !o.kv_int8 || !o.q_int8_scale || !o.k_int8_scale || !o.v_e4m3_scale))
     return ANEMOI_SM100_EINVAL;
-  if (s.has_fp16 && (!dense_prefix || rec::prefix_fp16(s)) && (!o.q_fp16 || !o.kv_fp16)) return ANEMOI_SM100_EINVAL;
-  if (dense_prefix) return s.has_int8 || rec::prefix_fp16(s) ? ANEMOI_SM100_OK : ANEMOI_SM100_EINVAL;
+  if (dense_prefix) return s.has_int8 ? ANEMOI_SM100_OK : ANEMOI_SM100_EINVAL;
+  if (s.has_fp16 && (!o.q_fp16 || !o.kv_fp16)) return ANEMOI_SM100_EINVAL;
   if (s.has_nvfp4 && (!o.q_nvfp4 || !o.kv_nvfp4)) return ANEMOI_SM100_EINVAL;
   return ANEMOI_SM100_OK;
 }
@@ -1297,7 +1294,6 @@ int video_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operands
   p.dense_prefix = 0;
   p.stages = rec::stages(*shape);
   p.q_tiles_int8 = shape->video_blocks + rec::prefix_query_tiles(*shape);
-  p.q_fp_tiles = shape->video_blocks;
   p.out_rows = shape->video_blocks * shape->query_block;
   set_rows(p, rows);
   const int tiles = pair_counts || pair_table ? (shape->video_blocks + 1) / 2 : shape->video_blocks;
@@ -1332,8 +1328,7 @@ int prefix_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operand
                      void* out_prefix, const TokenRows* rows, int32_t* status, void* stream) {
   if (rec::validate_shape(shape) != ANEMOI_SM100_OK || !ops || !valid_k || (!out_prefix && !rows) || !status)
     return ANEMOI_SM100_EINVAL;
-  const bool fp16 = rec::prefix_fp16(*shape);
-  if (!(shape->has_prefix_query_int8 || fp16) || shape->prefix_tokens == 0) return ANEMOI_SM100_EINVAL;
+  if (!shape->has_prefix_query_int8 || shape->prefix_tokens == 0) return ANEMOI_SM100_EINVAL;
   if (check_ops(*shape, *ops, true) != ANEMOI_SM100_OK) return ANEMOI_SM100_EINVAL;
   AttnParams p{};
   p.s = *shape;
@@ -1342,14 +1337,11 @@ int prefix_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operand
   p.out = static_cast<__half*>(out_prefix);
   p.status = status;
   p.wait_ns = g_wait_limit_ns;
-  p.dense_prefix = fp16 ? 2 : 1;
+  p.dense_prefix = 1;
   p.stages = rec::stages(*shape);
-  const int blocks = rec::prefix_query_tiles(*shape) + rec::prefix_fp16_tiles(*shape);
+  const int blocks = rec::prefix_query_tiles(*shape);
   const int tiles = shape->query_block == 64 ? (blocks + 1) / 2 : blocks;
-  p.prefix_tiles = blocks;
   p.q_tiles_int8 = shape->video_blocks + blocks;
-  p.q_fp_first = shape->heads * shape->video_blocks;
-  p.q_fp_tiles = blocks;
   p.out_rows = blocks * shape->query_block;
   set_rows(p, rows);
   cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -143,7 +143,7 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
     s.v_global_scale = nvfp4_scales[2];
     if (rec::validate_shape(&s) != ANEMOI_SM100_OK) return ANEMOI_SM100_EINVAL;
   }
-  const bool native_prefix = (s.has_prefix_query_int8 || rec::prefix_fp16(s)) && s.prefix_tokens > 0;
+  const bool native_prefix = s.has_prefix_query_int8 && s.prefix_tokens > 0;
   if (s.prefix_tokens > 0 && !native_prefix && prefix_out == nullptr) return ANEMOI_SM100_EINVAL;
   if (s.prefix_tokens > 0 && side_stream == nullptr) return ANEMOI_SM100_EINVAL;
   const Workspace w = cut(p, static_cast<uint8_t*>(workspace));
@@ -171,8 +171,7 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
       return ANEMOI_SM100_ELAUNCH;
     return layer::prefix_rows(s, w.ops, p.valid_k, rows, p.status, side);
   };
-  const int prefix_ctas =
-      ((rec::prefix_query_tiles(s) + rec::prefix_fp16_tiles(s)) * s.query_block + 127) / 128 * s.heads;
+  const int prefix_ctas = (rec::prefix_query_tiles(s) * s.query_block + 127) / 128 * s.heads;
   const bool late = native_prefix && prefix_ctas >= kPrefixFillsGpu;
   if (native_prefix && !late && (code = prefix()) != ANEMOI_SM100_OK) return done(code);
 

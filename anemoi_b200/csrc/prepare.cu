@@ -420,9 +420,9 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB, kOwnMaxima)) prepare_ke
   // pieces of the same token rows
   const int task = blockIdx.x / p.s.heads, head = blockIdx.x - task * p.s.heads;
   constexpr int kF = QB / 64;
-  const int64_t qtiles = R + p.prefix_q_tiles;
+  const int64_t qtiles_i8 = R + p.prefix_q_tiles;
 
-  if (task < qtiles) {
+  if (task < qtiles_i8) {
     // ---------------- query tile (video or prefix) ----------------
     // (after the maxima's kernel, whose CTAs all began when what was before it in the stream was
     // complete; without INT8 there is no such kernel)
@@ -450,14 +450,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB, kOwnMaxima)) prepare_ke
         write_nvfp4_rows<D>(r4, r4 + QB * D / 2, tile, 0, QB, p.s.q_global_scale);
       }
     }
-    if (!video && rec::prefix_fp16(p.s)) {
-      write_fp16_tile<D>(static_cast<uint8_t*>(p.o.q_fp16) +
-                             ((int64_t)p.s.heads * R + (int64_t)head * p.prefix_q_tiles + t) * rec::q_fp16_bytes(QB, D),
-                         tile, 0, QB);
-      return;
-    }
     if (has_int8()) {
-      const int64_t slot = (int64_t)head * (p.s.has_prefix_query_int8 ? qtiles : R) + task;
+      const int64_t slot = (int64_t)head * qtiles_i8 + task;
       const float amax = tile_amax<D>(tile, 0, QB, red);
       const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1.0e-7f);
       if (threadIdx.x == 0) p.o.q_int8_scale[slot] = scale;
@@ -469,8 +463,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas(QB, kOwnMaxima)) prepare_ke
 
   // ---------------- key or value block (video) or stage (prefix) ----------------
   const int blocks = R + p.prefix_stages;
-  const bool second_half = kSplit && task >= qtiles + blocks;
-  const int block = task - (int)qtiles - (second_half ? blocks : 0);
+  const bool second_half = kSplit && task >= qtiles_i8 + blocks;
+  const int block = task - (int)qtiles_i8 - (second_half ? blocks : 0);
   const bool video = block < R;
   const int b = video ? block : block - R;
   const int nst = video ? kF : 1;
@@ -674,7 +668,7 @@ int launch(const PrepParams& p, cudaStream_t stream) {
       const int n = p.s.heads * D;
       // (beside prefix rows that the library computes on another stream, the memset: its wait lets their few long CTAs in
       // first, each on an SM of its own; 5 heads x 19,425 tokens with 62 of prefix 494 us, with the kernel 628)
-      if (p.s.prefix_tokens > 0 && !p.s.has_prefix_query_int8 && !rec::prefix_fp16(p.s))
+      if (p.s.prefix_tokens > 0 && !p.s.has_prefix_query_int8)
         err = cudaMemsetAsync(p.o.v_amax, 0, sizeof(float) * n, stream);
       else
         err = layer::launch(zero_kernel, dim3(min(148, (n + kZeroThreads - 1) / kZeroThreads)), dim3(kZeroThreads), 0, stream,
@@ -707,7 +701,7 @@ extern "C" int64_t anemoi_sm100_operand_bytes(const anemoi_sm100_shape* s, int w
   const int64_t H = s->heads, D = s->head_dim, QB = s->query_block, R = s->video_blocks;
   const int64_t NS = rec::stages(*s), PQ = rec::prefix_query_tiles(*s);
   switch (which) {
-    case ANEMOI_SM100_BUF_Q_FP16: return s->has_fp16 ? H * (R + rec::prefix_fp16_tiles(*s)) * rec::q_fp16_bytes(QB, D) : 0;
+    case ANEMOI_SM100_BUF_Q_FP16: return s->has_fp16 ? H * R * rec::q_fp16_bytes(QB, D) : 0;
     case ANEMOI_SM100_BUF_KV_FP16: return s->has_fp16 ? H * NS * rec::kv_fp16_bytes(D) : 0;
     case ANEMOI_SM100_BUF_Q_INT8: return s->has_int8 ? H * (R + PQ) * rec::q_int8_bytes(QB, D) : 0;
     case ANEMOI_SM100_BUF_KV_INT8: return s->has_int8 ? H * NS * rec::kv_int8_bytes(D) : 0;
@@ -750,7 +744,7 @@ extern "C" int anemoi_sm100_prepare(const anemoi_sm100_shape* shape, const void*
   }
   p.prefix_stages = rec::prefix_stages(s);
   p.stages = rec::stages(s);
-  p.prefix_q_tiles = rec::prefix_query_tiles(s) + rec::prefix_fp16_tiles(s);
+  p.prefix_q_tiles = rec::prefix_query_tiles(s);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // Keys and values of a block in CTAs of their own: half the serial chain, which is quicker for
   // 128-row blocks (sweep's 4 heads 71 -> 64 us, 56 heads x 85,184 tokens 2,178 -> 2,128) and for small grids; for

@@ -24,11 +24,6 @@ __host__ __device__ inline int stages(const anemoi_sm100_shape& s) {
 __host__ __device__ inline int prefix_query_tiles(const anemoi_sm100_shape& s) {
   return s.has_prefix_query_int8 ? (s.prefix_tokens + s.query_block - 1) / s.query_block : 0;
 }
-// Prefix queries in the FP16 cell.
-__host__ __device__ inline bool prefix_fp16(const anemoi_sm100_shape& s) { return s.has_fp16 == 2; }
-__host__ __device__ inline int prefix_fp16_tiles(const anemoi_sm100_shape& s) {
-  return prefix_fp16(s) ? (s.prefix_tokens + s.query_block - 1) / s.query_block : 0;
-}
 
 inline int validate_shape(const anemoi_sm100_shape* s) {
   if (s == nullptr) return ANEMOI_SM100_EINVAL;
@@ -39,7 +34,6 @@ inline int validate_shape(const anemoi_sm100_shape* s) {
     return ANEMOI_SM100_EINVAL;
   if (!(s->has_nvfp4 || s->has_int8 || s->has_fp16)) return ANEMOI_SM100_EINVAL;
   if (s->has_prefix_query_int8 && !s->has_int8) return ANEMOI_SM100_EINVAL;
-  if (prefix_fp16(*s) && s->has_prefix_query_int8) return ANEMOI_SM100_EINVAL;
   if (s->has_nvfp4 && !(s->q_global_scale > 0.f && s->k_global_scale > 0.f && s->v_global_scale > 0.f))
     return ANEMOI_SM100_EINVAL;
   return ANEMOI_SM100_OK;

@@ -121,12 +121,12 @@ def _valid_k(device: torch.device, prefix_tokens: int, query_block: int, counts_
 
 def make_shape(q: torch.Tensor, *, prefix_tokens: int, video_blocks: int, query_block_size: int,
                active: tuple[str, ...], native_prefix: bool, has_maxpool: bool,
-               nvfp4_scales=(1.0, 1.0, 1.0), fp16_prefix: bool = False) -> native.Shape:
+               nvfp4_scales=(1.0, 1.0, 1.0)) -> native.Shape:
     return native.Shape(
         heads=q.size(2), head_dim=q.size(3), query_block=query_block_size, seq_tokens=q.size(1),
         prefix_tokens=prefix_tokens, video_blocks=video_blocks,
         has_nvfp4=int("nvfp4" in active), has_int8=int("int8" in active),
-        has_fp16=2 if fp16_prefix else int("fp16" in active), has_prefix_query_int8=int(native_prefix),
+        has_fp16=int("fp16" in active), has_prefix_query_int8=int(native_prefix),
         has_maxpool=int(has_maxpool), input_is_bf16=int(q.dtype == torch.bfloat16),
         q_global_scale=nvfp4_scales[0], k_global_scale=nvfp4_scales[1],
         v_global_scale=nvfp4_scales[2],
@@ -224,15 +224,10 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
     video = video_phases(retained_nvfp4_ratio, retained_int8_ratio, retained_fp16_ratio)
     if prefix_query_precision not in ("int8", "fp16"):
         raise ValueError("prefix_query_precision must be int8 or fp16")
-    int8_prefix = prefix_tokens > 0 and prefix_query_precision == "int8" and "int8" in video
+    native_prefix = prefix_tokens > 0 and prefix_query_precision == "int8" and "int8" in video
     active, prefix_phase = resolve_phases(video, prefix_tokens, prefix_kv_precision)
-    layout = materialize_ragged_2d_layout(device, frames=video_shape[0], height=video_shape[1], width=video_shape[2],
-                                          logical_block=query_block_size, enable_anchors=enable_anchors)
-    blocks = layout.video_blocks
-    fp16_prefix = not int8_prefix and _fp16_prefix(prefix_tokens, q_bshd.size(2), q_bshd.size(3), query_block_size,
-                                                   blocks, active, float(sparsity_ratio))
-    native_prefix = int8_prefix or fp16_prefix
 
+    frames, height, width = video_shape
     current = torch.cuda.current_stream(device)
     side = _prefix_stream(device)
     prefix_out = None
@@ -248,10 +243,13 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
                 is_causal=False,
             )[0].contiguous()
 
+    layout = materialize_ragged_2d_layout(device, frames=frames, height=height, width=width,
+                                          logical_block=query_block_size, enable_anchors=enable_anchors)
+    blocks = layout.video_blocks
     shape = make_shape(q_bshd, prefix_tokens=prefix_tokens, video_blocks=blocks,
                        query_block_size=query_block_size, active=active,
-                       native_prefix=int8_prefix, has_maxpool=2 if diag_jensen else maxpool_weight != 0.0,
-                       nvfp4_scales=nvfp4_scales, fp16_prefix=fp16_prefix)
+                       native_prefix=native_prefix, has_maxpool=2 if diag_jensen else maxpool_weight != 0.0,
+                       nvfp4_scales=nvfp4_scales)
     store = native.allocate_operands(shape, device)
     with _Stage("prepare"), _Range("anemoi.peripheral.prepare", nvtx):
         native.prepare(shape, q_bshd, k_bshd, v_bshd, layout.indices, layout.counts, store)
@@ -299,32 +297,6 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
     return out
 
 
-def _fp16_prefix(prefix_tokens, heads, dim, query_block, blocks, active, sparsity):
-    """Whether FP16 prefix queries take the FP16 cell's kernel rather than the library's dense attention.
-
-    They can where that cell's keys and values are there anyway.  The library's kernel is the better one for many
-    rows of D = 128; for few, its few CTAs walk the whole sequence each (slowly for D = 64), and its launch, the copy of
-    its result and the gaps around them cost 20 us.  So up to a number of (tile of 128 rows, 64-key stage) steps,
-    and while the tiles start beside draft and routing (fewer than one per SM).  Library / kernel, us, 80 % dropped:
-    FP16 and INT8, D = 128, 12 heads x 7,800 tokens + 500 (6,200 steps) 237 / 216, 20 heads (10,400) 352 / 341, 20 x 20,280 + 250
-    (13,000) 1,224 / 1,267; FP16 alone, D = 128, 16 x 3,120 + 250 (1,700) 100 / 82, 12 x 7,800 + 500 182 / 187; D = 64, 8 x 3,120 + 250
-    (840) 124 / 49, 12 x 20,280 + 500 (15,600) 577 / 556 and, with INT8, 689 / 678, 8 x 84,672 + 500 (42,000) 4,496 / 4,520.
-
-    The kernel's tiles start behind the preparation, the library's with it.  Where a tile's walk (0.8 us a stage) is long and
-    twice as long as the video's lists take (0.45 us a stage and SM), that counts, and D = 128 stays with the library:
-    5 heads x 19,680 tokens + 427 in host groups, 90 % dropped, 1,945 / 2,000."""
-    if not prefix_tokens or "fp16" not in active:
-        return False
-    tiles = math.ceil(prefix_tokens / 128) * heads
-    prefix_stages = math.ceil(prefix_tokens / 64)
-    stages = prefix_stages + blocks * (query_block // 64)
-    steps = tiles * stages
-    lists = heads * blocks * ((1.0 - sparsity) * blocks * (query_block // 64) + prefix_stages)
-    if dim == 128 and stages > 190 and lists < 131 * stages:
-        return False
-    return tiles < 148 and steps <= (20000 if dim == 64 else 10000 if len(active) > 1 else 5000)
-
-
 class _Plan:
     """The native plan of one configuration with the tensors it points to."""
 
@@ -334,14 +306,12 @@ class _Plan:
         video = video_phases(nvfp4, int8, fp16)
         if prefix_query not in ("int8", "fp16"):
             raise ValueError("prefix_query_precision must be int8 or fp16")
-        int8_prefix = prefix_tokens > 0 and prefix_query == "int8" and "int8" in video
+        self.native_prefix = prefix_tokens > 0 and prefix_query == "int8" and "int8" in video
         active, prefix_phase = resolve_phases(video, prefix_tokens, prefix_kv)
         frames, height, width = video_shape
         self.layout = materialize_ragged_2d_layout(device, frames=frames, height=height, width=width,
                                                    logical_block=query_block)
         blocks = self.layout.video_blocks
-        fp16_prefix = not int8_prefix and _fp16_prefix(prefix_tokens, heads, dim, query_block, blocks, active, sparsity)
-        self.native_prefix = int8_prefix or fp16_prefix
         self.valid_k = _valid_k(device, prefix_tokens, query_block, _counts_key(self.layout))
         self.status = _status_word(device)
         n16, n8, n4 = route_counts(blocks * blocks, sparsity_ratio=sparsity, nvfp4_ratio=nvfp4, int8_ratio=int8,
@@ -349,7 +319,7 @@ class _Plan:
         shape = native.Shape(
             heads=heads, head_dim=dim, query_block=query_block, seq_tokens=tokens, prefix_tokens=prefix_tokens,
             video_blocks=blocks, has_nvfp4=int("nvfp4" in active), has_int8=int("int8" in active),
-            has_fp16=2 if fp16_prefix else int("fp16" in active), has_prefix_query_int8=int(int8_prefix),
+            has_fp16=int("fp16" in active), has_prefix_query_int8=int(self.native_prefix),
             has_maxpool=int(maxpool_weight != 0.0), input_is_bf16=int(dtype == torch.bfloat16),
             q_global_scale=1.0, k_global_scale=1.0, v_global_scale=1.0)
         lib = native.library()

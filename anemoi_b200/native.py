@@ -62,10 +62,6 @@ class Shape(C.Structure):
             return 0
         return math.ceil(self.prefix_tokens / self.query_block)
 
-    @property
-    def prefix_fp16_tiles(self) -> int:
-        return math.ceil(self.prefix_tokens / self.query_block) if self.has_fp16 == 2 else 0
-
 
 class Operands(C.Structure):
     _fields_ = [(name, C.c_void_p) for name in (
@@ -397,7 +393,7 @@ def attention(shape: Shape, store: OperandStore, lists: RouteLists, valid_k: tor
 def prefix_attention(shape: Shape, store: OperandStore, valid_k: torch.Tensor,
                      status: torch.Tensor) -> torch.Tensor:
     dev = valid_k.device
-    rows = (shape.prefix_query_tiles + shape.prefix_fp16_tiles) * shape.query_block
+    rows = shape.prefix_query_tiles * shape.query_block
     out = torch.empty((shape.heads, rows, shape.head_dim), dtype=torch.float16, device=dev)
     _count("prefix_attention", 1)
     _check(library().anemoi_sm100_prefix_attention(

@@ -38,7 +38,7 @@ typedef struct anemoi_sm100_shape {
   int32_t video_blocks;     /* R = frames * blocks per frame */
   int32_t has_nvfp4;        /* cells that need operands (video phases + prefix phase) */
   int32_t has_int8;
-  int32_t has_fp16;         /* 2: and prefix queries run through this cell (not with has_prefix_query_int8) */
+  int32_t has_fp16;
   int32_t has_prefix_query_int8; /* prefix queries run through the INT8 cell */
   int32_t has_maxpool;          /* 1: max pools in the extra pool slots; 2: second moments (diag-Jensen) */
   int32_t input_is_bf16;    /* raw Q/K/V dtype: 1 bf16, 0 fp16 */
@@ -54,7 +54,7 @@ typedef struct anemoi_sm100_shape {
  * ready operand.  Pointers of inactive cells may be null.  Sizes in bytes come
  * from anemoi_sm100_operand_bytes(). */
 typedef struct anemoi_sm100_operands {
-  void* q_fp16;     /* [H][R] records: Q tile QBxD fp16; then, with has_fp16 == 2, [H][prefix query tiles] */
+  void* q_fp16;     /* [H][R] records: Q tile QBxD fp16 */
   void* kv_fp16;    /* [H][stages] records: K tile 64xD fp16 | V tile 64xD fp16 */
   void* q_int8;     /* [H][R + prefix query tiles] records: Q tile QBxD s8 */
   void* kv_int8;    /* [H][stages] records: K tile 64xD s8 | V tile Dx64 e4m3 */
@@ -241,7 +241,7 @@ int anemoi_sm100_attention_pairs(const anemoi_sm100_shape* shape, const anemoi_s
                                  int64_t list_capacity, const int32_t* valid_k, void* out_packed,
                                  int32_t* status, void* stream);
 
-/* Dense attention of the prefix query rows over every stage, in the INT8 or the FP16 cell.
+/* Dense INT8-cell attention of the prefix query rows over every stage.
  *   out_prefix   fp16 [H][prefix query tiles * QB][D]
  * Replaces sm120_q{64,128}_prefix_int8_attention_forward
  * (sm120/q64_attention_host.cu:410-544). */
@@ -277,7 +277,7 @@ int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan);
 /*   strides          as for anemoi_sm100_prepare
  *   nvfp4_scales     q, k, v tensor-level scales of this call, or null for the plan's
  *   prefix_out       prefix rows computed elsewhere on `side_stream` ([H][prefix_rows][D], the caller's
- *                    dtype if prefix_is_caller_dtype); null with has_prefix_query_int8, has_fp16 == 2 or without a prefix
+ *                    dtype if prefix_is_caller_dtype); null with has_prefix_query_int8 or without a prefix
  *   out              [S][H][D] contiguous, the input's dtype
  *   workspace        anemoi_sm100_layer_workspace_bytes() bytes, 256-byte aligned, free for reuse on
  *                    `stream` when the call returns
