@@ -124,6 +124,7 @@ struct AttnParams {
   int32_t* status;
   uint64_t wait_ns;  // limit of every mbarrier wait
   int dense_prefix;  // 1: prefix query tiles, INT8 cell over every stage
+  int prefix_tiles;  // prefix query tiles of such a launch
   int stages;        // 64-key stages per head
   int q_tiles_int8;  // records per head in q_int8 (R + prefix query tiles)
   int out_rows;      // rows per head in `out`
@@ -151,6 +152,8 @@ struct Shared {
   uint64_t qk_done;    // unwinding only
   WaitContext wc;
   int cnt[3], first_of[3];  // the tile's stages per phase, where each phase starts inside the list
+  // per block of the tile: which factors move O into the INT8, FP16 phase's domain (kStays: none), the domain at the end
+  int move[2][2], last[2];
   // which tile it is: read by the roles where they need it, or kept in registers from the start (kReread)
   volatile int head, block[2], tile_blocks;
   const int32_t* volatile list;
@@ -289,7 +292,7 @@ __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[16])
 }
 
 // O[row][c] *= (colf[c] when given, then) alpha, for all D columns of the thread's row, kCols at a time.  In that
-// order: a row whose first stage in a phase comes after its pair's has the two factors at two stages.
+// order: a row whose first stage in a phase comes after its partner's has the two factors at two stages.
 template <int D, int kCols>
 __device__ __forceinline__ void rescale_o(uint32_t tmem_row, float alpha, const float* colf) {
   const float2 alpha2 = make_float2(alpha, alpha);
@@ -583,6 +586,9 @@ __device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, i
   return ((int64_t)token * p.s.heads + head) * D;
 }
 
+constexpr int kStays = -1;  // in place of a block's factors: O stays in its domain
+__host__ __device__ constexpr int factor_sets(int cells, bool q64) { return cells == kAny && q64 ? 2 : 1; }
+
 template <int D, int CELLS, bool kQ64>
 __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -612,7 +618,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   // (prefix tiles of 64 rows also go in twos: both walk every stage)
   const bool twos = pairs || (kQ64 && p.dense_prefix);
   int tile_blocks =
-      twos && 2 * tile + 1 < (p.dense_prefix ? p.q_tiles_int8 - p.s.video_blocks : p.s.video_blocks) ? 2 : 1;
+      twos && 2 * tile + 1 < (p.dense_prefix ? p.prefix_tiles : p.s.video_blocks) ? 2 : 1;
   int block0 = twos ? 2 * tile : tile, block1 = block0 + 1;
 
   // ---- this tile's work list ----
@@ -654,8 +660,10 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
 
   uint8_t* q_smem = smem;
   uint8_t* ring = smem + p.q_region;
+  // (two sets of factors for the blocks of a pair, which may come from different phases)
+  constexpr int kFactors = factor_sets(CELLS, kQ64);
   float* colf = reinterpret_cast<float*>(ring + (size_t)p.ring_bytes);
-  Shared* b = reinterpret_cast<Shared*>(colf + D);
+  Shared* b = reinterpret_cast<Shared*>(colf + kFactors * D);
 
   if (warp == 0) {
     if (lane < kRing) {
@@ -697,6 +705,20 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     mbar_init_fence();
   } else if (warp < 5) {
     b->rec[kRing - 1][threadIdx.x - 32] = make_float2(-5.0e6f, 0.0f);  // before the first stage
+  } else if (kFactors == 2 && warp == 5 && lane < 2) {
+    // A block of a pair without a stage of a phase stays in its domain, and one without a phase before it has
+    // nothing to move, so that a block's result does not depend on its partner: two steps instead of one, or there
+    // and back, round differently.
+    bool has[3] = {false, true, false};  // prefix rows
+    if (!p.dense_prefix) {
+      const int32_t* n =
+          p.row_counts + ((int64_t)head * p.s.video_blocks + (lane < tile_blocks && lane ? block1 : block0)) * 4;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) has[c] = n[c] > 0;
+    }
+    b->move[lane][0] = has[0] && has[1] ? 0 : kStays;
+    b->move[lane][1] = has[2] && (has[0] || has[1]) ? (has[1] ? 0 : D) : kStays;
+    b->last[lane] = has[2] ? kF16 : has[1] ? kI8 : kNv;
   }
   // Query rows beyond QB (64-row tiles padded to the 128-row MMA shape) are never
   // initialised: rows are independent, their results stay in TMEM lanes nobody reads.
@@ -996,9 +1018,12 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
                                               : (prev_cell == kI8 ? vscale[row] * 0.0022326917f : 1.0f);
           const float to = cell == kI8 ? vscale[row] * 0.0022326917f : 1.0f;
           colf[row] = to == 0.0f ? 0.0f : from / to;
+          if (kFactors == 2) colf[D + row] = nv_dom;  // from NVFP4 into FP16 for a block without the phase between
         }
         asm volatile("bar.sync 5, 128;" ::: "memory");
       }
+      const int factors = kFactors == 2 && change ? b->move[row >= QB][cell - kI8] : 0;
+      const bool moves = change && (kFactors == 1 || factors != kStays);
       if (cell != kNv) {
         // Q into tensor memory.  Its columns are free: the INT8 phase's Q has been read when the record
         // that takes its place in shared memory arrives, the NVFP4 phase's scale factors below.
@@ -1024,13 +1049,13 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         const int at = g & (kRing - 1);
         wait<kRescaleRole>(&b->wc, &m_full[at], (g >> 3) & 1, 30);
         const float m_new = b->rec[at][row].x;
-        const bool first = change && i == 0;
+        const bool first = moves && i == 0;
         if (g > 0 && (first || __any_sync(0xffffffffu, m_new != m))) {
           const float alpha = ex2(m - m_new);
           // O may only be touched once the previous PV is complete
           wait<kRescaleRole>(&b->wc, &b->pv_done[(g - 1) & (kRing - 1)], ((g - 1) >> 3) & 1, 20);
           tc_fence_after_sync();
-          rescale_o<D, Regs<D, CELLS>::kRescaleColumns>(tmem_row, alpha, first ? colf : nullptr);
+          rescale_o<D, Regs<D, CELLS>::kRescaleColumns>(tmem_row, alpha, first ? colf + factors : nullptr);
           tc_fence_before_sync();
         }
         m = m_new;
@@ -1101,6 +1126,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     asm volatile("bar.sync 6, 256;" ::: "memory");
     if (live_warp) {
       tc_fence_after_sync();
+      if (kFactors == 2) last_cell = b->last[my_block];
       const float d = b->rec[1][row].x;
       const float inv = d > 0.0f ? 1.0f / d : 0.0f;
       const bool bf16 = p.tokens != nullptr && p.tokens_bf16;
@@ -1112,14 +1138,17 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         if (dst != nullptr) {
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
-            float f[8];
+            // (the channels' factors are loaded together: one by one under a condition that is not known to be the
+            // warp's, each is waited for, 3 us of a small call: 7 heads x 2,293 tokens, D = 128 65.3, now 62.1)
+            float f[8], factor[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              f[i] = __uint_as_float(r[j + i]);
-              if (last_cell == kNv) f[i] *= nv_dom;
-              if (last_cell == kI8) f[i] *= vscale[c0 + j + i] * 0.0022326917f;
-              f[i] *= inv;
+            for (int i = 0; i < 8; ++i) factor[i] = last_cell == kNv ? nv_dom : 1.0f;
+            if (last_cell == kI8) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) factor[i] = vscale[c0 + j + i] * 0.0022326917f;
             }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r[j + i]) * factor[i] * inv;
             uint4 v = make_uint4(f16x2(f[0], f[1]), f16x2(f[2], f[3]), f16x2(f[4], f[5]), f16x2(f[6], f[7]));
             if (bf16)
               v = make_uint4(bf16x2_of_f16x2(v.x), bf16x2_of_f16x2(v.y), bf16x2_of_f16x2(v.z), bf16x2_of_f16x2(v.w));
@@ -1192,7 +1221,7 @@ int launch(AttnParams& p, int tiles, cudaStream_t st) {
   // their code in the instruction cache.
   if (p.dense_prefix && (p.s.has_nvfp4 || p.s.has_fp16)) one = kAny;
   q_region = (q_region + 127) & ~127;
-  const int fixed = q_region + D * 4 + (int)sizeof(Shared);
+  const int fixed = q_region + factor_sets(one, kQ64) * D * 4 + (int)sizeof(Shared);
   // two CTAs per SM: measured limit is 115,528 bytes of dynamic shared memory per CTA
   const int budget = 115528;
   int ring = ((budget - fixed) / 128) * 128;
@@ -1341,6 +1370,7 @@ int prefix_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operand
   p.stages = rec::stages(*shape);
   const int blocks = rec::prefix_query_tiles(*shape);
   const int tiles = shape->query_block == 64 ? (blocks + 1) / 2 : blocks;
+  p.prefix_tiles = blocks;
   p.q_tiles_int8 = shape->video_blocks + blocks;
   p.out_rows = blocks * shape->query_block;
   set_rows(p, rows);

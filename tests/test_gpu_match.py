@@ -1,6 +1,7 @@
 """Q64 pairs chosen by what the blocks' lists share: bit for bit one block per CTA."""
 
 import ctypes as C
+import math
 
 import pytest
 import torch
@@ -70,3 +71,65 @@ def test_chosen_pairs_equal_one_block_per_cta(native_library, blocks, heads, dim
 def test_where_pairs_are_chosen(native_library, blocks, heads, cells, chosen):
     q = torch.empty((1, 1, 1, 1), device="cuda", dtype=torch.bfloat16).expand(1, blocks * 64, heads, 64)
     assert _chosen(native_library, q, _options(blocks, 0, cells, 0.8)) == chosen
+
+
+def _two_kinds(blocks, heads, dim, first_peaked, columns):
+    """Q/K/V in which every other block of queries has half its weight on one block of keys, or nearly all of it on two (of the
+    second less), and the others attend to all blocks about alike."""
+    gen = torch.Generator(device="cuda").manual_seed(blocks + heads)
+    # (orthogonal: the shares are what is asked for)
+    u = torch.linalg.qr(torch.randn(heads, dim, dim, generator=gen, device="cuda"))[0][:, :blocks]
+    u = u.permute(1, 0, 2)[:, None] * dim ** 0.5
+    q = 0.3 * torch.randn(blocks, 64, heads, dim, generator=gen, device="cuda")
+    for i in range(0 if first_peaked else 1, blocks, 2):
+        for c in range(columns):
+            q[i] += (math.log(blocks) if columns == 1 else 16.0 - 0.5 * c) * dim ** -0.5 * u[(i * 7 + c * 5) % blocks]
+    k = u + 0.3 * torch.randn(blocks, 64, heads, dim, generator=gen, device="cuda")
+    v = torch.randn(blocks, 64, heads, dim, generator=gen, device="cuda")
+    return tuple(t.reshape(1, blocks * 64, heads, dim).to(torch.float16) for t in (q, k, v))
+
+
+@pytest.mark.parametrize("first_peaked", [True, False])
+@pytest.mark.parametrize("columns, int8, fp16, without, partner", [
+    (2, 16, 0, (16, 0, 0), (14, 2, 0)),      # no INT8 phase, NVFP4 before it
+    (1, 128, 8, (15, 0, 1), (0, 16, 0)),     # no middle phase: three cells
+    (2, 8, 8, (16, 0, 0), (14, 1, 1)),       # the first phase alone
+])
+@pytest.mark.parametrize("dim", [64, 128])
+def test_rows_do_not_depend_on_the_phases_of_the_other_block(native_library, dim, first_peaked, columns, int8, fp16,
+                                                             without, partner):
+    """Pairs in which a block has no stage of a phase that its partner has: bit for bit one block per CTA."""
+    from anemoi_b200 import executor
+
+    blocks, heads = 16, 6
+    q, k, v = _two_kinds(blocks, heads, dim, first_peaked, columns)
+    int8, fp16 = int8 / blocks ** 2, fp16 / blocks ** 2
+    kw = _options(blocks, 0, (1.0 - int8 - fp16, int8, fp16), 0.0)
+    kw.update(layer=0, nvfp4_scales=(0.01, 0.01, 0.002))
+    paired, parts = executor.sm100_ragged_attention(q, k, v, return_parts=True, **kw)
+    own = parts["lists"].row_counts[..., :3].cpu()
+    kinds = [tuple(own[0, i].tolist()) for i in (0, 1)]
+    assert set(kinds) == {without, partner}, kinds
+    assert all(tuple(own[h, i].tolist()) == kinds[i % 2] for h in range(heads) for i in range(blocks))
+    called = executor.sm100_ragged_attention(q, k, v, **kw)
+    executor._PAIR_Q64 = False
+    try:
+        single = executor.sm100_ragged_attention(q, k, v, **kw)
+    finally:
+        executor._PAIR_Q64 = True
+    assert torch.isfinite(single).all()
+    assert torch.equal(paired, single) and torch.equal(called, single)
+
+
+def test_heads_alone_equal_one_call_with_chosen_pairs(native_library):
+    """The whole call chooses its pairs, a head alone takes neighbours; every block of one kind has no INT8 phase."""
+    from anemoi_b200 import executor
+
+    blocks, heads = 128, 10
+    q, k, v = _two_kinds(blocks, heads, 128, True, 1)
+    kw = _options(blocks, 0, (63.5 / 128, 64 / 128, 0.5 / 128), 0.0)
+    assert _chosen(native_library, q, kw) == 1 and _chosen(native_library, q[:, :, :1], kw) == 0
+    kw.update(layer=0, nvfp4_scales=(0.01, 0.01, 0.002))
+    whole = executor.sm100_ragged_attention(q, k, v, **kw)
+    for h in range(heads):
+        assert torch.equal(whole[:, :, h:h + 1], executor.sm100_ragged_attention(*(t[:, :, h:h + 1] for t in (q, k, v)), **kw))
