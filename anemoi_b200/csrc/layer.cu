@@ -2,9 +2,10 @@
 // prefix attention, with the results written straight to their tokens.
 //
 // A small call is bound by its launches, not by its kernels: with one Python wrapper, allocation and
-// marshaling per stage the 1,024-token call takes 210 us, here 19.5 (all of them host time).  The host work
-// is one function: one workspace cut up by offsets, three to eight kernels (routing is one for most shapes, and forms
-// the draft map of short calls; the output needs no assembly pass), programmatic dependent launches between them.
+// marshaling per stage the 1,024-token call takes 210 us, here 19.5 (host work and kernels are about as
+// long, call behind call).  The host work is one function: one workspace cut up by offsets, three to twelve kernels
+// (up to eight where routing is one, which it is for most shapes, forming the draft map of short calls, too; the output
+// needs no assembly pass), programmatic dependent launches between them.
 //
 // Order of the launches.  The prefix rows' tiles walk every stage of the head: few CTAs, each as
 // long as the whole video launch of a small call, so they start on the side stream as soon as the

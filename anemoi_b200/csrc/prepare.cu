@@ -643,6 +643,22 @@ inline bool own_maxima(const anemoi_sm100_shape& s) {
          ((int64_t)s.video_blocks + rec::prefix_stages(s)) * s.heads <= 148;
 }
 
+// The grid of the kernel of the maxima: about three CTAs per SM, each with at least sixteen loads per thread: every CTA
+// ends in 256 atomics (8 heads x 4,109 tokens with eight per SM and two loads: the preparation took 40 us, now 24).
+inline int maxima_chunks(const anemoi_sm100_shape& s) { return (s.heads * s.head_dim / 8 + 31) / 32; }
+inline int maxima_tokens(const anemoi_sm100_shape& s) {
+  const int rows = max(1, 3 * 148 / maxima_chunks(s));
+  return max(16 * kAmaxLanes, (s.seq_tokens + rows - 1) / rows);
+}
+// Up to eight token ranges are one cluster, which needs no zeroed memory: a launch less, and nothing
+// between this kernel and what was before it (1,024 tokens x 4 heads: the call 36.5 -> 34.4 us).
+inline bool zeroes_maxima(const anemoi_sm100_shape& s) {
+  return s.has_int8 && !own_maxima(s) && (s.seq_tokens + maxima_tokens(s) - 1) / maxima_tokens(s) > 8;
+}
+// Beside prefix rows that the library computes on another stream, with a memset: its wait lets their few long CTAs in
+// first, each on an SM of its own; 5 heads x 19,425 tokens with 62 of prefix 494 us, with the kernel 628.
+inline bool zeroes_by_memset(const anemoi_sm100_shape& s) { return s.prefix_tokens > 0 && !s.has_prefix_query_int8; }
+
 template <typename InT, int QB, int D, bool kSplit, bool kOwnMaxima, Cells kCells>
 int launch(const PrepParams& p, cudaStream_t stream) {
   const size_t smem = (size_t)QB * (D + kPad) * sizeof(__half);
@@ -651,24 +667,16 @@ int launch(const PrepParams& p, cudaStream_t stream) {
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
   if (p.s.has_int8 && !kOwnMaxima) {
-    const int chunks = (p.s.heads * D / 8 + 31) / 32;
-    // about three CTAs per SM, each with at least sixteen loads per thread: every CTA ends in 256 atomics
-    // (8 heads x 4,109 tokens with eight per SM and two loads: the preparation took 40 us, now 24)
-    const int rows = max(1, 3 * 148 / chunks);
-    const int tokens_per_block = max(16 * kAmaxLanes, (p.s.seq_tokens + rows - 1) / rows);
-    dim3 grid(chunks, (p.s.seq_tokens + tokens_per_block - 1) / tokens_per_block);
-    // Up to eight token ranges are one cluster, which needs no zeroed memory: a launch less, and nothing
-    // between this kernel and what was before it (1,024 tokens x 4 heads: the call 36.5 -> 34.4 us).
+    const int tokens_per_block = maxima_tokens(p.s);
+    dim3 grid(maxima_chunks(p.s), (p.s.seq_tokens + tokens_per_block - 1) / tokens_per_block);
     cudaError_t err;
-    if (grid.y <= 8) {
+    if (!zeroes_maxima(p.s)) {
       err = layer::launch_cluster(v_amax_kernel<InT, true>, grid, dim3(1, grid.y), dim3(32 * kAmaxLanes), 0, stream,
                                   static_cast<const InT*>(p.v), reinterpret_cast<int*>(p.o.v_amax), p.s.seq_tokens,
                                   p.s.heads, D / 8, p.stride[4], p.stride[5], tokens_per_block);
     } else {
       const int n = p.s.heads * D;
-      // (beside prefix rows that the library computes on another stream, the memset: its wait lets their few long CTAs in
-      // first, each on an SM of its own; 5 heads x 19,425 tokens with 62 of prefix 494 us, with the kernel 628)
-      if (p.s.prefix_tokens > 0 && !p.s.has_prefix_query_int8)
+      if (zeroes_by_memset(p.s))
         err = cudaMemsetAsync(p.o.v_amax, 0, sizeof(float) * n, stream);
       else
         err = layer::launch(zero_kernel, dim3(min(148, (n + kZeroThreads - 1) / kZeroThreads)), dim3(kZeroThreads), 0, stream,
@@ -694,6 +702,10 @@ extern "C" int anemoi_sm100_arch(void) { return 100; }
 
 extern "C" int anemoi_sm100_prepare_kernels(const anemoi_sm100_shape* shape) {
   return rec::validate_shape(shape) == ANEMOI_SM100_OK ? 1 + (shape->has_int8 && !own_maxima(*shape)) : 0;
+}
+
+extern "C" int anemoi_sm100_prepare_zero_kernels(const anemoi_sm100_shape* shape) {
+  return rec::validate_shape(shape) == ANEMOI_SM100_OK && zeroes_maxima(*shape) && !zeroes_by_memset(*shape);
 }
 
 extern "C" int64_t anemoi_sm100_operand_bytes(const anemoi_sm100_shape* s, int which) {

@@ -336,8 +336,8 @@ class _Plan:
         self.side = _prefix_stream(device) if prefix_tokens else None
         self.side_handle = self.side.cuda_stream if prefix_tokens else None
         self.uses_scales = "nvfp4" in active
-        # kernels per call: preparation (with V's maxima), draft, routing (and pair lists), attention, prefix rows
-        self.launches = 3 + lib.anemoi_sm100_prepare_kernels(C.byref(shape)) + int(prefix_tokens > 0)
+        # kernels per call: preparation (with V's maxima and their zeroes), draft, routing (and pair lists), attention, prefix rows
+        self.launches = 3 + native.prepare_launches(shape) + int(prefix_tokens > 0)
         self.launches -= lib.anemoi_sm100_drafts_in_routing(C.byref(shape))
         matched = lib.anemoi_sm100_matches_pairs(self.ref)
         self.launches += matched

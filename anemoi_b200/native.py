@@ -111,6 +111,7 @@ def library() -> C.CDLL:
         "anemoi_sm100_routes_in_one_kernel": (C.c_int, [SP]),
         "anemoi_sm100_drafts_in_routing": (C.c_int, [SP]),
         "anemoi_sm100_prepare_kernels": (C.c_int, [SP]),
+        "anemoi_sm100_prepare_zero_kernels": (C.c_int, [SP]),
         "anemoi_sm100_layer_workspace_bytes": (I64, [C.POINTER(LayerPlan)]),
         "anemoi_sm100_matches_pairs": (C.c_int, [C.POINTER(LayerPlan)]),
         "anemoi_sm100_layer": (C.c_int, [C.POINTER(LayerPlan), P, P, P, C.POINTER(I64), C.POINTER(F), P, I64, C.c_int,
@@ -157,6 +158,7 @@ EXPORTED = (
     "anemoi_sm100_attention_pairs", "anemoi_sm100_pair_lists", "anemoi_sm100_route_pairs",
     "anemoi_sm100_layer", "anemoi_sm100_layer_workspace_bytes", "anemoi_sm100_routes_in_one_kernel",
     "anemoi_sm100_drafts_in_routing", "anemoi_sm100_matches_pairs", "anemoi_sm100_prepare_kernels",
+    "anemoi_sm100_prepare_zero_kernels",
     "anemoi_sm100_route_anchored", "anemoi_sm100_route_anchored_scratch_bytes",
     "anemoi_sm100_prefix_attention", "anemoi_sm100_assemble", "anemoi_sm100_pack_qkv",
     "anemoi_sm100_merge_heads", "anemoi_sm100_pack_qkv_heads", "anemoi_sm100_merge_heads_into",
@@ -233,10 +235,16 @@ def allocate_operands(shape: Shape, device) -> OperandStore:
     return OperandStore(shape=shape, buffers=buffers, struct=struct)
 
 
+def prepare_launches(shape: Shape) -> int:
+    """Kernels of a preparation: (the maxima's zeroes, the maxima of V,) the fused pass."""
+    lib = library()
+    return lib.anemoi_sm100_prepare_kernels(C.byref(shape)) + lib.anemoi_sm100_prepare_zero_kernels(C.byref(shape))
+
+
 def prepare(shape: Shape, q, k, v, indices, counts, store: OperandStore) -> None:
     """Fill the operand store from raw ``[1, S, H, D]`` Q/K/V views (see anemoi_sm100_prepare)."""
     strides = (C.c_int64 * 6)(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2))
-    _count("prepare", library().anemoi_sm100_prepare_kernels(C.byref(shape)))  # (V amax pre-pass,) fused pass
+    _count("prepare", prepare_launches(shape))
     _check(library().anemoi_sm100_prepare(C.byref(shape), _ptr(q), _ptr(k), _ptr(v), strides,
                                           _ptr(indices), _ptr(counts), C.byref(store.struct),
                                           _stream(q.device)), "anemoi_sm100_prepare")

@@ -100,6 +100,8 @@ int anemoi_sm100_prepare(const anemoi_sm100_shape* shape, const void* q, const v
 /* Kernels of one such call, but for the one that zeroes memory: two, or one where there is no INT8 or the sequence is
  * short. */
 int anemoi_sm100_prepare_kernels(const anemoi_sm100_shape* shape);
+/* 1 if a kernel zeroes memory in front of them, 0 if nothing or a memset does. */
+int anemoi_sm100_prepare_zero_kernels(const anemoi_sm100_shape* shape);
 
 /* Pooled-QK row softmax -> fp16 probability [H][R][R]; with 0 < w < 1 the mean
  * and max maps are blended, w == 1 uses the max pools only.  Key pools are 16-byte
