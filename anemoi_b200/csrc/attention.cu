@@ -1352,6 +1352,16 @@ extern "C" int anemoi_sm100_attention_pairs(const anemoi_sm100_shape* shape,
                          list_capacity, valid_k, out_packed, nullptr, status, stream);
 }
 
+extern "C" int anemoi_sm100_attention_matched(const anemoi_sm100_shape* shape, const anemoi_sm100_operands* ops,
+                                              const int32_t* row_offset, const int32_t* row_counts,
+                                              const int32_t* pair_table, const int32_t* pair_ids, int64_t list_capacity,
+                                              const int32_t* valid_k, void* out_packed, int32_t* status, void* stream) {
+  if (!pair_table || reinterpret_cast<uintptr_t>(pair_table) % 16 || !pair_ids || !shape || shape->query_block != 64)
+    return ANEMOI_SM100_EINVAL;
+  return video_attention(shape, ops, row_offset, row_counts, nullptr, nullptr, pair_ids, list_capacity, valid_k, out_packed,
+                         nullptr, status, stream, pair_table);
+}
+
 namespace {
 int prefix_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operands* ops, const int32_t* valid_k,
                      void* out_prefix, const TokenRows* rows, int32_t* status, void* stream) {

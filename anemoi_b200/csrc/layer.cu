@@ -55,6 +55,29 @@ bool matches(const anemoi_sm100_layer_plan& p) {
          stages >= (cells > 1 ? kMatchStagesMixed : kMatchStages);
 }
 
+layer::PairBits pair_bits(const anemoi_sm100_layer_plan& p, uint32_t* words) {
+  const int64_t budget[3] = {p.n4, p.n8, p.n16};
+  layer::PairBits bits = {words, 0, {}};
+  for (int c = 0; c < 3; ++c) bits.slot[c] = budget[c] > 0 ? bits.phases++ : -1;
+  return bits;
+}
+int64_t pair_bits_bytes(const anemoi_sm100_layer_plan& p) {
+  const int64_t H = p.shape.heads, R = p.shape.video_blocks;
+  return H * pair_bits(p, nullptr).phases * R * layer::pair_bit_words(R) * 4;
+}
+
+// Routing and the chosen pairs' lists.
+int route_matched(const anemoi_sm100_layer_plan& p, const void* probability, void* scratch, int32_t* row_offset,
+                  int32_t* row_counts, const layer::PairBits& bits, int32_t* table, int32_t* pair_ids, cudaStream_t st) {
+  const anemoi_sm100_shape& s = p.shape;
+  const int phase = s.prefix_tokens > 0 || p.prefix_phase < 0 || p.prefix_phase > 2 ? p.prefix_phase : -1;
+  const int code = layer::route_bits(s, probability, p.n16, p.n8, p.n4, phase, scratch, row_offset, row_counts, bits,
+                                     p.list_capacity, st);
+  return code != ANEMOI_SM100_OK ? code
+                                 : layer::match_pairs(s, bits, phase, row_offset, row_counts, table, pair_ids,
+                                                      p.list_capacity, p.status, st);
+}
+
 // Cuts `base` (null: only the size is wanted) into the call's buffers.
 Workspace cut(const anemoi_sm100_layer_plan& p, uint8_t* base) {
   const anemoi_sm100_shape& s = p.shape;
@@ -92,9 +115,7 @@ Workspace cut(const anemoi_sm100_layer_plan& p, uint8_t* base) {
   // (routed in one kernel, the pairs need neither the blocks' own lists nor scratch)
   if (!fused && !matched) w.stage_ids = reinterpret_cast<int32_t*>(take(list));
   if (matched) {
-    const int64_t budget[3] = {p.n4, p.n8, p.n16};
-    for (int c = 0; c < 3; ++c) w.pair_bits.slot[c] = budget[c] > 0 ? w.pair_bits.phases++ : -1;
-    w.pair_bits.words = reinterpret_cast<uint32_t*>(take(H * w.pair_bits.phases * R * layer::pair_bit_words(R) * 4));
+    w.pair_bits = pair_bits(p, reinterpret_cast<uint32_t*>(take(pair_bits_bytes(p))));
     w.pair_table = reinterpret_cast<int32_t*>(take(H * ((R + 1) / 2) * 32));
   } else if (pairs) {
     w.pair_counts = reinterpret_cast<int32_t*>(take(H * ((R + 1) / 2) * 16));
@@ -125,6 +146,25 @@ extern "C" int anemoi_sm100_drafts_in_routing(const anemoi_sm100_shape* shape) {
 
 extern "C" int anemoi_sm100_matches_pairs(const anemoi_sm100_layer_plan* plan) {
   return valid(plan) && plan->pair_q64 && plan->shape.query_block == 64 && matches(*plan);
+}
+
+extern "C" int64_t anemoi_sm100_pair_bits_bytes(const anemoi_sm100_layer_plan* plan) {
+  return anemoi_sm100_matches_pairs(plan) ? pair_bits_bytes(*plan) : ANEMOI_SM100_EINVAL;
+}
+
+extern "C" int anemoi_sm100_route_matched(const anemoi_sm100_layer_plan* plan, const void* probability, void* scratch,
+                                          int64_t scratch_bytes, int32_t* row_offset, int32_t* row_counts, void* bits,
+                                          int32_t* pair_table, int32_t* pair_ids, void* stream) {
+  if (!anemoi_sm100_matches_pairs(plan) || !probability || !row_offset || !row_counts || !bits || !pair_table || !pair_ids)
+    return ANEMOI_SM100_EINVAL;
+  // (read 16 bytes at a time)
+  if ((reinterpret_cast<uintptr_t>(row_counts) | reinterpret_cast<uintptr_t>(bits) |
+       reinterpret_cast<uintptr_t>(pair_table)) % 16)
+    return ANEMOI_SM100_EINVAL;
+  if (!scratch || scratch_bytes < anemoi_sm100_route_scratch_bytes(&plan->shape)) return ANEMOI_SM100_EINVAL;
+  return route_matched(*plan, probability, scratch, row_offset, row_counts,
+                       pair_bits(*plan, static_cast<uint32_t*>(bits)), pair_table, pair_ids,
+                       static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan) {
@@ -185,12 +225,7 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
                                           p.maxpool_weight, w.prob, stream);
     if (code != ANEMOI_SM100_OK) return done(code);
     if (w.pair_table != nullptr) {
-      const int phase = s.prefix_tokens > 0 || p.prefix_phase < 0 || p.prefix_phase > 2 ? p.prefix_phase : -1;
-      code = layer::route_bits(s, w.prob, p.n16, p.n8, p.n4, phase, w.scratch, w.row_offset, w.row_counts,
-                               w.pair_bits, p.list_capacity, st);
-      if (code == ANEMOI_SM100_OK)
-        code = layer::match_pairs(s, w.pair_bits, phase, w.row_offset, w.row_counts, w.pair_table, w.pair_ids,
-                                  p.list_capacity, p.status, st);
+      code = route_matched(p, w.prob, w.scratch, w.row_offset, w.row_counts, w.pair_bits, w.pair_table, w.pair_ids, st);
     } else if (pair_counts != nullptr && layer::routes_pairs(s)) {
       code = anemoi_sm100_route_pairs(&s, w.prob, p.n16, p.n8, p.n4, p.prefix_phase, w.row_offset, w.row_counts,
                                       w.pair_counts, w.pair_ids, p.list_capacity, stream);

@@ -29,7 +29,8 @@ _STAGE_EVENTS: list | None = None
 
 
 def collect_stage_events(enable: bool) -> None:
-    """Start (or stop) recording CUDA events around each native stage of later calls."""
+    """Start (or stop) recording CUDA events around each native stage of later calls.  The stages are those of the one
+    call, launched one by one (without ``return_parts``, which pairs Q64 blocks by index)."""
     global _STAGE_EVENTS
     _STAGE_EVENTS = [] if enable else None
 
@@ -276,12 +277,25 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
                                    int8_ratio=float(retained_int8_ratio),
                                    fp16_ratio=float(retained_fp16_ratio))
         phase_index = -1 if prefix_phase is None else PHASE_ORDER.index(prefix_phase)
+        # Q64: two query blocks per CTA fill the 128-row MMA shape and walk the union of their lists: the pairs of
+        # the one call, neighbours where it has none or where the blocks' own lists are wanted
+        plan = None
+        if query_block_size == 64 and _PAIR_Q64 and not (return_parts or diag_jensen or enable_anchors):
+            plan = _plan(device, q_bshd.size(1), q_bshd.size(2), q_bshd.size(3), q_bshd.dtype, prefix_tokens,
+                         float(sparsity_ratio), float(retained_nvfp4_ratio), float(retained_int8_ratio),
+                         float(retained_fp16_ratio), video_shape, query_block_size, prefix_kv_precision,
+                         prefix_query_precision, float(maxpool_weight), True)
+        pairs = None
         with _Stage("route"):
-            lists = (native.route_anchored(shape, prob, n16, n8, n4, phase_index, layout.anchors, layout.anchor_ids)
-                     if enable_anchors else native.route(shape, prob, n16, n8, n4, phase_index))
+            if plan is not None and plan.matched:
+                lists, pairs = native.route_matched(plan.struct, prob)
+            elif enable_anchors:
+                lists = native.route_anchored(shape, prob, n16, n8, n4, phase_index, layout.anchors, layout.anchor_ids)
+            else:
+                lists = native.route(shape, prob, n16, n8, n4, phase_index)
     with _Stage("attention"), _Range("anemoi.mpa_mainloop", nvtx):
-        # Q64: two query blocks per CTA fill the 128-row MMA shape and walk the union of their lists
-        pairs = native.pair_lists(shape, lists) if query_block_size == 64 and _PAIR_Q64 else None
+        if pairs is None and query_block_size == 64 and _PAIR_Q64:
+            pairs = native.pair_lists(shape, lists)
         packed = native.attention(shape, store, lists, valid_k, status, pairs)
 
     current.wait_stream(side)
@@ -339,10 +353,10 @@ class _Plan:
         # kernels per call: preparation (with V's maxima and their zeroes), draft, routing (and pair lists), attention, prefix rows
         self.launches = 3 + native.prepare_launches(shape) + int(prefix_tokens > 0)
         self.launches -= lib.anemoi_sm100_drafts_in_routing(C.byref(shape))
-        matched = lib.anemoi_sm100_matches_pairs(self.ref)
-        self.launches += matched
+        self.matched = lib.anemoi_sm100_matches_pairs(self.ref)
+        self.launches += self.matched
         if not lib.anemoi_sm100_routes_in_one_kernel(C.byref(shape)):
-            self.launches += 4 + 2 * int(pair_q64 and query_block == 64 and not matched)
+            self.launches += 4 + 2 * int(pair_q64 and query_block == 64 and not self.matched)
         self.call = lib.anemoi_sm100_layer
 
 

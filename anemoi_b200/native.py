@@ -114,6 +114,9 @@ def library() -> C.CDLL:
         "anemoi_sm100_prepare_zero_kernels": (C.c_int, [SP]),
         "anemoi_sm100_layer_workspace_bytes": (I64, [C.POINTER(LayerPlan)]),
         "anemoi_sm100_matches_pairs": (C.c_int, [C.POINTER(LayerPlan)]),
+        "anemoi_sm100_pair_bits_bytes": (I64, [C.POINTER(LayerPlan)]),
+        "anemoi_sm100_route_matched": (C.c_int, [C.POINTER(LayerPlan), P, P, I64, P, P, P, P, P, P]),
+        "anemoi_sm100_attention_matched": (C.c_int, [SP, OP, P, P, P, P, I64, P, P, P, P]),
         "anemoi_sm100_layer": (C.c_int, [C.POINTER(LayerPlan), P, P, P, C.POINTER(I64), C.POINTER(F), P, I64, C.c_int,
                                          P, P, I64, P, P]),
         "anemoi_sm100_copy_rows": (C.c_int, [P, I64, P, I64, I64, I64, I32, P]),
@@ -158,7 +161,8 @@ EXPORTED = (
     "anemoi_sm100_attention_pairs", "anemoi_sm100_pair_lists", "anemoi_sm100_route_pairs",
     "anemoi_sm100_layer", "anemoi_sm100_layer_workspace_bytes", "anemoi_sm100_routes_in_one_kernel",
     "anemoi_sm100_drafts_in_routing", "anemoi_sm100_matches_pairs", "anemoi_sm100_prepare_kernels",
-    "anemoi_sm100_prepare_zero_kernels",
+    "anemoi_sm100_prepare_zero_kernels", "anemoi_sm100_pair_bits_bytes", "anemoi_sm100_route_matched",
+    "anemoi_sm100_attention_matched",
     "anemoi_sm100_route_anchored", "anemoi_sm100_route_anchored_scratch_bytes",
     "anemoi_sm100_prefix_attention", "anemoi_sm100_assemble", "anemoi_sm100_pack_qkv",
     "anemoi_sm100_merge_heads", "anemoi_sm100_pack_qkv_heads", "anemoi_sm100_merge_heads_into",
@@ -377,14 +381,48 @@ def pair_lists(shape: Shape, lists: RouteLists) -> PairLists:
     return pairs
 
 
+@dataclass
+class MatchedPairs:
+    """Union lists of the pairs that a plan's call chooses (any two Q64 query blocks of a head)."""
+    pair_table: torch.Tensor   # int32 [H, ceil(R/2), 8], launch order: blocks, start, stages, stages per phase
+    pair_ids: torch.Tensor     # int32 [H, capacity]: stage id | membership bits 30 (first block), 31 (second)
+
+
+def route_matched(plan: LayerPlan, prob: torch.Tensor) -> tuple[RouteLists, MatchedPairs]:
+    """Routing of a plan whose pairs are chosen, as its one call runs it (no lists of single blocks)."""
+    lib, shape, dev = library(), plan.shape, prob.device
+    h, r = shape.heads, shape.video_blocks
+    scratch, bits = (torch.empty(int(n), dtype=torch.uint8, device=dev) for n in (
+        lib.anemoi_sm100_route_scratch_bytes(C.byref(shape)), lib.anemoi_sm100_pair_bits_bytes(C.byref(plan))))
+    lists = RouteLists(
+        row_offset=torch.empty((h, r), dtype=torch.int32, device=dev),
+        row_counts=torch.empty((h, r, 4), dtype=torch.int32, device=dev),
+        stage_ids=torch.empty((h, 0), dtype=torch.int32, device=dev), capacity=plan.list_capacity)
+    pairs = MatchedPairs(
+        pair_table=torch.empty((h, (r + 1) // 2, 8), dtype=torch.int32, device=dev),
+        pair_ids=torch.empty((h, plan.list_capacity), dtype=torch.int32, device=dev))
+    # one kernel, or hist, threshold, rowstat, headscan, bits; the choice
+    _count("route", 2 if lib.anemoi_sm100_routes_in_one_kernel(C.byref(shape)) else 6)
+    _check(lib.anemoi_sm100_route_matched(
+        C.byref(plan), _ptr(prob), _ptr(scratch), scratch.numel(), _ptr(lists.row_offset), _ptr(lists.row_counts),
+        _ptr(bits), _ptr(pairs.pair_table), _ptr(pairs.pair_ids), _stream(dev)), "anemoi_sm100_route_matched")
+    return lists, pairs
+
+
 def attention(shape: Shape, store: OperandStore, lists: RouteLists, valid_k: torch.Tensor,
-              status: torch.Tensor, pairs: PairLists | None = None) -> torch.Tensor:
+              status: torch.Tensor, pairs: PairLists | MatchedPairs | None = None) -> torch.Tensor:
     """The video query blocks' attention.  With ``pairs`` (Q64) two query blocks share a CTA and
     walk the union of their lists; the result is the same."""
     dev = valid_k.device
     out = torch.empty((shape.heads, shape.video_blocks * shape.query_block, shape.head_dim),
                       dtype=torch.float16, device=dev)
     _count("attention", 1)
+    if isinstance(pairs, MatchedPairs):
+        _check(library().anemoi_sm100_attention_matched(
+            C.byref(shape), C.byref(store.struct), _ptr(lists.row_offset), _ptr(lists.row_counts),
+            _ptr(pairs.pair_table), _ptr(pairs.pair_ids), lists.capacity, _ptr(valid_k), _ptr(out),
+            _ptr(status), _stream(dev)), "anemoi_sm100_attention_matched")
+        return out
     if pairs is not None:
         _check(library().anemoi_sm100_attention_pairs(
             C.byref(shape), C.byref(store.struct), _ptr(lists.row_offset), _ptr(lists.row_counts),

@@ -275,6 +275,20 @@ typedef struct anemoi_sm100_layer_plan {
 /* 1 if the plan's Q64 blocks are paired by what their lists share (a launch for the choice) rather than by
  * index, 0 if not. */
 int anemoi_sm100_matches_pairs(const anemoi_sm100_layer_plan* plan);
+/* The stages of such a plan by themselves: routing with the choice of the pairs, and attention on them.
+ *   bits         scratch of anemoi_sm100_pair_bits_bytes() bytes
+ *   pair_table   [H][ceil(R/2)][8] in launch order: first block, second (-1: none), start of the list in a head's
+ *                pair_ids, its stages, those of each phase
+ *   pair_ids     [H][list_capacity] as from pair_lists (bit 30: first block, bit 31: second)
+ * row_counts, bits and pair_table on 16 bytes.  Refused where anemoi_sm100_matches_pairs() is 0. */
+int64_t anemoi_sm100_pair_bits_bytes(const anemoi_sm100_layer_plan* plan);
+int anemoi_sm100_route_matched(const anemoi_sm100_layer_plan* plan, const void* probability, void* scratch,
+                               int64_t scratch_bytes, int32_t* row_offset, int32_t* row_counts, void* bits,
+                               int32_t* pair_table, int32_t* pair_ids, void* stream);
+int anemoi_sm100_attention_matched(const anemoi_sm100_shape* shape, const anemoi_sm100_operands* ops,
+                                   const int32_t* row_offset, const int32_t* row_counts, const int32_t* pair_table,
+                                   const int32_t* pair_ids, int64_t list_capacity, const int32_t* valid_k,
+                                   void* out_packed, int32_t* status, void* stream);
 int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan);
 /*   strides          as for anemoi_sm100_prepare
  *   nvfp4_scales     q, k, v tensor-level scales of this call, or null for the plan's

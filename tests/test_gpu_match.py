@@ -133,3 +133,27 @@ def test_heads_alone_equal_one_call_with_chosen_pairs(native_library):
     whole = executor.sm100_ragged_attention(q, k, v, **kw)
     for h in range(heads):
         assert torch.equal(whole[:, :, h:h + 1], executor.sm100_ragged_attention(*(t[:, :, h:h + 1] for t in (q, k, v)), **kw))
+
+
+@pytest.mark.parametrize("blocks, heads, prefix, cells, counted", [
+    (129, 64, 37, (0.4, 0.4, 0.2), 2),
+    (1025, 1, 0, (0.0, 1.0, 0.0), 6),      # routing in several kernels
+    (64, 2, 0, (0.0, 1.0, 0.0), 1),        # neighbours
+])
+def test_stages_take_the_pairs_of_the_call(native_library, blocks, heads, prefix, cells, counted):
+    """Stage by stage (NVTX ranges, stage events) a call walks the lists that it walks in one."""
+    from anemoi_b200 import executor, native
+
+    gen = torch.Generator(device="cuda").manual_seed(blocks)
+    q, k, v = (torch.randn(1, prefix + blocks * 64, heads, 64, generator=gen, device="cuda").to(torch.bfloat16)
+               for _ in range(3))
+    kw = _options(blocks, prefix, cells, 0.8)
+    assert _chosen(native_library, q, kw) == (counted > 1)
+    kw.update(layer=0, nvfp4_scales=(0.01, 0.01, 0.002))
+    whole = executor.sm100_ragged_attention(q, k, v, **kw)
+    before = dict(native.LAUNCHES)
+    staged = executor.sm100_ragged_attention(q, k, v, profile_nvtx=True, **kw)
+    assert torch.equal(staged, whole)
+    assert native.LAUNCHES["route"] - before.get("route", 0) == counted
+    assert native.LAUNCHES.get("pair_lists", 0) - before.get("pair_lists", 0) == (2 if counted == 1 else 0)
+    assert executor.last_status() == 0
