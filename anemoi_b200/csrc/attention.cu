@@ -1177,11 +1177,13 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
 // 360 CTAs, 91.0 and 94.9 without; 1 x 43,680, 342 CTAs, 424 and 445; past four CTAs nothing).
 constexpr int kSms = 148;
 constexpr int64_t kHeadsBytes = 48 << 20;
-// FP16 alone at D = 128, whose stages are the largest, loses once a call has many waves (45 heads x 11,600 tokens, 15 waves,
-// 625 / 641; 16 x 14,040 with pairs, 6 waves, 563 / 553).
+// FP16 alone at D = 128, whose stages are the largest (one or two heads of 33,272 tokens at a time), gains the least: Q128, lists
+// of different lengths, 20 heads x 7,800 tokens (4 waves) 244 / 223, 16 x 20,280 (9) 913 / 883, 24 x 20,280 (13) 1,351 / 1,308,
+// 45 x 14,040 (17) 1,268 / 1,268, 20 x 33,272 (18) 2,599 / 2,595; with pairs 24 x 20,280 1,420 / 1,394, 20 x 33,272 2,882 / 2,785.
+// Equal lists, which past ten waves are limited by power, lose up to 1.3 % there (45 x 14,040 1,377 / 1,392, 20 x 33,272 2,740 /
+// 2,776, 12 x 20,280 729 / 721).
 int heads_at_a_time(const AttnParams& p, int64_t ctas) {
   if (p.dense_prefix || ctas <= kSms) return 1;
-  if (p.s.head_dim == 128 && !p.s.has_int8 && !p.s.has_nvfp4 && ctas > 16 * kSms) return 1;
   const int64_t bytes = (p.s.has_nvfp4 ? rec::kv_nvfp4_bytes(p.s.head_dim) : 0) +
                         (p.s.has_int8 ? rec::kv_int8_bytes(p.s.head_dim) : 0) +
                         (p.s.has_fp16 ? rec::kv_fp16_bytes(p.s.head_dim) : 0);
