@@ -1182,12 +1182,14 @@ constexpr int64_t kHeadsBytes = 48 << 20;
 // 45 x 14,040 (17) 1,268 / 1,268, 20 x 33,272 (18) 2,599 / 2,595; with pairs 24 x 20,280 1,420 / 1,394, 20 x 33,272 2,882 / 2,785.
 // Equal lists, which past ten waves are limited by power, lose up to 1.3 % there (45 x 14,040 1,377 / 1,392, 20 x 33,272 2,740 /
 // 2,776, 12 x 20,280 729 / 721).
-int heads_at_a_time(const AttnParams& p, int64_t ctas) {
-  if (p.dense_prefix || ctas <= kSms) return 1;
+// In how many groups the heads of a launch start: one after the other, the heads of a group in turns.
+int head_groups(const AttnParams& p, int64_t ctas) {
+  if (p.dense_prefix || ctas <= kSms) return p.s.heads;
   const int64_t bytes = (p.s.has_nvfp4 ? rec::kv_nvfp4_bytes(p.s.head_dim) : 0) +
                         (p.s.has_int8 ? rec::kv_int8_bytes(p.s.head_dim) : 0) +
                         (p.s.has_fp16 ? rec::kv_fp16_bytes(p.s.head_dim) : 0);
-  return (int)max((int64_t)1, min((int64_t)p.s.heads, kHeadsBytes / (bytes * p.stages)));
+  const int most = (int)max((int64_t)1, min((int64_t)p.s.heads, kHeadsBytes / (bytes * p.stages)));
+  return (p.s.heads + most - 1) / most;
 }
 
 template <int D, int CELLS, bool kQ64>
@@ -1197,7 +1199,7 @@ int launch_kernel(AttnParams& p, int tiles, size_t smem, cudaStream_t st) {
       cudaSuccess)
     return ANEMOI_SM100_ELAUNCH;
   const int64_t ctas = (int64_t)tiles * p.s.heads;
-  const int most = heads_at_a_time(p, ctas), groups = (p.s.heads + most - 1) / most;
+  const int groups = head_groups(p, ctas);
   p.turn = !p.dense_prefix && groups == 1 && ctas > kSms && ctas <= 4 * kSms ? kSms / p.s.heads : 0;
   // (the tiles of a head are the grid's y: a prefix of millions of rows takes several launches)
   for (p.first_place = 0; p.first_place < tiles; p.first_place += 65535) {
@@ -1341,6 +1343,15 @@ extern "C" int anemoi_sm100_attention(const anemoi_sm100_shape* shape,
   if (!stage_ids) return ANEMOI_SM100_EINVAL;
   return video_attention(shape, ops, row_offset, row_counts, stage_ids, nullptr, nullptr,
                          list_capacity, valid_k, out_packed, nullptr, status, stream);
+}
+
+extern "C" int anemoi_sm100_head_groups(const anemoi_sm100_shape* shape, int pairs) {
+  if (rec::validate_shape(shape) != ANEMOI_SM100_OK) return 0;
+  AttnParams p{};
+  p.s = *shape;
+  p.stages = rec::stages(*shape);
+  const int R = shape->video_blocks, tiles = pairs && shape->query_block == 64 ? (R + 1) / 2 : R;
+  return head_groups(p, (int64_t)tiles * shape->heads);
 }
 
 extern "C" int anemoi_sm100_attention_pairs(const anemoi_sm100_shape* shape,

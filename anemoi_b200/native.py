@@ -114,6 +114,7 @@ def library() -> C.CDLL:
         "anemoi_sm100_prepare_zero_kernels": (C.c_int, [SP]),
         "anemoi_sm100_layer_workspace_bytes": (I64, [C.POINTER(LayerPlan)]),
         "anemoi_sm100_matches_pairs": (C.c_int, [C.POINTER(LayerPlan)]),
+        "anemoi_sm100_head_groups": (C.c_int, [SP, C.c_int]),
         "anemoi_sm100_pair_bits_bytes": (I64, [C.POINTER(LayerPlan)]),
         "anemoi_sm100_route_matched": (C.c_int, [C.POINTER(LayerPlan), P, P, I64, P, P, P, P, P, P]),
         "anemoi_sm100_attention_matched": (C.c_int, [SP, OP, P, P, P, P, I64, P, P, P, P]),
@@ -162,7 +163,7 @@ EXPORTED = (
     "anemoi_sm100_layer", "anemoi_sm100_layer_workspace_bytes", "anemoi_sm100_routes_in_one_kernel",
     "anemoi_sm100_drafts_in_routing", "anemoi_sm100_matches_pairs", "anemoi_sm100_prepare_kernels",
     "anemoi_sm100_prepare_zero_kernels", "anemoi_sm100_pair_bits_bytes", "anemoi_sm100_route_matched",
-    "anemoi_sm100_attention_matched",
+    "anemoi_sm100_attention_matched", "anemoi_sm100_head_groups",
     "anemoi_sm100_route_anchored", "anemoi_sm100_route_anchored_scratch_bytes",
     "anemoi_sm100_prefix_attention", "anemoi_sm100_assemble", "anemoi_sm100_pack_qkv",
     "anemoi_sm100_merge_heads", "anemoi_sm100_pack_qkv_heads", "anemoi_sm100_merge_heads_into",

@@ -242,6 +242,9 @@ int anemoi_sm100_attention_pairs(const anemoi_sm100_shape* shape, const anemoi_s
                                  const int32_t* pair_counts, const int32_t* pair_ids,
                                  int64_t list_capacity, const int32_t* valid_k, void* out_packed,
                                  int32_t* status, void* stream);
+/* Groups of heads of an attention launch: a group's tiles start in turns, the groups one after the other (as many
+ * as heads: each head by itself). */
+int anemoi_sm100_head_groups(const anemoi_sm100_shape* shape, int pairs);
 
 /* Dense INT8-cell attention of the prefix query rows over every stage.
  *   out_prefix   fp16 [H][prefix query tiles * QB][D]
