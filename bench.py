@@ -909,17 +909,19 @@ def run_sweep(args) -> None:
             for drop in (0.5, 0.8, 0.9):
                 for cell, ratios in SWEEP_CELLS.items():
                     for weight in ((0.0, 0.5, 1.0) if cell == "nvfp4+int8+fp16" else (0.0,)):
-                        def call():
+                        def call(parts):
                             return executor.sm100_ragged_attention(
                                 q, k, v, prefix_tokens=0, sparsity_ratio=drop,
                                 retained_nvfp4_ratio=ratios[0], retained_int8_ratio=ratios[1],
                                 retained_fp16_ratio=ratios[2], video_shape=video, layer=0,
                                 query_block_size=qb, maxpool_weight=weight,
                                 nvfp4_scales=scales if ratios[0] > 0 else (1.0, 1.0, 1.0),
-                                return_parts=True)
-                        call()
+                                return_parts=parts)
+                        parts = call(True)[1]      # sizes (its Q64 pairs are neighbours: not what is timed)
                         executor.collect_stage_events(True)
-                        out, parts = call()
+                        call(False)
+                        executor.collect_stage_events(True)
+                        out = call(False)
                         st = executor.stage_times_ms()
                         executor.collect_stage_events(False)
                         if executor.last_status(device) != 0 or not bool(torch.isfinite(out).all()):
