@@ -1719,7 +1719,7 @@ int layer::route_bits(const anemoi_sm100_shape& s, const void* probability, int6
 
 bool layer::drafts_in_routing(const anemoi_sm100_shape& s) {
   // (one CTA per head, and one kernel for lists and pairs, whatever the number of heads)
-  static_assert(kDraftBlocks <= 64 && kDraftBlocks * kDraftBlocks <= 65536 && kDraftBlocks <= kFusedWarps);
+  static_assert(kDraftBlocks == 32 && 2 * kShortWarps >= kDraftBlocks, "a column per lane, two rows per warp");
   return s.prefix_tokens == 0 && s.video_blocks <= kDraftBlocks;
 }
 
