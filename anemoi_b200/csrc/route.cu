@@ -953,8 +953,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) route_fused_kernel(
       totals[i] = n0 + n1 + n2;
       offset[i] = off[0];
       row_offset[(int64_t)head * R + r0 + i] = off[0];
-      // (with pairs there is no launch order of single blocks; the other kernel fills it in)
-      *reinterpret_cast<int4*>(row_counts + ((int64_t)head * R + r0 + i) * 4) = make_int4(n0, n1, n2, 0);
+      // (with pairs there is no launch order of single blocks; the other kernel fills it in.  One by one: a caller's
+      // arrays are on four bytes)
+      int32_t* rc = row_counts + ((int64_t)head * R + r0 + i) * 4;
+      rc[0] = n0;
+      rc[1] = n1;
+      rc[2] = n2;
+      rc[3] = 0;
     }
   }
   __syncthreads();
@@ -1288,8 +1293,8 @@ __global__ void __launch_bounds__(kShortThreads) route_short_kernel(
     if (warp == h && row < R) {
       row_offset[(int64_t)head * R + row] = offset[h];
       int32_t* rc = row_counts + ((int64_t)head * R + row) * 4;
-      *reinterpret_cast<int2*>(rc) = make_int2(n[h][0], n[h][1]);
-      rc[2] = n[h][2];
+#pragma unroll
+      for (int b = 0; b < 3; ++b) rc[b] = n[h][b];
       if (kPairs) rc[3] = 0;
     }
   }
@@ -1395,8 +1400,8 @@ __global__ void __launch_bounds__(kShortThreads) route_short_kernel(
       }
       if (lane == 0) {
         int32_t* pc = pair_counts + ((int64_t)head * pairs_all + a / 2) * 4;
-        *reinterpret_cast<int2*>(pc) = make_int2(at[0] - start[0], at[1] - start[1]);
-        pc[2] = at[2] - start[2];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) pc[b] = at[b] - start[b];
         sh.unions[a / 2] = at[0] + at[1] + at[2] - start[1] - start[2];
       }
     }

@@ -144,3 +144,39 @@ def test_map_of_the_one_launch(native_library, video, query_block, dim, weight, 
 def test_short_maps(native_library, heads, blocks, cells, prefix, phase):
     """Up to 64 blocks a head's map is held in registers: one and two columns per lane, and the kernel past it."""
     lists_equal_the_oracle(native_library, heads, blocks, cells, prefix, phase)
+
+
+@pytest.mark.parametrize("pairs", [False, True])
+@pytest.mark.parametrize("heads, blocks", [(3, 7), (3, 40), (3, 64), (3, 101), (1, 1100)])
+def test_arrays_on_four_bytes(native_library, heads, blocks, pairs):
+    """The caller's arrays start at any int: the same lists as in arrays on 16 bytes."""
+    from anemoi_b200 import native
+
+    shape = native.Shape(heads=heads, head_dim=64, query_block=64, seq_tokens=blocks * 64, prefix_tokens=0, video_blocks=blocks,
+                         has_nvfp4=0, has_int8=1, has_fp16=1, has_prefix_query_int8=0, has_maxpool=0, input_is_bf16=1,
+                         q_global_scale=1.0, k_global_scale=1.0, v_global_scale=1.0)
+    if pairs and not native.library().anemoi_sm100_routes_in_one_kernel(C.byref(shape)):
+        pytest.skip("pairs of their own launches")
+    gen = torch.Generator(device="cuda").manual_seed(blocks)
+    prob = torch.rand(heads, blocks, blocks, generator=gen, device="cuda").to(torch.float16)
+    n16, n8 = blocks * blocks // 10, blocks * blocks // 10 + 1
+    capacity = native_library.anemoi_sm100_route_list_capacity(C.byref(shape), n16, n8, 0, -1)
+    scratch = torch.empty(native_library.anemoi_sm100_route_scratch_bytes(C.byref(shape)), dtype=torch.uint8, device="cuda")
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    tiles = (blocks + 1) // 2
+    sizes = [heads * blocks, heads * blocks * 4] + ([heads * tiles * 4] if pairs else []) + [heads * capacity]
+    got = []
+    for shift in (0, 1, 2, 3):
+        out = [torch.full((n + 4,), -7, dtype=torch.int32, device="cuda")[shift:shift + n] for n in sizes]
+        ptr = [C.c_void_p(t.data_ptr()) for t in out]
+        if pairs:
+            code = native_library.anemoi_sm100_route_pairs(C.byref(shape), C.c_void_p(prob.data_ptr()), n16, n8, 0, -1, *ptr,
+                                                           capacity, stream)
+        else:
+            code = native_library.anemoi_sm100_route(C.byref(shape), C.c_void_p(prob.data_ptr()), n16, n8, 0, -1,
+                                                     C.c_void_p(scratch.data_ptr()), scratch.numel(), *ptr, capacity, stream)
+        assert code == 0
+        got.append(out)
+    torch.cuda.synchronize()
+    for out in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(out, got[0]))
