@@ -5,7 +5,8 @@ that holds its activations on the host pays the copies in front of and behind it
 the other.  Heads are independent on this path (pools, routing budget, lists and attention are
 all per head), so this entry walks the heads in groups on three streams: while group ``g`` runs
 the layer, group ``g+1`` is copied in and group ``g-1`` is copied out.  Each group and tensor is
-ONE strided copy.  The result is bit-identical to a single call on all heads.
+ONE strided copy.  The result is bit-identical to a single call on all heads (as long as the values are
+finite in the types of the precision cells: Q64 blocks that share a CTA share infinities).
 
 With ``sharded=True`` (several GPUs of one node, one process each) every rank holds its rows of
 the sequence on its host; each head group is copied in, exchanged to head-sharded form by stores

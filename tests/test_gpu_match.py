@@ -157,3 +157,26 @@ def test_stages_take_the_pairs_of_the_call(native_library, blocks, heads, prefix
     assert native.LAUNCHES["route"] - before.get("route", 0) == counted
     assert native.LAUNCHES.get("pair_lists", 0) - before.get("pair_lists", 0) == (2 if counted == 1 else 0)
     assert executor.last_status() == 0
+
+
+@pytest.mark.parametrize("cells, prefix_kv", [((0.0, 1.0, 0.0), "fp16"), ((0.0, 1.0, 0.0), "nvfp4"), ((1.0, 0.0, 0.0), "int8"),
+                                              ((0.5, 0.0, 0.5), "int8"), ((0.0, 0.5, 0.5), "nvfp4")])
+def test_prefix_stages_in_a_phase_of_their_own(native_library, cells, prefix_kv):
+    """The prefix is all that the lists have of its phase: in front of the others, between or behind them."""
+    from anemoi_b200 import executor
+
+    blocks, heads, prefix = 129, 50, 150
+    gen = torch.Generator(device="cuda").manual_seed(blocks)
+    q, k, v = (torch.randn(1, prefix + blocks * 64, heads, 64, generator=gen, device="cuda").to(torch.bfloat16)
+               for _ in range(3))
+    kw = dict(_options(blocks, prefix, cells, 0.8), prefix_kv_precision=prefix_kv)
+    assert _chosen(native_library, q, kw) == 1
+    kw.update(layer=0, nvfp4_scales=(0.01, 0.01, 0.002))
+    paired = executor.sm100_ragged_attention(q, k, v, **kw)
+    executor._PAIR_Q64 = False
+    try:
+        single = executor.sm100_ragged_attention(q, k, v, **kw)
+    finally:
+        executor._PAIR_Q64 = True
+    assert torch.isfinite(single).all() and torch.equal(paired, single)
+    assert executor.last_status() == 0
