@@ -1138,17 +1138,28 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         if (dst != nullptr) {
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
-            // (the channels' factors are loaded together: one by one under a condition that is not known to be the
-            // warp's, each is waited for, 3 us of a small call: 7 heads x 2,293 tokens, D = 128 65.3, now 62.1)
-            float f[8], factor[8];
+            float f[8];
+            if constexpr (kFactors == 2) {
+              // (the channels' factors are loaded together: one by one under a condition that is not known to be the
+              // warp's, each is waited for, 3 us of a small call: 7 heads x 2,293 tokens, D = 128 65.3, now 62.1)
+              float factor[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) factor[i] = last_cell == kNv ? nv_dom : 1.0f;
-            if (last_cell == kI8) {
+              for (int i = 0; i < 8; ++i) factor[i] = last_cell == kNv ? nv_dom : 1.0f;
+              if (last_cell == kI8) {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) factor[i] = vscale[c0 + j + i] * 0.0022326917f;
+                for (int i = 0; i < 8; ++i) factor[i] = vscale[c0 + j + i] * 0.0022326917f;
+              }
+#pragma unroll
+              for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r[j + i]) * factor[i] * inv;
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                f[i] = __uint_as_float(r[j + i]);
+                if (last_cell == kNv) f[i] *= nv_dom;
+                if (last_cell == kI8) f[i] *= vscale[c0 + j + i] * 0.0022326917f;
+                f[i] *= inv;
+              }
             }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r[j + i]) * factor[i] * inv;
             uint4 v = make_uint4(f16x2(f[0], f[1]), f16x2(f[2], f[3]), f16x2(f[4], f[5]), f16x2(f[6], f[7]));
             if (bf16)
               v = make_uint4(bf16x2_of_f16x2(v.x), bf16x2_of_f16x2(v.y), bf16x2_of_f16x2(v.z), bf16x2_of_f16x2(v.w));
