@@ -49,7 +49,10 @@
 //   FP16 : P -> f16
 // Accumulation is fp32 in TMEM (the reference accumulates a stage in fp16 for the
 // INT8 and FP16 cells).
+#include <cuda.h>
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "bounded_wait.cuh"
 #include "layer.cuh"
@@ -91,12 +94,20 @@ constexpr int kColSfaP = 208;
 constexpr int kColSfbV = 212;
 constexpr int kRing = 8;       // entries of the per-stage rings, and the most key/value slots
 constexpr int kSplitKeys = 4, kSplitValues = 2;  // key and value buffers of phases that keep them apart
+constexpr int kMostParts = 8;    // CTAs that share the stages of a tile of dense rows: a portable cluster
 constexpr float kFp8Offset = 8.807f;
+constexpr float kLowest = -3.0e38f;  // maximum before the first stage of dense rows
 constexpr uint64_t kDrainNs = 100000000;  // limit of the waits for copies and MMAs in flight after a give-up
+
+// log2(e) / sqrt(D)
+__host__ __device__ constexpr float sigma(int d) { return (d == 64 ? 0.125f : 0.08838834764831845f) * 1.4426950408889634f; }
 
 enum Cell : int { kNv = 0, kI8 = 1, kF16 = 2 };
 // Which cells a kernel is built for: one, or any mix.
 enum Cells : int { kAny = 3 };
+
+// Kernels for dense rows of the caller's own tensors (prefix queries kept out of the cells), and their type.
+enum Raw : int { kNone = 0, kRawF16 = 1, kRawBf16 = 2 };
 
 constexpr int kColS1 = 128;    // D = 64: second score buffer
 
@@ -133,6 +144,24 @@ struct AttnParams {
   int turn;          // a head's lists before this place in the order start shortest first
   int first_place;   // of a launch's tiles
 };
+
+// Dense rows (prefix queries kept out of the cells): 128 queries per tile, every row attends to every token, operands
+// straight from the caller's tensors by tiled TMA.  Bound, as the FP16 cell, by shared memory (96 KB per stage of
+// D = 128) where there are tiles for every SM, which few calls have: a prefix is some tiles per head, each as long as the
+// head's keys, so the CTAs of a cluster (the grid's x) share a tile's stages and add up their parts through each other's
+// shared memory.  Alone, us, torch's attention (cuDNN for bf16) / one CTA per tile / parts: bf16 D = 128 3 heads x 7,159
+// tokens, 517 rows 84 / 83 / 30, 16 x 14,296, 256 rows 160 / 163 / 53, 7 x 33,272, 512 rows 350 / 357 / 101, 1 x 85,000,
+// 30 rows 1,297 / 845 / 118; fp16 D = 64 6 x 33,178, 58 rows 567 / 282 / 45.  Where rows and heads fill the GPU the library
+// is ahead (56 x 33,272, 512 rows 408 / 603 / 592).  Whole calls, of which these rows are a part beside the others: small
+// ones 100 -> 31-60 us (its host work alone took 90), 48 x 2,474 169 -> 161, 16 x 14,296 589 -> 580, 30 x 10,198 with 958 rows
+// 873 -> 909, 32 x 41,955 with 780 rows 6,170 -> 6,310.
+struct alignas(64) RawParams : AttnParams {
+  CUtensorMap q, k, v;  // [tokens][heads][D] as they lie in memory: 64 channels x 1 head x 64 tokens (Q: 128), swizzled
+  int rows, tokens_in, parts;
+  int64_t out_token, out_head;  // distances in `tokens`, in elements
+};
+template <int RAW>
+using Params = std::conditional_t<RAW == kNone, AttnParams, RawParams>;
 
 // Entry g % kRing of a ring belongs to stage g, in phase g / kRing of the barrier.  Stage
 // g + kRing cannot begin before PV of stage g is complete (it needs a key/value slot and there are
@@ -197,6 +226,52 @@ __device__ __forceinline__ uint32_t f16x2(float a, float b) {
   uint32_t v;
   asm("cvt.rn.f16x2.f32 %0, %2, %1;" : "=r"(v) : "f"(a), "f"(b));
   return v;
+}
+
+// Every thread of the cluster: what was written to shared memory before is visible after, across its CTAs.
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Shared memory of the cluster's CTA `rank` at the place that is `addr` in this one's.
+__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float2 peer_float2(uint32_t addr, int rank) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(peer_smem(addr, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 peer_float4(uint32_t addr, int rank) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(peer_smem(addr, rank))
+               : "memory");
+  return v;
+}
+
+__device__ __forceinline__ uint32_t bf16x2(float a, float b) {
+  uint32_t v;
+  asm("cvt.rn.bf16x2.f32 %0, %2, %1;" : "=r"(v) : "f"(a), "f"(b));
+  return v;
+}
+// 64 channels of 64 or 128 tokens of one head, rows of 128 bytes whose 16-byte pieces are swizzled (by TMA).
+__device__ __forceinline__ void tensor_g2s(uint8_t* dst, const CUtensorMap* map, int channel, int head, int token,
+                                           uint64_t* bar, uint32_t issue) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      "\n\t}" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(channel), "r"(head), "r"(token), "r"(smem_u32(bar)), "r"(issue)
+      : "memory");
+}
+// Operand of 128-byte rows swizzled in groups of eight (1,024 bytes); `lbo`: between blocks of 64 channels where these
+// are the operand's rows.
+__device__ __forceinline__ uint64_t swizzled_desc(uint32_t addr, uint32_t lbo) {
+  return smem_desc(addr, lbo, 1024) | (2ull << 61);
 }
 
 // Two fp32 -> fp16 (the result's precision) -> bf16, as the assembly of packed rows rounds.
@@ -327,7 +402,7 @@ __device__ __forceinline__ void rescale_o(uint32_t tmem_row, float alpha, const 
 // Probabilities of the thread's 64 scores, P = 2^(s * scale + bias), rounded to the cell's operand
 // format and stored into its row of the K-major P tile 16 bytes at a time (the conversions and
 // stores of one piece run under the exponentials of the next); returns their unrounded sum.
-template <int CELL>
+template <int CELL, int RAW = kNone>
 __device__ __forceinline__ float exp_store(const float (&s)[64], float scale, float bias,
                                            uint8_t* p_row) {
   const float2 scale2 = make_float2(scale, scale);
@@ -339,8 +414,10 @@ __device__ __forceinline__ float exp_store(const float (&s)[64], float scale, fl
     float e[kPer];
 #pragma unroll
     for (int j = 0; j < kPer; j += 4) {
-      const float2 a0 = ffma2(make_float2(s[c * kPer + j], s[c * kPer + j + 1]), scale2, bias2);
-      const float2 a1 = ffma2(make_float2(s[c * kPer + j + 2], s[c * kPer + j + 3]), scale2, bias2);
+      float2 a0 = make_float2(s[c * kPer + j], s[c * kPer + j + 1]);
+      float2 a1 = make_float2(s[c * kPer + j + 2], s[c * kPer + j + 3]);
+      a0 = RAW != kNone ? fmul2(fadd2(a0, bias2), scale2) : ffma2(a0, scale2, bias2);
+      a1 = RAW != kNone ? fmul2(fadd2(a1, bias2), scale2) : ffma2(a1, scale2, bias2);
       e[j] = ex2(a0.x);
       e[j + 1] = ex2(a0.y);
       e[j + 2] = ex2(a1.x);
@@ -349,7 +426,9 @@ __device__ __forceinline__ float exp_store(const float (&s)[64], float scale, fl
       acc1 = fadd2(acc1, make_float2(e[j + 2], e[j + 3]));
     }
     uint4 v;
-    if (CELL == kF16) {
+    if (RAW == kRawBf16) {
+      v = make_uint4(bf16x2(e[0], e[1]), bf16x2(e[2], e[3]), bf16x2(e[4], e[5]), bf16x2(e[6], e[7]));
+    } else if (CELL == kF16) {
       v = make_uint4(f16x2(e[0], e[1]), f16x2(e[2], e[3]), f16x2(e[4], e[5]), f16x2(e[6], e[7]));
     } else if (CELL == kI8) {
       v = make_uint4(e4m3x4(e[0], e[1], e[2], e[3]), e4m3x4(e[4 % kPer], e[5 % kPer], e[6 % kPer], e[7 % kPer]),
@@ -379,7 +458,7 @@ struct SoftmaxWalk {
 // untouched.  `kPass`: such a stage has a path of its own, without the scores.  A third of a pair's stages
 // are passed over so: Q64 kernels of one cell gain 1-3 % (INT8, 8 heads of S = 38,247: 1.42 -> 1.38 ms); the
 // mixed one, whose instruction cache is full, would lose 10 %.
-template <int D, bool kPairs, bool kPass>
+template <int D, bool kPairs, bool kPass, int RAW>
 __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_t tmem_row, int row, int g, int cell,
                                               bool live_warp, int my_block, SoftmaxWalk& w) {
   const int at = g & (kRing - 1), before_at = (g - 1) & (kRing - 1);
@@ -460,12 +539,12 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
   // (entry -1 was filled before the roles started, and the phase before a barrier's first counts as over)
   wait(&b->wc, &m_full[before_at], ((g - 1) >> 3) & 1, 9);
   const float2 before = b->rec[before_at][row];
-  const float m_new = fmaxf(before.x, mx * scale);
+  const float m_new = fmaxf(before.x, RAW != kNone ? mx : mx * scale);
   w.d = before.y * w.alpha + w.sum;
   b->rec[at][row] = make_float2(m_new, w.d);
   __syncwarp();
   mbar_arrive_if(&m_full[at], lead);
-  w.alpha = ex2(before.x - m_new);
+  w.alpha = ex2(RAW != kNone ? (before.x - m_new) * scale : before.x - m_new);
   if (kPairs) w.sum = 0.0f;
   if (active) {
     // exponent = s * scale + bias; the NVFP4 cell produces 6 P directly (e2m1 input range),
@@ -478,7 +557,7 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
     } else if (cell == kNv) {
       sum = exp_store<kNv>(s, scale, bias, p_row);
     } else {
-      sum = exp_store<kF16>(s, scale, bias, p_row);
+      sum = exp_store<kF16, RAW>(s, scale, bias, p_row);
     }
     w.sum = sum * sum_scale;
   } else if (live_warp) {
@@ -505,11 +584,16 @@ __device__ __forceinline__ uint64_t moved(uint64_t desc, uint32_t step) {
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo + step), "r"(hi));
   return d;
 }
-template <int D, int CELL>
+template <int D, int CELL, int RAW = kNone>
 __device__ __forceinline__ void issue_qk(uint32_t tmem_s, uint32_t tmem, uint64_t q_desc, uint64_t base,
                                          uint32_t step) {  // q_desc: NVFP4 only
   const uint64_t kd = moved(base, step);
-  if (CELL == kF16) {
+  if (RAW != kNone) {
+    constexpr uint32_t fmt = RAW == kRawBf16 ? kFmtBF16 : kFmtF16, idesc = instr_desc(fmt, fmt, kAccF32, 128, 64, 0, 0);
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k)
+      mma_f16_ts(tmem_s, tmem + kColQ + k * 8, kd + k / 4 * (64 * 128 / 16) + k % 4 * 2, idesc, k > 0);
+  } else if (CELL == kF16) {
     constexpr uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, 64, 0, 0);
 #pragma unroll
     for (int k = 0; k < D / 16; ++k) mma_f16_ts(tmem_s, tmem + kColQ + k * 8, kd + k * 16, idesc, k > 0);
@@ -534,9 +618,14 @@ __device__ __forceinline__ uint64_t k_desc(int d, int cell, uint32_t addr) {
   return smem_desc(addr, 128, (uint32_t)d * (cell == kF16 ? 16 : cell == kI8 ? 8 : 4));
 }
 
-template <int D, int CELL>
+template <int D, int CELL, int RAW = kNone>
 __device__ __forceinline__ void issue_pv(uint32_t tmem, uint64_t pd, uint64_t vd, uint32_t accumulate) {
-  if (CELL == kF16) {
+  if (RAW != kNone) {
+    constexpr uint32_t fmt = RAW == kRawBf16 ? kFmtBF16 : kFmtF16, idesc = instr_desc(fmt, fmt, kAccF32, 128, D, 0, 1);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      mma_f16_ss(tmem + kColO, pd + k * 16, vd + k * (2 * 1024 / 16), idesc, k > 0 ? 1u : accumulate);
+  } else if (CELL == kF16) {
     constexpr uint32_t idesc = instr_desc(kFmtF16, kFmtF16, kAccF32, 128, D, 0, 1);
     constexpr uint32_t v_lbo = (D / 8) * 128;  // between 8-key groups
 #pragma unroll
@@ -586,19 +675,70 @@ __device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, i
   return ((int64_t)token * p.s.heads + head) * D;
 }
 
+// The rows of a tile from the parts that the CTAs of the cluster left in their shared memory (softmax threads; a CTA
+// takes every parts-th row): O = sum of O_i 2^(m_i - M), the denominator alike.
+template <int D, int RAW>
+__device__ __forceinline__ void add_parts(const RawParams& p, const uint8_t* smem, int head, int tile) {
+  constexpr int kPieces = D / 8;
+  const uint32_t base = smem_u32(smem);
+#pragma unroll 1
+  for (int i = threadIdx.x; i < 128 * kPieces; i += 256) {
+    const int row = (i / kPieces) * p.parts + (int)blockIdx.x, piece = i % kPieces;
+    if (row >= 128 || tile * 128 + row >= p.rows) break;
+    float2 md[kMostParts];
+    float m = kLowest;
+#pragma unroll
+    for (int c = 0; c < kMostParts; ++c) {
+      md[c] = c < p.parts ? peer_float2(base + 512 * D + row * 8, c) : make_float2(kLowest, 0.0f);
+      m = fmaxf(m, md[c].x);
+    }
+    float d = 0.0f, o[8] = {};
+#pragma unroll
+    for (int c = 0; c < kMostParts; ++c) {
+      if (c < p.parts) {
+        const float f = ex2((md[c].x - m) * sigma(D));
+        d += md[c].y * f;
+        const float4 a = peer_float4(base + (row * (D / 4) + ((2 * piece) ^ (row & 7))) * 16, c);
+        const float4 z = peer_float4(base + (row * (D / 4) + ((2 * piece + 1) ^ (row & 7))) * 16, c);
+        o[0] += a.x * f;
+        o[1] += a.y * f;
+        o[2] += a.z * f;
+        o[3] += a.w * f;
+        o[4] += z.x * f;
+        o[5] += z.y * f;
+        o[6] += z.z * f;
+        o[7] += z.w * f;
+      }
+    }
+    const float inv = 1.0f / d;  // (no score above -inf: NaN, as 0 / 0)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) o[c] *= inv;
+    uint4 v;
+    if (RAW == kRawBf16) {
+      v = make_uint4(bf16x2(o[0], o[1]), bf16x2(o[2], o[3]), bf16x2(o[4], o[5]), bf16x2(o[6], o[7]));
+    } else {
+      v = make_uint4(f16x2(o[0], o[1]), f16x2(o[2], o[3]), f16x2(o[4], o[5]), f16x2(o[6], o[7]));
+    }
+    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.tokens) + (tile * 128 + row) * p.out_token + head * p.out_head +
+                              piece * 8) = v;
+  }
+}
+
 constexpr int kStays = -1;  // in place of a block's factors: O stays in its domain
 __host__ __device__ constexpr int factor_sets(int cells, bool q64) { return cells == kAny && q64 ? 2 : 1; }
 
-template <int D, int CELLS, bool kQ64>
-__global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams p) {
-  extern __shared__ __align__(128) uint8_t smem[];
+template <int D, int CELLS, bool kQ64, int RAW = kNone>
+__global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_constant__ Params<RAW> p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  constexpr bool kRaw = RAW != kNone;
+  static_assert(!kRaw || (CELLS == kF16 && !kQ64), "dense rows are walked as the FP16 cell's");
   constexpr int kFirst = CELLS == kAny ? 0 : CELLS, kLast = CELLS == kAny ? 2 : CELLS;
   constexpr int QB = kQ64 ? 64 : 128;
   // Kernels of one cell spill less (and are 1-5 % quicker) if the roles read again from shared memory which tile they
   // work on; those of any mix, and the ones with registers to spare, do not (4-12 % slower).
   constexpr bool kReread = CELLS != kAny && (kQ64 || Regs<D, CELLS>::kWide);
   // CTAs start in the order x, y, z: the longest lists of a few heads, the second ones, ..., then the next few heads
-  const int head = blockIdx.z * gridDim.x + blockIdx.x;
+  const int head = kRaw ? blockIdx.z : blockIdx.z * gridDim.x + blockIdx.x;
   if (head >= p.s.heads) return;
   const int place = p.first_place + ((int)blockIdx.y < p.turn ? p.turn - 1 - (int)blockIdx.y : (int)blockIdx.y);
   layer::grid_dependency_wait();
@@ -607,7 +747,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   int tile = place;
   const bool table = kQ64 && p.pair_table != nullptr, pairs = table || (kQ64 && p.pair_counts != nullptr);
   const int pair_tiles = (p.s.video_blocks + 1) / 2;
-  if (!p.dense_prefix && !table) {
+  if (!kRaw && !p.dense_prefix && !table) {
     const int ordered =
         pairs ? p.pair_counts[((int64_t)head * pair_tiles + place) * 4 + 3]
               : p.row_counts[((int64_t)head * p.s.video_blocks + place) * 4 + 3];
@@ -624,7 +764,12 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   // ---- this tile's work list ----
   int cnt[3] = {0, p.stages, 0};
   const int32_t* list = nullptr;
-  if (table) {
+  int begin = 0;
+  if constexpr (kRaw) {
+    begin = (int)((int64_t)p.stages * blockIdx.x / p.parts);
+    cnt[kI8] = 0;
+    cnt[kF16] = (int)((int64_t)p.stages * (blockIdx.x + 1) / p.parts) - begin;
+  } else if (table) {
     const int4* entry = p.pair_table + ((int64_t)head * pair_tiles + tile) * 2;
     const int4 e = entry[0], n = entry[1];
     block0 = e.x;
@@ -656,7 +801,14 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   // into its own wait limit.  One thread reads the word for the whole CTA: another CTA may set it at any
   // time, and if only some warps of this one left, the others would go on without tensor memory, without
   // barriers or with a warpgroup short of the warps its setmaxnreg waits for.
-  if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t*>(p.status) != 0)) return;
+  if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t*>(p.status) != 0)) {
+    if (kRaw) {
+      // (the other CTAs of the cluster may have seen the word clear: they read this one's shared memory)
+      cluster_sync();
+      cluster_sync();
+    }
+    return;
+  }
 
   uint8_t* q_smem = smem;
   uint8_t* ring = smem + p.q_region;
@@ -695,7 +847,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       // phase c of a union of neighbours sits where the two blocks' phases before it would end
       const bool apart = pairs && !table;
       const int32_t* ra = apart ? p.row_counts + ((int64_t)head * p.s.video_blocks + block0) * 4 : nullptr;
-      int before = 0;
+      int before = begin;
       for (int c = 0; c < 3; ++c) {
         b->cnt[c] = cnt[c];
         b->first_of[c] = before;
@@ -704,7 +856,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     }
     mbar_init_fence();
   } else if (warp < 5) {
-    b->rec[kRing - 1][threadIdx.x - 32] = make_float2(-5.0e6f, 0.0f);  // before the first stage
+    b->rec[kRing - 1][threadIdx.x - 32] = make_float2(kRaw ? kLowest : -5.0e6f, 0.0f);  // before the first stage
   } else if (kFactors == 2 && warp == 5 && lane < 2) {
     // A block of a pair without a stage of a phase stays in its domain, and one without a phase before it has
     // nothing to move, so that a block's result does not depend on its partner: two steps instead of one, or there
@@ -749,7 +901,6 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       const int64_t q_index_i8 =
           (int64_t)head_at * p.q_tiles_int8 + (p.dense_prefix ? p.s.video_blocks : 0) + first_block;
       const int step = (kReread ? b->block[1] : block1) - first_block;  // from a pair's first record to its second
-      const float sigma = (D == 64 ? 0.125f : 0.08838834764831845f) * 1.4426950408889634f;
       int phase_ord = 0, g = 0, v_fills = 0, moves = 0;
 #pragma unroll 1
       for (int cell = kFirst; cell <= kLast; ++cell) {
@@ -763,7 +914,10 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             : cell == kI8 ? static_cast<const uint8_t*>(p.o.q_int8) + q_index_i8 * qbytes
                           : static_cast<const uint8_t*>(p.o.q_fp16) + (int64_t)q_index_fp * qbytes;
         mbar_arrive_expect_tx(&b->q_full, qbytes * blocks, lead);
-        if (cell == kNv && kQ64) {
+        if constexpr (kRaw) {
+#pragma unroll
+          for (int c = 0; c < D; c += 64) tensor_g2s(q_smem + c * 256, &p.q, c, head_at, tile * 128, &b->q_full, lead);
+        } else if (cell == kNv && kQ64) {
           // codes fill the first half of the 128-row tile; scale blocks follow the full tile.
           // A pair's second record: codes into the second half of the tile, scale blocks behind
           // the first record's (the QK warp folds them into one block before it copies them).
@@ -799,7 +953,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           if (blocks == 2) q_scale[1] = p.o.q_int8_scale[q_index_i8 + step];
           kscale = p.o.k_int8_scale + (int64_t)head_at * p.stages;
         }
-        const float base = cell == kNv ? sigma * p.s.q_global_scale * p.s.k_global_scale : sigma;
+        const float base = cell == kNv ? sigma(D) * p.s.q_global_scale * p.s.k_global_scale : sigma(D);
         // list entries, 32 at a time, one per lane, with their metadata
         int stage_l = 0;
         float2 meta_l[2] = {make_float2(base, 0.0f), make_float2(base, 0.0f)};
@@ -813,15 +967,22 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
           if ((i & 31) == 0 && i < n) {
             const int at = i + lane;
             int entry = 0;
-            if (at < n) entry = list_at != nullptr ? list_at[first + at] : at;
-            stage_l = entry & 0x3fffffff;
-            const int valid = p.valid_k[stage_l];
+            int valid;
+            if constexpr (kRaw) {
+              entry = first + at;
+              stage_l = entry;
+              valid = p.tokens_in - stage_l * 64;
+            } else {
+              if (at < n) entry = list_at != nullptr ? list_at[first + at] : at;
+              stage_l = entry & 0x3fffffff;
+              valid = p.valid_k[stage_l];
+            }
             meta_l[0].y = __int_as_float(!pairs || ((entry >> 30) & 1) ? valid : -1);
             if (kQ64) meta_l[1].y = __int_as_float(entry < 0 || p.dense_prefix ? valid : -1);
             if (cell == kI8) {
               const float ks = kscale[stage_l];
-              meta_l[0].x = sigma * (q_scale[0] * ks);
-              if (kQ64) meta_l[1].x = sigma * (q_scale[1] * ks);
+              meta_l[0].x = sigma(D) * (q_scale[0] * ks);
+              if (kQ64) meta_l[1].x = sigma(D) * (q_scale[1] * ks);
             }
           }
           const int stage = __shfl_sync(0xffffffffu, stage_l, i & 31);
@@ -840,7 +1001,12 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             const uint8_t* src = kvbase + (int64_t)stage * kvbytes;
             uint8_t* dst = (split ? smem : ring) + (size_t)slot * slot_size;
             mbar_arrive_expect_tx(&b->kv_full[at], bytes, lead);
-            if (split || rest == kbytes) {
+            if constexpr (kRaw) {
+#pragma unroll
+              for (int c = 0; c < D; c += 64)
+                tensor_g2s(dst + c * 128, &p.k, c, head_at, stage * 64, &b->kv_full[at], lead);
+              if (!split) tensor_g2s(dst + rest, &p.v, 0, head_at, stage * 64, &b->kv_full[at], lead);
+            } else if (split || rest == kbytes) {
               bulk_g2s(dst, src, bytes, &b->kv_full[at], lead);
             } else {
               bulk_g2s(dst, src, kbytes, &b->kv_full[at], lead);
@@ -853,8 +1019,15 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             if (i > kSplitValues) wait<kMmaRole>(&b->wc, &b->pv_done[before & (kRing - 1)], (before >> 3) & 1, 2);
             uint64_t* full = &b->v_full[(i - 1) & 1];
             mbar_arrive_expect_tx(full, kvbytes - kbytes, lead);
-            bulk_g2s(smem + (kSplitKeys + ((i - 1) & 1)) * slot_size, kvbase + (int64_t)prev_stage * kvbytes + kbytes,
-                     kvbytes - kbytes, full, lead);
+            if constexpr (kRaw) {
+#pragma unroll
+              for (int c = 0; c < D; c += 64)
+                tensor_g2s(smem + (kSplitKeys + ((i - 1) & 1)) * slot_size + c * 128, &p.v, c, head_at, prev_stage * 64, full,
+                           lead);
+            } else {
+              bulk_g2s(smem + (kSplitKeys + ((i - 1) & 1)) * slot_size,
+                       kvbase + (int64_t)prev_stage * kvbytes + kbytes, kvbytes - kbytes, full, lead);
+            }
             ++v_fills;
           }
           prev_stage = stage;
@@ -892,7 +1065,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         tc_fence_after_sync();
         const int nslot = slot_count(p.ring_bytes, D, cell);
         const uint32_t stride = stage_bytes(D, cell);
-        const uint64_t base = k_desc(D, cell, split_kv(D, cell) ? smem_u32(smem) : ring_addr);
+        const uint32_t base_addr = split_kv(D, cell) ? smem_u32(smem) : ring_addr;
+        const uint64_t base = kRaw ? swizzled_desc(base_addr, 16) : k_desc(D, cell, base_addr);
         const uint64_t q_desc = k_desc(D, kNv, q_addr);
         if (cell == kNv) {
           if ((kReread ? b->tile_blocks : tile_blocks) == 2) {
@@ -936,7 +1110,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             } else if (cell == kNv) {
               issue_qk<D, kNv>(tmem_s, tmem, q_desc, base, step);
             } else {
-              issue_qk<D, kF16>(tmem_s, tmem, q_desc, base, step);
+              issue_qk<D, kF16, RAW>(tmem_s, tmem, q_desc, base, step);
             }
             mma_commit(&b->s_full[g & 1]);
             if (i == n - 1) mma_commit(&b->q_free);
@@ -964,8 +1138,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         const uint32_t stride = stage_bytes(D, cell);
         const uint32_t base_addr = split_kv(D, cell) ? smem_u32(smem) : ring_addr;
         const uint64_t p_base = p_desc(cell, base_addr);
-        const uint64_t v_base =
-            v_desc(D, cell, base_addr + (split_kv(D, cell) ? kSplitKeys * stride : rest_offset(D, cell)));
+        const uint32_t v_addr = base_addr + (split_kv(D, cell) ? kSplitKeys * stride : rest_offset(D, cell));
+        const uint64_t v_base = kRaw ? swizzled_desc(v_addr, 64 * 128) : v_desc(D, cell, v_addr);
         int slot = first_slot(D, cell);
 #pragma unroll 1
         for (int i = 0; i < n; ++i, ++g) {
@@ -981,7 +1155,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
             } else if (cell == kNv) {
               issue_pv<D, kNv>(tmem, pd, vd, g > 0);
             } else {
-              issue_pv<D, kF16>(tmem, pd, vd, g > 0);
+              issue_pv<D, kF16, RAW>(tmem, pd, vd, g > 0);
             }
             mma_commit(&b->pv_done[g & (kRing - 1)]);
             if (CELLS == kAny && cell == kNv && i == n - 1) mma_commit(&b->nv_done);
@@ -995,6 +1169,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       // unwinding: the MMAs in flight must be over before tensor memory is given back
       if (b->wc.abort) drain_wait(&b->all_done, 0, kDrainNs);
     }
+    if (kRaw) cluster_sync();  // as the softmax warps before they add up the tile's parts
   } else if (warp >= kCorrWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS>::kRescale));
     // =============================== O rescale ===============================
@@ -1002,7 +1177,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     uint64_t* m_full = b->m_full[warp - kCorrWarp];
     const uint32_t tmem_row = tmem + ((uint32_t)((warp - kCorrWarp) * 32) << 16);
     const uint32_t lead = lane == 0;
-    float m = -5.0e6f;
+    float m = kRaw ? kLowest : -5.0e6f;
     int g = 0, prev_cell = -1, phase_ord = 0;
 #pragma unroll 1
     for (int cell = kFirst; cell <= kLast; ++cell) {
@@ -1033,9 +1208,15 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
 #pragma unroll 1
         for (int c = 0; c < chunks; c += 2) {
           uint32_t r[8];
-          *reinterpret_cast<uint4*>(r) = *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c, chunks));
-          *reinterpret_cast<uint4*>(r + 4) =
-              *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c + 1, chunks));
+          if (kRaw) {
+            const uint8_t* from = q_smem + (c >> 3) * (128 * 128) + row * 128;
+            *reinterpret_cast<uint4*>(r) = *reinterpret_cast<const uint4*>(from + (((c & 7) ^ (row & 7)) << 4));
+            *reinterpret_cast<uint4*>(r + 4) = *reinterpret_cast<const uint4*>(from + ((((c + 1) & 7) ^ (row & 7)) << 4));
+          } else {
+            *reinterpret_cast<uint4*>(r) = *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c, chunks));
+            *reinterpret_cast<uint4*>(r + 4) =
+                *reinterpret_cast<const uint4*>(q_smem + rec::tile_offset(row, c + 1, chunks));
+          }
           tmem_st8(tmem_row + kColQ + c * 4, r);
         }
         tmem_wait_st();
@@ -1051,7 +1232,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
         const float m_new = b->rec[at][row].x;
         const bool first = moves && i == 0;
         if (g > 0 && (first || __any_sync(0xffffffffu, m_new != m))) {
-          const float alpha = ex2(m - m_new);
+          const float alpha = ex2(kRaw ? (m - m_new) * sigma(D) : m - m_new);
           // O may only be touched once the previous PV is complete
           wait<kRescaleRole>(&b->wc, &b->pv_done[(g - 1) & (kRing - 1)], ((g - 1) >> 3) & 1, 20);
           tc_fence_after_sync();
@@ -1064,6 +1245,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       }
       prev_cell = cell;
     }
+    if (kRaw) cluster_sync();
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS>::kSoftmax));
     // =============================== softmax rows ===============================
@@ -1090,7 +1272,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
       int slot = first_slot(D, cell) + first;
 #pragma unroll 1
       for (int i = first; i < n; i += 2) {
-        softmax_stage<D, kQ64, kQ64 && CELLS != kAny>(b, p_row + slot * stride, tmem_row, row, g + i, cell, live_warp,
+        softmax_stage<D, kQ64, kQ64 && CELLS != kAny, RAW>(b, p_row + slot * stride, tmem_row, row, g + i, cell, live_warp,
                                                         my_block, w);
         slot += 2;
         if (slot >= nslot) slot -= nslot;
@@ -1103,7 +1285,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     uint16_t* dst = nullptr;
     const int head_at = kReread ? b->head : head;
     const int first_block = kReread ? b->block[0] : block0, second_block = kReread ? b->block[1] : block1;
-    if (row < QB * (kReread ? b->tile_blocks : tile_blocks)) {
+    if (!kRaw && row < QB * (kReread ? b->tile_blocks : tile_blocks)) {
       if (p.tokens == nullptr) {
         dst = reinterpret_cast<uint16_t*>(p.out) +
               ((int64_t)head_at * p.out_rows + (kQ64 && row >= QB ? second_block * QB + row - QB : first_block * QB + row)) * D;
@@ -1117,14 +1299,35 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
     // d(G-1) from d(G-3) and the last two stages' (alpha, sum), which the two groups hold; every
     // other use of rec is over
     const bool last_mine = ((g - 1) & 1) == parity;
-    if (!last_mine) b->rec[0][row] = make_float2(w.alpha, w.sum);
+    // (a part's maxima are needed, too: its last stage's entries stay)
+    const int free0 = kRaw ? g & (kRing - 1) : 0, free1 = kRaw ? (g + 1) & (kRing - 1) : 1;
+    if (!last_mine) b->rec[free0][row] = make_float2(w.alpha, w.sum);
     asm volatile("bar.sync 6, 256;" ::: "memory");
     if (last_mine) {
-      const float2 other = b->rec[0][row];
-      b->rec[1][row] = make_float2((w.d * other.x + other.y) * w.alpha + w.sum, 0.0f);
+      const float2 other = b->rec[free0][row];
+      b->rec[free1][row] = make_float2((w.d * other.x + other.y) * w.alpha + w.sum, 0.0f);
     }
     asm volatile("bar.sync 6, 256;" ::: "memory");
-    if (live_warp) {
+    if constexpr (kRaw) {
+      // This CTA's part of the tile, before the division: rows of fp32 (16-byte pieces swizzled: a warp's
+      // rows are 4 * D bytes apart), maxima and denominators behind them.
+      tc_fence_after_sync();
+#pragma unroll 1
+      for (int c0 = parity * (D / 2); c0 < (parity + 1) * (D / 2); c0 += 32) {
+        uint32_t r[32];
+        tmem_ld32(tmem_row + kColO + c0, r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          reinterpret_cast<uint4*>(smem)[row * (D / 4) + (((c0 + j) / 4) ^ (row & 7))] =
+              make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+      }
+      if (parity == 0)
+        reinterpret_cast<float2*>(smem + 512 * D)[row] =
+            make_float2(b->rec[(g - 1) & (kRing - 1)][row].x, b->rec[free1][row].x);
+      cluster_sync();
+      add_parts<D, RAW>(p, smem, head_at, tile);
+    } else if (live_warp) {
       tc_fence_after_sync();
       if (kFactors == 2) last_cell = b->last[my_block];
       const float d = b->rec[1][row].x;
@@ -1175,6 +1378,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const AttnParams
   tc_fence_before_sync();
   __syncthreads();
   if (warp == kPvWarp) tmem_dealloc(tmem, kTmemCols);
+  if (kRaw) cluster_sync();  // the others have read this CTA's part
 }
 
 // Heads whose query tiles start in turns, longest lists first: as many as keep keys and values of up to 48 MB in use (they
@@ -1257,6 +1461,64 @@ int launch_for(AttnParams& p, int tiles, cudaStream_t st) {
   if (p.s.query_block == 64)
     return p.s.head_dim == 64 ? launch<64, true>(p, tiles, st) : launch<128, true>(p, tiles, st);
   return p.s.head_dim == 64 ? launch<64, false>(p, tiles, st) : launch<128, false>(p, tiles, st);
+}
+
+// ---- dense rows ----
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+  static const EncodeTiled fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &found) == cudaSuccess &&
+                   found == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<EncodeTiled>(f)
+               : nullptr;
+  }();
+  return fn;
+}
+
+bool encode(CUtensorMap* map, const void* base, bool bf16, int d, int heads, int tokens, int64_t token_stride,
+            int64_t head_stride, int box_tokens) {
+  const cuuint64_t dims[3] = {(cuuint64_t)d, (cuuint64_t)heads, (cuuint64_t)tokens};
+  const cuuint64_t strides[2] = {(cuuint64_t)head_stride * 2, (cuuint64_t)token_stride * 2};
+  const cuuint32_t box[3] = {64, 1, (cuuint32_t)box_tokens}, step[3] = {1, 1, 1};
+  return encode_tiled()(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
+                        const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Parts of a tile, by the sequence alone (a head's rows are then the same whichever heads are with it).  A part costs
+// some 8 us beside its stages (half a microsecond each, twice that with two CTAs on the SM), so short sequences have
+// few; and where a head has tiles enough more parts gain little.  One / two / four / eight parts, us: 16 heads x 2,500
+// tokens, 400 rows 36 / 24 / 26 / 38, 30 x 9,000, 200 rows 108 / 62 / 53 / 73, 53 x 13,093, 37 rows 153 / 84 / 73 / 83, 7 x 33,272,
+// 512 rows 357 / 186 / 101 / 85, 7 x 85,000, 900 rows 884 / 447 / 342 / 413.
+int dense_parts(int stages, int tiles) {
+  const int most = stages < 32 ? 1 : stages < 96 ? 2 : stages < 256 ? 4 : kMostParts;
+  return max(1, min(most, 16 / tiles));
+}
+
+template <int D, int RAW>
+int launch_dense(RawParams& p, cudaStream_t st) {
+  auto kernel = attention_kernel<D, kF16, false, RAW>;
+  constexpr int kQ = 256 * D, kFixed = kQ + D * 4 + (int)sizeof(Shared);
+  constexpr int kRingBytes = (115528 - kFixed) / 128 * 128;
+  static_assert(kQ + kRingBytes >= 512 * D + 1024, "a CTA's part takes the place of Q and the ring");
+  p.q_region = kQ;
+  p.ring_bytes = kRingBytes;
+  const size_t smem = kFixed + kRingBytes;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return ANEMOI_SM100_ELAUNCH;
+  const int tiles = (p.rows + 127) / 128;
+  p.parts = dense_parts(p.stages, tiles);
+  for (p.first_place = 0; p.first_place < tiles; p.first_place += 65535) {
+    const dim3 grid(p.parts, min(65535, tiles - p.first_place), p.s.heads);
+    if (layer::launch_cluster(kernel, grid, dim3(p.parts), dim3(kThreads), smem, st, p) != cudaSuccess)
+      return ANEMOI_SM100_ELAUNCH;
+  }
+  return ANEMOI_SM100_OK;
 }
 
 int check_ops(const anemoi_sm100_shape& s, const anemoi_sm100_operands& o, bool dense_prefix) {
@@ -1412,6 +1674,44 @@ int prefix_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operand
   return launch_for(p, tiles, st);
 }
 }  // namespace
+
+extern "C" int anemoi_sm100_dense_rows(int heads, int head_dim, int tokens, int rows, int is_bf16, const void* q,
+                                       const void* k, const void* v, const int64_t* strides, void* out, int64_t out_token,
+                                       int64_t out_head, int32_t* status, void* stream) {
+  if (heads <= 0 || heads > 65535 || (head_dim != 64 && head_dim != 128) || rows <= 0 || tokens < rows || !q || !k || !v ||
+      !out || !status)
+    return ANEMOI_SM100_EINVAL;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+       reinterpret_cast<uintptr_t>(out)) % 16 || out_token % 8 || out_head % 8)
+    return ANEMOI_SM100_EINVAL;
+  int64_t stride[6];
+  for (int i = 0; i < 6; ++i) {
+    const int64_t packed = i & 1 ? (int64_t)head_dim : (int64_t)heads * head_dim;
+    stride[i] = strides == nullptr || (heads == 1 && i & 1) ? packed : strides[i];
+    // (what a tensor map takes)
+    if (stride[i] <= 0 || stride[i] % 8 || stride[i] >= (1ll << 39)) return ANEMOI_SM100_EINVAL;
+  }
+  if (encode_tiled() == nullptr) return ANEMOI_SM100_ELAUNCH;
+  RawParams p{};
+  if (!encode(&p.q, q, is_bf16, head_dim, heads, tokens, stride[0], stride[1], 128) ||
+      !encode(&p.k, k, is_bf16, head_dim, heads, tokens, stride[2], stride[3], 64) ||
+      !encode(&p.v, v, is_bf16, head_dim, heads, tokens, stride[4], stride[5], 64))
+    return ANEMOI_SM100_EINVAL;
+  p.s.heads = heads;
+  p.s.head_dim = head_dim;
+  p.s.video_blocks = 1;
+  p.rows = rows;
+  p.tokens_in = tokens;
+  p.stages = (tokens + 63) / 64;
+  p.tokens = out;
+  p.out_token = out_token;
+  p.out_head = out_head;
+  p.status = status;
+  p.wait_ns = g_wait_limit_ns;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (head_dim == 64) return is_bf16 ? launch_dense<64, kRawBf16>(p, st) : launch_dense<64, kRawF16>(p, st);
+  return is_bf16 ? launch_dense<128, kRawBf16>(p, st) : launch_dense<128, kRawF16>(p, st);
+}
 
 extern "C" int anemoi_sm100_prefix_attention(const anemoi_sm100_shape* shape,
                                              const anemoi_sm100_operands* ops,

@@ -185,15 +185,14 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
     if (rec::validate_shape(&s) != ANEMOI_SM100_OK) return ANEMOI_SM100_EINVAL;
   }
   const bool native_prefix = s.has_prefix_query_int8 && s.prefix_tokens > 0;
-  if (s.prefix_tokens > 0 && !native_prefix && prefix_out == nullptr) return ANEMOI_SM100_EINVAL;
+  const bool dense_prefix = s.prefix_tokens > 0 && !native_prefix && prefix_out == nullptr &&
+                            prefix_is_caller_dtype == ANEMOI_SM100_PREFIX_DENSE;
+  if (s.prefix_tokens > 0 && !native_prefix && !dense_prefix && prefix_out == nullptr) return ANEMOI_SM100_EINVAL;
   if (s.prefix_tokens > 0 && side_stream == nullptr) return ANEMOI_SM100_EINVAL;
   const Workspace w = cut(p, static_cast<uint8_t*>(workspace));
   if (workspace_bytes < w.bytes) return ANEMOI_SM100_EINVAL;
   cudaStream_t st = static_cast<cudaStream_t>(stream), side = static_cast<cudaStream_t>(side_stream);
   const layer::TokenRows rows{out, p.indices, p.counts};
-
-  int code = anemoi_sm100_prepare(&s, q, k, v, strides, p.indices, p.counts, &w.ops, stream);
-  if (code != ANEMOI_SM100_OK) return code;
 
   // fork and join of the side stream: an event each, destroyed when its use is over
   cudaEvent_t fork = nullptr, join = nullptr;
@@ -206,12 +205,20 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
     if (join) cudaEventDestroy(join);
     return c;
   };
-  auto prefix = [&]() -> int {
-    if (cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventRecord(fork, st) != cudaSuccess || cudaStreamWaitEvent(side, fork, 0) != cudaSuccess)
-      return ANEMOI_SM100_ELAUNCH;
-    return layer::prefix_rows(s, w.ops, p.valid_k, rows, p.status, side);
+  auto to_side = [&]() {
+    return cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
+           cudaEventRecord(fork, st) == cudaSuccess && cudaStreamWaitEvent(side, fork, 0) == cudaSuccess;
   };
+  auto prefix = [&]() -> int {
+    return to_side() ? layer::prefix_rows(s, w.ops, p.valid_k, rows, p.status, side) : ANEMOI_SM100_ELAUNCH;
+  };
+  // (dense rows need the caller's tensors only)
+  if (dense_prefix && !to_side()) return done(ANEMOI_SM100_ELAUNCH);
+  int code = anemoi_sm100_prepare(&s, q, k, v, strides, p.indices, p.counts, &w.ops, stream);
+  if (code == ANEMOI_SM100_OK && dense_prefix)
+    code = anemoi_sm100_dense_rows(s.heads, s.head_dim, s.seq_tokens, s.prefix_tokens, s.input_is_bf16, q, k, v, strides, out,
+                                   (int64_t)s.heads * s.head_dim, s.head_dim, p.status, side_stream);
+  if (code != ANEMOI_SM100_OK) return done(code);
   const int prefix_ctas = (rec::prefix_query_tiles(s) * s.query_block + 127) / 128 * s.heads;
   const bool late = native_prefix && prefix_ctas >= kPrefixFillsGpu;
   if (native_prefix && !late && (code = prefix()) != ANEMOI_SM100_OK) return done(code);
@@ -246,7 +253,7 @@ extern "C" int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const voi
     if (cudaEventCreateWithFlags(&join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventRecord(join, side) != cudaSuccess || cudaStreamWaitEvent(st, join, 0) != cudaSuccess)
       return done(ANEMOI_SM100_ELAUNCH);
-    if (!native_prefix)
+    if (!native_prefix && !dense_prefix)
       code = layer::assemble_prefix(s, prefix_out, prefix_rows, prefix_is_caller_dtype, out, st);
   }
   return done(code);

@@ -17,7 +17,6 @@ import math
 from functools import lru_cache
 
 import torch
-import torch.nn.functional as F
 
 from . import native
 from .api import NVFP4Calibration, QuantConfig, SparseConfig, VisualLayout
@@ -105,6 +104,13 @@ def _prefix_stream(device: torch.device) -> torch.cuda.Stream:
     # first wherever an SM has room (launched with the video CTAs of a 9 ms call they would else start
     # behind them; 1 % of the call).
     return torch.cuda.Stream(device=device, priority=-1)
+
+
+@lru_cache(maxsize=8)
+def _dense_stream(device: torch.device) -> torch.cuda.Stream:
+    # FP16 prefix rows need nothing but the caller's tensors and start with the call, so at a high priority they would
+    # hold up preparation, draft map and routing, which everything else waits for (33 heads x 4,989 tokens 275 us, so 259).
+    return torch.cuda.Stream(device=device, priority=0)
 
 
 @lru_cache(maxsize=64)
@@ -230,19 +236,13 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
 
     frames, height, width = video_shape
     current = torch.cuda.current_stream(device)
-    side = _prefix_stream(device)
+    side = _prefix_stream(device) if native_prefix else _dense_stream(device)
     prefix_out = None
     if prefix_tokens and not native_prefix:
         # dense attention of the prefix rows on the caller's tensors, as the reference does
         side.wait_stream(current)
         with torch.cuda.stream(side), _Range("anemoi.dense_prefix", nvtx):
-            prefix_out = F.scaled_dot_product_attention(
-                q_bshd[:, :prefix_tokens].permute(0, 2, 1, 3),
-                k_bshd.permute(0, 2, 1, 3),
-                v_bshd.permute(0, 2, 1, 3),
-                dropout_p=0.0,
-                is_causal=False,
-            )[0].contiguous()
+            prefix_out = native.dense_rows(q_bshd, k_bshd, v_bshd, prefix_tokens, _status_word(device))
 
     layout = materialize_ragged_2d_layout(device, frames=frames, height=height, width=width,
                                           logical_block=query_block_size, enable_anchors=enable_anchors)
@@ -347,7 +347,7 @@ class _Plan:
         self.bytes = int(lib.anemoi_sm100_layer_workspace_bytes(self.ref))
         if self.bytes < 0:
             raise RuntimeError("invalid attention shape")
-        self.side = _prefix_stream(device) if prefix_tokens else None
+        self.side = (_prefix_stream if self.native_prefix else _dense_stream)(device) if prefix_tokens else None
         self.side_handle = self.side.cuda_stream if prefix_tokens else None
         self.uses_scales = "nvfp4" in active
         # kernels per call: preparation (with V's maxima and their zeroes), draft, routing (and pair lists), attention, prefix rows
@@ -383,27 +383,15 @@ def _one_call(q, k, v, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape, 
     plan = _plan(q.device, tokens, heads, dim, q.dtype, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape,
                  query_block, prefix_kv, prefix_query, maxpool_weight, _PAIR_Q64)
     (_, q1, q2, _), (_, k1, k2, _), (_, v1, v2, _) = q.stride(), k.stride(), v.stride()
-    return _launch(plan, q, k, v, q.device, prefix_tokens, _stride_array(q1, q2, k1, k2, v1, v2),
-                   _scale_array(nvfp4_scales))
+    return _launch(plan, q, k, v, q.device, _stride_array(q1, q2, k1, k2, v1, v2), _scale_array(nvfp4_scales))
 
 
-def _launch(plan, q, k, v, device, prefix_tokens, strides, scales):
-    prefix_out, prefix_ptr, prefix_rows = None, None, 0
-    if prefix_tokens and not plan.native_prefix:
-        # dense attention of the prefix rows on the caller's tensors, as the reference does
-        current = torch.cuda.current_stream(device)
-        plan.side.wait_stream(current)
-        with torch.cuda.stream(plan.side):
-            prefix_out = F.scaled_dot_product_attention(
-                q[:, :prefix_tokens].permute(0, 2, 1, 3), k.permute(0, 2, 1, 3), v.permute(0, 2, 1, 3),
-                dropout_p=0.0, is_causal=False)[0].contiguous()
-        prefix_out.record_stream(current)
-        prefix_ptr, prefix_rows = prefix_out.data_ptr(), prefix_tokens
+def _launch(plan, q, k, v, device, strides, scales):
     workspace = torch.empty(plan.bytes, dtype=torch.uint8, device=device)
     out = torch.empty(q.shape, dtype=q.dtype, device=device)
     code = plan.call(
-        plan.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, scales, prefix_ptr, prefix_rows, 1, out.data_ptr(),
-        workspace.data_ptr(), plan.bytes, torch._C._cuda_getCurrentRawStream(device.index), plan.side_handle)
+        plan.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, scales, None, 0, native.PREFIX_DENSE,
+        out.data_ptr(), workspace.data_ptr(), plan.bytes, torch._C._cuda_getCurrentRawStream(device.index), plan.side_handle)
     if code != 0:
         native._check(code, "anemoi_sm100_layer")
     native._count("layer", plan.launches)
@@ -444,7 +432,7 @@ def attention_call(query, key, value, layout, layer, sparse, quant, calib):
                 sparse.sparsity_for_layer(layer) if sparse.layer_sparsity_bands else sparse.sparsity_ratio,
                 sparse.maxpool_weight, quant.nvfp4_ratio, quant.int8_ratio, quant.fp16_ratio,
                 quant.prefix_kv_precision, quant.prefix_query_precision, _PAIR_Q64)
-            return _launch(plan, query, key, value, plan.device, prefix, _stride_array(q1, q2, k1, k2, v1, v2),
+            return _launch(plan, query, key, value, plan.device, _stride_array(q1, q2, k1, k2, v1, v2),
                            _Scales(calib.q_scale, calib.k_scale, calib.v_scale) if plan.uses_scales else None)
     return execute_ragged_attention(
         query, key, value, prefix_tokens=layout.prefix_tokens, video_shape=layout.video_shape, layer=layer,

@@ -107,6 +107,8 @@ def library() -> C.CDLL:
         "anemoi_sm100_attention_pairs": (C.c_int, [SP, OP, P, P, P, P, I64, P, P, P, P]),
         "anemoi_sm100_pair_lists": (C.c_int, [SP, P, P, P, I64, P, P, P]),
         "anemoi_sm100_prefix_attention": (C.c_int, [SP, OP, P, P, P, P]),
+        "anemoi_sm100_dense_rows": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, P, P, P, C.POINTER(I64), P,
+                                              I64, I64, P, P]),
         "anemoi_sm100_route_pairs": (C.c_int, [SP, P, I64, I64, I64, C.c_int, P, P, P, P, I64, P]),
         "anemoi_sm100_routes_in_one_kernel": (C.c_int, [SP]),
         "anemoi_sm100_drafts_in_routing": (C.c_int, [SP]),
@@ -165,7 +167,7 @@ EXPORTED = (
     "anemoi_sm100_prepare_zero_kernels", "anemoi_sm100_pair_bits_bytes", "anemoi_sm100_route_matched",
     "anemoi_sm100_attention_matched", "anemoi_sm100_head_groups",
     "anemoi_sm100_route_anchored", "anemoi_sm100_route_anchored_scratch_bytes",
-    "anemoi_sm100_prefix_attention", "anemoi_sm100_assemble", "anemoi_sm100_pack_qkv",
+    "anemoi_sm100_prefix_attention", "anemoi_sm100_dense_rows", "anemoi_sm100_assemble", "anemoi_sm100_pack_qkv",
     "anemoi_sm100_merge_heads", "anemoi_sm100_pack_qkv_heads", "anemoi_sm100_merge_heads_into",
     "anemoi_sm100_tensor_peak", "anemoi_sm100_qknorm_rope", "anemoi_sm100_set_wait_limit_ns",
     "anemoi_sm100_wait_selftest", "anemoi_sm100_copy_rows", "anemoi_sm100_push_qkv",
@@ -446,6 +448,21 @@ def prefix_attention(shape: Shape, store: OperandStore, valid_k: torch.Tensor,
     _check(library().anemoi_sm100_prefix_attention(
         C.byref(shape), C.byref(store.struct), _ptr(valid_k), _ptr(out), _ptr(status),
         _stream(dev)), "anemoi_sm100_prefix_attention")
+    return out
+
+
+PREFIX_DENSE = 2
+
+
+def dense_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, rows: int, status: torch.Tensor) -> torch.Tensor:
+    """Dense attention of the first ``rows`` tokens' queries over all tokens: ``[H][rows][D]`` in the tensors' type."""
+    _, tokens, heads, dim = q.shape
+    out = torch.empty((heads, rows, dim), dtype=q.dtype, device=q.device)
+    strides = (C.c_int64 * 6)(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2))
+    _count("dense_rows", 1)
+    _check(library().anemoi_sm100_dense_rows(
+        heads, dim, tokens, rows, int(q.dtype == torch.bfloat16), _ptr(q), _ptr(k), _ptr(v), strides, _ptr(out), dim,
+        rows * dim, _ptr(status), _stream(q.device)), "anemoi_sm100_dense_rows")
     return out
 
 

@@ -254,6 +254,15 @@ int anemoi_sm100_prefix_attention(const anemoi_sm100_shape* shape,
                                   const anemoi_sm100_operands* ops, const int32_t* valid_k,
                                   void* out_prefix, int32_t* status, void* stream);
 
+/* Dense attention of the first `rows` tokens' queries over all tokens, of the caller's own tensors (fp16 or bf16; 16-byte
+ * aligned, strides as for anemoi_sm100_prepare, positive): prefix queries that are kept out of the cells.  Probabilities
+ * in the tensors' type, sums in fp32.
+ *   out          in the tensors' type; `out_token`, `out_head`: its strides in elements (multiples of 8)
+ * Takes the place of scaled_dot_product_attention in anemoi/layers/attention/mpa/executor.py:598-611. */
+int anemoi_sm100_dense_rows(int heads, int head_dim, int tokens, int rows, int is_bf16, const void* q, const void* k,
+                            const void* v, const int64_t* strides, void* out, int64_t out_token, int64_t out_head,
+                            int32_t* status, void* stream);
+
 /* One whole call, from raw Q/K/V to the output in token order: prepare, draft_probability, route (and
  * pair_lists), attention and the prefix rows, with the attention's results written straight to their
  * tokens.  A plan holds what calls of one configuration share; the tables stay the caller's.
@@ -296,12 +305,14 @@ int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan);
 /*   strides          as for anemoi_sm100_prepare
  *   nvfp4_scales     q, k, v tensor-level scales of this call, or null for the plan's
  *   prefix_out       prefix rows computed elsewhere on `side_stream` ([H][prefix_rows][D], the caller's
- *                    dtype if prefix_is_caller_dtype); null with has_prefix_query_int8 or without a prefix
+ *                    dtype if prefix_is_caller_dtype); null with has_prefix_query_int8 or without a prefix.  Null and
+ *                    prefix_is_caller_dtype == ANEMOI_SM100_PREFIX_DENSE: anemoi_sm100_dense_rows of q, k, v
  *   out              [S][H][D] contiguous, the input's dtype
  *   workspace        anemoi_sm100_layer_workspace_bytes() bytes, 256-byte aligned, free for reuse on
  *                    `stream` when the call returns
  *   side_stream      runs beside `stream` and is joined before the call's work ends (with a prefix)
  * Counterpart of sm120_ragged_h3_attention (anemoi/layers/attention/mpa/executor.py:876-1224). */
+#define ANEMOI_SM100_PREFIX_DENSE 2
 int anemoi_sm100_layer(const anemoi_sm100_layer_plan* plan, const void* q, const void* k, const void* v,
                        const int64_t* strides, const float* nvfp4_scales, const void* prefix_out,
                        int64_t prefix_rows, int prefix_is_caller_dtype, void* out, void* workspace,
