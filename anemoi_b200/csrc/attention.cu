@@ -75,7 +75,7 @@ constexpr int kThreads = 512;
 constexpr int kOtherRegs = 32;
 template <int D, int CELLS>
 struct Regs {
-  static constexpr bool kWide = D == 64 || CELLS == 0;
+    static constexpr bool kWide = D == 64 || CELLS == 0;
   static constexpr int kSoftmax = kWide ? 96 : 88, kRescale = kWide ? 32 : 48;
   static constexpr int kRescaleColumns = kWide ? 16 : 32;
 };
@@ -103,8 +103,20 @@ constexpr uint64_t kDrainNs = 100000000;  // limit of the waits for copies and M
 __host__ __device__ constexpr float sigma(int d) { return (d == 64 ? 0.125f : 0.08838834764831845f) * 1.4426950408889634f; }
 
 enum Cell : int { kNv = 0, kI8 = 1, kF16 = 2 };
-// Which cells a kernel is built for: one, or any mix.
-enum Cells : int { kAny = 3 };
+// Which cells a kernel is built for: one, all, or two.
+enum Cells : int { kAny = 3, kNvI8 = 4, kI8F16 = 5, kNvF16 = 6 };
+__host__ __device__ constexpr bool mixed(int cells) { return cells >= kAny; }
+__host__ __device__ constexpr bool has_cell(int cells, int cell) {
+  return cells == cell || cells == kAny || (cells == kNvI8 && cell != kF16) || (cells == kI8F16 && cell != kNv) ||
+         (cells == kNvF16 && cell != kI8);
+}
+// Whether the stage is of `which`, in a kernel built for `CELLS` (code of cells that it is not built for drops out).
+template <int CELLS, int WHICH>
+__device__ __forceinline__ bool is(int cell) {
+  if constexpr (!has_cell(CELLS, WHICH)) return false;
+  else if constexpr (!mixed(CELLS)) return true;
+  else return cell == WHICH;
+}
 
 // Kernels for dense rows of the caller's own tensors (prefix queries kept out of the cells), and their type.
 enum Raw : int { kNone = 0, kRawF16 = 1, kRawBf16 = 2 };
@@ -442,6 +454,55 @@ __device__ __forceinline__ float exp_store(const float (&s)[64], float scale, fl
   return (acc0.x + acc0.y) + (acc1.x + acc1.y);
 }
 
+// The same where the cell is a run-time value: the exponentials take the scores' registers in code that the cells share,
+// and only conversion and stores are each cell's own.  That is 64 (128 with three cells) instructions less per copy in
+// kernels whose stage code fills the instruction cache, but a piece's conversions no longer run under the next one's
+// exponentials.  Separate / shared, us: three cells of D = 64, 7 heads x 11,994 tokens 178 / 166, 8 x 12,240 NVFP4 + INT8 Q64
+// 528 / 508.  Not where FP16 with its eight stores per stage meets INT8, and not for three cells of D = 128, which are ahead
+// by up to 2.5 % in small calls but lose 1 % in large ones (56 heads x 85,184 tokens 37.4 / 37.8 ms); in halves or with
+// two cells at a time the branches cost more than they save (5 x 3,834 three cells 71 / 74).
+__host__ __device__ constexpr bool shares(int d, int cells) {
+  return cells == kNvI8 || cells == kNvF16 || (d == 64 && cells == kAny);
+}
+template <int CELLS>
+__device__ __forceinline__ float exp_any(float (&s)[64], float scale, float bias, int cell, uint8_t* p_row) {
+  const float2 scale2 = make_float2(scale, scale);
+  const float2 bias2 = make_float2(bias, bias);
+  float2 acc0 = make_float2(0.0f, 0.0f), acc1 = make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int j = 0; j < 64; j += 4) {
+    const float2 a0 = ffma2(make_float2(s[j], s[j + 1]), scale2, bias2);
+    const float2 a1 = ffma2(make_float2(s[j + 2], s[j + 3]), scale2, bias2);
+    s[j] = ex2(a0.x);
+    s[j + 1] = ex2(a0.y);
+    s[j + 2] = ex2(a1.x);
+    s[j + 3] = ex2(a1.y);
+    acc0 = fadd2(acc0, make_float2(s[j], s[j + 1]));
+    acc1 = fadd2(acc1, make_float2(s[j + 2], s[j + 3]));
+  }
+  if (is<CELLS, kI8>(cell)) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      *reinterpret_cast<uint4*>(p_row + c * 128) = make_uint4(
+          e4m3x4(s[16 * c], s[16 * c + 1], s[16 * c + 2], s[16 * c + 3]),
+          e4m3x4(s[16 * c + 4], s[16 * c + 5], s[16 * c + 6], s[16 * c + 7]),
+          e4m3x4(s[16 * c + 8], s[16 * c + 9], s[16 * c + 10], s[16 * c + 11]),
+          e4m3x4(s[16 * c + 12], s[16 * c + 13], s[16 * c + 14], s[16 * c + 15]));
+  } else if (is<CELLS, kNv>(cell)) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      *reinterpret_cast<uint4*>(p_row + c * 128) = make_uint4(e2m1x8(s + 32 * c), e2m1x8(s + 32 * c + 8),
+                                                              e2m1x8(s + 32 * c + 16), e2m1x8(s + 32 * c + 24));
+  } else {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      *reinterpret_cast<uint4*>(p_row + c * 128) =
+          make_uint4(f16x2(s[8 * c], s[8 * c + 1]), f16x2(s[8 * c + 2], s[8 * c + 3]), f16x2(s[8 * c + 4], s[8 * c + 5]),
+                     f16x2(s[8 * c + 6], s[8 * c + 7]));
+  }
+  return (acc0.x + acc0.y) + (acc1.x + acc1.y);
+}
+
 // State of a softmax row.  The two softmax warpgroups alternate stages; the running maximum and
 // the denominator travel between them through shared memory.  The denominator is carried two stages
 // late, so that a group waits for nothing but the other's maximum: stage g publishes m(g) and d(g - 2),
@@ -458,7 +519,7 @@ struct SoftmaxWalk {
 // untouched.  `kPass`: such a stage has a path of its own, without the scores.  A third of a pair's stages
 // are passed over so: Q64 kernels of one cell gain 1-3 % (INT8, 8 heads of S = 38,247: 1.42 -> 1.38 ms); the
 // mixed one, whose instruction cache is full, would lose 10 %.
-template <int D, bool kPairs, bool kPass, int RAW>
+template <int D, int CELLS, bool kPairs, bool kPass, int RAW>
 __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_t tmem_row, int row, int g, int cell,
                                               bool live_warp, int my_block, SoftmaxWalk& w) {
   const int at = g & (kRing - 1), before_at = (g - 1) & (kRing - 1);
@@ -510,7 +571,7 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
   const bool active = !kPairs || kPass || (live_warp && valid >= 0);
   float mx = -INFINITY;
   if (active) {
-    if (cell == kI8) {
+    if (is<CELLS, kI8>(cell)) {
 #pragma unroll
       for (int j = 0; j < 64; ++j) s[j] = __int2float_rn(__float_as_int(s[j]));  // |score| < 2^22: exact
     }
@@ -549,12 +610,14 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
   if (active) {
     // exponent = s * scale + bias; the NVFP4 cell produces 6 P directly (e2m1 input range),
     // the INT8 cell P * 2^8.807 (e4m3 input range); the sums are scaled back.
-    const float bias = (cell == kI8 ? kFp8Offset : (cell == kNv ? 2.5849625007f : 0.0f)) - m_new;
-    const float sum_scale = cell == kI8 ? 0.0022326917f : (cell == kNv ? 0.16666667f : 1.0f);
+    const float bias = (is<CELLS, kI8>(cell) ? kFp8Offset : (is<CELLS, kNv>(cell) ? 2.5849625007f : 0.0f)) - m_new;
+    const float sum_scale = is<CELLS, kI8>(cell) ? 0.0022326917f : (is<CELLS, kNv>(cell) ? 0.16666667f : 1.0f);
     float sum;
-    if (cell == kI8) {
+    if (shares(D, CELLS)) {
+      sum = exp_any<CELLS>(s, scale, bias, cell, p_row);
+    } else if (is<CELLS, kI8>(cell)) {
       sum = exp_store<kI8>(s, scale, bias, p_row);
-    } else if (cell == kNv) {
+    } else if (is<CELLS, kNv>(cell)) {
       sum = exp_store<kNv>(s, scale, bias, p_row);
     } else {
       sum = exp_store<kF16, RAW>(s, scale, bias, p_row);
@@ -654,11 +717,14 @@ __device__ __forceinline__ uint64_t v_desc(int d, int cell, uint32_t addr) {
 // ------------------------------------------------------------------------------------------
 // kernel
 // ------------------------------------------------------------------------------------------
-// CELLS: the one cell of every stage, or kAny.  A kernel of one cell has that cell's code only and
-// its sizes as constants; in the mixed kernel the cell is a run-time value and one copy of the
+// CELLS: the cells that a stage can be of.  A kernel of one cell has that cell's code only and
+// its sizes as constants; in mixed kernels the cell is a run-time value and one copy of the
 // stage code serves all: the CTAs of an SM are in different phases, and hot code that outgrows the
 // instruction cache costs more than the constants give (three whole copies of the softmax stage,
-// 100 KB of code: 1.48 us per 64-key stage and SM at D = 64 instead of 1.11).
+// 100 KB of code: 1.48 us per 64-key stage and SM at D = 64 instead of 1.11).  For the same reason two cells
+// have a kernel without the third one's code.  In the kernel for all / their own, us: NVFP4 + INT8 30 heads x 8,415 tokens
+// D = 64 Q64 473 / 416, Q128 336 / 320, D = 128 Q64 546 / 513; INT8 + FP16 17 x 7,695 D = 64 184 / 179, 47 x 8,415 D = 128 Q128
+// 582 / 566; NVFP4 + FP16 48 x 2,442 D = 64 98 / 89.
 // Where a row of the tile goes in `tokens` (element offset of its first channel), -1: a padding row.
 template <int D, bool kQ64>
 __device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, int block0, int block1, int row) {
@@ -725,18 +791,20 @@ __device__ __forceinline__ void add_parts(const RawParams& p, const uint8_t* sme
 }
 
 constexpr int kStays = -1;  // in place of a block's factors: O stays in its domain
-__host__ __device__ constexpr int factor_sets(int cells, bool q64) { return cells == kAny && q64 ? 2 : 1; }
+__host__ __device__ constexpr int factor_sets(int cells, bool q64) { return mixed(cells) && q64 ? 2 : 1; }
 
 template <int D, int CELLS, bool kQ64, int RAW = kNone>
 __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_constant__ Params<RAW> p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr bool kRaw = RAW != kNone;
   static_assert(!kRaw || (CELLS == kF16 && !kQ64), "dense rows are walked as the FP16 cell's");
-  constexpr int kFirst = CELLS == kAny ? 0 : CELLS, kLast = CELLS == kAny ? 2 : CELLS;
+  constexpr bool kMixed = mixed(CELLS);
+  constexpr int kFirst = !kMixed ? CELLS : has_cell(CELLS, kNv) ? kNv : kI8;
+  constexpr int kLast = !kMixed ? CELLS : has_cell(CELLS, kF16) ? kF16 : kI8;
   constexpr int QB = kQ64 ? 64 : 128;
   // Kernels of one cell spill less (and are 1-5 % quicker) if the roles read again from shared memory which tile they
   // work on; those of any mix, and the ones with registers to spare, do not (4-12 % slower).
-  constexpr bool kReread = CELLS != kAny && (kQ64 || Regs<D, CELLS>::kWide);
+  constexpr bool kReread = !kMixed && (kQ64 || Regs<D, CELLS>::kWide);
   // CTAs start in the order x, y, z: the longest lists of a few heads, the second ones, ..., then the next few heads
   const int head = kRaw ? blockIdx.z : blockIdx.z * gridDim.x + blockIdx.x;
   if (head >= p.s.heads) return;
@@ -907,17 +975,17 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
         const int n = b->cnt[cell];
         if (n == 0) continue;
         if (phase_ord > 0) wait<kMmaRole>(&b->wc, &b->q_free, (phase_ord - 1) & 1, 1);
-        const int qbytes = cell == kNv ? (int)rec::q_nvfp4_bytes(QB, D)
-                                       : (cell == kI8 ? (int)rec::q_int8_bytes(QB, D) : (int)rec::q_fp16_bytes(QB, D));
+        const int qbytes = is<CELLS, kNv>(cell) ? (int)rec::q_nvfp4_bytes(QB, D)
+                                       : (is<CELLS, kI8>(cell) ? (int)rec::q_int8_bytes(QB, D) : (int)rec::q_fp16_bytes(QB, D));
         const uint8_t* qsrc =
-            cell == kNv ? static_cast<const uint8_t*>(p.o.q_nvfp4) + (int64_t)q_index_fp * qbytes
-            : cell == kI8 ? static_cast<const uint8_t*>(p.o.q_int8) + q_index_i8 * qbytes
+            is<CELLS, kNv>(cell) ? static_cast<const uint8_t*>(p.o.q_nvfp4) + (int64_t)q_index_fp * qbytes
+            : is<CELLS, kI8>(cell) ? static_cast<const uint8_t*>(p.o.q_int8) + q_index_i8 * qbytes
                           : static_cast<const uint8_t*>(p.o.q_fp16) + (int64_t)q_index_fp * qbytes;
         mbar_arrive_expect_tx(&b->q_full, qbytes * blocks, lead);
         if constexpr (kRaw) {
 #pragma unroll
           for (int c = 0; c < D; c += 64) tensor_g2s(q_smem + c * 256, &p.q, c, head_at, tile * 128, &b->q_full, lead);
-        } else if (cell == kNv && kQ64) {
+        } else if (is<CELLS, kNv>(cell) && kQ64) {
           // codes fill the first half of the 128-row tile; scale blocks follow the full tile.
           // A pair's second record: codes into the second half of the tile, scale blocks behind
           // the first record's (the QK warp folds them into one block before it copies them).
@@ -936,8 +1004,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
         }
         const int kvbytes = record_bytes(D, cell), kbytes = k_bytes(D, cell), rest = rest_offset(D, cell);
         const uint8_t* kvbase =
-            (cell == kNv ? static_cast<const uint8_t*>(p.o.kv_nvfp4)
-             : cell == kI8 ? static_cast<const uint8_t*>(p.o.kv_int8)
+            (is<CELLS, kNv>(cell) ? static_cast<const uint8_t*>(p.o.kv_nvfp4)
+             : is<CELLS, kI8>(cell) ? static_cast<const uint8_t*>(p.o.kv_int8)
                            : static_cast<const uint8_t*>(p.o.kv_fp16)) +
             (int64_t)head_at * p.stages * kvbytes;
         const int first = b->first_of[cell];
@@ -948,12 +1016,12 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
         if (g > 0) wait<kMmaRole>(&b->wc, &b->pv_done[(g - 1) & (kRing - 1)], ((g - 1) >> 3) & 1, 2);
         float q_scale[2] = {1.0f, 1.0f};
         const float* kscale = nullptr;
-        if (cell == kI8) {
+        if (is<CELLS, kI8>(cell)) {
           q_scale[0] = p.o.q_int8_scale[q_index_i8];
           if (blocks == 2) q_scale[1] = p.o.q_int8_scale[q_index_i8 + step];
           kscale = p.o.k_int8_scale + (int64_t)head_at * p.stages;
         }
-        const float base = cell == kNv ? sigma(D) * p.s.q_global_scale * p.s.k_global_scale : sigma(D);
+        const float base = is<CELLS, kNv>(cell) ? sigma(D) * p.s.q_global_scale * p.s.k_global_scale : sigma(D);
         // list entries, 32 at a time, one per lane, with their metadata
         int stage_l = 0;
         float2 meta_l[2] = {make_float2(base, 0.0f), make_float2(base, 0.0f)};
@@ -979,7 +1047,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
             }
             meta_l[0].y = __int_as_float(!pairs || ((entry >> 30) & 1) ? valid : -1);
             if (kQ64) meta_l[1].y = __int_as_float(entry < 0 || p.dense_prefix ? valid : -1);
-            if (cell == kI8) {
+            if (is<CELLS, kI8>(cell)) {
               const float ks = kscale[stage_l];
               meta_l[0].x = sigma(D) * (q_scale[0] * ks);
               if (kQ64) meta_l[1].x = sigma(D) * (q_scale[1] * ks);
@@ -1034,7 +1102,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
         }
         g += n;
         ++phase_ord;
-        moves += cell != kNv;
+        moves += !is<CELLS, kNv>(cell);
       }
       if (b->wc.abort) {
         // unwinding: the copies in flight must land before the CTA gives its shared memory back
@@ -1056,7 +1124,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
       for (int cell = kFirst; cell <= kLast; ++cell) {
         const int n = b->cnt[cell];
         if (n == 0) continue;
-        if (cell != kNv) {
+        if (!is<CELLS, kNv>(cell)) {
           wait<kMmaRole>(&b->wc, &b->q_moved, moves & 1, 3);
           ++moves;
         } else {
@@ -1068,7 +1136,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
         const uint32_t base_addr = split_kv(D, cell) ? smem_u32(smem) : ring_addr;
         const uint64_t base = kRaw ? swizzled_desc(base_addr, 16) : k_desc(D, cell, base_addr);
         const uint64_t q_desc = k_desc(D, kNv, q_addr);
-        if (cell == kNv) {
+        if (is<CELLS, kNv>(cell)) {
           if ((kReread ? b->tile_blocks : tile_blocks) == 2) {
             // Scale bytes of rows 0-63 sit in the low eight bytes of every 16-byte chunk, those of
             // rows 64-127 in the high eight.  Both records hold their 64 rows in the low halves:
@@ -1105,9 +1173,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
           tc_fence_after_sync();
           if (leader) {
             const uint32_t tmem_s = tmem + (sb ? kColS1 : kColS), step = slot * (stride / 16);
-            if (cell == kI8) {
+            if (is<CELLS, kI8>(cell)) {
               issue_qk<D, kI8>(tmem_s, tmem, q_desc, base, step);
-            } else if (cell == kNv) {
+            } else if (is<CELLS, kNv>(cell)) {
               issue_qk<D, kNv>(tmem_s, tmem, q_desc, base, step);
             } else {
               issue_qk<D, kF16, RAW>(tmem_s, tmem, q_desc, base, step);
@@ -1150,15 +1218,15 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
           if (leader) {
             const uint64_t pd = moved(p_base, slot * (stride / 16));
             const uint64_t vd = moved(v_base, (split_kv(D, cell) ? i & 1 : slot) * (stride / 16));
-            if (cell == kI8) {
+            if (is<CELLS, kI8>(cell)) {
               issue_pv<D, kI8>(tmem, pd, vd, g > 0);
-            } else if (cell == kNv) {
+            } else if (is<CELLS, kNv>(cell)) {
               issue_pv<D, kNv>(tmem, pd, vd, g > 0);
             } else {
               issue_pv<D, kF16, RAW>(tmem, pd, vd, g > 0);
             }
             mma_commit(&b->pv_done[g & (kRing - 1)]);
-            if (CELLS == kAny && cell == kNv && i == n - 1) mma_commit(&b->nv_done);
+            if (kMixed && is<CELLS, kNv>(cell) && i == n - 1) mma_commit(&b->nv_done);
           }
           __syncwarp();
           slot = slot + 1 == nslot ? 0 : slot + 1;
@@ -1183,15 +1251,15 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
     for (int cell = kFirst; cell <= kLast; ++cell) {
       const int n = b->cnt[cell];
       if (n == 0) continue;
-      const bool change = CELLS == kAny && prev_cell >= 0;
+      const bool change = kMixed && prev_cell >= 0;
       if (change) {
         // per-channel factor that moves O from the previous phase's domain into this one's
         asm volatile("bar.sync 5, 128;" ::: "memory");
         const float* vscale = kReread ? p.o.v_e4m3_scale + (int64_t)b->head * D : vscale_kept;
         if (row < D) {
-          const float from = prev_cell == kNv ? nv_dom
-                                              : (prev_cell == kI8 ? vscale[row] * 0.0022326917f : 1.0f);
-          const float to = cell == kI8 ? vscale[row] * 0.0022326917f : 1.0f;
+          const float from = is<CELLS, kNv>(prev_cell) ? nv_dom
+                                              : (is<CELLS, kI8>(prev_cell) ? vscale[row] * 0.0022326917f : 1.0f);
+          const float to = is<CELLS, kI8>(cell) ? vscale[row] * 0.0022326917f : 1.0f;
           colf[row] = to == 0.0f ? 0.0f : from / to;
           if (kFactors == 2) colf[D + row] = nv_dom;  // from NVFP4 into FP16 for a block without the phase between
         }
@@ -1199,12 +1267,12 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
       }
       const int factors = kFactors == 2 && change ? b->move[row >= QB][cell - kI8] : 0;
       const bool moves = change && (kFactors == 1 || factors != kStays);
-      if (cell != kNv) {
+      if (!is<CELLS, kNv>(cell)) {
         // Q into tensor memory.  Its columns are free: the INT8 phase's Q has been read when the record
         // that takes its place in shared memory arrives, the NVFP4 phase's scale factors below.
-        if (CELLS == kAny && b->cnt[kNv] > 0) wait<kRescaleRole>(&b->wc, &b->nv_done, 0, 31);
+        if (kMixed && b->cnt[kNv] > 0) wait<kRescaleRole>(&b->wc, &b->nv_done, 0, 31);
         wait<kRescaleRole>(&b->wc, &b->q_full, phase_ord & 1, 32);
-        const int chunks = cell == kI8 ? D / 16 : D / 8;
+        const int chunks = is<CELLS, kI8>(cell) ? D / 16 : D / 8;
 #pragma unroll 1
         for (int c = 0; c < chunks; c += 2) {
           uint32_t r[8];
@@ -1272,7 +1340,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
       int slot = first_slot(D, cell) + first;
 #pragma unroll 1
       for (int i = first; i < n; i += 2) {
-        softmax_stage<D, kQ64, kQ64 && CELLS != kAny, RAW>(b, p_row + slot * stride, tmem_row, row, g + i, cell, live_warp,
+        softmax_stage<D, CELLS, kQ64, kQ64 && !kMixed, RAW>(b, p_row + slot * stride, tmem_row, row, g + i, cell, live_warp,
                                                         my_block, w);
         slot += 2;
         if (slot >= nslot) slot -= nslot;
@@ -1347,8 +1415,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
               // warp's, each is waited for, 3 us of a small call: 7 heads x 2,293 tokens, D = 128 65.3, now 62.1)
               float factor[8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) factor[i] = last_cell == kNv ? nv_dom : 1.0f;
-              if (last_cell == kI8) {
+              for (int i = 0; i < 8; ++i) factor[i] = is<CELLS, kNv>(last_cell) ? nv_dom : 1.0f;
+              if (is<CELLS, kI8>(last_cell)) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) factor[i] = vscale[c0 + j + i] * 0.0022326917f;
               }
@@ -1358,8 +1426,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 f[i] = __uint_as_float(r[j + i]);
-                if (last_cell == kNv) f[i] *= nv_dom;
-                if (last_cell == kI8) f[i] *= vscale[c0 + j + i] * 0.0022326917f;
+                if (is<CELLS, kNv>(last_cell)) f[i] *= nv_dom;
+                if (is<CELLS, kI8>(last_cell)) f[i] *= vscale[c0 + j + i] * 0.0022326917f;
                 f[i] *= inv;
               }
             }
@@ -1426,19 +1494,19 @@ int launch_kernel(AttnParams& p, int tiles, size_t smem, cudaStream_t st) {
 
 template <int D, bool kQ64>
 int launch(AttnParams& p, int tiles, cudaStream_t st) {
-  int q_region = 0, slot = 0, cells = 0, one = kAny;
+  int q_region = 0, slot = 0;
   const bool use[3] = {p.s.has_nvfp4 && !p.dense_prefix, p.s.has_int8 != 0, p.s.has_fp16 && !p.dense_prefix};
   for (int cell = 0; cell < 3; ++cell) {
     if (!use[cell]) continue;
-    one = cells++ == 0 ? cell : kAny;
     // a pair of Q64 blocks brings a second set of scale blocks
     q_region = max(q_region, cell == kNv ? 128 * D / 2 + (D / 64) * 512 * (p.pair_counts || p.pair_table ? 2 : 1)
                                          : (cell == kI8 ? 128 * D : 256 * D));
     slot = max(slot, slot_bytes(D, cell));
   }
-  // Prefix tiles run beside video tiles: of a mixed call in the same kernel, so that an SM's CTAs share
-  // their code in the instruction cache.
-  if (p.dense_prefix && (p.s.has_nvfp4 || p.s.has_fp16)) one = kAny;
+  // Prefix tiles run beside video tiles: in the same kernel, so that an SM's CTAs share their code in the
+  // instruction cache.
+  constexpr int kKernel[8] = {kAny, kNv, kI8, kNvI8, kF16, kNvF16, kI8F16, kAny};
+  const int one = kKernel[(p.s.has_nvfp4 != 0) + 2 * (p.s.has_int8 != 0) + 4 * (p.s.has_fp16 != 0)];
   q_region = (q_region + 127) & ~127;
   const int fixed = q_region + factor_sets(one, kQ64) * D * 4 + (int)sizeof(Shared);
   // two CTAs per SM: measured limit is 115,528 bytes of dynamic shared memory per CTA
@@ -1453,6 +1521,9 @@ int launch(AttnParams& p, int tiles, cudaStream_t st) {
     case kNv: return launch_kernel<D, kNv, kQ64>(p, tiles, smem, st);
     case kI8: return launch_kernel<D, kI8, kQ64>(p, tiles, smem, st);
     case kF16: return launch_kernel<D, kF16, kQ64>(p, tiles, smem, st);
+    case kNvI8: return launch_kernel<D, kNvI8, kQ64>(p, tiles, smem, st);
+    case kI8F16: return launch_kernel<D, kI8F16, kQ64>(p, tiles, smem, st);
+    case kNvF16: return launch_kernel<D, kNvF16, kQ64>(p, tiles, smem, st);
     default: return launch_kernel<D, kAny, kQ64>(p, tiles, smem, st);
   }
 }
