@@ -509,7 +509,6 @@ __device__ __forceinline__ float exp_any(float (&s)[64], float scale, float bias
 // and d(g) = d(g - 1) * alpha(g) + sum(g) is formed by the group that ran stage g when it publishes
 // stage g + 2 - the order (and rounding) of a strictly sequential walk.
 struct SoftmaxWalk {
-  uint32_t s_par;     // parity of this group's next scores
   float d;            // denominator before the last two stages of this group's last stage
   float alpha, sum;   // of this group's last stage
 };
@@ -526,8 +525,7 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
   uint64_t* m_full = b->m_full[row >> 5];
   const uint32_t lead = (row & 31) == 0;
   const int sb = s_buffer<D>(g);
-  wait(&b->wc, &b->s_full[g & 1], w.s_par, 10);
-  w.s_par ^= 1u;
+  wait(&b->wc, &b->s_full[g & 1], (g >> 1) & 1, 10);
   tc_fence_after_sync();
   const uint32_t tmem_s = tmem_row + (sb ? kColS1 : kColS);
   const auto store_zeros = [&]() {
@@ -1117,7 +1115,6 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
       // Uniform control flow for the whole warp; the tcgen05 instructions are one elected lane's.
       int g = 0, phase_ord = 0;
       int moves = 0;
-      uint32_t used = 0, free_par = 0;
       const bool leader = elect_one();
       const uint32_t q_addr = smem_u32(q_smem), ring_addr = smem_u32(ring);
 #pragma unroll 1
@@ -1165,11 +1162,8 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
         for (int i = 0; i < n; ++i, ++g) {
           const int sb = s_buffer<D>(g);
           wait<kMmaRole>(&b->wc, &b->kv_full[g & (kRing - 1)], (g >> 3) & 1, 4);
-          if ((used >> sb) & 1u) {
-            wait<kMmaRole>(&b->wc, &b->s_free[sb], (free_par >> sb) & 1u, 5);
-            free_par ^= 1u << sb;
-          }
-          used |= 1u << sb;
+          // (the buffer's scores before: of the stage before, or, with two buffers, the one before that)
+          if (g > (D == 64)) wait<kMmaRole>(&b->wc, &b->s_free[sb], (D == 64 ? (g >> 1) - 1 : g - 1) & 1, 5);
           tc_fence_after_sync();
           if (leader) {
             const uint32_t tmem_s = tmem + (sb ? kColS1 : kColS), step = slot * (stride / 16);
@@ -1320,7 +1314,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
     const int row = (warp & 3) * 32 + lane;  // query row == TMEM lane
     const int parity = warp >> 2;            // which stages this warpgroup runs
     const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    SoftmaxWalk w{0u, 0.0f, 1.0f, 0.0f};
+    SoftmaxWalk w{0.0f, 1.0f, 0.0f};
     int g = 0, last_cell = kFirst;
     const int blocks = kReread ? b->tile_blocks : tile_blocks;
     const bool live_warp = !kQ64 || (warp & 3) * 32 < QB * blocks;
