@@ -1310,6 +1310,15 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
     if (kRaw) cluster_sync();
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS>::kSoftmax));
+    // Formed anew where that leaves the loop more registers: what is derived from the pointer that all roles have is
+    // kept from the kernel's start.  Kept / anew, us: FP16 D = 128 Q64 30 heads x 8,415 tokens 426 / 417, 16 x 14,296 575 / 557;
+    // INT8 D = 64 Q128 8 x 15,400 255 / 240, Q64 14 x 32,760 1,435 / 1,381; INT8 + FP16 D = 128 56 x 33,272 8,388 / 8,234.  With
+    // NVFP4 0 to 3 % slower, INT8 + FP16 D = 128 Q64 572 / 577.
+    constexpr bool kAnew = !has_cell(CELLS, kNv) && !(CELLS == kI8F16 && D == 128 && kQ64);
+    uint32_t b_at = p.q_region + p.ring_bytes + kFactors * D * 4;
+    if (kAnew) asm volatile("" : "+r"(b_at));
+    Shared* const b_kept = b;
+    Shared* const b = kAnew ? reinterpret_cast<Shared*>(smem + b_at) : b_kept;
     // =============================== softmax rows ===============================
     const int row = (warp & 3) * 32 + lane;  // query row == TMEM lane
     const int parity = warp >> 2;            // which stages this warpgroup runs
