@@ -164,9 +164,9 @@ struct AttnParams {
 // shared memory.  Alone, us, torch's attention (cuDNN for bf16) / one CTA per tile / parts: bf16 D = 128 3 heads x 7,159
 // tokens, 517 rows 84 / 83 / 30, 16 x 14,296, 256 rows 160 / 163 / 53, 7 x 33,272, 512 rows 350 / 357 / 101, 1 x 85,000,
 // 30 rows 1,297 / 845 / 118; fp16 D = 64 6 x 33,178, 58 rows 567 / 282 / 45.  Where rows and heads fill the GPU the library
-// is ahead (56 x 33,272, 512 rows 408 / 603 / 592).  Whole calls, of which these rows are a part beside the others: small
-// ones 100 -> 31-60 us (its host work alone took 90), 48 x 2,474 169 -> 161, 16 x 14,296 589 -> 580, 30 x 10,198 with 958 rows
-// 873 -> 909, 32 x 41,955 with 780 rows 6,170 -> 6,310.
+// is ahead (56 x 33,272, 512 rows 408 / 603 / 592), and long prefixes of long sequences are left to it.  Whole calls, of
+// which these rows are a part beside the others: small ones 100 -> 31-60 us (its host work alone took 90), 48 x 2,474 169 ->
+// 161, 8 x 3,360 with 210 rows 107 -> 61.
 struct alignas(64) RawParams : AttnParams {
   CUtensorMap q, k, v;  // [tokens][heads][D] as they lie in memory: 64 channels x 1 head x 64 tokens (Q: 128), swizzled
   int rows, tokens_in, parts;

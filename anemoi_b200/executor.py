@@ -17,6 +17,7 @@ import math
 from functools import lru_cache
 
 import torch
+import torch.nn.functional as F
 
 from . import native
 from .api import NVFP4Calibration, QuantConfig, SparseConfig, VisualLayout
@@ -236,13 +237,17 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
 
     frames, height, width = video_shape
     current = torch.cuda.current_stream(device)
-    side = _prefix_stream(device) if native_prefix else _dense_stream(device)
+    library_prefix = _library_prefix(native_prefix, prefix_tokens, q_bshd.size(1), q_bshd.size(3))
+    side = _prefix_stream(device) if native_prefix or library_prefix else _dense_stream(device)
     prefix_out = None
     if prefix_tokens and not native_prefix:
         # dense attention of the prefix rows on the caller's tensors, as the reference does
         side.wait_stream(current)
         with torch.cuda.stream(side), _Range("anemoi.dense_prefix", nvtx):
-            prefix_out = native.dense_rows(q_bshd, k_bshd, v_bshd, prefix_tokens, _status_word(device))
+            if library_prefix:
+                prefix_out = _library_rows(q_bshd, k_bshd, v_bshd, prefix_tokens)
+            else:
+                prefix_out = native.dense_rows(q_bshd, k_bshd, v_bshd, prefix_tokens, _status_word(device))
 
     layout = materialize_ragged_2d_layout(device, frames=frames, height=height, width=width,
                                           logical_block=query_block_size, enable_anchors=enable_anchors)
@@ -311,6 +316,22 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
     return out
 
 
+def _library_prefix(native_prefix: bool, prefix_tokens: int, tokens: int, dim: int) -> bool:
+    # Long prefixes of long sequences are left to torch's attention, by their lengths alone so that a head's rows do not
+    # depend on the others: where many heads fill the GPU its tiles cost less, and leave SMs to the preparation beside them.
+    # Whole calls, us, library / own kernel, D = 128, heads 4, 14 and 40: 16,112 tokens of which 512 are prefix 212 / 205, 613 /
+    # 637, 1,751 / 1,766; 8,200 of 400 (14) 237 / 247; 8,312 of 512 (40) 641 / 675; 5,680 of 1,000 (24) 275 / 295.  Shorter
+    # ones: 5,192 of 512 101 / 66, 142 / 137, 358 / 359; 3,632 of 512 101 / 52, 105 / 97, 220 / 229; 384 rows of 15,984 209 / 200,
+    # 599 / 608, 1,676 / 1,679 and fewer always ahead.  At D = 64 the library is half as quick: 18 x 9,514, 658 rows 330 / 311.
+    return not native_prefix and dim == 128 and prefix_tokens > 384 and prefix_tokens * tokens >= 3 << 20
+
+
+def _library_rows(q, k, v, prefix_tokens):
+    return F.scaled_dot_product_attention(
+        q[:, :prefix_tokens].permute(0, 2, 1, 3), k.permute(0, 2, 1, 3), v.permute(0, 2, 1, 3),
+        dropout_p=0.0, is_causal=False)[0].contiguous()
+
+
 class _Plan:
     """The native plan of one configuration with the tensors it points to."""
 
@@ -347,7 +368,9 @@ class _Plan:
         self.bytes = int(lib.anemoi_sm100_layer_workspace_bytes(self.ref))
         if self.bytes < 0:
             raise RuntimeError("invalid attention shape")
-        self.side = (_prefix_stream if self.native_prefix else _dense_stream)(device) if prefix_tokens else None
+        self.library_prefix = _library_prefix(self.native_prefix, prefix_tokens, tokens, dim)
+        high = self.native_prefix or self.library_prefix
+        self.side = (_prefix_stream if high else _dense_stream)(device) if prefix_tokens else None
         self.side_handle = self.side.cuda_stream if prefix_tokens else None
         self.uses_scales = "nvfp4" in active
         # kernels per call: preparation (with V's maxima and their zeroes), draft, routing (and pair lists), attention, prefix rows
@@ -387,11 +410,21 @@ def _one_call(q, k, v, prefix_tokens, sparsity, nvfp4, int8, fp16, video_shape, 
 
 
 def _launch(plan, q, k, v, device, strides, scales):
+    prefix_ptr, prefix_rows, prefix_kind = None, 0, native.PREFIX_DENSE
+    if plan.library_prefix:
+        current = torch.cuda.current_stream(device)
+        plan.side.wait_stream(current)
+        prefix_rows = plan.struct.shape.prefix_tokens
+        with torch.cuda.stream(plan.side):
+            prefix_out = _library_rows(q, k, v, prefix_rows)
+        prefix_out.record_stream(current)
+        prefix_ptr, prefix_kind = prefix_out.data_ptr(), 1
     workspace = torch.empty(plan.bytes, dtype=torch.uint8, device=device)
     out = torch.empty(q.shape, dtype=q.dtype, device=device)
     code = plan.call(
-        plan.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, scales, None, 0, native.PREFIX_DENSE,
-        out.data_ptr(), workspace.data_ptr(), plan.bytes, torch._C._cuda_getCurrentRawStream(device.index), plan.side_handle)
+        plan.ref, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, scales, prefix_ptr, prefix_rows,
+        prefix_kind, out.data_ptr(), workspace.data_ptr(), plan.bytes,
+        torch._C._cuda_getCurrentRawStream(device.index), plan.side_handle)
     if code != 0:
         native._check(code, "anemoi_sm100_layer")
     native._count("layer", plan.launches)

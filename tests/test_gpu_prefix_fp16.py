@@ -99,3 +99,25 @@ def test_heads_alone_and_in_host_groups_equal_one_call(native_library, query_blo
            quant_config=QuantConfig(*cells, "fp16", "fp16"), calibration=NVFP4Calibration(0.01, 0.01, 0.002))
     torch.cuda.synchronize()
     assert torch.equal(out, whole.cpu())
+
+
+@pytest.mark.parametrize("prefix, tokens, library", [(384, 8192, False), (385, 8171, True), (385, 8170, False)])
+def test_both_sides_of_the_library_rule(native_library, prefix, tokens, library):
+    """Prefixes on both sides of the line from which they are left to torch: the same rows to rounding, in both paths of a
+    call, with the heads together or alone."""
+    from anemoi_b200 import executor
+
+    heads, dim = 2, 128
+    gen = torch.Generator(device="cuda").manual_seed(prefix)
+    q, k, v = (torch.randn(1, tokens, heads, dim, generator=gen, device="cuda").bfloat16() for _ in range(3))
+    kw = dict(prefix_tokens=prefix, sparsity_ratio=0.9, retained_nvfp4_ratio=0.0, retained_int8_ratio=0.0,
+              retained_fp16_ratio=1.0, video_shape=(1, 1, tokens - prefix), layer=0, query_block_size=128,
+              prefix_kv_precision="fp16", prefix_query_precision="fp16")
+    assert executor._library_prefix(False, prefix, tokens, dim) == library
+    out = executor.sm100_ragged_attention(q, k, v, **kw)
+    staged, _ = executor.sm100_ragged_attention(q, k, v, return_parts=True, **kw)
+    assert torch.equal(out, staged)
+    assert torch.equal(out[:, :, 1:], executor.sm100_ragged_attention(q[:, :, 1:], k[:, :, 1:], v[:, :, 1:], **kw))
+    scores = torch.einsum("bqhd,bkhd->bhqk", q[:, :prefix].double(), k.double()) / dim ** 0.5
+    want = torch.einsum("bhqk,bkhd->bqhd", scores.softmax(-1), v.double())
+    assert (out[:, :prefix].double() - want).norm() / want.norm() < 2 ** -8
