@@ -118,6 +118,26 @@ __device__ __forceinline__ bool is(int cell) {
   else return cell == WHICH;
 }
 
+// What the roles keep in registers, kernel by kernel.  A loop that lacks registers is the better for a parity that follows
+// from the stage's number, or for a pointer formed anew; one that has them loses by it.  Same results bit for bit.  us at
+// 16 heads x 14,040, 9 x 6,528 and 30 x 8,415 tokens, the GPU kept busy for 40 ms per time:
+// - FP16 D = 128 Q64, parity of the scores from the number 540 / 117 / 431, kept 514 / 114 / 404 (Q128 475 / 92 / 378 and 467 /
+//   92 / 378); mixed kernels the other way (NVFP4 + INT8 D = 128 Q128 kept 454 / 119 / 403, from the number 445 / 115 / 389),
+//   and dense rows (NVFP4 + FP16 40 x 8,056, 256 prefix rows 597 and 594).
+__host__ __device__ constexpr bool keeps_s_parity(int d, int cells, bool raw) { return d == 128 && cells == kF16 && !raw; }
+// - three cells D = 128 Q128, parities of the QK warp from the number 552 / 129 / 454, kept 548 / 129 / 451; others 0 to 1 %
+//   slower if kept.
+__host__ __device__ constexpr bool keeps_free_parity(int d, int cells, bool q64) { return d == 128 && cells == kAny && !q64; }
+// - pointer kept / anew: INT8 D = 128 Q128 393 / 95 / 330 and 394 / 94 / 334, D = 64 Q64 378 / 98 / 307 and 367 / 98 / 300; FP16
+//   D = 64 Q64 364 / 94 / 294 and 360 / 92 / 292; NVFP4 + INT8 D = 128 Q128 445 / 115 / 389 and 442 / 113 / 388, D = 64 Q128 380 /
+//   94 / 319 and 383 / 95 / 321; INT8 + FP16 D = 64 Q64 455 / 117 / 430 and 449 / 115 / 425; three cells D = 128 Q64 665 / 158 /
+//   621 and 661 / 158 / 615, Q128 552 / 129 / 454 and 561 / 130 / 465.  INT8 D = 64 Q128 goes both ways: 338 / 79 / 272 and 340 /
+//   77 / 274, 14 x 32,760 1,292 / 1,303, 8 x 15,400 255 / 240, 7 x 7,200 67.5 / 68.6.
+__host__ __device__ constexpr bool pointer_anew(int d, int cells, bool q64) {
+  if (d == 64) return q64 ? cells != kNv : cells == kF16 || cells == kI8F16 || cells == kNvF16;
+  return q64 ? cells == kAny : cells == kNvI8 || cells == kI8F16;
+}
+
 // Kernels for dense rows of the caller's own tensors (prefix queries kept out of the cells), and their type.
 enum Raw : int { kNone = 0, kRawF16 = 1, kRawBf16 = 2 };
 
@@ -509,6 +529,7 @@ __device__ __forceinline__ float exp_any(float (&s)[64], float scale, float bias
 // and d(g) = d(g - 1) * alpha(g) + sum(g) is formed by the group that ran stage g when it publishes
 // stage g + 2 - the order (and rounding) of a strictly sequential walk.
 struct SoftmaxWalk {
+  uint32_t s_par;     // parity of this group's next scores, where it is kept
   float d;            // denominator before the last two stages of this group's last stage
   float alpha, sum;   // of this group's last stage
 };
@@ -525,7 +546,9 @@ __device__ __forceinline__ void softmax_stage(Shared* b, uint8_t* p_row, uint32_
   uint64_t* m_full = b->m_full[row >> 5];
   const uint32_t lead = (row & 31) == 0;
   const int sb = s_buffer<D>(g);
-  wait(&b->wc, &b->s_full[g & 1], (g >> 1) & 1, 10);
+  constexpr bool kKept = keeps_s_parity(D, CELLS, RAW != kNone);
+  wait(&b->wc, &b->s_full[g & 1], kKept ? w.s_par : (g >> 1) & 1, 10);
+  if (kKept) w.s_par ^= 1u;
   tc_fence_after_sync();
   const uint32_t tmem_s = tmem_row + (sb ? kColS1 : kColS);
   const auto store_zeros = [&]() {
@@ -1115,6 +1138,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
       // Uniform control flow for the whole warp; the tcgen05 instructions are one elected lane's.
       int g = 0, phase_ord = 0;
       int moves = 0;
+      uint32_t used = 0, free_par = 0;  // (where the parities are kept)
       const bool leader = elect_one();
       const uint32_t q_addr = smem_u32(q_smem), ring_addr = smem_u32(ring);
 #pragma unroll 1
@@ -1162,8 +1186,16 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
         for (int i = 0; i < n; ++i, ++g) {
           const int sb = s_buffer<D>(g);
           wait<kMmaRole>(&b->wc, &b->kv_full[g & (kRing - 1)], (g >> 3) & 1, 4);
-          // (the buffer's scores before: of the stage before, or, with two buffers, the one before that)
-          if (g > (D == 64)) wait<kMmaRole>(&b->wc, &b->s_free[sb], (D == 64 ? (g >> 1) - 1 : g - 1) & 1, 5);
+          if constexpr (keeps_free_parity(D, CELLS, kQ64)) {
+            if ((used >> sb) & 1u) {
+              wait<kMmaRole>(&b->wc, &b->s_free[sb], (free_par >> sb) & 1u, 5);
+              free_par ^= 1u << sb;
+            }
+            used |= 1u << sb;
+          } else {
+            // (the buffer's scores before: of the stage before, or, with two buffers, the one before that)
+            if (g > (D == 64)) wait<kMmaRole>(&b->wc, &b->s_free[sb], (D == 64 ? (g >> 1) - 1 : g - 1) & 1, 5);
+          }
           tc_fence_after_sync();
           if (leader) {
             const uint32_t tmem_s = tmem + (sb ? kColS1 : kColS), step = slot * (stride / 16);
@@ -1310,11 +1342,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
     if (kRaw) cluster_sync();
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS>::kSoftmax));
-    // Formed anew where that leaves the loop more registers: what is derived from the pointer that all roles have is
-    // kept from the kernel's start.  Kept / anew, us: FP16 D = 128 Q64 30 heads x 8,415 tokens 426 / 417, 16 x 14,296 575 / 557;
-    // INT8 D = 64 Q128 8 x 15,400 255 / 240, Q64 14 x 32,760 1,435 / 1,381; INT8 + FP16 D = 128 56 x 33,272 8,388 / 8,234.  With
-    // NVFP4 0 to 3 % slower, INT8 + FP16 D = 128 Q64 572 / 577.
-    constexpr bool kAnew = !has_cell(CELLS, kNv) && !(CELLS == kI8F16 && D == 128 && kQ64);
+    // Formed anew where that leaves the loop more registers (pointer_anew): what is derived from the pointer that all roles
+    // have is kept from the kernel's start.
+    constexpr bool kAnew = pointer_anew(D, CELLS, kQ64) || kRaw;
     uint32_t b_at = p.q_region + p.ring_bytes + kFactors * D * 4;
     if (kAnew) asm volatile("" : "+r"(b_at));
     Shared* const b_kept = b;
@@ -1323,7 +1353,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
     const int row = (warp & 3) * 32 + lane;  // query row == TMEM lane
     const int parity = warp >> 2;            // which stages this warpgroup runs
     const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    SoftmaxWalk w{0.0f, 1.0f, 0.0f};
+    SoftmaxWalk w{0u, 0.0f, 1.0f, 0.0f};
     int g = 0, last_cell = kFirst;
     const int blocks = kReread ? b->tile_blocks : tile_blocks;
     const bool live_warp = !kQ64 || (warp & 3) * 32 < QB * blocks;
