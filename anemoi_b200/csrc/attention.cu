@@ -68,17 +68,6 @@ using layer::TokenRows;
 // Four warpgroups: softmax of the even stages, softmax of the odd stages, rescale of O, and
 // loader / QK / PV (one warp each, the fourth idle).
 constexpr int kThreads = 512;
-// Registers per thread: 128 * (2 * softmax + rescale + other) == 512 * 64 (two CTAs per SM).  With 96 a
-// softmax thread spills nothing, but rescales then go 16 columns at a time.  That is the better
-// trade at D = 64 (where O is half as wide: the mixed Q64 kernel 834 -> 778 cycles per stage, FP16
-// 930 -> 846) and for NVFP4 (821 -> 796); at D = 128 FP16 and mixed lose (1,005 -> 1,071, 863 -> 899).
-constexpr int kOtherRegs = 32;
-template <int D, int CELLS>
-struct Regs {
-    static constexpr bool kWide = D == 64 || CELLS == 0;
-  static constexpr int kSoftmax = kWide ? 96 : 88, kRescale = kWide ? 32 : 48;
-  static constexpr int kRescaleColumns = kWide ? 16 : 32;
-};
 constexpr int kCorrWarp = 8;
 constexpr int kLoaderWarp = 12;
 constexpr int kQkWarp = 13;
@@ -129,14 +118,31 @@ __host__ __device__ constexpr bool keeps_s_parity(int d, int cells, bool raw) { 
 //   slower if kept.
 __host__ __device__ constexpr bool keeps_free_parity(int d, int cells, bool q64) { return d == 128 && cells == kAny && !q64; }
 // - pointer kept / anew: INT8 D = 128 Q128 393 / 95 / 330 and 394 / 94 / 334, D = 64 Q64 378 / 98 / 307 and 367 / 98 / 300; FP16
-//   D = 64 Q64 364 / 94 / 294 and 360 / 92 / 292; NVFP4 + INT8 D = 128 Q128 445 / 115 / 389 and 442 / 113 / 388, D = 64 Q128 380 /
-//   94 / 319 and 383 / 95 / 321; INT8 + FP16 D = 64 Q64 455 / 117 / 430 and 449 / 115 / 425; three cells D = 128 Q64 665 / 158 /
-//   621 and 661 / 158 / 615, Q128 552 / 129 / 454 and 561 / 130 / 465.  INT8 D = 64 Q128 goes both ways: 338 / 79 / 272 and 340 /
-//   77 / 274, 14 x 32,760 1,292 / 1,303, 8 x 15,400 255 / 240, 7 x 7,200 67.5 / 68.6.
+//   D = 64 Q64 364 / 94 / 294 and 360 / 92 / 292; NVFP4 + INT8 D = 128 Q128 445 / 115 / 389 and 442 / 113 / 388, D = 64 Q128 (with
+//   88 registers; with 96 it loses 1 %) 380 / 92 / 316 and 372 / 91 / 310; INT8 + FP16 D = 64 Q64 455 / 117 / 430 and 449 /
+//   115 / 425; three cells D = 128 Q64 665 / 158 / 621 and 661 / 158 / 615, Q128 552 / 129 / 454 and 561 / 130 / 465.  INT8
+//   D = 64 Q128 goes both ways: 338 / 79 / 272 and 340 / 77 / 274, 14 x 32,760 1,292 / 1,303, 8 x 15,400 255 / 240, 7 x 7,200
+//   67.5 / 68.6.
 __host__ __device__ constexpr bool pointer_anew(int d, int cells, bool q64) {
-  if (d == 64) return q64 ? cells != kNv : cells == kF16 || cells == kI8F16 || cells == kNvF16;
+  if (d == 64) return q64 ? cells != kNv : cells != kNv && cells != kI8 && cells != kAny;
   return q64 ? cells == kAny : cells == kNvI8 || cells == kI8F16;
 }
+
+// Registers per thread: 128 * (2 * softmax + rescale + other) == 512 * 64 (two CTAs per SM).  With 96 a
+// softmax thread spills nothing, but rescales then go 16 columns at a time.  That is the better
+// trade at D = 64 (where O is half as wide: the mixed Q64 kernel 834 -> 778 cycles per stage, FP16
+// 930 -> 846) and for NVFP4 (821 -> 796); at D = 128 FP16 and mixed lose (1,005 -> 1,071, 863 -> 899).
+// NVFP4 + INT8 D = 64 Q128, with the pointer formed anew, goes with 88: us, 96 / 88, 16 heads x 14,040 tokens 379 / 372,
+// 30 x 8,415 318 / 310, 48 x 2,442 102 / 97, 14 x 32,760 1,373 / 1,362; with 200 prefix rows 426 / 419, 369 / 361, 137 / 131,
+// 1,480 / 1,468 and, where the prefix tiles' walk is what a call takes, 2 x 11,380 163.2 / 163.6.  INT8 + FP16 and three cells
+// gain up to 7 % there too, but lose up to 3 % where prefix tiles are few and long.
+constexpr int kOtherRegs = 32;
+template <int D, int CELLS, bool kQ64>
+struct Regs {
+  static constexpr bool kWide = D == 64 ? kQ64 || CELLS != kNvI8 : CELLS == kNv;
+  static constexpr int kSoftmax = kWide ? 96 : 88, kRescale = kWide ? 32 : 48;
+  static constexpr int kRescaleColumns = kWide ? 16 : 32;
+};
 
 // Kernels for dense rows of the caller's own tensors (prefix queries kept out of the cells), and their type.
 enum Raw : int { kNone = 0, kRawF16 = 1, kRawBf16 = 2 };
@@ -825,7 +831,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
   constexpr int QB = kQ64 ? 64 : 128;
   // Kernels of one cell spill less (and are 1-5 % quicker) if the roles read again from shared memory which tile they
   // work on; those of any mix, and the ones with registers to spare, do not (4-12 % slower).
-  constexpr bool kReread = !kMixed && (kQ64 || Regs<D, CELLS>::kWide);
+  constexpr bool kReread = !kMixed && (kQ64 || Regs<D, CELLS, kQ64>::kWide);
   // CTAs start in the order x, y, z: the longest lists of a few heads, the second ones, ..., then the next few heads
   const int head = kRaw ? blockIdx.z : blockIdx.z * gridDim.x + blockIdx.x;
   if (head >= p.s.heads) return;
@@ -1265,7 +1271,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
     }
     if (kRaw) cluster_sync();  // as the softmax warps before they add up the tile's parts
   } else if (warp >= kCorrWarp) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS>::kRescale));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS, kQ64>::kRescale));
     // =============================== O rescale ===============================
     const int row = (warp - kCorrWarp) * 32 + lane;
     uint64_t* m_full = b->m_full[warp - kCorrWarp];
@@ -1330,7 +1336,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
           // O may only be touched once the previous PV is complete
           wait<kRescaleRole>(&b->wc, &b->pv_done[(g - 1) & (kRing - 1)], ((g - 1) >> 3) & 1, 20);
           tc_fence_after_sync();
-          rescale_o<D, Regs<D, CELLS>::kRescaleColumns>(tmem_row, alpha, first ? colf + factors : nullptr);
+          rescale_o<D, Regs<D, CELLS, kQ64>::kRescaleColumns>(tmem_row, alpha, first ? colf + factors : nullptr);
           tc_fence_before_sync();
         }
         m = m_new;
@@ -1341,7 +1347,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
     }
     if (kRaw) cluster_sync();
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS>::kSoftmax));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<D, CELLS, kQ64>::kSoftmax));
     // Formed anew where that leaves the loop more registers (pointer_anew): what is derived from the pointer that all roles
     // have is kept from the kernel's start.
     constexpr bool kAnew = pointer_anew(D, CELLS, kQ64) || kRaw;
