@@ -1600,14 +1600,18 @@ bool encode(CUtensorMap* map, const void* base, bool bf16, int d, int heads, int
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Parts of a tile, by the sequence alone (a head's rows are then the same whichever heads are with it).  A part costs
-// some 8 us beside its stages (half a microsecond each, twice that with two CTAs on the SM), so short sequences have
-// few; and where a head has tiles enough more parts gain little.  One / two / four / eight parts, us: 16 heads x 2,500
-// tokens, 400 rows 36 / 24 / 26 / 38, 30 x 9,000, 200 rows 108 / 62 / 53 / 73, 53 x 13,093, 37 rows 153 / 84 / 73 / 83, 7 x 33,272,
-// 512 rows 357 / 186 / 101 / 85, 7 x 85,000, 900 rows 884 / 447 / 342 / 413.
+// Parts of a tile, by the lengths of sequence and prefix alone (a head's rows are then the same whichever heads are with it).
+// A part costs some 8 us beside its stages (half a microsecond each, twice that with two CTAs on the SM), so short sequences
+// have few.  Alone, one / two / four / eight parts, us: 16 heads x 2,500 tokens, 400 rows 36 / 24 / 26 / 38, 30 x 9,000, 200
+// rows 108 / 62 / 53 / 73, 53 x 13,093, 37 rows 153 / 84 / 73 / 83, 7 x 33,272, 512 rows 357 / 186 / 101 / 85.  In a call what
+// many heads cost weighs more, and they are behind torch's attention first: more than one tile has at most two parts below
+// 256 stages, more than three only one below 96.  FP16 cells of D = 128, us, torch's attention / up to four parts / so:
+// 44 heads x 2,592 tokens, 392 rows 143 / 159 / 145, 56 x 2,080, 1,000 rows 171 / 192 / 169, 24 x 3,080, 1,000 rows 124 / 135 /
+// 121, 14 x 9,856, 256 rows 353 / 369 / 337, and where few heads want more, 6 x 3,032, 392 rows 119 / 43 / 51.
 int dense_parts(int stages, int tiles) {
+  if (tiles > 3) return stages < 96 ? 1 : 2;
   const int most = stages < 32 ? 1 : stages < 96 ? 2 : stages < 256 ? 4 : kMostParts;
-  return max(1, min(most, 16 / tiles));
+  return tiles > 1 ? min(most, stages < 256 ? 2 : 4) : most;
 }
 
 template <int D, int RAW>
@@ -1784,6 +1788,10 @@ int prefix_attention(const anemoi_sm100_shape* shape, const anemoi_sm100_operand
   return launch_for(p, tiles, st);
 }
 }  // namespace
+
+extern "C" int anemoi_sm100_dense_parts(int tokens, int rows) {
+  return rows > 0 && tokens >= rows ? dense_parts((tokens + 63) / 64, (rows + 127) / 128) : ANEMOI_SM100_EINVAL;
+}
 
 extern "C" int anemoi_sm100_dense_rows(int heads, int head_dim, int tokens, int rows, int is_bf16, const void* q,
                                        const void* k, const void* v, const int64_t* strides, void* out, int64_t out_token,

@@ -318,12 +318,14 @@ def _ragged_attention(q_bshd, k_bshd, v_bshd, *, prefix_tokens, sparsity_ratio, 
 
 def _library_prefix(native_prefix: bool, prefix_tokens: int, tokens: int, dim: int) -> bool:
     # Long prefixes of long sequences are left to torch's attention, by their lengths alone so that a head's rows do not
-    # depend on the others: where many heads fill the GPU its tiles cost less, and leave SMs to the preparation beside them.
-    # Whole calls, us, library / own kernel, D = 128, heads 4, 14 and 40: 16,112 tokens of which 512 are prefix 212 / 205, 613 /
-    # 637, 1,751 / 1,766; 8,200 of 400 (14) 237 / 247; 8,312 of 512 (40) 641 / 675; 5,680 of 1,000 (24) 275 / 295.  Shorter
-    # ones: 5,192 of 512 101 / 66, 142 / 137, 358 / 359; 3,632 of 512 101 / 52, 105 / 97, 220 / 229; 384 rows of 15,984 209 / 200,
-    # 599 / 608, 1,676 / 1,679 and fewer always ahead.  At D = 64 the library is half as quick: 18 x 9,514, 658 rows 330 / 311.
-    return not native_prefix and dim == 128 and prefix_tokens > 384 and prefix_tokens * tokens >= 3 << 20
+    # depend on the others (torch's do not either: 40 heads and 1 to 8 of them are bit-equal in both types): where many heads
+    # fill the GPU its tiles cost less, and leave SMs to the preparation beside them.  Whole calls of FP16 cells, us, library /
+    # own kernel, D = 128, heads 6, 24 and 40: 384 rows of 9,984 tokens 136 / 131, 478 / 492, 792 / 805; of 17,664 328 / 306,
+    # 1,168 / 1,218, 2,003 / 2,040.  D = 64, heads 6, 24 and 56: 512 of 9,872 147 / 141, 432 / 456, 951 / 992; 1,000 of 4,960 112 /
+    # 62, 178 / 190, 377 / 406; 14 heads, 1,000 of 17,720 528 / 559.  Shorter ones: D = 128, 6, 24 and 56 heads, 512 of 3,072 118 /
+    # 51, 111 / 95, 219 / 214; 392 of 7,192 122 / 93, 303 / 314, 675 / 692 (44 heads 540 / 567: the worst); 256 rows of 17,536
+    # 323 / 300, 1,146 / 1,162, 2,681 / 2,652, and fewer are the own kernel's.  The line is the same for both head dims.
+    return not native_prefix and prefix_tokens > 256 and prefix_tokens * tokens > 3 << 20
 
 
 def _library_rows(q, k, v, prefix_tokens):

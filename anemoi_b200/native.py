@@ -109,6 +109,7 @@ def library() -> C.CDLL:
         "anemoi_sm100_prefix_attention": (C.c_int, [SP, OP, P, P, P, P]),
         "anemoi_sm100_dense_rows": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, P, P, P, C.POINTER(I64), P,
                                               I64, I64, P, P]),
+        "anemoi_sm100_dense_parts": (C.c_int, [C.c_int, C.c_int]),
         "anemoi_sm100_route_pairs": (C.c_int, [SP, P, I64, I64, I64, C.c_int, P, P, P, P, I64, P]),
         "anemoi_sm100_routes_in_one_kernel": (C.c_int, [SP]),
         "anemoi_sm100_drafts_in_routing": (C.c_int, [SP]),
@@ -167,7 +168,8 @@ EXPORTED = (
     "anemoi_sm100_prepare_zero_kernels", "anemoi_sm100_pair_bits_bytes", "anemoi_sm100_route_matched",
     "anemoi_sm100_attention_matched", "anemoi_sm100_head_groups",
     "anemoi_sm100_route_anchored", "anemoi_sm100_route_anchored_scratch_bytes",
-    "anemoi_sm100_prefix_attention", "anemoi_sm100_dense_rows", "anemoi_sm100_assemble", "anemoi_sm100_pack_qkv",
+    "anemoi_sm100_prefix_attention", "anemoi_sm100_dense_rows", "anemoi_sm100_dense_parts", "anemoi_sm100_assemble",
+    "anemoi_sm100_pack_qkv",
     "anemoi_sm100_merge_heads", "anemoi_sm100_pack_qkv_heads", "anemoi_sm100_merge_heads_into",
     "anemoi_sm100_tensor_peak", "anemoi_sm100_qknorm_rope", "anemoi_sm100_set_wait_limit_ns",
     "anemoi_sm100_wait_selftest", "anemoi_sm100_copy_rows", "anemoi_sm100_push_qkv",

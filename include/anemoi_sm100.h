@@ -262,6 +262,8 @@ int anemoi_sm100_prefix_attention(const anemoi_sm100_shape* shape,
 int anemoi_sm100_dense_rows(int heads, int head_dim, int tokens, int rows, int is_bf16, const void* q, const void* k,
                             const void* v, const int64_t* strides, void* out, int64_t out_token, int64_t out_head,
                             int32_t* status, void* stream);
+/* CTAs that share the keys of 128 of those rows, by the lengths alone: what their sums' order depends on. */
+int anemoi_sm100_dense_parts(int tokens, int rows);
 
 /* One whole call, from raw Q/K/V to the output in token order: prepare, draft_probability, route (and
  * pair_lists), attention and the prefix rows, with the attention's results written straight to their
