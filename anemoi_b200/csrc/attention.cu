@@ -86,6 +86,7 @@ constexpr int kSplitKeys = 4, kSplitValues = 2;  // key and value buffers of pha
 constexpr int kMostParts = 8;    // CTAs that share the stages of a tile of dense rows: a portable cluster
 constexpr float kFp8Offset = 8.807f;
 constexpr float kLowest = -3.0e38f;  // maximum before the first stage of dense rows
+constexpr float kNoPart = -1.0f;     // denominator of a part that its CTA did not walk
 constexpr uint64_t kDrainNs = 100000000;  // limit of the waits for copies and MMAs in flight after a give-up
 
 // log2(e) / sqrt(D)
@@ -769,7 +770,7 @@ __device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, i
 }
 
 // The rows of a tile from the parts that the CTAs of the cluster left in their shared memory (softmax threads; a CTA
-// takes every parts-th row): O = sum of O_i 2^(m_i - M), the denominator alike.
+// takes every parts-th row): O = sum of O_i 2^(m_i - M), the denominator alike.  No row of a tile that misses a part.
 template <int D, int RAW>
 __device__ __forceinline__ void add_parts(const RawParams& p, const uint8_t* smem, int head, int tile) {
   constexpr int kPieces = D / 8;
@@ -779,12 +780,14 @@ __device__ __forceinline__ void add_parts(const RawParams& p, const uint8_t* sme
     const int row = (i / kPieces) * p.parts + (int)blockIdx.x, piece = i % kPieces;
     if (row >= 128 || tile * 128 + row >= p.rows) break;
     float2 md[kMostParts];
-    float m = kLowest;
+    float m = kLowest, least = 0.0f;
 #pragma unroll
     for (int c = 0; c < kMostParts; ++c) {
       md[c] = c < p.parts ? peer_float2(base + 512 * D + row * 8, c) : make_float2(kLowest, 0.0f);
       m = fmaxf(m, md[c].x);
+      least = fminf(least, md[c].y);
     }
+    if (least == kNoPart) break;  // a CTA left over a set status word: the rows stay as they are
     float d = 0.0f, o[8] = {};
 #pragma unroll
     for (int c = 0; c < kMostParts; ++c) {
@@ -897,8 +900,10 @@ __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_con
   // time, and if only some warps of this one left, the others would go on without tensor memory, without
   // barriers or with a warpgroup short of the warps its setmaxnreg waits for.
   if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t*>(p.status) != 0)) {
-    if (kRaw) {
-      // (the other CTAs of the cluster may have seen the word clear: they read this one's shared memory)
+    if constexpr (kRaw) {
+      // The other CTAs of the cluster may have seen the word clear.  They meet this one at two barriers (before they add up
+      // the parts and before they leave: each role passes exactly these), and find here that this part is missing.
+      if (threadIdx.x < 128) reinterpret_cast<float2*>(smem + 512 * D)[threadIdx.x] = make_float2(kLowest, kNoPart);
       cluster_sync();
       cluster_sync();
     }
