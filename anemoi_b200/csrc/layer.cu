@@ -136,6 +136,13 @@ bool valid(const anemoi_sm100_layer_plan* p) {
 
 }  // namespace
 
+extern "C" int anemoi_sm100_stream_create(void** stream) {
+  return stream == nullptr ? ANEMOI_SM100_EINVAL
+         : cudaStreamCreateWithFlags(reinterpret_cast<cudaStream_t*>(stream), cudaStreamNonBlocking) == cudaSuccess
+             ? ANEMOI_SM100_OK
+             : ANEMOI_SM100_ELAUNCH;
+}
+
 extern "C" int anemoi_sm100_routes_in_one_kernel(const anemoi_sm100_shape* shape) {
   return rec::validate_shape(shape) == ANEMOI_SM100_OK && layer::routes_pairs(*shape);
 }

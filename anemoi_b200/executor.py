@@ -111,7 +111,8 @@ def _prefix_stream(device: torch.device) -> torch.cuda.Stream:
 def _dense_stream(device: torch.device) -> torch.cuda.Stream:
     # FP16 prefix rows need nothing but the caller's tensors and start with the call, so at a high priority they would
     # hold up preparation, draft map and routing, which everything else waits for (33 heads x 4,989 tokens 275 us, so 259).
-    return torch.cuda.Stream(device=device, priority=0)
+    # Not of torch's 32 at that priority: a caller's own streams, and the copy streams of HostAttention, are among them.
+    return native.own_stream(device)
 
 
 @lru_cache(maxsize=64)

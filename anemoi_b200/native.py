@@ -110,6 +110,7 @@ def library() -> C.CDLL:
         "anemoi_sm100_dense_rows": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, P, P, P, C.POINTER(I64), P,
                                               I64, I64, P, P]),
         "anemoi_sm100_dense_parts": (C.c_int, [C.c_int, C.c_int]),
+        "anemoi_sm100_stream_create": (C.c_int, [C.POINTER(P)]),
         "anemoi_sm100_route_pairs": (C.c_int, [SP, P, I64, I64, I64, C.c_int, P, P, P, P, I64, P]),
         "anemoi_sm100_routes_in_one_kernel": (C.c_int, [SP]),
         "anemoi_sm100_drafts_in_routing": (C.c_int, [SP]),
@@ -163,7 +164,8 @@ EXPORTED = (
     "anemoi_sm100_route_list_capacity", "anemoi_sm100_route", "anemoi_sm100_route_static",
     "anemoi_sm100_route_static_max_bytes", "anemoi_sm100_attention",
     "anemoi_sm100_attention_pairs", "anemoi_sm100_pair_lists", "anemoi_sm100_route_pairs",
-    "anemoi_sm100_layer", "anemoi_sm100_layer_workspace_bytes", "anemoi_sm100_routes_in_one_kernel",
+    "anemoi_sm100_layer", "anemoi_sm100_layer_workspace_bytes", "anemoi_sm100_stream_create",
+    "anemoi_sm100_routes_in_one_kernel",
     "anemoi_sm100_drafts_in_routing", "anemoi_sm100_matches_pairs", "anemoi_sm100_prepare_kernels",
     "anemoi_sm100_prepare_zero_kernels", "anemoi_sm100_pair_bits_bytes", "anemoi_sm100_route_matched",
     "anemoi_sm100_attention_matched", "anemoi_sm100_head_groups",
@@ -466,6 +468,14 @@ def dense_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, rows: int, sta
         heads, dim, tokens, rows, int(q.dtype == torch.bfloat16), _ptr(q), _ptr(k), _ptr(v), strides, _ptr(out), dim,
         rows * dim, _ptr(status), _stream(q.device)), "anemoi_sm100_dense_rows")
     return out
+
+
+def own_stream(device: torch.device) -> torch.cuda.Stream:
+    """A new stream at the default priority that no ``torch.cuda.Stream()`` stands for: those share 32 per device."""
+    handle = C.c_void_p()
+    with torch.cuda.device(device):
+        _check(library().anemoi_sm100_stream_create(C.byref(handle)), "anemoi_sm100_stream_create")
+    return torch.cuda.ExternalStream(handle.value, device=device)
 
 
 def copy_head_group(dst: torch.Tensor, src: torch.Tensor, stream: torch.cuda.Stream) -> None:

@@ -304,6 +304,9 @@ int anemoi_sm100_attention_matched(const anemoi_sm100_shape* shape, const anemoi
                                    const int32_t* pair_ids, int64_t list_capacity, const int32_t* valid_k,
                                    void* out_packed, int32_t* status, void* stream);
 int64_t anemoi_sm100_layer_workspace_bytes(const anemoi_sm100_layer_plan* plan);
+/* A stream of the current device that waits for no other (at the default priority), as `side_stream` of a call whose prefix
+ * rows are dense rows.  The caller's to keep. */
+int anemoi_sm100_stream_create(void** stream);
 /*   strides          as for anemoi_sm100_prepare
  *   nvfp4_scales     q, k, v tensor-level scales of this call, or null for the plan's
  *   prefix_out       prefix rows computed elsewhere on `side_stream` ([H][prefix_rows][D], the caller's
