@@ -123,7 +123,11 @@ __host__ __device__ constexpr bool keeps_free_parity(int d, int cells, bool q64)
 //   88 registers; with 96 it loses 1 %) 380 / 92 / 316 and 372 / 91 / 310; INT8 + FP16 D = 64 Q64 455 / 117 / 430 and 449 /
 //   115 / 425; three cells D = 128 Q64 665 / 158 / 621 and 661 / 158 / 615, Q128 552 / 129 / 454 and 561 / 130 / 465.  INT8
 //   D = 64 Q128 goes both ways: 338 / 79 / 272 and 340 / 77 / 274, 14 x 32,760 1,292 / 1,303, 8 x 15,400 255 / 240, 7 x 7,200
-//   67.5 / 68.6.
+//   67.5 / 68.6.  The others that form it anew, at the same sizes: D = 64 Q64 NVFP4 + INT8 494 / 116 / 420 and 491 / 116 / 418,
+//   NVFP4 + FP16 503 / 114 / 425 and 502 / 114 / 425, three cells 546 / 129 / 467 and 542 / 128 / 465; D = 64 Q128 FP16 315 / 66 /
+//   269 and 317 / 66 / 273 (6 x 3,120 25.2 / 25.1, 1 x 25,600 115.1 / 114.5), INT8 + FP16 375 / 86 / 342 and 371 / 85 / 337,
+//   NVFP4 + FP16 336 / 76 / 309 and 334 / 76 / 308; D = 128 Q128 INT8 + FP16 493 / 108 / 447 and 493 / 108 / 448.  Over 110
+//   calls with a prefix of INT8 queries 1 % from it, over 130 without a prefix nothing beyond the runs' spread.
 __host__ __device__ constexpr bool pointer_anew(int d, int cells, bool q64) {
   if (d == 64) return q64 ? cells != kNv : cells != kNv && cells != kI8 && cells != kAny;
   return q64 ? cells == kAny : cells == kNvI8 || cells == kI8F16;
@@ -189,11 +193,11 @@ struct AttnParams {
 // D = 128) where there are tiles for every SM, which few calls have: a prefix is some tiles per head, each as long as the
 // head's keys, so the CTAs of a cluster (the grid's x) share a tile's stages and add up their parts through each other's
 // shared memory.  Alone, us, torch's attention (cuDNN for bf16) / one CTA per tile / parts: bf16 D = 128 3 heads x 7,159
-// tokens, 517 rows 84 / 83 / 30, 16 x 14,296, 256 rows 160 / 163 / 53, 7 x 33,272, 512 rows 350 / 357 / 101, 1 x 85,000,
-// 30 rows 1,297 / 845 / 118; fp16 D = 64 6 x 33,178, 58 rows 567 / 282 / 45.  Where rows and heads fill the GPU the library
-// is ahead (56 x 33,272, 512 rows 408 / 603 / 592), and long prefixes of long sequences are left to it.  Whole calls, of
-// which these rows are a part beside the others: small ones 100 -> 31-60 us (its host work alone took 90), 48 x 2,474 169 ->
-// 161, 8 x 3,360 with 210 rows 107 -> 61.
+// tokens, 517 rows 82 / 83 / 44, 16 x 14,296, 256 rows 158 / 163 / 86, 53 x 13,093, 37 rows 258 / 153 / 71, 1 x 85,000, 30 rows
+// 1,271 / 845 / 109; fp16 D = 64 6 x 33,178, 58 rows 564 / 282 / 44.  Where rows and heads fill the GPU the library is ahead
+// (56 x 33,272, 512 rows 408 / 603 / 597), and long prefixes of long sequences are left to it.  Whole calls, of which these
+// rows are a part beside the others: small ones 113 -> 37-58 us (its host work alone took 90), 48 x 2,474 with 74 rows 136 -> 122,
+// 8 x 3,360 with 210 rows 108 -> 44.
 struct alignas(64) RawParams : AttnParams {
   CUtensorMap q, k, v;  // [tokens][heads][D] as they lie in memory: 64 channels x 1 head x 64 tokens (Q: 128), swizzled
   int rows, tokens_in, parts;
@@ -485,7 +489,7 @@ __device__ __forceinline__ float exp_store(const float (&s)[64], float scale, fl
 // and only conversion and stores are each cell's own.  That is 64 (128 with three cells) instructions less per copy in
 // kernels whose stage code fills the instruction cache, but a piece's conversions no longer run under the next one's
 // exponentials.  Separate / shared, us: three cells of D = 64, 7 heads x 11,994 tokens 178 / 166, 8 x 12,240 NVFP4 + INT8 Q64
-// 528 / 508.  Not where FP16 with its eight stores per stage meets INT8, and not for three cells of D = 128, which are ahead
+// 528 / 508.  Not for INT8 + FP16, FP16 having eight stores per stage, and not for three cells of D = 128, which are ahead
 // by up to 2.5 % in small calls but lose 1 % in large ones (56 heads x 85,184 tokens 37.4 / 37.8 ms); in halves or with
 // two cells at a time the branches cost more than they save (5 x 3,834 three cells 71 / 74).
 __host__ __device__ constexpr bool shares(int d, int cells) {
@@ -745,14 +749,6 @@ __device__ __forceinline__ uint64_t v_desc(int d, int cell, uint32_t addr) {
 // ------------------------------------------------------------------------------------------
 // kernel
 // ------------------------------------------------------------------------------------------
-// CELLS: the cells that a stage can be of.  A kernel of one cell has that cell's code only and
-// its sizes as constants; in mixed kernels the cell is a run-time value and one copy of the
-// stage code serves all: the CTAs of an SM are in different phases, and hot code that outgrows the
-// instruction cache costs more than the constants give (three whole copies of the softmax stage,
-// 100 KB of code: 1.48 us per 64-key stage and SM at D = 64 instead of 1.11).  For the same reason two cells
-// have a kernel without the third one's code.  In the kernel for all / their own, us: NVFP4 + INT8 30 heads x 8,415 tokens
-// D = 64 Q64 473 / 416, Q128 336 / 320, D = 128 Q64 546 / 513; INT8 + FP16 17 x 7,695 D = 64 184 / 179, 47 x 8,415 D = 128 Q128
-// 582 / 566; NVFP4 + FP16 48 x 2,442 D = 64 98 / 89.
 // Where a row of the tile goes in `tokens` (element offset of its first channel), -1: a padding row.
 template <int D, bool kQ64>
 __device__ __forceinline__ int64_t token_offset(const AttnParams& p, int head, int block0, int block1, int row) {
@@ -823,6 +819,14 @@ __device__ __forceinline__ void add_parts(const RawParams& p, const uint8_t* sme
 constexpr int kStays = -1;  // in place of a block's factors: O stays in its domain
 __host__ __device__ constexpr int factor_sets(int cells, bool q64) { return mixed(cells) && q64 ? 2 : 1; }
 
+// CELLS: the cells that a stage can be of.  A kernel of one cell has that cell's code only and
+// its sizes as constants; in mixed kernels the cell is a run-time value and one copy of the
+// stage code serves all: the CTAs of an SM are in different phases, and hot code that outgrows the
+// instruction cache costs more than the constants give (three whole copies of the softmax stage,
+// 100 KB of code: 1.48 us per 64-key stage and SM at D = 64 instead of 1.11).  For the same reason two cells
+// have a kernel without the third one's code.  In the kernel for all / their own, us: NVFP4 + INT8 30 heads x 8,415 tokens
+// D = 64 Q64 473 / 416, Q128 336 / 320, D = 128 Q64 546 / 513; INT8 + FP16 17 x 7,695 D = 64 184 / 179, 47 x 8,415 D = 128 Q128
+// 582 / 566; NVFP4 + FP16 48 x 2,442 D = 64 98 / 89.
 template <int D, int CELLS, bool kQ64, int RAW = kNone>
 __global__ void __launch_bounds__(kThreads, 2) attention_kernel(const __grid_constant__ Params<RAW> p) {
   extern __shared__ __align__(1024) uint8_t smem[];

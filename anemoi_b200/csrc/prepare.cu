@@ -655,8 +655,11 @@ inline int maxima_tokens(const anemoi_sm100_shape& s) {
 inline bool zeroes_maxima(const anemoi_sm100_shape& s) {
   return s.has_int8 && !own_maxima(s) && (s.seq_tokens + maxima_tokens(s) - 1) / maxima_tokens(s) > 8;
 }
-// Beside prefix rows that the library computes on another stream, with a memset: its wait lets their few long CTAs in
-// first, each on an SM of its own; 5 heads x 19,425 tokens with 62 of prefix 494 us, with the kernel 628.
+// With FP16 prefix queries by a memset, for those that torch's attention computes on another stream: its wait lets their few
+// long CTAs in first, each on an SM of its own.  Calls of INT8 cells, us, memset / kernel: 14 heads x 10,872 tokens with 512 of
+// prefix 370 / 377, 14 x 6,940 with 700 203 / 214, 3 x 18,940 with 700 230 / 238.  Beside dense rows of this library the two are
+// alike: 8 x 2,542 with 62 49.1 / 50.2, 1 x 3,990 with 150 49.2 / 48.4, 30 x 18,782 with 62 1,639 / 1,647, 5 x 19,302 with 62
+// 305.0 / 304.5.
 inline bool zeroes_by_memset(const anemoi_sm100_shape& s) { return s.prefix_tokens > 0 && !s.has_prefix_query_int8; }
 
 template <typename InT, int QB, int D, bool kSplit, bool kOwnMaxima, Cells kCells>

@@ -3,8 +3,7 @@
 Plays the role of the reference's backend wrappers over ``torch.ops.mixed_attention.*``
 (anemoi/layers/attention/mpa/backends/sm120_q64.py, sm120_q128.py, sm89_k64.py and
 mpa/build_identity.py): one Python function per native entry point, marshaling
-tensors to raw device pointers on the current CUDA stream.  There is no fallback:
-a missing library raises.
+tensors to raw device pointers on the current CUDA stream.  A missing library raises.
 """
 
 from __future__ import annotations
